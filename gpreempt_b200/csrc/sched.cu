@@ -365,6 +365,9 @@ struct Dispatcher {
     // one): their queue drains in ~0.2 ms anyway and separate launches cost ~2 % of throughput
     // (ResNet-50 b32, 61 kernels: 11.65k -> 11.40k inf/s), whereas DenseNet-201 (373 kernels) gains
     // 80-100 us of latency-critical median latency and 3 % of its own throughput from the window.
+    // That holds for a captured graph.  Without one a whole run is one launch after another all the
+    // same, during which this loop sees no latency-critical request (61 launches take about as long
+    // as the GPU needs for a ResNet-50 of 16 images), so such a run always goes through the window.
     size_t be_window_min_kernels = 64;
 
     // A fresh best-effort run under the window: like a resume from kernel 0 with new cursors.
@@ -626,7 +629,7 @@ struct Dispatcher {
                     ++stats.be_launches;
                     stats_unlock();
                     if (be_window && t->exec && t->exec->kind == GPX_EXEC_BLP &&
-                        t->exec->model->kernels.size() > be_window_min_kernels) {
+                        (t->exec->model->kernels.size() > be_window_min_kernels || !t->exec->graph_exec)) {
                         GPX_TRY(windowed_begin(t));
                         t->state.store(ST_RESUMING, std::memory_order_release);
                         GPX_TRY(resume_continue(t, false));
