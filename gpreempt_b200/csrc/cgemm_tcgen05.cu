@@ -27,41 +27,50 @@
 #include "sm100.cuh"
 
 #include <cuda_bf16.h>
+#include <type_traits>
 
 namespace gpx {
 
 using namespace sm100;
 
 constexpr int kCBM = 128, kCBK = 64, kCUmmaK = 16;
-// Warp 0 feeds TMA, warp 1 issues MMAs, the other warps are the epilogue: kCEpiParts warps per
-// TMEM lane quarter, each taking an equal share of the columns in 16-column pieces, so that
-// enough independent TMEM loads, conversions and stores are in flight while a tile is drained
+// Warp 0 feeds TMA, warp 1 issues MMAs, warps 2..9 are the epilogue, the last warp polls the preempt
+// word: kCEpiParts epilogue warps per TMEM lane quarter, each taking an equal share of the columns,
+// so that enough independent TMEM loads, conversions and stores are in flight while a tile is drained
 // (the epilogue, not the tensor pipe, bounds the small-K layers).
 constexpr int kCEpiParts = 2;                       // epilogue warps per TMEM lane quarter
 constexpr int kCEpiThreads = 128 * kCEpiParts;
-constexpr int kCgemmThreads = 64 + kCEpiThreads;
+constexpr int kCPollWarp = 2 + kCEpiThreads / 32;
+constexpr int kCgemmThreads = 64 + kCEpiThreads + 32;
 constexpr unsigned long long kCWaitLimitNs = 2000000000ull;
-constexpr int kCPollEvery = 1;
+
+// fp32 spill area of one CTA: one accumulator buffer (at most 256 columns) of 128 rows.
+__host__ __device__ constexpr size_t cgemm_spill_floats() { return (size_t)kCBM * 256; }
 
 struct CgemmControlSize {
     unsigned char bytes[2560];  // room for CgemmControl (checked below)
 };
 
-template <int BN>
+// BN: columns of an output tile.  TWO: two-plane operands (float32 models), three products per K step;
+// otherwise one 16-bit plane and one product.
+template <int BN, bool TWO>
 struct CgemmCfg {
+    static constexpr uint32_t kPlanes = TWO ? 2 : 1;
     static constexpr uint32_t kABytes = kCBM * kCBK * 2;        // one plane of A: 16 KiB
     static constexpr uint32_t kWBytes = BN * kCBK * 2;          // one plane of W
-    static constexpr uint32_t kStageBytes = 2 * kABytes + 2 * kWBytes;
-    static constexpr int kStages = BN == 256 ? 2 : (BN == 128 ? 3 : 4);
+    static constexpr uint32_t kStageBytes = kPlanes * (kABytes + kWBytes);
+    static constexpr int kStages = (int)((192u * 1024u) / kStageBytes);  // 3..8
+    static constexpr uint32_t kWOff = kPlanes * kABytes;        // W (hi) tile inside a stage
     // ring + alignment slack + 64x64 identity tile + control block
     static constexpr uint32_t kIdentBytes = 64 * kCBK * 2;
     static constexpr size_t kSmem =
         (size_t)kStages * kStageBytes + 1024 + kIdentBytes + sizeof(CgemmControlSize);
-    // Four fp32 accumulators per tile (see the MMA issuer): hi*hi of even K steps, hi*hi of odd
-    // K steps, hi*lo, lo*hi.  256 or 512 TMEM columns, both powers of two.
-    // (256-column tiles exist for the two-accumulator plan only: 2 x 256 columns, one buffer.)
-    static constexpr int kAccs = BN == 256 ? 2 : 4;
-    static constexpr int kTmemCols = kAccs * BN;
+    // Accumulator columns of one tile: hi*hi and both cross terms for two-plane operands, one sum
+    // otherwise; two tiles' worth of them in tensor memory, so that the epilogue of one tile overlaps
+    // the K loop of the next.
+    static constexpr int kBufCols = (int)kPlanes * BN;
+    static constexpr int kTmemCols = 2 * kBufCols;
+    static_assert(kTmemCols <= 512 && kStages <= 8, "tile does not fit");
 };
 
 enum : int { CMSG_DATA = 0, CMSG_STOP = 1, CMSG_EXIT = 2, CMSG_RES = 3 };
@@ -77,9 +86,11 @@ struct CgemmControl {
     int epi_kind[2];
     int epi_k_done[2];
     int epi_go;
-    int raised;  // the word was up when this CTA started
+    int raised;      // the word was up when this CTA started
+    int word_up;     // the polling warp has seen the word raised
+    int poll_done;   // the producer is through: the polling warp returns
     int abort_flag;
-    float bias_s[2][256];  // bias of the tile each accumulator buffer holds, staged by the epilogue
+    alignas(16) float bias_s[2][256];  // bias of the tile each accumulator buffer holds, staged by the epilogue
 };
 
 static_assert(sizeof(CgemmControl) <= sizeof(CgemmControlSize), "control block outgrew its shared-memory budget");
@@ -131,11 +142,12 @@ __device__ unsigned long long g_cgemm_timing[32];
 #define TADD(slot, val)
 #endif
 
-template <int BN>
+template <int BN, bool TWO>
 __global__ void __launch_bounds__(kCgemmThreads, 1)
 cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
-    using Cfg = CgemmCfg<BN>;
+    using Cfg = CgemmCfg<BN, TWO>;
     constexpr int kStages = Cfg::kStages;
+    constexpr int kBufCols = Cfg::kBufCols;
     TCK(t_start);
     // The prologue below (barriers, tensor memory, descriptor prefetch) touches nothing a
     // predecessor kernel writes, so it runs while that kernel drains; pdl_wait() comes after it.
@@ -144,43 +156,29 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     uint32_t pad = (1024u - (raw_addr & 1023u)) & 1023u;
     unsigned char *smem = smem_raw + pad;
     // The identity tile follows the ring (1024-byte aligned, as its swizzled layout needs).
-    const uint32_t ident_off = kStages * Cfg::kStageBytes;
+    constexpr uint32_t ident_off = kStages * Cfg::kStageBytes;
     CgemmControl *ctl = reinterpret_cast<CgemmControl *>(smem + ident_off + Cfg::kIdentBytes);
     const uint32_t smem_base = smem_u32(smem);
     volatile int *abort_flag = &ctl->abort_flag;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     const int lane = threadIdx.x & 31;
     // A tile is (row block, column block, K split); splits of one output block are adjacent so
     // they run at the same time.  With k_splits == 1 a tile covers the whole K range.
     const int total_tiles = p.tiles_m * p.tiles_n * p.k_splits;
     const int all_kb = p.taps * p.cin_blocks;
-    auto tile_kb_begin = [&](int tile) { return (tile % p.k_splits) * p.kb_per_split; };
+    auto tile_kb_begin = [&](int tile) { return p.k_splits == 1 ? 0 : (tile % p.k_splits) * p.kb_per_split; };
     auto tile_kb_count = [&](int tile) {
-        int left = all_kb - (tile % p.k_splits) * p.kb_per_split;
+        int left = all_kb - tile_kb_begin(tile);
         return left < p.kb_per_split ? left : p.kb_per_split;
     };
     const bool resumable = blp.preempted != nullptr;
-    // Two-plane operands (float32 models) or one 16-bit plane (reduced-precision models).
-    const bool two_plane = p.fmt == PF_SPLIT;
-    // A ring stage holds the A and W tiles of one K block: hi and lo planes of both for float32
-    // models; single-plane models use half of that per stage and get twice as many stages, which
-    // doubles the bytes TMA keeps in flight.
-    const int nst = two_plane ? kStages : 2 * kStages;
-    const uint32_t stage_bytes = two_plane ? Cfg::kStageBytes : Cfg::kStageBytes / 2;
-    const uint32_t w_off = two_plane ? 2 * Cfg::kABytes : Cfg::kABytes;  // W (hi) tile inside a stage
-    // Accumulator plan.  dual: two accumulators per tile (BN columns each) in two buffers, so the
-    // epilogue of one tile overlaps the K loop of the next; used when the K range is short or the
-    // operands are single-plane.  Otherwise four accumulators in one buffer (see the MMA issuer).
-    const bool dual = p.dual != 0;
-    const int nbuf = (dual && 4 * BN <= 512) ? 2 : 1;
-    const int buf_cols = dual ? 2 * BN : Cfg::kTmemCols;
 
     CgemmSlot *slot = p.slots + blockIdx.x;
-    float *spill = p.spill + (size_t)blockIdx.x * (kCBM * Cfg::kTmemCols);
+    float *spill = p.spill + (size_t)blockIdx.x * cgemm_spill_floats();
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < nst; ++s) {
+        for (int s = 0; s < kStages; ++s) {
             mbar_init(smem_u32(&ctl->full[s]), 1);
             mbar_init(smem_u32(&ctl->empty[s]), 1);
         }
@@ -193,11 +191,13 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         ctl->abort_flag = 0;
         ctl->epi_go = 0;
         ctl->raised = 0;
+        ctl->word_up = 0;
+        ctl->poll_done = 0;
         fence_barrier_init();
         fence_proxy_async();
         prefetch_tensormap(&p.a_hi);
         prefetch_tensormap(&p.w_hi);
-        if (two_plane) {
+        if (TWO) {
             prefetch_tensormap(&p.a_lo);
             prefetch_tensormap(&p.w_lo);
         }
@@ -215,26 +215,33 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     // and every thread of a preemptible launch, waits here.
     const bool early_weights = !resumable && (int)blockIdx.x < total_tiles;
     int prearmed = 0;  // ring stages whose barrier is armed and whose weight loads are in flight
-    if (early_weights && threadIdx.x == 0) {
+    constexpr uint32_t kDataBytes = Cfg::kStageBytes;
+    if (early_weights && warp == 0) {
         const int tile = blockIdx.x;
         const int n_blk = (tile / p.k_splits) % p.tiles_n;
         const int main_kb = tile_kb_count(tile);
         const int kb_base = tile_kb_begin(tile);
-        uint32_t ident_bytes = p.res_kb ? Cfg::kIdentBytes : 0u;
-        for (int kb = 0; kb < main_kb && kb < nst; ++kb) {
-            const int tap = (kb_base + kb) / p.cin_blocks;
-            const int cb = (kb_base + kb) - tap * p.cin_blocks;
-            const uint32_t bar = smem_u32(&ctl->full[kb]);
-            ctl->stage_msg[kb] = CMSG_DATA;
-            mbar_arrive_expect_tx(bar, (two_plane ? Cfg::kStageBytes : Cfg::kABytes + Cfg::kWBytes) + ident_bytes);
-            if (ident_bytes) tma_load_2d(smem_base + ident_off, &p.ident, bar, 0, 0);
-            ident_bytes = 0;
-            const uint32_t dst = smem_base + kb * stage_bytes;
-            const int w_col = tap * p.cin + cb * kCBK;
-            tma_load_2d(dst + w_off, &p.w_hi, bar, w_col, n_blk * BN);
-            if (two_plane) tma_load_2d(dst + 2 * Cfg::kABytes + Cfg::kWBytes, &p.w_lo, bar, w_col, n_blk * BN);
-            ++prearmed;
+        prearmed = main_kb < kStages ? main_kb : kStages;
+        int tap = kb_base / p.cin_blocks;
+        int cb = kb_base - tap * p.cin_blocks;
+        for (int kb = 0; kb < prearmed; ++kb) {
+            if (elect_one()) {
+                const uint32_t bar = smem_u32(&ctl->full[kb]);
+                const uint32_t ident_bytes = (p.res_kb && kb == 0) ? Cfg::kIdentBytes : 0u;
+                ctl->stage_msg[kb] = CMSG_DATA;
+                mbar_arrive_expect_tx(bar, kDataBytes + ident_bytes);
+                if (ident_bytes) tma_load_2d(smem_base + ident_off, &p.ident, bar, 0, 0);
+                const uint32_t dst = smem_base + kb * Cfg::kStageBytes;
+                const int w_col = tap * p.cin + cb * kCBK;
+                tma_load_2d(dst + Cfg::kWOff, &p.w_hi, bar, w_col, n_blk * BN);
+                if (TWO) tma_load_2d(dst + Cfg::kWOff + Cfg::kWBytes, &p.w_lo, bar, w_col, n_blk * BN);
+            }
+            if (++cb == p.cin_blocks) {
+                cb = 0;
+                ++tap;
+            }
         }
+        __syncwarp();
     }
     pdl_wait();  // from here on the predecessor's results (and this executor's slots) are visible
     pdl_launch_dependents();
@@ -287,110 +294,106 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         if (threadIdx.x == 0) fail(900);
     } else if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            int flag = resumable ? load_word(blp.preempted) : 0;
-            int msg = CMSG_EXIT;
-            bool ok = true;
-            // The identity tile travels with the first stage this CTA fills.
-            uint32_t ident_bytes = (p.res_kb && prearmed == 0) ? Cfg::kIdentBytes : 0u;
-            TCK(t_prod0);
+        // The whole warp walks the schedule and one elected lane issues: warp-uniform control flow
+        // keeps coordinates, addresses and barriers on the uniform datapath, where the TMA instruction
+        // reads them.  (tap, channel block) advance by counting; dividing by cin_blocks for every K
+        // block, on a lone thread, was a third of the ~780 cycles a K block cost here before.
+        int stage = 0;
+        uint32_t phase = 0;
+        int msg = CMSG_EXIT;
+        bool ok = true;
+        // The identity tile travels with the first stage this CTA fills.
+        uint32_t ident_bytes = (p.res_kb && prearmed == 0) ? Cfg::kIdentBytes : 0u;
+        const volatile int *word_up = &ctl->word_up;
+        TCK(t_prod0);
 #ifdef GPX_CGEMM_TIMING
-            long long prod_wait = 0;
+        long long prod_wait = 0;
 #endif
-            for (int it = first_iter; ok; ++it) {
-                int tile = blockIdx.x + it * gridDim.x;
-                if (tile >= total_tiles) break;
-                // Column tiles vary fastest: CTAs that run together share the same A rows.
-                const int n_blk = (tile / p.k_splits) % p.tiles_n;
-                const int m_blk = (tile / p.k_splits) / p.tiles_n;
-                const int kb0 = it == first_iter ? first_k : 0;
-                const int main_kb = tile_kb_count(tile);
-                const int num_kb = main_kb + p.res_kb;  // the residual rides along as extra K blocks
-                const int kb_base = tile_kb_begin(tile);
-                for (int kb = kb0; kb < num_kb; ++kb) {
-                    TCK(t_w0);
-                    if (it == first_iter && kb < prearmed) {
-                        // armed before the wait for the predecessor, weights already on their way:
-                        // only the activation tiles are missing
-                        const int tap = (kb_base + kb) / p.cin_blocks;
-                        const int cb = (kb_base + kb) - tap * p.cin_blocks;
-                        const uint32_t bar = smem_u32(&ctl->full[stage]);
-                        const uint32_t dst = smem_base + stage * stage_bytes;
-                        const int a_row = m_blk * kCBM + p.tap_shift[tap];
-                        tma_load_2d(dst, &p.a_hi, bar, cb * kCBK, a_row);
-                        if (two_plane) tma_load_2d(dst + Cfg::kABytes, &p.a_lo, bar, cb * kCBK, a_row);
-                        if (++stage == nst) {
-                            stage = 0;
-                            phase ^= 1;
-                        }
-                        continue;
-                    }
-                    if (!mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1, abort_flag, kCWaitLimitNs)) {
-                        fail(101);
+        for (int it = first_iter; ok; ++it) {
+            const int tile = blockIdx.x + it * gridDim.x;
+            if (tile >= total_tiles) break;
+            // Column tiles vary fastest: CTAs that run together share the same A rows.
+            const int otile = p.k_splits == 1 ? tile : tile / p.k_splits;
+            const int m_blk = otile / p.tiles_n;
+            const int n_blk = otile - m_blk * p.tiles_n;
+            const int kb0 = it == first_iter ? first_k : 0;
+            const int main_kb = tile_kb_count(tile);
+            const int num_kb = main_kb + p.res_kb;  // the residual rides along as extra K blocks
+            const int kb_abs = tile_kb_begin(tile) + kb0;
+            int tap = p.taps == 1 ? 0 : kb_abs / p.cin_blocks;
+            int cb = kb_abs - tap * p.cin_blocks;
+            int a_row = m_blk * kCBM + p.tap_shift[tap < p.taps ? tap : 0];
+            int w_tap = tap * p.cin;
+            for (int kb = kb0; kb < num_kb; ++kb) {
+                const uint32_t bar = smem_u32(&ctl->full[stage]);
+                const uint32_t dst = smem_base + stage * Cfg::kStageBytes;
+                const bool armed = it == first_iter && kb < prearmed;  // weights already on their way
+                TCK(t_w0);
+                if (!armed) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1, abort_flag, kCWaitLimitNs))) {
+                        if (lane == 0) fail(101);
                         ok = false;
                         break;
                     }
-#ifdef GPX_CGEMM_TIMING
-                    prod_wait += clock64() - t_w0;
-#endif
-                    if (resumable && ((kb - kb0) % kCPollEvery) == 0) {
-                        if (flag != 0) {
-                            msg = CMSG_STOP;
-                            ok = false;
-                            break;
-                        }
-                        flag = load_word(blp.preempted);
-                    }
-                    const uint32_t bar = smem_u32(&ctl->full[stage]);
-                    if (kb >= main_kb) {
-                        // Residual block: A = 64 channels of the residual rows of this tile; the W
-                        // operand is the 64x64 identity that stays in shared memory, applied to the
-                        // matching 64 accumulator columns, so the tensor core adds the residual.
-                        const int rb = kb - main_kb;
-                        ctl->stage_msg[stage] = CMSG_RES + rb;
-                        mbar_arrive_expect_tx(bar, (two_plane ? 2 : 1) * Cfg::kABytes + ident_bytes);
-                        const uint32_t dst = smem_base + stage * stage_bytes;
-                        tma_load_2d(dst, &p.r_hi, bar, n_blk * BN + rb * kCBK, m_blk * kCBM);
-                        if (two_plane) tma_load_2d(dst + Cfg::kABytes, &p.r_lo, bar, n_blk * BN + rb * kCBK, m_blk * kCBM);
-                        if (ident_bytes) tma_load_2d(smem_base + ident_off, &p.ident, bar, 0, 0);
-                        ident_bytes = 0;
-                        if (++stage == nst) {
-                            stage = 0;
-                            phase ^= 1;
-                        }
-                        continue;
-                    }
-                    const int tap = (kb_base + kb) / p.cin_blocks;
-                    const int cb = (kb_base + kb) - tap * p.cin_blocks;
-                    ctl->stage_msg[stage] = CMSG_DATA;
-                    mbar_arrive_expect_tx(bar, (two_plane ? Cfg::kStageBytes : Cfg::kABytes + Cfg::kWBytes) + ident_bytes);
-                    if (ident_bytes) tma_load_2d(smem_base + ident_off, &p.ident, bar, 0, 0);
-                    ident_bytes = 0;
-                    const uint32_t dst = smem_base + stage * stage_bytes;
-                    const int a_row = m_blk * kCBM + p.tap_shift[tap];
-                    const int w_col = tap * p.cin + cb * kCBK;
-                    tma_load_2d(dst, &p.a_hi, bar, cb * kCBK, a_row);
-                    tma_load_2d(dst + w_off, &p.w_hi, bar, w_col, n_blk * BN);
-                    if (two_plane) {
-                        tma_load_2d(dst + Cfg::kABytes, &p.a_lo, bar, cb * kCBK, a_row);
-                        tma_load_2d(dst + 2 * Cfg::kABytes + Cfg::kWBytes, &p.w_lo, bar, w_col, n_blk * BN);
-                    }
-                    if (++stage == nst) {
-                        stage = 0;
-                        phase ^= 1;
+                    if (resumable && __any_sync(0xffffffffu, *word_up)) {
+                        msg = CMSG_STOP;
+                        ok = false;
+                        break;
                     }
                 }
-            }
 #ifdef GPX_CGEMM_TIMING
+                prod_wait += clock64() - t_w0;
+#endif
+                if (kb >= main_kb) {
+                    // Residual block: A = 64 channels of the residual rows of this tile; the W
+                    // operand is the 64x64 identity that stays in shared memory, applied to the
+                    // matching 64 accumulator columns, so the tensor core adds the residual.
+                    const int rb = kb - main_kb;
+                    if (elect_one()) {
+                        ctl->stage_msg[stage] = CMSG_RES + rb;
+                        mbar_arrive_expect_tx(bar, Cfg::kPlanes * Cfg::kABytes + ident_bytes);
+                        tma_load_2d(dst, &p.r_hi, bar, n_blk * BN + rb * kCBK, m_blk * kCBM);
+                        if (TWO) tma_load_2d(dst + Cfg::kABytes, &p.r_lo, bar, n_blk * BN + rb * kCBK, m_blk * kCBM);
+                        if (ident_bytes) tma_load_2d(smem_base + ident_off, &p.ident, bar, 0, 0);
+                    }
+                } else if (elect_one()) {
+                    if (!armed) {
+                        ctl->stage_msg[stage] = CMSG_DATA;
+                        mbar_arrive_expect_tx(bar, kDataBytes + ident_bytes);
+                        if (ident_bytes) tma_load_2d(smem_base + ident_off, &p.ident, bar, 0, 0);
+                    }
+                    tma_load_2d(dst, &p.a_hi, bar, cb * kCBK, a_row);
+                    if (TWO) tma_load_2d(dst + Cfg::kABytes, &p.a_lo, bar, cb * kCBK, a_row);
+                    if (!armed) {
+                        tma_load_2d(dst + Cfg::kWOff, &p.w_hi, bar, w_tap + cb * kCBK, n_blk * BN);
+                        if (TWO) tma_load_2d(dst + Cfg::kWOff + Cfg::kWBytes, &p.w_lo, bar, w_tap + cb * kCBK, n_blk * BN);
+                    }
+                }
+                __syncwarp();
+                if (!armed) ident_bytes = 0;
+                if (++cb == p.cin_blocks) {
+                    cb = 0;
+                    ++tap;
+                    w_tap += p.cin;
+                    if (tap < p.taps) a_row = m_blk * kCBM + p.tap_shift[tap];
+                }
+                if (++stage == kStages) {
+                    stage = 0;
+                    phase ^= 1;
+                }
+            }
+        }
+#ifdef GPX_CGEMM_TIMING
+        if (lane == 0) {
             TADD(0, prod_wait);
             TADD(1, clock64() - t_prod0);
+        }
 #endif
-            if (!*abort_flag) {
-                bool have_slot = msg == CMSG_STOP;
-                if (!have_slot)
-                    have_slot = mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1, abort_flag, kCWaitLimitNs);
+        if (!*abort_flag) {
+            bool have_slot = msg == CMSG_STOP;
+            if (!have_slot)
+                have_slot = mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1, abort_flag, kCWaitLimitNs);
+            if (lane == 0) {
                 if (have_slot) {
                     ctl->stage_msg[stage] = msg;
                     mbar_arrive(smem_u32(&ctl->full[stage]));
@@ -400,36 +403,45 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 if (msg == CMSG_STOP && blp.trace) atomicMin(blp.trace + 2, globaltimer_ns());
             }
         }
+        if (lane == 0) *(volatile int *)&ctl->poll_done = 1;
+        __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        // The whole warp walks the K loop in lock step and one lane issues the tensor-core
-        // instructions.  With the loop inside an `if (lane == 0)` the compiler has to treat every
-        // address and descriptor as a per-thread value and moves each operand of each
-        // tcgen05.mma into the uniform registers the instruction reads, ~100 cycles of a lone
-        // thread's issue time per instruction, more than a 128x128x16 product takes (64 cycles);
-        // warp-uniform control flow keeps that arithmetic on the uniform datapath.
-        {
-            const uint32_t idesc = p.fmt == PF_F16 ? make_idesc_f16_f32(kCBM, BN) : make_idesc_bf16_f32(kCBM, BN);
-            const uint32_t idesc64 = p.fmt == PF_F16 ? make_idesc_f16_f32(kCBM, 64) : make_idesc_bf16_f32(kCBM, 64);
-            constexpr int kWide = 2 * BN <= 256 ? 2 * BN : BN;  // (256-column tiles never take the packed path)
-            const uint32_t idesc_wide = make_idesc_bf16_f32(kCBM, kWide);
-            const uint64_t eye = make_smem_desc_sw128(smem_base + ident_off);
-            const bool issuer = lane == 0;
-            int stage = 0;
-            uint32_t phase = 0;
-            uint32_t seg = 0;
-            int kb = first_k;
-            int it = first_iter;
-            int num_kb = tile_kb_count(blockIdx.x + it * gridDim.x) + p.res_kb;
-            bool seg_open = false;
-            TCK(t_mma0);
+        // Warp-uniform like the producer, one elected lane issues the tensor-core instructions.
+        constexpr uint32_t idesc_bf16 = make_idesc_bf16_f32(kCBM, BN), idesc_f16 = make_idesc_f16_f32(kCBM, BN);
+        constexpr int kWide = TWO ? 2 * BN : BN;
+        constexpr uint32_t idesc_wide = make_idesc_bf16_f32(kCBM, kWide);
+        const uint32_t idesc = (!TWO && p.fmt == PF_F16) ? idesc_f16 : idesc_bf16;
+        const uint32_t idesc64 = (!TWO && p.fmt == PF_F16) ? make_idesc_f16_f32(kCBM, 64) : make_idesc_bf16_f32(kCBM, 64);
+        const uint64_t eye = make_smem_desc_sw128(smem_base + ident_off);
+        const uint64_t ring = make_smem_desc_sw128(smem_base);
+        int stage = 0;
+        uint32_t phase = 0;
+        int kb = first_k;
+        int it = first_iter;
+        TCK(t_mma0);
 #ifdef GPX_CGEMM_TIMING
-            long long mma_wait_full = 0, mma_wait_tmem = 0, mma_kb = 0;
+        long long mma_wait_full = 0, mma_wait_tmem = 0, mma_kb = 0;
 #endif
-            for (;;) {
+        for (uint32_t seg = 0;; ++seg) {
+            const int buf = (int)(seg & 1);
+            const uint32_t acc0 = tmem_base + buf * kBufCols;
+            const int num_kb = tile_kb_count(blockIdx.x + it * gridDim.x) + p.res_kb;
+            TCK(t_e0);
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->tmem_empty[buf]), (seg >> 1) & 1, abort_flag, kCWaitLimitNs))) {
+                if (lane == 0) fail(202);
+                break;
+            }
+#ifdef GPX_CGEMM_TIMING
+            mma_wait_tmem += clock64() - t_e0;
+#endif
+            tc_fence_after_sync();
+            int end = CEPI_COMPLETE;
+            for (; kb < num_kb; ++kb) {
                 TCK(t_f0);
                 if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->full[stage]), phase, abort_flag, kCWaitLimitNs))) {
-                    if (issuer) fail(201);
+                    if (lane == 0) fail(201);
+                    end = -1;
                     break;
                 }
 #ifdef GPX_CGEMM_TIMING
@@ -438,127 +450,96 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
 #endif
                 tc_fence_after_sync();
                 const int msg = __shfl_sync(0xffffffffu, ctl->stage_msg[stage], 0);
-                const int buf = (int)(seg % nbuf);
-                const uint32_t acc0 = tmem_base + buf * buf_cols;
-                if (!seg_open) {
-                    TCK(t_e0);
-                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->tmem_empty[buf]), (seg / nbuf) & 1, abort_flag,
-                                                           kCWaitLimitNs))) {
-                        if (issuer) fail(202);
-                        break;
-                    }
-#ifdef GPX_CGEMM_TIMING
-                    mma_wait_tmem += clock64() - t_e0;
-#endif
-                    tc_fence_after_sync();
-                    seg_open = true;
-                }
-                if (msg != CMSG_DATA && msg < CMSG_RES) {
-                    if (issuer) {
-                        ctl->epi_kind[buf] = msg == CMSG_STOP ? CEPI_PARTIAL : CEPI_EXIT;
-                        ctl->epi_k_done[buf] = kb;
-                        mma_commit(smem_u32(&ctl->tmem_full[buf]));
-                        mbar_arrive(smem_u32(&ctl->tmem_full[buf]));
-                    }
-                    __syncwarp();
+                if (msg == CMSG_STOP || msg == CMSG_EXIT) {
+                    end = msg == CMSG_STOP ? CEPI_PARTIAL : CEPI_EXIT;
                     break;
                 }
-                const uint32_t base = smem_base + stage * stage_bytes;
-                const uint64_t a_hi = make_smem_desc_sw128(base);
-                const uint64_t a_lo = make_smem_desc_sw128(base + Cfg::kABytes);
-                const uint64_t w_hi = make_smem_desc_sw128(base + w_off);
-                const uint64_t w_lo = make_smem_desc_sw128(base + 2 * Cfg::kABytes + Cfg::kWBytes);
-                // fp32 product from three bf16 products.  The tensor core truncates when it adds
-                // into the fp32 accumulator, a bias that grows with the length of the accumulation
-                // chain, so the chain is split over several accumulators that the epilogue adds with
-                // round-to-nearest.  The order is fixed, so a resumed tile replays exactly the
-                // instruction sequence of an uninterrupted one.
-                const uint32_t first = kb > 0 ? 1u : 0u;
-                if (issuer) {
+                // descriptor addresses are in 16-byte units
+                const uint64_t a_hi = ring + (uint64_t)(stage * (Cfg::kStageBytes >> 4));
+                const uint64_t a_lo = a_hi + (Cfg::kABytes >> 4);
+                const uint64_t w_hi = a_hi + (Cfg::kWOff >> 4);
+                const uint32_t acc = kb > 0 ? 1u : 0u;
+                if (elect_one()) {
                     if (msg >= CMSG_RES) {
-                        // residual x identity on 64 accumulator columns: the hi plane into a hi*hi
-                        // accumulator, the lo plane into a cross-term accumulator (exact products,
+                        // residual x identity on 64 accumulator columns: the hi plane into the hi*hi
+                        // accumulator, the lo plane into the cross-term accumulator (exact products,
                         // added like any other)
                         const uint32_t col = (uint32_t)(msg - CMSG_RES) * 64;
 #pragma unroll
                         for (int k = 0; k < kCBK / kCUmmaK; ++k) {
-                            if (dual && two_plane) {
-                                mma_f16_ss(acc0 + col, a_hi + 2 * k, eye + 2 * k, idesc64, 1u);
-                                mma_f16_ss(acc0 + BN + col, a_lo + 2 * k, eye + 2 * k, idesc64, 1u);
-                            } else {
-                                mma_f16_ss(acc0 + (k & 1) * BN + col, a_hi + 2 * k, eye + 2 * k, idesc64, 1u);
-                                if (two_plane) mma_f16_ss(acc0 + 3 * BN + col, a_lo + 2 * k, eye + 2 * k, idesc64, 1u);
-                            }
+                            mma_f16_ss(acc0 + col, a_hi + 2 * k, eye + 2 * k, idesc64, 1u);
+                            if (TWO) mma_f16_ss(acc0 + BN + col, a_lo + 2 * k, eye + 2 * k, idesc64, 1u);
                         }
-                    } else if (dual && two_plane && p.packed) {
-                        // hi*hi in one accumulator, both cross terms in the other.  The W_lo tile
+                    } else if (TWO) {
+                        // fp32 product from three bf16 products: hi*hi in one accumulator, both cross
+                        // terms in the other.  The tensor core truncates when it adds into the fp32
+                        // accumulator, a bias that grows with the length of the accumulation chain;
+                        // keeping the small cross terms apart keeps them clear of it.  The W_lo tile
                         // follows the W_hi tile in the stage and the two accumulators are adjacent
-                        // columns, so A_hi x [W_hi; W_lo] is ONE instruction of width 2*BN: the
-                        // kernel is bound by shared-memory bandwidth (operand reads plus the TMA
-                        // fill), and this reads the A_hi tile once instead of twice.  Every
-                        // accumulator element still receives the same additions in the same order.
+                        // columns, so A_hi x [W_hi; W_lo] is ONE instruction of width 2*BN, which
+                        // reads the A_hi tile once.  The order is fixed, so a resumed tile replays
+                        // exactly the instruction sequence of an uninterrupted one.
 #pragma unroll
                         for (int k = 0; k < kCBK / kCUmmaK; ++k) {
-                            mma_f16_ss(acc0, a_hi + 2 * k, w_hi + 2 * k, idesc_wide, (first || k > 0) ? 1u : 0u);
-                            mma_f16_ss(acc0 + BN, a_lo + 2 * k, w_hi + 2 * k, idesc, 1u);
-                        }
-                    } else if (dual && two_plane) {
-#pragma unroll
-                        for (int k = 0; k < kCBK / kCUmmaK; ++k) {
-                            mma_f16_ss(acc0, a_hi + 2 * k, w_hi + 2 * k, idesc, (first || k > 0) ? 1u : 0u);
-                            mma_f16_ss(acc0 + BN, a_hi + 2 * k, w_lo + 2 * k, idesc, (first || k > 0) ? 1u : 0u);
+                            mma_f16_ss(acc0, a_hi + 2 * k, w_hi + 2 * k, idesc_wide, k > 0 ? 1u : acc);
                             mma_f16_ss(acc0 + BN, a_lo + 2 * k, w_hi + 2 * k, idesc, 1u);
                         }
                     } else {
-                        // hi*hi terms alternate between two accumulators (even / odd K steps); the
-                        // small hi*lo and lo*hi terms get one each
 #pragma unroll
-                        for (int k = 0; k < kCBK / kCUmmaK; ++k) {
-                            mma_f16_ss(acc0 + (k & 1) * BN, a_hi + 2 * k, w_hi + 2 * k, idesc, (first || k > 1) ? 1u : 0u);
-                            if (two_plane) {
-                                mma_f16_ss(acc0 + 2 * BN, a_hi + 2 * k, w_lo + 2 * k, idesc, (first || k > 0) ? 1u : 0u);
-                                mma_f16_ss(acc0 + 3 * BN, a_lo + 2 * k, w_hi + 2 * k, idesc, (first || k > 0) ? 1u : 0u);
-                            }
-                        }
+                        for (int k = 0; k < kCBK / kCUmmaK; ++k)
+                            mma_f16_ss(acc0, a_hi + 2 * k, w_hi + 2 * k, idesc, k > 0 ? 1u : acc);
                     }
                     mma_commit(smem_u32(&ctl->empty[stage]));
                 }
                 __syncwarp();
-                if (++stage == nst) {
+                if (++stage == kStages) {
                     stage = 0;
                     phase ^= 1;
                 }
-                if (++kb == num_kb) {
-                    if (issuer) {
-                        ctl->epi_kind[buf] = CEPI_COMPLETE;
-                        ctl->epi_k_done[buf] = num_kb;
-                        mma_commit(smem_u32(&ctl->tmem_full[buf]));
-                        mbar_arrive(smem_u32(&ctl->tmem_full[buf]));
-                    }
-                    __syncwarp();
-                    ++seg;
-                    ++it;
-                    num_kb = tile_kb_count(blockIdx.x + it * gridDim.x) + p.res_kb;
-                    kb = 0;
-                    seg_open = false;
-                }
             }
-#ifdef GPX_CGEMM_TIMING
-            if (issuer) {
-                TADD(2, mma_wait_full);
-                TADD(3, mma_wait_tmem);
-                TADD(4, clock64() - t_mma0);
-                TADD(12, mma_kb);
+            if (end < 0) break;
+            if (elect_one()) {
+                ctl->epi_kind[buf] = end;
+                ctl->epi_k_done[buf] = kb;
+                mma_commit(smem_u32(&ctl->tmem_full[buf]));
+                mbar_arrive(smem_u32(&ctl->tmem_full[buf]));
             }
-#endif
+            __syncwarp();
+            if (end != CEPI_COMPLETE) break;
+            ++it;
+            kb = 0;
         }
+#ifdef GPX_CGEMM_TIMING
+        if (lane == 0) {
+            TADD(2, mma_wait_full);
+            TADD(3, mma_wait_tmem);
+            TADD(4, clock64() - t_mma0);
+            TADD(12, mma_kb);
+        }
+#endif
+    } else if (warp == kCPollWarp) {
+        // ------------------------------------------------------------------ preempt-word poller
+        // A read of the word takes longer than a K block of a single-plane model: on the producer's
+        // path, even one K block ahead, it set the pace of the ring.  Here one lane reads it back to
+        // back and the producer looks at a flag in shared memory.  Ends with the producer.
+        if (resumable && lane == 0) {
+            while (!*(volatile int *)&ctl->poll_done) {
+                if (load_word(blp.preempted) != 0) {
+                    *(volatile int *)&ctl->word_up = 1;
+                    break;
+                }
+                __nanosleep(100);
+            }
+        }
+        __syncwarp();
     } else {
         // ------------------------------------------------------------------ epilogue
         const int quarter = warp & 3;
         const int part = (warp - 2) >> 2;                 // which share of the columns
         const int c_lo = part * (BN / kCEpiParts), c_hi = c_lo + BN / kCEpiParts;
         // this warp's share of the columns of one accumulator buffer, for spill and restore
-        const int s_lo = part * (buf_cols / kCEpiParts), s_hi = s_lo + buf_cols / kCEpiParts;
+        constexpr int kSpillCols = kBufCols / kCEpiParts;
+        const int s_lo = part * kSpillCols, s_hi = s_lo + kSpillCols;
         const int row = quarter * 32 + lane;
         const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
         const bool leader = threadIdx.x == 64;
@@ -584,7 +565,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         tc_fence_before_sync();
         asm volatile("bar.sync 1, %0;" ::"n"(kCEpiThreads) : "memory");
         if (leader)
-            for (int b = 0; b < nbuf; ++b) mbar_arrive(smem_u32(&ctl->tmem_empty[b]));
+            for (int b = 0; b < 2; ++b) mbar_arrive(smem_u32(&ctl->tmem_empty[b]));
 
         int it = first_iter;
         int seg_k0 = first_k;
@@ -602,8 +583,8 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         long long e_wait = 0, e_tmem = 0, e_math = 0, e_store = 0, e_bar = 0;
 #endif
         for (uint32_t seg = 0;; ++seg) {
-            const int buf = (int)(seg % nbuf);
-            const uint32_t t_acc = t_lane + buf * buf_cols;
+            const int buf = (int)(seg & 1);
+            const uint32_t t_acc = t_lane + buf * kBufCols;
             TCK(t_wait0);
             // The bias of the tile this buffer holds goes to shared memory before the drain loop
             // (read from global memory inside it, its latency - an L2 round trip under load - was
@@ -619,7 +600,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 }
             }
             if (leader) {
-                bool ok = mbar_wait(smem_u32(&ctl->tmem_full[buf]), (seg / nbuf) & 1, abort_flag, kCWaitLimitNs);
+                bool ok = mbar_wait(smem_u32(&ctl->tmem_full[buf]), (seg >> 1) & 1, abort_flag, kCWaitLimitNs);
                 if (!ok) fail(301);
                 ctl->epi_go = ok ? 1 : 0;
             }
@@ -680,34 +661,32 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 // contiguous bytes of that row, one 256-bit access, a whole sector.
                 const bool planes_out = !p.partial && !p.out_f32;
                 const int col_lim = p.cout_valid - n_blk * BN;
-                for (int c = c_lo; c < c_hi; c += 16) {
-                    float f[16];
-                    uint32_t t16[16];
+                constexpr int CH = TWO ? 16 : 32;  // columns per piece
+#pragma unroll 1
+                for (int c = c_lo; c < c_hi; c += CH) {
+                    float f[CH];
                     // The residual is requested first so its latency overlaps the TMEM reads.
                     const bool use_res = planes_out && p.res_hi && valid;
                     TCK(t_p0);
-                    uint32_t rh[8], rl[8];
+                    uint32_t rh[CH / 2], rl[TWO ? CH / 2 : 1];
                     if (use_res) {
-                        ld_global_v8(p.res_hi + res_off + c, rh);
-                        if (two_plane) ld_global_v8(p.res_lo + res_off + c, rl);
+#pragma unroll
+                        for (int q = 0; q < CH / 16; ++q) ld_global_v8(p.res_hi + res_off + c + 16 * q, rh + 8 * q);
+                        if (TWO) ld_global_v8(p.res_lo + res_off + c, rl);
                     }
-                    {
-                        uint32_t u16[16];
+                    if constexpr (TWO) {
+                        uint32_t t16[16], u16[16];
                         tmem_ld_32x16(t_acc + c, t16);
                         tmem_ld_32x16(t_acc + BN + c, u16);
                         tmem_ld_wait();
 #pragma unroll
                         for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(t16[j]) + __uint_as_float(u16[j]);
-                    }
-                    if (two_plane && !dual) {
-                        tmem_ld_32x16(t_acc + 2 * BN + c, t16);
+                    } else {
+                        uint32_t t32[32];
+                        tmem_ld_32x32(t_acc + c, t32);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) f[j] += __uint_as_float(t16[j]);
-                        tmem_ld_32x16(t_acc + 3 * BN + c, t16);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) f[j] += __uint_as_float(t16[j]);
+                        for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(t32[j]);
                     }
 #ifdef GPX_CGEMM_TIMING
                     long long t_p1 = clock64();
@@ -720,7 +699,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                         // warp spread over the banks.
                         float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(smem) + (size_t)row * (BN + 4) + c);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
+                        for (int j = 0; j < CH / 4; ++j)
                             dst[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
                         continue;
                     }
@@ -731,7 +710,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                             float4 *dst = reinterpret_cast<float4 *>(
                                 p.partial + ((size_t)split * p.partial_rows + vrow) * p.partial_ld + n_blk * BN + c);
 #pragma unroll
-                            for (int j = 0; j < 4; ++j)
+                            for (int j = 0; j < CH / 4; ++j)
                                 dst[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
                         }
                         continue;
@@ -739,7 +718,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     if (p.bias) {
                         const float4 *b4 = reinterpret_cast<const float4 *>(&ctl->bias_s[buf][c]);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
+                        for (int j = 0; j < CH / 4; ++j) {
                             float4 b = b4[j];
                             f[4 * j + 0] += b.x;
                             f[4 * j + 1] += b.y;
@@ -749,12 +728,12 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     }
                     if (use_res) {
 #pragma unroll
-                        for (int q = 0; q < 8; ++q) {
-                            float2 r = pf_unpack2(rh[q], p.fmt);
+                        for (int q = 0; q < CH / 2; ++q) {
+                            float2 r = pf_unpack2(rh[q], TWO ? (int)PF_SPLIT : p.fmt);
                             f[2 * q] += r.x;
                             f[2 * q + 1] += r.y;
                         }
-                        if (two_plane) {
+                        if constexpr (TWO) {
 #pragma unroll
                             for (int q = 0; q < 8; ++q) {
                                 f[2 * q] += bf16_lo_to_f32(rl[q]);
@@ -767,27 +746,33 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                         const int col0 = n_blk * BN + c;
                         if (valid) {
 #pragma unroll
-                            for (int j = 0; j < 16; ++j)
+                            for (int j = 0; j < CH; ++j)
                                 if (col0 + j < p.cout_valid) p.out_f32[out_off + col0 + j] = f[j];
                         }
                         continue;
                     }
-                    uint32_t hi[8];
+                    uint32_t hi[CH / 2];
+                    if (TWO || p.fmt != PF_F16) {
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) hi[q] = pf_pack2(f[2 * q], f[2 * q + 1], p.fmt);
-                    // The output may be a channel slice: nothing is stored past cout_valid.
-                    const bool store = valid && c < col_lim;
+                        for (int q = 0; q < CH / 2; ++q) hi[q] = pack_bf16(f[2 * q], f[2 * q + 1]);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < CH / 2; ++q) hi[q] = pf_pack2(f[2 * q], f[2 * q + 1], PF_F16);
+                    }
 #ifdef GPX_CGEMM_TIMING
                     long long t_p2 = clock64();
                     e_math += t_p2 - t_p1;
 #endif
-                    if (store) st_global_v8(p.out_hi + out_off + c, hi);
-                    if (two_plane) {
+                    // The output may be a channel slice: nothing is stored past cout_valid.
+#pragma unroll
+                    for (int q = 0; q < CH / 16; ++q)
+                        if (valid && c + 16 * q < col_lim) st_global_v8(p.out_hi + out_off + c + 16 * q, hi + 8 * q);
+                    if constexpr (TWO) {
                         uint32_t lo[8];
 #pragma unroll
                         for (int q = 0; q < 8; ++q)
                             lo[q] = pack_bf16(f[2 * q] - bf16_lo_to_f32(hi[q]), f[2 * q + 1] - bf16_hi_to_f32(hi[q]));
-                        if (store) st_global_v8(p.out_lo + out_off + c, lo);
+                        if (valid && c < col_lim) st_global_v8(p.out_lo + out_off + c, lo);
                     }
 #ifdef GPX_CGEMM_TIMING
                     e_store += clock64() - t_p2;
@@ -851,7 +836,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         // shared memory and added in split order from zero, exactly as splitk_finish_kernel adds the
         // workspace rows, then bias, residual, activation and store by the same function.
         cluster_sync_all();
-        if (warp >= 2) {
+        if (warp >= 2 && warp < kCPollWarp) {
             const int S = p.k_splits;
             const int rank = (int)cluster_ctarank();
             const int otile = (int)blockIdx.x / S;
@@ -916,44 +901,35 @@ extern "C" int gpx_debug_cgemm_timing(unsigned long long *out, int reset) {
 }
 #endif
 
+// Calls f(std::integral_constant<int, BN>, std::bool_constant<TWO>) for the kernel instance of a tile
+// width and operand format.  (256-column tiles exist for single-plane operands only: two planes' two
+// accumulators in two buffers would not fit tensor memory.)
+template <typename F>
+static auto cgemm_instance(int bn, bool two, F &&f) {
+    if (two)
+        return bn == 128 ? f(std::integral_constant<int, 128>(), std::true_type()) : f(std::integral_constant<int, 64>(), std::true_type());
+    if (bn == 256) return f(std::integral_constant<int, 256>(), std::false_type());
+    return bn == 128 ? f(std::integral_constant<int, 128>(), std::false_type()) : f(std::integral_constant<int, 64>(), std::false_type());
+}
+
 cudaError_t cgemm_prepare(int device) {
     static bool done[64] = {false};
     if (device < 0 || device >= 64 || done[device]) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(cgemm_tcgen05_kernel<128>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)CgemmCfg<128>::kSmem);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(cgemm_tcgen05_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)CgemmCfg<256>::kSmem);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(cgemm_tcgen05_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)CgemmCfg<64>::kSmem);
-    if (e != cudaSuccess) return e;
+    for (int two = 0; two < 2; ++two)
+        for (int bn : {64, 128, 256}) {
+            if (two && bn == 256) continue;
+            cudaError_t e = cgemm_instance(bn, two != 0, [](auto b, auto t) {
+                return cudaFuncSetAttribute(cgemm_tcgen05_kernel<b(), t()>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)CgemmCfg<b(), t()>::kSmem);
+            });
+            if (e != cudaSuccess) return e;
+        }
     done[device] = true;
     return cudaSuccess;
 }
 
-template <int BN>
-static cudaError_t cgemm_launch_cluster(const CgemmParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)kCgemmThreads);
-    cfg.dynamicSmemBytes = CgemmCfg<BN>::kSmem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = (unsigned)p.k_splits;
-    at[1].val.clusterDim.y = 1;
-    at[1].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, cgemm_tcgen05_kernel<BN>, p, blp);
-}
-
 // CTAs of clusters of `cluster` CTAs of this kernel that the device keeps resident at once.
-int cgemm_max_cluster(int bn, int cluster) {
+int cgemm_max_cluster(int bn, int fmt, int cluster) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)cluster);
     cfg.blockDim = dim3((unsigned)kCgemmThreads);
@@ -965,14 +941,10 @@ int cgemm_max_cluster(int bn, int cluster) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int clusters = 0;
-    cudaError_t err;
-    if (bn == 128) {
-        cfg.dynamicSmemBytes = CgemmCfg<128>::kSmem;
-        err = cudaOccupancyMaxActiveClusters(&clusters, cgemm_tcgen05_kernel<128>, &cfg);
-    } else {
-        cfg.dynamicSmemBytes = CgemmCfg<64>::kSmem;
-        err = cudaOccupancyMaxActiveClusters(&clusters, cgemm_tcgen05_kernel<64>, &cfg);
-    }
+    cudaError_t err = cgemm_instance(bn, fmt == PF_SPLIT, [&](auto b, auto t) {
+        cfg.dynamicSmemBytes = CgemmCfg<b(), t()>::kSmem;
+        return cudaOccupancyMaxActiveClusters(&clusters, cgemm_tcgen05_kernel<b(), t()>, &cfg);
+    });
     if (err != cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -981,22 +953,27 @@ int cgemm_max_cluster(int bn, int cluster) {
 }
 
 cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &blp, cudaStream_t s) {
-    if (p.cluster_reduce) {
-        // (256-column tiles are never split)
-        if (bn == 128) return cgemm_launch_cluster<128>(p, grid, blp, s);
-        return cgemm_launch_cluster<64>(p, grid, blp, s);
-    }
-    if (bn == 256)
-        launch_layer(cgemm_tcgen05_kernel<256>, grid, kCgemmThreads, CgemmCfg<256>::kSmem, s, p, blp);
-    else if (bn == 128)
-        launch_layer(cgemm_tcgen05_kernel<128>, grid, kCgemmThreads, CgemmCfg<128>::kSmem, s, p, blp);
-    else
-        launch_layer(cgemm_tcgen05_kernel<64>, grid, kCgemmThreads, CgemmCfg<64>::kSmem, s, p, blp);
-    return cudaGetLastError();
+    return cgemm_instance(bn, p.fmt == PF_SPLIT, [&](auto b, auto t) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3((unsigned)kCgemmThreads);
+        cfg.dynamicSmemBytes = CgemmCfg<b(), t()>::kSmem;
+        cfg.stream = s;
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+        at[1].id = cudaLaunchAttributeClusterDimension;
+        at[1].val.clusterDim.x = (unsigned)p.k_splits;
+        at[1].val.clusterDim.y = 1;
+        at[1].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = p.cluster_reduce ? 2 : 1;
+        return cudaLaunchKernelEx(&cfg, cgemm_tcgen05_kernel<b(), t()>, p, blp);
+    });
 }
 
 int cgemm_threads() { return kCgemmThreads; }
 
-size_t cgemm_spill_floats_per_cta() { return (size_t)kCBM * CgemmCfg<128>::kTmemCols; }
+size_t cgemm_spill_floats_per_cta() { return cgemm_spill_floats(); }
 
 }  // namespace gpx

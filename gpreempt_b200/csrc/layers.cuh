@@ -82,10 +82,6 @@ struct CgemmParams {
     int res_kb;
     int drop_on_stop;        // 1: a tile interrupted by the word is recomputed from K block 0 after the
                              // resume instead of being saved (no spill on the way out)
-    int packed;              // 1 (two-plane operands, dual plan): hi*hi and hi*lo issued as one product of
-                             // width 2*BN against the adjacent W_hi / W_lo tiles
-    int dual;                // 1: two accumulators per tile in two TMEM buffers (short K ranges and
-                             // single-plane operands), 0: four accumulators in one buffer
     int k_splits;            // >= 1: the K range is cut into this many tiles per output block
     int kb_per_split;        // K blocks per split (the last split may be shorter)
     float *partial;          // k_splits > 1: fp32 workspace [split][partial_rows][partial_ld]
@@ -103,7 +99,7 @@ struct CgemmParams {
 
 cudaError_t cgemm_prepare(int device);
 cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &blp, cudaStream_t s);
-int cgemm_max_cluster(int bn, int cluster);  // CTAs of clusters of this size that can be resident at once
+int cgemm_max_cluster(int bn, int fmt, int cluster);  // CTAs of clusters of this size that can be resident at once
 size_t cgemm_spill_floats_per_cta();
 int cgemm_threads();
 

@@ -1077,11 +1077,8 @@ int finalize_model(gpx_model &m) {
             // they still fill the GPU and the K loop is long enough to outweigh the second
             // accumulator buffer they give up (ResNet-50's 1x1 convolutions with K <= 512 lose 6 %,
             // BERT's dense layers and VGG's 3x3 convolutions gain 17-19 %).
-            const char *wide = getenv("GPX_CGEMM_BN256");
-            const bool try_split = wide && wide[0] == 's';  // experiment: 256-column tiles for two-plane operands
-            if ((m.fmt != PF_SPLIT || try_split) && !head && cout_st % 256 == 0 && tiles128 / 2 >= m.sm_count &&
-                (long long)eff_k * eff_k * eff_cin >= 768 &&
-                !(wide && wide[0] == '0'))
+            if (m.fmt != PF_SPLIT && !head && cout_st % 256 == 0 && tiles128 / 2 >= m.sm_count &&
+                (long long)eff_k * eff_k * eff_cin >= 768)
                 bn = 256;
         }
         kn.tile = bn;
@@ -1156,21 +1153,6 @@ int finalize_model(gpx_model &m) {
                 p.kb_per_split = (all_kb + s_want - 1) / s_want;
                 p.k_splits = (all_kb + p.kb_per_split - 1) / p.kb_per_split;
             }
-        }
-        // Two accumulators per tile (hi*hi; both cross terms) in two TMEM buffers: the epilogue of one
-        // tile overlaps the K loop of the next.  The single hi*hi chain costs at most 9e-6 of
-        // truncation bias on the longest K range (4608) and keeps ResNet-50 b32 at 3.8e-5 of the
-        // 1e-4 layer bound; GPX_CGEMM_DUAL=0 selects four accumulators in one buffer (even / odd
-        // K steps, hi*lo, lo*hi), =1 uses that plan only for chains longer than 1024 products.
-        p.dual = 1;
-        if (const char *e = getenv("GPX_CGEMM_DUAL")) {
-            if (atoi(e) == 0) p.dual = 0;
-            if (atoi(e) == 1) p.dual = (m.fmt != PF_SPLIT || p.kb_per_split * 64 <= 1024) ? 1 : 0;
-        }
-        if (bn == 256) p.dual = 1;  // the only plan that fits 256-column tiles in tensor memory
-        {
-            const char *e = getenv("GPX_CGEMM_PACKED");
-            p.packed = (bn <= 128 && !(e && e[0] == '0')) ? 1 : 0;
         }
         // The residual of a 1x1 stride-1 convolution on plain rows has the rows of the GEMM itself:
         // it is then added by the tensor core as identity K blocks instead of by the epilogue.
@@ -1252,7 +1234,7 @@ int finalize_model(gpx_model &m) {
             // number of splits that divides the tile's rows, and every cluster resident at once.
             const char *e_cl = getenv("GPX_SPLITK_CLUSTER");
             const bool pow2 = p.k_splits == 2 || p.k_splits == 4 || p.k_splits == 8;
-            if (pow2 && bn <= 128 && !(e_cl && e_cl[0] == '0') && cgemm_max_cluster(bn, p.k_splits) >= kn.total_tiles &&
+            if (pow2 && bn <= 128 && !(e_cl && e_cl[0] == '0') && cgemm_max_cluster(bn, m.fmt, p.k_splits) >= kn.total_tiles &&
                 kn.grid == kn.total_tiles) {
                 p.cluster_reduce = 1;
                 p.fin = q;
