@@ -76,12 +76,7 @@ GPX_HD int layout_row(const ActLayout &l, int n, int h, int w) {
 enum ActKind : int { ACT_NONE = 0, ACT_RELU = 1, ACT_GELU = 2, ACT_RELU6 = 3 };
 
 #if defined(__CUDACC__)
-// Exact GELU, v * Phi(v) with Phi(v) = erfc(-v / sqrt 2) / 2.  The complementary error function is the
-// Chebyshev fit t * exp(-z*z + P(t)), t = 1 / (1 + z/2), z = |v| / sqrt 2, of W. J. Cody's form as
-// printed in Press et al., Numerical Recipes, section 6.2 ("erfcc"): relative error below 1.2e-7
-// everywhere, so the tail of negative v keeps its leading digits, which 1 + erf(v / sqrt 2) cancels
-// away.  Two elements share each step (packed fp32 FMA); with erff per element the epilogue of a
-// 768 -> 3072 layer took longer than its products (175 us against 115 us for 3072 -> 768 at 16 384 rows).
+// Packed fp32 arithmetic on two values (one instruction each on sm_100).
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     float2 r;
     asm("fma.rn.f32x2 %0, %1, %2, %3;"
@@ -90,28 +85,44 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
           "l"(reinterpret_cast<unsigned long long &>(c)));
     return r;
 }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long &>(r))
+        : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)));
+    return r;
+}
+
+// Exact GELU, v * Phi(v) = max(v, 0) - |v| * Phi(-|v|), for two values.  Phi(-|v|) = erfc(z) / 2 with
+// z = |v| / sqrt 2, and erfc(z) = exp(-z*z) * t * Q(t) with t = 1 / (1 + 0.37 z): the substitution of
+// Hastings (Abramowitz and Stegun 7.1.26) with the exponential and the leading t factored out, and Q
+// the degree-6 minimax polynomial of that quotient (own fit over 0 <= z <= 6.5: relative error 3.7e-7,
+// 7e-7 evaluated in fp32).  The error is relative, so the tail of negative v keeps its leading digits,
+// which 1 + erf(v / sqrt 2) cancels away.  Both reciprocals come from one: the special-function unit
+// bounds this (1.5 of its operations an element).  With erff per element the epilogue of a
+// 768 -> 3072 layer took longer than its products (175 us against 115 us for 3072 -> 768, 16 384 rows).
 __device__ __forceinline__ float2 gelu2(float a, float b) {
-    const float2 z = make_float2(fabsf(a) * 0.70710678118654752440f, fabsf(b) * 0.70710678118654752440f);
-    float2 t;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.x) : "f"(fmaf(0.5f, z.x, 1.0f)));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.y) : "f"(fmaf(0.5f, z.y, 1.0f)));
     auto c = [](float v) { return make_float2(v, v); };
-    float2 p = fma2(c(0.17087277f), t, c(-0.82215223f));
-    p = fma2(p, t, c(1.48851587f));
-    p = fma2(p, t, c(-1.13520398f));
-    p = fma2(p, t, c(0.27886807f));
-    p = fma2(p, t, c(-0.18628806f));
-    p = fma2(p, t, c(0.09678418f));
-    p = fma2(p, t, c(0.37409196f));
-    p = fma2(p, t, c(1.00002368f));
-    p = fma2(p, t, c(-1.26551223f));
-    p = fma2(make_float2(-z.x, -z.y), z, p);
-    const float log2e = 1.4426950408889634f;
+    // (beyond 64 the exponential is zero: the bound only keeps infinities out of the products)
+    const float ua = fminf(fabsf(a), 64.f), ub = fminf(fabsf(b), 64.f);
+    const float d0 = fmaf(0.261629508f, ua, 1.0f), d1 = fmaf(0.261629508f, ub, 1.0f);
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d0 * d1));
+    const float2 t = mul2(c(r), make_float2(d1, d0));
+    // Q / 2
+    float2 q = fma2(c(-0.0729324635f), t, c(0.22384969f));
+    q = fma2(q, t, c(-0.102016685f));
+    q = fma2(q, t, c(0.1653087285f));
+    q = fma2(q, t, c(0.073651064f));
+    q = fma2(q, t, c(0.107995136f));
+    q = fma2(q, t, c(0.104144361f));
+    const float2 v = make_float2(a, b);
+    const float2 x = mul2(mul2(v, c(-0.72134752044f)), v);  // -z*z * log2(e)
     float2 e;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(p.x * log2e));
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(p.y * log2e));
-    const float hx = 0.5f * t.x * e.x, hy = 0.5f * t.y * e.y;  // Phi(-|v|)
-    return make_float2(a * (a > 0.f ? 1.0f - hx : hx), b * (b > 0.f ? 1.0f - hy : hy));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(x.x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(x.y));
+    const float2 h = mul2(mul2(q, t), e);
+    return make_float2(fmaf(-ua, h.x, fmaxf(a, 0.f)), fmaf(-ub, h.y, fmaxf(b, 0.f)));
 }
 
 __device__ __forceinline__ float apply_act(float v, int act) {

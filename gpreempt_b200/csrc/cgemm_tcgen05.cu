@@ -58,9 +58,14 @@ struct CgemmCfg {
     static constexpr uint32_t kPlanes = TWO ? 2 : 1;
     static constexpr uint32_t kABytes = kCBM * kCBK * 2;        // one plane of A: 16 KiB
     static constexpr uint32_t kWBytes = BN * kCBK * 2;          // one plane of W
-    static constexpr uint32_t kStageBytes = kPlanes * (kABytes + kWBytes);
-    static constexpr int kStages = (int)((192u * 1024u) / kStageBytes);  // 3..8
-    static constexpr uint32_t kWOff = kPlanes * kABytes;        // W (hi) tile inside a stage
+    static constexpr uint32_t kKbBytes = kPlanes * (kABytes + kWBytes);  // operands of one K block
+    static constexpr uint32_t kWOff = kPlanes * kABytes;        // W (hi) tile inside a K block
+    // K blocks a ring stage holds at most.  The round of one stage (barrier waits, message, commit) costs
+    // either role ~300 cycles; a 64- or 128-column product of one plane takes 128 or 256, so two
+    // of them share a round (VGG-16's 64-column layer at batch 16: 168 -> see the table of cases).
+    static constexpr int kKps = (!TWO && BN <= 128) ? 2 : 1;
+    static constexpr uint32_t kStageBytes = kKps * kKbBytes;
+    static constexpr int kStages = (int)((192u * 1024u) / kStageBytes);  // 3 or 4
     // ring + alignment slack + 64x64 identity tile + control block
     static constexpr uint32_t kIdentBytes = 64 * kCBK * 2;
     static constexpr size_t kSmem =
@@ -73,8 +78,10 @@ struct CgemmCfg {
     static_assert(kTmemCols <= 512 && kStages <= 8, "tile does not fit");
 };
 
-enum : int { CMSG_DATA = 0, CMSG_STOP = 1, CMSG_EXIT = 2, CMSG_RES = 3 };
-enum : int { CEPI_COMPLETE = 0, CEPI_PARTIAL = 1, CEPI_EXIT = 2 };
+// Message of a ring stage: CMSG_DATA + number of K blocks, CMSG_RES + index of the residual block, or
+// the word was seen raised.  (The end of a CTA's schedule needs no message: every role counts tiles.)
+enum : int { CMSG_STOP = 1, CMSG_DATA = 4, CMSG_RES = 16 };
+enum : int { CEPI_COMPLETE = 0, CEPI_PARTIAL = 1 };
 
 struct CgemmControl {
     unsigned long long full[8];
@@ -167,12 +174,25 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     // they run at the same time.  With k_splits == 1 a tile covers the whole K range.
     const int total_tiles = p.tiles_m * p.tiles_n * p.k_splits;
     const int all_kb = p.taps * p.cin_blocks;
-    auto tile_kb_begin = [&](int tile) { return p.k_splits == 1 ? 0 : (tile % p.k_splits) * p.kb_per_split; };
-    auto tile_kb_count = [&](int tile) {
-        int left = all_kb - tile_kb_begin(tile);
-        return left < p.kb_per_split ? left : p.kb_per_split;
+    struct TileAt {
+        int m_blk, n_blk, split, kb_base, main_kb;
+    };
+    auto tile_at = [&](int tile) {
+        TileAt t;
+        const int otile = p.k_splits == 1 ? tile : fast_div(tile, p.k_splits, p.inv_k_splits);
+        t.split = tile - otile * p.k_splits;
+        // Column tiles vary fastest: CTAs that run together share the same A rows.
+        t.m_blk = p.tiles_n == 1 ? otile : fast_div(otile, p.tiles_n, p.inv_tiles_n);
+        t.n_blk = otile - t.m_blk * p.tiles_n;
+        t.kb_base = t.split * p.kb_per_split;
+        const int left = all_kb - t.kb_base;
+        t.main_kb = left < p.kb_per_split ? left : p.kb_per_split;
+        return t;
     };
     const bool resumable = blp.preempted != nullptr;
+    // Split K inside a cluster: the last ring stage is where the peers' partial sums land.
+    const bool in_cluster = BN == 64 && p.cluster_reduce;
+    const int nst = in_cluster ? kStages - 1 : kStages;
 
     CgemmSlot *slot = p.slots + blockIdx.x;
     float *spill = p.spill + (size_t)blockIdx.x * cgemm_spill_floats();
@@ -185,7 +205,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&ctl->tmem_full[b]), 2);
             mbar_init(smem_u32(&ctl->tmem_empty[b]), 1);
-            ctl->epi_kind[b] = CEPI_EXIT;
+            ctl->epi_kind[b] = CEPI_COMPLETE;
             ctl->epi_k_done[b] = 0;
         }
         ctl->abort_flag = 0;
@@ -207,6 +227,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = ctl->tmem_base;
+    if (in_cluster) cluster_arrive();  // this CTA runs: its shared memory may be written to
 
     // A non-preemptible launch knows its first tile without reading the cursor, and weights are
     // never written by a kernel: its producer thread fetches the weight tiles of the first ring
@@ -214,37 +235,50 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     // predecessor's tail (batch-1 forwards are chains of such latencies).  Every other thread,
     // and every thread of a preemptible launch, waits here.
     const bool early_weights = !resumable && (int)blockIdx.x < total_tiles;
-    int prearmed = 0;  // ring stages whose barrier is armed and whose weight loads are in flight
-    constexpr uint32_t kDataBytes = Cfg::kStageBytes;
+    int prearmed = 0;  // K blocks whose barrier is armed and whose weight loads are in flight
+    constexpr int KPS = Cfg::kKps;
+    TileAt first_tile{};
+    int tap0 = 0, cb0 = 0;  // filter tap and channel block of its first K block
+    if (early_weights) first_tile = tile_at(blockIdx.x);
+    const bool issuer = elect_one();
     if (early_weights && warp == 0) {
-        const int tile = blockIdx.x;
-        const int n_blk = (tile / p.k_splits) % p.tiles_n;
-        const int main_kb = tile_kb_count(tile);
-        const int kb_base = tile_kb_begin(tile);
-        prearmed = main_kb < kStages ? main_kb : kStages;
-        int tap = kb_base / p.cin_blocks;
-        int cb = kb_base - tap * p.cin_blocks;
-        for (int kb = 0; kb < prearmed; ++kb) {
-            if (elect_one()) {
-                const uint32_t bar = smem_u32(&ctl->full[kb]);
+        prearmed = first_tile.main_kb < nst * KPS ? first_tile.main_kb : nst * KPS;
+        tap0 = p.taps == 1 ? 0 : fast_div(first_tile.kb_base, p.cin_blocks, p.inv_cin_blocks);
+        cb0 = first_tile.kb_base - tap0 * p.cin_blocks;
+        int cb = cb0, w_tap = tap0 * p.cin, st = 0;
+        for (int kb = 0; kb < prearmed; ++st) {
+            const uint32_t bar = smem_u32(&ctl->full[st]);
+            const int n = prearmed - kb < KPS ? prearmed - kb : KPS;
+            if (issuer) {
                 const uint32_t ident_bytes = (p.res_kb && kb == 0) ? Cfg::kIdentBytes : 0u;
-                ctl->stage_msg[kb] = CMSG_DATA;
-                mbar_arrive_expect_tx(bar, kDataBytes + ident_bytes);
+                ctl->stage_msg[st] = CMSG_DATA + n;
+                mbar_arrive_expect_tx(bar, n * Cfg::kKbBytes + ident_bytes);
                 if (ident_bytes) tma_load_2d(smem_base + ident_off, &p.ident, bar, 0, 0);
-                const uint32_t dst = smem_base + kb * Cfg::kStageBytes;
-                const int w_col = tap * p.cin + cb * kCBK;
-                tma_load_2d(dst + Cfg::kWOff, &p.w_hi, bar, w_col, n_blk * BN);
-                if (TWO) tma_load_2d(dst + Cfg::kWOff + Cfg::kWBytes, &p.w_lo, bar, w_col, n_blk * BN);
             }
-            if (++cb == p.cin_blocks) {
-                cb = 0;
-                ++tap;
+#pragma unroll
+            for (int j = 0; j < KPS; ++j) {
+                if (j > 0 && j >= n) break;
+                const uint32_t dst = smem_base + st * Cfg::kStageBytes + j * Cfg::kKbBytes;
+                if (issuer) {
+                    tma_load_2d(dst + Cfg::kWOff, &p.w_hi, bar, w_tap + cb * kCBK, first_tile.n_blk * BN);
+                    if (TWO) tma_load_2d(dst + Cfg::kWOff + Cfg::kWBytes, &p.w_lo, bar, w_tap + cb * kCBK, first_tile.n_blk * BN);
+                }
+                if (++cb == p.cin_blocks) {
+                    cb = 0;
+                    w_tap += p.cin;
+                }
             }
+            kb += n;
         }
         __syncwarp();
     }
     pdl_wait();  // from here on the predecessor's results (and this executor's slots) are visible
     pdl_launch_dependents();
+    TCK(t_begin);
+    if (in_cluster) cluster_wait();
+#ifdef GPX_CGEMM_TIMING
+    if (threadIdx.x == 64) TADD(16, clock64() - t_begin);
+#endif
 
     // A non-preemptible launch never stops early, so it neither reads nor writes the cursor.
     const int first_iter = resumable ? slot->next_iter : 0;
@@ -290,6 +324,14 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         if (atomicCAS(p.error, 0, code) == 0) p.error[1] = blp.kernel_id * 1000 + (int)blockIdx.x;
     };
 
+    // Cluster reduction: what this thread finishes (eight-channel items; two of them when S = 2).
+    constexpr int kGroups = BN / 8, kFinItems = 64 * kGroups / kCEpiThreads;
+    bool fin_live[kFinItems] = {};
+    int fin_col[kFinItems];
+    size_t fin_off[kFinItems];
+    float fin_bias[kFinItems][8];
+    uint4 fin_rhi[kFinItems], fin_rlo[kFinItems];
+
     if (!grid_ok) {
         if (threadIdx.x == 0) fail(900);
     } else if (warp == 0) {
@@ -300,7 +342,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         // block, on a lone thread, was a third of the ~780 cycles a K block cost here before.
         int stage = 0;
         uint32_t phase = 0;
-        int msg = CMSG_EXIT;
         bool ok = true;
         // The identity tile travels with the first stage this CTA fills.
         uint32_t ident_bytes = (p.res_kb && prearmed == 0) ? Cfg::kIdentBytes : 0u;
@@ -309,75 +350,113 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
 #ifdef GPX_CGEMM_TIMING
         long long prod_wait = 0;
 #endif
-        for (int it = first_iter; ok; ++it) {
+        int kb = first_k;
+        int tap = tap0, cb = cb0;
+        if (prearmed) {
+            // The weights of these stages are already on their way: only activations are missing.
+            const int row0 = first_tile.m_blk * kCBM;
+            int a_row = row0 + p.tap_shift[tap];
+            for (; kb < prearmed; ++stage) {
+                const uint32_t bar = smem_u32(&ctl->full[stage]);
+                const int n = prearmed - kb < KPS ? prearmed - kb : KPS;
+#pragma unroll
+                for (int j = 0; j < KPS; ++j) {
+                    if (j > 0 && j >= n) break;
+                    const uint32_t dst = smem_base + stage * Cfg::kStageBytes + j * Cfg::kKbBytes;
+                    if (issuer) {
+                        tma_load_2d(dst, &p.a_hi, bar, cb * kCBK, a_row);
+                        if (TWO) tma_load_2d(dst + Cfg::kABytes, &p.a_lo, bar, cb * kCBK, a_row);
+                    }
+                    if (++cb == p.cin_blocks) {
+                        cb = 0;
+                        if (++tap < p.taps) a_row = row0 + p.tap_shift[tap];
+                    }
+                }
+                kb += n;
+            }
+            __syncwarp();
+            if (stage == nst) {
+                stage = 0;
+                phase ^= 1;
+            }
+        }
+        for (int it = first_iter; ok; ++it, kb = 0) {
             const int tile = blockIdx.x + it * gridDim.x;
             if (tile >= total_tiles) break;
-            // Column tiles vary fastest: CTAs that run together share the same A rows.
-            const int otile = p.k_splits == 1 ? tile : tile / p.k_splits;
-            const int m_blk = otile / p.tiles_n;
-            const int n_blk = otile - m_blk * p.tiles_n;
-            const int kb0 = it == first_iter ? first_k : 0;
-            const int main_kb = tile_kb_count(tile);
-            const int num_kb = main_kb + p.res_kb;  // the residual rides along as extra K blocks
-            const int kb_abs = tile_kb_begin(tile) + kb0;
-            int tap = p.taps == 1 ? 0 : kb_abs / p.cin_blocks;
-            int cb = kb_abs - tap * p.cin_blocks;
-            int a_row = m_blk * kCBM + p.tap_shift[tap < p.taps ? tap : 0];
+            const TileAt t = tile_at(tile);
+            const int num_kb = t.main_kb + p.res_kb;  // the residual rides along as extra K blocks
+            const int row0 = t.m_blk * kCBM, w_row = t.n_blk * BN;
+            if (it > first_iter || !prearmed) {
+                const int kb_abs = t.kb_base + kb;
+                tap = p.taps == 1 ? 0 : fast_div(kb_abs, p.cin_blocks, p.inv_cin_blocks);
+                cb = kb_abs - tap * p.cin_blocks;
+            }
+            int a_row = row0 + p.tap_shift[tap < p.taps ? tap : 0];
             int w_tap = tap * p.cin;
-            for (int kb = kb0; kb < num_kb; ++kb) {
+            while (kb < num_kb) {
                 const uint32_t bar = smem_u32(&ctl->full[stage]);
                 const uint32_t dst = smem_base + stage * Cfg::kStageBytes;
-                const bool armed = it == first_iter && kb < prearmed;  // weights already on their way
                 TCK(t_w0);
-                if (!armed) {
-                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1, abort_flag, kCWaitLimitNs))) {
-                        if (lane == 0) fail(101);
-                        ok = false;
-                        break;
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1, abort_flag, kCWaitLimitNs))) {
+                    if (lane == 0) fail(101);
+                    ok = false;
+                    break;
+                }
+                if (resumable && __any_sync(0xffffffffu, *word_up)) {
+                    if (issuer) {
+                        ctl->stage_msg[stage] = CMSG_STOP;
+                        mbar_arrive(bar);
+                        if (blp.trace) atomicMin(blp.trace + 2, globaltimer_ns());
                     }
-                    if (resumable && __any_sync(0xffffffffu, *word_up)) {
-                        msg = CMSG_STOP;
-                        ok = false;
-                        break;
-                    }
+                    ok = false;
+                    break;
                 }
 #ifdef GPX_CGEMM_TIMING
                 prod_wait += clock64() - t_w0;
 #endif
-                if (kb >= main_kb) {
+                if (kb >= t.main_kb) {
                     // Residual block: A = 64 channels of the residual rows of this tile; the W
                     // operand is the 64x64 identity that stays in shared memory, applied to the
                     // matching 64 accumulator columns, so the tensor core adds the residual.
-                    const int rb = kb - main_kb;
-                    if (elect_one()) {
+                    const int rb = kb - t.main_kb;
+                    if (issuer) {
                         ctl->stage_msg[stage] = CMSG_RES + rb;
                         mbar_arrive_expect_tx(bar, Cfg::kPlanes * Cfg::kABytes + ident_bytes);
-                        tma_load_2d(dst, &p.r_hi, bar, n_blk * BN + rb * kCBK, m_blk * kCBM);
-                        if (TWO) tma_load_2d(dst + Cfg::kABytes, &p.r_lo, bar, n_blk * BN + rb * kCBK, m_blk * kCBM);
+                        tma_load_2d(dst, &p.r_hi, bar, w_row + rb * kCBK, row0);
+                        if (TWO) tma_load_2d(dst + Cfg::kABytes, &p.r_lo, bar, w_row + rb * kCBK, row0);
                         if (ident_bytes) tma_load_2d(smem_base + ident_off, &p.ident, bar, 0, 0);
                     }
-                } else if (elect_one()) {
-                    if (!armed) {
-                        ctl->stage_msg[stage] = CMSG_DATA;
-                        mbar_arrive_expect_tx(bar, kDataBytes + ident_bytes);
+                    ++kb;
+                } else {
+                    const int n = t.main_kb - kb < KPS ? t.main_kb - kb : KPS;
+                    if (issuer) {
+                        ctl->stage_msg[stage] = CMSG_DATA + n;
+                        mbar_arrive_expect_tx(bar, n * Cfg::kKbBytes + ident_bytes);
                         if (ident_bytes) tma_load_2d(smem_base + ident_off, &p.ident, bar, 0, 0);
                     }
-                    tma_load_2d(dst, &p.a_hi, bar, cb * kCBK, a_row);
-                    if (TWO) tma_load_2d(dst + Cfg::kABytes, &p.a_lo, bar, cb * kCBK, a_row);
-                    if (!armed) {
-                        tma_load_2d(dst + Cfg::kWOff, &p.w_hi, bar, w_tap + cb * kCBK, n_blk * BN);
-                        if (TWO) tma_load_2d(dst + Cfg::kWOff + Cfg::kWBytes, &p.w_lo, bar, w_tap + cb * kCBK, n_blk * BN);
+#pragma unroll
+                    for (int j = 0; j < KPS; ++j) {
+                        if (j > 0 && j >= n) break;
+                        const uint32_t d = dst + j * Cfg::kKbBytes;
+                        if (issuer) {
+                            tma_load_2d(d, &p.a_hi, bar, cb * kCBK, a_row);
+                            tma_load_2d(d + Cfg::kWOff, &p.w_hi, bar, w_tap + cb * kCBK, w_row);
+                            if (TWO) {
+                                tma_load_2d(d + Cfg::kABytes, &p.a_lo, bar, cb * kCBK, a_row);
+                                tma_load_2d(d + Cfg::kWOff + Cfg::kWBytes, &p.w_lo, bar, w_tap + cb * kCBK, w_row);
+                            }
+                        }
+                        if (++cb == p.cin_blocks) {
+                            cb = 0;
+                            w_tap += p.cin;
+                            if (++tap < p.taps) a_row = row0 + p.tap_shift[tap];
+                        }
                     }
+                    kb += n;
                 }
                 __syncwarp();
-                if (!armed) ident_bytes = 0;
-                if (++cb == p.cin_blocks) {
-                    cb = 0;
-                    ++tap;
-                    w_tap += p.cin;
-                    if (tap < p.taps) a_row = m_blk * kCBM + p.tap_shift[tap];
-                }
-                if (++stage == kStages) {
+                ident_bytes = 0;
+                if (++stage == nst) {
                     stage = 0;
                     phase ^= 1;
                 }
@@ -389,20 +468,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             TADD(1, clock64() - t_prod0);
         }
 #endif
-        if (!*abort_flag) {
-            bool have_slot = msg == CMSG_STOP;
-            if (!have_slot)
-                have_slot = mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1, abort_flag, kCWaitLimitNs);
-            if (lane == 0) {
-                if (have_slot) {
-                    ctl->stage_msg[stage] = msg;
-                    mbar_arrive(smem_u32(&ctl->full[stage]));
-                } else {
-                    fail(102);
-                }
-                if (msg == CMSG_STOP && blp.trace) atomicMin(blp.trace + 2, globaltimer_ns());
-            }
-        }
         if (lane == 0) *(volatile int *)&ctl->poll_done = 1;
         __syncwarp();
     } else if (warp == 1) {
@@ -415,18 +480,19 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         const uint32_t idesc64 = (!TWO && p.fmt == PF_F16) ? make_idesc_f16_f32(kCBM, 64) : make_idesc_bf16_f32(kCBM, 64);
         const uint64_t eye = make_smem_desc_sw128(smem_base + ident_off);
         const uint64_t ring = make_smem_desc_sw128(smem_base);
+        const int res_kb = p.res_kb;
         int stage = 0;
         uint32_t phase = 0;
         int kb = first_k;
-        int it = first_iter;
         TCK(t_mma0);
 #ifdef GPX_CGEMM_TIMING
         long long mma_wait_full = 0, mma_wait_tmem = 0, mma_kb = 0;
 #endif
-        for (uint32_t seg = 0;; ++seg) {
+        uint32_t seg = 0;
+        for (int tile = blockIdx.x + first_iter * gridDim.x; tile < total_tiles; tile += gridDim.x, ++seg, kb = 0) {
             const int buf = (int)(seg & 1);
             const uint32_t acc0 = tmem_base + buf * kBufCols;
-            const int num_kb = tile_kb_count(blockIdx.x + it * gridDim.x) + p.res_kb;
+            const int num_kb = tile_at(tile).main_kb + res_kb;
             TCK(t_e0);
             if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->tmem_empty[buf]), (seg >> 1) & 1, abort_flag, kCWaitLimitNs))) {
                 if (lane == 0) fail(202);
@@ -437,7 +503,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
 #endif
             tc_fence_after_sync();
             int end = CEPI_COMPLETE;
-            for (; kb < num_kb; ++kb) {
+            while (kb < num_kb) {
                 TCK(t_f0);
                 if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->full[stage]), phase, abort_flag, kCWaitLimitNs))) {
                     if (lane == 0) fail(201);
@@ -450,16 +516,14 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
 #endif
                 tc_fence_after_sync();
                 const int msg = __shfl_sync(0xffffffffu, ctl->stage_msg[stage], 0);
-                if (msg == CMSG_STOP || msg == CMSG_EXIT) {
-                    end = msg == CMSG_STOP ? CEPI_PARTIAL : CEPI_EXIT;
+                if (msg == CMSG_STOP) {
+                    end = CEPI_PARTIAL;
                     break;
                 }
+                const int n = msg >= CMSG_RES ? 1 : msg - CMSG_DATA;  // K blocks in this stage
                 // descriptor addresses are in 16-byte units
-                const uint64_t a_hi = ring + (uint64_t)(stage * (Cfg::kStageBytes >> 4));
-                const uint64_t a_lo = a_hi + (Cfg::kABytes >> 4);
-                const uint64_t w_hi = a_hi + (Cfg::kWOff >> 4);
-                const uint32_t acc = kb > 0 ? 1u : 0u;
-                if (elect_one()) {
+                const uint64_t a0 = ring + (uint64_t)(stage * (Cfg::kStageBytes >> 4));
+                if (issuer) {
                     if (msg >= CMSG_RES) {
                         // residual x identity on 64 accumulator columns: the hi plane into the hi*hi
                         // accumulator, the lo plane into the cross-term accumulator (exact products,
@@ -467,38 +531,50 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                         const uint32_t col = (uint32_t)(msg - CMSG_RES) * 64;
 #pragma unroll
                         for (int k = 0; k < kCBK / kCUmmaK; ++k) {
-                            mma_f16_ss(acc0 + col, a_hi + 2 * k, eye + 2 * k, idesc64, 1u);
-                            if (TWO) mma_f16_ss(acc0 + BN + col, a_lo + 2 * k, eye + 2 * k, idesc64, 1u);
-                        }
-                    } else if (TWO) {
-                        // fp32 product from three bf16 products: hi*hi in one accumulator, both cross
-                        // terms in the other.  The tensor core truncates when it adds into the fp32
-                        // accumulator, a bias that grows with the length of the accumulation chain;
-                        // keeping the small cross terms apart keeps them clear of it.  The W_lo tile
-                        // follows the W_hi tile in the stage and the two accumulators are adjacent
-                        // columns, so A_hi x [W_hi; W_lo] is ONE instruction of width 2*BN, which
-                        // reads the A_hi tile once.  The order is fixed, so a resumed tile replays
-                        // exactly the instruction sequence of an uninterrupted one.
-#pragma unroll
-                        for (int k = 0; k < kCBK / kCUmmaK; ++k) {
-                            mma_f16_ss(acc0, a_hi + 2 * k, w_hi + 2 * k, idesc_wide, k > 0 ? 1u : acc);
-                            mma_f16_ss(acc0 + BN, a_lo + 2 * k, w_hi + 2 * k, idesc, 1u);
+                            mma_f16_ss(acc0 + col, a0 + 2 * k, eye + 2 * k, idesc64, 1u);
+                            if (TWO) mma_f16_ss(acc0 + BN + col, a0 + (Cfg::kABytes >> 4) + 2 * k, eye + 2 * k, idesc64, 1u);
                         }
                     } else {
 #pragma unroll
-                        for (int k = 0; k < kCBK / kCUmmaK; ++k)
-                            mma_f16_ss(acc0, a_hi + 2 * k, w_hi + 2 * k, idesc, k > 0 ? 1u : acc);
+                        for (int j = 0; j < KPS; ++j) {
+                            if (j > 0 && j >= n) break;
+                            const uint64_t a_hi = a0 + j * (Cfg::kKbBytes >> 4);
+                            const uint64_t a_lo = a_hi + (Cfg::kABytes >> 4);
+                            const uint64_t w_hi = a_hi + (Cfg::kWOff >> 4);
+                            const uint32_t acc = (j > 0 || kb > 0) ? 1u : 0u;
+                            if (TWO) {
+                                // fp32 product from three bf16 products: hi*hi in one accumulator, both
+                                // cross terms in the other.  The tensor core truncates when it adds into
+                                // the fp32 accumulator, a bias that grows with the length of the
+                                // accumulation chain; keeping the small cross terms apart keeps them
+                                // clear of it.  The W_lo tile follows the W_hi tile in the stage and
+                                // the two accumulators are adjacent columns, so A_hi x [W_hi; W_lo] is
+                                // ONE instruction of width 2*BN, which reads the A_hi tile once.  The
+                                // order is fixed, so a resumed tile replays exactly the instruction
+                                // sequence of an uninterrupted one.
+#pragma unroll
+                                for (int k = 0; k < kCBK / kCUmmaK; ++k) {
+                                    mma_f16_ss(acc0, a_hi + 2 * k, w_hi + 2 * k, idesc_wide, k > 0 ? 1u : acc);
+                                    mma_f16_ss(acc0 + BN, a_lo + 2 * k, w_hi + 2 * k, idesc, 1u);
+                                }
+                            } else {
+#pragma unroll
+                                for (int k = 0; k < kCBK / kCUmmaK; ++k)
+                                    mma_f16_ss(acc0, a_hi + 2 * k, w_hi + 2 * k, idesc, k > 0 ? 1u : acc);
+                            }
+                        }
                     }
                     mma_commit(smem_u32(&ctl->empty[stage]));
                 }
+                kb += n;
                 __syncwarp();
-                if (++stage == kStages) {
+                if (++stage == nst) {
                     stage = 0;
                     phase ^= 1;
                 }
             }
             if (end < 0) break;
-            if (elect_one()) {
+            if (issuer) {
                 ctl->epi_kind[buf] = end;
                 ctl->epi_k_done[buf] = kb;
                 mma_commit(smem_u32(&ctl->tmem_full[buf]));
@@ -506,8 +582,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             }
             __syncwarp();
             if (end != CEPI_COMPLETE) break;
-            ++it;
-            kb = 0;
         }
 #ifdef GPX_CGEMM_TIMING
         if (lane == 0) {
@@ -543,6 +617,50 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         const int row = quarter * 32 + lane;
         const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
         const bool leader = threadIdx.x == 64;
+        uint32_t push = 0;  // where the partial sums of this thread's row go (cluster reduction)
+        if (in_cluster) {
+            // What the finishing step needs, ahead of the products: destination, bias, residual.
+            const SplitKParams &fin = p.fin;
+            const int rows_share = kCBM / p.k_splits;
+            const int img = fin.in_hs * fin.in_ws;
+            const int rank = (int)cluster_ctarank();
+#pragma unroll
+            for (int i = 0; i < kFinItems; ++i) {
+                const int e = (int)threadIdx.x - 64 + i * kCEpiThreads;
+                const int lr = e / kGroups, col0 = first_tile.n_blk * BN + (e - lr * kGroups) * 8;
+                const int vrow = first_tile.m_blk * kCBM + rank * rows_share + lr;
+                bool live = lr < rows_share && vrow < fin.m_rows && col0 < fin.cout_padded;
+                int n_img = 0, h = 0, w = 0;
+                if (live) {
+                    n_img = fast_div(vrow, img, p.inv_img);
+                    const int r = vrow - n_img * img;
+                    const int hs = fast_div(r, fin.in_ws, p.inv_in_ws);
+                    h = hs - fin.in_off;
+                    w = r - hs * fin.in_ws - fin.in_off;
+                    live = h >= 0 && h < fin.out.H && w >= 0 && w < fin.out.W;
+                }
+                if (live) {
+                    if (fin.bias) {
+                        const float4 *b4 = reinterpret_cast<const float4 *>(fin.bias + col0);
+                        const float4 b0 = __ldg(b4), b1 = __ldg(b4 + 1);
+                        fin_bias[i][0] = b0.x, fin_bias[i][1] = b0.y, fin_bias[i][2] = b0.z, fin_bias[i][3] = b0.w;
+                        fin_bias[i][4] = b1.x, fin_bias[i][5] = b1.y, fin_bias[i][6] = b1.z, fin_bias[i][7] = b1.w;
+                    }
+                    if (fin.res_hi)
+                        planes_fetch8(fin.res_hi, fin.res_lo, (size_t)layout_row(fin.res, n_img, h, w) * fin.res.C + col0,
+                                      fin.res.fmt, fin_rhi[i], fin_rlo[i]);
+                    fin_off[i] = fin.out_f32 ? ((size_t)(n_img * fin.out.H + h) * fin.out.W + w) * fin.cout_valid + col0
+                                             : (size_t)layout_row(fin.out, n_img, h, w) * fin.out.C + col0;
+                    fin_col[i] = col0;
+                }
+                fin_live[i] = live;
+            }
+            const int rows_per = kCBM / p.k_splits;
+            const int owner = row / rows_per;
+            push = cluster_map_shared(smem_base + (uint32_t)(nst * Cfg::kStageBytes) +
+                                          (uint32_t)(((int)cluster_ctarank() * rows_per + row - owner * rows_per) * (BN + 4)) * 4,
+                                      (uint32_t)owner);
+        }
         uint32_t v[32];
         if (first_k > 0) {
             for (int c = s_lo; c < s_hi; c += 32) {
@@ -571,34 +689,84 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         int seg_k0 = first_k;
         int tiles_done = 0;
         const int img = p.in_hs * p.in_ws;
+        // Fields the drain loop needs, in registers: the loop is full of asm statements that clobber
+        // memory, after each of which they would be read from the parameter block again.
+        const float *const bias = p.partial ? nullptr : p.bias;
+        const int relu = p.relu, fmt = p.fmt;
+        float *const partial = p.partial;
+        float *const out_f32 = p.out_f32;
+        bf16_bits *const out_hi = p.out_hi, *const out_lo = p.out_lo;
+        const bf16_bits *const res_hi = p.res_hi, *const res_lo = p.res_lo;
         float bias_next = 0.f;  // this thread's bias element of the next tile to drain
-        if (p.bias && !p.partial) {
+        if (bias) {
             const int t = (int)threadIdx.x - 64;
-            const int first_tile = blockIdx.x + first_iter * gridDim.x;
-            if (t < BN && first_tile < total_tiles)
-                bias_next = __ldg(p.bias + ((first_tile / p.k_splits) % p.tiles_n) * BN + t);
+            const int first = blockIdx.x + first_iter * gridDim.x;
+            if (t < BN && first < total_tiles) bias_next = __ldg(bias + tile_at(first).n_blk * BN + t);
         }
         TCK(t_epi0);
 #ifdef GPX_CGEMM_TIMING
         long long e_wait = 0, e_tmem = 0, e_math = 0, e_store = 0, e_bar = 0;
 #endif
         for (uint32_t seg = 0;; ++seg) {
+            const int tile = blockIdx.x + it * gridDim.x;
+            if (tile >= total_tiles) {
+                if (leader && resumable) {
+                    slot->next_iter = it;
+                    slot->k_done = 0;
+                    slot->grid = gridDim.x;
+                }
+                break;
+            }
             const int buf = (int)(seg & 1);
             const uint32_t t_acc = t_lane + buf * kBufCols;
             TCK(t_wait0);
+            const TileAt at = tile_at(tile);
+            const int n_blk = at.n_blk;
             // The bias of the tile this buffer holds goes to shared memory before the drain loop
             // (read from global memory inside it, its latency - an L2 round trip under load - was
             // paid once per 16-column piece).  The value stored now was requested one tile ago
             // and the request for the tile after this one is issued here, so the round trip
             // overlaps the drain of this tile instead of delaying its start.
-            if (p.bias && !p.partial) {
+            if (bias) {
                 const int t = (int)threadIdx.x - 64;
                 if (t < BN) {
                     ctl->bias_s[buf][t] = bias_next;
-                    const int after = blockIdx.x + (it + 1) * gridDim.x;
-                    if (after < total_tiles) bias_next = __ldg(p.bias + ((after / p.k_splits) % p.tiles_n) * BN + t);
+                    const int after = tile + gridDim.x;
+                    if (after < total_tiles) bias_next = __ldg(bias + tile_at(after).n_blk * BN + t);
                 }
             }
+            // Which output pixel, if any, does this GEMM row stand for?  (Before the wait: the answer
+            // does not depend on the products.)
+            const int vrow = at.m_blk * kCBM + row;
+            bool valid = vrow < p.m_rows;
+            size_t out_off = 0, res_off = 0;
+            if (p.identity_rows) {
+                // plain rows in, plain rows out (and a plain residual): row m of the GEMM is
+                // row m of the output, no pixel arithmetic is needed
+                if (valid) {
+                    out_off = (size_t)vrow * p.out.C + (size_t)n_blk * BN;
+                    if (res_hi) res_off = (size_t)vrow * p.res.C + (size_t)n_blk * BN;
+                }
+            } else {
+                int n_img = 0, h = 0, w = 0;
+                if (valid) {
+                    n_img = fast_div(vrow, img, p.inv_img);
+                    int r = vrow - n_img * img;
+                    int hs = fast_div(r, p.in_ws, p.inv_in_ws);
+                    int ws = r - hs * p.in_ws;
+                    h = hs - p.in_off;
+                    w = ws - p.in_off;
+                    valid = h >= 0 && h < p.out.H && w >= 0 && w < p.out.W;
+                }
+                if (valid) {
+                    out_off = out_f32 ? ((size_t)(n_img * p.out.H + h) * p.out.W + w) * p.cout_valid
+                                      : (size_t)layout_row(p.out, n_img, h, w) * p.out.C + (size_t)n_blk * BN;
+                    if (res_hi) res_off = (size_t)layout_row(p.res, n_img, h, w) * p.res.C + (size_t)n_blk * BN;
+                }
+            }
+            float *const part_row = partial ? partial + ((size_t)at.split * p.partial_rows + vrow) * p.partial_ld + n_blk * BN : nullptr;
+            const bool part_valid = vrow < p.m_rows;
+            const int col_lim = p.cout_valid - n_blk * BN;
             if (leader) {
                 bool ok = mbar_wait(smem_u32(&ctl->tmem_full[buf]), (seg >> 1) & 1, abort_flag, kCWaitLimitNs);
                 if (!ok) fail(301);
@@ -608,71 +776,28 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
 #ifdef GPX_CGEMM_TIMING
             e_wait += clock64() - t_wait0;
 #endif
+#ifdef GPX_CGEMM_TIMING
+            if (leader && seg == 0) TADD(17, clock64() - t_begin);
+#endif
             if (!ctl->epi_go) break;
             tc_fence_after_sync();
             const int kind = ctl->epi_kind[buf];
             const int k_done = ctl->epi_k_done[buf];
-            if (kind == CEPI_EXIT) {
-                if (leader && resumable) {
-                    slot->next_iter = it;
-                    slot->k_done = 0;
-                    slot->grid = gridDim.x;
-                }
-                break;
-            }
             if (kind == CEPI_COMPLETE) {
-                const int tile = blockIdx.x + it * gridDim.x;
-                int otile = tile, split = 0;
-                if (p.k_splits > 1) {
-                    otile = fast_div(tile, p.k_splits, p.inv_k_splits);
-                    split = tile - otile * p.k_splits;
-                }
-                const int m_blk = p.tiles_n > 1 ? fast_div(otile, p.tiles_n, p.inv_tiles_n) : otile;
-                const int n_blk = otile - m_blk * p.tiles_n;
-                // Which output pixel, if any, does this GEMM row stand for?
-                const int vrow = m_blk * kCBM + row;
-                bool valid = vrow < p.m_rows;
-                size_t out_off = 0, res_off = 0;
-                if (p.identity_rows) {
-                    // plain rows in, plain rows out (and a plain residual): row m of the GEMM is
-                    // row m of the output, no pixel arithmetic is needed
-                    if (valid) {
-                        out_off = (size_t)vrow * p.out.C + (size_t)n_blk * BN;
-                        if (p.res_hi) res_off = (size_t)vrow * p.res.C + (size_t)n_blk * BN;
-                    }
-                } else {
-                    int n_img = 0, h = 0, w = 0;
-                    if (valid) {
-                        n_img = fast_div(vrow, img, p.inv_img);
-                        int r = vrow - n_img * img;
-                        int hs = fast_div(r, p.in_ws, p.inv_in_ws);
-                        int ws = r - hs * p.in_ws;
-                        h = hs - p.in_off;
-                        w = ws - p.in_off;
-                        valid = h >= 0 && h < p.out.H && w >= 0 && w < p.out.W;
-                    }
-                    if (valid) {
-                        out_off = p.out_f32 ? ((size_t)(n_img * p.out.H + h) * p.out.W + w) * p.cout_valid
-                                            : (size_t)layout_row(p.out, n_img, h, w) * p.out.C + (size_t)n_blk * BN;
-                        if (p.res_hi) res_off = (size_t)layout_row(p.res, n_img, h, w) * p.res.C + (size_t)n_blk * BN;
-                    }
-                }
                 // Every lane owns one row of the tile (its TMEM lane): 16 columns of a plane are 32
                 // contiguous bytes of that row, one 256-bit access, a whole sector.
-                const bool planes_out = !p.partial && !p.out_f32;
-                const int col_lim = p.cout_valid - n_blk * BN;
+                const bool use_res = !partial && !out_f32 && res_hi && valid;
                 constexpr int CH = TWO ? 16 : 32;  // columns per piece
 #pragma unroll 1
                 for (int c = c_lo; c < c_hi; c += CH) {
                     float f[CH];
                     // The residual is requested first so its latency overlaps the TMEM reads.
-                    const bool use_res = planes_out && p.res_hi && valid;
                     TCK(t_p0);
                     uint32_t rh[CH / 2], rl[TWO ? CH / 2 : 1];
                     if (use_res) {
 #pragma unroll
-                        for (int q = 0; q < CH / 16; ++q) ld_global_v8(p.res_hi + res_off + c + 16 * q, rh + 8 * q);
-                        if (TWO) ld_global_v8(p.res_lo + res_off + c, rl);
+                        for (int q = 0; q < CH / 16; ++q) ld_global_v8(res_hi + res_off + c + 16 * q, rh + 8 * q);
+                        if (TWO) ld_global_v8(res_lo + res_off + c, rl);
                     }
                     if constexpr (TWO) {
                         uint32_t t16[16], u16[16];
@@ -692,30 +817,28 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     long long t_p1 = clock64();
                     e_tmem += t_p1 - t_p0;
 #endif
-                    if (p.cluster_reduce) {
-                        // Split K inside a cluster: the raw fp32 sum of this K range stays in this
-                        // CTA's shared memory (the ring is idle: a CTA of such a launch runs one
-                        // tile); rows are 16 bytes longer than BN floats so that the 32 rows of a
-                        // warp spread over the banks.
-                        float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(smem) + (size_t)row * (BN + 4) + c);
+                    if (in_cluster) {
+                        // Split K inside a cluster: the raw fp32 sum of this row and K range goes
+                        // straight into the shared memory of the CTA that finishes the row (its last
+                        // ring stage: [split][row of its share][BN + 4 floats], the 4 spreading the
+                        // rows of a warp over the banks).
 #pragma unroll
                         for (int j = 0; j < CH / 4; ++j)
-                            dst[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+                            st_shared_cluster_f4(push + (uint32_t)(c + 4 * j) * 4, make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]));
                         continue;
                     }
-                    if (p.partial) {
+                    if (partial) {
                         // Split K: the raw fp32 sum of this K range goes to the workspace; the
                         // finishing kernel adds the ranges in split order and applies the rest.
-                        if (vrow < p.m_rows) {
-                            float4 *dst = reinterpret_cast<float4 *>(
-                                p.partial + ((size_t)split * p.partial_rows + vrow) * p.partial_ld + n_blk * BN + c);
+                        if (part_valid) {
+                            float4 *dst = reinterpret_cast<float4 *>(part_row + c);
 #pragma unroll
                             for (int j = 0; j < CH / 4; ++j)
                                 dst[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
                         }
                         continue;
                     }
-                    if (p.bias) {
+                    if (bias) {
                         const float4 *b4 = reinterpret_cast<const float4 *>(&ctl->bias_s[buf][c]);
 #pragma unroll
                         for (int j = 0; j < CH / 4; ++j) {
@@ -729,7 +852,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     if (use_res) {
 #pragma unroll
                         for (int q = 0; q < CH / 2; ++q) {
-                            float2 r = pf_unpack2(rh[q], TWO ? (int)PF_SPLIT : p.fmt);
+                            float2 r = pf_unpack2(rh[q], TWO ? (int)PF_SPLIT : fmt);
                             f[2 * q] += r.x;
                             f[2 * q + 1] += r.y;
                         }
@@ -741,18 +864,18 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                             }
                         }
                     }
-                    apply_act_n(f, p.relu);
-                    if (p.out_f32) {
+                    apply_act_n(f, relu);
+                    if (out_f32) {
                         const int col0 = n_blk * BN + c;
                         if (valid) {
 #pragma unroll
                             for (int j = 0; j < CH; ++j)
-                                if (col0 + j < p.cout_valid) p.out_f32[out_off + col0 + j] = f[j];
+                                if (c + j < col_lim) out_f32[out_off + col0 + j] = f[j];
                         }
                         continue;
                     }
                     uint32_t hi[CH / 2];
-                    if (TWO || p.fmt != PF_F16) {
+                    if (TWO || fmt != PF_F16) {
 #pragma unroll
                         for (int q = 0; q < CH / 2; ++q) hi[q] = pack_bf16(f[2 * q], f[2 * q + 1]);
                     } else {
@@ -766,13 +889,13 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     // The output may be a channel slice: nothing is stored past cout_valid.
 #pragma unroll
                     for (int q = 0; q < CH / 16; ++q)
-                        if (valid && c + 16 * q < col_lim) st_global_v8(p.out_hi + out_off + c + 16 * q, hi + 8 * q);
+                        if (valid && c + 16 * q < col_lim) st_global_v8(out_hi + out_off + c + 16 * q, hi + 8 * q);
                     if constexpr (TWO) {
                         uint32_t lo[8];
 #pragma unroll
                         for (int q = 0; q < 8; ++q)
                             lo[q] = pack_bf16(f[2 * q] - bf16_lo_to_f32(hi[q]), f[2 * q + 1] - bf16_hi_to_f32(hi[q]));
-                        if (valid && c < col_lim) st_global_v8(p.out_lo + out_off + c, lo);
+                        if (valid && c < col_lim) st_global_v8(out_lo + out_off + c, lo);
                     }
 #ifdef GPX_CGEMM_TIMING
                     e_store += clock64() - t_p2;
@@ -781,6 +904,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 ++it;
                 ++tiles_done;
                 seg_k0 = 0;
+                if (in_cluster) break;  // a CTA of such a launch runs one tile
                 tc_fence_before_sync();
                 TCK(t_b0);
                 asm volatile("bar.sync 1, %0;" ::"n"(kCEpiThreads) : "memory");
@@ -828,49 +952,88 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     }
 
     tc_fence_before_sync();
-    __syncthreads();
-    if (p.cluster_reduce) {
-        // Every CTA of the cluster has left its partial tile in shared memory (or has failed and set
-        // the error word: all waits above are bounded, so every thread gets here).  CTA r finishes
-        // rows [r, r+1) * 128/S of the output block: the S partial rows are read through distributed
-        // shared memory and added in split order from zero, exactly as splitk_finish_kernel adds the
-        // workspace rows, then bias, residual, activation and store by the same function.
-        cluster_sync_all();
+    if constexpr (BN != 64) {
+        __syncthreads();
+    } else if (in_cluster) {
+        // Every CTA of the cluster has pushed its partial rows to their owners (or has failed and set
+        // the error word: all waits above are bounded, so every thread gets here).  This CTA finishes
+        // rows [rank, rank+1) * 128/S of the output block from its own shared memory: the S partial
+        // rows are added in split order from zero, exactly as splitk_finish_kernel adds the workspace
+        // rows, then bias, residual, activation, store.  Where the rows go, the bias and the residual
+        // were fetched before the products were waited for.  Nothing is read from a peer, so a CTA may
+        // exit when it is done.
+        // (Pulling the rows from the peers after the barrier, one split at a time, and a second
+        // barrier before the exit made this step 4 us long; BERT-base b1: 7.4 us per projection.)
+#ifdef GPX_CGEMM_TIMING
+        if (threadIdx.x == 64) TADD(18, clock64() - t_begin);
+#endif
+        cluster_arrive();
+#ifdef GPX_CGEMM_TIMING
+        if (threadIdx.x == 64) TADD(19, clock64() - t_begin);
+#endif
+        cluster_wait();
+#ifdef GPX_CGEMM_TIMING
+        if (threadIdx.x == 64) TADD(20, clock64() - t_begin);
+#endif
         if (warp >= 2 && warp < kCPollWarp) {
-            const int S = p.k_splits;
-            const int rank = (int)cluster_ctarank();
-            const int otile = (int)blockIdx.x / S;
-            const int m_blk = otile / p.tiles_n, n_blk = otile - m_blk * p.tiles_n;
-            const int rows_per = kCBM / S;
-            const int img = p.fin.in_hs * p.fin.in_ws;
-            const uint32_t stage = smem_base;
-            for (int e = (int)threadIdx.x - 64; e < rows_per * (BN / 8); e += kCEpiThreads) {
-                const int lr = e / (BN / 8), c8 = e - lr * (BN / 8);
-                const int trow = rank * rows_per + lr;
-                const int vrow = m_blk * kCBM + trow;
-                const int col0 = n_blk * BN + c8 * 8;
-                if (vrow >= p.fin.m_rows || col0 >= p.fin.cout_padded) continue;
-                const int n_img = vrow / img;
-                const int r = vrow - n_img * img;
-                const int hs = r / p.fin.in_ws;
-                const int h = hs - p.fin.in_off;
-                const int w = r - hs * p.fin.in_ws - p.fin.in_off;
-                if (h < 0 || h >= p.fin.out.H || w < 0 || w >= p.fin.out.W) continue;
-                float f[8];
+            const float *land = reinterpret_cast<const float *>(smem + nst * Cfg::kStageBytes);
+            const SplitKParams &fin = p.fin;
+            auto finish = [&](auto splits) {
+                constexpr int S = decltype(splits)::value, rows_per = kCBM / S;
+                constexpr int kItems = rows_per * kGroups;  // eight-channel items of this CTA
 #pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = 0.f;
-                const uint32_t local = stage + (uint32_t)(((size_t)trow * (BN + 4) + c8 * 8) * sizeof(float));
-                for (int sidx = 0; sidx < S; ++sidx) {
-                    const uint32_t remote = cluster_map_shared(local, (uint32_t)sidx);
-                    const float4 a = ld_shared_cluster_f4(remote), b = ld_shared_cluster_f4(remote + 16);
-                    f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
-                    f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
+                for (int i = 0; i < (kItems + kCEpiThreads - 1) / kCEpiThreads; ++i) {
+                    if (!fin_live[i]) continue;
+                    const int e = (int)threadIdx.x - 64 + i * kCEpiThreads;
+                    const int lr = e / kGroups, c8 = (e - lr * kGroups) * 8;
+                    float4 q[2 * S];
+#pragma unroll
+                    for (int sidx = 0; sidx < S; ++sidx) {
+                        const float4 *src = reinterpret_cast<const float4 *>(land + (sidx * rows_per + lr) * (BN + 4) + c8);
+                        q[2 * sidx] = src[0];
+                        q[2 * sidx + 1] = src[1];
+                    }
+                    float f[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) f[j] = 0.f;
+#pragma unroll
+                    for (int sidx = 0; sidx < S; ++sidx) {
+                        const float4 a = q[2 * sidx], b = q[2 * sidx + 1];
+                        f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
+                        f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
+                    }
+                    if (fin.bias)
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) f[j] += fin_bias[i][j];
+                    if (fin.res_hi) {
+                        float r[8];
+                        planes_decode8(fin_rhi[i], fin_rlo[i], fin.res.fmt, r);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) f[j] += r[j];
+                    }
+                    apply_act_n(f, fin.relu);
+                    if (fin.out_f32) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (fin_col[i] + j < fin.cout_valid) fin.out_f32[fin_off[i] + j] = f[j];
+                    } else {
+                        planes_store8(fin.out_hi, fin.out_lo, fin_off[i], fin.out.fmt, f);
+                    }
                 }
-                splitk_apply(p.fin, n_img, h, w, col0, f);
-            }
+            };
+            if (p.k_splits == 8)
+                finish(std::integral_constant<int, 8>());
+            else if (p.k_splits == 4)
+                finish(std::integral_constant<int, 4>());
+            else
+                finish(std::integral_constant<int, 2>());
         }
-        // no CTA may exit (and release its shared memory) while a peer still reads it
-        cluster_sync_all();
+#ifdef GPX_CGEMM_TIMING
+        if (threadIdx.x == 64) TADD(21, clock64() - t_begin);
+#endif
+        __syncthreads();  // (tensor memory is released below by warp 1)
+    } else {
+        __syncthreads();
     }
     if (warp == 0 && lane == 0 && *abort_flag) {
         for (int spin = 0; spin < 64; ++spin) __nanosleep(1000);

@@ -63,7 +63,7 @@ struct CgemmParams {
     int tiles_m, tiles_n;
     // Reciprocals of the divisors the epilogue decodes a tile and a row with (fast_div), and whether
     // GEMM row m is output row m (plain rows on both sides: no decode at all).
-    float inv_k_splits, inv_tiles_n, inv_img, inv_in_ws;
+    float inv_k_splits, inv_tiles_n, inv_img, inv_in_ws, inv_cin_blocks;
     int identity_rows;
     int relu;
     const float *bias;       // [Cout] or null
@@ -86,10 +86,10 @@ struct CgemmParams {
     int kb_per_split;        // K blocks per split (the last split may be shorter)
     float *partial;          // k_splits > 1: fp32 workspace [split][partial_rows][partial_ld]
     int partial_rows, partial_ld;
-    // Cluster reduction (non-preemptible launches only): the k_splits CTAs of one output block form
-    // a thread-block cluster, leave their partial tiles in shared memory and each finishes a share
-    // of the rows, reading its peers' tiles through distributed shared memory in split order - the
-    // additions of splitk_finish_kernel without the workspace round trip and the second launch.
+    // Cluster reduction (non-preemptible launches only, 64-column tiles): the k_splits CTAs of one
+    // output block form a thread-block cluster, each finishes a share of the rows, and every CTA writes
+    // its partial rows into their owners' shared memory - the additions of splitk_finish_kernel
+    // without the workspace round trip and the second launch.
     int cluster_reduce;
     SplitKParams fin;        // what the finishing pass needs (bias, residual, activation, output)
     CgemmSlot *slots;        // one per CTA of this kernel
@@ -148,8 +148,8 @@ struct PoolParams {
 // split order, then bias, residual and ReLU, and stores the result like the one-pass epilogue.
 #if defined(__CUDACC__)
 // Tail of the finishing pass for eight channels (col0 .. col0+7) of output pixel (n_img, h, w):
-// f holds the sum of the splits.  One definition for both places that finish a split-K tile, so
-// they produce the same bits.
+// f holds the sum of the splits.  The cluster reduction inside the convolution kernel does the same
+// steps in the same order (with bias and residual fetched ahead), so both produce the same bits.
 __device__ __forceinline__ void splitk_apply(const SplitKParams &p, int n_img, int h, int w, int col0, float (&f)[8]) {
     if (p.bias) {
 #pragma unroll
@@ -235,8 +235,10 @@ struct LayerNormParams {
     int rows, H, S;
     int fmt;                                // PlaneFmt of the input and output planes
     float eps;
+    int rows_per_tile;                      // 8 or 16
     int total_tiles;
 };
+int layernorm_rows_per_tile(int rows, int sm_count);
 cudaError_t layernorm_launch(const LayerNormParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
 
 // Multi-head self-attention over [B*S][ld] matrices of queries, keys and values (head h owns

@@ -777,9 +777,10 @@ int finalize_model(gpx_model &m) {
             q.H = n.C;
             q.S = n.W;
             q.eps = 1e-12f;
-            q.total_tiles = (q.rows + 7) / 8;
+            q.rows_per_tile = layernorm_rows_per_tile(q.rows, m.sm_count);
+            q.total_tiles = (q.rows + q.rows_per_tile - 1) / q.rows_per_tile;
             kn.total_tiles = q.total_tiles;
-            kn.grid = (int)std::min<long long>((long long)m.sm_count * 8, q.total_tiles);
+            kn.grid = (int)std::min<long long>((long long)m.sm_count * (q.H <= 768 ? 3 : 2), q.total_tiles);
             kn.flops = 8.0 * q.rows * q.H;
             kn.bytes = 8.0 * q.rows * q.H;
             m.kernels.push_back(kn);
@@ -1138,17 +1139,23 @@ int finalize_model(gpx_model &m) {
         const int out_tiles = p.tiles_m * p.tiles_n;
         p.k_splits = 1;
         p.kb_per_split = all_kb;
-        // (GPX_SPLITK_MIN_KB: fewest K blocks per split, default 4; GPX_SPLITK_ALLKB: shortest K loop
-        // that is split at all, default 8 - tuning knobs for the batch-1 latency.)
+        // (GPX_SPLITK_MIN_KB: fewest K blocks per split, default 3; GPX_SPLITK_ALLKB: shortest K loop
+        // that is split at all, default 8 - tuning knobs for the batch-1 latency.  Three blocks instead
+        // of four: BERT-base b1 673 -> 624 us, DistilBERT b1 361 -> 335 us, ResNet-50 b1 unchanged; with
+        // two, ResNet-50 b1 loses 3 %.)
         const char *e_min = getenv("GPX_SPLITK_MIN_KB"), *e_all = getenv("GPX_SPLITK_ALLKB");
-        const int min_kb = e_min ? std::max(1, atoi(e_min)) : 4;
+        const int min_kb = e_min ? std::max(1, atoi(e_min)) : 3;
         const int split_from = e_all ? atoi(e_all) : 8;
         if (out_tiles * 2 <= m.sm_count && all_kb >= split_from) {
             int s_want = std::min(all_kb / min_kb, m.sm_count / out_tiles);
             // Powers of two up to eight: the splits of an output block can then form a thread-block
-            // cluster and reduce through distributed shared memory (non-preemptible launches).
+            // cluster and reduce through distributed shared memory (non-preemptible launches), if that
+            // many clusters are resident at once.
             const char *e_cl = getenv("GPX_SPLITK_CLUSTER");
-            if (!(e_cl && e_cl[0] == '0')) s_want = s_want >= 8 ? 8 : (s_want >= 4 ? 4 : (s_want >= 2 ? 2 : 1));
+            if (!(e_cl && e_cl[0] == '0')) {
+                s_want = s_want >= 8 ? 8 : (s_want >= 4 ? 4 : (s_want >= 2 ? 2 : 1));
+                while (bn == 64 && s_want > 2 && cgemm_max_cluster(bn, m.fmt, s_want) < out_tiles * s_want) s_want /= 2;
+            }
             if (s_want >= 2) {
                 p.kb_per_split = (all_kb + s_want - 1) / s_want;
                 p.k_splits = (all_kb + p.kb_per_split - 1) / p.kb_per_split;
@@ -1172,6 +1179,7 @@ int finalize_model(gpx_model &m) {
         p.inv_tiles_n = 1.0f / (float)p.tiles_n;
         p.inv_img = 1.0f / (float)(p.in_hs * p.in_ws);
         p.inv_in_ws = 1.0f / (float)p.in_ws;
+        p.inv_cin_blocks = 1.0f / (float)p.cin_blocks;
         // (the float quotient of fast_div is exact to within one below 2^24)
         GPX_REQUIRE((long long)p.tiles_m * 128 < (1 << 24) && (long long)out_tiles * p.k_splits < (1 << 24), GPX_OUT_OF_RANGE,
                     "%s: %d rows exceed what the tensor-core kernel indexes", n.name.c_str(), p.m_rows);
@@ -1234,7 +1242,7 @@ int finalize_model(gpx_model &m) {
             // number of splits that divides the tile's rows, and every cluster resident at once.
             const char *e_cl = getenv("GPX_SPLITK_CLUSTER");
             const bool pow2 = p.k_splits == 2 || p.k_splits == 4 || p.k_splits == 8;
-            if (pow2 && bn <= 128 && !(e_cl && e_cl[0] == '0') && cgemm_max_cluster(bn, m.fmt, p.k_splits) >= kn.total_tiles &&
+            if (pow2 && bn == 64 && !(e_cl && e_cl[0] == '0') && cgemm_max_cluster(bn, m.fmt, p.k_splits) >= kn.total_tiles &&
                 kn.grid == kn.total_tiles) {
                 p.cluster_reduce = 1;
                 p.fin = q;

@@ -9,6 +9,8 @@
 // preempted and resumed run is bit-identical to an uninterrupted one.
 #include "layers.cuh"
 
+#include <type_traits>
+
 namespace gpx {
 
 constexpr int kTfThreads = 256;
@@ -19,23 +21,21 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// One warp normalises one row of H <= 1024 channels held in registers (up to four 8-channel
-// vectors per lane): mean, then the variance of the deviations, then scale and shift.
-constexpr int kLnMaxVec = 4;
-
-__device__ __forceinline__ void layer_norm_row(float (&x)[kLnMaxVec][8], int nvec, int H, const float *gamma,
-                                               const float *beta, float eps, int lane) {
+// One warp normalises one row of H <= 1024 channels held in registers (NV 8-channel vectors per
+// lane): mean, then the variance of the deviations, then scale and shift.
+template <int NV>
+__device__ __forceinline__ void layer_norm_row(float (&x)[NV][8], int V, int H, const float *gamma, const float *beta,
+                                               float eps, int lane) {
     float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < kLnMaxVec; ++i)
-        if (i < nvec)
+    for (int i = 0; i < NV; ++i)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) s += x[i][j];
+        for (int j = 0; j < 8; ++j) s += x[i][j];  // lanes past the row hold zeros
     const float mean = warp_sum(s) / (float)H;
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < kLnMaxVec; ++i)
-        if (i < nvec)
+    for (int i = 0; i < NV; ++i)
+        if (lane + 32 * i < V)
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 float d = x[i][j] - mean;
@@ -43,16 +43,25 @@ __device__ __forceinline__ void layer_norm_row(float (&x)[kLnMaxVec][8], int nve
             }
     const float rstd = rsqrtf(warp_sum(ss) / (float)H + eps);
 #pragma unroll
-    for (int i = 0; i < kLnMaxVec; ++i)
-        if (i < nvec) {
-            const int c0 = (lane + 32 * i) * 8;
+    for (int i = 0; i < NV; ++i)
+        if (lane + 32 * i < V) {
+            const float4 *g4 = reinterpret_cast<const float4 *>(gamma) + (lane + 32 * i) * 2;
+            const float4 *b4 = reinterpret_cast<const float4 *>(beta) + (lane + 32 * i) * 2;
+            const float4 g0 = __ldg(g4), g1 = __ldg(g4 + 1), b0 = __ldg(b4), b1 = __ldg(b4 + 1);
+            const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-            for (int j = 0; j < 8; ++j) x[i][j] = (x[i][j] - mean) * rstd * gamma[c0 + j] + beta[c0 + j];
+            for (int j = 0; j < 8; ++j) x[i][j] = (x[i][j] - mean) * rstd * g[j] + b[j];
         }
 }
 
-// Rows of a [rows][H] matrix, one warp per row, eight rows per tile.
-__global__ void __launch_bounds__(kTfThreads)
+// Rows of a [rows][H] matrix, R rows per warp, 8 R rows per tile.  Bound by HBM (the row is read and
+// written once).  The R rows of a warp are requested as raw vectors before any is converted, and
+// the next tile is claimed while they are on their way, so that neither the claim (two dependent
+// round trips to L2) nor the first load of a tile is waited for with nothing in flight; gamma and
+// beta come as 128-bit loads (one float at a time they were 48 of a lane's 54 load instructions).
+template <int NV, int R, bool TWO>
+__global__ void __launch_bounds__(kTfThreads, NV <= 3 ? 3 : 2)
 layernorm_kernel(const __grid_constant__ LayerNormParams p, BlpArgs blp) {
     pdl_enter();
     __shared__ int s_tile;
@@ -61,58 +70,67 @@ layernorm_kernel(const __grid_constant__ LayerNormParams p, BlpArgs blp) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int V = p.H / 8;
     int iter = 0;
-    for (;;) {
-        int tile;
-        if (dynamic) {
-            if (threadIdx.x == 0) s_tile = blp_claim(blp, iter);
-            __syncthreads();
-            tile = s_tile;
-        } else {
-            tile = blp_claim(blp, iter);
-        }
-        if (tile < 0) break;
-        const int row = tile * (kTfThreads / 32) + wid;
-        if (row < p.rows) {
-            float x[kLnMaxVec][8];
-            int nvec = 0;
+    int tile;
+    if (dynamic) {
+        if (threadIdx.x == 0) s_tile = blp_claim(blp, 0);
+        __syncthreads();
+        tile = s_tile;
+    } else {
+        tile = blp_claim(blp, 0);
+    }
+    while (tile >= 0) {
+        const int row0 = (tile * (kTfThreads / 32) + wid) * R;
+        uint4 ra[R][NV], rb[TWO ? R : 1][TWO ? NV : 1];
+        if (!p.ids) {
 #pragma unroll
-            for (int i = 0; i < kLnMaxVec; ++i) {
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int i = 0; i < NV; ++i)
+                    if (row0 + r < p.rows && lane + 32 * i < V)
+                        planes_fetch8(p.in_hi, p.in_lo, (size_t)(row0 + r) * p.H + (lane + 32 * i) * 8, TWO ? PF_SPLIT : p.fmt,
+                                      ra[r][i], rb[TWO ? r : 0][TWO ? i : 0]);
+        }
+        int next = -1;
+        if (!dynamic || threadIdx.x == 0) next = blp_claim(blp, iter + 1);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int row = row0 + r;
+            if (row >= p.rows) break;
+            float x[NV][8];
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
                 const int v = lane + 32 * i;
-                if (v < V) {
-                    nvec = i + 1;
-                    if (p.ids) {
-                        // embedding row: word + position (+ token type 0 where the model has that table)
-                        const long long id = p.ids[row];
-                        const int pos = row % p.S;
-                        const float4 *w = reinterpret_cast<const float4 *>(p.word + (size_t)id * p.H + v * 8);
-                        const float4 *q = reinterpret_cast<const float4 *>(p.pos + (size_t)pos * p.H + v * 8);
-                        float4 a0 = w[0], a1 = w[1], b0 = q[0], b1 = q[1];
-                        float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0;
-                        if (p.type) {
-                            const float4 *t = reinterpret_cast<const float4 *>(p.type + v * 8);
-                            c0 = t[0];
-                            c1 = t[1];
-                        }
-                        x[i][0] = a0.x + b0.x + c0.x;
-                        x[i][1] = a0.y + b0.y + c0.y;
-                        x[i][2] = a0.z + b0.z + c0.z;
-                        x[i][3] = a0.w + b0.w + c0.w;
-                        x[i][4] = a1.x + b1.x + c1.x;
-                        x[i][5] = a1.y + b1.y + c1.y;
-                        x[i][6] = a1.z + b1.z + c1.z;
-                        x[i][7] = a1.w + b1.w + c1.w;
-                    } else {
-                        const size_t off = (size_t)row * p.H + v * 8;
-                        planes_load8(p.in_hi, p.in_lo, off, p.fmt, x[i]);
-                    }
-                } else {
+                if (v >= V) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j) x[i][j] = 0.f;
+                } else if (p.ids) {
+                    // embedding row: word + position (+ token type 0 where the model has that table)
+                    const long long id = p.ids[row];
+                    const int pos = row % p.S;
+                    const float4 *w = reinterpret_cast<const float4 *>(p.word + (size_t)id * p.H + v * 8);
+                    const float4 *q = reinterpret_cast<const float4 *>(p.pos + (size_t)pos * p.H + v * 8);
+                    float4 a0 = w[0], a1 = w[1], b0 = q[0], b1 = q[1];
+                    float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0;
+                    if (p.type) {
+                        const float4 *t = reinterpret_cast<const float4 *>(p.type + v * 8);
+                        c0 = t[0];
+                        c1 = t[1];
+                    }
+                    x[i][0] = a0.x + b0.x + c0.x;
+                    x[i][1] = a0.y + b0.y + c0.y;
+                    x[i][2] = a0.z + b0.z + c0.z;
+                    x[i][3] = a0.w + b0.w + c0.w;
+                    x[i][4] = a1.x + b1.x + c1.x;
+                    x[i][5] = a1.y + b1.y + c1.y;
+                    x[i][6] = a1.z + b1.z + c1.z;
+                    x[i][7] = a1.w + b1.w + c1.w;
+                } else {
+                    planes_decode8(ra[r][i], rb[TWO ? r : 0][TWO ? i : 0], TWO ? PF_SPLIT : p.fmt, x[i]);
                 }
             }
-            layer_norm_row(x, nvec, p.H, p.gamma, p.beta, p.eps, lane);
+            layer_norm_row<NV>(x, V, p.H, p.gamma, p.beta, p.eps, lane);
 #pragma unroll
-            for (int i = 0; i < kLnMaxVec; ++i) {
+            for (int i = 0; i < NV; ++i) {
                 const int v = lane + 32 * i;
                 if (v < V) {
                     const size_t off = (size_t)row * p.H + v * 8;
@@ -121,19 +139,46 @@ layernorm_kernel(const __grid_constant__ LayerNormParams p, BlpArgs blp) {
                         o[0] = make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
                         o[1] = make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
                     } else {
-                        planes_store8(p.out_hi, p.out_lo, off, p.fmt, x[i]);
+                        planes_store8(p.out_hi, p.out_lo, off, TWO ? PF_SPLIT : p.fmt, x[i]);
                     }
                 }
             }
         }
         ++iter;
-        if (dynamic) __syncthreads();
+        if (dynamic) {
+            __syncthreads();  // everyone has read the tile number of this round
+            if (threadIdx.x == 0) s_tile = next;
+            __syncthreads();
+            tile = s_tile;
+        } else {
+            tile = next;
+        }
     }
     if (threadIdx.x == 0) trace_end(blp, iter);
 }
 
+int layernorm_rows_per_tile(int rows, int sm_count) {
+    // Two rows a warp once that still leaves every SM a few tiles (16 384 rows of 768: 37 us with one).
+    return rows >= 16 * 4 * sm_count ? 16 : 8;
+}
+
 cudaError_t layernorm_launch(const LayerNormParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(layernorm_kernel, grid, kTfThreads, 0, s, p, blp);
+    const int nv = p.H <= 256 ? 1 : (p.H <= 768 ? 3 : 4);
+    const bool pair = p.rows_per_tile == 16;
+    auto go = [&](auto kernel) { launch_layer(kernel, grid, kTfThreads, 0, s, p, blp); };
+    auto pick = [&](auto two) {
+        constexpr bool T = decltype(two)::value;
+        if (nv == 1)
+            go(pair ? layernorm_kernel<1, 2, T> : layernorm_kernel<1, 1, T>);
+        else if (nv == 3)
+            go(pair ? layernorm_kernel<3, 2, T> : layernorm_kernel<3, 1, T>);
+        else
+            go(pair ? layernorm_kernel<4, 2, T> : layernorm_kernel<4, 1, T>);
+    };
+    if (p.fmt == PF_SPLIT)
+        pick(std::true_type());
+    else
+        pick(std::false_type());
     return cudaGetLastError();
 }
 
