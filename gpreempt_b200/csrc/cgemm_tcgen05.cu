@@ -42,6 +42,9 @@ constexpr int kCEpiParts = 2;                       // epilogue warps per TMEM l
 constexpr int kCEpiThreads = 128 * kCEpiParts;
 constexpr int kCPollWarp = 2 + kCEpiThreads / 32;
 constexpr int kCgemmThreads = 64 + kCEpiThreads + 32;
+constexpr int kCAffThreads = 256;  // eight more warps where the A operand goes through an affine map first
+constexpr int kCAffGroups = 2;       // groups of those warps that take K blocks in turn
+constexpr int kCAffMaxC = kCgemmMaxAffineC;
 constexpr unsigned long long kCWaitLimitNs = 2000000000ull;
 
 // fp32 spill area of one CTA: one accumulator buffer (at most 256 columns) of 128 rows.
@@ -53,8 +56,9 @@ struct CgemmControlSize {
 
 // BN: columns of an output tile.  TWO: two-plane operands (float32 models), three products per K step;
 // otherwise one 16-bit plane and one product.
-template <int BN, bool TWO>
+template <int BN, bool TWO, bool AFF>
 struct CgemmCfg {
+    static constexpr int kThreads = kCgemmThreads + (AFF ? kCAffThreads : 0);
     static constexpr uint32_t kPlanes = TWO ? 2 : 1;
     static constexpr uint32_t kABytes = kCBM * kCBK * 2;        // one plane of A: 16 KiB
     static constexpr uint32_t kWBytes = BN * kCBK * 2;          // one plane of W
@@ -62,20 +66,23 @@ struct CgemmCfg {
     static constexpr uint32_t kWOff = kPlanes * kABytes;        // W (hi) tile inside a K block
     // K blocks a ring stage holds at most.  The round of one stage (barrier waits, message, commit) costs
     // either role ~300 cycles; a 64- or 128-column product of one plane takes 128 or 256, so two
-    // of them share a round (VGG-16's 64-column layer at batch 16: 168 -> see the table of cases).
-    static constexpr int kKps = (!TWO && BN <= 128) ? 2 : 1;
+    // of them share a round, unless the affine map sets the pace (VGG-16's 64-column layer at batch 16: 168 -> see the table of cases).
+    static constexpr int kKps = (!TWO && !AFF && BN <= 128) ? 2 : 1;
     static constexpr uint32_t kStageBytes = kKps * kKbBytes;
-    static constexpr int kStages = (int)((192u * 1024u) / kStageBytes);  // 3 or 4
+    static constexpr int kStages = (int)((192u * 1024u) / kStageBytes);  // 3 to 8
+    // ring stages the landing area of a cluster reduction takes (128 rows of BN + 4 floats)
+    static constexpr int kLandStages = (int)((kCBM * (BN + 4) * 4 + kStageBytes - 1) / kStageBytes);
     // ring + alignment slack + 64x64 identity tile + control block
     static constexpr uint32_t kIdentBytes = 64 * kCBK * 2;
     static constexpr size_t kSmem =
-        (size_t)kStages * kStageBytes + 1024 + kIdentBytes + sizeof(CgemmControlSize);
+        (size_t)kStages * kStageBytes + 1024 + kIdentBytes + sizeof(CgemmControlSize) + (AFF ? 2 * kCAffMaxC * sizeof(float) : 0);
     // Accumulator columns of one tile: hi*hi and both cross terms for two-plane operands, one sum
     // otherwise; two tiles' worth of them in tensor memory, so that the epilogue of one tile overlaps
     // the K loop of the next.
     static constexpr int kBufCols = (int)kPlanes * BN;
     static constexpr int kTmemCols = 2 * kBufCols;
     static_assert(kTmemCols <= 512 && kStages <= 8, "tile does not fit");
+    static_assert(BN != 64 || kStages - kLandStages >= 3, "no ring left beside the landing area");
 };
 
 // Message of a ring stage: CMSG_DATA + number of K blocks, CMSG_RES + index of the residual block, or
@@ -86,6 +93,7 @@ enum : int { CEPI_COMPLETE = 0, CEPI_PARTIAL = 1 };
 struct CgemmControl {
     unsigned long long full[8];
     unsigned long long empty[8];
+    unsigned long long ready[8];       // the A tile of a stage has been through its affine map
     unsigned long long tmem_full[2];   // one per accumulator buffer
     unsigned long long tmem_empty[2];
     uint32_t tmem_base;
@@ -149,10 +157,10 @@ __device__ unsigned long long g_cgemm_timing[32];
 #define TADD(slot, val)
 #endif
 
-template <int BN, bool TWO>
-__global__ void __launch_bounds__(kCgemmThreads, 1)
+template <int BN, bool TWO, bool AFF>
+__global__ void __launch_bounds__(CgemmCfg<BN, TWO, AFF>::kThreads, 1)
 cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
-    using Cfg = CgemmCfg<BN, TWO>;
+    using Cfg = CgemmCfg<BN, TWO, AFF>;
     constexpr int kStages = Cfg::kStages;
     constexpr int kBufCols = Cfg::kBufCols;
     TCK(t_start);
@@ -190,9 +198,9 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         return t;
     };
     const bool resumable = blp.preempted != nullptr;
-    // Split K inside a cluster: the last ring stage is where the peers' partial sums land.
+    // Split K inside a cluster: the peers' partial sums land in the last ring stages.
     const bool in_cluster = BN == 64 && p.cluster_reduce;
-    const int nst = in_cluster ? kStages - 1 : kStages;
+    const int nst = in_cluster ? kStages - Cfg::kLandStages : kStages;
 
     CgemmSlot *slot = p.slots + blockIdx.x;
     float *spill = p.spill + (size_t)blockIdx.x * cgemm_spill_floats();
@@ -201,6 +209,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(smem_u32(&ctl->full[s]), 1);
             mbar_init(smem_u32(&ctl->empty[s]), 1);
+            if (AFF) mbar_init(smem_u32(&ctl->ready[s]), kCAffThreads / 32 / kCAffGroups);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&ctl->tmem_full[b]), 2);
@@ -222,6 +231,13 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             prefetch_tensormap(&p.w_lo);
         }
     }
+    // scale and shift of every input channel (parameters: no kernel writes them), zero past the last
+    float *aff_s = reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(ctl) + sizeof(CgemmControlSize));
+    if (AFF)
+        for (int c = threadIdx.x; c < p.cin_blocks * kCBK; c += Cfg::kThreads) {
+            aff_s[c] = c < p.aff_c ? __ldg(p.aff_scale + c) : 0.f;
+            aff_s[kCAffMaxC + c] = c < p.aff_c ? __ldg(p.aff_shift + c) : 0.f;
+        }
     if (warp == 1) tmem_alloc(smem_u32(&ctl->tmem_base), Cfg::kTmemCols);
     tc_fence_before_sync();
     __syncthreads();
@@ -408,6 +424,20 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                         mbar_arrive(bar);
                         if (blp.trace) atomicMin(blp.trace + 2, globaltimer_ns());
                     }
+                    if (AFF) {
+                        // each group of the affine map looks at its own stages only: one message for each
+                        for (int g = 1; g < kCAffGroups; ++g) {
+                            if (++stage == nst) {
+                                stage = 0;
+                                phase ^= 1;
+                            }
+                            if (!mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1, abort_flag, kCWaitLimitNs)) break;
+                            if (issuer) {
+                                ctl->stage_msg[stage] = CMSG_STOP;
+                                mbar_arrive(smem_u32(&ctl->full[stage]));
+                            }
+                        }
+                    }
                     ok = false;
                     break;
                 }
@@ -521,6 +551,14 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     break;
                 }
                 const int n = msg >= CMSG_RES ? 1 : msg - CMSG_DATA;  // K blocks in this stage
+                if (AFF) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->ready[stage]), phase, abort_flag, kCWaitLimitNs))) {
+                        if (lane == 0) fail(203);
+                        end = -1;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                }
                 // descriptor addresses are in 16-byte units
                 const uint64_t a0 = ring + (uint64_t)(stage * (Cfg::kStageBytes >> 4));
                 if (issuer) {
@@ -603,6 +641,91 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     break;
                 }
                 __nanosleep(100);
+            }
+        }
+        __syncwarp();
+    } else if (AFF && warp > kCPollWarp) {
+        // ------------------------------------------------------------------ affine map of A
+        // Every thread keeps one of the eight 16-byte pieces of a row (piece c of row r lies at position
+        // c XOR (r mod 8), the 128-byte swizzle) and takes eight rows 16 apart: its sixteen scales and
+        // shifts are read once per K block, and eight neighbouring threads touch one whole row, so no
+        // two of a quarter warp meet in a bank.  ~130 instructions a thread and K block; the normalised
+        // copy of the input that a kernel of its own wrote and this one read back (DenseNet-201 b64
+        // bf16: 40 % of the forward) is gone.  (One thread per row, re-reading the scales for every
+        // piece, took ~1500 cycles a K block on four warps.)
+        // Two groups of four warps take the K blocks in turn: a block is a chain of latencies (shared-memory
+        // reads, conversions, the fence to the tensor core's proxy) that the other group's overlaps.
+        constexpr int kGroupThreads = kCAffThreads / kCAffGroups;
+        const int group = (warp - kCPollWarp - 1) / (kGroupThreads / 32);
+        const int at = ((int)threadIdx.x - (kCPollWarp + 1) * 32) % kGroupThreads;
+        const int piece = at & 7, row = at >> 3;
+        constexpr int kAffRows = kCBM * 8 / kGroupThreads;  // rows per thread
+        const uint32_t off = (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4));  // (rows 16 apart: same swizzle)
+        const bool half_fmt = !TWO && p.fmt == PF_F16;
+        auto map_block = [&](unsigned char *a, int ch, auto half) {
+            const float4 *sc = reinterpret_cast<const float4 *>(aff_s + ch);
+            const float4 *sh = reinterpret_cast<const float4 *>(aff_s + kCAffMaxC + ch);
+            const float4 s0 = sc[0], s1 = sc[1], b0 = sh[0], b1 = sh[1];
+            const float2 ss[4] = {{s0.x, s0.y}, {s0.z, s0.w}, {s1.x, s1.y}, {s1.z, s1.w}};
+            const float2 bb[4] = {{b0.x, b0.y}, {b0.z, b0.w}, {b1.x, b1.y}, {b1.z, b1.w}};
+            uint4 hv[kAffRows], lv[TWO ? kAffRows : 1];
+#pragma unroll
+            for (int r = 0; r < kAffRows; ++r) {
+                hv[r] = *reinterpret_cast<const uint4 *>(a + r * 2048);
+                if (TWO) lv[TWO ? r : 0] = *reinterpret_cast<const uint4 *>(a + Cfg::kABytes + r * 2048);
+            }
+#pragma unroll
+            for (int r = 0; r < kAffRows; ++r) {
+                uint32_t h[4] = {hv[r].x, hv[r].y, hv[r].z, hv[r].w}, l[4];
+                if (TWO) {
+                    const uint4 q = lv[TWO ? r : 0];
+                    l[0] = q.x, l[1] = q.y, l[2] = q.z, l[3] = q.w;
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    float2 x = half ? pf_unpack2(h[q], PF_F16) : make_float2(bf16_lo_to_f32(h[q]), bf16_hi_to_f32(h[q]));
+                    if (TWO) x = make_float2(x.x + bf16_lo_to_f32(l[q]), x.y + bf16_hi_to_f32(l[q]));
+                    x = fma2(x, ss[q], bb[q]);
+                    x = make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f));
+                    h[q] = half ? pf_pack2(x.x, x.y, PF_F16) : pack_bf16(x.x, x.y);
+                    if (TWO) l[q] = pack_bf16(x.x - bf16_lo_to_f32(h[q]), x.y - bf16_hi_to_f32(h[q]));
+                }
+                *reinterpret_cast<uint4 *>(a + r * 2048) = make_uint4(h[0], h[1], h[2], h[3]);
+                if (TWO) *reinterpret_cast<uint4 *>(a + Cfg::kABytes + r * 2048) = make_uint4(l[0], l[1], l[2], l[3]);
+            }
+        };
+        static_assert(Cfg::kKps == 1 || !AFF, "one K block per stage");
+        int stage = 0, kb = first_k, turn = 0;
+        uint32_t phase = 0;
+        bool go = true;
+        for (int tile = blockIdx.x + first_iter * gridDim.x; go && tile < total_tiles; tile += gridDim.x, kb = 0) {
+            const TileAt t = tile_at(tile);
+            for (; kb < t.main_kb; ++kb) {
+                if (turn == group) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->full[stage]), phase, abort_flag, kCWaitLimitNs))) {
+                        if (lane == 0) fail(501);
+                        go = false;
+                        break;
+                    }
+                    if (__any_sync(0xffffffffu, ctl->stage_msg[stage] == CMSG_STOP)) {
+                        go = false;
+                        break;
+                    }
+                    unsigned char *a = smem + stage * Cfg::kStageBytes + off;
+                    const int ch = (t.kb_base + kb) * kCBK + piece * 8;
+                    if (half_fmt)
+                        map_block(a, ch, std::true_type());
+                    else
+                        map_block(a, ch, std::false_type());
+                    fence_proxy_async();  // ordinary stores, read by the tensor core
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&ctl->ready[stage]));
+                }
+                turn = turn + 1 == kCAffGroups ? 0 : turn + 1;
+                if (++stage == nst) {
+                    stage = 0;
+                    phase ^= 1;
+                }
             }
         }
         __syncwarp();
@@ -787,7 +910,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 // Every lane owns one row of the tile (its TMEM lane): 16 columns of a plane are 32
                 // contiguous bytes of that row, one 256-bit access, a whole sector.
                 const bool use_res = !partial && !out_f32 && res_hi && valid;
-                constexpr int CH = TWO ? 16 : 32;  // columns per piece
+                constexpr int CH = (TWO || AFF) ? 16 : 32;  // columns per piece
 #pragma unroll 1
                 for (int c = c_lo; c < c_hi; c += CH) {
                     float f[CH];
@@ -807,11 +930,14 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j) f[j] = __uint_as_float(t16[j]) + __uint_as_float(u16[j]);
                     } else {
-                        uint32_t t32[32];
-                        tmem_ld_32x32(t_acc + c, t32);
+                        uint32_t t32[CH];
+                        if constexpr (CH == 32)
+                            tmem_ld_32x32(t_acc + c, t32);
+                        else
+                            tmem_ld_32x16(t_acc + c, t32);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(t32[j]);
+                        for (int j = 0; j < CH; ++j) f[j] = __uint_as_float(t32[j]);
                     }
 #ifdef GPX_CGEMM_TIMING
                     long long t_p1 = clock64();
@@ -820,7 +946,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     if (in_cluster) {
                         // Split K inside a cluster: the raw fp32 sum of this row and K range goes
                         // straight into the shared memory of the CTA that finishes the row (its last
-                        // ring stage: [split][row of its share][BN + 4 floats], the 4 spreading the
+                        // ring stages: [split][row of its share][BN + 4 floats], the 4 spreading the
                         // rows of a warp over the banks).
 #pragma unroll
                         for (int j = 0; j < CH / 4; ++j)
@@ -1064,49 +1190,55 @@ extern "C" int gpx_debug_cgemm_timing(unsigned long long *out, int reset) {
 }
 #endif
 
-// Calls f(std::integral_constant<int, BN>, std::bool_constant<TWO>) for the kernel instance of a tile
-// width and operand format.  (256-column tiles exist for single-plane operands only: two planes' two
-// accumulators in two buffers would not fit tensor memory.)
+// Calls f with the kernel instance of a tile width, operand format and A treatment (as a struct of
+// constants).  256-column tiles exist for single-plane operands used as they are: two planes' two
+// accumulators in two buffers would not fit tensor memory, and no layer behind an affine map is wide.
+template <int BN, bool TWO, bool AFF>
+struct CgemmInstance {
+    using Cfg = CgemmCfg<BN, TWO, AFF>;
+    static constexpr auto kernel() { return cgemm_tcgen05_kernel<BN, TWO, AFF>; }
+};
 template <typename F>
-static auto cgemm_instance(int bn, bool two, F &&f) {
-    if (two)
-        return bn == 128 ? f(std::integral_constant<int, 128>(), std::true_type()) : f(std::integral_constant<int, 64>(), std::true_type());
-    if (bn == 256) return f(std::integral_constant<int, 256>(), std::false_type());
-    return bn == 128 ? f(std::integral_constant<int, 128>(), std::false_type()) : f(std::integral_constant<int, 64>(), std::false_type());
+static auto cgemm_instance(int bn, bool two, bool aff, F &&f) {
+    if (two && aff) return bn == 128 ? f(CgemmInstance<128, true, true>()) : f(CgemmInstance<64, true, true>());
+    if (two) return bn == 128 ? f(CgemmInstance<128, true, false>()) : f(CgemmInstance<64, true, false>());
+    if (aff) return bn == 128 ? f(CgemmInstance<128, false, true>()) : f(CgemmInstance<64, false, true>());
+    if (bn == 256) return f(CgemmInstance<256, false, false>());
+    return bn == 128 ? f(CgemmInstance<128, false, false>()) : f(CgemmInstance<64, false, false>());
 }
 
 cudaError_t cgemm_prepare(int device) {
     static bool done[64] = {false};
     if (device < 0 || device >= 64 || done[device]) return cudaSuccess;
     for (int two = 0; two < 2; ++two)
-        for (int bn : {64, 128, 256}) {
-            if (two && bn == 256) continue;
-            cudaError_t e = cgemm_instance(bn, two != 0, [](auto b, auto t) {
-                return cudaFuncSetAttribute(cgemm_tcgen05_kernel<b(), t()>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)CgemmCfg<b(), t()>::kSmem);
-            });
-            if (e != cudaSuccess) return e;
-        }
+        for (int aff = 0; aff < 2; ++aff)
+            for (int bn : {64, 128, 256}) {
+                if (bn == 256 && (two || aff)) continue;
+                cudaError_t e = cgemm_instance(bn, two != 0, aff != 0, [](auto k) {
+                    return cudaFuncSetAttribute(k.kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decltype(k)::Cfg::kSmem);
+                });
+                if (e != cudaSuccess) return e;
+            }
     done[device] = true;
     return cudaSuccess;
 }
 
 // CTAs of clusters of `cluster` CTAs of this kernel that the device keeps resident at once.
-int cgemm_max_cluster(int bn, int fmt, int cluster) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)cluster);
-    cfg.blockDim = dim3((unsigned)kCgemmThreads);
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)cluster;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+int cgemm_max_cluster(int bn, int fmt, bool aff, int cluster) {
     int clusters = 0;
-    cudaError_t err = cgemm_instance(bn, fmt == PF_SPLIT, [&](auto b, auto t) {
-        cfg.dynamicSmemBytes = CgemmCfg<b(), t()>::kSmem;
-        return cudaOccupancyMaxActiveClusters(&clusters, cgemm_tcgen05_kernel<b(), t()>, &cfg);
+    cudaError_t err = cgemm_instance(bn, fmt == PF_SPLIT, aff, [&](auto k) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)cluster);
+        cfg.blockDim = dim3((unsigned)decltype(k)::Cfg::kThreads);
+        cfg.dynamicSmemBytes = decltype(k)::Cfg::kSmem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)cluster;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cudaOccupancyMaxActiveClusters(&clusters, k.kernel(), &cfg);
     });
     if (err != cudaSuccess) {
         cudaGetLastError();
@@ -1116,11 +1248,11 @@ int cgemm_max_cluster(int bn, int fmt, int cluster) {
 }
 
 cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &blp, cudaStream_t s) {
-    return cgemm_instance(bn, p.fmt == PF_SPLIT, [&](auto b, auto t) {
+    return cgemm_instance(bn, p.fmt == PF_SPLIT, p.aff_scale != nullptr, [&](auto k) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)grid);
-        cfg.blockDim = dim3((unsigned)kCgemmThreads);
-        cfg.dynamicSmemBytes = CgemmCfg<b(), t()>::kSmem;
+        cfg.blockDim = dim3((unsigned)decltype(k)::Cfg::kThreads);
+        cfg.dynamicSmemBytes = decltype(k)::Cfg::kSmem;
         cfg.stream = s;
         cudaLaunchAttribute at[2];
         at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1131,11 +1263,11 @@ cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &
         at[1].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = p.cluster_reduce ? 2 : 1;
-        return cudaLaunchKernelEx(&cfg, cgemm_tcgen05_kernel<b(), t()>, p, blp);
+        return cudaLaunchKernelEx(&cfg, k.kernel(), p, blp);
     });
 }
 
-int cgemm_threads() { return kCgemmThreads; }
+int cgemm_threads(bool aff) { return kCgemmThreads + (aff ? kCAffThreads : 0); }
 
 size_t cgemm_spill_floats_per_cta() { return cgemm_spill_floats(); }
 

@@ -420,12 +420,12 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 int make_tmap_2d_bf16(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols,
-                      uint32_t box_rows, uint32_t box_cols) {
+                      uint32_t box_rows, uint32_t box_cols, uint64_t ld = 0) {
     static EncodeTiledFn encode = nullptr;
     if (!encode) encode = reinterpret_cast<EncodeTiledFn>(driver_entry("cuTensorMapEncodeTiled"));
     GPX_REQUIRE(encode, GPX_FAIL, "driver has no cuTensorMapEncodeTiled");
     cuuint64_t dims[2] = {cols, rows};
-    cuuint64_t strides[1] = {cols * 2};
+    cuuint64_t strides[1] = {(ld ? ld : cols) * 2};
     cuuint32_t box[2] = {box_cols, box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult rc = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims,

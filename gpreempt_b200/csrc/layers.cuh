@@ -80,6 +80,11 @@ struct CgemmParams {
     // identity; res_hi/res_lo are then null and the epilogue adds nothing.
     CUtensorMap r_hi, r_lo, ident;
     int res_kb;
+    // Affine + ReLU applied to the A operand between its arrival in shared memory and the products
+    // (a batch norm ahead of a 1x1 convolution): x -> max(x * aff_scale[c] + aff_shift[c], 0) for the
+    // first aff_c channels of the input, zero for the rest.  Null: the operand is used as it is.
+    const float *aff_scale, *aff_shift;
+    int aff_c;
     int drop_on_stop;        // 1: a tile interrupted by the word is recomputed from K block 0 after the
                              // resume instead of being saved (no spill on the way out)
     int k_splits;            // >= 1: the K range is cut into this many tiles per output block
@@ -97,11 +102,12 @@ struct CgemmParams {
     int *error;              // {code, kernel*1000+cta}
 };
 
+constexpr int kCgemmMaxAffineC = 2048;  // input channels of a layer with aff_scale
 cudaError_t cgemm_prepare(int device);
 cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &blp, cudaStream_t s);
-int cgemm_max_cluster(int bn, int fmt, int cluster);  // CTAs of clusters of this size that can be resident at once
+int cgemm_max_cluster(int bn, int fmt, bool aff, int cluster);  // CTAs of clusters of this size that can be resident at once
 size_t cgemm_spill_floats_per_cta();
-int cgemm_threads();
+int cgemm_threads(bool aff);
 
 // ---- CUDA-core convolution / dense (conv_simt.cu) --------------------------------------------
 

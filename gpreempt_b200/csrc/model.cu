@@ -594,6 +594,29 @@ int finalize_model(gpx_model &m) {
         if (n.residual >= 0 && m.storages[m.nodes[n.residual].storage].kind != Storage::ActSplit)
             n.tensor_core = false;
     }
+    // An affine map (batch norm + ReLU) whose only consumer is a 1x1 tensor-core convolution is applied
+    // by that kernel to its operand in shared memory: no kernel and no tensor of its own.
+    for (size_t ai = 0; ai < m.nodes.size(); ++ai) {
+        Node &a = m.nodes[ai];
+        const Node *user = nullptr;
+        int users = 0;
+        for (const Node &n : m.nodes) {
+            for (int in : n.inputs)
+                if (in == (int)ai) {
+                    ++users;
+                    user = &n;
+                }
+        }
+        if (a.op != Op::Affine || users != 1 || a.act != ACT_RELU || m.head_node == (int)ai) continue;
+        const Storage &in = m.storages[m.nodes[a.inputs[0]].storage];
+        if (user->op != Op::Conv || !user->tensor_core || user->via_im2col || user->k != 1 || user->stride != 1 ||
+            user->residual >= 0 || user->inputs[0] != (int)ai || in.kind != Storage::ActSplit || in.parent >= 0 ||
+            order[m.nodes[a.inputs[0]].storage] != ACT_PLAIN || order[a.storage] != ACT_PLAIN || stored_c(m, a) > kCgemmMaxAffineC ||
+            (user->N <= 8 && user->H == 1 && user->W == 1))
+            continue;
+        a.fused_affine = true;
+        m.storages[a.storage].affine_node = (int)ai;
+    }
     // 4. compact copies for stride-2 1x1 convolutions (hidden storages)
     for (size_t ni = 0; ni < m.nodes.size(); ++ni) {
         Node &n = m.nodes[ni];
@@ -648,6 +671,7 @@ int finalize_model(gpx_model &m) {
     for (size_t i = 0; i < m.storages.size(); ++i) {
         Storage &s = m.storages[i];
         if (s.kind == Storage::ActSplit && s.parent >= 0) continue;  // a slice: bound below
+        if (s.affine_node >= 0) continue;                            // formed on the fly
         if (s.kind == Storage::ActSplit) {
             int N = (int)s.dims[0], C = s.cs ? s.cs : (int)s.dims[1];
             int H = s.rank == 4 ? (int)s.dims[2] : 1, W = s.rank == 4 ? (int)s.dims[3] : 1;
@@ -879,6 +903,7 @@ int finalize_model(gpx_model &m) {
             continue;
         }
         if (n.op == Op::Affine) {
+            if (n.fused_affine) continue;
             GPX_REQUIRE(m.storages[src.storage].kind == Storage::ActSplit && n.in_c % 8 == 0, GPX_FAIL,
                         "%s: affine needs a plane activation and a channel count in eights", n.name.c_str());
             add_pool(n.name, view_of(m, src), out, 1, 1, 0, 2, n.in_c, n.scale, n.shift, n.act);
@@ -984,6 +1009,8 @@ int finalize_model(gpx_model &m) {
         }
         // tensor-core convolution
         const Storage *in = &m.storages[src.storage];
+        const bool aff = src.op == Op::Affine && src.fused_affine;
+        if (aff) in = &m.storages[m.nodes[src.inputs[0]].storage];
         int eff_k = n.k, eff_cin = stored_c(m, src);
         if (n.via_im2col) {
             const Storage &pm = m.storages[n.sub_storage];
@@ -1056,7 +1083,7 @@ int finalize_model(gpx_model &m) {
         kn.name = n.name;
         kn.node = (int)ni;
         kn.type = KernelType::Cgemm;
-        kn.threads = cgemm_threads();
+        kn.threads = cgemm_threads(aff);
         CgemmParams &p = kn.cgemm;
         ActLayout il = in->layout;
         if (full_map_dense(n, src) && !n.via_im2col) {
@@ -1079,7 +1106,7 @@ int finalize_model(gpx_model &m) {
             // accumulator buffer they give up (ResNet-50's 1x1 convolutions with K <= 512 lose 6 %,
             // BERT's dense layers and VGG's 3x3 convolutions gain 17-19 %).
             if (m.fmt != PF_SPLIT && !head && cout_st % 256 == 0 && tiles128 / 2 >= m.sm_count &&
-                (long long)eff_k * eff_k * eff_cin >= 768)
+                (long long)eff_k * eff_k * eff_cin >= 768 && !aff)
                 bn = 256;
         }
         kn.tile = bn;
@@ -1128,8 +1155,16 @@ int finalize_model(gpx_model &m) {
         // The epilogue moves 32 bytes per access: 16-channel granularity of rows and slices.
         GPX_REQUIRE(head || (out.layout.C % 16 == 0 && out.ch_off % 16 == 0), GPX_FAIL,
                     "%s: output channels %d (+%d) not in whole 16-channel groups", n.name.c_str(), out.layout.C, out.ch_off);
-        GPX_TRY(make_tmap_2d_bf16(&p.a_hi, in->hi, (uint64_t)il.rows, (uint64_t)eff_cin, 128, 64));
-        if (in->lo) GPX_TRY(make_tmap_2d_bf16(&p.a_lo, in->lo, (uint64_t)il.rows, (uint64_t)eff_cin, 128, 64));
+        // (behind an affine map: the channels the map reads, out of wider rows; the rest of the last K
+        // block is filled with zeros)
+        const uint64_t a_cols = aff ? (uint64_t)src.in_c : (uint64_t)eff_cin, a_ld = aff ? (uint64_t)il.C : 0;
+        GPX_TRY(make_tmap_2d_bf16(&p.a_hi, in->hi, (uint64_t)il.rows, a_cols, 128, 64, a_ld));
+        if (in->lo) GPX_TRY(make_tmap_2d_bf16(&p.a_lo, in->lo, (uint64_t)il.rows, a_cols, 128, 64, a_ld));
+        if (aff) {
+            p.aff_scale = m.storages[src.scale].dptr;
+            p.aff_shift = m.storages[src.shift].dptr;
+            p.aff_c = src.in_c;
+        }
         GPX_TRY(make_tmap_2d_bf16(&p.w_hi, w.hi, (uint64_t)w.cout_pad, (uint64_t)w.split_k, bn, 64));
         if (w.lo) GPX_TRY(make_tmap_2d_bf16(&p.w_lo, w.lo, (uint64_t)w.cout_pad, (uint64_t)w.split_k, bn, 64));
         p.fmt = m.fmt;
@@ -1154,7 +1189,7 @@ int finalize_model(gpx_model &m) {
             const char *e_cl = getenv("GPX_SPLITK_CLUSTER");
             if (!(e_cl && e_cl[0] == '0')) {
                 s_want = s_want >= 8 ? 8 : (s_want >= 4 ? 4 : (s_want >= 2 ? 2 : 1));
-                while (bn == 64 && s_want > 2 && cgemm_max_cluster(bn, m.fmt, s_want) < out_tiles * s_want) s_want /= 2;
+                while (bn == 64 && s_want > 2 && cgemm_max_cluster(bn, m.fmt, aff, s_want) < out_tiles * s_want) s_want /= 2;
             }
             if (s_want >= 2) {
                 p.kb_per_split = (all_kb + s_want - 1) / s_want;
@@ -1242,7 +1277,7 @@ int finalize_model(gpx_model &m) {
             // number of splits that divides the tile's rows, and every cluster resident at once.
             const char *e_cl = getenv("GPX_SPLITK_CLUSTER");
             const bool pow2 = p.k_splits == 2 || p.k_splits == 4 || p.k_splits == 8;
-            if (pow2 && bn == 64 && !(e_cl && e_cl[0] == '0') && cgemm_max_cluster(bn, m.fmt, p.k_splits) >= kn.total_tiles &&
+            if (pow2 && bn == 64 && !(e_cl && e_cl[0] == '0') && cgemm_max_cluster(bn, m.fmt, aff, p.k_splits) >= kn.total_tiles &&
                 kn.grid == kn.total_tiles) {
                 p.cluster_reduce = 1;
                 p.fin = q;
@@ -1320,6 +1355,7 @@ static int storage_set(gpx_model *m, Storage &s, const void *host, size_t len, c
         }
         return GPX_SUCC;
     }
+    GPX_REQUIRE(s.affine_node < 0, GPX_FAIL, "set %s: the tensor is formed by its consumer and has no storage", s.name.c_str());
     // ActSplit: NCHW fp32 -> hi/lo planes in the storage's row order (borders stay zero)
     const ActLayout &l = s.layout;
     if (s.parent >= 0) {
@@ -1384,6 +1420,26 @@ static int storage_get(gpx_model *m, Storage &s, void *host, size_t len, cudaStr
         GPX_CUDA(cudaMemcpyAsync(tmp.data(), s.dptr, s.bytes, cudaMemcpyDeviceToHost, st));
         GPX_CUDA(cudaStreamSynchronize(st));
         khwc_o_to_oihw(tmp.data(), dst, (int)s.dims[0], (int)s.dims[1], (int)s.dims[2], (int)s.dims[3]);
+        return GPX_SUCC;
+    }
+    if (s.affine_node >= 0) {
+        // Not stored: computed from the channels its consumer reads, as the consumer does.
+        const Node &a = m->nodes[s.affine_node];
+        Storage &src = m->storages[m->nodes[a.inputs[0]].storage];
+        const Storage &sc = m->storages[a.scale], &sh = m->storages[a.shift];
+        std::vector<float> scale(a.in_c), shift(a.in_c), x(src.bytes / sizeof(float));
+        GPX_CUDA(cudaMemcpyAsync(scale.data(), sc.dptr, scale.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
+        GPX_CUDA(cudaMemcpyAsync(shift.data(), sh.dptr, shift.size() * sizeof(float), cudaMemcpyDeviceToHost, st));
+        GPX_TRY(storage_get(m, src, x.data(), src.bytes, st));
+        GPX_CUDA(cudaStreamSynchronize(st));
+        const size_t px = (size_t)a.H * a.W;
+        std::vector<bf16_bits> q(plane_count(m->fmt));
+        for (int n = 0; n < a.N; ++n)
+            for (int c = 0; c < a.in_c; ++c)
+                for (size_t i = 0; i < px; ++i) {
+                    host_put(q, 1, 0, std::max(std::fma(x[((size_t)n * src.dims[1] + c) * px + i], scale[c], shift[c]), 0.f), m->fmt);
+                    dst[((size_t)n * a.in_c + c) * px + i] = host_take(q, 1, 0, m->fmt);
+                }
         return GPX_SUCC;
     }
     const ActLayout &l = s.layout;

@@ -51,6 +51,8 @@ struct Storage {
     bool token_major = false;        // activations of sequence models: canonical [N][S][C]
     int parent = -1;                 // ActSplit: this tensor is a channel slice of that storage
     int ch_off = 0;                  //   starting at this stored channel (concatenation by placement)
+    int affine_node = -1;            // ActSplit: output of that Affine node, formed by its only consumer as it
+                                     //   loads its operand; nothing is stored (get computes it)
 };
 
 // Buffer: a tensor other nodes write slices of (the running concatenation of a dense block).
@@ -80,6 +82,7 @@ struct Node {
     int Cs = 0;                    // stored output channels (C padded to 64 when the model pads)
     int in_c = 0;                  // channels of the input that are read (0 = all): a prefix of a Buffer
     int scale = -1, shift = -1;    // Affine, or a pooling node that normalises its input: Vec storages
+    bool fused_affine = false;     // Affine applied by the consuming convolution: no kernel of its own
 };
 
 enum class KernelType { ConvSimt, Cgemm, Pool, Im2col, SplitK, LayerNorm, Attention, DwConv, AttentionTc, TransposeV, Stencil, DenseRows, GraphWl };
@@ -107,8 +110,9 @@ struct Kernel {
     double flops = 0, bytes = 0;
 };
 
+// Tensor map of a [rows][cols] matrix of 16-bit elements with row stride `ld` (0 = cols).
 int make_tmap_2d_bf16(CUtensorMap *map, const void *base, uint64_t rows, uint64_t cols,
-                      uint32_t box_rows, uint32_t box_cols);
+                      uint32_t box_rows, uint32_t box_cols, uint64_t ld = 0);
 
 }  // namespace gpx
 
