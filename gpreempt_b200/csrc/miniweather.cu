@@ -53,9 +53,82 @@ __device__ __forceinline__ Grid grid_of(const StencilParams &p) {
 // sum to the assembler; its choice depends on the surrounding code, so relying on it here would
 // tie the results to register pressure.  These are the operations the reference's kernels
 // execute (checked on a GPU against that code: all cells of all variables identical).
+//
+// The kernels are bound by instruction issue, and half of what they issued was divisions: eleven
+// (eight along x, where three more are in double) with a divisor that is a constant, a parameter, or
+// shared by three of them.  A quotient by a divisor b whose reciprocal y is at hand is q + (a - b q) y
+// with q = a y (Markstein, IBM J. Res. Dev. 34, 1990): three operations, and the correctly rounded
+// quotient when y is the correctly rounded reciprocal and nothing under- or overflows.
+__device__ __forceinline__ float div_by(float a, float b, float y) {
+    const float q = __fmul_rn(a, y);
+    return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
+}
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+// Reciprocals: the hardware's approximation refined by Newton steps (one in float, two in double).
+__device__ __forceinline__ float reciprocal(float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return __fmaf_rn(__fmaf_rn(-b, y, 1.f), y, y);
+}
+__device__ __forceinline__ double reciprocal(double b) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+    return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
+}
+
+// x^g for x > 0 as 2^(g log2 x), relative error below 4e-15: log2 from the series of artanh,
+// log2 x = k + 2 / ln 2 * (s + s^3 / 3 + s^5 / 5 + ...), s = (m - 1) / (m + 1), x = 2^k m with m between
+// sqrt(1/2) and sqrt 2 (|s| < 0.172, twelve terms), and the Taylor series of 2^f, |f| <= 1/2.  The result
+// ends in a float flux, nine digits coarser; pow() spends most of its instructions on the last bits of
+// the double and on cases (signs, zeros, infinities) that take the call here.
+__device__ __forceinline__ double power(double x, double g) {
+    if (!(x > 1e-290 && x < 1e290)) return pow(x, g);
+    const int hi = __double2hiint(x);
+    int k = (hi - 0x3fe6a09e) >> 20;  // the exponent that leaves the mantissa at or above sqrt(1/2)
+    const double m = __hiloint2double(hi - (k << 20), __double2loint(x));
+    const double s = __dmul_rn(__dsub_rn(m, 1.0), reciprocal(__dadd_rn(m, 1.0)));
+    const double z = __dmul_rn(s, s);
+    double p = 1.0 / 23;
+    p = __fma_rn(p, z, 1.0 / 21);
+    p = __fma_rn(p, z, 1.0 / 19);
+    p = __fma_rn(p, z, 1.0 / 17);
+    p = __fma_rn(p, z, 1.0 / 15);
+    p = __fma_rn(p, z, 1.0 / 13);
+    p = __fma_rn(p, z, 1.0 / 11);
+    p = __fma_rn(p, z, 1.0 / 9);
+    p = __fma_rn(p, z, 1.0 / 7);
+    p = __fma_rn(p, z, 1.0 / 5);
+    p = __fma_rn(p, z, 1.0 / 3);
+    p = __fma_rn(__dmul_rn(p, z), s, s);
+    const double lg = __fma_rn(p, 2.8853900817779268, (double)k);  // 2 / ln 2
+    const double t = __dmul_rn(g, lg);
+    const double n = rint(t);
+    const double f = __dmul_rn(__dsub_rn(t, n), 0.69314718055994531);
+    double e = 1.0 / 6227020800.0;
+    e = __fma_rn(e, f, 1.0 / 479001600.0);
+    e = __fma_rn(e, f, 1.0 / 39916800.0);
+    e = __fma_rn(e, f, 1.0 / 3628800.0);
+    e = __fma_rn(e, f, 1.0 / 362880.0);
+    e = __fma_rn(e, f, 1.0 / 40320.0);
+    e = __fma_rn(e, f, 1.0 / 5040.0);
+    e = __fma_rn(e, f, 1.0 / 720.0);
+    e = __fma_rn(e, f, 1.0 / 120.0);
+    e = __fma_rn(e, f, 1.0 / 24.0);
+    e = __fma_rn(e, f, 1.0 / 6.0);
+    e = __fma_rn(e, f, 0.5);
+    e = __fma_rn(e, f, 1.0);
+    e = __fma_rn(e, f, 1.0);
+    if (fabs(n) > 1000.0) return pow(x, g);  // the exponent would leave the normal range
+    return __hiloint2double(__double2hiint(e) + ((int)n << 20), __double2loint(e));
+}
+
 __device__ __forceinline__ float interp4(float s0, float s1, float s2, float s3) {
     // (-s0 + 7*(s1 + s2) - s3) / 12
-    return __fdiv_rn(__fsub_rn(__fmaf_rn(7.f, __fadd_rn(s1, s2), -s0), s3), 12.f);
+    return div_by(__fsub_rn(__fmaf_rn(7.f, __fadd_rn(s1, s2), -s0), s3), 12.f, 1.f / 12.f);
 }
 __device__ __forceinline__ float third_derivative(float s0, float s1, float s2, float s3, float hv_coef) {
     // (-s0 + 3*(s1 - s2) + s3) * hv_coef
@@ -125,10 +198,11 @@ __device__ __forceinline__ void tile_x(const StencilParams &p, const Grid &g, in
             d3_vals[ll] = third_derivative(s0, s1, s2, s3, hv_coef);
         }
         const double r = (double)__fadd_rn(vals[ID_DENS], hd);
-        const double u = __ddiv_rn((double)vals[ID_UMOM], r);
-        const double w = __ddiv_rn((double)vals[ID_WMOM], r);
-        const double t = __ddiv_rn((double)__fadd_rn(vals[ID_RHOT], hdt), r);
-        const double pr = __dmul_rn((double)kC0, pow(__dmul_rn(r, t), (double)kGamm));
+        const double inv_r = reciprocal(r);
+        const double u = div_by((double)vals[ID_UMOM], r, inv_r);
+        const double w = div_by((double)vals[ID_WMOM], r, inv_r);
+        const double t = div_by((double)__fadd_rn(vals[ID_RHOT], hdt), r, inv_r);
+        const double pr = __dmul_rn((double)kC0, power(__dmul_rn(r, t), (double)kGamm));
         const double ru = __dmul_rn(r, u);
         // r*u feeds four fluxes; the mass flux subtracts from the rounded product, the others fuse
         sflux[ID_DENS * ldf + f] = (float)__dsub_rn(ru, (double)d3_vals[ID_DENS]);
@@ -137,6 +211,7 @@ __device__ __forceinline__ void tile_x(const StencilParams &p, const Grid &g, in
         sflux[ID_RHOT * ldf + f] = (float)__fma_rn(ru, t, -(double)d3_vals[ID_RHOT]);
     }
     __syncthreads();
+    const float inv_dx = __frcp_rn(p.dx);
 #pragma unroll
     for (int it = 0; it < kCellIters; ++it) {
         const int f = threadIdx.x + it * kMwThreads;
@@ -144,7 +219,7 @@ __device__ __forceinline__ void tile_x(const StencilParams &p, const Grid &g, in
             const unsigned at = row + (unsigned)(i0 + f + kMwHalo);
 #pragma unroll
             for (int ll = 0; ll < kMwVars; ++ll) {
-                const float tend = __fdiv_rn(-__fsub_rn(sflux[ll * ldf + f + 1], sflux[ll * ldf + f]), p.dx);
+                const float tend = div_by(-__fsub_rn(sflux[ll * ldf + f + 1], sflux[ll * ldf + f]), p.dx, inv_dx);
                 p.out[ll * g.plane + at] = advance(init_v[it][ll], p.dt, tend);
             }
         }
@@ -179,6 +254,7 @@ __device__ __forceinline__ void tile_z(const StencilParams &p, const Grid &g, in
     const int nr = min(p.tile_rows, g.nz - k0);
     const int ca = i + kMwHalo;
     const float hv_coef = __fdiv_rn(__fmul_rn(-kHvBeta, p.dz), __fmul_rn(16.f, p.dt));
+    const float inv_dz = __frcp_rn(p.dz);
     const float *__restrict__ forcing = p.forcing;
     float win[kMwVars][4];  // array rows k .. k+3 of interface k
 #pragma unroll
@@ -227,9 +303,10 @@ __device__ __forceinline__ void tile_z(const StencilParams &p, const Grid &g, in
             d3_vals[ll] = third_derivative(win[ll][0], win[ll][1], win[ll][2], win[ll][3], hv_coef);
         }
         const float r = __fadd_rn(vals[ID_DENS], p.hy_dens_int[k]);
-        const float u = __fdiv_rn(vals[ID_UMOM], r);
-        float w = __fdiv_rn(vals[ID_WMOM], r);
-        const float t = __fdiv_rn(__fadd_rn(vals[ID_RHOT], p.hy_dens_theta_int[k]), r);
+        const float inv_r = reciprocal(r);
+        const float u = div_by(vals[ID_UMOM], r, inv_r);
+        float w = div_by(vals[ID_WMOM], r, inv_r);
+        const float t = div_by(__fadd_rn(vals[ID_RHOT], p.hy_dens_theta_int[k]), r, inv_r);
         const float pr = __fmaf_rn(kC0, powf(__fmul_rn(r, t), kGamm), -p.hy_pressure_int[k]);
         if (k == 0 || k == g.nz) {
             w = 0;
@@ -251,7 +328,7 @@ __device__ __forceinline__ void tile_z(const StencilParams &p, const Grid &g, in
             float dens_new = 0.f;
 #pragma unroll
             for (int ll = 0; ll < kMwVars; ++ll) {
-                float tend = __fdiv_rn(-__fsub_rn(flux[ll], below[ll]), p.dz);
+                float tend = div_by(-__fsub_rn(flux[ll], below[ll]), p.dz, inv_dz);
                 if (ll == ID_WMOM) tend = __fmaf_rn(-(p.gravity_from_out ? dens_new : win[ID_DENS][1]), kGrav, tend);
                 const float v = advance(init_v[ll], p.dt, tend);
                 if (ll == ID_DENS) dens_new = v;
