@@ -45,7 +45,6 @@ static const char *kernel_type_name(KernelType t) {
         case KernelType::Attention: return "attention_kernel";
         case KernelType::DwConv: return "dwconv_kernel";
         case KernelType::AttentionTc: return "attention_tc_kernel";
-        case KernelType::TransposeV: return "transpose_v_kernel";
         case KernelType::Stencil: return "miniweather_step_kernel";
         case KernelType::DenseRows: return "dense_rows_kernel";
         case KernelType::GraphWl: return "graphwl_kernel";
@@ -153,7 +152,7 @@ static void render_graph(const gpx_model *m, Json *graph, Json *host) {
         if (n.heads) attrs.set("heads", Json(n.heads));
         if (n.in_c) attrs.set("in_channels", Json(n.in_c));
         if (out.token_major) attrs.set("token_major", Json(true));
-        if (out.parent >= 0) {
+        if (out.parent >= 0 && !m->storages[out.parent].hidden) {
             attrs.set("slice_of", Json(storage_to_json[out.parent]));
             attrs.set("channel_offset", Json(out.ch_off));
         }

@@ -4,42 +4,60 @@
 // Stands in for the batch_matmul + softmax + batch_matmul kernels TVM generates for the
 // reference's BERT workload (scripts/compile/compile-bert.py:33-91; replayed by
 // src/executor.cpp:157-162).  One tile = (batch item, head, block of 128 queries), claimed through
-// the block-level preemption loop (scripts/compile/convert_to_blp.py:39-70).  Per block of 128
-// keys: S = Q K^T as one 128x128x64 product into tensor memory; every thread owns one query row
-// (its TMEM lane), keeps the running maximum and normaliser of an online softmax and writes the
-// probabilities as a 16-bit A operand into shared memory (128-byte swizzled, as TMA would); then
-// P V as a 128x64x128 product whose B operand is the transposed value matrix (keys contiguous)
-// that transpose_v_kernel prepares; the per-block result is folded into fp32 registers.
-// Thread 0 issues TMA and MMA; every wait is bounded and its outcome is shared through a block
-// barrier, so all threads leave together when one gives up.
+// the block-level preemption loop (scripts/compile/convert_to_blp.py:39-70).
 //
-// A tile of 128 queries x 512 keys takes ~27 us, above the 20 us drain target, so the preempt word
-// is also polled once per block of 128 keys.  A CTA that sees it raised gives the tile up: nothing
-// has been written yet, the tile number goes into the CTA's slot, and the relaunched CTA computes
-// that tile from its first key block before it claims new ones (the reset-and-restart treatment of
-// REEF, src/reef-client/reef_scheduler.cpp:316-357, at tile granularity: at most one tile of work
-// per CTA is repeated, and the result is the same bits either way).
+// Two warpgroups share a tile's queries and take its blocks of 64 keys in turn, each with an online
+// softmax of its own; their two partial results are merged at the end.  Per block: S = Q K^T as one
+// 128x64x64 product into tensor memory; every thread owns one query row (its TMEM lane), reads the 64
+// scores once, exponentiates them and writes the probabilities as a 16-bit A operand into shared
+// memory (128-byte swizzled, as TMA would); P V is a 128x64x64 product accumulated in tensor memory,
+// whose B operand is the value tile as it lies in HBM (rows are keys): the descriptor names it
+// MN-major, so no transposed copy of the values exists.  The accumulated output is rescaled only when
+// a row's maximum has grown by more than 2^8 since its last rescaling (the exponent reference of a row
+// may lag behind its maximum: the factor cancels in the final division), which after the first block
+// hardly ever happens.
+//
+// What bounds it: the special-function unit has 128 x 64 exponentials a block (512 cycles at 16 an SM
+// and cycle), everything else is latency between the two products; two CTAs of two independent
+// warpgroups per SM overlap each other's.  BERT-base s512 b32: one warpgroup of 128 keys a block with
+// the output folded into registers and a transposing kernel in front took 89 + 16 us a layer.
+// One thread per warpgroup issues TMA and MMA; every wait is bounded, and a wait that gives up raises
+// a flag that ends all others, so the threads of a CTA pass the same barriers and leave together.
+//
+// A tile takes a few microseconds (~6 us at 512 keys with two CTAs per SM), so the word is read
+// between tiles only.
 #include "layers.cuh"
 #include "sm100.cuh"
+
+#include <type_traits>
 
 namespace gpx {
 
 using namespace sm100;
 
-constexpr int kFaThreads = 128;
-constexpr int kFaQ = 128, kFaKeys = 128, kFaD = 64;
-constexpr uint32_t kFaTileBytes = 128 * 64 * 2;  // one 128-row x 64-column 16-bit tile: 16 KiB
-constexpr uint32_t kFaSmem = 5 * kFaTileBytes + 1024 + 256;  // Q, K, Vt, P (two tiles), slack, control
-constexpr uint32_t kFaTmemCols = 256;                        // S: 128 columns, P V: 64 columns
+constexpr int kFaThreads = 256;
+constexpr int kFaQ = 128, kFaKeys = 64, kFaD = 64;
+constexpr uint32_t kFaQBytes = kFaQ * kFaD * 2;     // 16 KiB
+constexpr uint32_t kFaKBytes = kFaKeys * kFaD * 2;  // 8 KiB, keys or values of a block
+constexpr uint32_t kFaPBytes = kFaQ * kFaKeys * 2;  // 16 KiB
+// per warpgroup: K, two V, P; both: Q, slack, control
+constexpr uint32_t kFaGroupBytes = 3 * kFaKBytes + kFaPBytes;
+constexpr uint32_t kFaSmem = kFaQBytes + 2 * kFaGroupBytes + 1024 + 2304;
+constexpr uint32_t kFaTmemCols = 256;  // per warpgroup: S 64 columns, output 64 columns
 constexpr unsigned long long kFaWaitLimitNs = 2000000000ull;
+constexpr float kFaRescale = 8.0f;     // log2 of the growth of a row maximum that forces a rescale
 
 struct FaControl {
-    unsigned long long bar_q, bar_k, bar_v, bar_mma;
+    unsigned long long bar_q;
+    unsigned long long bar_k[2], bar_s[2], bar_o[2];  // per warpgroup
+    unsigned long long bar_v[2][2];
     uint32_t tmem_base;
     int tile;
     int abort_flag;
-    int stop;  // the word was seen raised: leave at this key-block boundary
+    int pad;
+    float ml[2][kFaQ][2];  // row maximum and normaliser of each warpgroup
 };
+static_assert(sizeof(FaControl) <= 2304, "control block outgrew its shared-memory budget");
 
 // 2^x, the hardware approximation (relative error ~2^-22; -inf gives 0).
 __device__ __forceinline__ float fa_ex2(float x) {
@@ -54,312 +72,277 @@ __device__ __forceinline__ void fa_st_v8(void *ptr, const uint32_t *r) {
                  : "memory");
 }
 
-__global__ void __launch_bounds__(kFaThreads)
+template <bool HALF>
+__global__ void __launch_bounds__(kFaThreads, 2)
 attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
+    constexpr int FMT = HALF ? PF_F16 : PF_BF16;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     unsigned char *smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-    const uint32_t sQ = smem_u32(smem), sK = sQ + kFaTileBytes, sV = sQ + 2 * kFaTileBytes,
-                   sP = sQ + 3 * kFaTileBytes;
-    unsigned char *pP = smem + 3 * kFaTileBytes;
-    FaControl *ctl = reinterpret_cast<FaControl *>(smem + 5 * kFaTileBytes);
+    FaControl *ctl = reinterpret_cast<FaControl *>(smem + kFaQBytes + 2 * kFaGroupBytes);
     volatile int *abort_flag = &ctl->abort_flag;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x;
+    const int wg = __shfl_sync(0xffffffffu, tid >> 7, 0);  // warpgroup
+    const int row = tid & 127;
+    const bool issuer = row == 0;  // this warpgroup's TMA and MMA thread
+    unsigned char *mine = smem + kFaQBytes + wg * kFaGroupBytes;
+    const uint32_t sQ = smem_u32(smem), sK = smem_u32(mine), sV = sK + kFaKBytes, sP = sK + 3 * kFaKBytes;
+    unsigned char *pV = mine + kFaKBytes, *pP = mine + 3 * kFaKBytes;
 
     if (tid == 0) {
         mbar_init(smem_u32(&ctl->bar_q), 1);
-        mbar_init(smem_u32(&ctl->bar_k), 1);
-        mbar_init(smem_u32(&ctl->bar_v), 1);
-        mbar_init(smem_u32(&ctl->bar_mma), 1);
+        for (int g = 0; g < 2; ++g) {
+            mbar_init(smem_u32(&ctl->bar_k[g]), 1);
+            mbar_init(smem_u32(&ctl->bar_s[g]), 1);
+            mbar_init(smem_u32(&ctl->bar_o[g]), 1);
+            mbar_init(smem_u32(&ctl->bar_v[g][0]), 1);
+            mbar_init(smem_u32(&ctl->bar_v[g][1]), 1);
+        }
         ctl->abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async();
     }
-    if (warp == 0) tmem_alloc(smem_u32(&ctl->tmem_base), kFaTmemCols);
+    if (tid < 32) tmem_alloc(smem_u32(&ctl->tmem_base), kFaTmemCols);
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
     pdl_wait();  // the prologue above overlapped the predecessor's tail
     pdl_launch_dependents();
     if (tid == 0) trace_begin(blp);
-    const uint32_t tmem = ctl->tmem_base;
-    const uint32_t t_lane = tmem + ((uint32_t)(warp * 32) << 16);
-    const uint32_t idesc_s = p.fmt == PF_F16 ? make_idesc_f16_f32(128, 128) : make_idesc_bf16_f32(128, 128);
-    const uint32_t idesc_o = p.fmt == PF_F16 ? make_idesc_f16_f32(128, 64) : make_idesc_bf16_f32(128, 64);
+    const uint32_t tmem_base = ctl->tmem_base;
+    const uint32_t t_s = tmem_base + wg * 128, t_o = t_s + 64;          // as the products address them
+    const uint32_t lane_off = (uint32_t)((row >> 5) * 32) << 16;        // as this warp's loads do
+    constexpr uint32_t idesc = HALF ? make_idesc_f16_f32(kFaQ, 64) : make_idesc_bf16_f32(kFaQ, 64);
+    constexpr uint32_t idesc_o = idesc | (1u << 16);  // B is MN-major: value rows are keys
     auto fail = [&](int code) {
-        ctl->abort_flag = 1;
+        *abort_flag = 1;
         if (p.error && atomicCAS(p.error, 0, code) == 0) p.error[1] = blp.kernel_id * 1000 + (int)blockIdx.x;
     };
-    // Thread 0 waits (bounded); the block barrier that follows publishes the outcome.
-    auto leader_wait = [&](unsigned long long *bar, uint32_t phase, int code) {
-        if (tid == 0 && !*abort_flag && !mbar_wait(smem_u32(bar), phase, abort_flag, kFaWaitLimitNs)) fail(code);
+    auto wait = [&](unsigned long long *bar, uint32_t phase, int code) {
+        if (!mbar_wait(smem_u32(bar), phase, abort_flag, kFaWaitLimitNs)) fail(code);
     };
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory"); };
 
     const int qblocks = (p.S + kFaQ - 1) / kFaQ;
     const int nkb = (p.S + kFaKeys - 1) / kFaKeys;
+    const int steps = (nkb - wg + 1) / 2;  // blocks wg, wg + 2, ... of this warpgroup
     const float scale_log2 = p.scale * 1.4426950408889634f;  // scores are exponentiated base 2
-    uint32_t ph_q = 0, ph_k = 0, ph_v = 0, ph_m = 0;
+    uint32_t ph_q = 0, ph_k = 0, ph_s = 0, ph_o = 0, ph_v[2] = {0, 0};
     int iter = 0;
-    int tiles_done = 0;
-    bool dead = false;
-    const bool resumable = blp.preempted != nullptr && p.slots != nullptr;
-    CgemmSlot *slot = resumable ? p.slots + blockIdx.x : nullptr;
-    // The tile this CTA gave up in the previous launch, if any (thread 0 only).
-    int pending = (resumable && tid == 0) ? slot->next_iter - 1 : -1;
-    for (; !dead; ++iter) {
-        if (tid == 0) {
-            int t;
-            if (pending >= 0) {
-                // An interrupted tile comes first; a kernel relaunched while the word is still up
-                // keeps it for the next launch and reports itself as the stop point.
-                if (load_word(blp.preempted) != 0) {
-                    atomicCAS(blp.stop_index, -1, blp.kernel_id);
-                    if (blp.trace) atomicMin(blp.trace + 2, globaltimer_ns());
-                    t = -1;
-                } else {
-                    t = pending;
-                    pending = -1;
-                    slot->next_iter = 0;
-                }
-            } else {
-                t = blp_claim(blp, iter);
-            }
-            ctl->tile = t;
-            ctl->stop = 0;
-        }
+    for (;; ++iter) {
+        if (tid == 0) ctl->tile = *abort_flag ? -1 : blp_claim(blp, iter);
         __syncthreads();
         const int tile = ctl->tile;
         if (tile < 0) break;
         const int qb = tile % qblocks;
         const int head = (tile / qblocks) % p.heads;
         const int b = tile / (qblocks * p.heads);
-        const int q0 = qb * kFaQ;
+        const int q0 = qb * kFaQ, key_row0 = b * p.S;
         const int col0 = head * kFaD;
-        const int vt_row = (b * p.heads + head) * kFaD;
         if (tid == 0) {
-            mbar_arrive_expect_tx(smem_u32(&ctl->bar_q), kFaTileBytes);
-            tma_load_2d(sQ, &p.tq, smem_u32(&ctl->bar_q), col0, b * p.S + q0);
-            mbar_arrive_expect_tx(smem_u32(&ctl->bar_k), kFaTileBytes);
-            tma_load_2d(sK, &p.tk, smem_u32(&ctl->bar_k), col0, b * p.S);
-            mbar_arrive_expect_tx(smem_u32(&ctl->bar_v), kFaTileBytes);
-            tma_load_2d(sV, &p.tvt, smem_u32(&ctl->bar_v), 0, vt_row);
-            tma_load_2d(sV + kFaTileBytes / 2, &p.tvt, smem_u32(&ctl->bar_v), 64, vt_row);
+            mbar_arrive_expect_tx(smem_u32(&ctl->bar_q), kFaQBytes);
+            tma_load_2d(sQ, &p.tq, smem_u32(&ctl->bar_q), col0, key_row0 + q0);
         }
+        auto fetch = [&](uint32_t dst, const void *map, unsigned long long *bar, int step) {
+            mbar_arrive_expect_tx(smem_u32(bar), kFaKBytes);
+            tma_load_2d(dst, map, smem_u32(bar), col0, key_row0 + (2 * step + wg) * kFaKeys);
+        };
+        auto scores = [&]() {  // S = Q K^T of the block whose keys are in sK (issuer only)
+            const uint64_t dq = make_smem_desc_sw128(sQ), dk = make_smem_desc_sw128(sK);
+#pragma unroll
+            for (int k = 0; k < kFaD / 16; ++k) mma_f16_ss(t_s, dq + 2 * k, dk + 2 * k, idesc, k > 0 ? 1u : 0u);
+            mma_commit(smem_u32(&ctl->bar_s[wg]));
+        };
         float m = -INFINITY, l = 0.f;
-        float o[kFaD];
-#pragma unroll
-        for (int d = 0; d < kFaD; ++d) o[d] = 0.f;
-        leader_wait(&ctl->bar_q, ph_q, 401);
-        ph_q ^= 1;
-        bool stopped = false;
-        for (int kb = 0; kb < nkb; ++kb) {
-            // The word is read at the top of every key block; its value is needed only after the
-            // first product of the block, so the load's latency is hidden.
-            int word_now = 0;
-            if (resumable && tid == 0 && kb > 0) word_now = load_word(blp.preempted);
-            // ---- S = Q K^T
-            leader_wait(&ctl->bar_k, ph_k, 402);
-            ph_k ^= 1;
-            if (tid == 0 && !*abort_flag) {
-                tc_fence_after_sync();
-                const uint64_t dq = make_smem_desc_sw128(sQ), dk = make_smem_desc_sw128(sK);
-#pragma unroll
-                for (int k = 0; k < kFaD / 16; ++k) mma_f16_ss(tmem, dq + 2 * k, dk + 2 * k, idesc_s, k > 0 ? 1u : 0u);
-                mma_commit(smem_u32(&ctl->bar_mma));
-            }
-            leader_wait(&ctl->bar_mma, ph_m, 403);
-            ph_m ^= 1;
-            if (tid == 0 && word_now != 0) ctl->stop = 1;
-            __syncthreads();
-            if (*abort_flag) {
-                dead = true;
-                break;
-            }
-            if (ctl->stop) {
-                // Give the tile up.  The value tile of this block is the only copy still in flight.
-                leader_wait(&ctl->bar_v, ph_v, 406);
-                ph_v ^= 1;
-                if (tid == 0) {
-                    slot->next_iter = tile + 1;
-                    atomicCAS(blp.stop_index, -1, blp.kernel_id);
-                    if (blp.trace) atomicMin(blp.trace + 2, globaltimer_ns());
-                }
-                __syncthreads();
-                stopped = true;
-                break;
-            }
+        if (steps > 0 && issuer) {
+            fetch(sK, &p.tk, &ctl->bar_k[wg], 0);
+            fetch(sV, &p.tv, &ctl->bar_v[wg][0], 0);
+            wait(&ctl->bar_q, ph_q, 401);
+            wait(&ctl->bar_k[wg], ph_k, 402);
             tc_fence_after_sync();
-            if (tid == 0 && kb + 1 < nkb) {  // the key tile is free again: fetch the next block
-                mbar_arrive_expect_tx(smem_u32(&ctl->bar_k), kFaTileBytes);
-                tma_load_2d(sK, &p.tk, smem_u32(&ctl->bar_k), col0, b * p.S + (kb + 1) * kFaKeys);
-            }
-            // ---- online softmax of this thread's row over the 128 keys of the block
-            const int key0 = kb * kFaKeys;
-            uint32_t v[32];
-            // Whole blocks (all 128 keys inside the sequence) skip the per-key bound test.
-            const bool whole = key0 + kFaKeys <= p.S;
-            float bmax = -INFINITY;  // of the raw scores: the scale is positive
-#pragma unroll
-            for (int c = 0; c < kFaKeys; c += 32) {
-                tmem_ld_32x32(t_lane + c, v);
+            if (!*abort_flag) scores();
+        }
+        ph_q ^= 1;
+        for (int j = 0; j < steps; ++j) {
+            const int buf = j & 1;
+            ph_k ^= 1;
+            wait(&ctl->bar_s[wg], ph_s, 403);
+            ph_s ^= 1;
+            tc_fence_after_sync();
+            if (issuer && j + 1 < steps && !*abort_flag) fetch(sK, &p.tk, &ctl->bar_k[wg], j + 1);  // S is done with the keys
+            uint32_t v[64];
+            {
+                uint32_t a[32], c[32];
+                __syncwarp();
+                tmem_ld_32x32(t_s + lane_off, a);
+                tmem_ld_32x32(t_s + lane_off + 32, c);
                 tmem_ld_wait();
-                if (whole) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) bmax = fmaxf(bmax, __uint_as_float(v[j]));
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        if (key0 + c + j < p.S) bmax = fmaxf(bmax, __uint_as_float(v[j]));
-                }
+                for (int i = 0; i < 32; ++i) v[i] = a[i], v[32 + i] = c[i];
             }
+            const int key0 = (2 * j + wg) * kFaKeys;
+            const int keys = p.S - key0 < kFaKeys ? p.S - key0 : kFaKeys;
+            if (keys < kFaKeys) {
+#pragma unroll
+                for (int i = 0; i < 64; ++i)
+                    if (i >= keys) v[i] = 0xff800000u;  // -inf
+            }
+            float bmax = __uint_as_float(v[0]);  // of the raw scores: the scale is positive
+#pragma unroll
+            for (int i = 1; i < 64; ++i) bmax = fmaxf(bmax, __uint_as_float(v[i]));
             const float m_new = fmaxf(m, bmax * scale_log2);
-            const float alpha = fa_ex2(m - m_new);
-            float lsum = 0.f;
-            const int r8 = tid & 7;
-            unsigned char *prow = pP + (tid >> 3) * 1024 + r8 * 128;
-#pragma unroll
-            for (int c = 0; c < kFaKeys; c += 32) {
-                tmem_ld_32x32(t_lane + c, v);
-                tmem_ld_wait();
-                uint32_t pk[16];
-#pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    float e0 = fa_ex2(fmaf(__uint_as_float(v[j]), scale_log2, -m_new));
-                    float e1 = fa_ex2(fmaf(__uint_as_float(v[j + 1]), scale_log2, -m_new));
-                    if (!whole) {
-                        if (key0 + c + j >= p.S) e0 = 0.f;
-                        if (key0 + c + j + 1 >= p.S) e1 = 0.f;
-                    }
-                    lsum += e0 + e1;
-                    pk[j >> 1] = pf_pack2(e0, e1, p.fmt);
-                }
-                // 32 keys = four 16-byte pieces of this row, in the 128-byte swizzled layout of
-                // an A tile: piece index XOR (row mod 8); keys 64..127 form the second tile.
-                unsigned char *tile_row = prow + (c >> 6) * kFaTileBytes;
-                const int piece0 = (c & 63) >> 3;
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    *reinterpret_cast<uint4 *>(tile_row + (((piece0 + q) ^ r8) << 4)) =
-                        make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
+            // P V of the block before: its probabilities and values are free, its output is complete
+            if (j > 0) {
+                wait(&ctl->bar_o[wg], ph_o, 404);
+                ph_o ^= 1;
+                if (issuer && j + 1 < steps && !*abort_flag) fetch(sV + (buf ^ 1) * kFaKBytes, &p.tv, &ctl->bar_v[wg][buf ^ 1], j + 1);
+            } else {
+                if (issuer && j + 1 < steps && !*abort_flag) fetch(sV + kFaKBytes, &p.tv, &ctl->bar_v[wg][1], 1);
+                m = m_new;
             }
-            l = l * alpha + lsum;
-            m = m_new;
+            if (__any_sync(0xffffffffu, m_new > m + kFaRescale)) {
+                const float m_to = m_new > m + kFaRescale ? m_new : m;
+                const float alpha = fa_ex2(m - m_to);
+                tc_fence_after_sync();
+#pragma unroll
+                for (int c = 0; c < kFaD; c += 16) {
+                    uint32_t o[16];
+                    tmem_ld_32x16(t_o + lane_off + c, o);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                    tmem_st_32x16(t_o + lane_off + c, o);
+                }
+                tmem_st_wait();
+                l *= alpha;
+                m = m_to;
+            }
+            const int r8 = row & 7;
+            unsigned char *prow = pP + (row >> 3) * 1024 + r8 * 128;
+            float lsum[4] = {0.f, 0.f, 0.f, 0.f};
+            const float2 sc2 = make_float2(scale_log2, scale_log2), neg_m = make_float2(-m, -m);
+#pragma unroll
+            for (int c = 0; c < 64; c += 8) {
+                uint32_t pk[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 x = fma2(make_float2(__uint_as_float(v[c + 2 * i]), __uint_as_float(v[c + 2 * i + 1])), sc2, neg_m);
+                    const float e0 = fa_ex2(x.x), e1 = fa_ex2(x.y);
+                    lsum[i] += e0 + e1;
+                    pk[i] = pf_pack2(e0, e1, FMT);
+                }
+                // eight keys = one 16-byte piece of this row, at piece index XOR (row mod 8)
+                *reinterpret_cast<uint4 *>(prow + (((c >> 3) ^ r8) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            }
+            l += (lsum[0] + lsum[1]) + (lsum[2] + lsum[3]);
+            if (keys < kFaKeys) {
+                // Rows past the sequence belong to the next batch item: their probabilities are zero, and
+                // so must they be (zero times an infinity is not).
+                wait(&ctl->bar_v[wg][buf], ph_v[buf], 405);
+                for (int e = row; e < (kFaKeys - keys) * 8; e += 128)
+                    *reinterpret_cast<uint4 *>(pV + buf * kFaKBytes + (keys + (e >> 3)) * 128 + (e & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+            }
             fence_proxy_async();  // the probabilities were written by ordinary stores, the MMA reads them
             tc_fence_before_sync();
-            leader_wait(&ctl->bar_v, ph_v, 404);
-            ph_v ^= 1;
-            __syncthreads();
-            if (*abort_flag) {
-                dead = true;
-                break;
-            }
-            // ---- P V
-            if (tid == 0) {
+            group_sync();
+            if (issuer && !*abort_flag) {
+                wait(&ctl->bar_v[wg][buf], ph_v[buf], 405);
                 tc_fence_after_sync();
+                const uint64_t dp = make_smem_desc_sw128(sP);
+                // Value tile: 64 keys x 128 bytes, 128-byte swizzle.  As an MN-major operand eight keys
+                // are 1024 bytes apart from the next eight, and the 64 output columns are one swizzle
+                // atom wide; a step of sixteen keys is 2048 bytes (128 in the descriptor's units).
+                const uint64_t dv = make_smem_desc_sw128(sV + buf * kFaKBytes) | ((uint64_t)(1024 >> 4) << 16);
 #pragma unroll
-                for (int kk = 0; kk < kFaKeys / 16; ++kk) {
-                    const uint64_t dp = make_smem_desc_sw128(sP + (kk >> 2) * kFaTileBytes) + 2 * (kk & 3);
-                    const uint64_t dv = make_smem_desc_sw128(sV + (kk >> 2) * (kFaTileBytes / 2)) + 2 * (kk & 3);
-                    mma_f16_ss(tmem + 128, dp, dv, idesc_o, kk > 0 ? 1u : 0u);
+                for (int k = 0; k < kFaKeys / 16; ++k)
+                    mma_f16_ss(t_o, dp + 2 * k, dv + 128 * k, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+                mma_commit(smem_u32(&ctl->bar_o[wg]));
+                if (j + 1 < steps) {
+                    wait(&ctl->bar_k[wg], ph_k, 402);
+                    tc_fence_after_sync();
+                    if (!*abort_flag) scores();
                 }
-                mma_commit(smem_u32(&ctl->bar_mma));
             }
-            leader_wait(&ctl->bar_mma, ph_m, 405);
-            ph_m ^= 1;
-            __syncthreads();
-            if (*abort_flag) {
-                dead = true;
-                break;
-            }
-            tc_fence_after_sync();
-            if (tid == 0 && kb + 1 < nkb) {  // value tile free: fetch the next block
-                mbar_arrive_expect_tx(smem_u32(&ctl->bar_v), kFaTileBytes);
-                tma_load_2d(sV, &p.tvt, smem_u32(&ctl->bar_v), (kb + 1) * kFaKeys, vt_row);
-                tma_load_2d(sV + kFaTileBytes / 2, &p.tvt, smem_u32(&ctl->bar_v), (kb + 1) * kFaKeys + 64, vt_row);
-            }
-#pragma unroll
-            for (int c = 0; c < kFaD; c += 32) {
-                tmem_ld_32x32(t_lane + 128 + c, v);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 32; ++j) o[c + j] = fmaf(o[c + j], alpha, __uint_as_float(v[j]));
-            }
-            tc_fence_before_sync();  // orders these TMEM reads before the next block's products
+            ph_v[buf] ^= 1;
         }
-        if (dead || stopped) break;
-        ++tiles_done;
-        if (q0 + tid < p.S) {
-            const float inv = 1.0f / l;
-            uint32_t w[kFaD / 2];
+        if (steps > 0) {
+            wait(&ctl->bar_o[wg], ph_o, 406);
+            ph_o ^= 1;
+        }
+        tc_fence_after_sync();
+        __syncwarp();
+        // ---- merge: warpgroup g finishes columns 32 g .. 32 g + 31, the other 32 go through shared memory
+        // (this warpgroup's V and P tiles, free by now: [column][row] floats)
+        float keep[32];
+        {
+            uint32_t o[32];
+            float *give = reinterpret_cast<float *>(pV);
 #pragma unroll
-            for (int d = 0; d < kFaD; d += 2) w[d >> 1] = pf_pack2(o[d] * inv, o[d + 1] * inv, p.fmt);
-            bf16_bits *dst = p.out_hi + ((size_t)b * p.S + q0 + tid) * p.ld + col0;
+            for (int half = 0; half < 2; ++half) {
+                if (steps > 0) {
+                    tmem_ld_32x32(t_o + lane_off + 32 * half, o);
+                    tmem_ld_wait();
+                } else {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) fa_st_v8(dst + 16 * q, w + 8 * q);
+                    for (int i = 0; i < 32; ++i) o[i] = 0u;
+                }
+                if (half == wg) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) keep[i] = __uint_as_float(o[i]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) give[i * kFaQ + row] = __uint_as_float(o[i]);
+                }
+            }
+            ctl->ml[wg][row][0] = m;
+            ctl->ml[wg][row][1] = l;
+        }
+        tc_fence_before_sync();
+        __syncthreads();
+        if (q0 + row < p.S) {
+            const float m0 = ctl->ml[0][row][0], m1 = ctl->ml[1][row][0];
+            const float mm = fmaxf(m0, m1);
+            const float a0 = fa_ex2(m0 - mm), a1 = fa_ex2(m1 - mm);
+            const float inv = 1.0f / (ctl->ml[0][row][1] * a0 + ctl->ml[1][row][1] * a1);
+            const float f_mine = (wg == 0 ? a0 : a1) * inv, f_other = (wg == 0 ? a1 : a0) * inv;
+            const float *take = reinterpret_cast<const float *>(smem + kFaQBytes + (wg ^ 1) * kFaGroupBytes + kFaKBytes);
+            uint32_t w[16];
+#pragma unroll
+            for (int i = 0; i < 32; i += 2) {
+                const float x = fmaf(take[i * kFaQ + row], f_other, keep[i] * f_mine);
+                const float y = fmaf(take[(i + 1) * kFaQ + row], f_other, keep[i + 1] * f_mine);
+                w[i >> 1] = pf_pack2(x, y, FMT);
+            }
+            bf16_bits *dst = p.out_hi + ((size_t)b * p.S + q0 + row) * p.ld_out + col0 + 32 * wg;
+            fa_st_v8(dst, w);
+            fa_st_v8(dst + 16, w + 8);
+        }
+        fence_proxy_async();  // TMA writes the next tile's operands where ordinary accesses were made
+        __syncthreads();
+        if (*abort_flag) {
+            for (int spin = 0; spin < 64; ++spin) __nanosleep(1000);  // copies in flight land before the CTA ends
+            break;
         }
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 0) {
+    if (tid < 32) {
         tc_fence_after_sync();
-        tmem_dealloc(tmem, kFaTmemCols);
+        tmem_dealloc(tmem_base, kFaTmemCols);
     }
-    if (tid == 0) trace_end(blp, tiles_done);
-}
-
-// Vt[(b*heads + h)*64 + d][key] = V[b*S + key][h*64 + d]: the value matrix with keys contiguous, the
-// K-major B operand of the second product.  One tile = 64 keys of one (batch item, head).
-__global__ void __launch_bounds__(256)
-transpose_v_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
-    pdl_enter();
-    __shared__ int s_tile;
-    __shared__ bf16_bits t[64][64 + 2];
-    if (threadIdx.x == 0) trace_begin(blp);
-    const int kblocks = (p.S + 63) / 64;
-    int iter = 0;
-    for (;; ++iter) {
-        if (threadIdx.x == 0) s_tile = blp_claim(blp, iter);
-        __syncthreads();
-        const int tile = s_tile;
-        if (tile < 0) break;
-        const int kblk = tile % kblocks, bh = tile / kblocks;
-        const int b = bh / p.heads, h = bh % p.heads;
-        for (int e = threadIdx.x; e < 64 * 8; e += 256) {
-            const int key = e >> 3, piece = e & 7;
-            uint4 q = make_uint4(0u, 0u, 0u, 0u);
-            if (kblk * 64 + key < p.S)
-                q = *reinterpret_cast<const uint4 *>(p.v_hi + ((size_t)b * p.S + kblk * 64 + key) * p.ld + h * 64 + piece * 8);
-            const bf16_bits *src = reinterpret_cast<const bf16_bits *>(&q);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) t[key][piece * 8 + j] = src[j];
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < 64 * 8; e += 256) {
-            const int d = e >> 3, piece = e & 7;
-            if (kblk * 64 + piece * 8 < p.S) {  // S is a multiple of 8: whole pieces are in or out
-                bf16_bits w[8];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) w[j] = t[piece * 8 + j][d];
-                *reinterpret_cast<uint4 *>(p.vt + ((size_t)bh * 64 + d) * p.S + kblk * 64 + piece * 8) =
-                    *reinterpret_cast<const uint4 *>(w);
-            }
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) trace_end(blp, iter);
+    if (tid == 0) trace_end(blp, iter);
 }
 
 cudaError_t attention_tc_prepare() {
-    return cudaFuncSetAttribute(attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFaSmem);
+    cudaError_t e = cudaFuncSetAttribute(attention_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFaSmem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(attention_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFaSmem);
 }
+
+int attention_tc_threads() { return kFaThreads; }
 
 cudaError_t attention_tc_launch(const AttnParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(attention_tc_kernel, grid, kFaThreads, kFaSmem, s, p, blp);
-    return cudaGetLastError();
-}
-
-cudaError_t transpose_v_launch(const AttnParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(transpose_v_kernel, grid, 256, 0, s, p, blp);
+    launch_layer(p.fmt == PF_F16 ? attention_tc_kernel<true> : attention_tc_kernel<false>, grid, kFaThreads, kFaSmem, s, p, blp);
     return cudaGetLastError();
 }
 

@@ -252,24 +252,20 @@ cudaError_t layernorm_launch(const LayerNormParams &p, int grid, const BlpArgs &
 struct AttnParams {
     const bf16_bits *q_hi, *q_lo, *k_hi, *k_lo, *v_hi, *v_lo;
     bf16_bits *out_hi, *out_lo;
-    int B, S, heads, ld;
+    int B, S, heads;
+    int ld, ld_out;         // row strides of q, k, v (columns of one wider matrix) and of the output
     int fmt;                // PlaneFmt of all four matrices
     float scale;
     int total_tiles;
-    // Tensor-core path (single-plane formats, attention_tcgen05.cu): TMA maps of Q and K
-    // ([B*S][ld], boxes of 128 rows x 64 columns) and of the transposed values
-    // ([B*heads*64][S], boxes of 64 x 64), the transposed-value scratch and the error word.
-    CUtensorMap tq, tk, tvt;
-    bf16_bits *vt;
+    // Tensor-core path (single-plane formats, attention_tcgen05.cu): TMA maps of Q ([B*S][64 heads],
+    // boxes of 128 rows x 64 columns), K and V (boxes of 64 x 64), and the error word.
+    CUtensorMap tq, tk, tv;
     int *error;
-    // One slot per CTA (this executor's): next_iter holds, plus one, the tile the CTA gave up when
-    // the word went up inside it; the relaunched CTA recomputes that tile before it claims new ones.
-    CgemmSlot *slots;
 };
 cudaError_t attention_launch(const AttnParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
 cudaError_t attention_tc_prepare();
 cudaError_t attention_tc_launch(const AttnParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
-cudaError_t transpose_v_launch(const AttnParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
+int attention_tc_threads();
 
 // Depthwise k x k convolution + bias + activation over split-plane activations; the filter is
 // stored [kh*kw][C] so that eight channels of one tap are one 32-byte load.

@@ -649,6 +649,65 @@ int finalize_model(gpx_model &m) {
         n.sub_storage = m.add_storage(s);
         order.push_back(ACT_PLAIN);
     }
+    // Query, key and value projections of an attention layer as one product: the input is read once,
+    // and at batch 1 one launch replaces three (and their reductions).
+    for (size_t ai = 0; ai < m.nodes.size(); ++ai) {
+        if (m.nodes[ai].op != Op::Attention) continue;
+        const int q = m.nodes[ai].inputs[0];
+        const Node &nq = m.nodes[q];
+        bool ok = true;
+        for (int i = 0; i < 3 && ok; ++i) {
+            const int id = m.nodes[ai].inputs[i];
+            const Node &n = m.nodes[id];
+            int users = 0;
+            for (const Node &o : m.nodes)
+                for (int in : o.inputs) users += in == id ? 1 : 0;
+            const Storage &out = m.storages[n.storage];
+            ok = id == q + i && n.op == Op::Conv && n.tensor_core && !n.via_im2col && n.k == 1 && n.stride == 1 && n.pad == 0 &&
+                 n.act == ACT_NONE && n.residual < 0 && users == 1 && n.inputs[0] == nq.inputs[0] && n.C == nq.C && n.C % 128 == 0 &&
+                 out.kind == Storage::ActSplit && out.token_major && out.parent < 0 && !out.cs && n.H == 1 && n.W > 1;
+        }
+        if (!ok) continue;
+        Storage so;
+        so.name = nq.name + ".qkv";
+        so.kind = Storage::ActSplit;
+        so.hidden = so.token_major = true;
+        so.rank = 4;
+        so.dims[0] = nq.N;
+        so.dims[1] = 3 * nq.C;
+        so.dims[2] = nq.H;
+        so.dims[3] = nq.W;
+        so.bytes = (size_t)nq.N * 3 * nq.C * nq.H * nq.W * sizeof(float);
+        const int out_idx = m.add_storage(so);
+        order.push_back(ACT_PLAIN);
+        Storage sw = m.storages[nq.weight];  // (planes only: the fp32 masters stay with the three parameters)
+        sw.name = nq.name + ".qkv.weight";
+        sw.hidden = true;
+        sw.is_param = false;
+        sw.dims[0] = 3 * nq.C;
+        sw.bytes *= 3;
+        const int w_idx = m.add_storage(sw);
+        order.push_back(ACT_PLAIN);
+        Storage sb = m.storages[nq.bias];
+        sb.name = nq.name + ".qkv.bias";
+        sb.hidden = true;
+        sb.is_param = false;
+        sb.dims[0] = 3 * nq.C;
+        sb.bytes *= 3;
+        const int b_idx = m.add_storage(sb);
+        order.push_back(ACT_PLAIN);
+        for (int i = 0; i < 3; ++i) {
+            Node &n = m.nodes[q + i];
+            n.fused_w = w_idx;
+            n.fused_b = b_idx;
+            n.fused_out = out_idx;
+            n.fused_into_other = i > 0;
+            m.storages[n.storage].parent = out_idx;
+            m.storages[n.storage].ch_off = i * n.C;
+            m.storages[n.weight].borrowed = true;
+            m.storages[n.bias].borrowed = true;
+        }
+    }
     for (auto &n : m.nodes)
         if (n.op == Op::DwConv) m.storages[n.weight].cin_pad = stored_c(m, n);
     for (auto &n : m.nodes)
@@ -664,6 +723,13 @@ int finalize_model(gpx_model &m) {
             if (n.via_s2d) {
                 w.s2d = true;
                 w.split_k = 256;  // four block rows x four blocks x 16 channels
+            }
+            if (n.fused_w >= 0) {
+                Storage &fw = m.storages[n.fused_w];
+                fw.wants_split = true;
+                fw.cin_pad = w.cin_pad;
+                fw.split_k = w.split_k;
+                fw.cout_pad = 3 * w.cout_pad;
             }
         }
 
@@ -690,10 +756,13 @@ int finalize_model(gpx_model &m) {
             // A depthwise filter is stored [kh*kw][stored channels].
             if (s.kind == Storage::Weight && s.depthwise)
                 alloc = (size_t)s.dims[2] * s.dims[3] * s.cin_pad * sizeof(float);
-            GPX_CUDA(cudaMalloc((void **)&s.dptr, alloc));
-            GPX_CUDA(cudaMemset(s.dptr, 0, alloc));
+            if (!(s.kind == Storage::Weight && s.hidden) && !(s.kind == Storage::Vec && s.borrowed)) {
+                GPX_CUDA(cudaMalloc((void **)&s.dptr, alloc));
+                GPX_CUDA(cudaMemset(s.dptr, 0, alloc));
+            }
             if (s.kind == Storage::Weight && s.wants_split) {
                 s.plane_elems = (size_t)s.cout_pad * s.split_k;
+                if (s.borrowed) continue;  // bound below
                 GPX_CUDA(cudaMalloc((void **)&s.hi, plane_count(m.fmt) * s.plane_elems * sizeof(bf16_bits)));
                 GPX_CUDA(cudaMemset(s.hi, 0, plane_count(m.fmt) * s.plane_elems * sizeof(bf16_bits)));
                 s.lo = m.fmt == PF_SPLIT ? s.hi + s.plane_elems : nullptr;
@@ -710,6 +779,14 @@ int finalize_model(gpx_model &m) {
         s.plane_elems = par.plane_elems;
         s.hi = par.hi + s.ch_off;
         s.lo = par.lo ? par.lo + s.ch_off : nullptr;
+    }
+    for (const Node &n : m.nodes) {
+        if (n.fused_w < 0) continue;
+        const int i = m.storages[n.storage].ch_off / n.C;  // which third
+        Storage &w = m.storages[n.weight], &fw = m.storages[n.fused_w];
+        w.hi = fw.hi + i * w.plane_elems;
+        w.lo = fw.lo ? fw.lo + i * w.plane_elems : nullptr;
+        m.storages[n.bias].dptr = m.storages[n.fused_b].dptr + i * n.C;
     }
     {
         // 128 x 128 identity in the plane format: the W operand of residual K blocks.
@@ -833,34 +910,24 @@ int finalize_model(gpx_model &m) {
             q.B = n.N;
             q.S = n.W;
             q.heads = n.heads;
-            q.ld = n.C;
+            q.ld = sq.layout.C;
+            q.ld_out = n.C;
+            GPX_REQUIRE(sk.layout.C == q.ld && sv.layout.C == q.ld, GPX_FAIL, "%s: row strides differ", n.name.c_str());
             q.scale = 0.125f;  // 1 / sqrt(64)
             kn.flops = 4.0 * n.N * n.heads * (double)n.W * n.W * 64;
             kn.bytes = 4.0 * 4 * (double)n.N * n.W * n.C;
             const char *force_simt = getenv("GPX_ATTN");
             if (m.fmt != PF_SPLIT && !(force_simt && std::string(force_simt) == "simt")) {
-                // Single-plane models: both products on the tensor cores.  The values are first
-                // written with keys contiguous (the B operand of the second product).
-                const size_t vt_elems = (size_t)n.N * n.heads * 64 * n.W;
-                GPX_CUDA(cudaMalloc((void **)&q.vt, vt_elems * sizeof(bf16_bits)));
-                GPX_CUDA(cudaMemset(q.vt, 0, vt_elems * sizeof(bf16_bits)));
-                m.scratch.push_back(q.vt);
+                // Single-plane models: both products on the tensor cores, the values read as they lie
+                // through a transposing descriptor (which the kernel's name tells).
                 const uint64_t rows = (uint64_t)n.N * n.W;
-                GPX_TRY(make_tmap_2d_bf16(&q.tq, sq.hi, rows, (uint64_t)n.C, 128, 64));
-                GPX_TRY(make_tmap_2d_bf16(&q.tk, sk.hi, rows, (uint64_t)n.C, 128, 64));
-                GPX_TRY(make_tmap_2d_bf16(&q.tvt, q.vt, (uint64_t)n.N * n.heads * 64, (uint64_t)n.W, 64, 64));
+                GPX_TRY(make_tmap_2d_bf16(&q.tq, sq.hi, rows, (uint64_t)n.C, 128, 64, (uint64_t)q.ld));
+                GPX_TRY(make_tmap_2d_bf16(&q.tk, sk.hi, rows, (uint64_t)n.C, 64, 64, (uint64_t)q.ld));
+                GPX_TRY(make_tmap_2d_bf16(&q.tv, sv.hi, rows, (uint64_t)n.C, 64, 64, (uint64_t)q.ld));
                 GPX_CUDA(attention_tc_prepare());
-                Kernel kt = kn;
-                kt.name = n.name + ".vt";
-                kt.type = KernelType::TransposeV;
-                kt.threads = 256;
-                kt.total_tiles = n.N * n.heads * ((n.W + 63) / 64);
-                kt.grid = (int)std::min<long long>((long long)m.sm_count * 8, kt.total_tiles);
-                kt.flops = 0;
-                kt.bytes = 2.0 * 2 * (double)n.N * n.W * n.C;
-                kt.attn.total_tiles = kt.total_tiles;
-                m.kernels.push_back(kt);
+                kn.name = n.name + ".vt";
                 kn.type = KernelType::AttentionTc;
+                kn.threads = attention_tc_threads();
                 q.total_tiles = n.N * n.heads * ((n.W + 127) / 128);
                 kn.total_tiles = q.total_tiles;
                 kn.grid = (int)std::min<long long>((long long)m.sm_count * 2, q.total_tiles);
@@ -916,11 +983,15 @@ int finalize_model(gpx_model &m) {
                      n.op == Op::MaxPool ? 0 : (n.count_pad ? 3 : 1), -1, n.scale, n.shift, n.act);
             continue;
         }
-        const Storage &w = m.storages[n.weight];
+        if (n.fused_into_other) continue;
+        const bool fused = n.fused_w >= 0;
+        const Storage &w = m.storages[fused ? n.fused_w : n.weight];
+        const float *const bias_ptr = m.storages[fused ? n.fused_b : n.bias].dptr;
         const int n_kw = n.kw ? n.kw : n.k;
-        const double flops = 2.0 * n.N * n.H * n.W * (double)n.k * n_kw * src.C * n.C;
-        const double bytes = 4.0 * ((double)src.N * src.H * src.W * src.C + (double)n.k * n_kw * src.C * n.C +
-                                    (double)n.N * n.H * n.W * n.C * (n.residual >= 0 ? 2 : 1));
+        const int n_C = fused ? 3 * n.C : n.C;  // output channels of the kernel
+        const double flops = 2.0 * n.N * n.H * n.W * (double)n.k * n_kw * src.C * n_C;
+        const double bytes = 4.0 * ((double)src.N * src.H * src.W * src.C + (double)n.k * n_kw * src.C * n_C +
+                                    (double)n.N * n.H * n.W * n_C * (n.residual >= 0 ? 2 : 1));
         if (!n.tensor_core) {
             Kernel kn;
             kn.name = n.name;
@@ -1093,7 +1164,7 @@ int finalize_model(gpx_model &m) {
             il = make_layout(n.N, 1, 1, eff_cin, ACT_PLAIN);
         }
         const bool head = out.kind == Storage::OutputF32;
-        const int cout_st = head ? n.C : stored_c(m, n);  // output channels as stored
+        const int cout_st = head ? n.C : (fused ? n_C : stored_c(m, n));  // output channels as stored
         int bn = (cout_st % 128 == 0 || head) ? 128 : 64;
         {
             // Few output tiles (batch 1, late stages): narrower column tiles expose more CTAs.
@@ -1137,7 +1208,7 @@ int finalize_model(gpx_model &m) {
         p.tiles_n = (cout_st + bn - 1) / bn;
         p.cout_valid = cout_st;
         p.relu = n.act;
-        p.bias = m.storages[n.bias].dptr;
+        p.bias = bias_ptr;
         if (n.residual >= 0) {
             const Storage &r = m.storages[m.nodes[n.residual].storage];
             p.res_hi = r.hi;
@@ -1148,9 +1219,10 @@ int finalize_model(gpx_model &m) {
             p.out_f32 = out.dptr;
             p.out = make_layout(n.N, n.H, n.W, n.C, ACT_PLAIN);
         } else {
-            p.out_hi = out.hi;
-            p.out_lo = out.lo;
-            p.out = out.layout;
+            const Storage &dst = fused ? m.storages[n.fused_out] : out;
+            p.out_hi = dst.hi;
+            p.out_lo = dst.lo;
+            p.out = dst.layout;
         }
         // The epilogue moves 32 bytes per access: 16-channel granularity of rows and slices.
         GPX_REQUIRE(head || (out.layout.C % 16 == 0 && out.ch_off % 16 == 0), GPX_FAIL,
@@ -1349,8 +1421,10 @@ static int storage_set(gpx_model *m, Storage &s, const void *host, size_t len, c
                             if (s.s2d) off = (size_t)o * K + (size_t)(h >> 1) * 64 + (size_t)(w >> 1) * 16 + (((h & 1) << 1) | (w & 1)) * I + i;
                             host_put(planes, s.plane_elems, off, v, fmt);
                         }
-            GPX_CUDA(cudaMemcpyAsync(s.hi, planes.data(), planes.size() * sizeof(bf16_bits),
-                                     cudaMemcpyHostToDevice, st));
+            // (the two planes are neighbours unless they are rows of a fused weight)
+            for (size_t pl = 0; pl < plane_count(fmt); ++pl)
+                GPX_CUDA(cudaMemcpyAsync(pl ? s.lo : s.hi, planes.data() + pl * s.plane_elems, s.plane_elems * sizeof(bf16_bits),
+                                         cudaMemcpyHostToDevice, st));
             GPX_CUDA(cudaStreamSynchronize(st));
         }
         return GPX_SUCC;
@@ -1369,7 +1443,7 @@ static int storage_set(gpx_model *m, Storage &s, const void *host, size_t len, c
             for (int c = 0; c < C; ++c)
                 for (int h = 0; h < l.H; ++h)
                     for (int w = 0; w < l.W; ++w) {
-                        float v = src[(((size_t)n * C + c) * l.H + h) * l.W + w];
+                        float v = s.token_major ? src[((size_t)n * l.W + w) * C + c] : src[(((size_t)n * C + c) * l.H + h) * l.W + w];
                         size_t off = (size_t)layout_row(l, n, h, w) * l.C + s.ch_off + c;
                         host_put(pl, par.plane_elems, off, v, l.fmt);
                     }
@@ -1450,10 +1524,10 @@ static int storage_get(gpx_model *m, Storage &s, void *host, size_t len, cudaStr
                              cudaMemcpyDeviceToHost, st));
     GPX_CUDA(cudaStreamSynchronize(st));
     if (s.token_major) {
-        // [N][S][C]: the stored rows in order
-        const size_t total = (size_t)l.N * l.W * l.C;
-        for (size_t i = 0; i < total; ++i)
-            dst[i] = host_take(planes, s.plane_elems, i, l.fmt);
+        // [N][S][C]: the stored rows in order (of a slice, its columns of them)
+        const size_t rows = (size_t)l.N * l.W, C = (size_t)s.dims[1];
+        for (size_t r = 0; r < rows; ++r)
+            for (size_t c = 0; c < C; ++c) dst[r * C + c] = host_take(planes, s.plane_elems, r * l.C + coff + c, l.fmt);
         return GPX_SUCC;
     }
     for (int n = 0; n < l.N; ++n)
@@ -1525,8 +1599,9 @@ int gpx_model_open(const char *name, const gpx_model_opts *opts, gpx_model **out
 int gpx_model_close(gpx_model *m) {
     if (!m) return GPX_SUCC;
     for (auto &s : m->storages) {
-        if (s.dptr) cudaFree(s.dptr);
-        if (s.hi && s.parent < 0) cudaFree(s.hi);  // lo lives in the same allocation; slices own nothing
+        if (s.dptr && !(s.borrowed && s.kind == Storage::Vec)) cudaFree(s.dptr);
+        // lo lives in the same allocation; slices and rows of fused weights own nothing
+        if (s.hi && s.parent < 0 && !s.borrowed) cudaFree(s.hi);
     }
     if (m->identity) cudaFree(m->identity);
     for (void *ptr : m->scratch) cudaFree(ptr);

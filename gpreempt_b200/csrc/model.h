@@ -51,6 +51,7 @@ struct Storage {
     bool token_major = false;        // activations of sequence models: canonical [N][S][C]
     int parent = -1;                 // ActSplit: this tensor is a channel slice of that storage
     int ch_off = 0;                  //   starting at this stored channel (concatenation by placement)
+    bool borrowed = false;           // Weight planes / Vec: rows of a fused storage, which owns the memory
     int affine_node = -1;            // ActSplit: output of that Affine node, formed by its only consumer as it
                                      //   loads its operand; nothing is stored (get computes it)
 };
@@ -82,10 +83,15 @@ struct Node {
     int Cs = 0;                    // stored output channels (C padded to 64 when the model pads)
     int in_c = 0;                  // channels of the input that are read (0 = all): a prefix of a Buffer
     int scale = -1, shift = -1;    // Affine, or a pooling node that normalises its input: Vec storages
+    // Projections of one attention layer that share their input run as one product of three times the
+    // columns: the first one's kernel computes all (weight, bias and output storages of the whole),
+    // the others have none.
+    int fused_w = -1, fused_b = -1, fused_out = -1;
+    bool fused_into_other = false;
     bool fused_affine = false;     // Affine applied by the consuming convolution: no kernel of its own
 };
 
-enum class KernelType { ConvSimt, Cgemm, Pool, Im2col, SplitK, LayerNorm, Attention, DwConv, AttentionTc, TransposeV, Stencil, DenseRows, GraphWl };
+enum class KernelType { ConvSimt, Cgemm, Pool, Im2col, SplitK, LayerNorm, Attention, DwConv, AttentionTc, Stencil, DenseRows, GraphWl };
 
 struct Kernel {
     std::string name;

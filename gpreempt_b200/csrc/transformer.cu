@@ -303,7 +303,7 @@ attention_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             if ((d >> 4) == part) mine[d & 15] = v * inv;
         }
         if (qvalid) {
-            const size_t off = ((size_t)b * p.S + qrow) * p.ld + col + part * 16;
+            const size_t off = ((size_t)b * p.S + qrow) * p.ld_out + col + part * 16;
 #pragma unroll
             for (int v = 0; v < 2; ++v) {
                 float x[8];
