@@ -159,10 +159,38 @@ class PreemptWord:
             self.handle = ctypes.c_void_p()
 
 
-class BlpContext:
+class _Resettable:
+    """A device context whose reset is enqueued, not waited for: copies on the default stream come
+    behind it by themselves, a kernel on another stream is told to wait for its event (`order`).
+    Waiting on the host for each reset was most of a small launch (17 us ahead of a 5 us kernel)."""
+
+    def __init__(self):
+        self._ready = ctypes.c_void_p()
+        self._ordered = None  # stream the last reset is already ordered with
+
+    def _enqueue_reset(self, entry) -> None:
+        check(entry(self.buf.ptr, ctypes.byref(self._ready)))
+        self._ordered = None
+
+    def order(self, stream) -> None:
+        """Orders later work on `stream` behind the last reset."""
+        key = getattr(stream, "value", stream) or 0
+        if self._ready and key and key != self._ordered:  # (the default stream needs no telling)
+            check(B.load().gpx_stream_wait_event(stream, self._ready))
+            self._ordered = key
+
+    def free(self) -> None:
+        if self._ready:
+            B.load().gpx_event_destroy(self._ready)
+            self._ready = ctypes.c_void_p()
+        self.buf.free()
+
+
+class BlpContext(_Resettable):
     """Device-side stop index, tile cursor and trace slots for one stand-alone kernel."""
 
     def __init__(self, word: PreemptWord | None, kernel_id: int = 0, trace: bool = True):
+        super().__init__()
         self.buf = DeviceBuffer(256)
         self.word = word
         self.kernel_id = kernel_id
@@ -170,15 +198,7 @@ class BlpContext:
         self.reset()
 
     def reset(self) -> None:
-        init = np.zeros(64, np.int32)
-        init[0] = -1  # stop index
-        init[1] = 0   # cursor
-        t = init[16:32].view(np.uint64)
-        t[0] = np.iinfo(np.uint64).max
-        t[1] = 0
-        t[2] = np.iinfo(np.uint64).max
-        t[3] = 0
-        self.buf.upload(init)
+        self._enqueue_reset(B.load().gpx_blp_ctx_reset)
 
     def rearm(self) -> None:
         """Clears the stop index only (cursor and trace are kept), as getStopPoint does."""
@@ -195,15 +215,20 @@ class BlpContext:
         return {"stop_index": int(raw[0]), "cursor": int(raw[1]), "t_start": int(t[0]),
                 "t_end": int(t[1]), "t_seen": int(t[2]), "tiles_run": int(t[3])}
 
-    def free(self) -> None:
-        self.buf.free()
+
+def _blp_for(blp: BlpContext | None, stream):
+    """The launch argument for `blp`, with `stream` ordered behind its last reset."""
+    if blp is None:
+        return None
+    blp.order(stream)
+    return ctypes.byref(blp.struct())
 
 
 def axpy(a: float, x: DeviceBuffer, y: DeviceBuffer, n: int, blp: BlpContext | None = None,
          stream=None, tile_elems: int = 0) -> None:
-    s = blp.struct() if blp is not None else None
-    check(B.load().gpx_axpy_f32(ctypes.c_float(a), x.ptr, y.ptr, n, tile_elems,
-                                ctypes.byref(s) if s is not None else None, _h(stream)))
+    h = _h(stream)
+    s = _blp_for(blp, h)
+    check(B.load().gpx_axpy_f32(a, x.ptr, y.ptr, n, tile_elems, s, h))
 
 
 def axpy_tiles(n: int, tile_elems: int = 0) -> int:
@@ -212,42 +237,39 @@ def axpy_tiles(n: int, tile_elems: int = 0) -> int:
     return t.value
 
 
-class GemmContext:
+class GemmContext(_Resettable):
     """Progress slots and accumulator spill area of the preemptible GEMM (zeroed = fresh)."""
 
     def __init__(self):
+        super().__init__()
         n = ctypes.c_size_t()
         check(B.load().gpx_gemm_ctx_bytes(ctypes.byref(n)))
         self.buf = DeviceBuffer(n.value)
         self.buf.zero()
 
     def reset(self) -> None:
-        self.buf.zero()
+        self._enqueue_reset(B.load().gpx_gemm_ctx_reset)
 
     def status(self) -> tuple[int, int]:
         err, cta = ctypes.c_int(), ctypes.c_int()
         check(B.load().gpx_gemm_status(self.buf.ptr, ctypes.byref(err), ctypes.byref(cta)))
         return err.value, cta.value
 
-    def free(self) -> None:
-        self.buf.free()
-
 
 def gemm_bf16(a: DeviceBuffer, b: DeviceBuffer, c: DeviceBuffer, m: int, n: int, k: int,
               ctx: GemmContext, blp: BlpContext | None = None, stream=None) -> None:
     """C[m][n] = A[m][k] x B[n][k]^T, bf16 in/out, fp32 accumulation on tcgen05."""
-    s = blp.struct() if blp is not None else None
-    check(B.load().gpx_gemm_bf16(a.ptr, b.ptr, c.ptr, m, n, k, ctx.buf.ptr,
-                                 ctypes.byref(s) if s is not None else None, _h(stream)))
+    h = _h(stream)
+    ctx.order(h)
+    check(B.load().gpx_gemm_bf16(a.ptr, b.ptr, c.ptr, m, n, k, ctx.buf.ptr, _blp_for(blp, h), h))
 
 
 def gemm_bf16_static(a: DeviceBuffer, b: DeviceBuffer, c: DeviceBuffer, m: int, n: int, k: int,
                      resume: bool = False, blp: BlpContext | None = None, stream=None) -> None:
     """The same GEMM with its scratch in the library's static device array: nothing is allocated
     by the call.  For callers that cannot allocate device memory; at most 64 output tiles."""
-    s = blp.struct() if blp is not None else None
-    check(B.load().gpx_gemm_bf16_static(a.ptr, b.ptr, c.ptr, m, n, k, int(resume),
-                                        ctypes.byref(s) if s is not None else None, _h(stream)))
+    h = _h(stream)
+    check(B.load().gpx_gemm_bf16_static(a.ptr, b.ptr, c.ptr, m, n, k, int(resume), _blp_for(blp, h), h))
 
 
 def gemm_static_status() -> tuple[int, int]:

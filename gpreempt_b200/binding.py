@@ -86,6 +86,7 @@ _SIGS = {
     "gpx_event_record": [vp, vp],
     "gpx_event_sync": [vp],
     "gpx_event_elapsed_ms": [vp, vp, P(ctypes.c_float)],
+    "gpx_stream_wait_event": [vp, vp],
     "gpx_set_priority": [ci],
     "gpx_word_create": [P(vp), ci],
     "gpx_word_destroy": [vp],
@@ -97,8 +98,10 @@ _SIGS = {
     "gpx_noop_launch": [vp],
     "gpx_axpy_f32": [ctypes.c_float, vp, vp, sz, sz, P(Blp), vp],
     "gpx_axpy_tiles": [sz, sz, P(ci)],
+    "gpx_blp_ctx_reset": [vp, P(vp)],
     "gpx_gemm_bf16": [vp, vp, vp, ci, ci, ci, vp, P(Blp), vp],
     "gpx_gemm_ctx_bytes": [P(sz)],
+    "gpx_gemm_ctx_reset": [vp, P(vp)],
     "gpx_gemm_tiles": [ci, ci, P(ci)],
     "gpx_gemm_status": [vp, P(ci), P(ci)],
     "gpx_gemm_bf16_static": [vp, vp, vp, ci, ci, ci, ci, P(Blp), vp],

@@ -81,6 +81,9 @@ axpy_f32_kernel(float a, const float *__restrict__ x, float *__restrict__ y, siz
         for (size_t i = begin + n4 * 4 + threadIdx.x; i < end; i += kAxpyThreads)
             y[i] = fmaf(a, x[i], y[i]);
         ++iter;
+        // With a CTA for every tile each runs one: asking for another would be two round trips to L2 at
+        // the end of a kernel that has lasted about four.
+        if (blp.total_tiles <= (int)gridDim.x) break;
         if (dynamic) __syncthreads();  // s_tile is rewritten by thread 0 in the next round
     }
     if (threadIdx.x == 0) trace_end(blp, iter);

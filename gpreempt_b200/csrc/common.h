@@ -52,6 +52,10 @@ inline uint64_t now_ns() {
 
 inline cudaStream_t as_stream(gpx_stream s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// Records *ready (created without timing on first use) behind what was enqueued on the legacy default
+// stream so far.
+int record_ready(gpx_event *ready);
+
 // Device properties cached by gpx_init for the current device.
 struct DeviceInfo {
     int device = -1;

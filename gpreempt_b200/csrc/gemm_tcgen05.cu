@@ -448,6 +448,12 @@ int gpx_gemm_ctx_bytes(size_t *bytes) {
     return GPX_SUCC;
 }
 
+int gpx_gemm_ctx_reset(void *ctx, gpx_event *ready) {
+    GPX_REQUIRE(ctx, GPX_FAIL, "ctx is NULL");
+    GPX_CUDA(cudaMemsetAsync(ctx, 0, kSpillOffset, nullptr));
+    return record_ready(ready);
+}
+
 int gpx_gemm_tiles(int M, int N, int *tiles) {
     GPX_REQUIRE(tiles, GPX_FAIL, "tiles is NULL");
     GPX_REQUIRE(M > 0 && N > 0 && M % kBM == 0 && N % kBN == 0, GPX_OUT_OF_RANGE,

@@ -101,6 +101,17 @@ __global__ void gpx_ping_kernel(const int *flag, unsigned long long *seen,
 
 namespace gpx {
 
+int record_ready(gpx_event *ready) {
+    if (!ready) return GPX_SUCC;
+    if (!*ready) {
+        cudaEvent_t e;
+        GPX_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        *ready = e;
+    }
+    GPX_CUDA(cudaEventRecord((cudaEvent_t)*ready, nullptr));
+    return GPX_SUCC;
+}
+
 int ClockProbe::init() {
     GPX_CUDA(cudaHostAlloc((void **)&flag, 64, cudaHostAllocMapped));
     GPX_CUDA(cudaHostAlloc((void **)&seen, 64, cudaHostAllocMapped));
@@ -323,6 +334,24 @@ int gpx_event_sync(gpx_event e) {
 int gpx_event_elapsed_ms(gpx_event start, gpx_event stop, float *ms) {
     GPX_CUDA(cudaEventElapsedTime(ms, (cudaEvent_t)start, (cudaEvent_t)stop));
     return GPX_SUCC;
+}
+
+int gpx_stream_wait_event(gpx_stream s, gpx_event e) {
+    GPX_REQUIRE(e, GPX_FAIL, "event is NULL");
+    GPX_CUDA(cudaStreamWaitEvent(as_stream(s), (cudaEvent_t)e, 0));
+    return GPX_SUCC;
+}
+
+int gpx_blp_ctx_reset(void *ctx, gpx_event *ready) {
+    GPX_REQUIRE(ctx, GPX_FAIL, "ctx is NULL");
+    static const struct {
+        int32_t head[16];
+        uint64_t trace[4];
+        int32_t tail[40];
+    } init = {{-1, 0}, {~0ull, 0, ~0ull, 0}, {0}};
+    static_assert(sizeof(init) == 256, "context layout");
+    GPX_CUDA(cudaMemcpyAsync(ctx, &init, sizeof(init), cudaMemcpyHostToDevice, nullptr));
+    return record_ready(ready);
 }
 
 // ---- preempt word ---------------------------------------------------------------------------

@@ -79,6 +79,8 @@ int gpx_event_destroy(gpx_event e);
 int gpx_event_record(gpx_event e, gpx_stream s);
 int gpx_event_sync(gpx_event e);
 int gpx_event_elapsed_ms(gpx_event start, gpx_event stop, float *ms);
+/* Work enqueued on `s` after the call waits for `e` (GPUStreamWaitEvent). */
+int gpx_stream_wait_event(gpx_stream s, gpx_event e);
 
 /* set_priority(NvContext, int), include/gpreempt.h:169-173 and src/gpreempt.cpp:61-72.  The
  * reference sets the channel-group timeslice of the calling thread's context by RM ioctl
@@ -145,6 +147,11 @@ typedef struct gpx_blp {
  * with the same cursor resumes exactly after the last claimed tile. */
 int gpx_axpy_f32(float a, const void *x, void *y, size_t n, size_t tile_elems,
                  const gpx_blp *blp, gpx_stream s);
+/* Puts a 256-byte context of one stand-alone kernel back to its initial state: stop index -1 at byte
+ * 0, cursor 0 at byte 4, trace slots {~0, 0, ~0, 0} at byte 64.  Asynchronous: it runs on the legacy
+ * default stream, behind which *ready is recorded (created if it is NULL; gpx_event_destroy); work
+ * on a non-blocking stream is ordered behind it by gpx_stream_wait_event. */
+int gpx_blp_ctx_reset(void *ctx, gpx_event *ready);
 /* Number of tiles gpx_axpy_f32 splits n elements into. */
 int gpx_axpy_tiles(size_t n, size_t tile_elems, int *tiles);
 
@@ -158,6 +165,9 @@ int gpx_axpy_tiles(size_t n, size_t tile_elems, int *tiles);
 int gpx_gemm_bf16(const void *A, const void *B, void *C, int M, int N, int K, void *ctx,
                   const gpx_blp *blp, gpx_stream s);
 int gpx_gemm_ctx_bytes(size_t *bytes);
+/* Makes a used context fresh again (its header and progress slots; the spill area needs no clearing).
+ * Asynchronous, with *ready as in gpx_blp_ctx_reset. */
+int gpx_gemm_ctx_reset(void *ctx, gpx_event *ready);
 int gpx_gemm_tiles(int M, int N, int *tiles);
 /* Blocking read of the context header: *error is 0, or the code of the bounded wait that
  * gave up inside the kernel (the kernel then returned early and C is incomplete). */
