@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <thread>
 #include <vector>
 
 namespace gpx {
@@ -200,6 +201,90 @@ __device__ __forceinline__ void pagerank_pair(const GraphWlParams &p, unsigned v
     }
 }
 
+// One tile of the packed form.  What bounds a pass over the lists in adj is the gather: neighbours of a
+// vertex are ~16 ids apart, so the 32 reads of one instruction touch ~16 lines of L1, one a cycle, and
+// 10 M edges are 43 k cycles an SM where the 41 MB of ids are 6 us from L2.  Here the window of deltas a
+// tile can reach is copied to shared memory once (12 KB for 64 vertices of a band of 1 500) and gathered
+// there (~3.5 conflicting banks an access); ids are half as wide and a lane gets eight of them with
+// one load.  Every lane adds the same edges in the same order as in pagerank_vertex and the same tree
+// adds the lanes, so both forms give the same bits.
+template <int K>
+struct IdPack;
+template <> struct IdPack<8> { typedef uint4 type; };
+template <> struct IdPack<4> { typedef uint2 type; };
+template <> struct IdPack<2> { typedef unsigned type; };
+template <> struct IdPack<1> { typedef unsigned short type; };
+
+template <int K>
+__device__ __forceinline__ float gather_pack(const typename IdPack<K>::type &q, const float *win, float s) {
+    const unsigned short *id = reinterpret_cast<const unsigned short *>(&q);
+    float d[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) d[k] = win[id[k]];
+#pragma unroll
+    for (int k = 0; k < K; ++k) s += d[k];
+    return s;
+}
+
+template <int K>
+__device__ __forceinline__ void pagerank_packed_tile(const GraphWlParams &p, int tile, float *win) {
+    typedef typename IdPack<K>::type Pack;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const float *dold = reinterpret_cast<const float *>((p.iter & 1) ? p.d1 : p.d0);
+    float *dnew = reinterpret_cast<float *>((p.iter & 1) ? p.d0 : p.d1);
+    float *value = reinterpret_cast<float *>(p.a), *residual = reinterpret_cast<float *>(p.b);
+    const Pack *packed = reinterpret_cast<const Pack *>(p.packed) + lane;
+    const int per_warp = p.tile_verts / (kGwThreads / 32);
+    const unsigned v = (unsigned)tile * p.tile_verts + wid * per_warp + lane;  // the vertex this lane updates
+    const bool mine = lane < per_warp && v < p.n;
+    unsigned b = 0, e = 0;
+    if (mine) {
+        b = p.blk[v];
+        e = p.blk[v + 1];
+    }
+    const uint2 w = p.win[tile];
+    for (unsigned i = threadIdx.x; i < w.y; i += kGwThreads) win[i] = dold[w.x + i];
+    if (threadIdx.x == 0) win[w.y] = 0.f;
+    float left = 0.f, val = 0.f, deg = 1.f;
+    if (mine) {
+        left = residual[v];
+        val = value[v];
+        deg = (float)p.outdeg[v];
+    }
+    __syncthreads();
+    float sum = 0.f;
+#pragma unroll 1
+    for (int j = 0; j < per_warp; j += 2) {  // two lists at a time (a missing one has no blocks)
+        const unsigned b0 = __shfl_sync(0xffffffffu, b, j), e0 = __shfl_sync(0xffffffffu, e, j);
+        const unsigned b1 = __shfl_sync(0xffffffffu, b, j + 1), e1 = __shfl_sync(0xffffffffu, e, j + 1);
+        float s0 = 0.f, s1 = 0.f;
+        unsigned i0 = b0, i1 = b1;
+        while (i0 < e0 && i1 < e1) {
+            const Pack q0 = packed[(size_t)i0++ * 32], q1 = packed[(size_t)i1++ * 32];
+            s0 = gather_pack<K>(q0, win, s0);
+            s1 = gather_pack<K>(q1, win, s1);
+        }
+        for (; i0 < e0; ++i0) s0 = gather_pack<K>(packed[(size_t)i0 * 32], win, s0);
+        for (; i1 < e1; ++i1) s1 = gather_pack<K>(packed[(size_t)i1 * 32], win, s1);
+        s0 = warp_sum(s0);
+        s1 = warp_sum(s1);
+        if (lane == j) sum = s0;
+        if (lane == j + 1) sum = s1;
+    }
+    if (mine) {
+        const float r = left + sum;
+        if (r > p.tol) {
+            value[v] = val + r;
+            dnew[v] = r * p.alpha / deg;
+            residual[v] = 0.f;
+            p.active[p.iter + 1] = 1;
+        } else {
+            residual[v] = r;
+            dnew[v] = 0.f;
+        }
+    }
+}
+
 // One tile of an edge pass: p.tile_verts neighbouring vertices, an eighth of them per warp.  The
 // first lanes of a warp fetch, for its vertices at once, whether the vertex takes part and where its
 // edge list lies; the warp then walks the lists one after another (PageRank: two at a time).  Neighbouring vertices of a
@@ -298,10 +383,13 @@ __device__ __forceinline__ void init_tile(const GraphWlParams &p, int tile) {
     }
 }
 
-template <int ALGO, int PHASE>
-__global__ void __launch_bounds__(kGwThreads)
+// PACK: PageRank's packed form (ids per lane and block), 0 = edge lists.  The packed form runs a tile per
+// CTA at the size it was measured at, and six CTAs per SM keep all of them resident.
+template <int ALGO, int PHASE, int PACK = 0>
+__global__ void __launch_bounds__(kGwThreads, PACK ? 6 : 1)
 graphwl_kernel(const __grid_constant__ GraphWlParams p, BlpArgs blp) {
     pdl_enter();
+    extern __shared__ float s_win[];
     __shared__ int s_tile;
     const bool dynamic = blp.preempted != nullptr;
     if (PHASE != GW_INIT && p.active[p.iter] == 0) {
@@ -344,7 +432,12 @@ graphwl_kernel(const __grid_constant__ GraphWlParams p, BlpArgs blp) {
         }
         if (tile < 0) break;
         if (PHASE == GW_INIT) init_tile(p, tile);
-        if (PHASE == GW_EDGES) edge_tile<ALGO>(p, tile);
+        if constexpr (PACK != 0) {
+            pagerank_packed_tile<PACK>(p, tile, s_win);
+            __syncthreads();  // the window is the next tile's
+        } else if (PHASE == GW_EDGES) {
+            edge_tile<ALGO>(p, tile);
+        }
         if (PHASE == GW_VERTICES) found |= vertex_tile<ALGO>(p, tile);
         ++iter;
         if (dynamic) __syncthreads();
@@ -357,6 +450,10 @@ graphwl_kernel(const __grid_constant__ GraphWlParams p, BlpArgs blp) {
 
 typedef void (*GraphKernel)(const GraphWlParams, BlpArgs);
 
+size_t window_bytes(const GraphWlParams &p) {
+    return p.phase == GW_EDGES && p.pack ? (size_t)(p.win_max + 1) * sizeof(float) : 0;
+}
+
 GraphKernel pick_kernel(const GraphWlParams &p) {
     if (p.phase == GW_INIT) return graphwl_kernel<GW_BFS, GW_INIT>;
     if (p.phase == GW_VERTICES) return p.algo == GW_SSSP ? graphwl_kernel<GW_SSSP, GW_VERTICES> : graphwl_kernel<GW_CC, GW_VERTICES>;
@@ -364,6 +461,13 @@ GraphKernel pick_kernel(const GraphWlParams &p) {
         case GW_BFS: return graphwl_kernel<GW_BFS, GW_EDGES>;
         case GW_SSSP: return graphwl_kernel<GW_SSSP, GW_EDGES>;
         case GW_CC: return graphwl_kernel<GW_CC, GW_EDGES>;
+        default: break;
+    }
+    switch (p.pack) {
+        case 8: return graphwl_kernel<GW_PAGERANK, GW_EDGES, 8>;
+        case 4: return graphwl_kernel<GW_PAGERANK, GW_EDGES, 4>;
+        case 2: return graphwl_kernel<GW_PAGERANK, GW_EDGES, 2>;
+        case 1: return graphwl_kernel<GW_PAGERANK, GW_EDGES, 1>;
         default: return graphwl_kernel<GW_PAGERANK, GW_EDGES>;
     }
 }
@@ -443,6 +547,57 @@ void transpose(const HostGraph &g, std::vector<unsigned long long> &trow, std::v
         for (unsigned long long i = g.row[u]; i < g.row[u + 1]; ++i) tadj[at[g.adj[i]]++] = (unsigned)u;
 }
 
+// PageRank's packed in-edge lists (GraphWlParams::packed), if every tile of `tile_verts` vertices reads
+// ids that lie within one window; false otherwise.
+bool pack_lists(const std::vector<unsigned long long> &trow, const std::vector<unsigned> &tadj, uint64_t n, int tile_verts,
+                int &pack, std::vector<uint16_t> &packed, std::vector<unsigned> &blk, std::vector<uint2> &win, int &win_max) {
+    const uint64_t tiles = (n + tile_verts - 1) / tile_verts;
+    win.resize(tiles);
+    win_max = 0;
+    for (uint64_t t = 0; t < tiles; ++t) {
+        unsigned lo = kGwInfinity, hi = 0;
+        for (uint64_t v = t * tile_verts; v < std::min<uint64_t>(n, (t + 1) * tile_verts); ++v)
+            if (trow[v] < trow[v + 1]) {  // sources ascend
+                lo = std::min(lo, tadj[trow[v]]);
+                hi = std::max(hi, tadj[trow[v + 1] - 1]);
+            }
+        const unsigned len = lo == kGwInfinity ? 0 : hi - lo + 1;
+        if (len > (unsigned)kGwWindowMax) return false;
+        win[t] = make_uint2(len ? lo : 0, len);
+        win_max = std::max(win_max, (int)len);
+    }
+    // ids per lane and block: the block next above the average list
+    const uint64_t avg = tadj.size() / n;
+    pack = avg > 128 ? 8 : (avg > 64 ? 4 : (avg > 32 ? 2 : 1));
+    const unsigned per = 32u * (unsigned)pack;
+    blk.resize(n + 1);
+    uint64_t blocks = 0;
+    for (uint64_t v = 0; v < n; ++v) {
+        blk[v] = (unsigned)blocks;
+        blocks += (trow[v + 1] - trow[v] + per - 1) / per;
+    }
+    if (blocks >= (1ull << 32)) return false;
+    blk[n] = (unsigned)blocks;
+    packed.resize(blocks * per);
+    auto fill = [&](uint64_t t0, uint64_t t1) {
+        for (uint64_t v = t0 * tile_verts; v < std::min<uint64_t>(n, t1 * tile_verts); ++v) {
+            const uint2 w = win[v / tile_verts];
+            const uint64_t deg = trow[v + 1] - trow[v];
+            for (uint64_t b = blk[v]; b < blk[v + 1]; ++b)
+                for (unsigned l = 0; l < 32; ++l)
+                    for (int k = 0; k < pack; ++k) {
+                        const uint64_t i = (b - blk[v]) * per + (uint64_t)k * 32 + l;
+                        packed[(b * 32 + l) * pack + k] = (uint16_t)(i < deg ? tadj[trow[v] + i] - w.x : w.y);
+                    }
+        }
+    };
+    std::vector<std::thread> pool;
+    const uint64_t workers = std::min<uint64_t>(8, std::max<uint64_t>(1, tiles / 64));
+    for (uint64_t i = 0; i < workers; ++i) pool.emplace_back(fill, tiles * i / workers, tiles * (i + 1) / workers);
+    for (auto &th : pool) th.join();
+    return true;
+}
+
 template <typename T>
 int to_device(gpx_model &m, const std::vector<T> &host, T **out) {
     T *d = nullptr;
@@ -497,7 +652,7 @@ bool split_name(const std::string &name, int &algo, std::string &path) {
 
 int graphwl_grid(const GraphWlParams &p, int total_tiles, int sm_count) {
     int blocks = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, pick_kernel(p), kGwThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, pick_kernel(p), kGwThreads, window_bytes(p));
     if (blocks < 1) blocks = 1;
     long long grid = (long long)blocks * sm_count;
     if (grid > total_tiles) grid = total_tiles;
@@ -505,7 +660,7 @@ int graphwl_grid(const GraphWlParams &p, int total_tiles, int sm_count) {
 }
 
 cudaError_t graphwl_launch(const GraphWlParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(pick_kernel(p), grid, kGwThreads, 0, s, p, blp);
+    launch_layer(pick_kernel(p), grid, kGwThreads, window_bytes(p), s, p, blp);
     return cudaGetLastError();
 }
 
@@ -564,8 +719,25 @@ int build_graph_workload(gpx_model &m, const std::string &name, const gpx_model_
         std::vector<unsigned> tadj, outdeg(g.n);
         transpose(g, trow, tadj);
         for (uint64_t v = 0; v < g.n; ++v) outdeg[v] = (unsigned)(g.row[v + 1] - g.row[v]);
-        GPX_TRY(to_device(m, trow, &row));
-        GPX_TRY(to_device(m, tadj, &adj));
+        std::vector<uint16_t> packed;
+        std::vector<unsigned> blk;
+        std::vector<uint2> win;
+        if (g.n && pack_lists(trow, tadj, g.n, kGwPackedTileVerts, base.pack, packed, blk, win, base.win_max)) {
+            base.tile_verts = kGwPackedTileVerts;
+            uint16_t *d_packed = nullptr;
+            unsigned *d_blk = nullptr;
+            uint2 *d_win = nullptr;
+            GPX_TRY(to_device(m, packed, &d_packed));
+            GPX_TRY(to_device(m, blk, &d_blk));
+            GPX_TRY(to_device(m, win, &d_win));
+            base.packed = d_packed;
+            base.blk = d_blk;
+            base.win = d_win;
+        } else {
+            base.pack = 0;
+            GPX_TRY(to_device(m, trow, &row));
+            GPX_TRY(to_device(m, tadj, &adj));
+        }
         unsigned *deg = nullptr;
         GPX_TRY(to_device(m, outdeg, &deg));
         base.outdeg = deg;

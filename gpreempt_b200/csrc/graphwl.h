@@ -18,6 +18,7 @@
 // point in a handful of iterations.
 #pragma once
 
+#include <cstdint>
 #include <cuda_runtime.h>
 #include <string>
 
@@ -39,6 +40,9 @@ constexpr int kGwThreads = 256;
 constexpr int kGwEdgeTileVertsMax = 256;  // vertices per tile of an edge pass at most (32 per warp)
 constexpr int kGwVertexTileVerts = 1024;  // vertices per tile of a per-vertex pass
 constexpr int kGwMaxIters = 16384;        // iteration flags a graph workload has: no run may need more rounds
+// (packed PageRank: 52 804 vertices are 826 tiles, fewer than six CTAs on each of 148 SMs)
+constexpr int kGwPackedTileVerts = 64;
+constexpr int kGwWindowMax = 12287;       // floats of a tile's window (with the zero behind it: 48 KiB)
 constexpr unsigned kGwInfinity = 0xFFFFFFFFu;  // MYINFINITY, include/workloads/graphcompute.h:14
 
 struct GraphWlParams {
@@ -57,6 +61,15 @@ struct GraphWlParams {
     unsigned *d0, *d1;    // pagerank: delta, read from d<iter & 1>, written to the other
     unsigned char *f0;    // sssp: label (the frontier)
     int *active;          // [kGwMaxIters + 1]: active[i] != 0 <=> iteration i has work
+    // pagerank, where the in-neighbours of every tile lie within kGwWindowMax ids (a graph ordered for
+    // locality): the ids as 16-bit offsets into the tile's window, in blocks of 32 x pack (lane l of a
+    // block holds edges l, l + 32, ... next to one another), padded with the window's length, where the
+    // shared-memory copy of the window holds a zero.
+    int pack;                       // ids a lane holds per block: 1, 2, 4 or 8; 0 = lists in adj
+    const uint16_t *packed;
+    const unsigned *blk;            // [n + 1] first block of every vertex
+    const uint2 *win;               // [tiles] first id and length of the window
+    int win_max;                    // longest window
     float alpha, tol;     // pagerank (0.85, 0.001: include/workloads/graphcompute.h:85-86)
 };
 
