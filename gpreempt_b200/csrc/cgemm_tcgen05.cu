@@ -94,6 +94,7 @@ struct CgemmControl {
     unsigned long long full[8];
     unsigned long long empty[8];
     unsigned long long ready[8];       // the A tile of a stage has been through its affine map
+    unsigned long long landed;         // cluster reduction: every peer's partial rows have arrived
     unsigned long long tmem_full[2];   // one per accumulator buffer
     unsigned long long tmem_empty[2];
     uint32_t tmem_base;
@@ -216,6 +217,10 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             mbar_init(smem_u32(&ctl->tmem_empty[b]), 1);
             ctl->epi_kind[b] = CEPI_COMPLETE;
             ctl->epi_k_done[b] = 0;
+        }
+        if (in_cluster) {
+            mbar_init(smem_u32(&ctl->landed), 1);
+            mbar_arrive_expect_tx(smem_u32(&ctl->landed), kCBM * (BN + 4) * 4);
         }
         ctl->abort_flag = 0;
         ctl->epi_go = 0;
@@ -740,7 +745,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         const int row = quarter * 32 + lane;
         const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
         const bool leader = threadIdx.x == 64;
-        uint32_t push = 0;  // where the partial sums of this thread's row go (cluster reduction)
         if (in_cluster) {
             // What the finishing step needs, ahead of the products: destination, bias, residual.
             const SplitKParams &fin = p.fin;
@@ -778,11 +782,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 }
                 fin_live[i] = live;
             }
-            const int rows_per = kCBM / p.k_splits;
-            const int owner = row / rows_per;
-            push = cluster_map_shared(smem_base + (uint32_t)(nst * Cfg::kStageBytes) +
-                                          (uint32_t)(((int)cluster_ctarank() * rows_per + row - owner * rows_per) * (BN + 4)) * 4,
-                                      (uint32_t)owner);
         }
         uint32_t v[32];
         if (first_k > 0) {
@@ -944,13 +943,13 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     e_tmem += t_p1 - t_p0;
 #endif
                     if (in_cluster) {
-                        // Split K inside a cluster: the raw fp32 sum of this row and K range goes
-                        // straight into the shared memory of the CTA that finishes the row (its last
-                        // ring stages: [split][row of its share][BN + 4 floats], the 4 spreading the
-                        // rows of a warp over the banks).
+                        // Split K inside a cluster: the raw fp32 sum of this K range stays in this CTA's
+                        // ring (idle: such a launch runs one tile) until the tile is complete; rows are
+                        // 16 bytes longer than BN floats so that the rows of a warp spread over the banks.
+                        float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(smem) + row * (BN + 4) + c);
 #pragma unroll
                         for (int j = 0; j < CH / 4; ++j)
-                            st_shared_cluster_f4(push + (uint32_t)(c + 4 * j) * 4, make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]));
+                            dst[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
                         continue;
                     }
                     if (partial) {
@@ -1030,7 +1029,21 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 ++it;
                 ++tiles_done;
                 seg_k0 = 0;
-                if (in_cluster) break;  // a CTA of such a launch runs one tile
+                if (in_cluster) {
+                    // Every share of rows goes to the CTA that finishes it as one bulk copy (landing area:
+                    // [split][row of the share][BN + 4 floats] in that CTA's last ring stages).
+                    fence_proxy_async();
+                    asm volatile("bar.sync 1, %0;" ::"n"(kCEpiThreads) : "memory");
+                    const int owner = (int)threadIdx.x - 64;
+                    if (owner < p.k_splits) {
+                        const uint32_t share = (uint32_t)(kCBM / p.k_splits * (BN + 4) * 4);
+                        bulk_copy_to_cluster(cluster_map_shared(smem_base + (uint32_t)(nst * Cfg::kStageBytes) + cluster_ctarank() * share, (uint32_t)owner),
+                                             smem_base + (uint32_t)owner * share, share,
+                                             cluster_map_shared(smem_u32(&ctl->landed), (uint32_t)owner));
+                        bulk_copies_done();  // the source is this CTA's memory: it stays until they are through
+                    }
+                    break;
+                }
                 tc_fence_before_sync();
                 TCK(t_b0);
                 asm volatile("bar.sync 1, %0;" ::"n"(kCEpiThreads) : "memory");
@@ -1081,26 +1094,19 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     if constexpr (BN != 64) {
         __syncthreads();
     } else if (in_cluster) {
-        // Every CTA of the cluster has pushed its partial rows to their owners (or has failed and set
-        // the error word: all waits above are bounded, so every thread gets here).  This CTA finishes
-        // rows [rank, rank+1) * 128/S of the output block from its own shared memory: the S partial
-        // rows are added in split order from zero, exactly as splitk_finish_kernel adds the workspace
+        // This CTA finishes rows [rank, rank+1) * 128/S of the output block from its own shared memory
+        // once every CTA of the cluster has copied its partial rows of them there: the S partial rows
+        // are added in split order from zero, exactly as splitk_finish_kernel adds the workspace
         // rows, then bias, residual, activation, store.  Where the rows go, the bias and the residual
         // were fetched before the products were waited for.  Nothing is read from a peer, so a CTA may
-        // exit when it is done.
-        // (Pulling the rows from the peers after the barrier, one split at a time, and a second
-        // barrier before the exit made this step 4 us long; BERT-base b1: 7.4 us per projection.)
-#ifdef GPX_CGEMM_TIMING
-        if (threadIdx.x == 64) TADD(18, clock64() - t_begin);
-#endif
-        cluster_arrive();
-#ifdef GPX_CGEMM_TIMING
-        if (threadIdx.x == 64) TADD(19, clock64() - t_begin);
-#endif
-        cluster_wait();
-#ifdef GPX_CGEMM_TIMING
-        if (threadIdx.x == 64) TADD(20, clock64() - t_begin);
-#endif
+        // exit when it is done.  (Pulling the rows from the peers after a cluster barrier, one split at
+        // a time, and a second barrier before the exit made this step 4 us long, BERT-base b1 7.4 us per
+        // projection; storing them to the peers element by element, 2 us.)  A CTA that failed waits
+        // here as well, so that no copy finds its memory gone.
+        if (warp >= 2 && warp < kCPollWarp) {
+            volatile int never = 0;
+            if (!mbar_wait(smem_u32(&ctl->landed), 0, &never, kCWaitLimitNs + kCWaitLimitNs / 2)) fail(601);
+        }
         if (warp >= 2 && warp < kCPollWarp) {
             const float *land = reinterpret_cast<const float *>(smem + nst * Cfg::kStageBytes);
             const SplitKParams &fin = p.fin;

@@ -10,6 +10,8 @@
 // does not depend on which CTA runs a tile: preempt + resume is bit-identical.
 #include "layers.cuh"
 
+#include <algorithm>
+
 namespace gpx {
 
 constexpr int kConvThreads = 256;
@@ -281,12 +283,49 @@ __device__ __forceinline__ void pool_store8(const PoolParams &p, size_t off, con
     planes_store8(p.out_hi, p.out_lo, off, p.out.fmt, x);
 }
 
+// The tiles of a CTA.  Under the preemptible schedule a claim is two dependent round trips to L2 (the
+// word, the cursor), more than a tile of 256 vectors takes; ahead(), called once the loads of a tile are
+// on their way, claims the following tile while they travel.  The tile so claimed is run whatever the
+// word says by then: a CTA leaves after at most two tiles instead of one, a few microseconds.
+struct TileClaims {
+    const BlpArgs &blp;
+    const bool dynamic;
+    int &s_tile;  // shared
+    int iter = 0, upcoming = 0;
+    bool asked = false;
+    __device__ __forceinline__ TileClaims(const BlpArgs &b, bool d, int &s) : blp(b), dynamic(d), s_tile(s) {}
+    __device__ __forceinline__ int first() {
+        if (!dynamic) return blp_claim(blp, 0);
+        if (threadIdx.x == 0) s_tile = blp_claim(blp, 0);
+        __syncthreads();
+        return s_tile;
+    }
+    __device__ __forceinline__ void ahead() {
+        if (dynamic && threadIdx.x == 0 && !asked) {
+            upcoming = blp_claim(blp, iter + 1);
+            asked = true;
+        }
+    }
+    __device__ __forceinline__ int next() {
+        ++iter;
+        if (!dynamic) return blp_claim(blp, iter);
+        __syncthreads();  // every thread has read this round's number
+        if (threadIdx.x == 0) s_tile = asked ? upcoming : blp_claim(blp, iter);
+        asked = false;
+        __syncthreads();
+        return s_tile;
+    }
+    __device__ __forceinline__ int done() const { return iter; }
+};
+
 // Max / average pooling, or a strided copy, over split-plane activations; eight channels (one
 // 16-byte vector per plane) per thread-iteration.  A tile is tile_elems consecutive output
 // vectors in (n, ho, wo, c/8) order.
-// kMax3 selects the 3x3 max-pooling instance, which keeps nine taps in registers and so runs at a
-// lower occupancy than the other modes want.
-template <bool kMax3>
+// K = 3: 3x3 max pooling, K = 2: 2x2 pooling of either kind, both without an affine map: the K*K taps are
+// fetched before any is converted, so a thread waits for memory once instead of K*K times (VGG's first
+// 2x2 pooling, 16 images fp16: 61 us one tap at a time).  K = 0: every other mode, at a higher occupancy
+// than the taps in registers allow.
+template <int K>
 __global__ void __launch_bounds__(kPoolThreads)
 pool_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
     pdl_enter();
@@ -298,20 +337,11 @@ pool_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
     const int Ho = p.out.H, Wo = p.out.W;
     const int H = p.in.l.H, W = p.in.l.W;
     const unsigned total = (unsigned)p.out.N * Ho * Wo * C8;  // < 2^31, checked when the model is built
-    int iter = 0;
-    for (;;) {
-        int tile;
-        if (dynamic) {
-            if (threadIdx.x == 0) s_tile = blp_claim(blp, iter);
-            __syncthreads();
-            tile = s_tile;
-        } else {
-            tile = blp_claim(blp, iter);
-        }
-        if (tile < 0) break;
+    TileClaims claims(blp, dynamic, s_tile);
+    for (int tile = claims.first(); tile >= 0; tile = claims.next()) {
         const unsigned begin = (unsigned)tile * p.tile_elems;
         const unsigned end = begin + p.tile_elems < total ? begin + p.tile_elems : total;
-        if (p.mode == 1 && p.k * p.k >= 16) {
+        if (K == 0 && p.mode == 1 && p.k * p.k >= 16) {
             // Large averaging window (global average pool): one warp per output vector, lanes
             // take taps lane, lane+32, ...; a fixed shuffle tree adds the lane sums, so the
             // result is the same on every run.
@@ -353,8 +383,6 @@ pool_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
                     pool_store8(p, (size_t)layout_row(p.out, n, ho, wo) * Cout + c8 * 8, acc);
                 }
             }
-            ++iter;
-            if (dynamic) __syncthreads();
             continue;
         }
         for (unsigned e = begin + threadIdx.x; e < end; e += kPoolThreads) {
@@ -366,30 +394,38 @@ pool_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
             int n = (int)(t / Ho);
             float acc[8];
             const bool readable = c8 * 8 < p.in_valid;
-            if (kMax3 && readable) {
-                // 3x3 max pooling: the nine taps are fetched before any is converted, so a thread
-                // waits for memory once instead of nine times.
-                uint4 ra[9], rb[9];
-                bool ok[9];
+            if (K != 0 && readable) {
+                constexpr int T = K ? K * K : 1, KW = K ? K : 1;
+                uint4 ra[T], rb[T];
+                bool ok[T];
                 const int fmt = p.in.l.fmt;
+                const bool is_max = K == 3 || p.mode == 0;
 #pragma unroll
-                for (int t9 = 0; t9 < 9; ++t9) {
-                    const int hi = ho * p.stride - p.pad + t9 / 3, wi = wo * p.stride - p.pad + t9 % 3;
+                for (int t9 = 0; t9 < T; ++t9) {
+                    const int hi = ho * p.stride - p.pad + t9 / KW, wi = wo * p.stride - p.pad + t9 % KW;
                     ok[t9] = hi >= 0 && hi < H && wi >= 0 && wi < W;
                     ra[t9] = rb[t9] = make_uint4(0, 0, 0, 0);
                     if (ok[t9])
                         planes_fetch8(p.in.hi, p.in.lo, (size_t)layout_row(p.in.l, n, hi, wi) * Cin + c8 * 8, fmt,
                                       ra[t9], rb[t9]);
                 }
+                claims.ahead();
+                int cnt = 0;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[j] = -INFINITY;
+                for (int j = 0; j < 8; ++j) acc[j] = is_max ? -INFINITY : 0.f;
 #pragma unroll
-                for (int t9 = 0; t9 < 9; ++t9) {
+                for (int t9 = 0; t9 < T; ++t9) {
                     if (!ok[t9]) continue;
+                    ++cnt;
                     float x[8];
                     planes_decode8(ra[t9], rb[t9], fmt, x);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[j] = fmaxf(acc[j], x[j]);
+                    for (int j = 0; j < 8; ++j) acc[j] = is_max ? fmaxf(acc[j], x[j]) : acc[j] + x[j];
+                }
+                if (!is_max) {
+                    const float inv = 1.0f / (float)(p.mode == 1 ? cnt : T);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc[j] *= inv;
                 }
                 pool_store8(p, (size_t)layout_row(p.out, n, ho, wo) * Cout + c8 * 8, acc);
                 continue;
@@ -424,10 +460,8 @@ pool_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
             }
             pool_store8(p, (size_t)layout_row(p.out, n, ho, wo) * Cout + c8 * 8, acc);
         }
-        ++iter;
-        if (dynamic) __syncthreads();
     }
-    if (threadIdx.x == 0) trace_end(blp, iter);
+    if (threadIdx.x == 0) trace_end(blp, claims.done());
 }
 
 // Patch matrix for the tensor-core GEMM: one thread-iteration writes eight consecutive columns
@@ -785,8 +819,97 @@ dense_rows_kernel(const __grid_constant__ DenseRowsParams p, BlpArgs blp) {
     if (threadIdx.x == 0) trace_end(blp, iter);
 }
 
+// The same layer with short rows (at most kDenseShortK input elements: the classifiers behind a global
+// average pool): one warp per output column, eight columns per tile.  Such a row is a few KB, the matrix
+// a few MB that L2 keeps; what costs is the chain of steps, so the columns of a tile run side by side
+// instead of one after the other with a block-wide sum each, and every lane's part of its first row is
+// requested ahead of the wait for the predecessor (weights are never written by a kernel).
+// ResNet-50's 2048 -> 1000 at batch 1: 12.5 us with the whole CTA on one row.
+constexpr int kDenseShortVec = kDenseShortK / 256;  // 16-byte vectors per lane and plane
+
+__global__ void __launch_bounds__(kPoolThreads)
+dense_short_kernel(const __grid_constant__ DenseRowsParams p, BlpArgs blp) {
+    extern __shared__ float s_a[];  // [M][K] input rows
+    __shared__ int s_tile;
+    const bool dynamic = blp.preempted != nullptr;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    uint4 wa[kDenseShortVec], wb[kDenseShortVec];
+    auto fetch = [&](int n) {
+#pragma unroll
+        for (int u = 0; u < kDenseShortVec; ++u)
+            if (n < p.cout && (u * 32 + lane) * 8 < p.K)
+                planes_fetch8(p.w_hi, p.w_lo, (size_t)n * p.w_ld + (u * 32 + lane) * 8, p.fmt, wa[u], wb[u]);
+    };
+    int have = dynamic ? -1 : (int)blockIdx.x;  // tile whose weights are in wa, wb
+    if (have >= 0) fetch(have * 8 + wid);
+    pdl_enter();
+    if (threadIdx.x == 0) trace_begin(blp);
+    for (int v = threadIdx.x; v < p.M * (p.K / 8); v += kPoolThreads) {
+        const int m = v / (p.K / 8), k = (v - m * (p.K / 8)) * 8;
+        float a[8];
+        planes_load8(p.a_hi, p.a_lo, (size_t)m * p.a_ld + k, p.fmt, a);
+        float4 *dst = reinterpret_cast<float4 *>(s_a + m * p.K + k);
+        dst[0] = make_float4(a[0], a[1], a[2], a[3]);
+        dst[1] = make_float4(a[4], a[5], a[6], a[7]);
+    }
+    __syncthreads();
+    int iter = 0;
+    for (;;) {
+        int tile;
+        if (dynamic) {
+            __syncthreads();
+            if (threadIdx.x == 0) s_tile = blp_claim(blp, iter);
+            __syncthreads();
+            tile = s_tile;
+        } else {
+            tile = blp_claim(blp, iter);
+        }
+        if (tile < 0) break;
+        const int n = tile * 8 + wid;
+        if (tile != have) fetch(n);
+        have = -1;
+        if (n < p.cout) {
+            float w[kDenseShortVec][8];
+#pragma unroll
+            for (int u = 0; u < kDenseShortVec; ++u) planes_decode8(wa[u], wb[u], p.fmt, w[u]);
+            const float bias = p.bias ? __ldg(p.bias + n) : 0.f;
+#pragma unroll 1
+            for (int m = 0; m < p.M; ++m) {
+                float acc = 0.f;
+#pragma unroll
+                for (int u = 0; u < kDenseShortVec; ++u) {
+                    const int k0 = (u * 32 + lane) * 8;
+                    if (k0 < p.K) {
+                        const float4 *a4 = reinterpret_cast<const float4 *>(s_a + m * p.K + k0);
+                        const float4 x = a4[0], y = a4[1];
+                        const float a[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) acc = fmaf(a[j], w[u][j], acc);
+                    }
+                }
+#pragma unroll
+                for (int sh = 16; sh >= 1; sh >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, sh);
+                if (lane == 0) {
+                    const float v = apply_act(acc + bias, p.relu);
+                    if (p.out_f32)
+                        p.out_f32[(size_t)m * p.cout + n] = v;
+                    else
+                        planes_store1(p.out_hi, p.out_lo, (size_t)m * p.out_ld + n, p.fmt, v);
+                }
+            }
+        }
+        ++iter;
+    }
+    if (threadIdx.x == 0) trace_end(blp, iter);
+}
+
 cudaError_t dense_rows_launch(const DenseRowsParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(dense_rows_kernel, grid, kPoolThreads, 0, s, p, blp);
+    // (input rows of the short form in the default 48 KB of shared memory)
+    const size_t rows = (size_t)p.M * p.K * sizeof(float);
+    if (p.K <= kDenseShortK && rows <= 48 * 1024)
+        launch_layer(dense_short_kernel, grid, kPoolThreads, rows, s, p, blp);
+    else
+        launch_layer(dense_rows_kernel, grid, kPoolThreads, 0, s, p, blp);
     return cudaGetLastError();
 }
 
@@ -795,82 +918,150 @@ cudaError_t splitk_launch(const SplitKParams &p, int grid, const BlpArgs &blp, c
     return cudaGetLastError();
 }
 
+// Output pixel and channel group of element e of a tensor walked in (n, ho, wo, c / 8) order.
+struct PixelAt {
+    int c8, wo, ho, n;
+};
+__device__ __forceinline__ PixelAt pixel_at(unsigned e, int C8, int Wo, int Ho) {
+    PixelAt a;
+    a.c8 = (int)(e % C8);
+    unsigned t = e / C8;
+    a.wo = (int)(t % Wo);
+    t /= Wo;
+    a.ho = (int)(t % Ho);
+    a.n = (int)(t / Ho);
+    return a;
+}
+
 // Depthwise convolution: one thread-iteration produces eight channels of one output pixel,
 // taps walked in (fh, fw) order with one FFMA each, so the result is independent of the tiling.
-__global__ void __launch_bounds__(kPoolThreads)
+// At batch 1 this is latency: the filter (never written by a kernel) is copied to shared memory ahead
+// of the wait for the predecessor, the element a thread starts with is decoded there too, and the nine
+// taps of a 3x3 filter are requested before any is used (one round trip instead of nine;
+// MobileNetV2 b1: 4.4 us a layer before).
+//
+// BATCH: taps of a 3x3 filter in flight at once.  Nine where the tensor is a tile or two per CTA; three
+// (a filter row) in larger tensors, which want the occupancy the registers of nine take
+// (56x56x144, 64 images fp16: 190 us with nine); 0 for other filter sizes.
+template <int BATCH, bool TWO>
+__global__ void __launch_bounds__(kPoolThreads, BATCH == 9 ? (TWO ? 2 : 3) : (TWO ? 4 : 5))
 dwconv_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
-    pdl_enter();
+    extern __shared__ float s_w[];  // [k * k][C], or nothing where it does not fit
     __shared__ int s_tile;
     const bool dynamic = blp.preempted != nullptr;
-    if (threadIdx.x == 0) trace_begin(blp);
     const int C = p.out.C;
     const int C8 = C / 8;
     const int Ho = p.out.H, Wo = p.out.W;
     const int H = p.in.l.H, W = p.in.l.W;
     const unsigned total = (unsigned)p.out.N * Ho * Wo * C8;  // < 2^31, checked when the model is built
-    int iter = 0;
-    for (;;) {
-        int tile;
-        if (dynamic) {
-            if (threadIdx.x == 0) s_tile = blp_claim(blp, iter);
-            __syncthreads();
-            tile = s_tile;
-        } else {
-            tile = blp_claim(blp, iter);
-        }
-        if (tile < 0) break;
+    const float *wts = p.w;
+    if (p.w_in_smem) {
+        const int n4 = p.k * p.k * C / 4;
+        for (int i = threadIdx.x; i < n4; i += kPoolThreads)
+            reinterpret_cast<float4 *>(s_w)[i] = __ldg(reinterpret_cast<const float4 *>(p.w) + i);
+        wts = s_w;
+    }
+    unsigned known = (unsigned)blockIdx.x * p.tile_elems + threadIdx.x;  // decoded ahead for a static schedule
+    PixelAt ahead = pixel_at(known < total ? known : 0, C8, Wo, Ho);
+    __syncthreads();
+    pdl_enter();
+    if (threadIdx.x == 0) trace_begin(blp);
+    TileClaims claims(blp, dynamic, s_tile);
+    for (int tile = claims.first(); tile >= 0; tile = claims.next()) {
         const unsigned begin = (unsigned)tile * p.tile_elems;
         const unsigned end = begin + p.tile_elems < total ? begin + p.tile_elems : total;
         for (unsigned e = begin + threadIdx.x; e < end; e += kPoolThreads) {
-            int c8 = (int)(e % C8);
-            unsigned t = e / C8;
-            int wo = (int)(t % Wo);
-            t /= Wo;
-            int ho = (int)(t % Ho);
-            int n = (int)(t / Ho);
+            const PixelAt at = e == known ? ahead : pixel_at(e, C8, Wo, Ho);
+            const int c0 = at.c8 * 8, h0 = at.ho * p.stride - p.pad, w0 = at.wo * p.stride - p.pad;
             float acc[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-            for (int fh = 0; fh < p.k; ++fh) {
-                int hi = ho * p.stride - p.pad + fh;
-                if (hi < 0 || hi >= H) continue;
-                for (int fw = 0; fw < p.k; ++fw) {
-                    int wi = wo * p.stride - p.pad + fw;
-                    if (wi < 0 || wi >= W) continue;
-                    size_t off = (size_t)layout_row(p.in.l, n, hi, wi) * p.in.l.C + c8 * 8;
-                    float x[8];
-                    planes_load8(p.in.hi, p.in.lo, off, p.in.l.fmt, x);
-                    const float4 *wv = reinterpret_cast<const float4 *>(p.w + (size_t)(fh * p.k + fw) * C + c8 * 8);
-                    float4 w0 = wv[0], w1 = wv[1];
-                    const float wf[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+            auto tap = [&](const float (&x)[8], int t) {
+                const float4 *wv = reinterpret_cast<const float4 *>(wts + (size_t)t * C + c0);
+                const float4 a = wv[0], b = wv[1];
+                const float wf[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[j] = fmaf(x[j], wf[j], acc[j]);
+                for (int j = 0; j < 8; ++j) acc[j] = fmaf(x[j], wf[j], acc[j]);
+            };
+            if (BATCH != 0) {
+                constexpr int B = BATCH ? BATCH : 1;
+                const int fmt = TWO ? (int)PF_SPLIT : p.in.l.fmt;
+#pragma unroll
+                for (int t0 = 0; t0 < 9; t0 += B) {
+                    uint4 ra[B], rb[TWO ? B : 1];
+                    bool ok[B];
+#pragma unroll
+                    for (int t = 0; t < B; ++t) {
+                        const int hi = h0 + (t0 + t) / 3, wi = w0 + (t0 + t) % 3;
+                        ok[t] = hi >= 0 && hi < H && wi >= 0 && wi < W;
+                        if (ok[t])
+                            planes_fetch8(p.in.hi, p.in.lo, (size_t)layout_row(p.in.l, at.n, hi, wi) * p.in.l.C + c0, fmt, ra[t],
+                                          rb[TWO ? t : 0]);
+                    }
+                    if (t0 == 0) claims.ahead();
+#pragma unroll
+                    for (int t = 0; t < B; ++t) {
+                        if (!ok[t]) continue;
+                        float x[8];
+                        planes_decode8(ra[t], rb[TWO ? t : 0], fmt, x);
+                        tap(x, t0 + t);
+                    }
+                }
+            } else {
+                for (int fh = 0; fh < p.k; ++fh) {
+                    const int hi = h0 + fh;
+                    if (hi < 0 || hi >= H) continue;
+                    for (int fw = 0; fw < p.k; ++fw) {
+                        const int wi = w0 + fw;
+                        if (wi < 0 || wi >= W) continue;
+                        float x[8];
+                        planes_load8(p.in.hi, p.in.lo, (size_t)layout_row(p.in.l, at.n, hi, wi) * p.in.l.C + c0, p.in.l.fmt, x);
+                        tap(x, fh * p.k + fw);
+                    }
                 }
             }
             if (p.bias) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[j] += p.bias[c8 * 8 + j];
+                const float4 *b4 = reinterpret_cast<const float4 *>(p.bias + c0);
+                const float4 a = __ldg(b4), b = __ldg(b4 + 1);
+                acc[0] += a.x, acc[1] += a.y, acc[2] += a.z, acc[3] += a.w;
+                acc[4] += b.x, acc[5] += b.y, acc[6] += b.z, acc[7] += b.w;
             }
             apply_act_n(acc, p.act);
-            planes_store8(p.out_hi, p.out_lo, (size_t)layout_row(p.out, n, ho, wo) * C + c8 * 8, p.out.fmt, acc);
+            planes_store8(p.out_hi, p.out_lo, (size_t)layout_row(p.out, at.n, at.ho, at.wo) * C + c0, p.out.fmt, acc);
         }
-        ++iter;
-        if (dynamic) __syncthreads();
     }
-    if (threadIdx.x == 0) trace_end(blp, iter);
+    if (threadIdx.x == 0) trace_end(blp, claims.done());
+}
+
+static auto dwconv_instance(const DwConvParams &p) {
+    const bool two = p.out.fmt == PF_SPLIT;
+    if (p.k != 3) return two ? dwconv_kernel<0, true> : dwconv_kernel<0, false>;
+    if (p.small) return two ? dwconv_kernel<9, true> : dwconv_kernel<9, false>;
+    return two ? dwconv_kernel<3, true> : dwconv_kernel<3, false>;
+}
+static size_t dwconv_smem(const DwConvParams &p) { return p.w_in_smem ? (size_t)p.k * p.k * p.out.C * sizeof(float) : 0; }
+
+int dwconv_grid(const DwConvParams &p, int sm_count) {
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dwconv_instance(p), kPoolThreads, dwconv_smem(p));
+    return (int)std::min<long long>((long long)sm_count * std::max(per_sm, 1), p.total_tiles);
 }
 
 cudaError_t dwconv_launch(const DwConvParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(dwconv_kernel, grid, kPoolThreads, 0, s, p, blp);
+    launch_layer(dwconv_instance(p), grid, kPoolThreads, dwconv_smem(p), s, p, blp);
     return cudaGetLastError();
 }
 
-static bool pool_is_max3(const PoolParams &p) { return p.mode == 0 && p.k == 3 && !p.scale; }
+static int pool_taps(const PoolParams &p) {
+    if (p.scale) return 0;
+    if (p.mode == 0 && p.k == 3) return 3;
+    return p.mode != 2 && p.k == 2 ? 2 : 0;
+}
 
 int pool_grid(const PoolParams &p, int sm_count) {
     int per_sm = 8;
-    if (pool_is_max3(p)) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pool_kernel<true>, kPoolThreads, 0);
+    if (const int t = pool_taps(p)) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, t == 3 ? pool_kernel<3> : pool_kernel<2>, kPoolThreads, 0);
         if (per_sm < 1) per_sm = 1;
     }
     long long grid = (long long)sm_count * per_sm;
@@ -880,10 +1071,8 @@ int pool_grid(const PoolParams &p, int sm_count) {
 }
 
 cudaError_t pool_launch(const PoolParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    if (pool_is_max3(p))
-        launch_layer(pool_kernel<true>, grid, kPoolThreads, 0, s, p, blp);
-    else
-        launch_layer(pool_kernel<false>, grid, kPoolThreads, 0, s, p, blp);
+    const int t = pool_taps(p);
+    launch_layer(t == 3 ? pool_kernel<3> : (t == 2 ? pool_kernel<2> : pool_kernel<0>), grid, kPoolThreads, 0, s, p, blp);
     return cudaGetLastError();
 }
 

@@ -197,6 +197,7 @@ struct DenseRowsParams {
     int relu, fmt;
     int total_tiles;               // eight output columns per tile
 };
+constexpr int kDenseShortK = 2048;  // rows up to this length: one warp per column
 cudaError_t dense_rows_launch(const DenseRowsParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
 
 // Patch matrix of a convolution whose input has too few channels for the tensor-core kernel
@@ -276,9 +277,12 @@ struct DwConvParams {
     bf16_bits *out_hi, *out_lo;
     ActLayout out;
     int k, stride, pad, act;
+    int small;           // 1: at most a tile or two per CTA: latency, not occupancy
+    int w_in_smem;       // 1: the filter is copied to shared memory once per CTA
     int total_tiles;
     int tile_elems;      // output 8-channel vectors per tile
 };
+int dwconv_grid(const DwConvParams &p, int sm_count);
 cudaError_t dwconv_launch(const DwConvParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
 
 enum ConvTile { CONV_TILE_128 = 0, CONV_TILE_64 = 1, CONV_TILE_32 = 2 };

@@ -830,12 +830,17 @@ int finalize_model(gpx_model &m) {
             long long total = (long long)dst.layout.N * dst.layout.H * dst.layout.W * (p.channels / 8);
             // Enough tiles to fill the GPU even when the tensor is small (global average pool).
             long long want_tiles = 4LL * m.sm_count;
+            // 3x3 max pooling keeps two CTAs on an SM: a small tensor is cut so that each runs one tile
+            // (ResNet's at batch 1: 392 tiles of 64 vectors on 296 CTAs were two rounds).
+            const bool max3 = mode == 0 && k == 3 && scale < 0;
+            const long long max3_tile = (total + 2LL * m.sm_count - 1) / (2LL * m.sm_count);
             // the cap is per unit of work: a copy or an affine map reads one tap per vector, a 3x3
             // pooling nine
             const int taps_per_vec = mode == 2 ? 1 : k * k;
             const long long tile_cap = std::min<long long>(2048, std::max<long long>(kMaxTileVectors, 9 * kMaxTileVectors / taps_per_vec));
             p.tile_elems = (int)std::max<long long>(mode == 1 && k * k >= 16 ? 8 : 64,
                                                     std::min<long long>(tile_cap, total / want_tiles / 8 * 8));
+            if (max3 && max3_tile <= 256) p.tile_elems = (int)std::max<long long>(32, (max3_tile + 7) / 8 * 8);
             p.total_tiles = (int)((total + p.tile_elems - 1) / p.tile_elems);
             kn.total_tiles = p.total_tiles;
             kn.grid = pool_grid(p, m.sm_count);
@@ -959,11 +964,15 @@ int finalize_model(gpx_model &m) {
             q.stride = n.stride;
             q.pad = n.pad;
             q.act = n.act;
+            // The filter goes to shared memory where that pays: with a tile or two per CTA (small
+            // batches) its latency hides behind the predecessor's tail; up to the default 48 KB.
+            q.w_in_smem = (size_t)n.k * n.k * q.out.C * sizeof(float) <= 48 * 1024 ? 1 : 0;
             long long total = (long long)n.N * n.H * n.W * (q.out.C / 8);
             q.tile_elems = (int)std::max<long long>(256, std::min<long long>(kMaxTileVectors, total / (8LL * m.sm_count) / 32 * 32));
             q.total_tiles = (int)((total + q.tile_elems - 1) / q.tile_elems);
             kn.total_tiles = q.total_tiles;
-            kn.grid = (int)std::min<long long>((long long)m.sm_count * 8, q.total_tiles);
+            q.small = q.total_tiles <= 4 * m.sm_count ? 1 : 0;
+            kn.grid = dwconv_grid(q, m.sm_count);
             kn.flops = 2.0 * n.N * n.H * n.W * (double)n.k * n.k * n.C;
             kn.bytes = 4.0 * ((double)src.N * src.H * src.W * src.C + (double)n.N * n.H * n.W * n.C);
             m.kernels.push_back(kn);

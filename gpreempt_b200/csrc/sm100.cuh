@@ -109,9 +109,17 @@ __device__ __forceinline__ uint32_t cluster_map_shared(uint32_t addr, uint32_t r
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void st_shared_cluster_f4(uint32_t addr, float4 v) {
-    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+// Bulk copy from this CTA's shared memory to `dst` in another CTA of the cluster, counted in bytes on that
+// CTA's mbarrier `bar` (both mapped by cluster_map_shared; 16-byte aligned, a multiple of 16 bytes).
+__device__ __forceinline__ void bulk_copy_to_cluster(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "r"(src), "r"(bytes), "r"(bar)
                  : "memory");
+}
+// Waits until the bulk copies this thread has issued have completed.
+__device__ __forceinline__ void bulk_copies_done() {
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // ---- tensor memory --------------------------------------------------------------------------
