@@ -3,6 +3,8 @@
 //
 //   C[M][N] (bf16) = A[M][K] (bf16) x B[N][K]^T (bf16), fp32 accumulation in tensor memory.
 //
+// Products of at least one tile per SM go to pairs of CTAs (gemm_bf16_pair_kernel, below); the rest, and
+// the variant without a context, to this form:
 // One persistent CTA per SM walks output tiles of 128 x 256 on a static schedule
 // (tile = cta + iteration * grid).  Inside a CTA three roles run concurrently:
 //   warp 0 (one lane)  TMA producer: streams 128x64 A and 256x64 B blocks (128-byte swizzle)
@@ -30,6 +32,7 @@
 #include "sm100.cuh"
 
 #include <cuda.h>
+#include <algorithm>
 #include <cuda_bf16.h>
 
 namespace gpx {
@@ -414,6 +417,399 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a,
     if (threadIdx.x == 0 && blp.trace) atomicMax(blp.trace + 1, globaltimer_ns());
 }
 
+// ---- the same product by CTA pairs -----------------------------------------------------------------
+//
+// A pair takes a 256 x 256 tile: each CTA holds its own 128 rows of A and its own 128 of the 256 rows of
+// B, one tcgen05.mma of the pair reads both halves of B from where they lie, and each CTA accumulates
+// its 128 x 256 half of the tile.  Per K block and CTA that is 32 KB of fill and 32 KB of operand reads
+// through shared memory instead of 48 + 48, six ring stages instead of four, and a third less traffic
+// from L2: the single-CTA form runs out of shared-memory bandwidth at 768 cycles a K block where the
+// products take 512.  8192^3, a call with its resets: 946 -> 863 us under the power cap.
+//
+// The even CTA leads: it alone reads the word and issues the products.  Where to stop has to be one
+// decision: the leader grants the pair's producers K blocks ahead (a limit in the shared memory of
+// each); once it has seen the word raised it grants no more, both load up to the last limit, and the
+// leader's STOP message follows.  A drain so begins at most kGrant K blocks (~2.5 us) late.
+constexpr int kPairStages = 6;
+constexpr uint32_t kPairBBytes = (kBN / 2) * kBK * 2;           // this CTA's half of the B tile
+constexpr uint32_t kPairStageBytes = kABytes + kPairBBytes;     // 32 KiB
+constexpr int kPairThreads = 224;                               // TMA, MMA, four epilogue warps, poller
+constexpr int kGrant = 8;
+
+struct PairControl {
+    unsigned long long full[kPairStages];   // the leader's: loads of both CTAs
+    unsigned long long empty[kPairStages];
+    unsigned long long tmem_full[2];
+    unsigned long long tmem_empty[2];       // the leader's: both epilogues
+    uint32_t tmem_base;
+    int stage_msg[kPairStages];
+    int epi_kind[2];                        // written by the leader in both CTAs
+    int epi_k_done[2];
+    int epi_go;
+    int abort_flag;
+    int word_up;
+    int poll_done;
+    uint32_t limit;                         // K blocks granted so far << 1 | no more will be
+};
+constexpr size_t kPairSmem = (size_t)kPairStages * kPairStageBytes + 1024 + 512;
+static_assert(sizeof(PairControl) <= 512, "control block outgrew its shared-memory budget");
+
+__global__ void __launch_bounds__(kPairThreads, 1) __cluster_dims__(2, 1, 1)
+gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, __nv_bfloat16 *C,
+                      int M, int N, int K, unsigned char *ctx, BlpArgs blp) {
+    extern __shared__ unsigned char smem_raw[];
+    uint32_t raw_addr = smem_u32(smem_raw);
+    uint32_t pad = (1024u - (raw_addr & 1023u)) & 1023u;
+    unsigned char *smem = smem_raw + pad;
+    PairControl *ctl = reinterpret_cast<PairControl *>(smem + (size_t)kPairStages * kPairStageBytes);
+    const uint32_t smem_base = smem_u32(smem);
+    volatile int *abort_flag = &ctl->abort_flag;
+    auto at_leader = [&](const void *p) { return cluster_map_shared(smem_u32(p), 0); };
+    auto at_peer = [&](const void *p) { return cluster_map_shared(smem_u32(p), 1); };
+
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    const int lane = threadIdx.x & 31;
+    const int rank = (int)cluster_ctarank();
+    const bool leads = rank == 0;
+    const int tiles_m = M / kBM, tiles_n = N / kBN;
+    const int pairs_m = (tiles_m + 1) / 2;  // (the last pair of an odd number of row blocks has an empty half)
+    const int total = pairs_m * tiles_n;
+    const int num_kb = K / kBK;
+    const int first_tile = blockIdx.x >> 1, stride = gridDim.x >> 1;
+    const bool resumable = blp.preempted != nullptr;
+
+    GemmHeader *hdr = reinterpret_cast<GemmHeader *>(ctx);
+    GemmSlot *slot = reinterpret_cast<GemmSlot *>(ctx + kSlotOffset) + blockIdx.x;
+    float *spill = reinterpret_cast<float *>(ctx + kSpillOffset + (size_t)blockIdx.x * kSpillBytesPerCta);
+    const int first_iter = slot->next_iter;
+    const int first_k = slot->k_done;
+    const int slot_grid = slot->grid;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kPairStages; ++s) {
+            mbar_init(smem_u32(&ctl->full[s]), 1);
+            mbar_init(smem_u32(&ctl->empty[s]), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&ctl->tmem_full[b]), 2);   // the commit + the issuer's own arrive
+            mbar_init(smem_u32(&ctl->tmem_empty[b]), 2);  // both CTAs' epilogues
+            ctl->epi_kind[b] = EPI_EXIT;
+            ctl->epi_k_done[b] = 0;
+        }
+        ctl->abort_flag = 0;
+        ctl->word_up = 0;
+        ctl->poll_done = 0;
+        ctl->limit = 0;
+        fence_barrier_init();
+        fence_proxy_async();
+        trace_begin(blp);
+    }
+    if (warp == 1) tmem_alloc_pair(smem_u32(&ctl->tmem_base), kTmemCols);
+    tc_fence_before_sync();
+    cluster_arrive();  // from here on either CTA may reach the other's barriers
+    cluster_wait();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = ctl->tmem_base;
+    const bool issuer = elect_one();
+
+    const bool grid_ok = slot_grid == 0 || slot_grid == (int)gridDim.x;  // (the same in both CTAs)
+    auto fail = [&](int code) {
+        *abort_flag = 1;
+        st_cluster_u32(leads ? at_peer(&ctl->abort_flag) : at_leader(&ctl->abort_flag), 1u);
+        if (atomicCAS(&hdr->error, 0, code) == 0) hdr->error_cta = blockIdx.x;
+    };
+    auto coords = [&](int tile, int &m_blk, int &n_blk) {
+        int pm;
+        tile_coords(tile, pairs_m, tiles_n, pm, n_blk);
+        m_blk = 2 * pm + rank;
+    };
+
+    if (!grid_ok) {
+        if (threadIdx.x == 0) fail(900);
+    } else if (warp == 0) {
+        // ---------------------------------------------------------------- TMA producer (both CTAs)
+        int stage = 0;
+        uint32_t phase = 0;
+        bool ok = true, stop = false;
+        uint32_t g = 0, limit = 0;  // K blocks loaded, K blocks granted
+        bool last_grant = false;
+        const volatile int *word_up = &ctl->word_up;
+        int kb = first_k;
+        for (int it = first_iter; ok && !stop; ++it, kb = 0) {
+            const int tile = first_tile + it * stride;
+            if (tile >= total) break;
+            int m_blk, n_blk;
+            coords(tile, m_blk, n_blk);
+            for (; kb < num_kb; ++kb, ++g) {
+                if (resumable) {
+                    if (leads) {
+                        if ((g & (kGrant / 2 - 1)) == 0 && !last_grant) {
+                            // (the first look goes to the word itself: nothing may run if it is up already)
+                            const bool up = __any_sync(0xffffffffu, g == 0 ? load_word(blp.preempted) : *word_up);
+                            if (up)
+                                last_grant = true;
+                            else
+                                limit = g + kGrant;
+                            if (issuer) st_cluster_u32(at_peer(&ctl->limit), limit << 1 | (last_grant ? 1u : 0u));
+                        }
+                        stop = last_grant && g == limit;
+                    } else if (g == limit) {
+                        uint32_t v = 0;
+                        const unsigned long long t0 = globaltimer_ns();
+                        for (;;) {
+                            v = __shfl_sync(0xffffffffu, ld_cluster_u32(smem_u32(&ctl->limit)), 0);
+                            if ((v >> 1) > g || (v & 1u)) break;
+                            if (__any_sync(0xffffffffu, *abort_flag != 0 || globaltimer_ns() - t0 > kWaitLimitNs)) {
+                                ok = false;
+                                break;
+                            }
+                        }
+                        if (!ok) {
+                            if (issuer) fail(103);
+                            break;
+                        }
+                        limit = v >> 1;
+                        stop = g == limit;  // only a last grant leaves it where it was
+                    }
+                    if (stop && !leads) break;
+                }
+                if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1, abort_flag, kWaitLimitNs))) {
+                    if (issuer) fail(101);
+                    ok = false;
+                    break;
+                }
+                if (stop) {
+                    if (issuer) {
+                        ctl->stage_msg[stage] = MSG_STOP;
+                        mbar_arrive(smem_u32(&ctl->full[stage]));
+                        if (blp.trace) atomicMin(blp.trace + 2, globaltimer_ns());
+                    }
+                    break;
+                }
+                if (issuer) {
+                    const uint32_t bar = at_leader(&ctl->full[stage]);
+                    const uint32_t a_dst = smem_base + stage * kPairStageBytes;
+                    if (leads) {
+                        ctl->stage_msg[stage] = MSG_DATA;
+                        mbar_arrive_expect_tx(smem_u32(&ctl->full[stage]), 2 * kPairStageBytes);
+                    }
+                    tma_load_2d_pair(a_dst, &tmap_a, bar, kb * kBK, m_blk * kBM);
+                    tma_load_2d_pair(a_dst + kABytes, &tmap_b, bar, kb * kBK, n_blk * kBN + rank * (kBN / 2));
+                }
+                __syncwarp();
+                if (++stage == kPairStages) {
+                    stage = 0;
+                    phase ^= 1;
+                }
+            }
+        }
+        if (lane == 0) *(volatile int *)&ctl->poll_done = 1;
+        __syncwarp();
+    } else if (warp == 1) {
+        // ---------------------------------------------------------------- MMA issuer (the leader)
+        if (leads) {
+            constexpr uint32_t idesc = make_idesc_bf16_f32(2 * kBM, kBN);
+            const uint64_t ring = make_smem_desc_sw128(smem_base);
+            int stage = 0;
+            uint32_t phase = 0, seg = 0;
+            int kb = first_k;
+            for (int tile = first_tile + first_iter * stride; tile < total; tile += stride, ++seg, kb = 0) {
+                const int buf = (int)(seg & 1);
+                const uint32_t acc = tmem_base + buf * kBN;
+                if (!__all_sync(0xffffffffu, mbar_wait_cluster(smem_u32(&ctl->tmem_empty[buf]), (seg >> 1) & 1, abort_flag, kWaitLimitNs))) {
+                    if (issuer) fail(202);
+                    break;
+                }
+                tc_fence_after_sync();
+                int end = EPI_COMPLETE;
+                for (; kb < num_kb; ++kb) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->full[stage]), phase, abort_flag, kWaitLimitNs))) {
+                        if (issuer) fail(201);
+                        end = -1;
+                        break;
+                    }
+                    tc_fence_after_sync();
+                    if (__any_sync(0xffffffffu, ((volatile int *)ctl->stage_msg)[stage] == MSG_STOP)) {
+                        end = EPI_PARTIAL;
+                        break;
+                    }
+                    if (issuer) {
+                        const uint64_t a = ring + (uint64_t)(stage * (kPairStageBytes >> 4));
+                        const uint64_t b = a + (kABytes >> 4);
+#pragma unroll
+                        for (int k = 0; k < kBK / kUmmaK; ++k)
+                            mma_f16_ss_pair(acc, a + 2 * k, b + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        mma_commit_pair(smem_u32(&ctl->empty[stage]));
+                    }
+                    __syncwarp();
+                    if (++stage == kPairStages) {
+                        stage = 0;
+                        phase ^= 1;
+                    }
+                }
+                if (end < 0) break;
+                if (issuer) {
+                    ctl->epi_kind[buf] = end;
+                    ctl->epi_k_done[buf] = kb;
+                    st_cluster_u32(at_peer(&ctl->epi_kind[buf]), (uint32_t)end);
+                    st_cluster_u32(at_peer(&ctl->epi_k_done[buf]), (uint32_t)kb);
+                    mma_commit_pair(smem_u32(&ctl->tmem_full[buf]));
+                    mbar_arrive(smem_u32(&ctl->tmem_full[buf]));
+                    mbar_arrive_cluster(at_peer(&ctl->tmem_full[buf]));
+                }
+                __syncwarp();
+                if (end != EPI_COMPLETE) break;
+            }
+        }
+    } else if (warp == 6) {
+        // ---------------------------------------------------------------- preempt-word poller (the leader)
+        if (resumable && leads && lane == 0) {
+            while (!*(volatile int *)&ctl->poll_done) {
+                if (load_word(blp.preempted) != 0) {
+                    *(volatile int *)&ctl->word_up = 1;
+                    break;
+                }
+                __nanosleep(100);
+            }
+        }
+        __syncwarp();
+    } else {
+        // ---------------------------------------------------------------- epilogue (4 warps, both CTAs)
+        const int quarter = warp & 3;                 // TMEM lanes this warp may access
+        const int row = quarter * 32 + lane;          // accumulator row == TMEM lane
+        const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
+        const bool leader = threadIdx.x == 64;
+        uint32_t v[32];
+        if (first_k > 0) {
+            // Resume: reload this CTA's half of the spilled accumulator into tensor memory.
+            for (int c = 0; c < kBN; c += 32) {
+                // (layout of the spill area: see the store below)
+                const uint4 *src = reinterpret_cast<const uint4 *>(spill) + (size_t)(c / 32) * 8 * 128 + row;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    uint4 q = src[j * 128];
+                    v[4 * j + 0] = q.x;
+                    v[4 * j + 1] = q.y;
+                    v[4 * j + 2] = q.z;
+                    v[4 * j + 3] = q.w;
+                }
+                tmem_st_32x32(t_lane + c, v);
+            }
+            tmem_st_wait();
+        }
+        tc_fence_before_sync();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (leader) {
+            mbar_arrive_cluster(at_leader(&ctl->tmem_empty[0]));  // a restored tile sits in buffer 0: segment 0 uses it
+            mbar_arrive_cluster(at_leader(&ctl->tmem_empty[1]));
+        }
+        int it = first_iter;
+        int seg_k0 = first_k;
+        int tiles_done = 0;
+        for (uint32_t seg = 0;; ++seg) {
+            const int tile = first_tile + it * stride;
+            if (tile >= total) {
+                if (leader) {
+                    slot->next_iter = it;
+                    slot->k_done = 0;
+                    slot->grid = gridDim.x;
+                }
+                break;
+            }
+            const int buf = (int)(seg & 1);
+            const uint32_t t_acc = t_lane + buf * kBN;
+            int m_blk, n_blk;
+            coords(tile, m_blk, n_blk);
+            if (leader) {
+                bool ok = mbar_wait_cluster(smem_u32(&ctl->tmem_full[buf]), (seg >> 1) & 1, abort_flag, kWaitLimitNs);
+                if (!ok) fail(301);
+                ctl->epi_go = ok ? 1 : 0;
+            }
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (!ctl->epi_go) break;
+            tc_fence_after_sync();
+            const int kind = ((volatile int *)ctl->epi_kind)[buf];
+            const int k_done = ((volatile int *)ctl->epi_k_done)[buf];
+            if (kind == EPI_COMPLETE) {
+                const bool mine = m_blk < tiles_m;
+                __nv_bfloat16 *crow = C + (size_t)(m_blk * kBM + row) * N + (size_t)n_blk * kBN;
+#pragma unroll 2
+                for (int c = 0; c < kBN; c += 32) {
+                    tmem_ld_32x32(t_acc + c, v);
+                    tmem_ld_wait();
+                    if (!mine) continue;
+                    uint32_t h[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+                        h[j] = *reinterpret_cast<uint32_t *>(&p);
+                    }
+                    // 32 columns are 64 contiguous bytes of this thread's row
+                    uint4 *dst = reinterpret_cast<uint4 *>(crow + c);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) dst[j] = make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]);
+                }
+                ++it;
+                seg_k0 = 0;
+                // Hand the accumulator back to the MMA issuer.
+                tc_fence_before_sync();
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (leader) {
+                    mbar_arrive_cluster(at_leader(&ctl->tmem_empty[buf]));
+                    if (mine) {
+                        ++tiles_done;
+                        if (blp.executed) atomicAdd(blp.executed, 1);
+                    }
+                }
+                continue;
+            }
+            // EPI_PARTIAL: spill the accumulator if this launch added to it, record the cursor.
+            if (k_done > seg_k0) {
+                for (int c = 0; c < kBN; c += 32) {
+                    tmem_ld_32x32(t_acc + c, v);
+                    tmem_ld_wait();
+                    // private to this kernel: one warp store writes 512 consecutive bytes
+                    uint4 *dst = reinterpret_cast<uint4 *>(spill) + (size_t)(c / 32) * 8 * 128 + row;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        dst[j * 128] = make_uint4(v[4 * j + 0], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                }
+            }
+            if (leader) {
+                slot->next_iter = it;
+                slot->k_done = k_done;
+                slot->grid = gridDim.x;
+                if (blp.stop_index) atomicCAS(blp.stop_index, -1, blp.kernel_id);
+            }
+            break;
+        }
+        if (leader && blp.trace && tiles_done) atomicAdd(blp.trace + 3, (unsigned long long)tiles_done);
+    }
+
+    // All roles of both CTAs meet here: neither may leave while the other can still arrive on its barriers,
+    // and tensor memory is released by the pair.
+    tc_fence_before_sync();
+    __syncwarp();
+    if (warp == 0 && lane == 0 && *abort_flag) {
+        for (int spin = 0; spin < 64; ++spin) __nanosleep(1000);  // loads in flight get a chance to land
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (warp == 1) {
+        tc_fence_after_sync();
+        tmem_dealloc_pair(tmem_base, kTmemCols);
+    }
+    if (threadIdx.x == 0 && blp.trace) atomicMax(blp.trace + 1, globaltimer_ns());
+}
+
+// Pairs take over where every pair of CTAs gets a tile of its own; with fewer tiles than SMs the single-CTA
+// form spreads over more of them in the same number of rounds.
+static bool gemm_by_pairs(int M, int N, int sm_count) {
+    const int tiles_m = M / kBM, tiles_n = N / kBN;
+    return tiles_m * tiles_n >= sm_count && (tiles_m % 2 == 0 || tiles_m >= 9);
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
                                   const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                                   const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -481,13 +877,16 @@ int gpx_gemm_bf16(const void *A, const void *B, void *C, int M, int N, int K, vo
                 GPX_FAIL, "A, B, C and ctx must be 16-byte aligned");
     const DeviceInfo &d = device_info();
     GPX_REQUIRE(d.device >= 0, GPX_FAIL, "gpx_init was not called");
+    const bool pairs = gemm_by_pairs(M, N, d.sm_count);
     CUtensorMap ta, tb;
     GPX_TRY(make_tmap_2d_bf16(&ta, A, (uint64_t)M, (uint64_t)K, kBM, kBK));
-    GPX_TRY(make_tmap_2d_bf16(&tb, B, (uint64_t)N, (uint64_t)K, kBN, kBK));
+    GPX_TRY(make_tmap_2d_bf16(&tb, B, (uint64_t)N, (uint64_t)K, pairs ? kBN / 2 : kBN, kBK));
     static bool attr_set[64] = {false};
     if (!attr_set[d.device]) {
         GPX_CUDA(cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
+        GPX_CUDA(cudaFuncSetAttribute(gemm_bf16_pair_kernel,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
         attr_set[d.device] = true;
     }
     BlpArgs b{};
@@ -503,8 +902,15 @@ int gpx_gemm_bf16(const void *A, const void *B, void *C, int M, int N, int K, vo
     }
     int grid = d.sm_count < kMaxGemmCtas ? d.sm_count : kMaxGemmCtas;
     if (grid > tiles) grid = tiles;
-    gemm_bf16_tcgen05_kernel<<<grid, kGemmThreads, kGemmSmem, as_stream(s)>>>(
-        ta, tb, (__nv_bfloat16 *)C, M, N, K, (unsigned char *)ctx, b);
+    if (pairs) {
+        const int pair_tiles = (M / kBM + 1) / 2 * (N / kBN);
+        grid = 2 * std::min(pair_tiles, std::min(d.sm_count, kMaxGemmCtas) / 2);
+        gemm_bf16_pair_kernel<<<grid, kPairThreads, kPairSmem, as_stream(s)>>>(ta, tb, (__nv_bfloat16 *)C, M, N, K,
+                                                                               (unsigned char *)ctx, b);
+    } else {
+        gemm_bf16_tcgen05_kernel<<<grid, kGemmThreads, kGemmSmem, as_stream(s)>>>(ta, tb, (__nv_bfloat16 *)C, M, N, K,
+                                                                                  (unsigned char *)ctx, b);
+    }
     GPX_CUDA(cudaGetLastError());
     return GPX_SUCC;
 }
