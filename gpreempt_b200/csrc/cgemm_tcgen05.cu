@@ -66,7 +66,7 @@ struct CgemmCfg {
     static constexpr uint32_t kWOff = kPlanes * kABytes;        // W (hi) tile inside a K block
     // K blocks a ring stage holds at most.  The round of one stage (barrier waits, message, commit) costs
     // either role ~300 cycles; a 64- or 128-column product of one plane takes 128 or 256, so two
-    // of them share a round, unless the affine map sets the pace (VGG-16's 64-column layer at batch 16: 168 -> see the table of cases).
+    // of them share a round, unless the affine map sets the pace (VGG-16's 64-column layer at batch 16: 168 -> 121 us).
     static constexpr int kKps = (!TWO && !AFF && BN <= 128) ? 2 : 1;
     static constexpr uint32_t kStageBytes = kKps * kKbBytes;
     static constexpr int kStages = (int)((192u * 1024u) / kStageBytes);  // 3 to 8

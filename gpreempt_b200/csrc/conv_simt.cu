@@ -904,9 +904,9 @@ dense_short_kernel(const __grid_constant__ DenseRowsParams p, BlpArgs blp) {
 }
 
 cudaError_t dense_rows_launch(const DenseRowsParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    // (input rows of the short form in the default 48 KB of shared memory)
+    // (input rows of the short form, beside its own variables, in the default 48 KB of shared memory)
     const size_t rows = (size_t)p.M * p.K * sizeof(float);
-    if (p.K <= kDenseShortK && rows <= 48 * 1024)
+    if (p.K <= kDenseShortK && rows + 256 <= 48 * 1024)
         launch_layer(dense_short_kernel, grid, kPoolThreads, rows, s, p, blp);
     else
         launch_layer(dense_rows_kernel, grid, kPoolThreads, 0, s, p, blp);
@@ -942,9 +942,9 @@ __device__ __forceinline__ PixelAt pixel_at(unsigned e, int C8, int Wo, int Ho) 
 //
 // BATCH: taps of a 3x3 filter in flight at once.  Nine where the tensor is a tile or two per CTA; three
 // (a filter row) in larger tensors, which want the occupancy the registers of nine take
-// (56x56x144, 64 images fp16: 190 us with nine); 0 for other filter sizes.
+// (56x56x144, 64 images fp16: 190 us with nine, 145 with three); 0 for other filter sizes.
 template <int BATCH, bool TWO>
-__global__ void __launch_bounds__(kPoolThreads, BATCH == 9 ? (TWO ? 2 : 3) : (TWO ? 4 : 5))
+__global__ void __launch_bounds__(kPoolThreads, BATCH == 9 ? (TWO ? 2 : 3) : 4)
 dwconv_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
     extern __shared__ float s_w[];  // [k * k][C], or nothing where it does not fit
     __shared__ int s_tile;
