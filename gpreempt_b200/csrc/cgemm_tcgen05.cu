@@ -34,14 +34,10 @@ namespace gpx {
 using namespace sm100;
 
 constexpr int kCBM = 128, kCBK = 64, kCUmmaK = 16;
-// Warp 0 feeds TMA, warp 1 issues MMAs, warps 2..9 are the epilogue, the last warp polls the preempt
-// word: kCEpiParts epilogue warps per TMEM lane quarter, each taking an equal share of the columns,
+// Warp 0 feeds TMA, warp 1 issues MMAs, warps from 2 on are the epilogue, the last warp polls the preempt
+// word: kEpiParts epilogue warps per TMEM lane quarter, each taking an equal share of the columns,
 // so that enough independent TMEM loads, conversions and stores are in flight while a tile is drained
 // (the epilogue, not the tensor pipe, bounds the small-K layers).
-constexpr int kCEpiParts = 2;                       // epilogue warps per TMEM lane quarter
-constexpr int kCEpiThreads = 128 * kCEpiParts;
-constexpr int kCPollWarp = 2 + kCEpiThreads / 32;
-constexpr int kCgemmThreads = 64 + kCEpiThreads + 32;
 constexpr int kCAffThreads = 256;  // eight more warps where the A operand goes through an affine map first
 constexpr int kCAffGroups = 2;       // groups of those warps that take K blocks in turn
 constexpr int kCAffMaxC = kCgemmMaxAffineC;
@@ -58,7 +54,10 @@ struct CgemmControlSize {
 // otherwise one 16-bit plane and one product.
 template <int BN, bool TWO, bool AFF>
 struct CgemmCfg {
-    static constexpr int kThreads = kCgemmThreads + (AFF ? kCAffThreads : 0);
+    static constexpr int kEpiParts = BN == 256 ? 4 : 2;          // epilogue warps per TMEM lane quarter
+    static constexpr int kEpiThreads = 128 * kEpiParts;
+    static constexpr int kPollWarp = 2 + kEpiThreads / 32;
+    static constexpr int kThreads = 64 + kEpiThreads + 32 + (AFF ? kCAffThreads : 0);
     static constexpr uint32_t kPlanes = TWO ? 2 : 1;
     static constexpr uint32_t kABytes = kCBM * kCBK * 2;        // one plane of A: 16 KiB
     static constexpr uint32_t kWBytes = BN * kCBK * 2;          // one plane of W
@@ -346,7 +345,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     };
 
     // Cluster reduction: what this thread finishes (eight-channel items; two of them when S = 2).
-    constexpr int kGroups = BN / 8, kFinItems = 64 * kGroups / kCEpiThreads;
+    constexpr int kGroups = BN / 8, kFinItems = 64 * kGroups / Cfg::kEpiThreads;
     bool fin_live[kFinItems] = {};
     int fin_col[kFinItems];
     size_t fin_off[kFinItems];
@@ -634,7 +633,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             TADD(12, mma_kb);
         }
 #endif
-    } else if (warp == kCPollWarp) {
+    } else if (warp == Cfg::kPollWarp) {
         // ------------------------------------------------------------------ preempt-word poller
         // A read of the word takes longer than a K block of a single-plane model: on the producer's
         // path, even one K block ahead, it set the pace of the ring.  Here one lane reads it back to
@@ -649,7 +648,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             }
         }
         __syncwarp();
-    } else if (AFF && warp > kCPollWarp) {
+    } else if (AFF && warp > Cfg::kPollWarp) {
         // ------------------------------------------------------------------ affine map of A
         // Every thread keeps one of the eight 16-byte pieces of a row (piece c of row r lies at position
         // c XOR (r mod 8), the 128-byte swizzle) and takes eight rows 16 apart: its sixteen scales and
@@ -661,8 +660,8 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         // Two groups of four warps take the K blocks in turn: a block is a chain of latencies (shared-memory
         // reads, conversions, the fence to the tensor core's proxy) that the other group's overlaps.
         constexpr int kGroupThreads = kCAffThreads / kCAffGroups;
-        const int group = (warp - kCPollWarp - 1) / (kGroupThreads / 32);
-        const int at = ((int)threadIdx.x - (kCPollWarp + 1) * 32) % kGroupThreads;
+        const int group = (warp - Cfg::kPollWarp - 1) / (kGroupThreads / 32);
+        const int at = ((int)threadIdx.x - (Cfg::kPollWarp + 1) * 32) % kGroupThreads;
         const int piece = at & 7, row = at >> 3;
         constexpr int kAffRows = kCBM * 8 / kGroupThreads;  // rows per thread
         const uint32_t off = (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4));  // (rows 16 apart: same swizzle)
@@ -738,9 +737,9 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         // ------------------------------------------------------------------ epilogue
         const int quarter = warp & 3;
         const int part = (warp - 2) >> 2;                 // which share of the columns
-        const int c_lo = part * (BN / kCEpiParts), c_hi = c_lo + BN / kCEpiParts;
+        const int c_lo = part * (BN / Cfg::kEpiParts), c_hi = c_lo + BN / Cfg::kEpiParts;
         // this warp's share of the columns of one accumulator buffer, for spill and restore
-        constexpr int kSpillCols = kBufCols / kCEpiParts;
+        constexpr int kSpillCols = kBufCols / Cfg::kEpiParts;
         const int s_lo = part * kSpillCols, s_hi = s_lo + kSpillCols;
         const int row = quarter * 32 + lane;
         const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
@@ -753,7 +752,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             const int rank = (int)cluster_ctarank();
 #pragma unroll
             for (int i = 0; i < kFinItems; ++i) {
-                const int e = (int)threadIdx.x - 64 + i * kCEpiThreads;
+                const int e = (int)threadIdx.x - 64 + i * Cfg::kEpiThreads;
                 const int lr = e / kGroups, col0 = first_tile.n_blk * BN + (e - lr * kGroups) * 8;
                 const int vrow = first_tile.m_blk * kCBM + rank * rows_share + lr;
                 bool live = lr < rows_share && vrow < fin.m_rows && col0 < fin.cout_padded;
@@ -803,7 +802,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             tmem_st_wait();
         }
         tc_fence_before_sync();
-        asm volatile("bar.sync 1, %0;" ::"n"(kCEpiThreads) : "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
         if (leader)
             for (int b = 0; b < 2; ++b) mbar_arrive(smem_u32(&ctl->tmem_empty[b]));
 
@@ -894,7 +893,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 if (!ok) fail(301);
                 ctl->epi_go = ok ? 1 : 0;
             }
-            asm volatile("bar.sync 1, %0;" ::"n"(kCEpiThreads) : "memory");
+            asm volatile("bar.sync 1, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
 #ifdef GPX_CGEMM_TIMING
             e_wait += clock64() - t_wait0;
 #endif
@@ -909,7 +908,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 // Every lane owns one row of the tile (its TMEM lane): 16 columns of a plane are 32
                 // contiguous bytes of that row, one 256-bit access, a whole sector.
                 const bool use_res = !partial && !out_f32 && res_hi && valid;
-                constexpr int CH = (TWO || AFF) ? 16 : 32;  // columns per piece
+                constexpr int CH = (TWO || AFF || BN == 256) ? 16 : 32;  // columns per piece
 #pragma unroll 1
                 for (int c = c_lo; c < c_hi; c += CH) {
                     float f[CH];
@@ -1033,7 +1032,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     // Every share of rows goes to the CTA that finishes it as one bulk copy (landing area:
                     // [split][row of the share][BN + 4 floats] in that CTA's last ring stages).
                     fence_proxy_async();
-                    asm volatile("bar.sync 1, %0;" ::"n"(kCEpiThreads) : "memory");
+                    asm volatile("bar.sync 1, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
                     const int owner = (int)threadIdx.x - 64;
                     if (owner < p.k_splits) {
                         const uint32_t share = (uint32_t)(kCBM / p.k_splits * (BN + 4) * 4);
@@ -1046,7 +1045,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 }
                 tc_fence_before_sync();
                 TCK(t_b0);
-                asm volatile("bar.sync 1, %0;" ::"n"(kCEpiThreads) : "memory");
+                asm volatile("bar.sync 1, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
 #ifdef GPX_CGEMM_TIMING
                 e_bar += clock64() - t_b0;
 #endif
@@ -1103,20 +1102,20 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         // a time, and a second barrier before the exit made this step 4 us long, BERT-base b1 7.4 us per
         // projection; storing them to the peers element by element, 2 us.)  A CTA that failed waits
         // here as well, so that no copy finds its memory gone.
-        if (warp >= 2 && warp < kCPollWarp) {
+        if (warp >= 2 && warp < Cfg::kPollWarp) {
             volatile int never = 0;
             if (!mbar_wait(smem_u32(&ctl->landed), 0, &never, kCWaitLimitNs + kCWaitLimitNs / 2)) fail(601);
         }
-        if (warp >= 2 && warp < kCPollWarp) {
+        if (warp >= 2 && warp < Cfg::kPollWarp) {
             const float *land = reinterpret_cast<const float *>(smem + nst * Cfg::kStageBytes);
             const SplitKParams &fin = p.fin;
             auto finish = [&](auto splits) {
                 constexpr int S = decltype(splits)::value, rows_per = kCBM / S;
                 constexpr int kItems = rows_per * kGroups;  // eight-channel items of this CTA
 #pragma unroll
-                for (int i = 0; i < (kItems + kCEpiThreads - 1) / kCEpiThreads; ++i) {
+                for (int i = 0; i < (kItems + Cfg::kEpiThreads - 1) / Cfg::kEpiThreads; ++i) {
                     if (!fin_live[i]) continue;
-                    const int e = (int)threadIdx.x - 64 + i * kCEpiThreads;
+                    const int e = (int)threadIdx.x - 64 + i * Cfg::kEpiThreads;
                     const int lr = e / kGroups, c8 = (e - lr * kGroups) * 8;
                     float4 q[2 * S];
 #pragma unroll
@@ -1273,7 +1272,9 @@ cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &
     });
 }
 
-int cgemm_threads(bool aff) { return kCgemmThreads + (aff ? kCAffThreads : 0); }
+int cgemm_threads(int bn, int fmt, bool aff) {
+    return cgemm_instance(bn, fmt == PF_SPLIT, aff, [](auto k) { return decltype(k)::Cfg::kThreads; });
+}
 
 size_t cgemm_spill_floats_per_cta() { return cgemm_spill_floats(); }
 

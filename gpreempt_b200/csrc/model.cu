@@ -1163,7 +1163,6 @@ int finalize_model(gpx_model &m) {
         kn.name = n.name;
         kn.node = (int)ni;
         kn.type = KernelType::Cgemm;
-        kn.threads = cgemm_threads(aff);
         CgemmParams &p = kn.cgemm;
         ActLayout il = in->layout;
         if (full_map_dense(n, src) && !n.via_im2col) {
@@ -1190,6 +1189,7 @@ int finalize_model(gpx_model &m) {
                 bn = 256;
         }
         kn.tile = bn;
+        kn.threads = cgemm_threads(bn, m.fmt, aff);
         p.taps = eff_k * eff_k;
         p.cin = eff_cin;
         p.cin_blocks = (eff_cin + 63) / 64;
