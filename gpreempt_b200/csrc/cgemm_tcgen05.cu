@@ -417,12 +417,14 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 const uint32_t bar = smem_u32(&ctl->full[stage]);
                 const uint32_t dst = smem_base + stage * Cfg::kStageBytes;
                 TCK(t_w0);
+                // (looked at before the wait, which hides it: what follows the wait delays the ring)
+                const bool stop = resumable && __any_sync(0xffffffffu, *word_up);
                 if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->empty[stage]), phase ^ 1, abort_flag, kCWaitLimitNs))) {
                     if (lane == 0) fail(101);
                     ok = false;
                     break;
                 }
-                if (resumable && __any_sync(0xffffffffu, *word_up)) {
+                if (stop) {
                     if (issuer) {
                         ctl->stage_msg[stage] = CMSG_STOP;
                         mbar_arrive(bar);
@@ -463,11 +465,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     ++kb;
                 } else {
                     const int n = t.main_kb - kb < KPS ? t.main_kb - kb : KPS;
-                    if (issuer) {
-                        ctl->stage_msg[stage] = CMSG_DATA + n;
-                        mbar_arrive_expect_tx(bar, n * Cfg::kKbBytes + ident_bytes);
-                        if (ident_bytes) tma_load_2d(smem_base + ident_off, &p.ident, bar, 0, 0);
-                    }
+                    if (issuer && ident_bytes) tma_load_2d(smem_base + ident_off, &p.ident, bar, 0, 0);
 #pragma unroll
                     for (int j = 0; j < KPS; ++j) {
                         if (j > 0 && j >= n) break;
@@ -485,6 +483,10 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                             w_tap += p.cin;
                             if (++tap < p.taps) a_row = row0 + p.tap_shift[tap];
                         }
+                    }
+                    if (issuer) {  // (the bytes may be announced after the loads: the arrival still holds the phase)
+                        ctl->stage_msg[stage] = CMSG_DATA + n;
+                        mbar_arrive_expect_tx(bar, n * Cfg::kKbBytes + ident_bytes);
                     }
                     kb += n;
                 }
