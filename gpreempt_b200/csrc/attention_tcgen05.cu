@@ -17,11 +17,18 @@
 // may lag behind its maximum: the factor cancels in the final division), which after the first block
 // hardly ever happens.
 //
+// The scores of the next block are computed as soon as this block's have left tensor memory for
+// registers (two key buffers), under this block's softmax; the values of the next block arrive
+// under its exponentials (one value buffer: the next values are fetched when P V is complete).
+//
 // What bounds it: the special-function unit has 128 x 64 exponentials a block (512 cycles at 16 an SM
-// and cycle), everything else is latency between the two products; two CTAs of two independent
-// warpgroups per SM overlap each other's.  BERT-base s512 b32: one warpgroup of 128 keys a block with
-// the output folded into registers and a transposing kernel in front took 89 + 16 us a layer.
-// One thread per warpgroup issues TMA and MMA; every wait is bounded, and a wait that gives up raises
+// and cycle, 22 us a layer of BERT-base s512 b32), everything else is latency between the two products;
+// two CTAs of two independent warpgroups per SM overlap each other's, to ~40 % of that unit's rate.
+// BERT-base s512 b32, a layer: one warpgroup of 128 keys a block with the output folded into registers
+// and a transposing kernel in front took 89 + 16 us; scores and context issued in line, 82; this, 72.
+// (Tried, at the same time or slower: a warp of its own for copies and products, two buffers of
+// values, the next tile claimed under the merge of this one.)
+// The first warp of a warpgroup issues TMA and MMA; every wait is bounded, and a wait that gives up raises
 // a flag that ends all others, so the threads of a CTA pass the same barriers and leave together.
 //
 // A tile takes a few microseconds (~6 us at 512 keys with two CTAs per SM), so the word is read
@@ -40,7 +47,7 @@ constexpr int kFaQ = 128, kFaKeys = 64, kFaD = 64;
 constexpr uint32_t kFaQBytes = kFaQ * kFaD * 2;     // 16 KiB
 constexpr uint32_t kFaKBytes = kFaKeys * kFaD * 2;  // 8 KiB, keys or values of a block
 constexpr uint32_t kFaPBytes = kFaQ * kFaKeys * 2;  // 16 KiB
-// per warpgroup: K, two V, P; both: Q, slack, control
+// per warpgroup: two K, V, P; both: Q, slack, control
 constexpr uint32_t kFaGroupBytes = 3 * kFaKBytes + kFaPBytes;
 constexpr uint32_t kFaSmem = kFaQBytes + 2 * kFaGroupBytes + 1024 + 2304;
 constexpr uint32_t kFaTmemCols = 256;  // per warpgroup: S 64 columns, output 64 columns
@@ -49,8 +56,8 @@ constexpr float kFaRescale = 8.0f;     // log2 of the growth of a row maximum th
 
 struct FaControl {
     unsigned long long bar_q;
-    unsigned long long bar_k[2], bar_s[2], bar_o[2];  // per warpgroup
-    unsigned long long bar_v[2][2];
+    unsigned long long bar_s[2], bar_o[2], bar_v[2];  // per warpgroup
+    unsigned long long bar_k[2][2];
     uint32_t tmem_base;
     int tile;
     int abort_flag;
@@ -66,6 +73,12 @@ __device__ __forceinline__ float fa_ex2(float x) {
     return y;
 }
 
+// The largest of three (one instruction on this architecture).
+__device__ __forceinline__ float fa_max3(float a, float b, float c) {
+    float y;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+    return y;
+}
 __device__ __forceinline__ void fa_st_v8(void *ptr, const uint32_t *r) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(ptr), "r"(r[0]), "r"(r[1]),
                  "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
@@ -84,19 +97,20 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
     const int tid = threadIdx.x;
     const int wg = __shfl_sync(0xffffffffu, tid >> 7, 0);  // warpgroup
     const int row = tid & 127;
-    const bool issuer = row == 0;  // this warpgroup's TMA and MMA thread
+    const bool warp0 = __shfl_sync(0xffffffffu, row >> 5, 0) == 0;  // this warpgroup's TMA and MMA warp
+    const bool issuer = elect_one() && warp0;                       // its thread that issues them
     unsigned char *mine = smem + kFaQBytes + wg * kFaGroupBytes;
-    const uint32_t sQ = smem_u32(smem), sK = smem_u32(mine), sV = sK + kFaKBytes, sP = sK + 3 * kFaKBytes;
-    unsigned char *pV = mine + kFaKBytes, *pP = mine + 3 * kFaKBytes;
+    const uint32_t sQ = smem_u32(smem), sK = smem_u32(mine), sV = sK + 2 * kFaKBytes, sP = sK + 3 * kFaKBytes;
+    unsigned char *pV = mine + 2 * kFaKBytes, *pP = mine + 3 * kFaKBytes;
 
     if (tid == 0) {
         mbar_init(smem_u32(&ctl->bar_q), 1);
         for (int g = 0; g < 2; ++g) {
-            mbar_init(smem_u32(&ctl->bar_k[g]), 1);
             mbar_init(smem_u32(&ctl->bar_s[g]), 1);
             mbar_init(smem_u32(&ctl->bar_o[g]), 1);
-            mbar_init(smem_u32(&ctl->bar_v[g][0]), 1);
-            mbar_init(smem_u32(&ctl->bar_v[g][1]), 1);
+            mbar_init(smem_u32(&ctl->bar_v[g]), 1);
+            mbar_init(smem_u32(&ctl->bar_k[g][0]), 1);
+            mbar_init(smem_u32(&ctl->bar_k[g][1]), 1);
         }
         ctl->abort_flag = 0;
         fence_barrier_init();
@@ -127,7 +141,7 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
     const int nkb = (p.S + kFaKeys - 1) / kFaKeys;
     const int steps = (nkb - wg + 1) / 2;  // blocks wg, wg + 2, ... of this warpgroup
     const float scale_log2 = p.scale * 1.4426950408889634f;  // scores are exponentiated base 2
-    uint32_t ph_q = 0, ph_k = 0, ph_s = 0, ph_o = 0, ph_v[2] = {0, 0};
+    uint32_t ph_q = 0, ph_s = 0, ph_o = 0, ph_v = 0, ph_k = 0;  // (ph_k: bit b for key buffer b)
     int iter = 0;
     for (;; ++iter) {
         if (tid == 0) ctl->tile = *abort_flag ? -1 : blp_claim(blp, iter);
@@ -147,29 +161,37 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             mbar_arrive_expect_tx(smem_u32(bar), kFaKBytes);
             tma_load_2d(dst, map, smem_u32(bar), col0, key_row0 + (2 * step + wg) * kFaKeys);
         };
-        auto scores = [&]() {  // S = Q K^T of the block whose keys are in sK (issuer only)
-            const uint64_t dq = make_smem_desc_sw128(sQ), dk = make_smem_desc_sw128(sK);
+        // S = Q K^T of block j (warp 0; the lane that issues it)
+        auto scores = [&](int j) {
+            const int kb = j & 1;
+            wait(&ctl->bar_k[wg][kb], (ph_k >> kb) & 1, 402);
+            ph_k ^= 1u << kb;
+            tc_fence_after_sync();
+            if (issuer && !*abort_flag) {
+                const uint64_t dq = make_smem_desc_sw128(sQ), dk = make_smem_desc_sw128(sK + kb * kFaKBytes);
 #pragma unroll
-            for (int k = 0; k < kFaD / 16; ++k) mma_f16_ss(t_s, dq + 2 * k, dk + 2 * k, idesc, k > 0 ? 1u : 0u);
-            mma_commit(smem_u32(&ctl->bar_s[wg]));
+                for (int k = 0; k < kFaD / 16; ++k) mma_f16_ss(t_s, dq + 2 * k, dk + 2 * k, idesc, k > 0 ? 1u : 0u);
+                mma_commit(smem_u32(&ctl->bar_s[wg]));
+            }
+            __syncwarp();
         };
         float m = -INFINITY, l = 0.f;
-        if (steps > 0 && issuer) {
-            fetch(sK, &p.tk, &ctl->bar_k[wg], 0);
-            fetch(sV, &p.tv, &ctl->bar_v[wg][0], 0);
+        if (steps > 0 && warp0) {
+            if (issuer) {
+                fetch(sK, &p.tk, &ctl->bar_k[wg][0], 0);
+                fetch(sV, &p.tv, &ctl->bar_v[wg], 0);
+                if (steps > 1) fetch(sK + kFaKBytes, &p.tk, &ctl->bar_k[wg][1], 1);
+            }
+            __syncwarp();
             wait(&ctl->bar_q, ph_q, 401);
-            wait(&ctl->bar_k[wg], ph_k, 402);
-            tc_fence_after_sync();
-            if (!*abort_flag) scores();
+            scores(0);
         }
         ph_q ^= 1;
         for (int j = 0; j < steps; ++j) {
-            const int buf = j & 1;
-            ph_k ^= 1;
             wait(&ctl->bar_s[wg], ph_s, 403);
             ph_s ^= 1;
             tc_fence_after_sync();
-            if (issuer && j + 1 < steps && !*abort_flag) fetch(sK, &p.tk, &ctl->bar_k[wg], j + 1);  // S is done with the keys
+            if (issuer && j + 2 < steps && !*abort_flag) fetch(sK + (j & 1) * kFaKBytes, &p.tk, &ctl->bar_k[wg][j & 1], j + 2);  // S is done with the keys
             uint32_t v[64];
             {
                 uint32_t a[32], c[32];
@@ -180,6 +202,12 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
 #pragma unroll
                 for (int i = 0; i < 32; ++i) v[i] = a[i], v[32 + i] = c[i];
             }
+            if (j + 1 < steps) {
+                // The scores are in registers: the next block's products run under this block's softmax.
+                tc_fence_before_sync();
+                group_sync();
+                if (warp0) scores(j + 1);
+            }
             const int key0 = (2 * j + wg) * kFaKeys;
             const int keys = p.S - key0 < kFaKeys ? p.S - key0 : kFaKeys;
             if (keys < kFaKeys) {
@@ -187,17 +215,22 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
                 for (int i = 0; i < 64; ++i)
                     if (i >= keys) v[i] = 0xff800000u;  // -inf
             }
-            float bmax = __uint_as_float(v[0]);  // of the raw scores: the scale is positive
+            // (of the raw scores: the scale is positive)
+            float bmax = fa_max3(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]));
+            float bmax2 = fa_max3(__uint_as_float(v[3]), __uint_as_float(v[4]), __uint_as_float(v[5]));
 #pragma unroll
-            for (int i = 1; i < 64; ++i) bmax = fmaxf(bmax, __uint_as_float(v[i]));
+            for (int i = 6; i < 62; i += 4) {
+                bmax = fa_max3(bmax, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+                bmax2 = fa_max3(bmax2, __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
+            }
+            bmax = fa_max3(fmaxf(bmax, bmax2), __uint_as_float(v[62]), __uint_as_float(v[63]));
             const float m_new = fmaxf(m, bmax * scale_log2);
             // P V of the block before: its probabilities and values are free, its output is complete
             if (j > 0) {
                 wait(&ctl->bar_o[wg], ph_o, 404);
                 ph_o ^= 1;
-                if (issuer && j + 1 < steps && !*abort_flag) fetch(sV + (buf ^ 1) * kFaKBytes, &p.tv, &ctl->bar_v[wg][buf ^ 1], j + 1);
+                if (issuer && !*abort_flag) fetch(sV, &p.tv, &ctl->bar_v[wg], j);
             } else {
-                if (issuer && j + 1 < steps && !*abort_flag) fetch(sV + kFaKBytes, &p.tv, &ctl->bar_v[wg][1], 1);
                 m = m_new;
             }
             if (__any_sync(0xffffffffu, m_new > m + kFaRescale)) {
@@ -238,32 +271,30 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             if (keys < kFaKeys) {
                 // Rows past the sequence belong to the next batch item: their probabilities are zero, and
                 // so must they be (zero times an infinity is not).
-                wait(&ctl->bar_v[wg][buf], ph_v[buf], 405);
+                wait(&ctl->bar_v[wg], ph_v, 405);
                 for (int e = row; e < (kFaKeys - keys) * 8; e += 128)
-                    *reinterpret_cast<uint4 *>(pV + buf * kFaKBytes + (keys + (e >> 3)) * 128 + (e & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+                    *reinterpret_cast<uint4 *>(pV + (keys + (e >> 3)) * 128 + (e & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
             }
             fence_proxy_async();  // the probabilities were written by ordinary stores, the MMA reads them
             tc_fence_before_sync();
             group_sync();
-            if (issuer && !*abort_flag) {
-                wait(&ctl->bar_v[wg][buf], ph_v[buf], 405);
+            if (warp0) {
+                wait(&ctl->bar_v[wg], ph_v, 405);
                 tc_fence_after_sync();
-                const uint64_t dp = make_smem_desc_sw128(sP);
-                // Value tile: 64 keys x 128 bytes, 128-byte swizzle.  As an MN-major operand eight keys
-                // are 1024 bytes apart from the next eight, and the 64 output columns are one swizzle
-                // atom wide; a step of sixteen keys is 2048 bytes (128 in the descriptor's units).
-                const uint64_t dv = make_smem_desc_sw128(sV + buf * kFaKBytes) | ((uint64_t)(1024 >> 4) << 16);
+                if (issuer && !*abort_flag) {
+                    const uint64_t dp = make_smem_desc_sw128(sP);
+                    // Value tile: 64 keys x 128 bytes, 128-byte swizzle.  As an MN-major operand eight keys
+                    // are 1024 bytes apart from the next eight, and the 64 output columns are one swizzle
+                    // atom wide; a step of sixteen keys is 2048 bytes (128 in the descriptor's units).
+                    const uint64_t dv = make_smem_desc_sw128(sV) | ((uint64_t)(1024 >> 4) << 16);
 #pragma unroll
-                for (int k = 0; k < kFaKeys / 16; ++k)
-                    mma_f16_ss(t_o, dp + 2 * k, dv + 128 * k, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-                mma_commit(smem_u32(&ctl->bar_o[wg]));
-                if (j + 1 < steps) {
-                    wait(&ctl->bar_k[wg], ph_k, 402);
-                    tc_fence_after_sync();
-                    if (!*abort_flag) scores();
+                    for (int k = 0; k < kFaKeys / 16; ++k)
+                        mma_f16_ss(t_o, dp + 2 * k, dv + 128 * k, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+                    mma_commit(smem_u32(&ctl->bar_o[wg]));
                 }
+                __syncwarp();
             }
-            ph_v[buf] ^= 1;
+            ph_v ^= 1;
         }
         if (steps > 0) {
             wait(&ctl->bar_o[wg], ph_o, 406);
@@ -272,7 +303,7 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
         tc_fence_after_sync();
         __syncwarp();
         // ---- merge: warpgroup g finishes columns 32 g .. 32 g + 31, the other 32 go through shared memory
-        // (this warpgroup's V and P tiles, free by now: [column][row] floats)
+        // (this warpgroup's V tile and half its P tile, free by now: [column][row] floats)
         float keep[32];
         {
             uint32_t o[32];
@@ -305,7 +336,7 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             const float a0 = fa_ex2(m0 - mm), a1 = fa_ex2(m1 - mm);
             const float inv = 1.0f / (ctl->ml[0][row][1] * a0 + ctl->ml[1][row][1] * a1);
             const float f_mine = (wg == 0 ? a0 : a1) * inv, f_other = (wg == 0 ? a1 : a0) * inv;
-            const float *take = reinterpret_cast<const float *>(smem + kFaQBytes + (wg ^ 1) * kFaGroupBytes + kFaKBytes);
+            const float *take = reinterpret_cast<const float *>(smem + kFaQBytes + (wg ^ 1) * kFaGroupBytes + 2 * kFaKBytes);
             uint32_t w[16];
 #pragma unroll
             for (int i = 0; i < 32; i += 2) {
