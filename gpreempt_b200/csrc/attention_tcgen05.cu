@@ -373,8 +373,7 @@ cudaError_t attention_tc_prepare() {
 int attention_tc_threads() { return kFaThreads; }
 
 cudaError_t attention_tc_launch(const AttnParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(p.fmt == PF_F16 ? attention_tc_kernel<true> : attention_tc_kernel<false>, grid, kFaThreads, kFaSmem, s, p, blp);
-    return cudaGetLastError();
+    return launch_layer(p.fmt == PF_F16 ? attention_tc_kernel<true> : attention_tc_kernel<false>, grid, kFaThreads, kFaSmem, s, p, blp);
 }
 
 }  // namespace gpx

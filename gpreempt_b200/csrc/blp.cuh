@@ -87,7 +87,7 @@ __device__ __forceinline__ int blp_claim(const BlpArgs &b, int iter) {
 }
 
 #if defined(__CUDACC__)
-// Launch of a layer kernel with the programmatic-serialization attribute (GPX_PDL=0 turns it off).
+// Layer kernels are launched with the programmatic-serialization attribute (GPX_PDL=0 turns it off).
 inline bool pdl_enabled() {
     static int on = -1;
     if (on < 0) {
@@ -97,20 +97,17 @@ inline bool pdl_enabled() {
     return on == 1;
 }
 
-template <typename... KArgs, typename... Args>
+// Launch through the driver's entry point: the runtime's looks the kernel up and copies its argument
+// block (1.3 KB of it for a tensor-core layer) for every launch, and an eager forward of a small
+// model is bound by the thread that launches it.  `cluster` CTAs form a cluster (1: no clusters).
+cudaError_t launch_direct(const void *kernel, unsigned grid, unsigned block, size_t smem, cudaStream_t s, unsigned cluster,
+                          void **args);
+
+template <typename... KArgs>
 inline cudaError_t launch_layer(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s,
-                                Args &&...args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+                                const KArgs &...args) {
+    void *list[] = {const_cast<void *>(static_cast<const void *>(&args))...};
+    return launch_direct(reinterpret_cast<const void *>(kernel), (unsigned)grid, (unsigned)block, smem, s, 1, list);
 }
 #endif
 

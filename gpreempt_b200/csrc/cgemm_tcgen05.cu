@@ -1256,21 +1256,9 @@ int cgemm_max_cluster(int bn, int fmt, bool aff, int cluster) {
 
 cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &blp, cudaStream_t s) {
     return cgemm_instance(bn, p.fmt == PF_SPLIT, p.aff_scale != nullptr, [&](auto k) {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)grid);
-        cfg.blockDim = dim3((unsigned)decltype(k)::Cfg::kThreads);
-        cfg.dynamicSmemBytes = decltype(k)::Cfg::kSmem;
-        cfg.stream = s;
-        cudaLaunchAttribute at[2];
-        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
-        at[1].id = cudaLaunchAttributeClusterDimension;
-        at[1].val.clusterDim.x = (unsigned)p.k_splits;
-        at[1].val.clusterDim.y = 1;
-        at[1].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = p.cluster_reduce ? 2 : 1;
-        return cudaLaunchKernelEx(&cfg, k.kernel(), p, blp);
+        void *args[] = {const_cast<CgemmParams *>(&p), const_cast<BlpArgs *>(&blp)};
+        return launch_direct(reinterpret_cast<const void *>(k.kernel()), (unsigned)grid, (unsigned)decltype(k)::Cfg::kThreads,
+                             decltype(k)::Cfg::kSmem, s, p.cluster_reduce ? (unsigned)p.k_splits : 1u, args);
     });
 }
 

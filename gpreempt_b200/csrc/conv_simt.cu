@@ -247,16 +247,12 @@ cudaError_t conv_launch(const ConvParams &p, int tile, int grid, const BlpArgs &
                         cudaStream_t s) {
     switch (tile) {
         case CONV_TILE_128:
-            launch_layer(conv_simt_kernel<128, 128, 8, 8>, grid, kConvThreads, 0, s, p, blp);
-            break;
+            return launch_layer(conv_simt_kernel<128, 128, 8, 8>, grid, kConvThreads, 0, s, p, blp);
         case CONV_TILE_64:
-            launch_layer(conv_simt_kernel<64, 64, 4, 4>, grid, kConvThreads, 0, s, p, blp);
-            break;
+            return launch_layer(conv_simt_kernel<64, 64, 4, 4>, grid, kConvThreads, 0, s, p, blp);
         default:
-            launch_layer(conv_simt_kernel<32, 32, 2, 2>, grid, kConvThreads, 0, s, p, blp);
-            break;
+            return launch_layer(conv_simt_kernel<32, 32, 2, 2>, grid, kConvThreads, 0, s, p, blp);
     }
-    return cudaGetLastError();
 }
 
 // ---- pooling / sub-sampling ---------------------------------------------------------------
@@ -681,8 +677,7 @@ im2col_kernel(const __grid_constant__ Im2colParams p, BlpArgs blp) {
 }
 
 cudaError_t im2col_launch(const Im2colParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(im2col_kernel, grid, kPoolThreads, 0, s, p, blp);
-    return cudaGetLastError();
+    return launch_layer(im2col_kernel, grid, kPoolThreads, 0, s, p, blp);
 }
 
 // Finishing pass of a split-K tensor-core convolution: one thread-iteration handles eight
@@ -907,15 +902,12 @@ cudaError_t dense_rows_launch(const DenseRowsParams &p, int grid, const BlpArgs 
     // (input rows of the short form, beside its own variables, in the default 48 KB of shared memory)
     const size_t rows = (size_t)p.M * p.K * sizeof(float);
     if (p.K <= kDenseShortK && rows + 256 <= 48 * 1024)
-        launch_layer(dense_short_kernel, grid, kPoolThreads, rows, s, p, blp);
-    else
-        launch_layer(dense_rows_kernel, grid, kPoolThreads, 0, s, p, blp);
-    return cudaGetLastError();
+        return launch_layer(dense_short_kernel, grid, kPoolThreads, rows, s, p, blp);
+    return launch_layer(dense_rows_kernel, grid, kPoolThreads, 0, s, p, blp);
 }
 
 cudaError_t splitk_launch(const SplitKParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(splitk_finish_kernel, grid, kPoolThreads, 0, s, p, blp);
-    return cudaGetLastError();
+    return launch_layer(splitk_finish_kernel, grid, kPoolThreads, 0, s, p, blp);
 }
 
 // Output pixel and channel group of element e of a tensor walked in (n, ho, wo, c / 8) order.
@@ -1048,8 +1040,7 @@ int dwconv_grid(const DwConvParams &p, int sm_count) {
 }
 
 cudaError_t dwconv_launch(const DwConvParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(dwconv_instance(p), grid, kPoolThreads, dwconv_smem(p), s, p, blp);
-    return cudaGetLastError();
+    return launch_layer(dwconv_instance(p), grid, kPoolThreads, dwconv_smem(p), s, p, blp);
 }
 
 static int pool_taps(const PoolParams &p) {
@@ -1072,8 +1063,7 @@ int pool_grid(const PoolParams &p, int sm_count) {
 
 cudaError_t pool_launch(const PoolParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
     const int t = pool_taps(p);
-    launch_layer(t == 3 ? pool_kernel<3> : (t == 2 ? pool_kernel<2> : pool_kernel<0>), grid, kPoolThreads, 0, s, p, blp);
-    return cudaGetLastError();
+    return launch_layer(t == 3 ? pool_kernel<3> : (t == 2 ? pool_kernel<2> : pool_kernel<0>), grid, kPoolThreads, 0, s, p, blp);
 }
 
 }  // namespace gpx

@@ -83,13 +83,17 @@ int exec_launch(gpx_exec *e, size_t idx, cudaStream_t s) {
     return GPX_SUCC;
 }
 
+// The cursors (one int a kernel) and the tensor-core kernels' slots lie in one allocation: starting afresh is
+// one memset.
+static size_t cursors_padded(size_t nk) { return (nk + 1 + 63) / 64 * 64; }
+static size_t progress_bytes(size_t nk) { return sizeof(int) * cursors_padded(nk) + sizeof(CgemmSlot) * kSlotsPerKernel * (nk + 1); }
+
 int exec_prologue(gpx_exec *e, cudaStream_t s) {
     size_t nk = e->model->kernels.size();
     if (e->kind == GPX_EXEC_BLP) {
         GPX_REQUIRE(e->word_dptr, GPX_FAIL, "BLP executor has no preempt word (gpx_exec_set_word)");
         // BLPExecutor::execute zeroes executed[] first (src/executor.cpp:212-214).
-        GPX_CUDA(cudaMemsetAsync(e->d_executed, 0, sizeof(int) * nk, s));
-        GPX_CUDA(cudaMemsetAsync(e->d_slots, 0, sizeof(CgemmSlot) * kSlotsPerKernel * nk, s));
+        GPX_CUDA(cudaMemsetAsync(e->d_executed, 0, progress_bytes(nk), s));
     }
     if (e->trace_on)
         GPX_CUDA(cudaMemcpyAsync(e->d_trace, e->h_trace_init, sizeof(uint64_t) * 4 * nk,
@@ -111,12 +115,11 @@ int gpx_exec_create(gpx_model *m, int kind, gpx_exec **out) {
     size_t nk = m->kernels.size();
     // dpStopIndex and executed[] are owned by the executor (src/executor.cpp:329-333).
     GPX_CUDA(cudaMalloc((void **)&e->d_stop_index, 256));
-    GPX_CUDA(cudaMalloc((void **)&e->d_executed, sizeof(int) * (nk + 1)));
+    GPX_CUDA(cudaMalloc((void **)&e->d_executed, progress_bytes(nk)));
     GPX_CUDA(cudaMalloc((void **)&e->d_trace, sizeof(uint64_t) * 4 * (nk + 1)));
     // Tensor-core convolutions: per-kernel progress slots, one spill area (only one kernel of an
     // executor can hold partial tiles at a time) and an error word.
-    GPX_CUDA(cudaMalloc((void **)&e->d_slots, sizeof(CgemmSlot) * kSlotsPerKernel * (nk + 1)));
-    GPX_CUDA(cudaMemset(e->d_slots, 0, sizeof(CgemmSlot) * kSlotsPerKernel * (nk + 1)));
+    e->d_slots = reinterpret_cast<CgemmSlot *>(e->d_executed + cursors_padded(nk));
     size_t spill_bytes = sizeof(float) * cgemm_spill_floats_per_cta() * (size_t)(m->max_cgemm_grid + 1);
     GPX_CUDA(cudaMalloc((void **)&e->d_spill, spill_bytes));
     GPX_CUDA(cudaMalloc((void **)&e->d_partial, sizeof(float) * (m->max_partial_floats + 64)));
@@ -137,7 +140,7 @@ int gpx_exec_create(gpx_model *m, int kind, gpx_exec **out) {
         e->h_trace_init[4 * i + 3] = 0;
     }
     GPX_CUDA(cudaMemcpy(e->d_stop_index, e->h_minus_one, sizeof(int), cudaMemcpyHostToDevice));
-    GPX_CUDA(cudaMemset(e->d_executed, 0, sizeof(int) * (nk + 1)));
+    GPX_CUDA(cudaMemset(e->d_executed, 0, progress_bytes(nk)));
     GPX_CUDA(cudaMemcpy(e->d_trace, e->h_trace_init, sizeof(uint64_t) * 4 * (nk + 1),
                         cudaMemcpyHostToDevice));
     *out = e;
@@ -151,7 +154,6 @@ int gpx_exec_destroy(gpx_exec *e) {
     cudaFree(e->d_stop_index);
     cudaFree(e->d_executed);
     cudaFree(e->d_trace);
-    cudaFree(e->d_slots);
     cudaFree(e->d_spill);
     cudaFree(e->d_partial);
     cudaFree(e->d_error);
@@ -362,8 +364,7 @@ int gpx_exec_set_restart_policy(gpx_exec *e, int drop_tile_in_flight) {
 int gpx_exec_reset_cursors(gpx_exec *e, gpx_stream stream) {
     GPX_REQUIRE(e, GPX_FAIL, "NULL executor");
     size_t nk = e->model->kernels.size();
-    GPX_CUDA(cudaMemsetAsync(e->d_executed, 0, sizeof(int) * nk, as_stream(stream)));
-    GPX_CUDA(cudaMemsetAsync(e->d_slots, 0, sizeof(CgemmSlot) * kSlotsPerKernel * nk, as_stream(stream)));
+    GPX_CUDA(cudaMemsetAsync(e->d_executed, 0, progress_bytes(nk), as_stream(stream)));
     return GPX_SUCC;
 }
 

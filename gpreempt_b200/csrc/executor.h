@@ -9,7 +9,7 @@ struct gpx_exec {
     int kind = GPX_EXEC_BASE;
     const int *word_dptr = nullptr;   // BLPExecutor::dpStop, owned by the caller
     int *d_stop_index = nullptr;      // BLPExecutor::dpStopIndex
-    int *d_executed = nullptr;        // BLPExecutor::executed, one cursor per kernel
+    int *d_executed = nullptr;        // BLPExecutor::executed, one cursor per kernel; the slots follow it
     unsigned long long *d_trace = nullptr;
     gpx::CgemmSlot *d_slots = nullptr;  // [kernel][kSlotsPerKernel] progress of tensor-core kernels
     float *d_partial = nullptr;         // split-K partial sums of the tensor-core kernels

@@ -660,8 +660,7 @@ int graphwl_grid(const GraphWlParams &p, int total_tiles, int sm_count) {
 }
 
 cudaError_t graphwl_launch(const GraphWlParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(pick_kernel(p), grid, kGwThreads, window_bytes(p), s, p, blp);
-    return cudaGetLastError();
+    return launch_layer(pick_kernel(p), grid, kGwThreads, window_bytes(p), s, p, blp);
 }
 
 bool is_graph_workload(const std::string &name) {

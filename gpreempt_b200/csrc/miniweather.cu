@@ -514,10 +514,8 @@ int stencil_grid(int dir, int total_tiles, int sm_count) {
 
 cudaError_t stencil_launch(const StencilParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
     if (p.dir == 1)
-        launch_layer(miniweather_step_kernel<1>, grid, kMwThreads, 0, s, p, blp);
-    else
-        launch_layer(miniweather_step_kernel<2>, grid, kMwThreads, 0, s, p, blp);
-    return cudaGetLastError();
+        return launch_layer(miniweather_step_kernel<1>, grid, kMwThreads, 0, s, p, blp);
+    return launch_layer(miniweather_step_kernel<2>, grid, kMwThreads, 0, s, p, blp);
 }
 
 // "miniweather" is the reference's grid (3200 x 1600, miniweather.cu:21-22); "miniweather_tiny"

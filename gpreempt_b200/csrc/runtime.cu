@@ -7,6 +7,7 @@
 #include "word.h"
 
 #include <atomic>
+#include <cuda.h>
 #include <mutex>
 #include <pthread.h>
 #include <sched.h>
@@ -44,6 +45,54 @@ void *driver_entry(const char *name) {
         q != cudaDriverEntryPointSuccess)
         return nullptr;
     return fn;
+}
+
+cudaError_t launch_direct(const void *kernel, unsigned grid, unsigned block, size_t smem, cudaStream_t s, unsigned cluster,
+                          void **args) {
+    typedef CUresult (*LaunchFn)(const CUlaunchConfig *, CUfunction, void **, void **);
+    static std::atomic<void *> cached{nullptr};
+    void *launch = cached.load(std::memory_order_acquire);
+    if (!launch) {
+        launch = driver_entry("cuLaunchKernelEx");
+        if (!launch) return cudaErrorInsufficientDriver;
+        cached.store(launch, std::memory_order_release);
+    }
+    // The driver's handle of a kernel on the current device: a small table per thread, kept for good (the
+    // library is never unloaded from under its contexts).
+    struct Known {
+        const void *kernel;
+        int device;
+        CUfunction fn;
+    };
+    static thread_local Known known[128] = {};
+    int device = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err != cudaSuccess) return err;
+    Known &k = known[(reinterpret_cast<uintptr_t>(kernel) >> 4 ^ (uintptr_t)device) % 128];
+    if (k.kernel != kernel || k.device != device) {
+        cudaFunction_t fn = nullptr;
+        err = cudaGetFuncBySymbol(&fn, kernel);
+        if (err != cudaSuccess) return err;
+        k = Known{kernel, device, reinterpret_cast<CUfunction>(fn)};
+    }
+    CUlaunchAttribute at[2];
+    at[0].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+    at[0].value.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    at[1].id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+    at[1].value.clusterDim.x = cluster;
+    at[1].value.clusterDim.y = 1;
+    at[1].value.clusterDim.z = 1;
+    CUlaunchConfig cfg{};
+    cfg.gridDimX = grid;
+    cfg.gridDimY = cfg.gridDimZ = 1;
+    cfg.blockDimX = block;
+    cfg.blockDimY = cfg.blockDimZ = 1;
+    cfg.sharedMemBytes = (unsigned)smem;
+    cfg.hStream = reinterpret_cast<CUstream>(s);
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    // (the two interfaces share their error numbers)
+    return static_cast<cudaError_t>(reinterpret_cast<LaunchFn>(launch)(&cfg, k.fn, args, nullptr));
 }
 
 cuStreamWriteValue32_t driver_stream_write32() {

@@ -165,21 +165,16 @@ int layernorm_rows_per_tile(int rows, int sm_count) {
 cudaError_t layernorm_launch(const LayerNormParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
     const int nv = p.H <= 256 ? 1 : (p.H <= 768 ? 3 : 4);
     const bool pair = p.rows_per_tile == 16;
-    auto go = [&](auto kernel) { launch_layer(kernel, grid, kTfThreads, 0, s, p, blp); };
+    auto go = [&](auto kernel) { return launch_layer(kernel, grid, kTfThreads, 0, s, p, blp); };
     auto pick = [&](auto two) {
         constexpr bool T = decltype(two)::value;
         if (nv == 1)
-            go(pair ? layernorm_kernel<1, 2, T> : layernorm_kernel<1, 1, T>);
-        else if (nv == 3)
-            go(pair ? layernorm_kernel<3, 2, T> : layernorm_kernel<3, 1, T>);
-        else
-            go(pair ? layernorm_kernel<4, 2, T> : layernorm_kernel<4, 1, T>);
+            return go(pair ? layernorm_kernel<1, 2, T> : layernorm_kernel<1, 1, T>);
+        if (nv == 3)
+            return go(pair ? layernorm_kernel<3, 2, T> : layernorm_kernel<3, 1, T>);
+        return go(pair ? layernorm_kernel<4, 2, T> : layernorm_kernel<4, 1, T>);
     };
-    if (p.fmt == PF_SPLIT)
-        pick(std::true_type());
-    else
-        pick(std::false_type());
-    return cudaGetLastError();
+    return p.fmt == PF_SPLIT ? pick(std::true_type()) : pick(std::false_type());
 }
 
 // ---- multi-head attention ---------------------------------------------------------------------
@@ -318,8 +313,7 @@ attention_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
 }
 
 cudaError_t attention_launch(const AttnParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    launch_layer(attention_kernel, grid, kAttnThreads, 0, s, p, blp);
-    return cudaGetLastError();
+    return launch_layer(attention_kernel, grid, kAttnThreads, 0, s, p, blp);
 }
 
 }  // namespace gpx
