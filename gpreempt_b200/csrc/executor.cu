@@ -150,6 +150,7 @@ int gpx_exec_create(gpx_model *m, int kind, gpx_exec **out) {
 int gpx_exec_destroy(gpx_exec *e) {
     if (!e) return GPX_SUCC;
     if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);
+    if (e->own_graph) cudaGraphExecDestroy(e->own_graph);
     if (e->graph) cudaGraphDestroy(e->graph);
     cudaFree(e->d_stop_index);
     cudaFree(e->d_executed);
@@ -190,9 +191,63 @@ int gpx_exec_enable_trace(gpx_exec *e, int on) {
     return GPX_SUCC;
 }
 
+// Kernels of the longest forward that execute turns into a graph of its own.  With the word up every kernel
+// still queued starts once to find that out, ~2 us each, and a graph queues all of them at once: beyond
+// this many the drain would show it.
+constexpr size_t kOwnGraphKernels = 64;
+
+// The forward as a graph, made by the first execute (and again when what it depends on has changed): kernel by
+// kernel the host takes up to 4 us a launch, longer than most kernels of a small model run (15-kernel BERT:
+// 63 us of host for 80 us of GPU).
+static int refresh_own_graph(gpx_exec *e, cudaStream_t s) {
+    int priority = 0;
+    if (s) GPX_CUDA(cudaStreamGetPriority(s, &priority));
+    if (e->own_graph && e->own_word == e->word_dptr && e->own_priority == priority && e->own_trace == e->trace_on &&
+        e->own_drop == e->drop_tile_in_flight)
+        return GPX_SUCC;
+    if (e->own_graph) GPX_CUDA(cudaGraphExecDestroy(e->own_graph));  // (a run in flight keeps it until it is through)
+    e->own_graph = nullptr;
+    // captured on a stream of its own: the caller's may be the default stream, which cannot be captured
+    cudaStream_t c = nullptr;
+    cudaGraph_t graph = nullptr;
+    GPX_CUDA(cudaStreamCreateWithPriority(&c, cudaStreamNonBlocking, priority));
+    cudaError_t err = cudaStreamBeginCapture(c, cudaStreamCaptureModeThreadLocal);
+    int st = GPX_SUCC;
+    if (err == cudaSuccess) {
+        const size_t nk = e->model->kernels.size();
+        st = exec_prologue(e, c);
+        for (size_t i = 0; st == GPX_SUCC && i < nk; ++i) {
+            st = exec_launch(e, i, c);
+            if (st == GPX_SUCC) g_kernel_launches.fetch_sub(1, std::memory_order_relaxed);  // captured, not run
+        }
+        err = cudaStreamEndCapture(c, &graph);
+        if (st == GPX_SUCC && err == cudaSuccess) err = cudaGraphInstantiate(&e->own_graph, graph, 0);
+        if (graph) cudaGraphDestroy(graph);
+    }
+    cudaStreamDestroy(c);
+    if (st != GPX_SUCC) return st;
+    GPX_CUDA(err);
+    e->own_word = e->word_dptr;
+    e->own_priority = priority;
+    e->own_trace = e->trace_on;
+    e->own_drop = e->drop_tile_in_flight;
+    return GPX_SUCC;
+}
+
 int gpx_exec_execute(gpx_exec *e, gpx_stream stream) {
     GPX_REQUIRE(e, GPX_FAIL, "NULL executor");
     cudaStream_t s = as_stream(stream);
+    if (!e->graph_exec && e->kind == GPX_EXEC_BLP && e->model->kernels.size() <= kOwnGraphKernels) {
+        GPX_REQUIRE(e->word_dptr, GPX_FAIL, "BLP executor has no preempt word (gpx_exec_set_word)");
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if (s) GPX_CUDA(cudaStreamIsCapturing(s, &capturing));
+        if (capturing == cudaStreamCaptureStatusNone) {
+            GPX_TRY(refresh_own_graph(e, s));
+            GPX_CUDA(cudaGraphLaunch(e->own_graph, s));
+            g_kernel_launches.fetch_add(e->model->kernels.size(), std::memory_order_relaxed);
+            return GPX_SUCC;
+        }
+    }
     if (e->graph_exec) {
         GPX_CUDA(cudaGraphLaunch(e->graph_exec, s));
         g_kernel_launches.fetch_add(e->model->kernels.size(), std::memory_order_relaxed);

@@ -24,6 +24,12 @@ struct gpx_exec {
     bool drop_tile_in_flight = false;  // restart policy of the tensor-core kernels (gpx_exec_set_restart_policy)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
+    // What execute launches for a short preemptible forward that nobody has captured, and what it was
+    // captured for.
+    cudaGraphExec_t own_graph = nullptr;
+    const int *own_word = nullptr;
+    int own_priority = 0;
+    bool own_trace = false, own_drop = false;
 };
 
 namespace gpx {
