@@ -1,0 +1,207 @@
+"""Sizes at which the layer kernels change form: edges of tiles, remainders, both sides of each limit."""
+import numpy as np
+import pytest
+
+from gpreempt_b200 import graph_files
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"float32": 1e-4, "float16": 5e-3, "bfloat16": 2e-2}  # of the largest value of a tensor
+
+
+def _rel(a, b):
+    return float(np.max(np.abs(a.astype(np.float64) - b.astype(np.float64))) / max(float(np.max(np.abs(b))), 1e-30))
+
+
+def _images(gpx, batch, seed=0):
+    return gpx.synth_normal(batch * 3 * 224 * 224, seed, 0).reshape(batch, 3, 224, 224)
+
+
+def _bert(gpx, oracle, batch, seq, dtype):
+    """bert_tiny on seeded ids: the executor after one forward, and the oracle's tensors."""
+    ex = gpx.BaseExecutor()
+    ex.init("bert_tiny", batch=batch, seed=7, seq_len=seq, dtype=dtype)
+    ids = np.random.default_rng(seq).integers(0, 1000, (batch, seq)).astype(np.int64)
+    ex.set_input("data", ids)
+    ex.execute()
+    assert ex.error() == (0, 0)
+    params = {k: v.reshape(v.shape[0], -1) if v.ndim == 4 else v for k, v in ex.model.params().items()}
+    taps = {}
+    heads = oracle.bert_forward(params, ids, layers=2, heads=2, taps=taps)
+    return ex, taps, heads
+
+
+# One block of keys (the second warpgroup has none), a partial second block, odd and even numbers of
+# blocks, a partial last block of the first warpgroup, the longest sequence.
+@pytest.mark.parametrize("seq", [8, 64, 72, 128, 136, 200, 320, 512])
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+def test_attention_key_blocks(gpx, oracle, seq, dtype):
+    ex, taps, _ = _bert(gpx, oracle, 3, seq, dtype)
+    for layer in (0, 1):
+        name = f"encoder.layer.{layer}.attention.context"
+        assert _rel(ex.model.get(name).reshape(taps[name].shape), taps[name]) <= TOL[dtype], name
+    ex.clear()
+
+
+# Two rows a warp from 9472 rows on a 148-SM device: below, at a multiple of the 16-row tile, and with half a
+# tile left over.
+@pytest.mark.parametrize("batch,seq", [(74, 120), (80, 120), (79, 120)])
+def test_layernorm_rows_per_tile(gpx, oracle, batch, seq):
+    ex, taps, heads = _bert(gpx, oracle, batch, seq, "float32")
+    name = "encoder.layer.0.attention.output"
+    assert _rel(ex.model.get(name).reshape(taps[name].shape), taps[name]) <= TOL["float32"]
+    assert _rel(ex.get_output("heads"), heads) <= TOL["float32"]
+    ex.clear()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16"])
+def test_projections_share_one_product_and_keep_their_tensors(gpx, oracle, dtype):
+    """Query, key and value weights are slices of one matrix: each is read and written by its own name."""
+    ex, taps, heads = _bert(gpx, oracle, 2, 40, dtype)
+    p = "encoder.layer.0.attention.self."
+    for part in ("query", "key", "value"):
+        assert _rel(ex.model.get(p + part + ".out").reshape(taps[p + part + ".out"].shape), taps[p + part + ".out"]) <= TOL[dtype]
+    before = {part: ex.model.get(p + part + ".weight") for part in ("query", "key", "value")}
+    ex.model.set(p + "key.weight", before["key"] * 2)
+    for part in ("query", "key", "value"):
+        assert np.array_equal(ex.model.get(p + part + ".weight"), before[part] * (2 if part == "key" else 1))
+    query, value = ex.model.get(p + "query.out"), ex.model.get(p + "value.out")
+    ex.execute()
+    assert np.array_equal(ex.model.get(p + "query.out"), query) and np.array_equal(ex.model.get(p + "value.out"), value)
+    assert not np.array_equal(ex.get_output("heads"), heads.astype(np.float32))
+    ex.clear()
+
+
+@pytest.mark.parametrize("batch,dtype", [(1, "float16"), (5, "float32")])
+def test_batch_norm_in_the_operand(gpx, oracle, batch, dtype):
+    """The normalised copy exists only in shared memory: reading it computes it, writing it is refused."""
+    ex = gpx.BaseExecutor()
+    ex.init("densenet_tiny", batch=batch, seed=1, dtype=dtype)
+    data = _images(gpx, batch)
+    ex.set_input("data", data)
+    ex.execute()
+    assert ex.error() == (0, 0)
+    taps = {}
+    heads = oracle.forward("densenet_tiny", ex.model.params(), data, taps=taps)
+    norms = [n for n in taps if ".norm" in n]
+    assert norms
+    for n in norms + [n for n in taps if n.endswith(".conv1") or n.endswith(".conv")]:
+        assert _rel(ex.model.get(n).reshape(taps[n].shape), taps[n]) <= TOL[dtype], n
+    assert _rel(ex.get_output("heads"), heads) <= TOL[dtype]
+    with pytest.raises(gpx.GpxError):
+        ex.model.set(norms[0], ex.model.get(norms[0]))
+    ex.clear()
+
+
+# 2048 inputs: five rows are the most the short form keeps in shared memory.
+@pytest.mark.parametrize("model,batch", [("resnet_tiny", 5), ("resnet_tiny", 6), ("resnet_tiny", 8), ("mobilenet_v2", 4)])
+@pytest.mark.parametrize("dtype", ["float32", "float16"])
+def test_classifier_rows_and_large_depthwise_layers(gpx, oracle, model, batch, dtype):
+    """(At four images the first depthwise layers exceed four tiles an SM.)"""
+    ex = gpx.BaseExecutor()
+    ex.init(model, batch=batch, seed=3, dtype=dtype)
+    data = _images(gpx, batch, 2)
+    ex.set_input("data", data)
+    ex.execute()
+    assert ex.error() == (0, 0)
+    taps = {}
+    heads = oracle.forward(model, ex.model.params(), data, taps=taps)
+    for name in [n for n in taps if n.endswith(".dw")]:
+        assert _rel(ex.model.get(name).reshape(taps[name].shape), taps[name]) <= TOL[dtype], name
+    assert _rel(ex.get_output("heads"), heads) <= TOL[dtype]
+    ex.clear()
+
+
+def test_wide_tiles_agree_with_narrow_ones(gpx):
+    """80 images give the deep 3x3 layers 256-column tiles, eight images narrower ones; the sums are the same."""
+    data = _images(gpx, 80, 5)
+    heads = {}
+    for batch in (80, 8):
+        ex = gpx.BaseExecutor()
+        ex.init("resnet_tiny", batch=batch, seed=3, dtype="float16")
+        ex.set_input("data", data[:batch])
+        ex.execute()
+        assert ex.error() == (0, 0)
+        heads[batch] = ex.get_output("heads")
+        ex.clear()
+    assert _rel(heads[80][:8], heads[8]) <= 2e-3
+
+
+# Average in-degree around 200, 100, 50 and 16: eight, four, two and one id a lane; the last graph's
+# neighbours lie too far apart for a window and stay lists.
+@pytest.mark.parametrize("vertices,degree,band", [(3001, 200, 1500), (2999, 100, 900), (4000, 50, 600), (65, 16, 60), (40001, 20, 39000)])
+def test_pagerank_list_forms(gpx, tmp_path, vertices, degree, band):
+    from oracle import graphs
+
+    graphs.build()
+    prefix = str(tmp_path / "g" / "g.bel")
+    rng = np.random.default_rng(vertices)
+    rows = []
+    for v in range(vertices):
+        near = np.arange(max(0, v - band), min(vertices, v + band + 1))
+        deg = int(rng.integers(0, 2 * degree))  # vertices without in- or out-edges among them
+        rows.append(np.sort(rng.choice(near, size=min(deg, len(near)), replace=False)))
+    offsets = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.uint64)
+    neighbours = np.concatenate(rows).astype(np.uint64)
+    graph_files.write_bel(prefix, offsets, neighbours, np.ones(len(neighbours), np.uint32))
+    want = graphs.pagerank(offsets, neighbours)[0].astype(np.float64)
+    for kind in ("base", "blp"):
+        ex = gpx.BaseExecutor() if kind == "base" else gpx.BLPExecutor()
+        ex.set_graph_path(prefix)
+        ex.init("pagerank")
+        if kind == "blp":
+            word = gpx.PreemptWord(1)
+            ex.set_word(word)
+        ex.execute()
+        err = np.abs(ex.model.get("value").astype(np.float64) - want)
+        assert err.max() <= 1.1e-3 and err.mean() <= 1e-5, kind
+        ex.clear()
+
+
+def test_short_preemptible_forward_follows_word_and_stream(gpx):
+    """execute keeps a graph of a short forward: another word, stream or trace setting has to show in it."""
+    ex = gpx.BLPExecutor()
+    ex.init("resnet_tiny", batch=1, seed=3)
+    ex.set_input("data", _images(gpx, 1))
+    words = [gpx.PreemptWord(1), gpx.PreemptWord(1)]
+    streams = [gpx.Stream(1), gpx.Stream(0)]
+    ex.set_word(words[0])
+    ex.execute()
+    want = ex.get_output("heads")
+    for word in words:
+        ex.set_word(word)
+        for s in streams:
+            word.raise_()
+            ex.execute(s)
+            s.sync()
+            word.clear()
+            assert ex.resume(s) == 0  # nothing had run
+            s.sync()
+            assert ex.resume(s) == -1 and np.array_equal(ex.get_output("heads"), want)
+            ex.execute(s)
+            assert ex.resume(s) == -1 and np.array_equal(ex.get_output("heads"), want)
+    ex.clear()
+    for o in words + streams:
+        o.destroy()
+
+
+def test_resets_are_ordered_before_later_launches(gpx, oracle):
+    """A context's reset is not waited for: launches on any stream and copies still come behind it."""
+    n = 300_001
+    x, y = gpx.synth_uniform(n, 4, 0), gpx.synth_uniform(n, 4, 1)
+    dx, dy = gpx.DeviceBuffer.from_numpy(x), gpx.DeviceBuffer.from_numpy(y)
+    word = gpx.PreemptWord(1)
+    ctx = gpx.BlpContext(word, kernel_id=2)
+    streams = [gpx.Stream(1), gpx.Stream(0)]
+    want = y
+    for i in range(40):
+        s = streams[i % 2]
+        ctx.reset()
+        gpx.axpy(0.5, dx, dy, n, ctx, s)
+        s.sync()
+        want = oracle.axpy(0.5, x, want)
+    st = ctx.read()
+    assert st["stop_index"] == -1 and st["tiles_run"] == gpx.axpy_tiles(n)
+    assert np.array_equal(dy.download(np.float32, n).view(np.uint32), want.view(np.uint32))
+    for o in (dx, dy, ctx, word, *streams):
+        (o.free if hasattr(o, "free") else o.destroy)()
