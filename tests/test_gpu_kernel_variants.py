@@ -48,7 +48,7 @@ def test_attention_key_blocks(gpx, oracle, seq, dtype):
 @pytest.mark.parametrize("batch,seq", [(74, 120), (80, 120), (79, 120)])
 def test_layernorm_rows_per_tile(gpx, oracle, batch, seq):
     ex, taps, heads = _bert(gpx, oracle, batch, seq, "float32")
-    name = "encoder.layer.0.attention.output"
+    name = "encoder.layer.0.output"
     assert _rel(ex.model.get(name).reshape(taps[name].shape), taps[name]) <= TOL["float32"]
     assert _rel(ex.get_output("heads"), heads) <= TOL["float32"]
     ex.clear()
@@ -59,8 +59,11 @@ def test_projections_share_one_product_and_keep_their_tensors(gpx, oracle, dtype
     """Query, key and value weights are slices of one matrix: each is read and written by its own name."""
     ex, taps, heads = _bert(gpx, oracle, 2, 40, dtype)
     p = "encoder.layer.0.attention.self."
+    x = taps["embeddings"].astype(np.float64)
     for part in ("query", "key", "value"):
-        assert _rel(ex.model.get(p + part + ".out").reshape(taps[p + part + ".out"].shape), taps[p + part + ".out"]) <= TOL[dtype]
+        w, b = ex.model.get(p + part + ".weight"), ex.model.get(p + part + ".bias")
+        want = x @ w.reshape(w.shape[0], -1).astype(np.float64).T + b
+        assert _rel(ex.model.get(p + part + ".out").reshape(want.shape), want) <= TOL[dtype], part
     before = {part: ex.model.get(p + part + ".weight") for part in ("query", "key", "value")}
     ex.model.set(p + "key.weight", before["key"] * 2)
     for part in ("query", "key", "value"):
@@ -138,9 +141,8 @@ def test_pagerank_list_forms(gpx, tmp_path, vertices, degree, band):
     rng = np.random.default_rng(vertices)
     rows = []
     for v in range(vertices):
-        near = np.arange(max(0, v - band), min(vertices, v + band + 1))
-        deg = int(rng.integers(0, 2 * degree))  # vertices without in- or out-edges among them
-        rows.append(np.sort(rng.choice(near, size=min(deg, len(near)), replace=False)))
+        deg = int(rng.integers(0, 2 * degree))  # (vertices without edges among them)
+        rows.append(np.unique(rng.integers(max(0, v - band), min(vertices, v + band + 1), deg)))
     offsets = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.uint64)
     neighbours = np.concatenate(rows).astype(np.uint64)
     graph_files.write_bel(prefix, offsets, neighbours, np.ones(len(neighbours), np.uint32))
