@@ -587,38 +587,37 @@ im2col_kernel(const __grid_constant__ Im2colParams p, BlpArgs blp) {
         // Row-window mode.  The window of the tile - Cin x kh input rows, (win_w-1)*stride + kw
         // wide, zeros outside the image - is staged with coalesced loads; a patch-matrix element
         // is then one table lookup and one shared-memory read, and the stores stay row-contiguous.
-        // What bounds it is the chain claim, window, copy of a tile, so a tile is as wide as leaves every
-        // SM a few, the next one is claimed while its window travels, and a warp stages pieces of
-        // 64 columns, decoded once each (224x224x3, 16 images fp16: FIGURES).
         __shared__ float s_win[kIm2colWindowFloats];
         const int win_cols = (p.win_w - 1) * p.stride + p.kw;
         const int seg = p.Cin * p.kh;  // window rows
         for (int k = threadIdx.x; k < p.Kp; k += kPoolThreads)
             s_off[k] = s_fh[k] == 255 ? -1 : ((int)s_ci[k] * p.kh + (int)s_fh[k]) * win_cols + (int)s_fw[k];
-        const int pieces = (win_cols + 63) / 64;
-        const int lane = threadIdx.x & 31;
-        TileClaims claims(blp, dynamic, s_tile);
-        for (int tile = claims.first(); tile >= 0; tile = claims.next()) {
+        for (;;) {
+            int tile;
             __syncthreads();  // the table is complete / the previous window has been consumed
+            if (dynamic) {
+                if (threadIdx.x == 0) s_tile = blp_claim(blp, iter);
+                __syncthreads();
+                tile = s_tile;
+            } else {
+                tile = blp_claim(blp, iter);
+            }
+            if (tile < 0) break;
             const int chunk = tile % p.win_chunks;
             const int t = tile / p.win_chunks;
             const int ho = t % p.Ho, n = t / p.Ho;
             const int wo0 = chunk * p.win_w;
             const int nw = min(p.win_w, p.Wo - wo0);
             const int h0 = ho * p.stride - p.pad, w0 = wo0 * p.stride - p.pad;
-#pragma unroll 4
-            for (int u = threadIdx.x >> 5; u < seg * pieces; u += kPoolThreads / 32) {
-                const int r = u / pieces, c0 = (u - r * pieces) * 64 + lane;
-                const int ci = r / p.kh, hi = h0 + r - ci * p.kh;
-                const bool row_in = hi >= 0 && hi < H;
-                const float *src = p.in.f32 + (((size_t)n * p.Cin + ci) * H + hi) * W;
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int c = c0 + 32 * i, wi = w0 + c;
-                    if (c < win_cols) s_win[r * win_cols + c] = row_in && wi >= 0 && wi < W ? src[wi] : 0.f;
-                }
+            for (int e = threadIdx.x; e < seg * win_cols; e += kPoolThreads) {
+                const int r = e / win_cols, c = e - r * win_cols;
+                const int ci = r / p.kh, fh = r - ci * p.kh;
+                const int hi = h0 + fh, wi = w0 + c;
+                float v = 0.f;
+                if (hi >= 0 && hi < H && wi >= 0 && wi < W)
+                    v = p.in.f32[(((size_t)n * p.Cin + ci) * H + hi) * W + wi];
+                s_win[e] = v;
             }
-            claims.ahead();
             __syncthreads();
             const size_t m0 = ((size_t)n * p.Ho + ho) * p.Wo + wo0;
             for (int e = threadIdx.x; e < nw * K8; e += kPoolThreads) {
@@ -632,8 +631,9 @@ im2col_kernel(const __grid_constant__ Im2colParams p, BlpArgs blp) {
                 }
                 planes_store8(p.out_hi, p.out_lo, (m0 + wl) * p.Kp + k8 * 8, p.fmt, x);
             }
+            ++iter;
         }
-        if (threadIdx.x == 0) trace_end(blp, claims.done());
+        if (threadIdx.x == 0) trace_end(blp, iter);
         return;
     }
     for (;;) {

@@ -1134,16 +1134,11 @@ int finalize_model(gpx_model &m) {
             q.tile_elems = (int)std::max<long long>(256, std::min<long long>(2 * kMaxTileVectors, total / (8LL * m.sm_count) / 32 * 32));
             q.total_tiles = (int)((total + q.tile_elems - 1) / q.tile_elems);
             {
-                // fp32 NCHW input: tiles of one output row or an equal part of it (64 pixels at most where whole
-                // rows would not give every SM four tiles, or their window does not fit), staged window
+                // fp32 NCHW input: tiles of up to 64 output pixels of one output row, staged window
                 const char *off = getenv("GPX_IM2COL_WINDOW");
-                int chunks = 1, win_w = n.W;
-                auto window_of = [&]() { return (long long)src.C * n.k * ((win_w - 1) * n.stride + n.k); };
-                while (win_w > 64 && (window_of() > kIm2colWindowFloats || (long long)n.N * n.H * chunks < 4LL * m.sm_count)) {
-                    ++chunks;
-                    win_w = (n.W + chunks - 1) / chunks;
-                }
-                const long long window = window_of();
+                const int chunks = (n.W + 63) / 64;
+                const int win_w = (n.W + chunks - 1) / chunks;
+                const long long window = (long long)src.C * n.k * ((win_w - 1) * n.stride + n.k);
                 if (m.storages[src.storage].kind == Storage::InputF32 && window <= kIm2colWindowFloats &&
                     !(off && off[0] == '0') && !n.via_s2d) {
                     q.win_w = win_w;
