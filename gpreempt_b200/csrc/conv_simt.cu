@@ -460,6 +460,13 @@ pool_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
     if (threadIdx.x == 0) trace_end(blp, claims.done());
 }
 
+// Eight packed words to 32-byte aligned global memory, one whole sector.
+__device__ __forceinline__ void st_sector(plane_bits *ptr, const unsigned (&r)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(ptr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
+                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+
 // Patch matrix for the tensor-core GEMM: one thread-iteration writes eight consecutive columns
 // (one 16-byte vector per plane) of one row.
 __global__ void __launch_bounds__(kPoolThreads)
@@ -676,7 +683,74 @@ im2col_kernel(const __grid_constant__ Im2colParams p, BlpArgs blp) {
     if (threadIdx.x == 0) trace_end(blp, iter);
 }
 
+// Patch matrix of a 3x3 filter over a three-channel fp32 NCHW input (VGG, MobileNetV2, Inception-v3): a thread
+// takes one pixel and writes its whole row of 27 values and five zeros.  Neighbouring threads read
+// neighbouring elements, 27 independent loads each that L1 and L2 serve after the first, and a row is two
+// 32-byte stores a plane, whole sectors.  Bound by the writes and, at one image, by one chain
+// load - convert - store.  (A window of the image in shared memory, a vector of eight columns a thread: four barriers
+// and ~2 800 cycles a tile of one image row, 63 us for 224x224, 16 images fp16; FIGURES.)
+constexpr int kRgbK = 27, kRgbKp = 32;
+
+template <int FMT>
+__global__ void __launch_bounds__(kPoolThreads)
+patches_rgb_kernel(const __grid_constant__ Im2colParams p, BlpArgs blp) {
+    pdl_enter();
+    __shared__ int s_tile;
+    if (threadIdx.x == 0) trace_begin(blp);
+    const int H = p.in.l.H, W = p.in.l.W;
+    TileClaims claims(blp, blp.preempted != nullptr, s_tile);
+    for (int tile = claims.first(); tile >= 0; tile = claims.next()) {
+        const unsigned begin = (unsigned)tile * p.tile_elems;
+        const unsigned end = min(begin + (unsigned)p.tile_elems, (unsigned)p.M);
+        for (unsigned m = begin + threadIdx.x; m < end; m += kPoolThreads) {
+            const int wo = (int)(m % (unsigned)p.Wo);
+            const unsigned t = m / (unsigned)p.Wo;
+            const int ho = (int)(t % (unsigned)p.Ho), n = (int)(t / (unsigned)p.Ho);
+            const int h0 = ho * p.stride - p.pad, w0 = wo * p.stride - p.pad;
+            const float *img = p.in.f32 + (size_t)n * 3 * H * W;
+            float x[kRgbKp];
+#pragma unroll
+            for (int k = 0; k < kRgbKp; ++k) {  // columns are (fh, fw, channel)
+                x[k] = 0.f;
+                if (k < kRgbK) {
+                    const int hi = h0 + k / 9, wi = w0 + k / 3 % 3;
+                    if (hi >= 0 && hi < H && wi >= 0 && wi < W) x[k] = __ldg(img + ((size_t)(k % 3) * H + hi) * W + wi);
+                }
+            }
+            claims.ahead();
+            const size_t off = (size_t)m * kRgbKp;
+#pragma unroll
+            for (int c = 0; c < kRgbKp; c += 16) {
+                unsigned hi[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) hi[q] = pf_pack2(x[c + 2 * q], x[c + 2 * q + 1], FMT);
+                st_sector(p.out_hi + off + c, hi);
+                if (FMT == PF_SPLIT) {
+                    unsigned lo[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        lo[q] = pf_pack2(x[c + 2 * q] - __uint_as_float(hi[q] << 16),
+                                         x[c + 2 * q + 1] - __uint_as_float(hi[q] & 0xffff0000u), PF_SPLIT);
+                    st_sector(p.out_lo + off + c, lo);
+                }
+            }
+        }
+    }
+    if (threadIdx.x == 0) trace_end(blp, claims.done());
+}
+
+static auto patches_rgb_instance(int fmt) {
+    return fmt == PF_SPLIT ? patches_rgb_kernel<PF_SPLIT> : (fmt == PF_F16 ? patches_rgb_kernel<PF_F16> : patches_rgb_kernel<PF_BF16>);
+}
+
+int im2col_rgb_grid(int sm_count, int total_tiles) {
+    int per_sm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, patches_rgb_instance(PF_SPLIT), kPoolThreads, 0);
+    return (int)std::min<long long>((long long)sm_count * std::max(per_sm, 1), total_tiles);
+}
+
 cudaError_t im2col_launch(const Im2colParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
+    if (p.rgb) return launch_layer(patches_rgb_instance(p.fmt), grid, kPoolThreads, 0, s, p, blp);
     return launch_layer(im2col_kernel, grid, kPoolThreads, 0, s, p, blp);
 }
 

@@ -225,10 +225,13 @@ struct Im2colParams {
     // eight consecutive columns are eight channels of one tap, so a thread-iteration copies one
     // 16-byte vector per plane, or writes zeros where the tap falls outside the image.
     int planes_vec;
+    // Pixel mode (3x3 filter of a three-channel fp32 NCHW input): one thread writes a whole row.
+    int rgb;
     int pad_w;              // horizontal padding (plane mode; `pad` is the vertical one)
 };
 constexpr int kIm2colWindowFloats = 4096;
 cudaError_t im2col_launch(const Im2colParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
+int im2col_rgb_grid(int sm_count, int total_tiles);
 
 // LayerNorm over the channels of a [rows][H] matrix (H <= 1024, multiple of 8).  With `ids` set
 // the input row is the sum of the word, position and token-type embeddings instead of planes.

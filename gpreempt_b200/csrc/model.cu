@@ -1146,8 +1146,15 @@ int finalize_model(gpx_model &m) {
                     q.total_tiles = n.N * n.H * chunks;
                 }
             }
+            if (m.storages[src.storage].kind == Storage::InputF32 && !n.via_s2d && src.C == 3 && n.k == 3 && q.Kp == 32) {
+                // a block of pixels for every SM, at most four pixels a thread
+                q.rgb = 1;
+                q.win_w = 0;
+                q.tile_elems = (int)std::max<long long>(32, std::min<long long>(1024, (q.M / (8LL * m.sm_count) + 31) / 32 * 32));
+                q.total_tiles = (q.M + q.tile_elems - 1) / q.tile_elems;
+            }
             ki.total_tiles = q.total_tiles;
-            ki.grid = (int)std::min<long long>((long long)m.sm_count * 8, q.total_tiles);
+            ki.grid = q.rgb ? im2col_rgb_grid(m.sm_count, q.total_tiles) : (int)std::min<long long>((long long)m.sm_count * 8, q.total_tiles);
             ki.flops = 0;
             ki.bytes = 4.0 * (double)src.N * src.H * src.W * src.C + 4.0 * (double)q.M * q.Kp;
             m.kernels.push_back(ki);
