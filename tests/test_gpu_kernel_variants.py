@@ -109,7 +109,7 @@ def test_classifier_rows_and_large_depthwise_layers(gpx, oracle, model, batch, d
     assert ex.error() == (0, 0)
     taps = {}
     heads = oracle.forward(model, ex.model.params(), data, taps=taps)
-    for name in [n for n in taps if n.endswith(".dw")]:
+    for name in [n for n in taps if n.endswith(".dw") or n == "features.0"]:
         assert _rel(ex.model.get(name).reshape(taps[name].shape), taps[name]) <= TOL[dtype], name
     assert _rel(ex.get_output("heads"), heads) <= TOL[dtype]
     ex.clear()
