@@ -87,7 +87,7 @@ struct CgemmCfg {
 // Message of a ring stage: CMSG_DATA + number of K blocks, CMSG_RES + index of the residual block, or
 // the word was seen raised.  (The end of a CTA's schedule needs no message: every role counts tiles.)
 enum : int { CMSG_STOP = 1, CMSG_DATA = 4, CMSG_RES = 16 };
-enum : int { CEPI_COMPLETE = 0, CEPI_PARTIAL = 1 };
+enum : int { CEPI_COMPLETE = 0, CEPI_PARTIAL = 1, CEPI_EXIT = 2 };
 
 struct CgemmControl {
     unsigned long long full[8];
@@ -100,7 +100,7 @@ struct CgemmControl {
     int stage_msg[8];
     int epi_kind[2];
     int epi_k_done[2];
-    int epi_go;
+    int epi_go[2];
     int raised;      // the word was up when this CTA started
     int word_up;     // the polling warp has seen the word raised
     int poll_done;   // the producer is through: the polling warp returns
@@ -222,7 +222,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             mbar_arrive_expect_tx(smem_u32(&ctl->landed), kCBM * (BN + 4) * 4);
         }
         ctl->abort_flag = 0;
-        ctl->epi_go = 0;
+        ctl->epi_go[0] = ctl->epi_go[1] = 0;
         ctl->raised = 0;
         ctl->word_up = 0;
         ctl->poll_done = 0;
@@ -625,7 +625,23 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 mbar_arrive(smem_u32(&ctl->tmem_full[buf]));
             }
             __syncwarp();
-            if (end != CEPI_COMPLETE) break;
+            if (end != CEPI_COMPLETE) {
+                if (p.alternate) {
+                    // the other group of epilogue warps waits for a tile that will not come
+                    const int other = buf ^ 1;
+                    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->tmem_empty[other]), ((seg + 1) >> 1) & 1, abort_flag, kCWaitLimitNs))) {
+                        if (lane == 0) fail(204);
+                        break;
+                    }
+                    if (issuer) {
+                        ctl->epi_kind[other] = CEPI_EXIT;
+                        mma_commit(smem_u32(&ctl->tmem_full[other]));
+                        mbar_arrive(smem_u32(&ctl->tmem_full[other]));
+                    }
+                    __syncwarp();
+                }
+                break;
+            }
         }
 #ifdef GPX_CGEMM_TIMING
         if (lane == 0) {
@@ -738,14 +754,22 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     } else {
         // ------------------------------------------------------------------ epilogue
         const int quarter = warp & 3;
-        const int part = (warp - 2) >> 2;                 // which share of the columns
-        const int c_lo = part * (BN / Cfg::kEpiParts), c_hi = c_lo + BN / Cfg::kEpiParts;
-        // this warp's share of the columns of one accumulator buffer, for spill and restore
-        constexpr int kSpillCols = kBufCols / Cfg::kEpiParts;
-        const int s_lo = part * kSpillCols, s_hi = s_lo + kSpillCols;
+        // Either all warps drain every tile, each its share of the columns, or (p.alternate) two groups take
+        // the tiles, and with them the accumulator buffers, in turn: draining a tile is a chain of
+        // ~2 800 cycles (wait, tensor memory, conversion, store, hand-over) however few columns a warp has,
+        // and a layer of one or two K blocks waits for it.
+        const int groups = p.alternate ? 2 : 1;
+        const int parts = Cfg::kEpiParts / groups;        // warps of a group per lane quarter
+        const int share = (warp - 2) >> 2, group = share / parts, part = share - group * parts;
+        const int group_threads = 128 * parts;
+        const int c_lo = part * (BN / parts), c_hi = c_lo + BN / parts;
+        auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(group_threads) : "memory"); };
+        // this warp's columns of one accumulator buffer when it restores (all warps) or spills (its group)
+        constexpr int kRestoreCols = kBufCols / Cfg::kEpiParts;
+        const int spill_cols = kBufCols / parts;
         const int row = quarter * 32 + lane;
         const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
-        const bool leader = threadIdx.x == 64;
+        const bool leader = (int)threadIdx.x == 64 + group * group_threads;
         if (in_cluster) {
             // What the finishing step needs, ahead of the products: destination, bias, residual.
             const SplitKParams &fin = p.fin;
@@ -786,7 +810,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         }
         uint32_t v[32];
         if (first_k > 0) {
-            for (int c = s_lo; c < s_hi; c += 32) {
+            for (int c = share * kRestoreCols; c < (share + 1) * kRestoreCols; c += 32) {
                 // Spill layout: private to this kernel, so it is chosen for the stores: the j-th
                 // 16-byte piece of a 32-column chunk of all 128 rows is contiguous, one warp store
                 // writes 512 consecutive bytes (row-major rows 2 KB apart cost a line per thread).
@@ -804,12 +828,12 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             tmem_st_wait();
         }
         tc_fence_before_sync();
-        asm volatile("bar.sync 1, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
-        if (leader)
+        asm volatile("bar.sync 3, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
+        if (threadIdx.x == 64)
             for (int b = 0; b < 2; ++b) mbar_arrive(smem_u32(&ctl->tmem_empty[b]));
 
-        int it = first_iter;
-        int seg_k0 = first_k;
+        int it = first_iter + group;
+        int seg_k0 = group == 0 ? first_k : 0;
         int tiles_done = 0;
         const int img = p.in_hs * p.in_ws;
         // Fields the drain loop needs, in registers: the loop is full of asm statements that clobber
@@ -822,18 +846,19 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         const bf16_bits *const res_hi = p.res_hi, *const res_lo = p.res_lo;
         float bias_next = 0.f;  // this thread's bias element of the next tile to drain
         if (bias) {
-            const int t = (int)threadIdx.x - 64;
-            const int first = blockIdx.x + first_iter * gridDim.x;
+            const int t = (int)threadIdx.x - 64 - group * group_threads;
+            const int first = blockIdx.x + it * gridDim.x;
             if (t < BN && first < total_tiles) bias_next = __ldg(bias + tile_at(first).n_blk * BN + t);
         }
         TCK(t_epi0);
 #ifdef GPX_CGEMM_TIMING
         long long e_wait = 0, e_tmem = 0, e_math = 0, e_store = 0, e_bar = 0;
 #endif
-        for (uint32_t seg = 0;; ++seg) {
+        for (uint32_t seg = group;; seg += groups) {
             const int tile = blockIdx.x + it * gridDim.x;
             if (tile >= total_tiles) {
-                if (leader && resumable) {
+                // (of two groups, the one that had the last tile: the other's end says nothing about that tile)
+                if (leader && resumable && (groups == 1 || tile - (int)gridDim.x >= total_tiles)) {
                     slot->next_iter = it;
                     slot->k_done = 0;
                     slot->grid = gridDim.x;
@@ -851,10 +876,10 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             // and the request for the tile after this one is issued here, so the round trip
             // overlaps the drain of this tile instead of delaying its start.
             if (bias) {
-                const int t = (int)threadIdx.x - 64;
+                const int t = (int)threadIdx.x - 64 - group * group_threads;
                 if (t < BN) {
                     ctl->bias_s[buf][t] = bias_next;
-                    const int after = tile + gridDim.x;
+                    const int after = tile + groups * gridDim.x;
                     if (after < total_tiles) bias_next = __ldg(bias + tile_at(after).n_blk * BN + t);
                 }
             }
@@ -893,19 +918,20 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             if (leader) {
                 bool ok = mbar_wait(smem_u32(&ctl->tmem_full[buf]), (seg >> 1) & 1, abort_flag, kCWaitLimitNs);
                 if (!ok) fail(301);
-                ctl->epi_go = ok ? 1 : 0;
+                ctl->epi_go[group] = ok ? 1 : 0;
             }
-            asm volatile("bar.sync 1, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
+            group_sync();
 #ifdef GPX_CGEMM_TIMING
             e_wait += clock64() - t_wait0;
 #endif
 #ifdef GPX_CGEMM_TIMING
             if (leader && seg == 0) TADD(17, clock64() - t_begin);
 #endif
-            if (!ctl->epi_go) break;
+            if (!ctl->epi_go[group]) break;
             tc_fence_after_sync();
             const int kind = ctl->epi_kind[buf];
             const int k_done = ctl->epi_k_done[buf];
+            if (kind == CEPI_EXIT) break;
             if (kind == CEPI_COMPLETE) {
                 // Every lane owns one row of the tile (its TMEM lane): 16 columns of a plane are 32
                 // contiguous bytes of that row, one 256-bit access, a whole sector.
@@ -1027,14 +1053,14 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     e_store += clock64() - t_p2;
 #endif
                 }
-                ++it;
+                it += groups;
                 ++tiles_done;
                 seg_k0 = 0;
                 if (in_cluster) {
                     // Every share of rows goes to the CTA that finishes it as one bulk copy (landing area:
                     // [split][row of the share][BN + 4 floats] in that CTA's last ring stages).
                     fence_proxy_async();
-                    asm volatile("bar.sync 1, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
+                    group_sync();
                     const int owner = (int)threadIdx.x - 64;
                     if (owner < p.k_splits) {
                         const uint32_t share = (uint32_t)(kCBM / p.k_splits * (BN + 4) * 4);
@@ -1047,7 +1073,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 }
                 tc_fence_before_sync();
                 TCK(t_b0);
-                asm volatile("bar.sync 1, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
+                group_sync();
 #ifdef GPX_CGEMM_TIMING
                 e_bar += clock64() - t_b0;
 #endif
@@ -1060,7 +1086,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             // CEPI_PARTIAL
             const int keep_k = p.drop_on_stop ? 0 : k_done;
             if (keep_k > seg_k0) {
-                for (int c = s_lo; c < s_hi; c += 32) {
+                for (int c = part * spill_cols; c < (part + 1) * spill_cols; c += 32) {
                     tmem_ld_32x32(t_acc + c, v);
                     tmem_ld_wait();
                     uint4 *dst = reinterpret_cast<uint4 *>(spill) + (size_t)(c / 32) * 8 * kCBM + row;

@@ -96,6 +96,7 @@ struct CgemmParams {
     // its partial rows into their owners' shared memory - the additions of splitk_finish_kernel
     // without the workspace round trip and the second launch.
     int cluster_reduce;
+    int alternate;           // 1: two groups of epilogue warps take the tiles in turn (short K loops, many tiles)
     SplitKParams fin;        // what the finishing pass needs (bias, residual, activation, output)
     CgemmSlot *slots;        // one per CTA of this kernel
     float *spill;            // [grid][128*BN] fp32, shared by the kernels of one executor

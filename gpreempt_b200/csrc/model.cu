@@ -1313,6 +1313,11 @@ int finalize_model(gpx_model &m) {
                                out.layout.rows == il.rows && p.in_off == 0 && res_plain && !(full_map_dense(n, src) && !n.via_im2col))
                                   ? 1 : 0;
         }
+        {
+            const char *e1 = getenv("GPX_ALT1"), *e2 = getenv("GPX_ALT2");
+            const int lim = m.fmt == PF_SPLIT ? (e2 ? atoi(e2) : 0) : (e1 ? atoi(e1) : 0);
+            p.alternate = p.k_splits == 1 && all_kb + p.res_kb <= lim && out_tiles >= 4 * m.sm_count ? 1 : 0;
+        }
         kn.total_tiles = out_tiles * p.k_splits;
         kn.grid = std::min(kn.total_tiles, m.sm_count);
         m.max_cgemm_grid = std::max(m.max_cgemm_grid, kn.grid);
