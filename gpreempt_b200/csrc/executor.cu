@@ -166,42 +166,19 @@ int gpx_exec_destroy(gpx_exec *e) {
     return GPX_SUCC;
 }
 
-int gpx_exec_set_word(gpx_exec *e, gpx_word *w) {
-    GPX_REQUIRE(e && w, GPX_FAIL, "NULL argument");
-    void *d = nullptr;
-    GPX_TRY(gpx_word_dptr(w, &d));
-    GPX_REQUIRE(!e->graph_exec, GPX_FAIL, "set the preempt word before capturing the graph");
-    e->word_dptr = (const int *)d;
-    return GPX_SUCC;
-}
-
-int gpx_exec_set_word_dptr(gpx_exec *e, const void *dptr) {
-    GPX_REQUIRE(e && dptr, GPX_FAIL, "NULL argument");
-    GPX_REQUIRE(((uintptr_t)dptr % 4) == 0, GPX_FAIL, "the preempt word must be 4-byte aligned");
-    GPX_REQUIRE(!e->graph_exec || e->word_dptr == (const int *)dptr, GPX_FAIL,
-                "set the preempt word before capturing the graph");
-    e->word_dptr = (const int *)dptr;
-    return GPX_SUCC;
-}
-
-int gpx_exec_enable_trace(gpx_exec *e, int on) {
-    GPX_REQUIRE(e, GPX_FAIL, "NULL executor");
-    GPX_REQUIRE(!e->graph_exec, GPX_FAIL, "enable tracing before capturing the graph");
-    e->trace_on = on != 0;
-    return GPX_SUCC;
-}
-
 // Kernels of the longest forward that execute turns into a graph of its own.  With the word up every kernel
 // still queued starts once to find that out, ~2 us each, and a graph queues all of them at once: beyond
 // this many the drain would show it.
 constexpr size_t kOwnGraphKernels = 64;
 
-// The forward as a graph, made by the first execute (and again when what it depends on has changed): kernel by
-// kernel the host takes up to 4 us a launch, longer than most kernels of a small model run (15-kernel BERT:
+static bool own_graph_applies(const gpx_exec *e) {
+    return !e->graph_exec && e->kind == GPX_EXEC_BLP && e->word_dptr && e->model->kernels.size() <= kOwnGraphKernels;
+}
+
+// The forward as a graph, made when the word is set (for best-effort streams, ~0.4 ms) and again by an execute for
+// which something it depends on has changed: kernel by kernel the host takes up to 4 us a launch, longer than most kernels of a small model run (15-kernel BERT:
 // 63 us of host for 80 us of GPU).
-static int refresh_own_graph(gpx_exec *e, cudaStream_t s) {
-    int priority = 0;
-    if (s) GPX_CUDA(cudaStreamGetPriority(s, &priority));
+static int refresh_own_graph(gpx_exec *e, int priority) {
     if (e->own_graph && e->own_word == e->word_dptr && e->own_priority == priority && e->own_trace == e->trace_on &&
         e->own_drop == e->drop_tile_in_flight)
         return GPX_SUCC;
@@ -222,6 +199,7 @@ static int refresh_own_graph(gpx_exec *e, cudaStream_t s) {
         }
         err = cudaStreamEndCapture(c, &graph);
         if (st == GPX_SUCC && err == cudaSuccess) err = cudaGraphInstantiate(&e->own_graph, graph, 0);
+        if (st == GPX_SUCC && err == cudaSuccess) err = cudaGraphUpload(e->own_graph, c);
         if (graph) cudaGraphDestroy(graph);
     }
     cudaStreamDestroy(c);
@@ -234,15 +212,41 @@ static int refresh_own_graph(gpx_exec *e, cudaStream_t s) {
     return GPX_SUCC;
 }
 
+int gpx_exec_set_word(gpx_exec *e, gpx_word *w) {
+    GPX_REQUIRE(e && w, GPX_FAIL, "NULL argument");
+    void *d = nullptr;
+    GPX_TRY(gpx_word_dptr(w, &d));
+    GPX_REQUIRE(!e->graph_exec, GPX_FAIL, "set the preempt word before capturing the graph");
+    e->word_dptr = (const int *)d;
+    return own_graph_applies(e) ? refresh_own_graph(e, device_info().prio_least) : GPX_SUCC;
+}
+
+int gpx_exec_set_word_dptr(gpx_exec *e, const void *dptr) {
+    GPX_REQUIRE(e && dptr, GPX_FAIL, "NULL argument");
+    GPX_REQUIRE(((uintptr_t)dptr % 4) == 0, GPX_FAIL, "the preempt word must be 4-byte aligned");
+    GPX_REQUIRE(!e->graph_exec || e->word_dptr == (const int *)dptr, GPX_FAIL,
+                "set the preempt word before capturing the graph");
+    e->word_dptr = (const int *)dptr;
+    return own_graph_applies(e) ? refresh_own_graph(e, device_info().prio_least) : GPX_SUCC;
+}
+
+int gpx_exec_enable_trace(gpx_exec *e, int on) {
+    GPX_REQUIRE(e, GPX_FAIL, "NULL executor");
+    GPX_REQUIRE(!e->graph_exec, GPX_FAIL, "enable tracing before capturing the graph");
+    e->trace_on = on != 0;
+    return GPX_SUCC;
+}
+
 int gpx_exec_execute(gpx_exec *e, gpx_stream stream) {
     GPX_REQUIRE(e, GPX_FAIL, "NULL executor");
     cudaStream_t s = as_stream(stream);
-    if (!e->graph_exec && e->kind == GPX_EXEC_BLP && e->model->kernels.size() <= kOwnGraphKernels) {
-        GPX_REQUIRE(e->word_dptr, GPX_FAIL, "BLP executor has no preempt word (gpx_exec_set_word)");
+    if (own_graph_applies(e)) {
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         if (s) GPX_CUDA(cudaStreamIsCapturing(s, &capturing));
         if (capturing == cudaStreamCaptureStatusNone) {
-            GPX_TRY(refresh_own_graph(e, s));
+            int priority = 0;
+            if (s) GPX_CUDA(cudaStreamGetPriority(s, &priority));
+            GPX_TRY(refresh_own_graph(e, priority));
             GPX_CUDA(cudaGraphLaunch(e->own_graph, s));
             g_kernel_launches.fetch_add(e->model->kernels.size(), std::memory_order_relaxed);
             return GPX_SUCC;
@@ -272,6 +276,10 @@ int gpx_exec_capture_graph(gpx_exec *e, gpx_stream stream) {
     GPX_REQUIRE(e, GPX_FAIL, "NULL executor");
     GPX_REQUIRE(stream, GPX_FAIL, "graph capture needs a non-default stream");
     GPX_REQUIRE(!e->graph_exec, GPX_FAIL, "graph already captured");
+    if (e->own_graph) {
+        GPX_CUDA(cudaGraphExecDestroy(e->own_graph));
+        e->own_graph = nullptr;
+    }
     cudaStream_t s = as_stream(stream);
     size_t nk = e->model->kernels.size();
     // Projection shortcuts as a parallel branch (non-preemptible executors): the kernels of a
