@@ -937,8 +937,11 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 // contiguous bytes of that row, one 256-bit access, a whole sector.
                 const bool use_res = !partial && !out_f32 && res_hi && valid;
                 constexpr int CH = (TWO || AFF || BN == 256) ? 16 : 32;  // columns per piece
+                // (columns past the real output, a quarter to a half of a tile for a DenseNet layer, are left out;
+                // partial sums go out whole)
+                const int c_end = partial || in_cluster || c_hi < col_lim ? c_hi : col_lim;
 #pragma unroll 1
-                for (int c = c_lo; c < c_hi; c += CH) {
+                for (int c = c_lo; c < c_end; c += CH) {
                     float f[CH];
                     // The residual is requested first so its latency overlaps the TMEM reads.
                     TCK(t_p0);
