@@ -757,7 +757,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         // Either all warps drain every tile, each its share of the columns, or (p.alternate) two groups take
         // the tiles, and with them the accumulator buffers, in turn: draining a tile is a chain of
         // ~2 800 cycles (wait, tensor memory, conversion, store, hand-over) however few columns a warp has,
-        // and a layer of one or two K blocks waits for it.
+        // and a layer of one or two K blocks waits for it (VGG-16's first, 16 images fp16: 70 -> 54 us).
         const int groups = p.alternate ? 2 : 1;
         const int parts = Cfg::kEpiParts / groups;        // warps of a group per lane quarter
         const int share = (warp - 2) >> 2, group = share / parts, part = share - group * parts;
