@@ -1070,7 +1070,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                         bulk_copy_to_cluster(cluster_map_shared(smem_base + (uint32_t)(nst * Cfg::kStageBytes) + cluster_ctarank() * share, (uint32_t)owner),
                                              smem_base + (uint32_t)owner * share, share,
                                              cluster_map_shared(smem_u32(&ctl->landed), (uint32_t)owner));
-                        bulk_copies_done();  // the source is this CTA's memory: it stays until they are through
                     }
                     break;
                 }
@@ -1128,16 +1127,21 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         // once every CTA of the cluster has copied its partial rows of them there: the S partial rows
         // are added in split order from zero, exactly as splitk_finish_kernel adds the workspace
         // rows, then bias, residual, activation, store.  Where the rows go, the bias and the residual
-        // were fetched before the products were waited for.  Nothing is read from a peer, so a CTA may
-        // exit when it is done.  (Pulling the rows from the peers after a cluster barrier, one split at
-        // a time, and a second barrier before the exit made this step 4 us long, BERT-base b1 7.4 us per
-        // projection; storing them to the peers element by element, 2 us.)  A CTA that failed waits
-        // here as well, so that no copy finds its memory gone.
-        if (warp >= 2 && warp < Cfg::kPollWarp) {
+        // were fetched before the products were waited for.  The copies this CTA sent still read its ring
+        // until they have landed, and only their owners see that: every CTA arrives on the cluster barrier
+        // once its own rows are complete and leaves when all have, so no ring is handed to a successor's
+        // loads under a copy.  The barrier hides behind the finishing step.  (Pulling the rows from the
+        // peers after a cluster barrier, one split at a time, and a second barrier before the exit made this
+        // step 4 us long, BERT-base b1 7.4 us per projection; storing them to the peers element by element,
+        // 2 us.)  A CTA that failed waits here as well, so that no copy finds its memory gone.
+        const bool finishes = warp >= 2 && warp < Cfg::kPollWarp;
+        if (finishes) {
             volatile int never = 0;
             if (!mbar_wait(smem_u32(&ctl->landed), 0, &never, kCWaitLimitNs + kCWaitLimitNs / 2)) fail(601);
         }
-        if (warp >= 2 && warp < Cfg::kPollWarp) {
+        __syncwarp();
+        cluster_arrive();
+        if (finishes) {
             const float *land = reinterpret_cast<const float *>(smem + nst * Cfg::kStageBytes);
             const SplitKParams &fin = p.fin;
             auto finish = [&](auto splits) {
@@ -1193,7 +1197,8 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
 #ifdef GPX_CGEMM_TIMING
         if (threadIdx.x == 64) TADD(21, clock64() - t_begin);
 #endif
-        __syncthreads();  // (tensor memory is released below by warp 1)
+        __syncwarp();
+        cluster_wait();  // (tensor memory is released below by warp 1)
     } else {
         __syncthreads();
     }

@@ -116,11 +116,6 @@ __device__ __forceinline__ void bulk_copy_to_cluster(uint32_t dst, uint32_t src,
                  "r"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
-// Waits until the bulk copies this thread has issued have completed.
-__device__ __forceinline__ void bulk_copies_done() {
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-}
 
 // ---- CTA pairs (cta_group::2): two CTAs of a cluster work on one tile -----------------------------
 // The even CTA leads: its barriers count the loads of both, it issues the products, and commits arrive

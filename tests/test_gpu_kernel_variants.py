@@ -207,3 +207,28 @@ def test_resets_are_ordered_before_later_launches(gpx, oracle):
     assert np.array_equal(dy.download(np.float32, n).view(np.uint32), want.view(np.uint32))
     for o in (dx, dy, ctx, word, *streams):
         (o.free if hasattr(o, "free") else o.destroy)()
+
+
+@pytest.mark.parametrize("model,seq,dtype", [("resnet50", 0, "float32"), ("mobilenet_v2", 0, "bfloat16"), ("bert_base", 128, "float16")])
+def test_cluster_reduction_back_to_back(gpx, model, seq, dtype):
+    """Batch-1 forwards queued behind one another: a CTA of a cluster may leave only when its partial sums have
+    reached their owners, because the kernel behind it fills the shared memory it leaves.  The preemptible
+    executor reduces through memory and has the same sums in the same order."""
+    data = np.random.default_rng(4).integers(0, 30522, (1, seq)).astype(np.int64) if seq else _images(gpx, 1, 4)
+    blp = gpx.BLPExecutor()
+    blp.init(model, batch=1, seed=3, seq_len=seq, dtype=dtype)
+    word, s = gpx.PreemptWord(1), gpx.Stream(0)
+    blp.set_word(word)
+    blp.set_input("data", data)
+    blp.execute(s)
+    s.sync()
+    want = blp.get_output("heads")
+    ex = gpx.BaseExecutor()
+    ex.init(model, batch=1, seed=3, seq_len=seq, dtype=dtype)
+    ex.set_input("data", data)
+    for _ in range(20):
+        for _ in range(20):
+            ex.execute(s)
+        s.sync()
+        assert ex.error() == (0, 0) and np.array_equal(ex.get_output("heads"), want)
+    ex.clear(), blp.clear(), word.destroy(), s.destroy()
