@@ -12,10 +12,13 @@
 // scores once, exponentiates them and writes the probabilities as a 16-bit A operand into shared
 // memory (128-byte swizzled, as TMA would); P V is a 128x64x64 product accumulated in tensor memory,
 // whose B operand is the value tile as it lies in HBM (rows are keys): the descriptor names it
-// MN-major, so no transposed copy of the values exists.  The accumulated output is rescaled only when
-// a row's maximum has grown by more than 2^8 since its last rescaling (the exponent reference of a row
-// may lag behind its maximum: the factor cancels in the final division), which after the first block
-// hardly ever happens.
+// MN-major, so no transposed copy of the values exists.  The accumulated output is rescaled whenever a row's
+// maximum has grown, so that the largest probability of a block is 1 and exact in 16 bits, and the normaliser
+// sums the probabilities as rounded, so that an error they share cancels.  (Letting the exponent's
+// reference lag behind the maximum by up to 2^8, as published attention kernels do, rounds the largest
+// probability too.  Distance from 64 bits of rows that one key dominates, fp16: 2.32e-4 of the norm with
+// the lag, 2.08e-4 without, 2.07e-4 with the rounded sum as well, where rounding the result is 2.06e-4; a layer
+// of BERT-base s512 b32: 72, 77 and 78 us.)
 //
 // The scores of the next block are computed as soon as this block's have left tensor memory for
 // registers (two key buffers), under this block's softmax; the values of the next block arrive
@@ -23,9 +26,9 @@
 //
 // What bounds it: the special-function unit has 128 x 64 exponentials a block (512 cycles at 16 an SM
 // and cycle, 22 us a layer of BERT-base s512 b32), everything else is latency between the two products;
-// two CTAs of two independent warpgroups per SM overlap each other's, to ~40 % of that unit's rate.
+// two CTAs of two independent warpgroups per SM overlap each other's, to ~30 % of that unit's rate.
 // BERT-base s512 b32, a layer: one warpgroup of 128 keys a block with the output folded into registers
-// and a transposing kernel in front took 89 + 16 us; scores and context issued in line, 82; this, 72.
+// and a transposing kernel in front took 89 + 16 us; scores and context issued in line, 82; this, 78.
 // (Tried, at the same time or slower: a warp of its own for copies and products, two buffers of
 // values, the next tile claimed under the merge of this one.)
 // The first warp of a warpgroup issues TMA and MMA; every wait is bounded, and a wait that gives up raises
@@ -52,7 +55,6 @@ constexpr uint32_t kFaGroupBytes = 3 * kFaKBytes + kFaPBytes;
 constexpr uint32_t kFaSmem = kFaQBytes + 2 * kFaGroupBytes + 1024 + 2304;
 constexpr uint32_t kFaTmemCols = 256;  // per warpgroup: S 64 columns, output 64 columns
 constexpr unsigned long long kFaWaitLimitNs = 2000000000ull;
-constexpr float kFaRescale = 8.0f;     // log2 of the growth of a row maximum that forces a rescale
 
 struct FaControl {
     unsigned long long bar_q;
@@ -233,9 +235,8 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             } else {
                 m = m_new;
             }
-            if (__any_sync(0xffffffffu, m_new > m + kFaRescale)) {
-                const float m_to = m_new > m + kFaRescale ? m_new : m;
-                const float alpha = fa_ex2(m - m_to);
+            if (__any_sync(0xffffffffu, m_new > m)) {
+                const float alpha = fa_ex2(m - m_new);
                 tc_fence_after_sync();
 #pragma unroll
                 for (int c = 0; c < kFaD; c += 16) {
@@ -248,7 +249,7 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
                 }
                 tmem_st_wait();
                 l *= alpha;
-                m = m_to;
+                m = m_new;
             }
             const int r8 = row & 7;
             unsigned char *prow = pP + (row >> 3) * 1024 + r8 * 128;
@@ -260,9 +261,9 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const float2 x = fma2(make_float2(__uint_as_float(v[c + 2 * i]), __uint_as_float(v[c + 2 * i + 1])), sc2, neg_m);
-                    const float e0 = fa_ex2(x.x), e1 = fa_ex2(x.y);
-                    lsum[i] += e0 + e1;
-                    pk[i] = pf_pack2(e0, e1, FMT);
+                    pk[i] = pf_pack2(fa_ex2(x.x), fa_ex2(x.y), FMT);
+                    const float2 e = pf_unpack2(pk[i], FMT);
+                    lsum[i] += e.x + e.y;
                 }
                 // eight keys = one 16-byte piece of this row, at piece index XOR (row mod 8)
                 *reinterpret_cast<uint4 *>(prow + (((c >> 3) ^ r8) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);

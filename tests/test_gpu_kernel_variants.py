@@ -232,3 +232,28 @@ def test_cluster_reduction_back_to_back(gpx, model, seq, dtype):
         s.sync()
         assert ex.error() == (0, 0) and np.array_equal(ex.get_output("heads"), want)
     ex.clear(), blp.clear(), word.destroy(), s.destroy()
+
+
+@pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
+def test_attention_rows_that_one_key_dominates(gpx, dtype):
+    """With scores spread wide a row of the context is nearly one row of the values, so its only error is the
+    rounding of the result, the probability of the dominating key being exactly 1.  From the stored queries,
+    keys and values, in 64 bits."""
+    import torch
+
+    ex = gpx.BaseExecutor()
+    ex.init("bert_tiny", batch=16, seed=1, seq_len=512, dtype=dtype)
+    name = "encoder.layer.0.attention."
+    ex.model.set(name + "self.query.weight", ex.model.get(name + "self.query.weight") * 192)
+    ex.set_input("data", np.random.default_rng(1).integers(0, 1000, (16, 512)).astype(np.int64))
+    ex.execute()
+    assert ex.error() == (0, 0)
+    q, k, v = (torch.from_numpy(ex.model.get(name + "self." + part + ".out")).double() for part in ("query", "key", "value"))
+    got = torch.from_numpy(ex.model.get(name + "context")).double()
+    batch, seq, width = q.shape
+    q, k, v = (t.reshape(batch, seq, width // 64, 64).transpose(1, 2) for t in (q, k, v))
+    want = (torch.softmax(q @ k.transpose(-1, -2) / 8.0, -1) @ v).transpose(1, 2).reshape(batch, seq, width)
+    rounded = want.to(torch.float16 if dtype == "float16" else torch.bfloat16).double()
+    error, rounding = (float((t - want).norm() / want.norm()) for t in (got, rounded))
+    assert error <= 1.03 * rounding, (error, rounding)
+    ex.clear()
