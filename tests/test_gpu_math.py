@@ -1,0 +1,48 @@
+"""The GELU of act_layout.h swept on its own: tests/cpp/math_sweep.cu compares it with the form that uses erff and
+with double."""
+import math
+import os
+import subprocess
+
+import pytest
+
+from gpreempt_b200 import build as gpx_build
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def _compile(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("math") / "math_sweep")
+    res = subprocess.run([gpx_build.nvcc(), *[f for f in gpx_build.NVCC_FLAGS if f != "-lineinfo"],
+                          "-I", os.path.join(ROOT, "gpreempt_b200", "csrc"),
+                          os.path.join(ROOT, "tests", "cpp", "math_sweep.cu"), "-o", exe], capture_output=True, text=True)
+    assert res.returncode == 0, res.stderr
+    return exe
+
+
+def test_sweep_compiles(tmp_path_factory):
+    _compile(tmp_path_factory)
+
+
+@pytest.fixture(scope="module")
+def sweep(gpx, tmp_path_factory):
+    res = subprocess.run([_compile(tmp_path_factory)], capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stdout
+    rows = [line.split() for line in res.stdout.splitlines()]
+    return lambda name: [[float(v) for v in r[1:]] for r in rows if r[0] == name]
+
+
+@pytest.mark.gpu
+def test_gelu_is_as_accurate_as_the_form_with_erff(sweep):
+    rows = sweep("gelu")
+    assert len(rows) == 18
+    for lo, hi, worst, worst_erff, rms, rms_erff, rel in rows:
+        # (an ulp of the smallest results: both forms round the same product there)
+        assert worst <= worst_erff * 1.001 + 1e-12 and rms <= rms_erff * 1.001 + 1e-12, (lo, hi)
+        if lo >= -6:
+            assert rel <= 1e-5, (lo, hi)
+    inf, ninf, nan, big, nbig, zero, nzero, tiny, ntiny, edge, nedge = sweep("gelu_odd")[0]
+    assert inf == math.inf and abs(ninf) < 1e-30 and math.isnan(nan)
+    assert big == pytest.approx(3e38, rel=1e-6) and abs(nbig) < 1e-30 and zero == 0 and nzero == 0
+    assert tiny == pytest.approx(5e-41, rel=1e-3) and ntiny == pytest.approx(-5e-41, rel=1e-3)
+    assert edge == pytest.approx(1.25 * 0.8943502263331446, rel=2e-7) and nedge == pytest.approx(-1.25 * 0.10564977366685535, rel=1e-6)
