@@ -6,6 +6,7 @@
 #include "stencil.h"
 
 #include "model.h"
+#include "quotients.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -56,81 +57,20 @@ __device__ __forceinline__ Grid grid_of(const StencilParams &p) {
 //
 // The kernels are bound by instruction issue, and half of what they issued was divisions: eleven
 // (eight along x, where three more are in double) with a divisor that is a constant, a parameter, or
-// shared by three of them.  A quotient by a divisor b whose reciprocal y is at hand is q + (a - b q) y
-// with q = a y (Markstein, IBM J. Res. Dev. 34, 1990): three operations, and the correctly rounded
-// quotient when y is the correctly rounded reciprocal and nothing under- or overflows.  Divisions and the
-// power were half of the instructions that bound both kernels (3200 x 1600, ten time steps with state
-// in and out: 19.1 -> 12.4 ms).
-__device__ __forceinline__ float div_by(float a, float b, float y) {
-    const float q = __fmul_rn(a, y);
-    return __fmaf_rn(__fmaf_rn(-b, q, a), y, q);
-}
-__device__ __forceinline__ double div_by(double a, double b, double y) {
-    const double q = __dmul_rn(a, y);
-    return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
-// Reciprocals: the hardware's approximation refined by Newton steps (one in float, two in double).
-__device__ __forceinline__ float reciprocal(float b) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-    return __fmaf_rn(__fmaf_rn(-b, y, 1.f), y, y);
-}
-__device__ __forceinline__ double reciprocal(double b) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    y = __fma_rn(__fma_rn(-b, y, 1.0), y, y);
-    return __fma_rn(__fma_rn(-b, y, 1.0), y, y);
-}
+// shared by three of them.  They are taken by reciprocals (quotients.cuh): the quotients of the divisions
+// bit for bit, except that a numerator below 2^-100 (the fringe ahead of a disturbance, where values
+// fall to nothing within cells) may miss by one or two in the last place.  A horizontal tile that reads an
+// infinity, a NaN, a value of 1e15 or a density beyond half the hydrostatic one divides; along z
+// div_by_any keeps infinities, and a density of zero, of which either way makes NaN, needs no care.
+// 3200 x 1600, a time step: 1 727 us with divisions and pow, 958 like this.
+template <bool DIVIDE>
+__device__ __forceinline__ float quotient(float a, float b, float y) { return DIVIDE ? __fdiv_rn(a, b) : div_by(a, b, y); }
+template <bool DIVIDE>
+__device__ __forceinline__ double quotient(double a, double b, double y) { return DIVIDE ? __ddiv_rn(a, b) : div_by(a, b, y); }
 
-// x^g for x > 0 as 2^(g log2 x), relative error below 4e-15: log2 from the series of artanh,
-// log2 x = k + 2 / ln 2 * (s + s^3 / 3 + s^5 / 5 + ...), s = (m - 1) / (m + 1), x = 2^k m with m between
-// sqrt(1/2) and sqrt 2 (|s| < 0.172, twelve terms), and the Taylor series of 2^f, |f| <= 1/2.  The result
-// ends in a float flux, nine digits coarser; pow() spends most of its instructions on the last bits of
-// the double and on cases (signs, zeros, infinities) that take the call here.
-__device__ __forceinline__ double power(double x, double g) {
-    if (!(x > 1e-290 && x < 1e290)) return pow(x, g);
-    const int hi = __double2hiint(x);
-    int k = (hi - 0x3fe6a09e) >> 20;  // the exponent that leaves the mantissa at or above sqrt(1/2)
-    const double m = __hiloint2double(hi - (k << 20), __double2loint(x));
-    const double s = __dmul_rn(__dsub_rn(m, 1.0), reciprocal(__dadd_rn(m, 1.0)));
-    const double z = __dmul_rn(s, s);
-    double p = 1.0 / 23;
-    p = __fma_rn(p, z, 1.0 / 21);
-    p = __fma_rn(p, z, 1.0 / 19);
-    p = __fma_rn(p, z, 1.0 / 17);
-    p = __fma_rn(p, z, 1.0 / 15);
-    p = __fma_rn(p, z, 1.0 / 13);
-    p = __fma_rn(p, z, 1.0 / 11);
-    p = __fma_rn(p, z, 1.0 / 9);
-    p = __fma_rn(p, z, 1.0 / 7);
-    p = __fma_rn(p, z, 1.0 / 5);
-    p = __fma_rn(p, z, 1.0 / 3);
-    p = __fma_rn(__dmul_rn(p, z), s, s);
-    const double lg = __fma_rn(p, 2.8853900817779268, (double)k);  // 2 / ln 2
-    const double t = __dmul_rn(g, lg);
-    const double n = rint(t);
-    const double f = __dmul_rn(__dsub_rn(t, n), 0.69314718055994531);
-    double e = 1.0 / 6227020800.0;
-    e = __fma_rn(e, f, 1.0 / 479001600.0);
-    e = __fma_rn(e, f, 1.0 / 39916800.0);
-    e = __fma_rn(e, f, 1.0 / 3628800.0);
-    e = __fma_rn(e, f, 1.0 / 362880.0);
-    e = __fma_rn(e, f, 1.0 / 40320.0);
-    e = __fma_rn(e, f, 1.0 / 5040.0);
-    e = __fma_rn(e, f, 1.0 / 720.0);
-    e = __fma_rn(e, f, 1.0 / 120.0);
-    e = __fma_rn(e, f, 1.0 / 24.0);
-    e = __fma_rn(e, f, 1.0 / 6.0);
-    e = __fma_rn(e, f, 0.5);
-    e = __fma_rn(e, f, 1.0);
-    e = __fma_rn(e, f, 1.0);
-    if (fabs(n) > 1000.0) return pow(x, g);  // the exponent would leave the normal range
-    return __hiloint2double(__double2hiint(e) + ((int)n << 20), __double2loint(e));
-}
-
-__device__ __forceinline__ float interp4(float s0, float s1, float s2, float s3) {
-    // (-s0 + 7*(s1 + s2) - s3) / 12
-    return div_by(__fsub_rn(__fmaf_rn(7.f, __fadd_rn(s1, s2), -s0), s3), 12.f, 1.f / 12.f);
+__device__ __forceinline__ float interp4_by_12(float s0, float s1, float s2, float s3) {
+    // -s0 + 7*(s1 + s2) - s3
+    return __fsub_rn(__fmaf_rn(7.f, __fadd_rn(s1, s2), -s0), s3);
 }
 __device__ __forceinline__ float third_derivative(float s0, float s1, float s2, float s3, float hv_coef) {
     // (-s0 + 3*(s1 - s2) + s3) * hv_coef
@@ -138,72 +78,30 @@ __device__ __forceinline__ float third_derivative(float s0, float s1, float s2, 
 }
 __device__ __forceinline__ float advance(float init, float dt, float tend) { return __fmaf_rn(dt, tend, init); }
 
-// Horizontal tile: cells [i0, i1) of row k.  compute_tendencies_x (:222-258) then
-// compute_tendencies_x_r (:260-272).  The row segment with two cells on either side is staged in
-// shared memory; the cells beyond the ends of the row wrap around as set_halo_values_x (:331-341)
-// would have written them, and the tiles at the ends of the row store those halo cells.
-__device__ __forceinline__ void tile_x(const StencilParams &p, const Grid &g, int tile, float *smem) {
+constexpr float kWild = 1.0e15f;  // (products of two, over a third of the density, stay finite)
+constexpr int kMwCellIters = kMwTileXMax / kMwThreads;
+
+// Fluxes and update of a horizontal tile whose row segment is staged.
+template <bool DIVIDE>
+__device__ __forceinline__ void update_x(const StencilParams &p, const Grid &g, const float *sin, float *sflux, int i0, int n, unsigned row,
+                                         float hd, float hdt, const float (&init_v)[kMwCellIters][kMwVars]) {
     constexpr int ldi = kMwTileXMax + 2 * kMwHalo;  // staged values per variable
     constexpr int ldf = kMwTileXMax + 1;            // fluxes per variable
-    float *sin = smem, *sflux = smem + kMwVars * ldi;
-    const int k = tile / p.tiles_per_row;
-    const int i0 = (tile - k * p.tiles_per_row) * p.tile_x;
-    const int i1 = min(i0 + p.tile_x, g.nx);
-    const int n = i1 - i0;
-    const unsigned row = (unsigned)(k + kMwHalo) * (unsigned)g.W;
-    const float *__restrict__ forcing = p.forcing;
-    // Every global load of the tile is issued up front: the row segment to stage (up to three
-    // values per variable and thread) and the cells' starting values, which are not needed until
-    // the update and so overlap the flux arithmetic.
-    constexpr int kStageIters = (kMwTileXMax + 2 * kMwHalo + kMwThreads - 1) / kMwThreads;
-    constexpr int kCellIters = kMwTileXMax / kMwThreads;
-    float staged[kStageIters][kMwVars], init_v[kCellIters][kMwVars];
-#pragma unroll
-    for (int it = 0; it < kStageIters; ++it) {
-        const int c = threadIdx.x + it * kMwThreads;
-        const int ca = i0 + c;  // array column
-        const int src = ca < kMwHalo ? ca + g.nx : (ca >= g.nx + kMwHalo ? ca - g.nx : ca);
-#pragma unroll
-        for (int ll = 0; ll < kMwVars; ++ll)
-            staged[it][ll] = c < n + 2 * kMwHalo ? forcing[ll * g.plane + row + src] : 0.f;
-    }
-#pragma unroll
-    for (int it = 0; it < kCellIters; ++it) {
-        const int f = threadIdx.x + it * kMwThreads;
-#pragma unroll
-        for (int ll = 0; ll < kMwVars; ++ll)
-            init_v[it][ll] = f < n ? p.init[ll * g.plane + row + (unsigned)(i0 + f + kMwHalo)] : 0.f;
-    }
-#pragma unroll
-    for (int it = 0; it < kStageIters; ++it) {
-        const int c = threadIdx.x + it * kMwThreads;
-        const int ca = i0 + c;
-        if (c < n + 2 * kMwHalo) {
-            const bool halo = ca < kMwHalo || ca >= g.nx + kMwHalo;
-#pragma unroll
-            for (int ll = 0; ll < kMwVars; ++ll) {
-                sin[ll * ldi + c] = staged[it][ll];
-                if (halo) p.forcing[ll * g.plane + row + ca] = staged[it][ll];
-            }
-        }
-    }
-    __syncthreads();
     const float hv_coef = __fdiv_rn(__fmul_rn(-kHvBeta, p.dx), __fmul_rn(16.f, p.dt));
-    const float hd = p.hy_dens_cell[k + kMwHalo], hdt = p.hy_dens_theta_cell[k + kMwHalo];
     for (int f = threadIdx.x; f <= n; f += kMwThreads) {  // interface between cells i0+f-1 and i0+f
         float vals[kMwVars], d3_vals[kMwVars];
 #pragma unroll
         for (int ll = 0; ll < kMwVars; ++ll) {
             const float s0 = sin[ll * ldi + f], s1 = sin[ll * ldi + f + 1];
             const float s2 = sin[ll * ldi + f + 2], s3 = sin[ll * ldi + f + 3];
-            vals[ll] = interp4(s0, s1, s2, s3);
+            vals[ll] = quotient<DIVIDE>(interp4_by_12(s0, s1, s2, s3), 12.f, 1.f / 12.f);
             d3_vals[ll] = third_derivative(s0, s1, s2, s3, hv_coef);
         }
         const double r = (double)__fadd_rn(vals[ID_DENS], hd);
-        const double inv_r = reciprocal(r);
-        const double u = div_by((double)vals[ID_UMOM], r, inv_r);
-        const double w = div_by((double)vals[ID_WMOM], r, inv_r);
-        const double t = div_by((double)__fadd_rn(vals[ID_RHOT], hdt), r, inv_r);
+        const double inv_r = DIVIDE ? 0.0 : reciprocal(r);
+        const double u = quotient<DIVIDE>((double)vals[ID_UMOM], r, inv_r);
+        const double w = quotient<DIVIDE>((double)vals[ID_WMOM], r, inv_r);
+        const double t = quotient<DIVIDE>((double)__fadd_rn(vals[ID_RHOT], hdt), r, inv_r);
         const double pr = __dmul_rn((double)kC0, power(__dmul_rn(r, t), (double)kGamm));
         const double ru = __dmul_rn(r, u);
         // r*u feeds four fluxes; the mass flux subtracts from the rounded product, the others fuse
@@ -215,17 +113,74 @@ __device__ __forceinline__ void tile_x(const StencilParams &p, const Grid &g, in
     __syncthreads();
     const float inv_dx = __frcp_rn(p.dx);
 #pragma unroll
-    for (int it = 0; it < kCellIters; ++it) {
+    for (int it = 0; it < kMwCellIters; ++it) {
         const int f = threadIdx.x + it * kMwThreads;
         if (f < n) {
             const unsigned at = row + (unsigned)(i0 + f + kMwHalo);
 #pragma unroll
             for (int ll = 0; ll < kMwVars; ++ll) {
-                const float tend = div_by(-__fsub_rn(sflux[ll * ldf + f + 1], sflux[ll * ldf + f]), p.dx, inv_dx);
+                const float tend = -quotient<DIVIDE>(__fsub_rn(sflux[ll * ldf + f + 1], sflux[ll * ldf + f]), p.dx, inv_dx);
                 p.out[ll * g.plane + at] = advance(init_v[it][ll], p.dt, tend);
             }
         }
     }
+}
+
+// Horizontal tile: cells [i0, i1) of row k.  compute_tendencies_x (:222-258) then
+// compute_tendencies_x_r (:260-272).  The row segment with two cells on either side is staged in
+// shared memory; the cells beyond the ends of the row wrap around as set_halo_values_x (:331-341)
+// would have written them, and the tiles at the ends of the row store those halo cells.
+__device__ __forceinline__ void tile_x(const StencilParams &p, const Grid &g, int tile, float *smem) {
+    constexpr int ldi = kMwTileXMax + 2 * kMwHalo;  // staged values per variable
+    float *sin = smem, *sflux = smem + kMwVars * ldi;
+    const int k = tile / p.tiles_per_row;
+    const int i0 = (tile - k * p.tiles_per_row) * p.tile_x;
+    const int i1 = min(i0 + p.tile_x, g.nx);
+    const int n = i1 - i0;
+    const unsigned row = (unsigned)(k + kMwHalo) * (unsigned)g.W;
+    const float *__restrict__ forcing = p.forcing;
+    // Every global load of the tile is issued up front: the row segment to stage (up to three
+    // values per variable and thread) and the cells' starting values, which are not needed until
+    // the update and so overlap the flux arithmetic.
+    constexpr int kStageIters = (kMwTileXMax + 2 * kMwHalo + kMwThreads - 1) / kMwThreads;
+    float staged[kStageIters][kMwVars], init_v[kMwCellIters][kMwVars];
+#pragma unroll
+    for (int it = 0; it < kStageIters; ++it) {
+        const int c = threadIdx.x + it * kMwThreads;
+        const int ca = i0 + c;  // array column
+        const int src = ca < kMwHalo ? ca + g.nx : (ca >= g.nx + kMwHalo ? ca - g.nx : ca);
+#pragma unroll
+        for (int ll = 0; ll < kMwVars; ++ll)
+            staged[it][ll] = c < n + 2 * kMwHalo ? forcing[ll * g.plane + row + src] : 0.f;
+    }
+#pragma unroll
+    for (int it = 0; it < kMwCellIters; ++it) {
+        const int f = threadIdx.x + it * kMwThreads;
+#pragma unroll
+        for (int ll = 0; ll < kMwVars; ++ll)
+            init_v[it][ll] = f < n ? p.init[ll * g.plane + row + (unsigned)(i0 + f + kMwHalo)] : 0.f;
+    }
+    const float hd = p.hy_dens_cell[k + kMwHalo], hdt = p.hy_dens_theta_cell[k + kMwHalo];
+    bool wild = !(fabsf(hdt) < kWild && hd > 1.0e-6f && hd < kWild);
+#pragma unroll
+    for (int it = 0; it < kStageIters; ++it) {
+        const int c = threadIdx.x + it * kMwThreads;
+        const int ca = i0 + c;
+        if (c < n + 2 * kMwHalo) {
+            // (four thirds of the largest density around is the most the interpolation makes of it)
+            wild |= !(2.f * fabsf(staged[it][ID_DENS]) < hd && largest(staged[it][ID_UMOM], staged[it][ID_WMOM], staged[it][ID_RHOT]) < kWild);
+            const bool halo = ca < kMwHalo || ca >= g.nx + kMwHalo;
+#pragma unroll
+            for (int ll = 0; ll < kMwVars; ++ll) {
+                sin[ll * ldi + c] = staged[it][ll];
+                if (halo) p.forcing[ll * g.plane + row + ca] = staged[it][ll];
+            }
+        }
+    }
+    if (__syncthreads_or(wild))
+        update_x<true>(p, g, sin, sflux, i0, n, row, hd, hdt, init_v);
+    else
+        update_x<false>(p, g, sin, sflux, i0, n, row, hd, hdt, init_v);
 }
 
 // Value of variable ll in array row ka (a row outside the interior) of column ca as the
@@ -280,7 +235,7 @@ __device__ __forceinline__ void tile_z(const StencilParams &p, const Grid &g, in
     float below[kMwVars] = {0.f, 0.f, 0.f, 0.f};  // flux through the interface under the cell about to be updated
     for (int j = 0; j <= nr; ++j) {
         const int k = k0 + j;  // interface below cell row k
-        float vals[kMwVars], d3_vals[kMwVars], init_v[kMwVars];
+        float init_v[kMwVars];
         const unsigned cell = (unsigned)(k - 1 + kMwHalo) * (unsigned)g.W + (unsigned)ca;  // cell above interface k-1
 #pragma unroll
         for (int ll = 0; ll < kMwVars; ++ll) {
@@ -299,16 +254,18 @@ __device__ __forceinline__ void tile_z(const StencilParams &p, const Grid &g, in
                 next_init[ll] = p.init[ll * g.plane + cell + (unsigned)g.W];  // cell row k, updated next step
             }
         }
+        const float hd = p.hy_dens_int[k], hdt = p.hy_dens_theta_int[k];
+        float vals[kMwVars], d3_vals[kMwVars];
 #pragma unroll
         for (int ll = 0; ll < kMwVars; ++ll) {
-            vals[ll] = interp4(win[ll][0], win[ll][1], win[ll][2], win[ll][3]);
+            vals[ll] = div_by_any(interp4_by_12(win[ll][0], win[ll][1], win[ll][2], win[ll][3]), 12.f, 1.f / 12.f);
             d3_vals[ll] = third_derivative(win[ll][0], win[ll][1], win[ll][2], win[ll][3], hv_coef);
         }
-        const float r = __fadd_rn(vals[ID_DENS], p.hy_dens_int[k]);
+        const float r = __fadd_rn(vals[ID_DENS], hd);
         const float inv_r = reciprocal(r);
-        const float u = div_by(vals[ID_UMOM], r, inv_r);
-        float w = div_by(vals[ID_WMOM], r, inv_r);
-        const float t = div_by(__fadd_rn(vals[ID_RHOT], p.hy_dens_theta_int[k]), r, inv_r);
+        const float u = div_by_any(vals[ID_UMOM], r, inv_r);
+        float w = div_by_any(vals[ID_WMOM], r, inv_r);
+        const float t = div_by_any(__fadd_rn(vals[ID_RHOT], hdt), r, inv_r);
         const float pr = __fmaf_rn(kC0, powf(__fmul_rn(r, t), kGamm), -p.hy_pressure_int[k]);
         if (k == 0 || k == g.nz) {
             w = 0;
@@ -330,7 +287,7 @@ __device__ __forceinline__ void tile_z(const StencilParams &p, const Grid &g, in
             float dens_new = 0.f;
 #pragma unroll
             for (int ll = 0; ll < kMwVars; ++ll) {
-                float tend = div_by(-__fsub_rn(flux[ll], below[ll]), p.dz, inv_dz);
+                float tend = -div_by_any(__fsub_rn(flux[ll], below[ll]), p.dz, inv_dz);
                 if (ll == ID_WMOM) tend = __fmaf_rn(-(p.gravity_from_out ? dens_new : win[ID_DENS][1]), kGrav, tend);
                 const float v = advance(init_v[ll], p.dt, tend);
                 if (ll == ID_DENS) dens_new = v;

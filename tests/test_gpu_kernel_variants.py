@@ -257,3 +257,37 @@ def test_attention_rows_that_one_key_dominates(gpx, dtype):
     error, rounding = (float((t - want).norm() / want.norm()) for t in (got, rounded))
     assert error <= 1.03 * rounding, (error, rounding)
     ex.clear()
+
+
+@pytest.mark.parametrize("value", [0.9, -2.0, np.inf, np.nan, 3e20])
+def test_miniweather_tiles_that_divide(gpx, value):
+    """One density beyond what the quotients by reciprocals take makes its tile divide: every cell its stencil does
+    not reach keeps its bits, along x and along z."""
+    ex = gpx.BaseExecutor()
+    ex.init("miniweather_320x160")
+    state = ex.model.get("state").copy()
+    rng = np.random.default_rng(3)
+    state[:, 2:-2, 2:-2] += rng.normal(0, [[[1e-3]], [[1]], [[1]], [[0.3]]], (4, 160, 320)).astype(np.float32)
+    row, col = 70, 150
+    outs = {}
+    for wild in (False, True):
+        for kernel in (0, 3):  # the first stage along x, the first along z
+            s = state.copy()
+            if wild:
+                s[0, row, col] = value
+            for name in ("state", "state_tmp", "state_tmp2"):
+                ex.model.set(name, s)
+            ex.launch_kernel(kernel)
+            outs[wild, kernel] = ex.model.get("state_tmp")[:, 2:-2, 2:-2]
+    r, c = row - 2, col - 2
+    for kernel in (0, 3):
+        a, b = outs[False, kernel], outs[True, kernel]
+        assert np.all(np.isfinite(a))
+        near = np.zeros(a.shape[1:], bool)
+        if kernel == 0:
+            near[r, c - 3:c + 4] = True
+        else:
+            near[r - 3:r + 4, c] = True
+        assert np.array_equal(a[:, ~near].view(np.uint32), b[:, ~near].view(np.uint32)), kernel
+        assert not np.array_equal(a[:, near], b[:, near])
+    ex.clear()

@@ -1,5 +1,5 @@
-"""The GELU of act_layout.h swept on its own: tests/cpp/math_sweep.cu compares it with the form that uses erff and
-with double."""
+"""Device functions that stand in for divisions, pow and erff (quotients.cuh, the GELU of act_layout.h), swept on
+their own: tests/cpp/math_sweep.cu compares them with the functions they stand in for and with long double."""
 import math
 import os
 import subprocess
@@ -30,6 +30,36 @@ def sweep(gpx, tmp_path_factory):
     assert res.returncode == 0, res.stdout
     rows = [line.split() for line in res.stdout.splitlines()]
     return lambda name: [[float(v) for v in r[1:]] for r in rows if r[0] == name]
+
+
+@pytest.mark.gpu
+def test_reciprocals_are_correctly_rounded(sweep):
+    """Every mantissa at nine exponents in float; in double within two ulps' product."""
+    assert sweep("reciprocal") == [[0.0, 0.0]]
+
+
+@pytest.mark.gpu
+def test_quotients_are_those_of_the_division(sweep):
+    """Every float over eight divisors, and 2^32 pairs with extremes among them: bit-identical to the division, except
+    that infinities and NaN are the caller's business and a numerator below 2^-100 may miss by one or two in the last place."""
+    rows = sweep("numerators")
+    assert len(rows) == 16
+    for same, left, near, wrong in rows:
+        # (of 256 exponents one is infinities and NaN, a divisor of 0.3 overflows over two more, and the residuals
+        # of the lowest 24 round to fewer bits: they decide in few of the quotients)
+        assert wrong == 0 and left <= 2 ** 32 * 3 / 256 and near <= 2 ** 32 * 4e-3 and same + left + near == 2 ** 32
+    (same, left, near, wrong), = sweep("pairs")
+    # (24 of 256 exponents overflow over the smallest divisors: 12 on average, and the extremes)
+    assert wrong == 0 and left <= 2 ** 32 * 0.15 and near <= 2 ** 32 * 2e-2
+
+
+@pytest.mark.gpu
+def test_power_gives_the_float_pressures_of_pow(sweep):
+    rows = sweep("power")
+    assert len(rows) == 5
+    for mine, cuda, differ in rows:
+        assert mine <= 3.2 and differ == 0, (mine, cuda)  # units of 1e-16: an ulp and a half at most
+    assert sweep("power_outside") == [[0.0]]
 
 
 @pytest.mark.gpu
