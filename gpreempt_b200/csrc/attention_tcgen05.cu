@@ -34,8 +34,11 @@
 // The first warp of a warpgroup issues TMA and MMA; every wait is bounded, and a wait that gives up raises
 // a flag that ends all others, so the threads of a CTA pass the same barriers and leave together.
 //
-// A tile takes a few microseconds (~6 us at 512 keys with two CTAs per SM), so the word is read
-// between tiles only.
+// A tile takes ~14 us at 512 keys with two CTAs per SM, so the word is read in every block of keys as
+// well as between tiles: on a raised word both warpgroups leave at the end of a softmax, the CTA waits for
+// its copies and products in flight, notes the tile and returns; launched again it recomputes that tile first
+// (a redo costs at most a tile and keeps the instruction sequence, so results stay the same bits).  From the
+// first look at the raised word to the last CTA's exit: p99 7.7 us, 13.7 when a claimed tile always completed.
 #include "layers.cuh"
 #include "sm100.cuh"
 
@@ -63,7 +66,9 @@ struct FaControl {
     uint32_t tmem_base;
     int tile;
     int abort_flag;
-    int pad;
+    int stop;         // the word was seen raised inside the tile
+    int leave[2][2];  // [warpgroup][step parity] what its first thread made of that: the same for all of them
+    int gave_up;      // a warpgroup has left the tile unfinished
     float ml[2][kFaQ][2];  // row maximum and normaliser of each warpgroup
 };
 static_assert(sizeof(FaControl) <= 2304, "control block outgrew its shared-memory budget");
@@ -144,9 +149,32 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
     const int steps = (nkb - wg + 1) / 2;  // blocks wg, wg + 2, ... of this warpgroup
     const float scale_log2 = p.scale * 1.4426950408889634f;  // scores are exponentiated base 2
     uint32_t ph_q = 0, ph_s = 0, ph_o = 0, ph_v = 0, ph_k = 0;  // (ph_k: bit b for key buffer b)
+    // A preemptible launch gives an unfinished tile up when the word goes up: the CTA notes it (two CTAs
+    // share a slot) and takes it first when it is launched again.
+    int *const given_up = blp.preempted && p.slots
+                              ? (blockIdx.x & 1 ? &p.slots[blockIdx.x >> 1].k_done : &p.slots[blockIdx.x >> 1].next_iter) : nullptr;
+    int pending = given_up && tid == 0 ? *given_up - 1 : -1;
+    auto stop_here = [&]() {
+        if (blp.trace) atomicMin(blp.trace + 2, globaltimer_ns());
+        atomicCAS(blp.stop_index, -1, blp.kernel_id);
+    };
     int iter = 0;
     for (;; ++iter) {
-        if (tid == 0) ctl->tile = *abort_flag ? -1 : blp_claim(blp, iter);
+        if (tid == 0) {
+            int t = -1;
+            if (*abort_flag) {
+            } else if (pending < 0) {
+                t = blp_claim(blp, iter);
+            } else if (load_word(blp.preempted) != 0) {
+                stop_here();  // (the note stays)
+            } else {
+                t = pending;
+                pending = -1;
+                *given_up = 0;
+            }
+            ctl->tile = t;
+            ctl->stop = ctl->gave_up = 0;
+        }
         __syncthreads();
         const int tile = ctl->tile;
         if (tile < 0) break;
@@ -189,10 +217,14 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             scores(0);
         }
         ph_q ^= 1;
+        bool left = false;
         for (int j = 0; j < steps; ++j) {
             wait(&ctl->bar_s[wg], ph_s, 403);
             ph_s ^= 1;
             tc_fence_after_sync();
+            const bool may_leave = given_up && j + 1 < steps;
+            int word = 0;  // looked at when the softmax, which hides the read, is through
+            if (may_leave && tid == 0) word = load_word(blp.preempted);
             if (issuer && j + 2 < steps && !*abort_flag) fetch(sK + (j & 1) * kFaKBytes, &p.tk, &ctl->bar_k[wg][j & 1], j + 2);  // S is done with the keys
             uint32_t v[64];
             {
@@ -278,7 +310,20 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             }
             fence_proxy_async();  // the probabilities were written by ordinary stores, the MMA reads them
             tc_fence_before_sync();
+            if (may_leave && row == 0) {
+                if (word != 0) *(volatile int *)&ctl->stop = 1;
+                ctl->leave[wg][j & 1] = *(volatile int *)&ctl->stop;
+            }
             group_sync();
+            if (may_leave && ctl->leave[wg][j & 1]) {
+                // what is still on its way lands first: these values, the next scores, the keys after them
+                wait(&ctl->bar_v[wg], ph_v, 407);
+                wait(&ctl->bar_s[wg], ph_s, 407);
+                if (warp0 && j + 2 < steps) wait(&ctl->bar_k[wg][j & 1], (ph_k >> (j & 1)) & 1, 407);
+                if (row == 0) ctl->gave_up = 1;
+                left = true;
+                break;
+            }
             if (warp0) {
                 wait(&ctl->bar_v[wg], ph_v, 405);
                 tc_fence_after_sync();
@@ -297,7 +342,7 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             }
             ph_v ^= 1;
         }
-        if (steps > 0) {
+        if (steps > 0 && !left) {
             wait(&ctl->bar_o[wg], ph_o, 406);
             ph_o ^= 1;
         }
@@ -306,7 +351,7 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
         // ---- merge: warpgroup g finishes columns 32 g .. 32 g + 31, the other 32 go through shared memory
         // (this warpgroup's V tile and half its P tile, free by now: [column][row] floats)
         float keep[32];
-        {
+        if (!left) {
             uint32_t o[32];
             float *give = reinterpret_cast<float *>(pV);
 #pragma unroll
@@ -331,6 +376,13 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
         }
         tc_fence_before_sync();
         __syncthreads();
+        if (ctl->gave_up) {
+            if (tid == 0) {
+                *given_up = tile + 1;
+                stop_here();
+            }
+            break;
+        }
         if (q0 + row < p.S) {
             const float m0 = ctl->ml[0][row][0], m1 = ctl->ml[1][row][0];
             const float mm = fmaxf(m0, m1);

@@ -33,7 +33,7 @@ struct gpx_exec {
 };
 
 namespace gpx {
-constexpr size_t kSlotsPerKernel = 160;  // >= the largest grid that keeps per-CTA state (one CTA per SM)
+constexpr size_t kSlotsPerKernel = 160;  // >= one per SM (a CTA of the tensor-core layers, two of attention)
 BlpArgs exec_blp_args(gpx_exec *e, size_t idx);
 int exec_launch(gpx_exec *e, size_t idx, cudaStream_t s);
 // Re-arms cursors, progress slots and trace for a run from kernel 0 (what execute does first).

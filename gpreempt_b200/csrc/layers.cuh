@@ -266,6 +266,9 @@ struct AttnParams {
     // boxes of 128 rows x 64 columns), K and V (boxes of 64 x 64), and the error word.
     CUtensorMap tq, tk, tv;
     int *error;
+    // Of a preemptible executor, one for two CTAs: next_iter (even CTA) and k_done (odd) hold, plus one, the
+    // tile it gave up when the word went up inside it.
+    CgemmSlot *slots;
 };
 cudaError_t attention_launch(const AttnParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
 cudaError_t attention_tc_prepare();

@@ -335,8 +335,8 @@ def test_bert_matches_oracle(gpx, oracle, model, batch, seq, layers, heads, voca
 
 @pytest.mark.parametrize("dtype,seq", [("float32", 128), ("float16", 128), ("bfloat16", 512)])
 def test_bert_preempt_resume_bit_identical(gpx, dtype, seq):
-    """(At 512 tokens a tensor-core attention tile spans four key blocks and is given up at a
-    key-block boundary when the word goes up, then recomputed by the relaunched CTA.)"""
+    """(At 512 tokens each warpgroup of a tensor-core attention tile has four blocks of keys; the tile is
+    given up at the end of one when the word goes up, then recomputed by the relaunched CTA.)"""
     base = gpx.BaseExecutor()
     base.init("bert_tiny", batch=8, seed=7, seq_len=seq, dtype=dtype)
     ids = _ids(8, seq, 1000)
