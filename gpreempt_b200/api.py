@@ -166,24 +166,34 @@ class _Resettable:
 
     def __init__(self):
         self._ready = ctypes.c_void_p()
-        self._ordered = None  # stream the last reset is already ordered with
+        self._pending = False  # a reset may still be on its way
 
     def _enqueue_reset(self, entry) -> None:
-        check(entry(self.buf.ptr, ctypes.byref(self._ready)))
-        self._ordered = None
+        check(entry(self._buf.ptr, ctypes.byref(self._ready)))
+        self._pending = True
 
     def order(self, stream) -> None:
         """Orders later work on `stream` behind the last reset."""
-        key = getattr(stream, "value", stream) or 0
-        if self._ready and key and key != self._ordered:  # (the default stream needs no telling)
-            check(B.load().gpx_stream_wait_event(stream, self._ready))
-            self._ordered = key
+        if self._pending and (getattr(stream, "value", stream) or 0):  # (the default stream needs no telling)
+            check(B.load().gpx_ctx_order(stream, self._ready))
+
+    def settle(self) -> None:
+        """Waits for the last reset: whoever takes the device addresses may use them in any order."""
+        if self._pending:
+            check(B.load().gpx_event_sync(self._ready))
+            self._pending = False
+
+    @property
+    def buf(self) -> DeviceBuffer:
+        self.settle()
+        return self._buf
 
     def free(self) -> None:
         if self._ready:
             B.load().gpx_event_destroy(self._ready)
             self._ready = ctypes.c_void_p()
-        self.buf.free()
+        self._pending = False
+        self._buf.free()
 
 
 class BlpContext(_Resettable):
@@ -191,7 +201,7 @@ class BlpContext(_Resettable):
 
     def __init__(self, word: PreemptWord | None, kernel_id: int = 0, trace: bool = True):
         super().__init__()
-        self.buf = DeviceBuffer(256)
+        self._buf = DeviceBuffer(256)
         self.word = word
         self.kernel_id = kernel_id
         self.trace = trace
@@ -205,7 +215,11 @@ class BlpContext(_Resettable):
         self.buf.upload(np.array([-1], np.int32))
 
     def struct(self) -> Blp:
-        base = self.buf.ptr.value
+        self.settle()
+        return self._struct()
+
+    def _struct(self) -> Blp:
+        base = self._buf.ptr.value
         return Blp(self.word.dptr if self.word else None, base, base + 4, self.kernel_id,
                    base + 64 if self.trace else None)
 
@@ -221,7 +235,7 @@ def _blp_for(blp: BlpContext | None, stream):
     if blp is None:
         return None
     blp.order(stream)
-    return ctypes.byref(blp.struct())
+    return ctypes.byref(blp._struct())
 
 
 def axpy(a: float, x: DeviceBuffer, y: DeviceBuffer, n: int, blp: BlpContext | None = None,
@@ -244,8 +258,8 @@ class GemmContext(_Resettable):
         super().__init__()
         n = ctypes.c_size_t()
         check(B.load().gpx_gemm_ctx_bytes(ctypes.byref(n)))
-        self.buf = DeviceBuffer(n.value)
-        self.buf.zero()
+        self._buf = DeviceBuffer(n.value)
+        self._buf.zero()
 
     def reset(self) -> None:
         self._enqueue_reset(B.load().gpx_gemm_ctx_reset)
@@ -261,7 +275,7 @@ def gemm_bf16(a: DeviceBuffer, b: DeviceBuffer, c: DeviceBuffer, m: int, n: int,
     """C[m][n] = A[m][k] x B[n][k]^T, bf16 in/out, fp32 accumulation on tcgen05."""
     h = _h(stream)
     ctx.order(h)
-    check(B.load().gpx_gemm_bf16(a.ptr, b.ptr, c.ptr, m, n, k, ctx.buf.ptr, _blp_for(blp, h), h))
+    check(B.load().gpx_gemm_bf16(a.ptr, b.ptr, c.ptr, m, n, k, ctx._buf.ptr, _blp_for(blp, h), h))
 
 
 def gemm_bf16_static(a: DeviceBuffer, b: DeviceBuffer, c: DeviceBuffer, m: int, n: int, k: int,

@@ -99,6 +99,7 @@ _SIGS = {
     "gpx_axpy_f32": [ctypes.c_float, vp, vp, sz, sz, P(Blp), vp],
     "gpx_axpy_tiles": [sz, sz, P(ci)],
     "gpx_blp_ctx_reset": [vp, P(vp)],
+    "gpx_ctx_order": [vp, vp],
     "gpx_gemm_bf16": [vp, vp, vp, ci, ci, ci, vp, P(Blp), vp],
     "gpx_gemm_ctx_bytes": [P(sz)],
     "gpx_gemm_ctx_reset": [vp, P(vp)],

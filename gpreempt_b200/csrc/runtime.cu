@@ -403,6 +403,24 @@ int gpx_blp_ctx_reset(void *ctx, gpx_event *ready) {
     return record_ready(ready);
 }
 
+int gpx_ctx_order(gpx_stream s, gpx_event ready) {
+    GPX_REQUIRE(ready, GPX_FAIL, "event is NULL");
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    GPX_CUDA(cudaStreamIsCapturing(as_stream(s), &capturing));
+    if (capturing == cudaStreamCaptureStatusNone) {
+        GPX_CUDA(cudaStreamWaitEvent(as_stream(s), (cudaEvent_t)ready, 0));
+        return GPX_SUCC;
+    }
+    // (waiting for an event that is not part of the capture is harmless to it, but a thread in the global or
+    // thread-local mode may not; the exchange lifts that for this call)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    GPX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t err = cudaEventSynchronize((cudaEvent_t)ready);
+    GPX_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    GPX_CUDA(err);
+    return GPX_SUCC;
+}
+
 // ---- preempt word ---------------------------------------------------------------------------
 
 int gpx_word_create(gpx_word **w, int transport) {

@@ -150,8 +150,12 @@ int gpx_axpy_f32(float a, const void *x, void *y, size_t n, size_t tile_elems,
 /* Puts a 256-byte context of one stand-alone kernel back to its initial state: stop index -1 at byte
  * 0, cursor 0 at byte 4, trace slots {~0, 0, ~0, 0} at byte 64.  Asynchronous: it runs on the legacy
  * default stream, behind which *ready is recorded (created if it is NULL; gpx_event_destroy); work
- * on a non-blocking stream is ordered behind it by gpx_stream_wait_event. */
+ * on a non-blocking stream is ordered behind it by gpx_ctx_order. */
 int gpx_blp_ctx_reset(void *ctx, gpx_event *ready);
+/* Orders work enqueued on `s` after the call behind the reset that recorded `ready`.  On a stream that
+ * is being captured into a graph the host waits for the reset instead: a graph cannot wait for an
+ * event from outside, and it may be launched on any stream. */
+int gpx_ctx_order(gpx_stream s, gpx_event ready);
 /* Number of tiles gpx_axpy_f32 splits n elements into. */
 int gpx_axpy_tiles(size_t n, size_t tile_elems, int *tiles);
 

@@ -234,6 +234,84 @@ def test_cluster_reduction_back_to_back(gpx, model, seq, dtype):
     ex.clear(), blp.clear(), word.destroy(), s.destroy()
 
 
+@pytest.mark.parametrize("mode", ["global", "thread_local", "relaxed"])
+def test_launch_behind_a_reset_can_be_captured(gpx, oracle, mode):
+    """A launch with a context goes into a CUDA graph: the reset before it is not part of the graph, so a
+    replay needs a reset of its own, and a replay without one finds every tile done."""
+    import ctypes
+
+    import torch
+
+    n = 100_003
+    x, y = gpx.synth_uniform(n, 4, 0), gpx.synth_uniform(n, 4, 1)
+    dx, dy = gpx.DeviceBuffer.from_numpy(x), gpx.DeviceBuffer.from_numpy(y)
+    word = gpx.PreemptWord(1)
+    ctx = gpx.BlpContext(word, kernel_id=2)
+    m, nn, k = 256, 512, 128
+    a = oracle.f32_to_bf16(gpx.synth_uniform(m * k, 3, 0).reshape(m, k))
+    b = oracle.f32_to_bf16(gpx.synth_uniform(nn * k, 3, 1).reshape(nn, k))
+    da, db, dc = gpx.DeviceBuffer.from_numpy(a), gpx.DeviceBuffer.from_numpy(b), gpx.DeviceBuffer(m * nn * 2)
+    gctx, gblp = gpx.GemmContext(), gpx.BlpContext(word, kernel_id=3)
+    gctx.reset()
+    stream = torch.cuda.Stream()
+    handle = ctypes.c_void_p(stream.cuda_stream)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    ctx.reset()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode=mode):
+        gpx.axpy(0.5, dx, dy, n, ctx, handle)
+        gpx.gemm_bf16(da, db, dc, m, nn, k, gctx, gblp, handle)
+    assert np.array_equal(dy.download(np.float32, n), y)  # captured, not run
+    want = y
+    for fresh in (True, False, True):
+        if fresh and want is not y:
+            ctx.reset(), gctx.reset(), gblp.reset()
+            gpx.device_sync()
+        with torch.cuda.stream(stream):
+            graph.replay()
+        stream.synchronize()
+        want = oracle.axpy(0.5, x, want) if fresh else want
+        assert np.array_equal(dy.download(np.float32, n).view(np.uint32), want.view(np.uint32))
+    assert gctx.status() == (0, 0)
+    got = oracle.bf16_to_f32(dc.download(np.uint16, m * nn)).reshape(m, nn).astype(np.float64)
+    exact = oracle.gemm_bf16_nt(a, b)
+    assert np.all(np.abs(got - exact) <= np.abs(exact) * 2.0 ** -8 + np.abs(exact).max() * 1e-5)
+    del graph
+    for o in (dx, dy, da, db, dc, ctx, gctx, gblp, word):
+        (o.free if hasattr(o, "free") else o.destroy)()
+
+
+def test_context_addresses_and_new_streams_come_behind_a_reset(gpx, oracle):
+    """The raw launch argument is handed out only when the reset is through, and a stream that reuses the handle
+    of a destroyed one is ordered like any other."""
+    import ctypes
+
+    from gpreempt_b200 import binding as B
+
+    n = 100_003
+    x, y = gpx.synth_uniform(n, 4, 0), gpx.synth_uniform(n, 4, 1)
+    dx, dy = gpx.DeviceBuffer.from_numpy(x), gpx.DeviceBuffer.from_numpy(y)
+    word = gpx.PreemptWord(1)
+    ctx = gpx.BlpContext(word, kernel_id=2)
+    want = y
+    for i in range(20):
+        s = gpx.Stream(1)
+        ctx.reset()
+        if i % 2:
+            gpx.axpy(0.5, dx, dy, n, ctx, s)
+        else:
+            arg = ctx.struct()
+            assert not ctx._pending
+            B.check(B.load().gpx_axpy_f32(0.5, dx.ptr, dy.ptr, n, 0, ctypes.byref(arg), s.handle))
+        s.sync()
+        s.destroy()
+        want = oracle.axpy(0.5, x, want)
+        assert ctx.read()["tiles_run"] == gpx.axpy_tiles(n)
+    assert np.array_equal(dy.download(np.float32, n).view(np.uint32), want.view(np.uint32))
+    for o in (dx, dy, ctx, word):
+        (o.free if hasattr(o, "free") else o.destroy)()
+
+
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
 def test_attention_rows_that_one_key_dominates(gpx, dtype):
     """With scores spread wide a row of the context is nearly one row of the values, so its only error is the
