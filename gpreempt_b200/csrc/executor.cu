@@ -32,6 +32,7 @@ int exec_launch(gpx_exec *e, size_t idx, cudaStream_t s) {
     const Kernel &k = e->model->kernels[idx];
     BlpArgs b = exec_blp_args(e, idx);
     cudaError_t err;
+    e->model->forget_given();
     if (k.type == KernelType::Cgemm) {
         // The descriptor is the model's; progress slots, spill area and error word are this
         // executor's.
@@ -254,6 +255,7 @@ int gpx_exec_execute(gpx_exec *e, gpx_stream stream) {
         }
     }
     if (e->graph_exec) {
+        e->model->forget_given();
         GPX_CUDA(cudaGraphLaunch(e->graph_exec, s));
         g_kernel_launches.fetch_add(e->model->kernels.size(), std::memory_order_relaxed);
         return GPX_SUCC;

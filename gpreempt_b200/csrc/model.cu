@@ -1449,7 +1449,19 @@ static int storage_set(gpx_model *m, Storage &s, const void *host, size_t len, c
         }
         return GPX_SUCC;
     }
-    GPX_REQUIRE(s.affine_node < 0, GPX_FAIL, "set %s: the tensor is formed by its consumer and has no storage", s.name.c_str());
+    if (s.affine_node >= 0) {
+        // No storage: its consumer forms it.  What is given is what a stored tensor would hold.
+        std::vector<float> v(s.bytes / sizeof(float));
+        std::vector<bf16_bits> q(plane_count(m->fmt));
+        for (size_t i = 0; i < v.size(); ++i) {
+            host_put(q, 1, 0, src[i], m->fmt);
+            v[i] = host_take(q, 1, 0, m->fmt);
+        }
+        std::lock_guard<std::mutex> hold(m->given_lock);
+        m->given[(size_t)(&s - m->storages.data())] = std::move(v);
+        m->any_given.store(true, std::memory_order_release);
+        return GPX_SUCC;
+    }
     // ActSplit: NCHW fp32 -> hi/lo planes in the storage's row order (borders stay zero)
     const ActLayout &l = s.layout;
     if (s.parent >= 0) {
@@ -1517,6 +1529,14 @@ static int storage_get(gpx_model *m, Storage &s, void *host, size_t len, cudaStr
         return GPX_SUCC;
     }
     if (s.affine_node >= 0) {
+        {
+            std::lock_guard<std::mutex> hold(m->given_lock);
+            auto it = m->given.find((size_t)(&s - m->storages.data()));
+            if (it != m->given.end()) {
+                memcpy(dst, it->second.data(), s.bytes);
+                return GPX_SUCC;
+            }
+        }
         // Not stored: computed from the channels its consumer reads, as the consumer does.
         const Node &a = m->nodes[s.affine_node];
         Storage &src = m->storages[m->nodes[a.inputs[0]].storage];

@@ -9,6 +9,8 @@
 #include "stencil.h"
 #include "graphwl.h"
 
+#include <atomic>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -53,7 +55,8 @@ struct Storage {
     int ch_off = 0;                  //   starting at this stored channel (concatenation by placement)
     bool borrowed = false;           // Weight planes / Vec: rows of a fused storage, which owns the memory
     int affine_node = -1;            // ActSplit: output of that Affine node, formed by its only consumer as it
-                                     //   loads its operand; nothing is stored (get computes it)
+                                     //   loads its operand; nothing is stored (get computes it, set is kept
+                                     //   on the host until the model runs)
 };
 
 // Buffer: a tensor other nodes write slices of (the running concatenation of a dense block).
@@ -150,6 +153,18 @@ struct gpx_model {
     uint64_t graph_vertices = 0, graph_edges = 0;
     int graph_iterations = 0;     // live iterations of the run that sized the kernel list
     int *graph_active = nullptr;  // device: iteration flags (owned through `scratch`)
+
+    // Values a client has given to tensors that have no storage (Storage::affine_node), by storage index:
+    // read back until a kernel of the model is launched, which would have overwritten a stored one.
+    std::unordered_map<size_t, std::vector<float>> given;
+    std::mutex given_lock;
+    std::atomic<bool> any_given{false};
+    void forget_given() {
+        if (!any_given.load(std::memory_order_acquire)) return;
+        std::lock_guard<std::mutex> hold(given_lock);
+        given.clear();
+        any_given.store(false, std::memory_order_release);
+    }
 
     int add_storage(const gpx::Storage &s);
     int find(const std::string &name) const;
