@@ -174,22 +174,23 @@ int gpx_exec_destroy(gpx_exec *e) {
 constexpr size_t kOwnGraphKernels = 64;
 
 static bool own_graph_applies(const gpx_exec *e) {
-    return !e->graph_exec && e->kind == GPX_EXEC_BLP && e->word_dptr && e->model->kernels.size() <= kOwnGraphKernels;
+    return !e->graph_exec && e->kind == GPX_EXEC_BLP && e->word_dptr && !e->own_refused &&
+           e->model->kernels.size() <= kOwnGraphKernels;
 }
 
-// The forward as a graph, made when the word is set (for best-effort streams, ~0.4 ms) and again by an execute for
-// which something it depends on has changed: kernel by kernel the host takes up to 4 us a launch, longer than most kernels of a small model run (15-kernel BERT:
-// 63 us of host for 80 us of GPU).
-static int refresh_own_graph(gpx_exec *e, int priority) {
-    if (e->own_graph && e->own_word == e->word_dptr && e->own_priority == priority && e->own_trace == e->trace_on &&
-        e->own_drop == e->drop_tile_in_flight)
-        return GPX_SUCC;
+// The forward as a graph.  Launched kernel by kernel it has gaps between its kernels and holds the host
+// (one pass alone, kernel by kernel against the graph: 15-kernel BERT 87 against 76 us and 40 against 2 us
+// of host, ResNet-50 of 16 images 1 000 against 948 and 157 against 3, VGG-16 of one 421 against 403).  Making it
+// takes 0.3 to 1.3 ms, so it is made by the second execute in a row with the same word, stream
+// priority, tracing and restart policy, behind the kernels that execute has launched: a client that captures
+// the forward itself, runs it once or changes these from run to run does not pay for it.
+static int make_own_graph(gpx_exec *e, const gpx_exec::OwnKey &key) {
     if (e->own_graph) GPX_CUDA(cudaGraphExecDestroy(e->own_graph));  // (a run in flight keeps it until it is through)
     e->own_graph = nullptr;
     // captured on a stream of its own: the caller's may be the default stream, which cannot be captured
     cudaStream_t c = nullptr;
     cudaGraph_t graph = nullptr;
-    GPX_CUDA(cudaStreamCreateWithPriority(&c, cudaStreamNonBlocking, priority));
+    GPX_CUDA(cudaStreamCreateWithPriority(&c, cudaStreamNonBlocking, key.priority));
     cudaError_t err = cudaStreamBeginCapture(c, cudaStreamCaptureModeThreadLocal);
     int st = GPX_SUCC;
     if (err == cudaSuccess) {
@@ -207,10 +208,7 @@ static int refresh_own_graph(gpx_exec *e, int priority) {
     cudaStreamDestroy(c);
     if (st != GPX_SUCC) return st;
     GPX_CUDA(err);
-    e->own_word = e->word_dptr;
-    e->own_priority = priority;
-    e->own_trace = e->trace_on;
-    e->own_drop = e->drop_tile_in_flight;
+    e->own_key = key;
     return GPX_SUCC;
 }
 
@@ -220,7 +218,7 @@ int gpx_exec_set_word(gpx_exec *e, gpx_word *w) {
     GPX_TRY(gpx_word_dptr(w, &d));
     GPX_REQUIRE(!e->graph_exec, GPX_FAIL, "set the preempt word before capturing the graph");
     e->word_dptr = (const int *)d;
-    return own_graph_applies(e) ? refresh_own_graph(e, device_info().prio_least) : GPX_SUCC;
+    return GPX_SUCC;
 }
 
 int gpx_exec_set_word_dptr(gpx_exec *e, const void *dptr) {
@@ -229,7 +227,7 @@ int gpx_exec_set_word_dptr(gpx_exec *e, const void *dptr) {
     GPX_REQUIRE(!e->graph_exec || e->word_dptr == (const int *)dptr, GPX_FAIL,
                 "set the preempt word before capturing the graph");
     e->word_dptr = (const int *)dptr;
-    return own_graph_applies(e) ? refresh_own_graph(e, device_info().prio_least) : GPX_SUCC;
+    return GPX_SUCC;
 }
 
 int gpx_exec_enable_trace(gpx_exec *e, int on) {
@@ -242,16 +240,21 @@ int gpx_exec_enable_trace(gpx_exec *e, int on) {
 int gpx_exec_execute(gpx_exec *e, gpx_stream stream) {
     GPX_REQUIRE(e, GPX_FAIL, "NULL executor");
     cudaStream_t s = as_stream(stream);
+    gpx_exec::OwnKey key;  // (word null: no graph of the executor's own for this run)
     if (own_graph_applies(e)) {
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         if (s) GPX_CUDA(cudaStreamIsCapturing(s, &capturing));
         if (capturing == cudaStreamCaptureStatusNone) {
-            int priority = 0;
-            if (s) GPX_CUDA(cudaStreamGetPriority(s, &priority));
-            GPX_TRY(refresh_own_graph(e, priority));
-            GPX_CUDA(cudaGraphLaunch(e->own_graph, s));
-            g_kernel_launches.fetch_add(e->model->kernels.size(), std::memory_order_relaxed);
-            return GPX_SUCC;
+            if (s) GPX_CUDA(cudaStreamGetPriority(s, &key.priority));
+            key.trace = e->trace_on;
+            key.drop = e->drop_tile_in_flight;
+            key.word = e->word_dptr;
+            if (e->own_graph && e->own_key == key) {
+                e->model->forget_given();
+                GPX_CUDA(cudaGraphLaunch(e->own_graph, s));
+                g_kernel_launches.fetch_add(e->model->kernels.size(), std::memory_order_relaxed);
+                return GPX_SUCC;
+            }
         }
     }
     if (e->graph_exec) {
@@ -263,6 +266,13 @@ int gpx_exec_execute(gpx_exec *e, gpx_stream stream) {
     GPX_TRY(exec_prologue(e, s));
     size_t nk = e->model->kernels.size();
     for (size_t i = 0; i < nk; ++i) GPX_TRY(exec_launch(e, i, s));
+    if (key.word && e->own_last == key && make_own_graph(e, key) != GPX_SUCC) {
+        // (the forward itself is on its way: only the shortcut is not to be had)
+        cudaGetLastError();
+        e->own_graph = nullptr;
+        e->own_refused = true;
+    }
+    if (key.word) e->own_last = key;
     return GPX_SUCC;
 }
 

@@ -24,12 +24,19 @@ struct gpx_exec {
     bool drop_tile_in_flight = false;  // restart policy of the tensor-core kernels (gpx_exec_set_restart_policy)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
-    // What execute launches for a short preemptible forward that nobody has captured, and what it was
-    // captured for.
+    // What execute launches for a short preemptible forward that nobody has captured.
+    struct OwnKey {
+        const int *word = nullptr;
+        int priority = 0;
+        bool trace = false, drop = false;
+        bool operator==(const OwnKey &o) const {
+            return word == o.word && priority == o.priority && trace == o.trace && drop == o.drop;
+        }
+    };
     cudaGraphExec_t own_graph = nullptr;
-    const int *own_word = nullptr;
-    int own_priority = 0;
-    bool own_trace = false, own_drop = false;
+    OwnKey own_key;            // what it was captured for
+    OwnKey own_last;           // what the last execute without it ran with (word null: none has)
+    bool own_refused = false;  // it could not be made: kernels are launched one by one
 };
 
 namespace gpx {

@@ -336,9 +336,9 @@ int gpx_exec_set_word(gpx_exec *e, gpx_word *w); /* blp_executor->dpStop = g_sto
  * then poll across the bus. */
 int gpx_exec_set_word_dptr(gpx_exec *e, const void *dptr);
 /* Executor::execute (src/executor.cpp:119-134) / BLPExecutor::execute (:211-232).  A preemptible forward of at
- * most 64 kernels that nobody has captured is launched as a graph the executor keeps.  It is made when the
- * word is set (~0.4 ms), and again by the first execute on a stream of another priority or after a change
- * of tracing or restart policy. */
+ * most 64 kernels that nobody has captured is launched as a graph the executor keeps, from the third
+ * execute in a row with the same word, stream priority, tracing and restart policy on: the second makes it
+ * (0.3 to 1.3 ms) behind the kernels it has launched. */
 int gpx_exec_execute(gpx_exec *e, gpx_stream s);
 /* Executor::launch_kernel, src/executor.cpp:136-164. */
 int gpx_exec_launch_kernel(gpx_exec *e, size_t idx, gpx_stream s);

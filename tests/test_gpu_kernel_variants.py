@@ -317,6 +317,38 @@ def test_context_addresses_and_new_streams_come_behind_a_reset(gpx, oracle):
         (o.free if hasattr(o, "free") else o.destroy)()
 
 
+def test_short_forward_is_made_a_graph_only_when_it_repeats(gpx):
+    """Setting the word makes nothing, a run after the graph of one's own was captured uses that, and runs that
+    alternate between settings go kernel by kernel; all end with the same bits."""
+    import time
+
+    word = gpx.PreemptWord(1)
+    streams = [gpx.Stream(1), gpx.Stream(0)]
+    outs, host = [], {}
+    for use in ("alternating", "repeating", "captured"):
+        ex = gpx.BLPExecutor()
+        ex.init("resnet_tiny", batch=1, seed=3)
+        ex.set_input("data", _images(gpx, 1))
+        ex.set_word(word)
+        if use == "captured":
+            ex.capture_graph(streams[0])
+        for i in range(12):
+            s = streams[i % 2 if use == "alternating" else 0]
+            s.sync()
+            t0 = time.perf_counter()
+            ex.execute(s)
+            host.setdefault(use, []).append(time.perf_counter() - t0)
+            s.sync()
+            outs.append(ex.get_output("heads"))
+            assert ex.getStopPoint(s) == -1
+        ex.clear()
+    assert all(np.array_equal(o, outs[0]) for o in outs)
+    # 33 launches against one: the host time of the last runs tells which way they went
+    assert np.median(host["repeating"][4:]) < 0.5 * np.median(host["alternating"][4:])
+    for o in [word] + streams:
+        o.destroy()
+
+
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
 def test_attention_rows_that_one_key_dominates(gpx, dtype):
     """With scores spread wide a row of the context is nearly one row of the values, so its only error is the
