@@ -192,8 +192,16 @@ static void render_graph(const gpx_model *m, Json *graph, Json *host) {
         Json jf = Json::object();
         jf.set("name", func_name_of(n));
         Json kernels = Json::array();
+        // (a node computed by another's kernel - a norm applied to its consumer's operand, one of the
+        // projections that share a product - lists that kernel: every function has one)
+        int by = (int)ni;
+        for (size_t o = 0; o < m->nodes.size(); ++o) {
+            const Node &other = m->nodes[o];
+            if (n.fused_affine && !other.inputs.empty() && other.inputs[0] == (int)ni) by = (int)o;
+            if (n.fused_into_other && other.fused_w == n.fused_w && !other.fused_into_other) by = (int)o;
+        }
         for (const Kernel &k : m->kernels) {
-            if (k.node != (int)ni) continue;
+            if (k.node != by) continue;
             Json jk = Json::object();
             jk.set("name", std::string(kernel_type_name(k.type)) + ":" + k.name);
             Json lp = Json::array();

@@ -1401,6 +1401,24 @@ static void khwc_o_to_oihw(const float *src, float *dst, int O, int I, int KH, i
                         src[(((size_t)h * KW + w) * I + i) * O + o];
 }
 
+static int storage_set(gpx_model *m, Storage &s, const void *host, size_t len, cudaStream_t st);
+static int storage_get(gpx_model *m, Storage &s, void *host, size_t len, cudaStream_t st);
+
+// The weight of a fused product holds planes only: its rows in fp32 are its parts' parameters.
+static bool is_fused_weight(const Storage &s) { return s.kind == Storage::Weight && s.hidden && !s.dptr; }
+template <typename F>
+static int for_fused_parts(gpx_model *m, const Storage &s, F &&f) {
+    const int idx = (int)(&s - m->storages.data());
+    size_t off = 0;
+    for (const Node &n : m->nodes) {
+        if (n.fused_w != idx) continue;
+        Storage &part = m->storages[n.weight];
+        GPX_TRY(f(part, off));
+        off += part.bytes;
+    }
+    return GPX_SUCC;
+}
+
 static int storage_set(gpx_model *m, Storage &s, const void *host, size_t len, cudaStream_t st) {
     // Model::set, src/model.cpp:313-321: `len < size` is rejected.
     GPX_REQUIRE(len >= s.bytes, GPX_OUT_OF_RANGE, "set %s: %zu bytes given, %zu needed",
@@ -1411,6 +1429,10 @@ static int storage_set(gpx_model *m, Storage &s, const void *host, size_t len, c
         GPX_CUDA(cudaMemcpyAsync(s.dptr, host, s.bytes, cudaMemcpyHostToDevice, st));
         return GPX_SUCC;
     }
+    if (is_fused_weight(s))
+        return for_fused_parts(m, s, [&](Storage &part, size_t off) {
+            return storage_set(m, part, (const char *)host + off, part.bytes, st);
+        });
     if (s.kind == Storage::Weight) {
         const int O = (int)s.dims[0], I = (int)s.dims[1], KH = (int)s.dims[2], KW = (int)s.dims[3];
         if (s.depthwise) {
@@ -1512,6 +1534,10 @@ static int storage_get(gpx_model *m, Storage &s, void *host, size_t len, cudaStr
         GPX_CUDA(cudaMemcpyAsync(host, s.dptr, s.bytes, cudaMemcpyDeviceToHost, st));
         return GPX_SUCC;
     }
+    if (is_fused_weight(s))
+        return for_fused_parts(m, s, [&](Storage &part, size_t off) {
+            return storage_get(m, part, (char *)host + off, part.bytes, st);
+        });
     if (s.kind == Storage::Weight) {
         if (s.depthwise) {
             const int C = (int)s.dims[0], T = (int)(s.dims[2] * s.dims[3]);

@@ -317,6 +317,35 @@ def test_context_addresses_and_new_streams_come_behind_a_reset(gpx, oracle):
         (o.free if hasattr(o, "free") else o.destroy)()
 
 
+@pytest.mark.parametrize("model", ["bert_tiny", "densenet_tiny"])
+def test_every_tensor_and_function_has_its_own_name(gpx, tmp_path, model):
+    """Tensors of fused layers are read and written under their names, the fused ones' too, and an exported
+    directory lists a kernel for every function."""
+    import json
+
+    ex = gpx.BaseExecutor()
+    ex.init(model, batch=2, seed=7, seq_len=16 if model == "bert_tiny" else 0)
+    data = np.random.default_rng(1).integers(0, 1000, (2, 16)).astype(np.int64) if model == "bert_tiny" else _images(gpx, 2)
+    ex.set_input("data", data)
+    ex.execute()
+    heads = ex.get_output("heads")
+    infos = [ex.model.get_storage_info(i) for i in range(ex.model.get_storage_num())]
+    values = {i["name"]: ex.model.get(i["name"]) for i in infos if i["stype"] == "float32" and i["name"] != "data"}
+    for name, v in values.items():
+        ex.model.set(name, v)
+        assert np.array_equal(ex.model.get(name), v), name
+    for name, v in values.items():
+        if name.endswith(".qkv.weight"):
+            parts = [values[name.replace(".query.out.qkv", "." + part)] for part in ("query", "key", "value")]
+            assert np.array_equal(v, np.concatenate(parts))
+    ex.execute()
+    assert np.array_equal(ex.get_output("heads"), heads)
+    ex.model.export_dir(str(tmp_path / model))
+    host = json.load(open(tmp_path / model / "host.json"))
+    assert all(f["kernels"] for f in host["funcs"])
+    ex.clear()
+
+
 def test_short_forward_is_made_a_graph_only_when_it_repeats(gpx):
     """Setting the word makes nothing, a run after the graph of one's own was captured uses that, and runs that
     alternate between settings go kernel by kernel; all end with the same bits."""
