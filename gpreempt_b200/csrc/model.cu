@@ -965,8 +965,9 @@ int finalize_model(gpx_model &m) {
             q.pad = n.pad;
             q.act = n.act;
             // The filter goes to shared memory where that pays: with a tile or two per CTA (small
-            // batches) its latency hides behind the predecessor's tail; up to the default 48 KB.
-            q.w_in_smem = (size_t)n.k * n.k * q.out.C * sizeof(float) <= 48 * 1024 ? 1 : 0;
+            // batches) its latency hides behind the predecessor's tail; beside the kernel's own variables
+            // in the default 48 KB.
+            q.w_in_smem = (size_t)n.k * n.k * q.out.C * sizeof(float) + 256 <= 48 * 1024 ? 1 : 0;
             long long total = (long long)n.N * n.H * n.W * (q.out.C / 8);
             q.tile_elems = (int)std::max<long long>(256, std::min<long long>(kMaxTileVectors, total / (8LL * m.sm_count) / 32 * 32));
             q.total_tiles = (int)((total + q.tile_elems - 1) / q.tile_elems);

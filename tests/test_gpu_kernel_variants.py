@@ -346,6 +346,51 @@ def test_every_tensor_and_function_has_its_own_name(gpx, tmp_path, model):
     ex.clear()
 
 
+@pytest.mark.parametrize("channels", [752, 768, 784])
+def test_depthwise_filter_beside_the_kernels_own_shared_memory(gpx, tmp_path, channels):
+    """A 4x4 filter of 768 channels is the whole of the default 48 KB: it does not go to shared memory."""
+    import ctypes
+    import json
+
+    import torch
+
+    from gpreempt_b200 import binding as B
+
+    def param(name):
+        return {"op": "null", "name": name, "inputs": [], "attrs": {"gpx_kind": "param", "init_std": 0.1, "init_mean": 0.0}}
+
+    def layer(name, fn, inputs, kernel, stride, pad):
+        return {"op": "tvm_op", "name": name, "inputs": [[i, 0, 0] for i in inputs],
+                "attrs": {"func_name": fn, "kernel": kernel, "stride": stride, "padding": pad, "activation": 0}}
+
+    n, hw = 2, 9
+    nodes = [{"op": "null", "name": "data", "inputs": [], "attrs": {"gpx_kind": "input"}},
+             param("a.weight"), param("a.bias"), layer("a", "gpx_conv2d", [0, 1, 2], 1, 1, 0),
+             param("b.weight"), param("b.bias"), layer("b", "gpx_depthwise_conv2d", [3, 4, 5], 4, 1, 1),
+             layer("pool", "gpx_avg_pool2d", [6], hw - 1, 1, 0),
+             param("heads.weight"), param("heads.bias"), layer("heads", "gpx_conv2d", [7, 8, 9], 1, 1, 0)]
+    shapes = [[n, 3, hw, hw], [channels, 3, 1, 1], [channels], [n, channels, hw, hw], [channels, 1, 4, 4], [channels],
+              [n, channels, hw - 1, hw - 1], [n, channels, 1, 1], [1000, channels, 1, 1], [1000], [n, 1000]]
+    graph = {"nodes": nodes, "heads": [[10, 0, 0]], "gpx": {"model": "dw4", "batch": n, "dtype": "float32", "pad_channels": False},
+             "attrs": {"dltype": ["list_str", ["float32"] * len(nodes)], "shape": ["list_shape", shapes]}}
+    (tmp_path / "mod.json").write_text(json.dumps(graph))
+    (tmp_path / "host.json").write_text(json.dumps(
+        {"temp_args": [], "funcs": [{"name": x["attrs"]["func_name"], "kernels": [{}]} for x in nodes if x["inputs"]]}))
+    ex = gpx.BaseExecutor()
+    ex.model = gpx.Model(str(tmp_path))
+    B.check(B.load().gpx_exec_create(ex.model.handle, B.EXEC_BASE, ctypes.byref(ex.handle)))
+    ex.model.init_random(5)
+    x = gpx.synth_normal(n * 3 * hw * hw, 2, 0).reshape(n, 3, hw, hw)
+    ex.set_input("data", x)
+    ex.execute()
+    assert ex.error() == (0, 0)
+    p = {k: torch.from_numpy(v).double() for k, v in ex.model.params().items()}
+    a = torch.nn.functional.conv2d(torch.from_numpy(x).double(), p["a.weight"], p["a.bias"])
+    want = torch.nn.functional.conv2d(a, p["b.weight"], p["b.bias"], padding=1, groups=channels).numpy()
+    assert _rel(ex.model.get("b"), want) <= TOL["float32"]
+    ex.clear()
+
+
 def test_short_forward_is_made_a_graph_only_when_it_repeats(gpx):
     """Setting the word makes nothing, a run after the graph of one's own was captured uses that, and runs that
     alternate between settings go kernel by kernel; all end with the same bits."""
