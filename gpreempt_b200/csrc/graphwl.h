@@ -42,7 +42,8 @@ constexpr int kGwVertexTileVerts = 1024;  // vertices per tile of a per-vertex p
 constexpr int kGwMaxIters = 16384;        // iteration flags a graph workload has: no run may need more rounds
 // (packed PageRank: 52 804 vertices are 826 tiles, fewer than six CTAs on each of 148 SMs)
 constexpr int kGwPackedTileVerts = 64;
-constexpr int kGwWindowMax = 12287;       // floats of a tile's window (with the zero behind it: 48 KiB)
+// floats of a tile's window: with the zero behind it and the kernel's own variables in the default 48 KiB
+constexpr int kGwWindowMax = (48 * 1024 - 256) / 4 - 1;
 constexpr unsigned kGwInfinity = 0xFFFFFFFFu;  // MYINFINITY, include/workloads/graphcompute.h:14
 
 struct GraphWlParams {

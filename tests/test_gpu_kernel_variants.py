@@ -423,6 +423,38 @@ def test_short_forward_is_made_a_graph_only_when_it_repeats(gpx):
         o.destroy()
 
 
+def _pagerank(gpx, tmp_path, rows, prefix_name="g"):
+    """The graph in files, its kernels' edge-pass tiles, and one run against the oracle."""
+    from oracle import graphs
+
+    graphs.build()
+    prefix = str(tmp_path / prefix_name / "g.bel")
+    offsets = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.uint64)
+    neighbours = np.concatenate(rows).astype(np.uint64)
+    graph_files.write_bel(prefix, offsets, neighbours, None)
+    ex = gpx.BaseExecutor()
+    ex.set_graph_path(prefix)
+    ex.init("pagerank")
+    tiles = {i["total_tiles"] for i in (ex.model.get_kernel_info(k) for k in range(ex.get_kernel_num())) if ".edges." in i["name"]}
+    ex.execute()
+    err = np.abs(ex.model.get("value").astype(np.float64) - graphs.pagerank(offsets, neighbours)[0].astype(np.float64))
+    assert err.max() <= 1.1e-3 and err.mean() <= 1e-5
+    ex.clear()
+    assert len(tiles) == 1
+    return tiles.pop()
+
+
+@pytest.mark.parametrize("vertices", [12223, 12224, 12287, 12288])
+def test_pagerank_longest_window(gpx, tmp_path, vertices):
+    """Every tile reads the first and the last vertex, so its window is the whole graph: up to 12 223 deltas go to
+    shared memory beside the kernel's own variables, more stay in lists (tiles of 16 vertices)."""
+    rng = np.random.default_rng(vertices)
+    rows = [np.unique(rng.integers(0, vertices, 400)) for _ in range(vertices)]
+    rows[0] = rows[-1] = np.arange(vertices)
+    lists = _pagerank(gpx, tmp_path, rows) == -(-vertices // 16)
+    assert lists == (vertices > 12223)
+
+
 @pytest.mark.parametrize("dtype", ["float16", "bfloat16"])
 def test_attention_rows_that_one_key_dominates(gpx, dtype):
     """With scores spread wide a row of the context is nearly one row of the values, so its only error is the
