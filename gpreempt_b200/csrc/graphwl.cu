@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -593,7 +594,15 @@ bool pack_lists(const std::vector<unsigned long long> &trow, const std::vector<u
     };
     std::vector<std::thread> pool;
     const uint64_t workers = std::min<uint64_t>(8, std::max<uint64_t>(1, tiles / 64));
-    for (uint64_t i = 0; i < workers; ++i) pool.emplace_back(fill, tiles * i / workers, tiles * (i + 1) / workers);
+    pool.reserve(workers);
+    for (uint64_t i = 0; i < workers; ++i) {
+        const uint64_t t0 = tiles * i / workers, t1 = tiles * (i + 1) / workers;
+        try {
+            pool.emplace_back(fill, t0, t1);
+        } catch (const std::system_error &) {
+            fill(t0, t1);  // no thread to be had
+        }
+    }
     for (auto &th : pool) th.join();
     return true;
 }
