@@ -384,8 +384,8 @@ __device__ __forceinline__ void init_tile(const GraphWlParams &p, int tile) {
     }
 }
 
-// PACK: PageRank's packed form (ids per lane and block), 0 = edge lists.  The packed form runs a tile per
-// CTA at the size it was measured at, and six CTAs per SM keep all of them resident.
+// PACK: PageRank's packed form (ids per lane and block), 0 = edge lists.  Six CTAs of the packed form on an SM hide
+// one another's barriers and copies.
 template <int ALGO, int PHASE, int PACK = 0>
 __global__ void __launch_bounds__(kGwThreads, PACK ? 6 : 1)
 graphwl_kernel(const __grid_constant__ GraphWlParams p, BlpArgs blp) {
@@ -548,13 +548,31 @@ void transpose(const HostGraph &g, std::vector<unsigned long long> &trow, std::v
         for (unsigned long long i = g.row[u]; i < g.row[u + 1]; ++i) tadj[at[g.adj[i]]++] = (unsigned)u;
 }
 
-// PageRank's packed in-edge lists (GraphWlParams::packed), if every tile of `tile_verts` vertices reads
-// ids that lie within one window; false otherwise.
+// Vertices per tile of the packed form: a tile's window is copied once, so larger tiles copy less, as long as
+// each SM has tiles enough to keep its CTAs busy: four of 64 vertices, else two of 32, else none (the
+// lists, in tiles of 16).  A run in us, lists / 16 / 32 / 64 / 128 vertices: 52 804 vertices of degree 193
+// 1 282 / 1 162 / 866 / 700 / 934, of degree 41 1 971 / 1 439 / 1 006 / 821 / 1 004; 20 000 of 97
+// 944 / 801 / 692 / 718 / 830; 10 000 of 183 349 / 332 / 324 / 346 / 422; 3 000 of 163
+// 203 / 210 / 224 / 261 / 349.
+int packed_tile_verts(uint64_t n, int sm_count) {
+    if (n >= 64ull * 4 * sm_count) return 64;
+    return n >= 32ull * 2 * sm_count ? 32 : 0;
+}
+
+// PageRank's packed in-edge lists (GraphWlParams::packed), false if the lists are the better form:
+//  - every tile of `tile_verts` vertices has to read ids that lie within one window of kGwWindowMax;
+//  - the gathers have to be worth the copies: at least three for every four deltas copied (band of 1 500, degree
+//    41: 0.86, 821 against 1 971 us a run; 12 000 vertices with random neighbours, degree 200: 0.53, 412
+//    against 388; degree 20: 0.06, 419 against 360);
+//  - no warp may have much more than its share, since a list goes by 32 x pack ids at a time where the other form
+//    takes 256: four times the average (degrees up to 1 500 around an average of 17, 40 000 vertices:
+//    1 770 us against 1 112; up to 7 350 around 21: 2 123 against 830).
 bool pack_lists(const std::vector<unsigned long long> &trow, const std::vector<unsigned> &tadj, uint64_t n, int tile_verts,
                 int &pack, std::vector<uint16_t> &packed, std::vector<unsigned> &blk, std::vector<uint2> &win, int &win_max) {
     const uint64_t tiles = (n + tile_verts - 1) / tile_verts;
     win.resize(tiles);
     win_max = 0;
+    uint64_t copies = 0;
     for (uint64_t t = 0; t < tiles; ++t) {
         unsigned lo = kGwInfinity, hi = 0;
         for (uint64_t v = t * tile_verts; v < std::min<uint64_t>(n, (t + 1) * tile_verts); ++v)
@@ -566,19 +584,25 @@ bool pack_lists(const std::vector<unsigned long long> &trow, const std::vector<u
         if (len > (unsigned)kGwWindowMax) return false;
         win[t] = make_uint2(len ? lo : 0, len);
         win_max = std::max(win_max, (int)len);
+        copies += len;
     }
+    if (4 * (uint64_t)tadj.size() < 3 * copies) return false;
     // ids per lane and block: the block next above the average list
     const uint64_t avg = tadj.size() / n;
     pack = avg > 128 ? 8 : (avg > 64 ? 4 : (avg > 32 ? 2 : 1));
     const unsigned per = 32u * (unsigned)pack;
+    const uint64_t warp_verts = (uint64_t)tile_verts / (kGwThreads / 32);
     blk.resize(n + 1);
-    uint64_t blocks = 0;
+    uint64_t blocks = 0, most = 0;
     for (uint64_t v = 0; v < n; ++v) {
         blk[v] = (unsigned)blocks;
         blocks += (trow[v + 1] - trow[v] + per - 1) / per;
+        const uint64_t first = v / warp_verts * warp_verts;
+        most = std::max(most, blocks - blk[first]);
+        if (blocks >= (1ull << 32)) return false;
     }
-    if (blocks >= (1ull << 32)) return false;
     blk[n] = (unsigned)blocks;
+    if (most * n > 4 * warp_verts * std::max<uint64_t>(blocks, n)) return false;
     packed.resize(blocks * per);
     auto fill = [&](uint64_t t0, uint64_t t1) {
         for (uint64_t v = t0 * tile_verts; v < std::min<uint64_t>(n, t1 * tile_verts); ++v) {
@@ -709,6 +733,7 @@ int build_graph_workload(gpx_model &m, const std::string &name, const gpx_model_
     base.src = 0;
     base.alpha = 0.85f;
     base.tol = 0.001f;
+    int tile_asked = 0;  // GPX_GRAPH_TILE
     // Vertices per tile of the edge passes.  The searches touch few vertices per pass, and what a
     // CTA pays per tile is the latency of asking which: larger tiles, fewer rounds.  PageRank walks
     // every edge list in every pass and balances better in small tiles: two vertices per warp, walked
@@ -718,7 +743,8 @@ int build_graph_workload(gpx_model &m, const std::string &name, const gpx_model_
         const int by_algo[4] = {64, 32, 32, 16};
         base.tile_verts = by_algo[algo];
         const char *e = getenv("GPX_GRAPH_TILE");
-        if (e && atoi(e) >= 8) base.tile_verts = std::min(atoi(e) / 8 * 8, kGwEdgeTileVertsMax);
+        if (e && atoi(e) >= 8) tile_asked = std::min(atoi(e) / 8 * 8, kGwEdgeTileVertsMax);
+        if (tile_asked) base.tile_verts = tile_asked;
     }
     unsigned long long *row = nullptr;
     unsigned *adj = nullptr;
@@ -730,8 +756,9 @@ int build_graph_workload(gpx_model &m, const std::string &name, const gpx_model_
         std::vector<uint16_t> packed;
         std::vector<unsigned> blk;
         std::vector<uint2> win;
-        if (g.n && pack_lists(trow, tadj, g.n, kGwPackedTileVerts, base.pack, packed, blk, win, base.win_max)) {
-            base.tile_verts = kGwPackedTileVerts;
+        const int packed_tile = tile_asked ? tile_asked : packed_tile_verts(g.n, m.sm_count);
+        if (g.n && packed_tile && pack_lists(trow, tadj, g.n, packed_tile, base.pack, packed, blk, win, base.win_max)) {
+            base.tile_verts = packed_tile;
             uint16_t *d_packed = nullptr;
             unsigned *d_blk = nullptr;
             uint2 *d_win = nullptr;

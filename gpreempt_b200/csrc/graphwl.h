@@ -40,8 +40,6 @@ constexpr int kGwThreads = 256;
 constexpr int kGwEdgeTileVertsMax = 256;  // vertices per tile of an edge pass at most (32 per warp)
 constexpr int kGwVertexTileVerts = 1024;  // vertices per tile of a per-vertex pass
 constexpr int kGwMaxIters = 16384;        // iteration flags a graph workload has: no run may need more rounds
-// (packed PageRank: 52 804 vertices are 826 tiles, fewer than six CTAs on each of 148 SMs)
-constexpr int kGwPackedTileVerts = 64;
 // floats of a tile's window: with the zero behind it and the kernel's own variables in the default 48 KiB
 constexpr int kGwWindowMax = (48 * 1024 - 256) / 4 - 1;
 constexpr unsigned kGwInfinity = 0xFFFFFFFFu;  // MYINFINITY, include/workloads/graphcompute.h:14
@@ -62,8 +60,8 @@ struct GraphWlParams {
     unsigned *d0, *d1;    // pagerank: delta, read from d<iter & 1>, written to the other
     unsigned char *f0;    // sssp: label (the frontier)
     int *active;          // [kGwMaxIters + 1]: active[i] != 0 <=> iteration i has work
-    // pagerank, where the in-neighbours of every tile lie within kGwWindowMax ids (a graph ordered for
-    // locality): the ids as 16-bit offsets into the tile's window, in blocks of 32 x pack (lane l of a
+    // pagerank, for graphs ordered for locality (pack_lists): the ids as 16-bit offsets into the window of ids
+    // the tile can reach, at most kGwWindowMax long, in blocks of 32 x pack (lane l of a
     // block holds edges l, l + 32, ... next to one another), padded with the window's length, where the
     // shared-memory copy of the window holds a zero.
     int pack;                       // ids a lane holds per block: 1, 2, 4 or 8; 0 = lists in adj

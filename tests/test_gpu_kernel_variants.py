@@ -135,11 +135,15 @@ def test_wide_tiles_agree_with_narrow_ones(gpx):
     assert _rel(heads[80][:8], heads[8]) <= 2e-3
 
 
-# Average in-degree around 200, 100, 50 and 16: eight, four, two and one id a lane; the last graph's
-# neighbours lie too far apart for a window and stay lists.
+# Average in-degree around 200, 100, 50 and 16: eight, four, two and one id a lane (in the tiles asked for; by
+# themselves graphs this small stay lists); the last graph's neighbours lie too far apart for a window.
+@pytest.mark.parametrize("tile", [64, 8, 256, None])
 @pytest.mark.parametrize("vertices,degree,band", [(3001, 200, 1500), (2999, 100, 900), (4000, 50, 600), (65, 16, 60), (40001, 20, 39000)])
-def test_pagerank_list_forms(gpx, tmp_path, vertices, degree, band):
+def test_pagerank_list_forms(gpx, tmp_path, monkeypatch, vertices, degree, band, tile):
     from oracle import graphs
+
+    if tile:
+        monkeypatch.setenv("GPX_GRAPH_TILE", str(tile))
 
     graphs.build()
     prefix = str(tmp_path / "g" / "g.bel")
@@ -512,3 +516,38 @@ def test_miniweather_tiles_that_divide(gpx, value):
         assert np.array_equal(a[:, ~near].view(np.uint32), b[:, ~near].view(np.uint32)), kernel
         assert not np.array_equal(a[:, near], b[:, near])
     ex.clear()
+
+
+def _sym(vertices, a, b):
+    """Rows of the symmetric graph with these edges and a chain through all vertices."""
+    chain = np.arange(vertices - 1)
+    a, b = np.concatenate([a, chain]), np.concatenate([b, chain + 1])
+    key = np.unique(np.concatenate([a * vertices + b, b * vertices + a]))
+    return np.split(key % vertices, np.cumsum(np.bincount(key // vertices, minlength=vertices))[:-1])
+
+
+def _banded(rng, vertices, degree, band):
+    a = np.repeat(np.arange(vertices), degree // 2)
+    b = a + rng.integers(1, band + 1, len(a)) * (rng.integers(0, 2, len(a)) * 2 - 1)
+    inside = (b >= 0) & (b < vertices)
+    return _sym(vertices, a[inside], b[inside])
+
+
+def test_pagerank_form_follows_the_graph(gpx, tmp_path, monkeypatch):
+    """Packed tiles of 64 or 32 vertices where there are enough of them, lists (tiles of 16) for small graphs, for
+    neighbours without locality and for skewed degrees; GPX_GRAPH_TILE sets the tile of either form."""
+    rng = np.random.default_rng(5)
+    sm = gpx.device_info()["sm_count"]
+    large, middle, small = 256 * sm + 37, 128 * sm + 5, 60 * sm + 3
+    band = _banded(rng, large, 20, 300)
+    assert _pagerank(gpx, tmp_path, band, "a") == -(-large // 64)
+    assert _pagerank(gpx, tmp_path, _banded(rng, middle, 20, 200), "b") == -(-middle // 32)
+    assert _pagerank(gpx, tmp_path, _banded(rng, small, 60, 300), "c") == -(-small // 16)
+    n = min(12000, middle // 32 * 32)
+    assert _pagerank(gpx, tmp_path, _sym(n, rng.integers(0, n, 10 * n), rng.integers(0, n, 10 * n)), "d") == -(-n // 16)
+    hubs = (large * rng.random(8 * large) ** 4).astype(int)
+    near = np.clip(hubs + rng.integers(-1500, 1501, len(hubs)), 0, large - 1)
+    assert _pagerank(gpx, tmp_path, _sym(large, hubs, near), "e") == -(-large // 16)
+    for tile in (16, 40, 128):
+        monkeypatch.setenv("GPX_GRAPH_TILE", str(tile))
+        assert _pagerank(gpx, tmp_path, band, "f%d" % tile) == -(-large // tile)
