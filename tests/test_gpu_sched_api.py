@@ -1,5 +1,6 @@
 """The scheduler API driven by client threads of the caller: the counterpart of the reference's
 REEF client loop (new_task / wait_task, src/reef-client/reefclient.cpp:105-110)."""
+import random
 import threading
 import time
 
@@ -47,6 +48,7 @@ def test_two_client_threads_share_one_gpu_through_the_scheduler(gpx):
     errors = []
     hp_done, be_done = [0], [0]
     stop = threading.Event()
+    rng = random.Random(7)
 
     def hp_client():
         try:
@@ -57,7 +59,7 @@ def test_two_client_threads_share_one_gpu_through_the_scheduler(gpx):
                 if not np.array_equal(hp.get_output("heads"), hp_want):
                     errors.append("latency-critical result differs")
                 hp_done[0] += 1
-                time.sleep(0.002)
+                time.sleep(rng.uniform(0.0005, 0.0035))  # (a fixed pause can lock to the best-effort period)
         except Exception as e:  # noqa: BLE001
             errors.append(repr(e))
 
