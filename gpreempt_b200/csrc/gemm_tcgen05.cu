@@ -804,7 +804,11 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 }
 
 // Pairs take over where every pair of CTAs gets a tile of its own; with fewer tiles than SMs the single-CTA
-// form spreads over more of them in the same number of rounds.
+// form spreads over more of them in the same number of rounds.  Of an odd number of row blocks the last pair
+// works half for nothing: a tenth and less from nine on.  With fewer the two forms measure alike (3 x 160
+// tiles, K 4096: 150 us single, 149 pairs; 5 x 64, 2048: 69 and 66; 7 x 24, 4096: 74 and 75; a call with its
+// resets; only 3 x 50, where the single form starts a round for two tiles, 84 and 75), and the single one
+// does no work for padding.
 static bool gemm_by_pairs(int M, int N, int sm_count) {
     const int tiles_m = M / kBM, tiles_n = N / kBN;
     return tiles_m * tiles_n >= sm_count && (tiles_m % 2 == 0 || tiles_m >= 9);

@@ -1189,9 +1189,10 @@ int finalize_model(gpx_model &m) {
             // Single-plane operands do one product per K step, so a 128x128 tile cannot be fed
             // fast enough (32 KB of TMA fill per 0.13 us of products): 256-column tiles halve the
             // activation bytes per product, as the stand-alone GEMM's 128x256 tiles do, wherever
-            // they still fill the GPU and the K loop is long enough to outweigh the second
-            // accumulator buffer they give up (ResNet-50's 1x1 convolutions with K <= 512 lose 6 %,
-            // BERT's dense layers and VGG's 3x3 convolutions gain 17-19 %).
+            // they still fill the GPU and the K loop is long enough for the ring to matter: from K = 256
+            // on ResNet-152 b24 fp16 takes 1 541 us instead of 1 503, from 512 or 768 on all models
+            // measure the same, and from 1 152 on BERT-base s512 b32 takes 4 660 instead of 4 390 (never:
+            // 4 752, and VGG-16 b16 769 instead of 720).
             if (m.fmt != PF_SPLIT && !head && cout_st % 256 == 0 && tiles128 / 2 >= m.sm_count &&
                 (long long)eff_k * eff_k * eff_cin >= 768 && !aff)
                 bn = 256;
