@@ -50,30 +50,42 @@ void *driver_entry(const char *name) {
 cudaError_t launch_direct(const void *kernel, unsigned grid, unsigned block, size_t smem, cudaStream_t s, unsigned cluster,
                           void **args) {
     typedef CUresult (*LaunchFn)(const CUlaunchConfig *, CUfunction, void **, void **);
-    static std::atomic<void *> cached{nullptr};
-    void *launch = cached.load(std::memory_order_acquire);
-    if (!launch) {
-        launch = driver_entry("cuLaunchKernelEx");
-        if (!launch) return cudaErrorInsufficientDriver;
-        cached.store(launch, std::memory_order_release);
-    }
-    // The driver's handle of a kernel on the current device: a small table per thread, kept for good (the
-    // library is never unloaded from under its contexts).
+    typedef CUresult (*CurrentFn)(CUcontext *);
+    typedef CUresult (*IdFn)(CUcontext, unsigned long long *);
+    struct Entries {
+        LaunchFn launch;
+        CurrentFn current;
+        IdFn id;
+    };
+    static const Entries driver = {reinterpret_cast<LaunchFn>(driver_entry("cuLaunchKernelEx")),
+                                   reinterpret_cast<CurrentFn>(driver_entry("cuCtxGetCurrent")),
+                                   reinterpret_cast<IdFn>(driver_entry("cuCtxGetId"))};
+    if (!driver.launch || !driver.current || !driver.id) return cudaErrorInsufficientDriver;
+    // The driver's handle of a kernel in a context: a small table per thread.  A context's number is never given
+    // twice, so the handles of one that is gone, or that another has been pushed over, are not met again.
     struct Known {
         const void *kernel;
-        int device;
+        unsigned long long context;
         CUfunction fn;
     };
     static thread_local Known known[128] = {};
-    int device = 0;
-    cudaError_t err = cudaGetDevice(&device);
-    if (err != cudaSuccess) return err;
-    Known &k = known[(reinterpret_cast<uintptr_t>(kernel) >> 4 ^ (uintptr_t)device) % 128];
-    if (k.kernel != kernel || k.device != device) {
-        cudaFunction_t fn = nullptr;
-        err = cudaGetFuncBySymbol(&fn, kernel);
+    CUcontext current = nullptr;
+    unsigned long long context = 0;
+    if (driver.current(&current) != CUDA_SUCCESS || !current) {
+        const cudaError_t err = cudaFree(nullptr);  // (a thread's first call: the runtime makes its context current)
         if (err != cudaSuccess) return err;
-        k = Known{kernel, device, reinterpret_cast<CUfunction>(fn)};
+        driver.current(&current);
+    }
+    CUresult rc = driver.id(current, &context);
+    Known &k = known[(reinterpret_cast<uintptr_t>(kernel) >> 4 ^ (uintptr_t)context) % 128];
+    if (rc != CUDA_SUCCESS || k.kernel != kernel || k.context != context) {
+        cudaFunction_t fn = nullptr;
+        const cudaError_t err = cudaGetFuncBySymbol(&fn, kernel);
+        if (err != cudaSuccess) return err;
+        rc = driver.current(&current);  // (the call may have made a context where the old one was no longer valid)
+        if (rc == CUDA_SUCCESS) rc = driver.id(current, &context);
+        if (rc != CUDA_SUCCESS) return static_cast<cudaError_t>(rc);
+        k = Known{kernel, context, reinterpret_cast<CUfunction>(fn)};
     }
     CUlaunchAttribute at[2];
     at[0].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
@@ -92,7 +104,7 @@ cudaError_t launch_direct(const void *kernel, unsigned grid, unsigned block, siz
     cfg.attrs = at;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
     // (the two interfaces share their error numbers)
-    return static_cast<cudaError_t>(reinterpret_cast<LaunchFn>(launch)(&cfg, k.fn, args, nullptr));
+    return static_cast<cudaError_t>(driver.launch(&cfg, k.fn, args, nullptr));
 }
 
 cuStreamWriteValue32_t driver_stream_write32() {

@@ -551,3 +551,30 @@ def test_pagerank_form_follows_the_graph(gpx, tmp_path, monkeypatch):
     for tile in (16, 40, 128):
         monkeypatch.setenv("GPX_GRAPH_TILE", str(tile))
         assert _pagerank(gpx, tmp_path, band, "f%d" % tile) == -(-large // tile)
+
+
+def test_launches_follow_the_current_context(gpx):
+    """The handle of a kernel belongs to a context, and a thread may change its own: a model made and run in a second
+    context of the device gives the bits of one in the first, before, between and after."""
+    import ctypes
+
+    driver = ctypes.CDLL("libcuda.so.1")
+
+    def run():
+        ex = gpx.BaseExecutor()
+        ex.init("miniweather_200x104")
+        ex.execute()
+        state = ex.model.get("state")
+        ex.clear()
+        return state
+
+    want = run()
+    for _ in range(2):
+        ctx = ctypes.c_void_p()
+        assert driver.cuCtxCreate_v2(ctypes.byref(ctx), 0, 0) == 0  # (and makes it current)
+        try:
+            assert np.array_equal(run(), want)
+        finally:
+            driver.cuCtxPopCurrent_v2(ctypes.byref(ctypes.c_void_p()))
+            driver.cuCtxDestroy_v2(ctx)
+        assert np.array_equal(run(), want)
