@@ -923,14 +923,14 @@ int finalize_model(gpx_model &m) {
             kn.bytes = 4.0 * 4 * (double)n.N * n.W * n.C;
             const char *force_simt = getenv("GPX_ATTN");
             if (m.fmt != PF_SPLIT && !(force_simt && std::string(force_simt) == "simt")) {
-                // Single-plane models: both products on the tensor cores, the values read as they lie
-                // through a transposing descriptor (which the kernel's name tells).
+                // Single-plane models: both products on the tensor cores (".tc"), the values read as they
+                // lie through a transposing descriptor.
                 const uint64_t rows = (uint64_t)n.N * n.W;
                 GPX_TRY(make_tmap_2d_bf16(&q.tq, sq.hi, rows, (uint64_t)n.C, 128, 64, (uint64_t)q.ld));
                 GPX_TRY(make_tmap_2d_bf16(&q.tk, sk.hi, rows, (uint64_t)n.C, 64, 64, (uint64_t)q.ld));
                 GPX_TRY(make_tmap_2d_bf16(&q.tv, sv.hi, rows, (uint64_t)n.C, 64, 64, (uint64_t)q.ld));
                 GPX_CUDA(attention_tc_prepare());
-                kn.name = n.name + ".vt";
+                kn.name = n.name + ".tc";
                 kn.type = KernelType::AttentionTc;
                 kn.threads = attention_tc_threads();
                 q.total_tiles = n.N * n.heads * ((n.W + 127) / 128);

@@ -118,7 +118,7 @@ def test_c4_bert_base_s512_b32_bfloat16(gpx, oracle):
     batch, seq = 32, 512
     ex = gpx.BaseExecutor()
     ex.init("bert_base", batch=batch, seed=7, seq_len=seq, dtype="bfloat16")
-    assert any(n.endswith(".vt") for n in _kernel_names(ex)), "tensor-core attention not selected"
+    assert any(n.endswith(".tc") for n in _kernel_names(ex)), "tensor-core attention not selected"
     ids = np.random.default_rng(6).integers(0, 30522, (batch, seq)).astype(np.int64)
     ex.set_input("data", ids)
     ex.execute()

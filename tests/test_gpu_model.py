@@ -422,7 +422,7 @@ def test_reduced_precision_bert_matches_oracle(gpx, oracle, model, batch, seq, l
     ex = gpx.BaseExecutor()
     ex.init(model, batch=batch, seed=7, seq_len=seq, dtype=dtype)
     names = [ex.model.get_kernel_info(i)["name"] for i in range(ex.get_kernel_num())]
-    assert any(n.endswith(".vt") for n in names), "tensor-core attention not selected"
+    assert any(n.endswith(".tc") for n in names), "tensor-core attention not selected"
     ids = _ids(batch, seq, vocab)
     ex.set_input("data", ids)
     ex.execute()
