@@ -86,11 +86,6 @@ __device__ __forceinline__ float fa_max3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
     return y;
 }
-__device__ __forceinline__ void fa_st_v8(void *ptr, const uint32_t *r) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(ptr), "r"(r[0]), "r"(r[1]),
-                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
 
 template <bool HALF>
 __global__ void __launch_bounds__(kFaThreads, 2)
@@ -398,8 +393,8 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
                 w[i >> 1] = pf_pack2(x, y, FMT);
             }
             bf16_bits *dst = p.out_hi + ((size_t)b * p.S + q0 + row) * p.ld_out + col0 + 32 * wg;
-            fa_st_v8(dst, w);
-            fa_st_v8(dst + 16, w + 8);
+            st_sector(dst, w);
+            st_sector(dst + 16, w + 8);
         }
         fence_proxy_async();  // TMA writes the next tile's operands where ordinary accesses were made
         __syncthreads();

@@ -130,16 +130,11 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 __device__ __forceinline__ void prefetch_tensormap(const void *tmap) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
-// 256-bit global accesses (32-byte aligned): one whole sector per lane.
+// 256-bit global load (32-byte aligned): one whole sector per lane.
 __device__ __forceinline__ void ld_global_v8(const void *ptr, uint32_t *r) {
     asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "l"(ptr));
-}
-__device__ __forceinline__ void st_global_v8(void *ptr, const uint32_t *r) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(ptr), "r"(r[0]), "r"(r[1]),
-                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
 }
 __device__ __forceinline__ float bf16_lo_to_f32(uint32_t packed) { return __uint_as_float(packed << 16); }
 __device__ __forceinline__ float bf16_hi_to_f32(uint32_t packed) {
@@ -1044,13 +1039,13 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     // The output may be a channel slice: nothing is stored past cout_valid.
 #pragma unroll
                     for (int q = 0; q < CH / 16; ++q)
-                        if (valid && c + 16 * q < col_lim) st_global_v8(out_hi + out_off + c + 16 * q, hi + 8 * q);
+                        if (valid && c + 16 * q < col_lim) st_sector(out_hi + out_off + c + 16 * q, hi + 8 * q);
                     if constexpr (TWO) {
                         uint32_t lo[8];
 #pragma unroll
                         for (int q = 0; q < 8; ++q)
                             lo[q] = pack_bf16(f[2 * q] - bf16_lo_to_f32(hi[q]), f[2 * q + 1] - bf16_hi_to_f32(hi[q]));
-                        if (valid && c < col_lim) st_global_v8(out_lo + out_off + c, lo);
+                        if (valid && c < col_lim) st_sector(out_lo + out_off + c, lo);
                     }
 #ifdef GPX_CGEMM_TIMING
                     e_store += clock64() - t_p2;

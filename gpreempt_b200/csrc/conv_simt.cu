@@ -460,13 +460,6 @@ pool_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
     if (threadIdx.x == 0) trace_end(blp, claims.done());
 }
 
-// Eight packed words to 32-byte aligned global memory, one whole sector.
-__device__ __forceinline__ void st_sector(plane_bits *ptr, const unsigned (&r)[8]) {
-    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(ptr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
-                 "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-
 // Patch matrix for the tensor-core GEMM: one thread-iteration writes eight consecutive columns
 // (one 16-byte vector per plane) of one row.
 __global__ void __launch_bounds__(kPoolThreads)

@@ -106,6 +106,13 @@ __device__ __forceinline__ void planes_store8(plane_bits *hi, plane_bits *lo, si
     }
 }
 
+// 256-bit global store of eight packed words (32-byte aligned): one whole sector per lane.
+__device__ __forceinline__ void st_sector(void *ptr, const unsigned *r) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(ptr), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+
 // One channel (the CUDA-core convolution path).
 __device__ __forceinline__ float planes_load1(const plane_bits *hi, const plane_bits *lo, size_t off, int fmt) {
     if (fmt == PF_F16) return __half2float(*reinterpret_cast<const __half *>(hi + off));
