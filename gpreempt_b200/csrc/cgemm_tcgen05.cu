@@ -244,11 +244,12 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     const uint32_t tmem_base = ctl->tmem_base;
     if (in_cluster) cluster_arrive();  // this CTA runs: its shared memory may be written to
 
-    // A non-preemptible launch knows its first tile without reading the cursor, and weights are
-    // never written by a kernel: its producer thread fetches the weight tiles of the first ring
+    // A non-preemptible launch knows its first tile without reading the cursor, and parameters are
+    // never written by a kernel: its producer warp fetches the weight tiles of the first ring
     // stages before it waits for the predecessor, so that their latency overlaps the
-    // predecessor's tail (batch-1 forwards are chains of such latencies).  Every other thread,
-    // and every thread of a preemptible launch, waits here.
+    // predecessor's tail (batch-1 forwards are chains of such latencies).  The other roles go to their
+    // places before the predecessor has finished too: only activations (the producer's A tiles, the
+    // epilogue's residual and its stores) wait for it.  Every thread of a preemptible launch waits here.
     const bool early_weights = !resumable && (int)blockIdx.x < total_tiles;
     int prearmed = 0;  // K blocks whose barrier is armed and whose weight loads are in flight
     constexpr int KPS = Cfg::kKps;
@@ -287,13 +288,12 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         }
         __syncwarp();
     }
-    pdl_wait();  // from here on the predecessor's results (and this executor's slots) are visible
-    pdl_launch_dependents();
+    if (resumable || warp == 0) {
+        pdl_wait();  // from here on the predecessor's results (and this executor's slots) are visible
+        pdl_launch_dependents();
+    }
     TCK(t_begin);
-    if (in_cluster) cluster_wait();
-#ifdef GPX_CGEMM_TIMING
-    if (threadIdx.x == 64) TADD(16, clock64() - t_begin);
-#endif
+    bool cluster_runs = !in_cluster;  // this thread knows that every CTA of the cluster runs
 
     // A non-preemptible launch never stops early, so it neither reads nor writes the cursor.
     const int first_iter = resumable ? slot->next_iter : 0;
@@ -343,7 +343,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     constexpr int kGroups = BN / 8, kFinItems = 64 * kGroups / Cfg::kEpiThreads;
     bool fin_live[kFinItems] = {};
     int fin_col[kFinItems];
-    size_t fin_off[kFinItems];
+    size_t fin_off[kFinItems], fin_res[kFinItems];
     float fin_bias[kFinItems][8];
     uint4 fin_rhi[kFinItems], fin_rlo[kFinItems];
 
@@ -766,7 +766,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
         const bool leader = (int)threadIdx.x == 64 + group * group_threads;
         if (in_cluster) {
-            // What the finishing step needs, ahead of the products: destination, bias, residual.
+            // What the finishing step needs, ahead of the products: destination, bias, where the residual is.
             const SplitKParams &fin = p.fin;
             const int rows_share = kCBM / p.k_splits;
             const int img = fin.in_hs * fin.in_ws;
@@ -793,9 +793,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                         fin_bias[i][0] = b0.x, fin_bias[i][1] = b0.y, fin_bias[i][2] = b0.z, fin_bias[i][3] = b0.w;
                         fin_bias[i][4] = b1.x, fin_bias[i][5] = b1.y, fin_bias[i][6] = b1.z, fin_bias[i][7] = b1.w;
                     }
-                    if (fin.res_hi)
-                        planes_fetch8(fin.res_hi, fin.res_lo, (size_t)layout_row(fin.res, n_img, h, w) * fin.res.C + col0,
-                                      fin.res.fmt, fin_rhi[i], fin_rlo[i]);
+                    if (fin.res_hi) fin_res[i] = (size_t)layout_row(fin.res, n_img, h, w) * fin.res.C + col0;
                     fin_off[i] = fin.out_f32 ? ((size_t)(n_img * fin.out.H + h) * fin.out.W + w) * fin.cout_valid + col0
                                              : (size_t)layout_row(fin.out, n_img, h, w) * fin.out.C + col0;
                     fin_col[i] = col0;
@@ -822,10 +820,18 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             }
             tmem_st_wait();
         }
-        tc_fence_before_sync();
-        asm volatile("bar.sync 3, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
+        if (resumable) {
+            tc_fence_before_sync();
+            asm volatile("bar.sync 3, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
+        }
         if (threadIdx.x == 64)
             for (int b = 0; b < 2; ++b) mbar_arrive(smem_u32(&ctl->tmem_empty[b]));
+        if (!resumable) pdl_wait();  // the residual is the predecessor's business, everything above is not
+        if (in_cluster && p.fin.res_hi) {
+#pragma unroll
+            for (int i = 0; i < kFinItems; ++i)
+                if (fin_live[i]) planes_fetch8(p.fin.res_hi, p.fin.res_lo, fin_res[i], p.fin.res.fmt, fin_rhi[i], fin_rlo[i]);
+        }
 
         int it = first_iter + group;
         int seg_k0 = group == 0 ? first_k : 0;
@@ -1059,7 +1065,13 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     // [split][row of the share][BN + 4 floats] in that CTA's last ring stages).
                     fence_proxy_async();
                     group_sync();
+                    TCK(t_c1);
+                    cluster_wait();  // every CTA of the cluster runs
+                    cluster_runs = true;
                     const int owner = (int)threadIdx.x - 64;
+#ifdef GPX_CGEMM_TIMING
+                    if (threadIdx.x == 64) TADD(22, t_c1 - t_begin);
+#endif
                     if (owner < p.k_splits) {
                         const uint32_t share = (uint32_t)(kCBM / p.k_splits * (BN + 4) * 4);
                         bulk_copy_to_cluster(cluster_map_shared(smem_base + (uint32_t)(nst * Cfg::kStageBytes) + cluster_ctarank() * share, (uint32_t)owner),
@@ -1135,7 +1147,11 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             if (!mbar_wait(smem_u32(&ctl->landed), 0, &never, kCWaitLimitNs + kCWaitLimitNs / 2)) fail(601);
         }
         __syncwarp();
+        if (!cluster_runs) cluster_wait();
         cluster_arrive();
+#ifdef GPX_CGEMM_TIMING
+        if (threadIdx.x == 64) TADD(23, clock64() - t_begin);
+#endif
         if (finishes) {
             const float *land = reinterpret_cast<const float *>(smem + nst * Cfg::kStageBytes);
             const SplitKParams &fin = p.fin;
