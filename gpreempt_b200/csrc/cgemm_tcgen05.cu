@@ -52,9 +52,12 @@ struct CgemmControlSize {
 
 // BN: columns of an output tile.  TWO: two-plane operands (float32 models), three products per K step;
 // otherwise one 16-bit plane and one product.
-template <int BN, bool TWO, bool AFF>
+// CL: the CTAs of a cluster share the K range of a 64-column tile and reduce it among themselves
+// (latency-critical launches, one tile a CTA); the sixteen epilogue warps halve the chain of
+// instructions behind the products, which is what such a launch waits for.
+template <int BN, bool TWO, bool AFF, bool CL>
 struct CgemmCfg {
-    static constexpr int kEpiParts = BN == 256 ? 4 : 2;          // epilogue warps per TMEM lane quarter
+    static constexpr int kEpiParts = BN == 256 || (CL && !AFF) ? 4 : 2;  // epilogue warps per TMEM lane quarter
     static constexpr int kEpiThreads = 128 * kEpiParts;
     static constexpr int kPollWarp = 2 + kEpiThreads / 32;
     static constexpr int kThreads = 64 + kEpiThreads + 32 + (AFF ? kCAffThreads : 0);
@@ -69,8 +72,9 @@ struct CgemmCfg {
     static constexpr int kKps = (!TWO && !AFF && BN <= 128) ? 2 : 1;
     static constexpr uint32_t kStageBytes = kKps * kKbBytes;
     static constexpr int kStages = (int)((192u * 1024u) / kStageBytes);  // 3 to 8
-    // ring stages the landing area of a cluster reduction takes (128 rows of BN + 4 floats)
-    static constexpr int kLandStages = (int)((kCBM * (BN + 4) * 4 + kStageBytes - 1) / kStageBytes);
+    // ring stages the landing area of a cluster reduction takes (128 rows of BN floats)
+    static constexpr int kLandStages = CL ? (int)((kCBM * BN * 4 + kStageBytes - 1) / kStageBytes) : 0;
+    static constexpr int kRing = kStages - kLandStages;  // stages in use as the ring
     // ring + alignment slack + 64x64 identity tile + control block
     static constexpr uint32_t kIdentBytes = 64 * kCBK * 2;
     static constexpr size_t kSmem =
@@ -81,7 +85,7 @@ struct CgemmCfg {
     static constexpr int kBufCols = (int)kPlanes * BN;
     static constexpr int kTmemCols = 2 * kBufCols;
     static_assert(kTmemCols <= 512 && kStages <= 8, "tile does not fit");
-    static_assert(BN != 64 || kStages - kLandStages >= 3, "no ring left beside the landing area");
+    static_assert(kRing >= 3 && (!CL || BN == 64), "no ring left beside the landing area");
 };
 
 // Message of a ring stage: CMSG_DATA + number of K blocks, CMSG_RES + index of the residual block, or
@@ -152,10 +156,10 @@ __device__ unsigned long long g_cgemm_timing[32];
 #define TADD(slot, val)
 #endif
 
-template <int BN, bool TWO, bool AFF>
-__global__ void __launch_bounds__(CgemmCfg<BN, TWO, AFF>::kThreads, 1)
+template <int BN, bool TWO, bool AFF, bool CL>
+__global__ void __launch_bounds__(CgemmCfg<BN, TWO, AFF, CL>::kThreads, 1)
 cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
-    using Cfg = CgemmCfg<BN, TWO, AFF>;
+    using Cfg = CgemmCfg<BN, TWO, AFF, CL>;
     constexpr int kStages = Cfg::kStages;
     constexpr int kBufCols = Cfg::kBufCols;
     TCK(t_start);
@@ -192,10 +196,8 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         t.main_kb = left < p.kb_per_split ? left : p.kb_per_split;
         return t;
     };
-    const bool resumable = blp.preempted != nullptr;
-    // Split K inside a cluster: the peers' partial sums land in the last ring stages.
-    const bool in_cluster = BN == 64 && p.cluster_reduce;
-    const int nst = in_cluster ? kStages - Cfg::kLandStages : kStages;
+    const bool resumable = !CL && blp.preempted != nullptr;
+    constexpr int nst = Cfg::kRing;
 
     CgemmSlot *slot = p.slots + blockIdx.x;
     float *spill = p.spill + (size_t)blockIdx.x * cgemm_spill_floats();
@@ -212,9 +214,15 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             ctl->epi_kind[b] = CEPI_COMPLETE;
             ctl->epi_k_done[b] = 0;
         }
-        if (in_cluster) {
+        if (CL) {
+            // a row of the share this CTA finishes comes from each of the k_splits CTAs, if it is a row of the GEMM
+            const int share = kCBM / p.k_splits;
+            const int rows = p.m_rows - tile_at(blockIdx.x).m_blk * kCBM - (int)cluster_ctarank() * share;
             mbar_init(smem_u32(&ctl->landed), 1);
-            mbar_arrive_expect_tx(smem_u32(&ctl->landed), kCBM * (BN + 4) * 4);
+            if (rows > 0)
+                mbar_arrive_expect_tx(smem_u32(&ctl->landed), (uint32_t)((rows < share ? rows : share) * p.k_splits * BN * 4));
+            else
+                mbar_arrive(smem_u32(&ctl->landed));
         }
         ctl->abort_flag = 0;
         ctl->epi_go[0] = ctl->epi_go[1] = 0;
@@ -242,7 +250,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = ctl->tmem_base;
-    if (in_cluster) cluster_arrive();  // this CTA runs: its shared memory may be written to
+    if (CL) cluster_arrive();  // this CTA runs: its shared memory may be written to
 
     // A non-preemptible launch knows its first tile without reading the cursor, and parameters are
     // never written by a kernel: its producer warp fetches the weight tiles of the first ring
@@ -293,7 +301,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         pdl_launch_dependents();
     }
     TCK(t_begin);
-    bool cluster_runs = !in_cluster;  // this thread knows that every CTA of the cluster runs
 
     // A non-preemptible launch never stops early, so it neither reads nor writes the cursor.
     const int first_iter = resumable ? slot->next_iter : 0;
@@ -338,14 +345,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         ctl->abort_flag = 1;
         if (atomicCAS(p.error, 0, code) == 0) p.error[1] = blp.kernel_id * 1000 + (int)blockIdx.x;
     };
-
-    // Cluster reduction: what this thread finishes (eight-channel items; two of them when S = 2).
-    constexpr int kGroups = BN / 8, kFinItems = 64 * kGroups / Cfg::kEpiThreads;
-    bool fin_live[kFinItems] = {};
-    int fin_col[kFinItems];
-    size_t fin_off[kFinItems], fin_res[kFinItems];
-    float fin_bias[kFinItems][8];
-    uint4 fin_rhi[kFinItems], fin_rlo[kFinItems];
 
     if (!grid_ok) {
         if (threadIdx.x == 0) fail(900);
@@ -746,6 +745,124 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             }
         }
         __syncwarp();
+    } else if constexpr (CL) {
+        // ------------------------------------------------------------------ epilogue of a cluster reduction
+        // Each of the k_splits CTAs finishes 128 / k_splits rows of the tile: every CTA stores the rows of its
+        // partial sums, straight from its accumulators, into their owners' shared memory
+        // ([split][column / 4][row of the share] of 16 bytes), counted on the owner's barrier, and the
+        // owner adds the splits in order from zero, exactly as splitk_finish_kernel adds the workspace rows,
+        // then bias, residual, activation, store.  What that needs besides the sums is at hand before.
+        // (Staged and copied in bulk, the rows took 2 100 cycles to arrive and another 2 000 to 3 600 to
+        // be finished by eight warps; through the workspace the release in front of the barrier alone took 2 800.)
+        // Nobody leaves before its own rows are complete, and nothing else is ever stored to it.
+        const SplitKParams &fin = p.fin;
+        const int splits = p.k_splits, share = kCBM / splits, lg_share = 31 - __clz(share);
+        const int rank = (int)cluster_ctarank();
+        const int row0 = first_tile.m_blk * kCBM;
+        constexpr int kItems = kCBM / 2 * (BN / 4) / Cfg::kEpiThreads;  // four-channel items a thread finishes (two splits)
+        bool live[kItems];
+        int col[kItems];
+        uint32_t land_at[kItems];
+        size_t out_at[kItems], res_at[kItems];
+        float4 bias4[kItems];
+        uint2 r_hi[kItems], r_lo[kItems];
+        const uint32_t land = smem_base + (uint32_t)(nst * Cfg::kStageBytes);
+        const int img = fin.in_hs * fin.in_ws;
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            // eight rows by four pieces a warp: sixteen-byte reads without bank conflicts, whole sectors stored
+            const int e = (int)threadIdx.x - 64 + i * Cfg::kEpiThreads;
+            const int lr = (e & 7) | (((e >> 5) & ((share >> 3) - 1)) << 3), piece = ((e >> 3) & 3) | ((e >> (2 + lg_share)) << 2);
+            const int vrow = row0 + rank * share + lr;
+            col[i] = first_tile.n_blk * BN + piece * 4;
+            land_at[i] = land + (uint32_t)(piece * share + lr) * 16;
+            live[i] = piece < BN / 4 && vrow < fin.m_rows && col[i] < fin.cout_padded;
+            if (live[i]) {
+                const int n_img = fast_div(vrow, img, p.inv_img);
+                const int r = vrow - n_img * img;
+                const int hs = fast_div(r, fin.in_ws, p.inv_in_ws);
+                const int h = hs - fin.in_off, w = r - hs * fin.in_ws - fin.in_off;
+                live[i] = h >= 0 && h < fin.out.H && w >= 0 && w < fin.out.W;
+                if (live[i]) {
+                    if (fin.bias) bias4[i] = __ldg(reinterpret_cast<const float4 *>(fin.bias + col[i]));
+                    if (fin.res_hi) res_at[i] = (size_t)layout_row(fin.res, n_img, h, w) * fin.res.C + col[i];
+                    out_at[i] = fin.out_f32 ? ((size_t)(n_img * fin.out.H + h) * fin.out.W + w) * fin.cout_valid + col[i]
+                                            : (size_t)layout_row(fin.out, n_img, h, w) * fin.out.C + col[i];
+                }
+            }
+        }
+        if (threadIdx.x == 64)
+            for (int b = 0; b < 2; ++b) mbar_arrive(smem_u32(&ctl->tmem_empty[b]));
+        cluster_wait();  // every CTA of the cluster runs
+        pdl_wait();      // the residual is the predecessor's business, everything above is not
+        if (fin.res_hi)
+#pragma unroll
+            for (int i = 0; i < kItems; ++i)
+                if (live[i]) {
+                    r_hi[i] = *reinterpret_cast<const uint2 *>(fin.res_hi + res_at[i]);
+                    if (TWO) r_lo[i] = *reinterpret_cast<const uint2 *>(fin.res_lo + res_at[i]);
+                }
+        const int row = (warp & 3) * 32 + lane;
+        constexpr int kCols = BN / Cfg::kEpiParts;
+        const int c_lo = ((warp - 2) >> 2) * kCols;
+        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->tmem_full[0]), 0, abort_flag, kCWaitLimitNs))) {
+            if (lane == 0) fail(301);
+        } else {
+            tc_fence_after_sync();
+            const uint32_t t_acc = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+            const uint32_t owner = (uint32_t)row >> lg_share;
+            const uint32_t bar = cluster_map_shared(smem_u32(&ctl->landed), owner);
+            const uint32_t to = cluster_map_shared(land + ((uint32_t)(rank * (BN / 4)) * share + (row & (share - 1))) * 16, owner);
+#pragma unroll
+            for (int c = c_lo; c < c_lo + kCols; c += 16) {
+                uint32_t u[16], w[16];
+                tmem_ld_32x16(t_acc + c, u);
+                if (TWO) tmem_ld_32x16(t_acc + BN + c, w);
+                tmem_ld_wait();
+                if (TWO)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) u[j] = __float_as_uint(__uint_as_float(u[j]) + __uint_as_float(w[j]));
+                if (row0 + row < p.m_rows)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) st_async_v4(to + (uint32_t)((c / 4 + j) * share) * 16, u + 4 * j, bar);
+            }
+        }
+        volatile int never = 0;  // (a CTA that failed waits here as well, so that no store finds its memory gone)
+        if (!mbar_wait(smem_u32(&ctl->landed), 0, &never, kCWaitLimitNs + kCWaitLimitNs / 2)) fail(601);
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            if (!live[i]) continue;
+            float f[4] = {0.f, 0.f, 0.f, 0.f};
+            const uint32_t stride = (uint32_t)(share * (BN / 4)) * 16;
+            for (int sp = 0; sp < splits; sp += 2) {
+                const float4 a = lds_f4(land_at[i] + sp * stride), b = lds_f4(land_at[i] + (sp + 1) * stride);
+                f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
+                f[0] += b.x; f[1] += b.y; f[2] += b.z; f[3] += b.w;
+            }
+            if (fin.bias) f[0] += bias4[i].x, f[1] += bias4[i].y, f[2] += bias4[i].z, f[3] += bias4[i].w;
+            if (fin.res_hi) {
+                float2 r0 = pf_unpack2(r_hi[i].x, TWO ? (int)PF_SPLIT : fin.res.fmt), r1 = pf_unpack2(r_hi[i].y, TWO ? (int)PF_SPLIT : fin.res.fmt);
+                if (TWO) {
+                    r0.x += bf16_lo_to_f32(r_lo[i].x), r0.y += bf16_hi_to_f32(r_lo[i].x);
+                    r1.x += bf16_lo_to_f32(r_lo[i].y), r1.y += bf16_hi_to_f32(r_lo[i].y);
+                }
+                f[0] += r0.x, f[1] += r0.y, f[2] += r1.x, f[3] += r1.y;
+            }
+            apply_act_n(f, fin.relu);
+            if (fin.out_f32) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (col[i] + j < fin.cout_valid) fin.out_f32[out_at[i] + j] = f[j];
+            } else {
+                const int fmt = TWO ? (int)PF_SPLIT : fin.out.fmt;
+                const uint32_t h0 = pf_pack2(f[0], f[1], fmt), h1 = pf_pack2(f[2], f[3], fmt);
+                *reinterpret_cast<uint2 *>(fin.out_hi + out_at[i]) = make_uint2(h0, h1);
+                if (TWO)
+                    *reinterpret_cast<uint2 *>(fin.out_lo + out_at[i]) =
+                        make_uint2(pack_bf16(f[0] - bf16_lo_to_f32(h0), f[1] - bf16_hi_to_f32(h0)),
+                                   pack_bf16(f[2] - bf16_lo_to_f32(h1), f[3] - bf16_hi_to_f32(h1)));
+            }
+        }
     } else {
         // ------------------------------------------------------------------ epilogue
         const int quarter = warp & 3;
@@ -765,42 +882,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         const int row = quarter * 32 + lane;
         const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
         const bool leader = (int)threadIdx.x == 64 + group * group_threads;
-        if (in_cluster) {
-            // What the finishing step needs, ahead of the products: destination, bias, where the residual is.
-            const SplitKParams &fin = p.fin;
-            const int rows_share = kCBM / p.k_splits;
-            const int img = fin.in_hs * fin.in_ws;
-            const int rank = (int)cluster_ctarank();
-#pragma unroll
-            for (int i = 0; i < kFinItems; ++i) {
-                const int e = (int)threadIdx.x - 64 + i * Cfg::kEpiThreads;
-                const int lr = e / kGroups, col0 = first_tile.n_blk * BN + (e - lr * kGroups) * 8;
-                const int vrow = first_tile.m_blk * kCBM + rank * rows_share + lr;
-                bool live = lr < rows_share && vrow < fin.m_rows && col0 < fin.cout_padded;
-                int n_img = 0, h = 0, w = 0;
-                if (live) {
-                    n_img = fast_div(vrow, img, p.inv_img);
-                    const int r = vrow - n_img * img;
-                    const int hs = fast_div(r, fin.in_ws, p.inv_in_ws);
-                    h = hs - fin.in_off;
-                    w = r - hs * fin.in_ws - fin.in_off;
-                    live = h >= 0 && h < fin.out.H && w >= 0 && w < fin.out.W;
-                }
-                if (live) {
-                    if (fin.bias) {
-                        const float4 *b4 = reinterpret_cast<const float4 *>(fin.bias + col0);
-                        const float4 b0 = __ldg(b4), b1 = __ldg(b4 + 1);
-                        fin_bias[i][0] = b0.x, fin_bias[i][1] = b0.y, fin_bias[i][2] = b0.z, fin_bias[i][3] = b0.w;
-                        fin_bias[i][4] = b1.x, fin_bias[i][5] = b1.y, fin_bias[i][6] = b1.z, fin_bias[i][7] = b1.w;
-                    }
-                    if (fin.res_hi) fin_res[i] = (size_t)layout_row(fin.res, n_img, h, w) * fin.res.C + col0;
-                    fin_off[i] = fin.out_f32 ? ((size_t)(n_img * fin.out.H + h) * fin.out.W + w) * fin.cout_valid + col0
-                                             : (size_t)layout_row(fin.out, n_img, h, w) * fin.out.C + col0;
-                    fin_col[i] = col0;
-                }
-                fin_live[i] = live;
-            }
-        }
         uint32_t v[32];
         if (first_k > 0) {
             for (int c = share * kRestoreCols; c < (share + 1) * kRestoreCols; c += 32) {
@@ -827,12 +908,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         if (threadIdx.x == 64)
             for (int b = 0; b < 2; ++b) mbar_arrive(smem_u32(&ctl->tmem_empty[b]));
         if (!resumable) pdl_wait();  // the residual is the predecessor's business, everything above is not
-        if (in_cluster && p.fin.res_hi) {
-#pragma unroll
-            for (int i = 0; i < kFinItems; ++i)
-                if (fin_live[i]) planes_fetch8(p.fin.res_hi, p.fin.res_lo, fin_res[i], p.fin.res.fmt, fin_rhi[i], fin_rlo[i]);
-        }
-
         int it = first_iter + group;
         int seg_k0 = group == 0 ? first_k : 0;
         int tiles_done = 0;
@@ -940,7 +1015,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 constexpr int CH = (TWO || AFF || BN == 256) ? 16 : 32;  // columns per piece
                 // (columns past the real output, a quarter to a half of a tile for a DenseNet layer, are left out;
                 // partial sums go out whole)
-                const int c_end = partial || in_cluster || c_hi < col_lim ? c_hi : col_lim;
+                const int c_end = partial || c_hi < col_lim ? c_hi : col_lim;
 #pragma unroll 1
                 for (int c = c_lo; c < c_end; c += CH) {
                     float f[CH];
@@ -973,16 +1048,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     long long t_p1 = clock64();
                     e_tmem += t_p1 - t_p0;
 #endif
-                    if (in_cluster) {
-                        // Split K inside a cluster: the raw fp32 sum of this K range stays in this CTA's
-                        // ring (idle: such a launch runs one tile) until the tile is complete; rows are
-                        // 16 bytes longer than BN floats so that the rows of a warp spread over the banks.
-                        float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(smem) + row * (BN + 4) + c);
-#pragma unroll
-                        for (int j = 0; j < CH / 4; ++j)
-                            dst[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
-                        continue;
-                    }
                     if (partial) {
                         // Split K: the raw fp32 sum of this K range goes to the workspace; the
                         // finishing kernel adds the ranges in split order and applies the rest.
@@ -1060,26 +1125,6 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 it += groups;
                 ++tiles_done;
                 seg_k0 = 0;
-                if (in_cluster) {
-                    // Every share of rows goes to the CTA that finishes it as one bulk copy (landing area:
-                    // [split][row of the share][BN + 4 floats] in that CTA's last ring stages).
-                    fence_proxy_async();
-                    group_sync();
-                    TCK(t_c1);
-                    cluster_wait();  // every CTA of the cluster runs
-                    cluster_runs = true;
-                    const int owner = (int)threadIdx.x - 64;
-#ifdef GPX_CGEMM_TIMING
-                    if (threadIdx.x == 64) TADD(22, t_c1 - t_begin);
-#endif
-                    if (owner < p.k_splits) {
-                        const uint32_t share = (uint32_t)(kCBM / p.k_splits * (BN + 4) * 4);
-                        bulk_copy_to_cluster(cluster_map_shared(smem_base + (uint32_t)(nst * Cfg::kStageBytes) + cluster_ctarank() * share, (uint32_t)owner),
-                                             smem_base + (uint32_t)owner * share, share,
-                                             cluster_map_shared(smem_u32(&ctl->landed), (uint32_t)owner));
-                    }
-                    break;
-                }
                 tc_fence_before_sync();
                 TCK(t_b0);
                 group_sync();
@@ -1127,92 +1172,8 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     }
 
     tc_fence_before_sync();
-    if constexpr (BN != 64) {
-        __syncthreads();
-    } else if (in_cluster) {
-        // This CTA finishes rows [rank, rank+1) * 128/S of the output block from its own shared memory
-        // once every CTA of the cluster has copied its partial rows of them there: the S partial rows
-        // are added in split order from zero, exactly as splitk_finish_kernel adds the workspace
-        // rows, then bias, residual, activation, store.  Where the rows go, the bias and the residual
-        // were fetched before the products were waited for.  The copies this CTA sent still read its ring
-        // until they have landed, and only their owners see that: every CTA arrives on the cluster barrier
-        // once its own rows are complete and leaves when all have, so no ring is handed to a successor's
-        // loads under a copy.  The barrier hides behind the finishing step.  (Pulling the rows from the
-        // peers after a cluster barrier, one split at a time, and a second barrier before the exit made this
-        // step 4 us long, BERT-base b1 7.4 us per projection; storing them to the peers element by element,
-        // 2 us.)  A CTA that failed waits here as well, so that no copy finds its memory gone.
-        const bool finishes = warp >= 2 && warp < Cfg::kPollWarp;
-        if (finishes) {
-            volatile int never = 0;
-            if (!mbar_wait(smem_u32(&ctl->landed), 0, &never, kCWaitLimitNs + kCWaitLimitNs / 2)) fail(601);
-        }
-        __syncwarp();
-        if (!cluster_runs) cluster_wait();
-        cluster_arrive();
-#ifdef GPX_CGEMM_TIMING
-        if (threadIdx.x == 64) TADD(23, clock64() - t_begin);
-#endif
-        if (finishes) {
-            const float *land = reinterpret_cast<const float *>(smem + nst * Cfg::kStageBytes);
-            const SplitKParams &fin = p.fin;
-            auto finish = [&](auto splits) {
-                constexpr int S = decltype(splits)::value, rows_per = kCBM / S;
-                constexpr int kItems = rows_per * kGroups;  // eight-channel items of this CTA
-#pragma unroll
-                for (int i = 0; i < (kItems + Cfg::kEpiThreads - 1) / Cfg::kEpiThreads; ++i) {
-                    if (!fin_live[i]) continue;
-                    const int e = (int)threadIdx.x - 64 + i * Cfg::kEpiThreads;
-                    const int lr = e / kGroups, c8 = (e - lr * kGroups) * 8;
-                    float4 q[2 * S];
-#pragma unroll
-                    for (int sidx = 0; sidx < S; ++sidx) {
-                        const float4 *src = reinterpret_cast<const float4 *>(land + (sidx * rows_per + lr) * (BN + 4) + c8);
-                        q[2 * sidx] = src[0];
-                        q[2 * sidx + 1] = src[1];
-                    }
-                    float f[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) f[j] = 0.f;
-#pragma unroll
-                    for (int sidx = 0; sidx < S; ++sidx) {
-                        const float4 a = q[2 * sidx], b = q[2 * sidx + 1];
-                        f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
-                        f[4] += b.x; f[5] += b.y; f[6] += b.z; f[7] += b.w;
-                    }
-                    if (fin.bias)
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) f[j] += fin_bias[i][j];
-                    if (fin.res_hi) {
-                        float r[8];
-                        planes_decode8(fin_rhi[i], fin_rlo[i], fin.res.fmt, r);
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) f[j] += r[j];
-                    }
-                    apply_act_n(f, fin.relu);
-                    if (fin.out_f32) {
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (fin_col[i] + j < fin.cout_valid) fin.out_f32[fin_off[i] + j] = f[j];
-                    } else {
-                        planes_store8(fin.out_hi, fin.out_lo, fin_off[i], fin.out.fmt, f);
-                    }
-                }
-            };
-            if (p.k_splits == 8)
-                finish(std::integral_constant<int, 8>());
-            else if (p.k_splits == 4)
-                finish(std::integral_constant<int, 4>());
-            else
-                finish(std::integral_constant<int, 2>());
-        }
-#ifdef GPX_CGEMM_TIMING
-        if (threadIdx.x == 64) TADD(21, clock64() - t_begin);
-#endif
-        __syncwarp();
-        cluster_wait();  // (tensor memory is released below by warp 1)
-    } else {
-        __syncthreads();
-    }
+    if (CL && (warp < 2 || warp >= Cfg::kPollWarp)) cluster_wait();
+    __syncthreads();
     if (warp == 0 && lane == 0 && *abort_flag) {
         for (int spin = 0; spin < 64; ++spin) __nanosleep(1000);
     }
@@ -1242,43 +1203,51 @@ extern "C" int gpx_debug_cgemm_timing(unsigned long long *out, int reset) {
 }
 #endif
 
-// Calls f with the kernel instance of a tile width, operand format and A treatment (as a struct of
+// Calls f with the kernel instance of a tile width, operand format, A treatment and reduction (as a struct of
 // constants).  256-column tiles exist for single-plane operands used as they are: two planes' two
 // accumulators in two buffers would not fit tensor memory, and no layer behind an affine map is wide.
-template <int BN, bool TWO, bool AFF>
+template <int BN, bool TWO, bool AFF, bool CL>
 struct CgemmInstance {
-    using Cfg = CgemmCfg<BN, TWO, AFF>;
-    static constexpr auto kernel() { return cgemm_tcgen05_kernel<BN, TWO, AFF>; }
+    using Cfg = CgemmCfg<BN, TWO, AFF, CL>;
+    static constexpr auto kernel() { return cgemm_tcgen05_kernel<BN, TWO, AFF, CL>; }
 };
 template <typename F>
-static auto cgemm_instance(int bn, bool two, bool aff, F &&f) {
-    if (two && aff) return bn == 128 ? f(CgemmInstance<128, true, true>()) : f(CgemmInstance<64, true, true>());
-    if (two) return bn == 128 ? f(CgemmInstance<128, true, false>()) : f(CgemmInstance<64, true, false>());
-    if (aff) return bn == 128 ? f(CgemmInstance<128, false, true>()) : f(CgemmInstance<64, false, true>());
-    if (bn == 256) return f(CgemmInstance<256, false, false>());
-    return bn == 128 ? f(CgemmInstance<128, false, false>()) : f(CgemmInstance<64, false, false>());
+static auto cgemm_instance(int bn, bool two, bool aff, bool cluster, F &&f) {
+    if (cluster) {
+        if (two) return aff ? f(CgemmInstance<64, true, true, true>()) : f(CgemmInstance<64, true, false, true>());
+        return aff ? f(CgemmInstance<64, false, true, true>()) : f(CgemmInstance<64, false, false, true>());
+    }
+    if (two && aff) return bn == 128 ? f(CgemmInstance<128, true, true, false>()) : f(CgemmInstance<64, true, true, false>());
+    if (two) return bn == 128 ? f(CgemmInstance<128, true, false, false>()) : f(CgemmInstance<64, true, false, false>());
+    if (aff) return bn == 128 ? f(CgemmInstance<128, false, true, false>()) : f(CgemmInstance<64, false, true, false>());
+    if (bn == 256) return f(CgemmInstance<256, false, false, false>());
+    return bn == 128 ? f(CgemmInstance<128, false, false, false>()) : f(CgemmInstance<64, false, false, false>());
 }
 
 cudaError_t cgemm_prepare(int device) {
     static bool done[64] = {false};
     if (device < 0 || device >= 64 || done[device]) return cudaSuccess;
+    auto allow = [](auto k) {
+        return cudaFuncSetAttribute(k.kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decltype(k)::Cfg::kSmem);
+    };
     for (int two = 0; two < 2; ++two)
-        for (int aff = 0; aff < 2; ++aff)
+        for (int aff = 0; aff < 2; ++aff) {
             for (int bn : {64, 128, 256}) {
                 if (bn == 256 && (two || aff)) continue;
-                cudaError_t e = cgemm_instance(bn, two != 0, aff != 0, [](auto k) {
-                    return cudaFuncSetAttribute(k.kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)decltype(k)::Cfg::kSmem);
-                });
+                cudaError_t e = cgemm_instance(bn, two != 0, aff != 0, false, allow);
                 if (e != cudaSuccess) return e;
             }
+            cudaError_t e = cgemm_instance(64, two != 0, aff != 0, true, allow);
+            if (e != cudaSuccess) return e;
+        }
     done[device] = true;
     return cudaSuccess;
 }
 
-// CTAs of clusters of `cluster` CTAs of this kernel that the device keeps resident at once.
-int cgemm_max_cluster(int bn, int fmt, bool aff, int cluster) {
+// CTAs of clusters of `cluster` CTAs of the reducing kernel that the device keeps resident at once.
+int cgemm_max_cluster(int fmt, bool aff, int cluster) {
     int clusters = 0;
-    cudaError_t err = cgemm_instance(bn, fmt == PF_SPLIT, aff, [&](auto k) {
+    cudaError_t err = cgemm_instance(64, fmt == PF_SPLIT, aff, true, [&](auto k) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)cluster);
         cfg.blockDim = dim3((unsigned)decltype(k)::Cfg::kThreads);
@@ -1300,7 +1269,7 @@ int cgemm_max_cluster(int bn, int fmt, bool aff, int cluster) {
 }
 
 cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &blp, cudaStream_t s) {
-    return cgemm_instance(bn, p.fmt == PF_SPLIT, p.aff_scale != nullptr, [&](auto k) {
+    return cgemm_instance(bn, p.fmt == PF_SPLIT, p.aff_scale != nullptr, p.cluster_reduce != 0, [&](auto k) {
         void *args[] = {const_cast<CgemmParams *>(&p), const_cast<BlpArgs *>(&blp)};
         return launch_direct(reinterpret_cast<const void *>(k.kernel()), (unsigned)grid, (unsigned)decltype(k)::Cfg::kThreads,
                              decltype(k)::Cfg::kSmem, s, p.cluster_reduce ? (unsigned)p.k_splits : 1u, args);
@@ -1308,7 +1277,7 @@ cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &
 }
 
 int cgemm_threads(int bn, int fmt, bool aff) {
-    return cgemm_instance(bn, fmt == PF_SPLIT, aff, [](auto k) { return decltype(k)::Cfg::kThreads; });
+    return cgemm_instance(bn, fmt == PF_SPLIT, aff, false, [](auto k) { return decltype(k)::Cfg::kThreads; });
 }
 
 size_t cgemm_spill_floats_per_cta() { return cgemm_spill_floats(); }

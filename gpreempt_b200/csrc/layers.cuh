@@ -106,7 +106,7 @@ struct CgemmParams {
 constexpr int kCgemmMaxAffineC = 2048;  // input channels of a layer with aff_scale
 cudaError_t cgemm_prepare(int device);
 cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &blp, cudaStream_t s);
-int cgemm_max_cluster(int bn, int fmt, bool aff, int cluster);  // CTAs of clusters of this size that can be resident at once
+int cgemm_max_cluster(int fmt, bool aff, int cluster);  // CTAs of reducing clusters of this size that can be resident at once
 size_t cgemm_spill_floats_per_cta();
 int cgemm_threads(int bn, int fmt, bool aff);
 

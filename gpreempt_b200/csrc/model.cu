@@ -1279,7 +1279,7 @@ int finalize_model(gpx_model &m) {
             const char *e_cl = getenv("GPX_SPLITK_CLUSTER");
             if (!(e_cl && e_cl[0] == '0')) {
                 s_want = s_want >= 8 ? 8 : (s_want >= 4 ? 4 : (s_want >= 2 ? 2 : 1));
-                while (bn == 64 && s_want > 2 && cgemm_max_cluster(bn, m.fmt, aff, s_want) < out_tiles * s_want) s_want /= 2;
+                while (bn == 64 && s_want > 2 && cgemm_max_cluster(m.fmt, aff, s_want) < out_tiles * s_want) s_want /= 2;
             }
             if (s_want >= 2) {
                 p.kb_per_split = (all_kb + s_want - 1) / s_want;
@@ -1371,7 +1371,7 @@ int finalize_model(gpx_model &m) {
             // number of splits that divides the tile's rows, and every cluster resident at once.
             const char *e_cl = getenv("GPX_SPLITK_CLUSTER");
             const bool pow2 = p.k_splits == 2 || p.k_splits == 4 || p.k_splits == 8;
-            if (pow2 && bn == 64 && !(e_cl && e_cl[0] == '0') && cgemm_max_cluster(bn, m.fmt, aff, p.k_splits) >= kn.total_tiles &&
+            if (pow2 && bn == 64 && !(e_cl && e_cl[0] == '0') && cgemm_max_cluster(m.fmt, aff, p.k_splits) >= kn.total_tiles &&
                 kn.grid == kn.total_tiles) {
                 p.cluster_reduce = 1;
                 p.fin = q;

@@ -109,12 +109,17 @@ __device__ __forceinline__ uint32_t cluster_map_shared(uint32_t addr, uint32_t r
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
-// Bulk copy from this CTA's shared memory to `dst` in another CTA of the cluster, counted in bytes on that
-// CTA's mbarrier `bar` (both mapped by cluster_map_shared; 16-byte aligned, a multiple of 16 bytes).
-__device__ __forceinline__ void bulk_copy_to_cluster(uint32_t dst, uint32_t src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "r"(src), "r"(bytes), "r"(bar)
+// Sixteen bytes from registers to shared memory of a CTA of the cluster, counted on that CTA's mbarrier
+// (addresses mapped by cluster_map_shared).
+__device__ __forceinline__ void st_async_v4(uint32_t dst, const uint32_t *r, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "r"(r[0]),
+                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(bar)
                  : "memory");
+}
+__device__ __forceinline__ float4 lds_f4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
 }
 
 // ---- CTA pairs (cta_group::2): two CTAs of a cluster work on one tile -----------------------------
