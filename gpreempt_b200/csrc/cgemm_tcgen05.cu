@@ -215,12 +215,13 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             ctl->epi_k_done[b] = 0;
         }
         if (CL) {
-            // a row of the share this CTA finishes comes from each of the k_splits CTAs, if it is a row of the GEMM
+            // a row of the share this CTA finishes comes from each of the other CTAs, if it is a row of the GEMM,
+            // and from this CTA's own epilogue warps
             const int share = kCBM / p.k_splits;
             const int rows = p.m_rows - tile_at(blockIdx.x).m_blk * kCBM - (int)cluster_ctarank() * share;
-            mbar_init(smem_u32(&ctl->landed), 1);
-            if (rows > 0)
-                mbar_arrive_expect_tx(smem_u32(&ctl->landed), (uint32_t)((rows < share ? rows : share) * p.k_splits * BN * 4));
+            mbar_init(smem_u32(&ctl->landed), 1 + Cfg::kEpiThreads / 32);
+            if (rows > 0 && p.k_splits > 1)
+                mbar_arrive_expect_tx(smem_u32(&ctl->landed), (uint32_t)((rows < share ? rows : share) * (p.k_splits - 1) * BN * 4));
             else
                 mbar_arrive(smem_u32(&ctl->landed));
         }
@@ -753,114 +754,207 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         // owner adds the splits in order from zero, exactly as splitk_finish_kernel adds the workspace rows,
         // then bias, residual, activation, store.  What that needs besides the sums is at hand before.
         // (Staged and copied in bulk, the rows took 2 100 cycles to arrive and another 2 000 to 3 600 to
-        // be finished by eight warps; through the workspace the release in front of the barrier alone took 2 800.)
+        // be finished by eight warps; through the workspace the release in front of the barrier alone took 2 800.
+        // What travels between SMs moves at about 16 bytes a cycle, so the owner's own rows do not.)
         // Nobody leaves before its own rows are complete, and nothing else is ever stored to it.
-        const SplitKParams &fin = p.fin;
-        const int splits = p.k_splits, share = kCBM / splits, lg_share = 31 - __clz(share);
-        const int rank = (int)cluster_ctarank();
-        const int row0 = first_tile.m_blk * kCBM;
-        constexpr int kItems = kCBM / 2 * (BN / 4) / Cfg::kEpiThreads;  // four-channel items a thread finishes (two splits)
-        bool live[kItems];
-        int col[kItems];
-        uint32_t land_at[kItems];
-        size_t out_at[kItems], res_at[kItems];
-        float4 bias4[kItems];
-        uint2 r_hi[kItems], r_lo[kItems];
-        const uint32_t land = smem_base + (uint32_t)(nst * Cfg::kStageBytes);
-        const int img = fin.in_hs * fin.in_ws;
-#pragma unroll
-        for (int i = 0; i < kItems; ++i) {
-            // eight rows by four pieces a warp: sixteen-byte reads without bank conflicts, whole sectors stored
-            const int e = (int)threadIdx.x - 64 + i * Cfg::kEpiThreads;
-            const int lr = (e & 7) | (((e >> 5) & ((share >> 3) - 1)) << 3), piece = ((e >> 3) & 3) | ((e >> (2 + lg_share)) << 2);
-            const int vrow = row0 + rank * share + lr;
-            col[i] = first_tile.n_blk * BN + piece * 4;
-            land_at[i] = land + (uint32_t)(piece * share + lr) * 16;
-            live[i] = piece < BN / 4 && vrow < fin.m_rows && col[i] < fin.cout_padded;
-            if (live[i]) {
-                const int n_img = fast_div(vrow, img, p.inv_img);
-                const int r = vrow - n_img * img;
-                const int hs = fast_div(r, fin.in_ws, p.inv_in_ws);
-                const int h = hs - fin.in_off, w = r - hs * fin.in_ws - fin.in_off;
-                live[i] = h >= 0 && h < fin.out.H && w >= 0 && w < fin.out.W;
-                if (live[i]) {
-                    if (fin.bias) bias4[i] = __ldg(reinterpret_cast<const float4 *>(fin.bias + col[i]));
-                    if (fin.res_hi) res_at[i] = (size_t)layout_row(fin.res, n_img, h, w) * fin.res.C + col[i];
-                    out_at[i] = fin.out_f32 ? ((size_t)(n_img * fin.out.H + h) * fin.out.W + w) * fin.cout_valid + col[i]
-                                            : (size_t)layout_row(fin.out, n_img, h, w) * fin.out.C + col[i];
-                }
-            }
-        }
-        if (threadIdx.x == 64)
-            for (int b = 0; b < 2; ++b) mbar_arrive(smem_u32(&ctl->tmem_empty[b]));
-        cluster_wait();  // every CTA of the cluster runs
-        pdl_wait();      // the residual is the predecessor's business, everything above is not
-        if (fin.res_hi)
-#pragma unroll
-            for (int i = 0; i < kItems; ++i)
-                if (live[i]) {
-                    r_hi[i] = *reinterpret_cast<const uint2 *>(fin.res_hi + res_at[i]);
-                    if (TWO) r_lo[i] = *reinterpret_cast<const uint2 *>(fin.res_lo + res_at[i]);
-                }
+        // With one split there is nothing to exchange: a thread takes its row's columns through bias, residual
+        // and activation to memory, with everything but the sums at hand before the products end (the loop
+        // of the general epilogue takes 2 400 cycles for a tile of two planes).
         const int row = (warp & 3) * 32 + lane;
         constexpr int kCols = BN / Cfg::kEpiParts;
         const int c_lo = ((warp - 2) >> 2) * kCols;
-        if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->tmem_full[0]), 0, abort_flag, kCWaitLimitNs))) {
-            if (lane == 0) fail(301);
-        } else {
-            tc_fence_after_sync();
-            const uint32_t t_acc = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-            const uint32_t owner = (uint32_t)row >> lg_share;
-            const uint32_t bar = cluster_map_shared(smem_u32(&ctl->landed), owner);
-            const uint32_t to = cluster_map_shared(land + ((uint32_t)(rank * (BN / 4)) * share + (row & (share - 1))) * 16, owner);
+        const uint32_t t_acc = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+        auto sums = [&](int c, float *f) {  // sixteen columns of this thread's row
+            uint32_t u[16], w[16];
+            tmem_ld_32x16(t_acc + c, u);
+            if (TWO) tmem_ld_32x16(t_acc + BN + c, w);
+            tmem_ld_wait();
 #pragma unroll
-            for (int c = c_lo; c < c_lo + kCols; c += 16) {
-                uint32_t u[16], w[16];
-                tmem_ld_32x16(t_acc + c, u);
-                if (TWO) tmem_ld_32x16(t_acc + BN + c, w);
-                tmem_ld_wait();
-                if (TWO)
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) u[j] = __float_as_uint(__uint_as_float(u[j]) + __uint_as_float(w[j]));
-                if (row0 + row < p.m_rows)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) st_async_v4(to + (uint32_t)((c / 4 + j) * share) * 16, u + 4 * j, bar);
+            for (int j = 0; j < 16; ++j) f[j] = TWO ? __uint_as_float(u[j]) + __uint_as_float(w[j]) : __uint_as_float(u[j]);
+        };
+        if (threadIdx.x == 64)
+            for (int b = 0; b < 2; ++b) mbar_arrive(smem_u32(&ctl->tmem_empty[b]));
+        if (p.k_splits == 1) {
+            const int vrow = first_tile.m_blk * kCBM + row, col0 = first_tile.n_blk * BN;
+            bool live = vrow < p.m_rows;
+            size_t out_at = (size_t)vrow * p.out.C + col0, res_at = (size_t)vrow * p.res.C + col0;
+            if (!p.identity_rows) {
+                const int img = p.in_hs * p.in_ws;
+                const int n_img = fast_div(live ? vrow : 0, img, p.inv_img);
+                const int r = (live ? vrow : 0) - n_img * img;
+                const int hs = fast_div(r, p.in_ws, p.inv_in_ws);
+                const int h = hs - p.in_off, w = r - hs * p.in_ws - p.in_off;
+                live = live && h >= 0 && h < p.out.H && w >= 0 && w < p.out.W;
+                out_at = p.out_f32 ? ((size_t)(n_img * p.out.H + h) * p.out.W + w) * p.cout_valid + col0
+                                   : (size_t)layout_row(p.out, n_img, h, w) * p.out.C + col0;
+                res_at = (size_t)layout_row(p.res, n_img, h, w) * p.res.C + col0;
             }
-        }
-        volatile int never = 0;  // (a CTA that failed waits here as well, so that no store finds its memory gone)
-        if (!mbar_wait(smem_u32(&ctl->landed), 0, &never, kCWaitLimitNs + kCWaitLimitNs / 2)) fail(601);
+            constexpr int kPieces = kCols / 16;
+            const int fmt = TWO ? (int)PF_SPLIT : p.fmt, col_lim = p.cout_valid - col0;
+            float4 bias4[kPieces][4];
+            uint32_t rh[kPieces][8], rl[kPieces][TWO ? 8 : 1];
+            if (p.bias)  // (padded to whole column tiles)
 #pragma unroll
-        for (int i = 0; i < kItems; ++i) {
-            if (!live[i]) continue;
-            float f[4] = {0.f, 0.f, 0.f, 0.f};
-            const uint32_t stride = (uint32_t)(share * (BN / 4)) * 16;
-            for (int sp = 0; sp < splits; sp += 2) {
-                const float4 a = lds_f4(land_at[i] + sp * stride), b = lds_f4(land_at[i] + (sp + 1) * stride);
-                f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
-                f[0] += b.x; f[1] += b.y; f[2] += b.z; f[3] += b.w;
-            }
-            if (fin.bias) f[0] += bias4[i].x, f[1] += bias4[i].y, f[2] += bias4[i].z, f[3] += bias4[i].w;
-            if (fin.res_hi) {
-                float2 r0 = pf_unpack2(r_hi[i].x, TWO ? (int)PF_SPLIT : fin.res.fmt), r1 = pf_unpack2(r_hi[i].y, TWO ? (int)PF_SPLIT : fin.res.fmt);
-                if (TWO) {
-                    r0.x += bf16_lo_to_f32(r_lo[i].x), r0.y += bf16_hi_to_f32(r_lo[i].x);
-                    r1.x += bf16_lo_to_f32(r_lo[i].y), r1.y += bf16_hi_to_f32(r_lo[i].y);
+                for (int q = 0; q < kPieces; ++q)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) bias4[q][j] = __ldg(reinterpret_cast<const float4 *>(p.bias + col0 + c_lo + 16 * q) + j);
+            pdl_wait();  // the residual is the predecessor's business, everything above is not
+            const bool use_res = live && p.res_hi && !p.out_f32;
+            if (use_res)
+#pragma unroll
+                for (int q = 0; q < kPieces; ++q) {
+                    if (c_lo + 16 * q >= col_lim) break;
+                    ld_global_v8(p.res_hi + res_at + c_lo + 16 * q, rh[q]);
+                    if (TWO) ld_global_v8(p.res_lo + res_at + c_lo + 16 * q, rl[q]);
                 }
-                f[0] += r0.x, f[1] += r0.y, f[2] += r1.x, f[3] += r1.y;
-            }
-            apply_act_n(f, fin.relu);
-            if (fin.out_f32) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (col[i] + j < fin.cout_valid) fin.out_f32[out_at[i] + j] = f[j];
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->tmem_full[0]), 0, abort_flag, kCWaitLimitNs))) {
+                if (lane == 0) fail(301);
             } else {
-                const int fmt = TWO ? (int)PF_SPLIT : fin.out.fmt;
-                const uint32_t h0 = pf_pack2(f[0], f[1], fmt), h1 = pf_pack2(f[2], f[3], fmt);
-                *reinterpret_cast<uint2 *>(fin.out_hi + out_at[i]) = make_uint2(h0, h1);
-                if (TWO)
-                    *reinterpret_cast<uint2 *>(fin.out_lo + out_at[i]) =
-                        make_uint2(pack_bf16(f[0] - bf16_lo_to_f32(h0), f[1] - bf16_hi_to_f32(h0)),
-                                   pack_bf16(f[2] - bf16_lo_to_f32(h1), f[3] - bf16_hi_to_f32(h1)));
+                tc_fence_after_sync();
+#pragma unroll
+                for (int q = 0; q < kPieces; ++q) {
+                    const int c = c_lo + 16 * q;
+                    float f[16];
+                    sums(c, f);
+                    if (p.bias)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            f[4 * j] += bias4[q][j].x, f[4 * j + 1] += bias4[q][j].y, f[4 * j + 2] += bias4[q][j].z, f[4 * j + 3] += bias4[q][j].w;
+                    if (use_res) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const float2 r = pf_unpack2(rh[q][j], fmt);
+                            f[2 * j] += r.x, f[2 * j + 1] += r.y;
+                        }
+                        if (TWO)
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) f[2 * j] += bf16_lo_to_f32(rl[q][j]), f[2 * j + 1] += bf16_hi_to_f32(rl[q][j]);
+                    }
+                    apply_act_n(f, p.relu);
+                    if (!live || c >= col_lim) continue;
+                    if (p.out_f32) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (c + j < col_lim) p.out_f32[out_at + c + j] = f[j];
+                        continue;
+                    }
+                    uint32_t hi[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) hi[j] = pf_pack2(f[2 * j], f[2 * j + 1], fmt);
+                    st_sector(p.out_hi + out_at + c, hi);
+                    if (TWO) {
+                        uint32_t lo[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) lo[j] = pack_bf16(f[2 * j] - bf16_lo_to_f32(hi[j]), f[2 * j + 1] - bf16_hi_to_f32(hi[j]));
+                        st_sector(p.out_lo + out_at + c, lo);
+                    }
+                }
+            }
+        } else {
+            const SplitKParams &fin = p.fin;
+            const int splits = p.k_splits, share = kCBM / splits, lg_share = 31 - __clz(share);
+            const int rank = (int)cluster_ctarank();
+            const int row0 = first_tile.m_blk * kCBM;
+            constexpr int kItems = kCBM / 2 * (BN / 4) / Cfg::kEpiThreads;  // four-channel items a thread finishes (two splits)
+            bool live[kItems];
+            int col[kItems];
+            uint32_t land_at[kItems];
+            size_t out_at[kItems], res_at[kItems];
+            float4 bias4[kItems];
+            uint2 r_hi[kItems], r_lo[kItems];
+            const uint32_t land = smem_base + (uint32_t)(nst * Cfg::kStageBytes);
+            const int img = fin.in_hs * fin.in_ws;
+#pragma unroll
+            for (int i = 0; i < kItems; ++i) {
+                // eight rows by four pieces a warp: sixteen-byte reads without bank conflicts, whole sectors stored
+                const int e = (int)threadIdx.x - 64 + i * Cfg::kEpiThreads;
+                const int lr = (e & 7) | (((e >> 5) & ((share >> 3) - 1)) << 3), piece = ((e >> 3) & 3) | ((e >> (2 + lg_share)) << 2);
+                const int vrow = row0 + rank * share + lr;
+                col[i] = first_tile.n_blk * BN + piece * 4;
+                land_at[i] = land + (uint32_t)(piece * share + lr) * 16;
+                live[i] = piece < BN / 4 && vrow < fin.m_rows && col[i] < fin.cout_padded;
+                if (live[i]) {
+                    const int n_img = fast_div(vrow, img, p.inv_img);
+                    const int r = vrow - n_img * img;
+                    const int hs = fast_div(r, fin.in_ws, p.inv_in_ws);
+                    const int h = hs - fin.in_off, w = r - hs * fin.in_ws - fin.in_off;
+                    live[i] = h >= 0 && h < fin.out.H && w >= 0 && w < fin.out.W;
+                    if (live[i]) {
+                        if (fin.bias) bias4[i] = __ldg(reinterpret_cast<const float4 *>(fin.bias + col[i]));
+                        if (fin.res_hi) res_at[i] = (size_t)layout_row(fin.res, n_img, h, w) * fin.res.C + col[i];
+                        out_at[i] = fin.out_f32 ? ((size_t)(n_img * fin.out.H + h) * fin.out.W + w) * fin.cout_valid + col[i]
+                                                : (size_t)layout_row(fin.out, n_img, h, w) * fin.out.C + col[i];
+                    }
+                }
+            }
+            cluster_wait();  // every CTA of the cluster runs
+            pdl_wait();      // the residual is the predecessor's business, everything above is not
+            if (fin.res_hi)
+#pragma unroll
+                for (int i = 0; i < kItems; ++i)
+                    if (live[i]) {
+                        r_hi[i] = *reinterpret_cast<const uint2 *>(fin.res_hi + res_at[i]);
+                        if (TWO) r_lo[i] = *reinterpret_cast<const uint2 *>(fin.res_lo + res_at[i]);
+                    }
+            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->tmem_full[0]), 0, abort_flag, kCWaitLimitNs))) {
+                if (lane == 0) fail(301);
+            } else {
+                tc_fence_after_sync();
+                const int owner = row >> lg_share;
+                const uint32_t bar = cluster_map_shared(smem_u32(&ctl->landed), (uint32_t)owner);
+                const uint32_t mine = land + ((uint32_t)(rank * (BN / 4)) * share + (row & (share - 1))) * 16;
+                const uint32_t to = cluster_map_shared(mine, (uint32_t)owner);
+#pragma unroll
+                for (int c = c_lo; c < c_lo + kCols; c += 16) {
+                    float f[16];
+                    sums(c, f);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t at = (uint32_t)((c / 4 + j) * share) * 16;
+                        if (owner == rank)
+                            sts_f4(mine + at, f + 4 * j);
+                        else if (row0 + row < p.m_rows)
+                            st_async_v4(to + at, f + 4 * j, bar);
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&ctl->landed));
+            volatile int never = 0;  // (a CTA that failed waits here as well, so that no store finds its memory gone)
+            if (!mbar_wait(smem_u32(&ctl->landed), 0, &never, kCWaitLimitNs + kCWaitLimitNs / 2)) fail(601);
+#pragma unroll
+            for (int i = 0; i < kItems; ++i) {
+                if (!live[i]) continue;
+                float f[4] = {0.f, 0.f, 0.f, 0.f};
+                const uint32_t stride = (uint32_t)(share * (BN / 4)) * 16;
+                for (int sp = 0; sp < splits; sp += 2) {
+                    const float4 a = lds_f4(land_at[i] + sp * stride), b = lds_f4(land_at[i] + (sp + 1) * stride);
+                    f[0] += a.x; f[1] += a.y; f[2] += a.z; f[3] += a.w;
+                    f[0] += b.x; f[1] += b.y; f[2] += b.z; f[3] += b.w;
+                }
+                if (fin.bias) f[0] += bias4[i].x, f[1] += bias4[i].y, f[2] += bias4[i].z, f[3] += bias4[i].w;
+                if (fin.res_hi) {
+                    float2 r0 = pf_unpack2(r_hi[i].x, TWO ? (int)PF_SPLIT : fin.res.fmt), r1 = pf_unpack2(r_hi[i].y, TWO ? (int)PF_SPLIT : fin.res.fmt);
+                    if (TWO) {
+                        r0.x += bf16_lo_to_f32(r_lo[i].x), r0.y += bf16_hi_to_f32(r_lo[i].x);
+                        r1.x += bf16_lo_to_f32(r_lo[i].y), r1.y += bf16_hi_to_f32(r_lo[i].y);
+                    }
+                    f[0] += r0.x, f[1] += r0.y, f[2] += r1.x, f[3] += r1.y;
+                }
+                apply_act_n(f, fin.relu);
+                if (fin.out_f32) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (col[i] + j < fin.cout_valid) fin.out_f32[out_at[i] + j] = f[j];
+                } else {
+                    const int fmt = TWO ? (int)PF_SPLIT : fin.out.fmt;
+                    const uint32_t h0 = pf_pack2(f[0], f[1], fmt), h1 = pf_pack2(f[2], f[3], fmt);
+                    *reinterpret_cast<uint2 *>(fin.out_hi + out_at[i]) = make_uint2(h0, h1);
+                    if (TWO)
+                        *reinterpret_cast<uint2 *>(fin.out_lo + out_at[i]) =
+                            make_uint2(pack_bf16(f[0] - bf16_lo_to_f32(h0), f[1] - bf16_hi_to_f32(h0)),
+                                       pack_bf16(f[2] - bf16_lo_to_f32(h1), f[3] - bf16_hi_to_f32(h1)));
+                }
             }
         }
     } else {

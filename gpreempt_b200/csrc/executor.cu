@@ -45,6 +45,8 @@ int exec_launch(gpx_exec *e, size_t idx, cudaStream_t s) {
         // The cluster reduction has no stop / resume form: preemptible executors keep the workspace
         // and the finishing kernel.
         if (e->kind != GPX_EXEC_BASE) p.cluster_reduce = 0;
+        // The same instance serves latency-critical launches of one 64-column tile a CTA (a cluster of one).
+        if (e->kind == GPX_EXEC_BASE && k.tile == 64 && p.k_splits == 1 && k.grid == k.total_tiles) p.cluster_reduce = 1;
         err = cgemm_launch(p, k.tile, k.grid, b, s);
     } else if (k.type == KernelType::SplitK) {
         // The convolution kernel before it has already finished the tiles (cluster reduction).

@@ -111,10 +111,13 @@ __device__ __forceinline__ uint32_t cluster_map_shared(uint32_t addr, uint32_t r
 }
 // Sixteen bytes from registers to shared memory of a CTA of the cluster, counted on that CTA's mbarrier
 // (addresses mapped by cluster_map_shared).
-__device__ __forceinline__ void st_async_v4(uint32_t dst, const uint32_t *r, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "r"(r[0]),
-                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(bar)
+__device__ __forceinline__ void st_async_v4(uint32_t dst, const float *f, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "f"(f[0]),
+                 "f"(f[1]), "f"(f[2]), "f"(f[3]), "r"(bar)
                  : "memory");
+}
+__device__ __forceinline__ void sts_f4(uint32_t addr, const float *f) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]) : "memory");
 }
 __device__ __forceinline__ float4 lds_f4(uint32_t addr) {
     float4 v;
