@@ -85,6 +85,14 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
           "l"(reinterpret_cast<unsigned long long &>(c)));
     return r;
 }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, r;\n\t"
+        "mov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 r, x, y;\n\tmov.b64 {%0, %1}, r;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     float2 r;
     asm("mul.rn.f32x2 %0, %1, %2;"

@@ -246,10 +246,10 @@ struct LayerNormParams {
     int rows, H, S;
     int fmt;                                // PlaneFmt of the input and output planes
     float eps;
-    int rows_per_tile;                      // 8 or 16
+    int few_rows;                           // 1: a row is cut over several warps
     int total_tiles;
 };
-int layernorm_rows_per_tile(int rows, int sm_count);
+void layernorm_plan(LayerNormParams &p, int sm_count, int &grid, int &threads);  // fills few_rows and total_tiles
 cudaError_t layernorm_launch(const LayerNormParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
 
 // Multi-head self-attention over [B*S][ld] matrices of queries, keys and values (head h owns

@@ -883,10 +883,8 @@ int finalize_model(gpx_model &m) {
             q.H = n.C;
             q.S = n.W;
             q.eps = 1e-12f;
-            q.rows_per_tile = layernorm_rows_per_tile(q.rows, m.sm_count);
-            q.total_tiles = (q.rows + q.rows_per_tile - 1) / q.rows_per_tile;
+            layernorm_plan(q, m.sm_count, kn.grid, kn.threads);
             kn.total_tiles = q.total_tiles;
-            kn.grid = (int)std::min<long long>((long long)m.sm_count * (q.H <= 768 ? 3 : 2), q.total_tiles);
             kn.flops = 8.0 * q.rows * q.H;
             kn.bytes = 8.0 * q.rows * q.H;
             m.kernels.push_back(kn);

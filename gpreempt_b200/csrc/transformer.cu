@@ -9,6 +9,7 @@
 // preempted and resumed run is bit-identical to an uninterrupted one.
 #include "layers.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace gpx {
@@ -21,160 +22,255 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
-// One warp normalises one row of H <= 1024 channels held in registers (NV 8-channel vectors per
-// lane): mean, then the variance of the deviations, then scale and shift.
-template <int NV>
-__device__ __forceinline__ void layer_norm_row(float (&x)[NV][8], int V, int H, const float *gamma, const float *beta,
-                                               float eps, int lane) {
-    float s = 0.f;
+// Eight channels of a row as four pairs (the packed instructions halve the arithmetic of a row).
+struct Vec8 {
+    float2 v[4];
+};
+template <bool TWO>
+__device__ __forceinline__ Vec8 vec8_decode(const uint4 &a, const uint4 &b, int fmt) {
+    float x[8];
+    planes_decode8(a, b, TWO ? (int)PF_SPLIT : fmt, x);
+    return {{{x[0], x[1]}, {x[2], x[3]}, {x[4], x[5]}, {x[6], x[7]}}};
+}
+__device__ __forceinline__ Vec8 vec8_load(const float *p) {
+    const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+    return {{{a.x, a.y}, {a.z, a.w}, {b.x, b.y}, {b.z, b.w}}};
+}
+__device__ __forceinline__ Vec8 vec8_zero() { return {}; }
+__device__ __forceinline__ void vec8_add(Vec8 &a, const Vec8 &b) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i)
+    for (int j = 0; j < 4; ++j) a.v[j] = add2(a.v[j], b.v[j]);
+}
+__device__ __forceinline__ float vec8_sum(const Vec8 &a) {
+    const float2 s = add2(add2(a.v[0], a.v[1]), add2(a.v[2], a.v[3]));
+    return s.x + s.y;
+}
+// a - mean, and the sum of its squares
+__device__ __forceinline__ float vec8_centre(Vec8 &a, float mean) {
+    const float2 m = make_float2(-mean, -mean);
+    float2 s = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) s += x[i][j];  // lanes past the row hold zeros
-    const float mean = warp_sum(s) / (float)H;
-    float ss = 0.f;
+    for (int j = 0; j < 4; ++j) {
+        a.v[j] = add2(a.v[j], m);
+        s = fma2(a.v[j], a.v[j], s);
+    }
+    return s.x + s.y;
+}
+// a * rstd * gamma + beta, stored
+template <bool TWO>
+__device__ __forceinline__ void vec8_finish(const LayerNormParams &p, Vec8 &a, float rstd, const Vec8 &gamma, const Vec8 &beta, size_t off) {
+    float x[8];
 #pragma unroll
-    for (int i = 0; i < NV; ++i)
-        if (lane + 32 * i < V)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float d = x[i][j] - mean;
-                ss += d * d;
-            }
-    const float rstd = rsqrtf(warp_sum(ss) / (float)H + eps);
-#pragma unroll
-    for (int i = 0; i < NV; ++i)
-        if (lane + 32 * i < V) {
-            const float4 *g4 = reinterpret_cast<const float4 *>(gamma) + (lane + 32 * i) * 2;
-            const float4 *b4 = reinterpret_cast<const float4 *>(beta) + (lane + 32 * i) * 2;
-            const float4 g0 = __ldg(g4), g1 = __ldg(g4 + 1), b0 = __ldg(b4), b1 = __ldg(b4 + 1);
-            const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-            for (int j = 0; j < 8; ++j) x[i][j] = (x[i][j] - mean) * rstd * g[j] + b[j];
-        }
+    for (int j = 0; j < 4; ++j) {
+        const float2 y = fma2(mul2(a.v[j], make_float2(rstd, rstd)), gamma.v[j], beta.v[j]);
+        x[2 * j] = y.x, x[2 * j + 1] = y.y;
+    }
+    if (p.out_f32) {
+        float4 *o = reinterpret_cast<float4 *>(p.out_f32 + off);
+        o[0] = make_float4(x[0], x[1], x[2], x[3]);
+        o[1] = make_float4(x[4], x[5], x[6], x[7]);
+    } else {
+        planes_store8(p.out_hi, p.out_lo, off, TWO ? (int)PF_SPLIT : p.fmt, x);
+    }
 }
 
-// Rows of a [rows][H] matrix, R rows per warp, 8 R rows per tile.  Bound by HBM (the row is read and
-// written once).  The R rows of a warp are requested as raw vectors before any is converted, and
-// the next tile is claimed while they are on their way, so that neither the claim (two dependent
-// round trips to L2) nor the first load of a tile is waited for with nothing in flight; gamma and
-// beta come as 128-bit loads (one float at a time they were 48 of a lane's 54 load instructions).
-template <int NV, int R, bool TWO>
-__global__ void __launch_bounds__(kTfThreads, NV <= 3 ? 3 : 2)
+// What a lane fetches of a row before it is worked on: eight channels in planes, or of the word's embedding.
+template <bool TWO, bool EMB>
+struct RawVec {
+    uint4 a, b;
+};
+template <bool TWO, bool EMB>
+__device__ __forceinline__ void raw_fetch(const LayerNormParams &p, int row, int v, RawVec<TWO, EMB> &r) {
+    if (EMB) {
+        const uint4 *w = reinterpret_cast<const uint4 *>(p.word + (size_t)p.ids[row] * p.H + v * 8);
+        r.a = w[0], r.b = w[1];
+    } else {
+        planes_fetch8(p.in_hi, p.in_lo, (size_t)row * p.H + v * 8, TWO ? (int)PF_SPLIT : p.fmt, r.a, r.b);
+    }
+}
+// word + position (+ token type 0 where the model has that table), or the row as it is
+template <bool TWO, bool EMB>
+__device__ __forceinline__ Vec8 raw_decode(const LayerNormParams &p, int row, int v, const RawVec<TWO, EMB> &r) {
+    if (!EMB) return vec8_decode<TWO>(r.a, r.b, p.fmt);
+    auto f = [](unsigned u) { return __uint_as_float(u); };
+    Vec8 x = {{{f(r.a.x), f(r.a.y)}, {f(r.a.z), f(r.a.w)}, {f(r.b.x), f(r.b.y)}, {f(r.b.z), f(r.b.w)}}};
+    vec8_add(x, vec8_load(p.pos + (size_t)(row % p.S) * p.H + v * 8));
+    if (p.type) vec8_add(x, vec8_load(p.type + v * 8));
+    return x;
+}
+
+// Many rows: one row a warp (NV 8-channel vectors a lane), eight rows a tile.  Bound by memory in principle
+// (a row is read and written once); what it waits for in practice is latency, so the next tile's rows are on
+// their way while this tile's are worked on, the claim after that is in flight beside them, gamma and
+// beta lie in shared memory, and the arithmetic is packed.  16 384 rows of 768 bf16: 18.9 us with a claim and a
+// load per tile and scalar arithmetic, LN_BIG_US like this.
+template <int NV, bool TWO, bool EMB>
+__global__ void __launch_bounds__(kTfThreads, NV <= 3 && !TWO && !EMB ? 4 : 2)
 layernorm_kernel(const __grid_constant__ LayerNormParams p, BlpArgs blp) {
+    __shared__ __align__(16) float s_gamma[256 * NV], s_beta[256 * NV];
+    __shared__ int s_tile[2];
+    // (parameters: no kernel writes them, so they are fetched while the predecessor drains)
+    for (int i = threadIdx.x; i < p.H / 4; i += kTfThreads) {
+        reinterpret_cast<float4 *>(s_gamma)[i] = __ldg(reinterpret_cast<const float4 *>(p.gamma) + i);
+        reinterpret_cast<float4 *>(s_beta)[i] = __ldg(reinterpret_cast<const float4 *>(p.beta) + i);
+    }
     pdl_enter();
-    __shared__ int s_tile;
     const bool dynamic = blp.preempted != nullptr;
     if (threadIdx.x == 0) trace_begin(blp);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int V = p.H / 8;
-    int iter = 0;
-    int tile;
+    int iter = 0, tile, next;
     if (dynamic) {
-        if (threadIdx.x == 0) s_tile = blp_claim(blp, 0);
-        __syncthreads();
-        tile = s_tile;
-    } else {
-        tile = blp_claim(blp, 0);
-    }
-    while (tile >= 0) {
-        const int row0 = (tile * (kTfThreads / 32) + wid) * R;
-        uint4 ra[R][NV], rb[TWO ? R : 1][TWO ? NV : 1];
-        if (!p.ids) {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-#pragma unroll
-                for (int i = 0; i < NV; ++i)
-                    if (row0 + r < p.rows && lane + 32 * i < V)
-                        planes_fetch8(p.in_hi, p.in_lo, (size_t)(row0 + r) * p.H + (lane + 32 * i) * 8, TWO ? PF_SPLIT : p.fmt,
-                                      ra[r][i], rb[TWO ? r : 0][TWO ? i : 0]);
+        if (threadIdx.x == 0) {
+            const int first = blp_claim(blp, 0);
+            s_tile[0] = first;
+            s_tile[1] = first >= 0 ? blp_claim(blp, 1) : -1;
         }
-        int next = -1;
-        if (!dynamic || threadIdx.x == 0) next = blp_claim(blp, iter + 1);
+        __syncthreads();
+        tile = s_tile[0], next = s_tile[1];
+    } else {
+        __syncthreads();
+        tile = blp_claim(blp, 0), next = blp_claim(blp, 1);
+    }
+    RawVec<TWO, EMB> now[NV], ahead[NV];
+    auto fetch = [&](int t, RawVec<TWO, EMB> (&raw)[NV]) {
+        const int row = t * (kTfThreads / 32) + wid;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int row = row0 + r;
-            if (row >= p.rows) break;
-            float x[NV][8];
+        for (int i = 0; i < NV; ++i)
+            if (t >= 0 && row < p.rows && lane + 32 * i < V) raw_fetch<TWO, EMB>(p, row, lane + 32 * i, raw[i]);
+    };
+    fetch(tile, now);
+    while (tile >= 0) {
+        fetch(next, ahead);
+        int after = -1;
+        if (next >= 0 && (!dynamic || threadIdx.x == 0)) after = blp_claim(blp, iter + 2);
+        const int row = tile * (kTfThreads / 32) + wid;
+        if (row < p.rows) {
+            Vec8 x[NV];
+            float s = 0.f;
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
-                const int v = lane + 32 * i;
-                if (v >= V) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) x[i][j] = 0.f;
-                } else if (p.ids) {
-                    // embedding row: word + position (+ token type 0 where the model has that table)
-                    const long long id = p.ids[row];
-                    const int pos = row % p.S;
-                    const float4 *w = reinterpret_cast<const float4 *>(p.word + (size_t)id * p.H + v * 8);
-                    const float4 *q = reinterpret_cast<const float4 *>(p.pos + (size_t)pos * p.H + v * 8);
-                    float4 a0 = w[0], a1 = w[1], b0 = q[0], b1 = q[1];
-                    float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0;
-                    if (p.type) {
-                        const float4 *t = reinterpret_cast<const float4 *>(p.type + v * 8);
-                        c0 = t[0];
-                        c1 = t[1];
-                    }
-                    x[i][0] = a0.x + b0.x + c0.x;
-                    x[i][1] = a0.y + b0.y + c0.y;
-                    x[i][2] = a0.z + b0.z + c0.z;
-                    x[i][3] = a0.w + b0.w + c0.w;
-                    x[i][4] = a1.x + b1.x + c1.x;
-                    x[i][5] = a1.y + b1.y + c1.y;
-                    x[i][6] = a1.z + b1.z + c1.z;
-                    x[i][7] = a1.w + b1.w + c1.w;
-                } else {
-                    planes_decode8(ra[r][i], rb[TWO ? r : 0][TWO ? i : 0], TWO ? PF_SPLIT : p.fmt, x[i]);
-                }
+                x[i] = lane + 32 * i < V ? raw_decode<TWO, EMB>(p, row, lane + 32 * i, now[i]) : vec8_zero();
+                s += vec8_sum(x[i]);
             }
-            layer_norm_row<NV>(x, V, p.H, p.gamma, p.beta, p.eps, lane);
+            const float mean = warp_sum(s) / (float)p.H;
+            float ss = 0.f;
+#pragma unroll
+            for (int i = 0; i < NV; ++i)
+                if (lane + 32 * i < V) ss += vec8_centre(x[i], mean);
+            const float rstd = rsqrtf(warp_sum(ss) / (float)p.H + p.eps);
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
                 const int v = lane + 32 * i;
-                if (v < V) {
-                    const size_t off = (size_t)row * p.H + v * 8;
-                    if (p.out_f32) {
-                        float4 *o = reinterpret_cast<float4 *>(p.out_f32 + off);
-                        o[0] = make_float4(x[i][0], x[i][1], x[i][2], x[i][3]);
-                        o[1] = make_float4(x[i][4], x[i][5], x[i][6], x[i][7]);
-                    } else {
-                        planes_store8(p.out_hi, p.out_lo, off, TWO ? PF_SPLIT : p.fmt, x[i]);
-                    }
-                }
+                if (v < V) vec8_finish<TWO>(p, x[i], rstd, vec8_load(s_gamma + v * 8), vec8_load(s_beta + v * 8), (size_t)row * p.H + v * 8);
             }
         }
         ++iter;
-        if (dynamic) {
-            __syncthreads();  // everyone has read the tile number of this round
-            if (threadIdx.x == 0) s_tile = next;
+        if (dynamic && next >= 0) {  // (next is the same for the whole CTA)
+            if (threadIdx.x == 0) s_tile[iter & 1] = after;
             __syncthreads();
-            tile = s_tile;
-        } else {
-            tile = next;
+            after = s_tile[iter & 1];
         }
+        tile = next, next = after;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) now[i] = ahead[i];
     }
     if (threadIdx.x == 0) trace_end(blp, iter);
 }
 
-int layernorm_rows_per_tile(int rows, int sm_count) {
-    // Two rows a warp once that still leaves every SM a few tiles (16 384 rows of 768: 37 us with one).
-    return rows >= 16 * 4 * sm_count ? 16 : 8;
+// Few rows (a latency-critical request): a row is a chain of loads, sums and roundings, so it is cut over NV
+// warps with one vector a lane, and its scale and shift are in registers before the predecessor ends.
+// 128 rows of 768 fp16: 3.3 us with a warp to a row, LN_SMALL_US like this.
+template <int NV>
+constexpr int ln_few_rows() { return NV == 1 ? 8 : (NV == 2 ? 4 : 2); }
+template <int NV, bool TWO, bool EMB>
+__global__ void __launch_bounds__(32 * NV * ln_few_rows<NV>())
+layernorm_few_kernel(const __grid_constant__ LayerNormParams p, BlpArgs blp) {
+    constexpr int kRows = ln_few_rows<NV>();
+    __shared__ float s_sum[kRows * NV], s_sq[kRows * NV];
+    __shared__ int s_tile;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int V = p.H / 8;
+    const int r = wid / NV, v = (wid - r * NV) * 32 + lane;
+    Vec8 gamma = vec8_zero(), beta = vec8_zero();
+    if (v < V) gamma = vec8_load(p.gamma + v * 8), beta = vec8_load(p.beta + v * 8);
+    pdl_enter();
+    const bool dynamic = blp.preempted != nullptr;
+    if (threadIdx.x == 0) trace_begin(blp);
+    auto row_sum = [&](float s, float *part) {
+        s = warp_sum(s);
+        if (NV == 1) return s;
+        if (lane == 0) part[wid] = s;
+        __syncthreads();
+        float all = part[r * NV];
+#pragma unroll
+        for (int i = 1; i < NV; ++i) all += part[r * NV + i];
+        return all;
+    };
+    int iter = 0;
+    for (;; ++iter) {
+        int tile;
+        if (dynamic) {
+            if (threadIdx.x == 0) s_tile = blp_claim(blp, iter);
+            __syncthreads();
+            tile = s_tile;
+        } else {
+            tile = blp_claim(blp, iter);
+        }
+        if (tile < 0) break;
+        const int row = tile * kRows + r;
+        const bool live = row < p.rows && v < V;
+        Vec8 x = vec8_zero();
+        if (live) {
+            RawVec<TWO, EMB> raw;
+            raw_fetch<TWO, EMB>(p, row, v, raw);
+            x = raw_decode<TWO, EMB>(p, row, v, raw);
+        }
+        const float mean = row_sum(vec8_sum(x), s_sum) / (float)p.H;
+        float ss = 0.f;
+        if (live) ss = vec8_centre(x, mean);
+        const float rstd = rsqrtf(row_sum(ss, s_sq) / (float)p.H + p.eps);
+        if (live) vec8_finish<TWO>(p, x, rstd, gamma, beta, (size_t)row * p.H + v * 8);
+        if (dynamic) __syncthreads();  // s_tile
+    }
+    if (threadIdx.x == 0) trace_end(blp, iter);
+}
+
+static int layernorm_vectors(int H) { return (H + 255) / 256; }
+
+// The instance for a width, format and kind of input, as f(kernel, threads).
+template <typename F>
+static auto layernorm_instance(const LayerNormParams &p, F &&f) {
+    auto width = [&](auto two, auto emb) {
+        constexpr bool T = decltype(two)::value, E = decltype(emb)::value;
+        const bool few = p.few_rows != 0;
+        switch (layernorm_vectors(p.H)) {
+            case 1: return few ? f(layernorm_few_kernel<1, T, E>, 32 * ln_few_rows<1>()) : f(layernorm_kernel<1, T, E>, kTfThreads);
+            case 2: return few ? f(layernorm_few_kernel<2, T, E>, 64 * ln_few_rows<2>()) : f(layernorm_kernel<2, T, E>, kTfThreads);
+            case 3: return few ? f(layernorm_few_kernel<3, T, E>, 96 * ln_few_rows<3>()) : f(layernorm_kernel<3, T, E>, kTfThreads);
+            default: return few ? f(layernorm_few_kernel<4, T, E>, 128 * ln_few_rows<4>()) : f(layernorm_kernel<4, T, E>, kTfThreads);
+        }
+    };
+    if (p.ids) return p.fmt == PF_SPLIT ? width(std::true_type(), std::true_type()) : width(std::false_type(), std::true_type());
+    return p.fmt == PF_SPLIT ? width(std::true_type(), std::false_type()) : width(std::false_type(), std::false_type());
+}
+
+// A row over several warps up to eight rows an SM: beyond that one row a warp has as many warps at work.
+void layernorm_plan(LayerNormParams &p, int sm_count, int &grid, int &threads) {
+    p.few_rows = p.rows <= 8 * sm_count;
+    const int nv = layernorm_vectors(p.H);
+    const int rows = !p.few_rows ? kTfThreads / 32 : (nv == 1 ? ln_few_rows<1>() : (nv == 2 ? ln_few_rows<2>() : ln_few_rows<3>()));
+    p.total_tiles = (p.rows + rows - 1) / rows;
+    int per_sm = 1;
+    threads = layernorm_instance(p, [&](auto kernel, int t) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, t, 0);
+        return t;
+    });
+    grid = (int)std::min<long long>((long long)sm_count * std::max(per_sm, 1), p.total_tiles);
 }
 
 cudaError_t layernorm_launch(const LayerNormParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    const int nv = p.H <= 256 ? 1 : (p.H <= 768 ? 3 : 4);
-    const bool pair = p.rows_per_tile == 16;
-    auto go = [&](auto kernel) { return launch_layer(kernel, grid, kTfThreads, 0, s, p, blp); };
-    auto pick = [&](auto two) {
-        constexpr bool T = decltype(two)::value;
-        if (nv == 1)
-            return go(pair ? layernorm_kernel<1, 2, T> : layernorm_kernel<1, 1, T>);
-        if (nv == 3)
-            return go(pair ? layernorm_kernel<3, 2, T> : layernorm_kernel<3, 1, T>);
-        return go(pair ? layernorm_kernel<4, 2, T> : layernorm_kernel<4, 1, T>);
-    };
-    return p.fmt == PF_SPLIT ? pick(std::true_type()) : pick(std::false_type());
+    return layernorm_instance(p, [&](auto kernel, int threads) { return launch_layer(kernel, grid, threads, 0, s, p, blp); });
 }
 
 // ---- multi-head attention ---------------------------------------------------------------------
