@@ -993,26 +993,51 @@ __device__ __forceinline__ PixelAt pixel_at(unsigned e, int C8, int Wo, int Ho) 
 }
 
 // Depthwise convolution: one thread-iteration produces eight channels of one output pixel,
-// taps walked in (fh, fw) order with one FFMA each, so the result is independent of the tiling.
-// At batch 1 this is latency: the filter (never written by a kernel) is copied to shared memory ahead
-// of the wait for the predecessor, the element a thread starts with is decoded there too, and the nine
-// taps of a 3x3 filter are requested before any is used (one round trip instead of nine;
-// MobileNetV2 b1: 4.4 us a layer before).
+// taps walked in (fh, fw) order with one FMA each, so the result is independent of the tiling.  Channels that only
+// pad the stored width are left as the zeros they are (MobileNetV2's first layers: 32 of 64, 96 of 128, 144 of 192).
+// At batch 1 this is latency: ahead of the wait for the predecessor the filter (never written by a kernel) is
+// copied to shared memory, and for the element a thread starts with the addresses, the taps inside the image
+// and the bias are found; behind it the nine taps of a 3x3 filter are requested before any is used
+// (MobileNetV2 b1, us a layer: 4.4 a tap at a time, 3.3 to 4.9 with nine in flight and addresses behind the wait,
+// 2.5 to 3.7 like this).
 //
-// BATCH: taps of a 3x3 filter in flight at once.  Nine where the tensor is a tile or two per CTA; three
-// (a filter row) in larger tensors, which want the occupancy the registers of nine take
-// (56x56x144, 64 images fp16: 190 us with nine, 145 with three); 0 for other filter sizes.
+// BATCH: taps of a 3x3 filter in flight at once, where the tensor is a tile or two per CTA and the filter has
+// nine; 0: a tap at a time (other filter sizes, strides and row orders).
+struct DwElem {
+    long long in;    // element offset of tap (0, 0) in a plain input (it may lie outside)
+    size_t out;      // element offset of the output
+    int c0;
+    unsigned taps;   // of a 3x3 filter: inside the image
+};
+__device__ __forceinline__ DwElem dw_elem(const DwConvParams &p, unsigned e, int C8) {
+    const PixelAt at = pixel_at(e, C8, p.out.W, p.out.H);
+    DwElem a;
+    a.c0 = at.c8 * 8;
+    const int h0 = at.ho * p.stride - p.pad, w0 = at.wo * p.stride - p.pad;
+    a.in = ((long long)(at.n * p.in.l.Hs + h0) * p.in.l.Ws + w0) * p.in.l.C + a.c0;
+    a.out = (size_t)layout_row(p.out, at.n, at.ho, at.wo) * p.out.C + a.c0;
+    unsigned rows = 0, cols = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        rows |= (unsigned)(h0 + i) < (unsigned)p.in.l.H ? 7u << (3 * i) : 0u;
+        cols |= (unsigned)(w0 + i) < (unsigned)p.in.l.W ? 0x49u << i : 0u;
+    }
+    a.taps = rows & cols;
+    return a;
+}
+
 template <int BATCH, bool TWO>
-__global__ void __launch_bounds__(kPoolThreads, BATCH == 9 ? (TWO ? 2 : 3) : 4)
+__global__ void __launch_bounds__(kPoolThreads, 2)
 dwconv_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
     extern __shared__ float s_w[];  // [k * k][C], or nothing where it does not fit
     __shared__ int s_tile;
     const bool dynamic = blp.preempted != nullptr;
     const int C = p.out.C;
-    const int C8 = C / 8;
-    const int Ho = p.out.H, Wo = p.out.W;
+    const int C8 = p.channels / 8;
     const int H = p.in.l.H, W = p.in.l.W;
-    const unsigned total = (unsigned)p.out.N * Ho * Wo * C8;  // < 2^31, checked when the model is built
+    const bool plain = p.in.l.order == ACT_PLAIN;
+    const long long row_step = (long long)p.in.l.Ws * p.in.l.C;
+    const unsigned total = (unsigned)p.out.N * p.out.H * p.out.W * C8;  // < 2^31, checked when the model is built
     const float *wts = p.w;
     if (p.w_in_smem) {
         const int n4 = p.k * p.k * C / 4;
@@ -1020,8 +1045,16 @@ dwconv_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
             reinterpret_cast<float4 *>(s_w)[i] = __ldg(reinterpret_cast<const float4 *>(p.w) + i);
         wts = s_w;
     }
-    unsigned known = (unsigned)blockIdx.x * p.tile_elems + threadIdx.x;  // decoded ahead for a static schedule
-    PixelAt ahead = pixel_at(known < total ? known : 0, C8, Wo, Ho);
+    unsigned known = (unsigned)blockIdx.x * p.tile_elems + threadIdx.x;  // found ahead for a static schedule
+    if (dynamic || known >= total) known = ~0u;
+    const DwElem ahead = dw_elem(p, known == ~0u ? 0 : known, C8);
+    float4 bias_a = make_float4(0.f, 0.f, 0.f, 0.f), bias_b = bias_a;
+    auto fetch_bias = [&](int c0) {
+        if (!p.bias) return;
+        bias_a = __ldg(reinterpret_cast<const float4 *>(p.bias + c0));
+        bias_b = __ldg(reinterpret_cast<const float4 *>(p.bias + c0) + 1);
+    };
+    if (BATCH == 9) fetch_bias(ahead.c0);
     __syncthreads();
     pdl_enter();
     if (threadIdx.x == 0) trace_begin(blp);
@@ -1030,17 +1063,17 @@ dwconv_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
         const unsigned begin = (unsigned)tile * p.tile_elems;
         const unsigned end = begin + p.tile_elems < total ? begin + p.tile_elems : total;
         for (unsigned e = begin + threadIdx.x; e < end; e += kPoolThreads) {
-            const PixelAt at = e == known ? ahead : pixel_at(e, C8, Wo, Ho);
-            const int c0 = at.c8 * 8, h0 = at.ho * p.stride - p.pad, w0 = at.wo * p.stride - p.pad;
-            float acc[8];
+            const DwElem at = e == known ? ahead : dw_elem(p, e, C8);
+            float2 acc[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+            for (int j = 0; j < 4; ++j) acc[j] = make_float2(0.f, 0.f);
             auto tap = [&](const float (&x)[8], int t) {
-                const float4 *wv = reinterpret_cast<const float4 *>(wts + (size_t)t * C + c0);
+                const float4 *wv = reinterpret_cast<const float4 *>(wts + (size_t)t * C + at.c0);
                 const float4 a = wv[0], b = wv[1];
-                const float wf[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[j] = fmaf(x[j], wf[j], acc[j]);
+                acc[0] = fma2(make_float2(x[0], x[1]), make_float2(a.x, a.y), acc[0]);
+                acc[1] = fma2(make_float2(x[2], x[3]), make_float2(a.z, a.w), acc[1]);
+                acc[2] = fma2(make_float2(x[4], x[5]), make_float2(b.x, b.y), acc[2]);
+                acc[3] = fma2(make_float2(x[6], x[7]), make_float2(b.z, b.w), acc[3]);
             };
             if (BATCH != 0) {
                 constexpr int B = BATCH ? BATCH : 1;
@@ -1048,45 +1081,153 @@ dwconv_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
 #pragma unroll
                 for (int t0 = 0; t0 < 9; t0 += B) {
                     uint4 ra[B], rb[TWO ? B : 1];
-                    bool ok[B];
+                    if (plain) {
 #pragma unroll
-                    for (int t = 0; t < B; ++t) {
-                        const int hi = h0 + (t0 + t) / 3, wi = w0 + (t0 + t) % 3;
-                        ok[t] = hi >= 0 && hi < H && wi >= 0 && wi < W;
-                        if (ok[t])
-                            planes_fetch8(p.in.hi, p.in.lo, (size_t)layout_row(p.in.l, at.n, hi, wi) * p.in.l.C + c0, fmt, ra[t],
-                                          rb[TWO ? t : 0]);
+                        for (int t = 0; t < B; ++t)
+                            if (at.taps >> (t0 + t) & 1)
+                                planes_fetch8(p.in.hi, p.in.lo, (size_t)(at.in + (t0 + t) / 3 * row_step + (t0 + t) % 3 * p.in.l.C), fmt, ra[t],
+                                              rb[TWO ? t : 0]);
+                    } else {
+                        const PixelAt px = pixel_at(e, C8, p.out.W, p.out.H);
+#pragma unroll
+                        for (int t = 0; t < B; ++t)
+                            if (at.taps >> (t0 + t) & 1)
+                                planes_fetch8(p.in.hi, p.in.lo,
+                                              (size_t)layout_row(p.in.l, px.n, px.ho * p.stride - p.pad + (t0 + t) / 3,
+                                                                 px.wo * p.stride - p.pad + (t0 + t) % 3) * p.in.l.C + at.c0,
+                                              fmt, ra[t], rb[TWO ? t : 0]);
                     }
                     if (t0 == 0) claims.ahead();
+                    if (t0 == 0 && !(BATCH == 9 && e == known)) fetch_bias(at.c0);
 #pragma unroll
                     for (int t = 0; t < B; ++t) {
-                        if (!ok[t]) continue;
+                        if (!(at.taps >> (t0 + t) & 1)) continue;
                         float x[8];
                         planes_decode8(ra[t], rb[TWO ? t : 0], fmt, x);
                         tap(x, t0 + t);
                     }
                 }
             } else {
+                fetch_bias(at.c0);
+                const PixelAt px = pixel_at(e, C8, p.out.W, p.out.H);
                 for (int fh = 0; fh < p.k; ++fh) {
-                    const int hi = h0 + fh;
+                    const int hi = px.ho * p.stride - p.pad + fh;
                     if (hi < 0 || hi >= H) continue;
                     for (int fw = 0; fw < p.k; ++fw) {
-                        const int wi = w0 + fw;
+                        const int wi = px.wo * p.stride - p.pad + fw;
                         if (wi < 0 || wi >= W) continue;
                         float x[8];
-                        planes_load8(p.in.hi, p.in.lo, (size_t)layout_row(p.in.l, at.n, hi, wi) * p.in.l.C + c0, p.in.l.fmt, x);
+                        planes_load8(p.in.hi, p.in.lo, (size_t)layout_row(p.in.l, px.n, hi, wi) * p.in.l.C + at.c0, p.in.l.fmt, x);
                         tap(x, fh * p.k + fw);
                     }
                 }
             }
+            float f[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) f[2 * j] = acc[j].x, f[2 * j + 1] = acc[j].y;
             if (p.bias) {
-                const float4 *b4 = reinterpret_cast<const float4 *>(p.bias + c0);
-                const float4 a = __ldg(b4), b = __ldg(b4 + 1);
-                acc[0] += a.x, acc[1] += a.y, acc[2] += a.z, acc[3] += a.w;
-                acc[4] += b.x, acc[5] += b.y, acc[6] += b.z, acc[7] += b.w;
+                f[0] += bias_a.x, f[1] += bias_a.y, f[2] += bias_a.z, f[3] += bias_a.w;
+                f[4] += bias_b.x, f[5] += bias_b.y, f[6] += bias_b.z, f[7] += bias_b.w;
             }
-            apply_act_n(acc, p.act);
-            planes_store8(p.out_hi, p.out_lo, (size_t)layout_row(p.out, at.n, at.ho, at.wo) * C + c0, p.out.fmt, acc);
+            apply_act_n(f, p.act);
+            planes_store8(p.out_hi, p.out_lo, at.out, TWO ? (int)PF_SPLIT : p.out.fmt, f);
+        }
+    }
+    if (threadIdx.x == 0) trace_end(blp, claims.done());
+}
+
+// The 3x3 filter over a large tensor in plain rows: a thread produces eight channels of four neighbouring output
+// pixels, so that a vector of the input is fetched and unpacked 1.5 times (2.25 at stride 2) instead of
+// nine, and a tap's filter values are read once for four pixels.  Bound by instruction issue: 56x56x144, 64 images
+// fp16, 142 us a pixel at a time over the padded width of 192, 122 over 144, 71 in strips
+// (its bytes alone: 18); all of MobileNetV2 b64 fp16 1 302 -> 1 013.  The order of an output's taps is that of the other form, so its bits are too.
+constexpr int dw_strip(int stride, bool two) { return stride == 2 && two ? 2 : 4; }  // (nine columns of two planes spill)
+template <int STRIDE, bool TWO>
+__global__ void __launch_bounds__(kPoolThreads, 2)
+dwconv_strip_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
+    extern __shared__ float s_w[];
+    __shared__ int s_tile;
+    constexpr int kDwStrip = dw_strip(STRIDE, TWO), kCols = (kDwStrip - 1) * STRIDE + 3;
+    const bool dynamic = blp.preempted != nullptr;
+    const int C = p.out.C, C8 = p.channels / 8;
+    const int H = p.in.l.H, W = p.in.l.W, strips = (p.out.W + kDwStrip - 1) / kDwStrip;
+    const unsigned total = (unsigned)p.out.N * p.out.H * strips * C8;
+    const float *wts = p.w;
+    if (p.w_in_smem) {
+        const int n4 = 9 * C / 4;
+        for (int i = threadIdx.x; i < n4; i += kPoolThreads)
+            reinterpret_cast<float4 *>(s_w)[i] = __ldg(reinterpret_cast<const float4 *>(p.w) + i);
+        wts = s_w;
+    }
+    __syncthreads();
+    pdl_enter();
+    if (threadIdx.x == 0) trace_begin(blp);
+    TileClaims claims(blp, dynamic, s_tile);
+    const int fmt = TWO ? (int)PF_SPLIT : p.in.l.fmt;
+    for (int tile = claims.first(); tile >= 0; tile = claims.next()) {
+        const unsigned begin = (unsigned)tile * p.tile_elems;
+        const unsigned end = begin + p.tile_elems < total ? begin + p.tile_elems : total;
+        for (unsigned e = begin + threadIdx.x; e < end; e += kPoolThreads) {
+            const PixelAt at = pixel_at(e, C8, strips, p.out.H);
+            const int c0 = at.c8 * 8, wo0 = at.wo * kDwStrip;
+            const int h0 = at.ho * STRIDE - p.pad, w0 = wo0 * STRIDE - p.pad;
+            float2 acc[kDwStrip][4];
+#pragma unroll
+            for (int o = 0; o < kDwStrip; ++o)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[o][j] = make_float2(0.f, 0.f);
+#pragma unroll 1
+            for (int fh = 0; fh < 3; ++fh) {
+                if ((unsigned)(h0 + fh) >= (unsigned)H) continue;
+                const long long row = ((long long)(at.n * H + h0 + fh) * W + w0) * p.in.l.C + c0;
+                uint4 ra[kCols], rb[TWO ? kCols : 1];
+#pragma unroll
+                for (int c = 0; c < kCols; ++c)
+                    if ((unsigned)(w0 + c) < (unsigned)W)
+                        planes_fetch8(p.in.hi, p.in.lo, (size_t)(row + (long long)c * p.in.l.C), fmt, ra[c], rb[TWO ? c : 0]);
+                if (fh == 1) claims.ahead();
+                float2 wt[3][4];
+#pragma unroll
+                for (int fw = 0; fw < 3; ++fw) {
+                    const float4 *wv = reinterpret_cast<const float4 *>(wts + (size_t)(fh * 3 + fw) * C + c0);
+                    const float4 a = wv[0], b = wv[1];
+                    wt[fw][0] = make_float2(a.x, a.y), wt[fw][1] = make_float2(a.z, a.w);
+                    wt[fw][2] = make_float2(b.x, b.y), wt[fw][3] = make_float2(b.z, b.w);
+                }
+#pragma unroll
+                for (int c = 0; c < kCols; ++c) {
+                    if ((unsigned)(w0 + c) >= (unsigned)W) continue;
+                    float x[8];
+                    planes_decode8(ra[c], rb[TWO ? c : 0], fmt, x);
+#pragma unroll
+                    for (int o = 0; o < kDwStrip; ++o) {
+                        const int fw = c - o * STRIDE;
+                        if (fw < 0 || fw > 2) continue;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) acc[o][j] = fma2(make_float2(x[2 * j], x[2 * j + 1]), wt[fw][j], acc[o][j]);
+                    }
+                }
+            }
+            float4 bias_a = make_float4(0.f, 0.f, 0.f, 0.f), bias_b = bias_a;
+            if (p.bias) {
+                bias_a = __ldg(reinterpret_cast<const float4 *>(p.bias + c0));
+                bias_b = __ldg(reinterpret_cast<const float4 *>(p.bias + c0) + 1);
+            }
+            const size_t out = (size_t)layout_row(p.out, at.n, at.ho, wo0) * C + c0;
+#pragma unroll
+            for (int o = 0; o < kDwStrip; ++o) {
+                if (wo0 + o >= p.out.W) break;
+                float f[8];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) f[2 * j] = acc[o][j].x, f[2 * j + 1] = acc[o][j].y;
+                if (p.bias) {
+                    f[0] += bias_a.x, f[1] += bias_a.y, f[2] += bias_a.z, f[3] += bias_a.w;
+                    f[4] += bias_b.x, f[5] += bias_b.y, f[6] += bias_b.z, f[7] += bias_b.w;
+                }
+                apply_act_n(f, p.act);
+                const size_t off = p.out.order == ACT_PHASED ? (size_t)layout_row(p.out, at.n, at.ho, wo0 + o) * C + c0 : out + (size_t)o * C;
+                planes_store8(p.out_hi, p.out_lo, off, TWO ? (int)PF_SPLIT : p.out.fmt, f);
+            }
         }
     }
     if (threadIdx.x == 0) trace_end(blp, claims.done());
@@ -1094,13 +1235,24 @@ dwconv_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
 
 static auto dwconv_instance(const DwConvParams &p) {
     const bool two = p.out.fmt == PF_SPLIT;
+    if (p.strip) {
+        if (p.stride == 1) return two ? dwconv_strip_kernel<1, true> : dwconv_strip_kernel<1, false>;
+        return two ? dwconv_strip_kernel<2, true> : dwconv_strip_kernel<2, false>;
+    }
     if (p.k != 3) return two ? dwconv_kernel<0, true> : dwconv_kernel<0, false>;
-    if (p.small) return two ? dwconv_kernel<9, true> : dwconv_kernel<9, false>;
-    return two ? dwconv_kernel<3, true> : dwconv_kernel<3, false>;
+    return two ? dwconv_kernel<9, true> : dwconv_kernel<9, false>;
 }
 static size_t dwconv_smem(const DwConvParams &p) { return p.w_in_smem ? (size_t)p.k * p.k * p.out.C * sizeof(float) : 0; }
 
-int dwconv_grid(const DwConvParams &p, int sm_count) {
+// Tiles, form and grid of a layer whose shapes, filter and stride are set.  Strips of four pixels where the tensor
+// has more than four tiles of 256 vectors an SM; below that a thread per pixel has more threads at work.
+int dwconv_plan(DwConvParams &p, int sm_count) {
+    const long long pixels = (long long)p.out.N * p.out.H * p.out.W, c8 = p.channels / 8;
+    p.strip = p.k == 3 && p.in.l.order == ACT_PLAIN && (p.stride == 1 || p.stride == 2) && pixels * c8 > 4LL * 256 * sm_count;
+    const int len = dw_strip(p.stride, p.out.fmt == PF_SPLIT);
+    const long long total = p.strip ? (long long)p.out.N * p.out.H * ((p.out.W + len - 1) / len) * c8 : pixels * c8;
+    p.tile_elems = 256;
+    p.total_tiles = (int)((total + p.tile_elems - 1) / p.tile_elems);
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dwconv_instance(p), kPoolThreads, dwconv_smem(p));
     return (int)std::min<long long>((long long)sm_count * std::max(per_sm, 1), p.total_tiles);

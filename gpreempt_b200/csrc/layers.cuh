@@ -261,6 +261,7 @@ struct AttnParams {
     int ld, ld_out;         // row strides of q, k, v (columns of one wider matrix) and of the output
     int fmt;                // PlaneFmt of all four matrices
     float scale;
+    int few_keys;           // CUDA-core path: 1: a warp to a query (at most 64 tokens)
     int total_tiles;
     // Tensor-core path (single-plane formats, attention_tcgen05.cu): TMA maps of Q ([B*S][64 heads],
     // boxes of 128 rows x 64 columns), K and V (boxes of 64 x 64), and the error word.
@@ -270,6 +271,7 @@ struct AttnParams {
     // tile it gave up when the word went up inside it.
     CgemmSlot *slots;
 };
+void attention_plan(AttnParams &p, int sm_count, int &threads);  // of the CUDA-core kernels: few_keys, total_tiles
 cudaError_t attention_launch(const AttnParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
 cudaError_t attention_tc_prepare();
 cudaError_t attention_tc_launch(const AttnParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
@@ -284,12 +286,13 @@ struct DwConvParams {
     bf16_bits *out_hi, *out_lo;
     ActLayout out;
     int k, stride, pad, act;
-    int small;           // 1: at most a tile or two per CTA: latency, not occupancy
+    int strip;           // 1: a thread produces four pixels of a row
     int w_in_smem;       // 1: the filter is copied to shared memory once per CTA
     int total_tiles;
-    int tile_elems;      // output 8-channel vectors per tile
+    int tile_elems;      // output 8-channel vectors (of a strip) per tile
+    int channels;        // computed (a multiple of eight); what the stored width has beyond them stays zero
 };
-int dwconv_grid(const DwConvParams &p, int sm_count);
+int dwconv_plan(DwConvParams &p, int sm_count);  // fills strip, tile_elems and total_tiles; returns the grid
 cudaError_t dwconv_launch(const DwConvParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
 
 enum ConvTile { CONV_TILE_128 = 0, CONV_TILE_64 = 1, CONV_TILE_32 = 2 };

@@ -895,7 +895,6 @@ int finalize_model(gpx_model &m) {
             kn.name = n.name;
             kn.node = (int)ni;
             kn.type = KernelType::Attention;
-            kn.threads = 128;
             AttnParams &q = kn.attn;
             const Storage &sq = m.storages[m.nodes[n.inputs[0]].storage];
             const Storage &sk = m.storages[m.nodes[n.inputs[1]].storage];
@@ -937,7 +936,7 @@ int finalize_model(gpx_model &m) {
                 m.kernels.push_back(kn);
                 continue;
             }
-            q.total_tiles = n.N * n.heads * ((n.W + 31) / 32);
+            attention_plan(q, m.sm_count, kn.threads);
             kn.total_tiles = q.total_tiles;
             kn.grid = (int)std::min<long long>((long long)m.sm_count * 4, q.total_tiles);
             m.kernels.push_back(kn);
@@ -966,12 +965,9 @@ int finalize_model(gpx_model &m) {
             // batches) its latency hides behind the predecessor's tail; beside the kernel's own variables
             // in the default 48 KB.
             q.w_in_smem = (size_t)n.k * n.k * q.out.C * sizeof(float) + 256 <= 48 * 1024 ? 1 : 0;
-            long long total = (long long)n.N * n.H * n.W * (q.out.C / 8);
-            q.tile_elems = (int)std::max<long long>(256, std::min<long long>(kMaxTileVectors, total / (8LL * m.sm_count) / 32 * 32));
-            q.total_tiles = (int)((total + q.tile_elems - 1) / q.tile_elems);
+            q.channels = (n.C + 7) / 8 * 8;
+            kn.grid = dwconv_plan(q, m.sm_count);
             kn.total_tiles = q.total_tiles;
-            q.small = q.total_tiles <= 4 * m.sm_count ? 1 : 0;
-            kn.grid = dwconv_grid(q, m.sm_count);
             kn.flops = 2.0 * n.N * n.H * n.W * (double)n.k * n.k * n.C;
             kn.bytes = 4.0 * ((double)src.N * src.H * src.W * src.C + (double)n.N * n.H * n.W * n.C);
             m.kernels.push_back(kn);

@@ -103,9 +103,9 @@ __device__ __forceinline__ Vec8 raw_decode(const LayerNormParams &p, int row, in
 // (a row is read and written once); what it waits for in practice is latency, so the next tile's rows are on
 // their way while this tile's are worked on, the claim after that is in flight beside them, gamma and
 // beta lie in shared memory, and the arithmetic is packed.  16 384 rows of 768 bf16: 18.9 us with a claim and a
-// load per tile and scalar arithmetic, LN_BIG_US like this.
+// load per tile and scalar arithmetic, 14.7 like this.
 template <int NV, bool TWO, bool EMB>
-__global__ void __launch_bounds__(kTfThreads, NV <= 3 && !TWO && !EMB ? 4 : 2)
+__global__ void __launch_bounds__(kTfThreads, NV <= 3 && !EMB ? 3 : 2)
 layernorm_kernel(const __grid_constant__ LayerNormParams p, BlpArgs blp) {
     __shared__ __align__(16) float s_gamma[256 * NV], s_beta[256 * NV];
     __shared__ int s_tile[2];
@@ -180,7 +180,7 @@ layernorm_kernel(const __grid_constant__ LayerNormParams p, BlpArgs blp) {
 
 // Few rows (a latency-critical request): a row is a chain of loads, sums and roundings, so it is cut over NV
 // warps with one vector a lane, and its scale and shift are in registers before the predecessor ends.
-// 128 rows of 768 fp16: 3.3 us with a warp to a row, LN_SMALL_US like this.
+// 128 rows of 768 fp16: 3.3 us with a warp to a row, 1.2 like this.
 template <int NV>
 constexpr int ln_few_rows() { return NV == 1 ? 8 : (NV == 2 ? 4 : 2); }
 template <int NV, bool TWO, bool EMB>
@@ -255,9 +255,11 @@ static auto layernorm_instance(const LayerNormParams &p, F &&f) {
     return p.fmt == PF_SPLIT ? width(std::true_type(), std::false_type()) : width(std::false_type(), std::false_type());
 }
 
-// A row over several warps up to eight rows an SM: beyond that one row a warp has as many warps at work.
+// A row over several warps up to 32 rows an SM: with fewer the chain is what counts, with more the loads under
+// way are.  One warp a row against several, 768 channels: 2 048 rows bf16 4.3 / 4.0 us, 4 096 rows 6.5 / 5.7 and
+// float32 8.4 / 6.6, 16 384 rows 14.7 / 16.7.
 void layernorm_plan(LayerNormParams &p, int sm_count, int &grid, int &threads) {
-    p.few_rows = p.rows <= 8 * sm_count;
+    p.few_rows = p.rows <= 32 * sm_count;
     const int nv = layernorm_vectors(p.H);
     const int rows = !p.few_rows ? kTfThreads / 32 : (nv == 1 ? ln_few_rows<1>() : (nv == 2 ? ln_few_rows<2>() : ln_few_rows<3>()));
     p.total_tiles = (p.rows + rows - 1) / rows;
@@ -408,7 +410,123 @@ attention_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
     if (tid == 0) trace_end(blp, iter);
 }
 
+// The same for sequences of at most 64 tokens, where a request is a chain of latencies: eight queries of a head per
+// tile, a warp to a query.  Keys and values are staged once, a lane scores the keys `lane` and `lane` + 32, the
+// softmax is two warp reductions, and for the weighted sum a lane owns two of the 64 channels.
+// Six tokens, 12 heads: 5.7 us with four lanes to a query walking the keys one by one, 2.0 like this.
+constexpr int kShortKeys = 64, kShortQueries = 8;
+__global__ void __launch_bounds__(32 * kShortQueries)
+attention_short_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
+    __shared__ int s_tile;
+    __shared__ __align__(16) float s_k[kShortKeys][kAttnLd], s_v[kShortKeys][kAttnDh], s_q[kShortQueries][kAttnDh];
+    pdl_enter();
+    const bool dynamic = blp.preempted != nullptr;
+    if (threadIdx.x == 0) trace_begin(blp);
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int qblocks = (p.S + kShortQueries - 1) / kShortQueries;
+    const int vecs = p.S * (kAttnDh / 8);  // of the keys, and of the values
+    constexpr int kLoads = kShortKeys * (kAttnDh / 8) / (32 * kShortQueries);
+    int iter = 0;
+    for (;; ++iter) {
+        int tile;
+        if (dynamic) {
+            if (tid == 0) s_tile = blp_claim(blp, iter);
+            __syncthreads();
+            tile = s_tile;
+        } else {
+            tile = blp_claim(blp, iter);
+        }
+        if (tile < 0) break;
+        const int qb = tile % qblocks;
+        const int head = (tile / qblocks) % p.heads;
+        const int b = tile / (qblocks * p.heads);
+        const int qrow = qb * kShortQueries + wid;
+        const size_t col = (size_t)head * kAttnDh, row0 = (size_t)b * p.S;
+        // every load of the tile is requested before any is converted
+        uint4 kh[kLoads], kl[kLoads], vh[kLoads], vl[kLoads];
+        unsigned qh = 0, ql = 0;
+        const size_t q_at = (row0 + (qrow < p.S ? qrow : 0)) * p.ld + col + 2 * lane;
+        qh = *reinterpret_cast<const unsigned *>(p.q_hi + q_at);
+        if (p.fmt == PF_SPLIT) ql = *reinterpret_cast<const unsigned *>(p.q_lo + q_at);
+#pragma unroll
+        for (int i = 0; i < kLoads; ++i) {
+            const int e = tid + i * 32 * kShortQueries;
+            if (e < vecs) {
+                const size_t off = (row0 + e / (kAttnDh / 8)) * p.ld + col + e % (kAttnDh / 8) * 8;
+                planes_fetch8(p.k_hi, p.k_lo, off, p.fmt, kh[i], kl[i]);
+                planes_fetch8(p.v_hi, p.v_lo, off, p.fmt, vh[i], vl[i]);
+            }
+        }
+        float2 q2 = pf_unpack2(qh, p.fmt);
+        if (p.fmt == PF_SPLIT) q2.x += __uint_as_float(ql << 16), q2.y += __uint_as_float(ql & 0xffff0000u);
+        *reinterpret_cast<float2 *>(&s_q[wid][2 * lane]) = make_float2(q2.x * p.scale, q2.y * p.scale);
+#pragma unroll
+        for (int i = 0; i < kLoads; ++i) {
+            const int e = tid + i * 32 * kShortQueries;
+            if (e < vecs) {
+                const int kr = e / (kAttnDh / 8), c = e % (kAttnDh / 8) * 8;
+                float x[8];
+                planes_decode8(kh[i], kl[i], p.fmt, x);
+                *reinterpret_cast<float4 *>(&s_k[kr][c]) = make_float4(x[0], x[1], x[2], x[3]);
+                *reinterpret_cast<float4 *>(&s_k[kr][c + 4]) = make_float4(x[4], x[5], x[6], x[7]);
+                planes_decode8(vh[i], vl[i], p.fmt, x);
+                *reinterpret_cast<float4 *>(&s_v[kr][c]) = make_float4(x[0], x[1], x[2], x[3]);
+                *reinterpret_cast<float4 *>(&s_v[kr][c + 4]) = make_float4(x[4], x[5], x[6], x[7]);
+            }
+        }
+        __syncthreads();
+        if (qrow < p.S) {
+            float sc[2];
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int key = lane + 32 * half;
+                sc[half] = -INFINITY;
+                if (key >= p.S) continue;
+                float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int d = 0; d < kAttnDh; d += 4) {
+                    const float4 kv = *reinterpret_cast<const float4 *>(&s_k[key][d]);
+                    const float4 qv = *reinterpret_cast<const float4 *>(&s_q[wid][d]);
+                    a.x = fmaf(qv.x, kv.x, a.x), a.y = fmaf(qv.y, kv.y, a.y);
+                    a.z = fmaf(qv.z, kv.z, a.z), a.w = fmaf(qv.w, kv.w, a.w);
+                }
+                sc[half] = (a.x + a.y) + (a.z + a.w);
+            }
+            float m = fmaxf(sc[0], sc[1]);
+#pragma unroll
+            for (int sh = 16; sh >= 1; sh >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, sh));
+            const float w0 = __expf(sc[0] - m), w1 = __expf(sc[1] - m);  // (0 for keys past the sequence)
+            const float inv = 1.0f / warp_sum(w0 + w1);
+            float2 o = make_float2(0.f, 0.f);
+            for (int j = 0; j < p.S; ++j) {
+                const float w = __shfl_sync(0xffffffffu, j < 32 ? w0 : w1, j & 31);
+                o = fma2(make_float2(w, w), *reinterpret_cast<const float2 *>(&s_v[j][2 * lane]), o);
+            }
+            o.x *= inv, o.y *= inv;
+            const size_t off = (row0 + qrow) * p.ld_out + col + 2 * lane;
+            const unsigned hi = pf_pack2(o.x, o.y, p.fmt);
+            *reinterpret_cast<unsigned *>(p.out_hi + off) = hi;
+            if (p.fmt == PF_SPLIT)
+                *reinterpret_cast<unsigned *>(p.out_lo + off) =
+                    pf_pack2(o.x - __uint_as_float(hi << 16), o.y - __uint_as_float(hi & 0xffff0000u), PF_SPLIT);
+        }
+        __syncthreads();  // the staging area and the tile number are rewritten
+    }
+    if (tid == 0) trace_end(blp, iter);
+}
+
+// Tiles, form and threads of a launch.  The short form wherever it applies, except for many sequences of more
+// than 48 tokens, whose keys it stages four times as often (12 heads, us a layer, walking the keys / short: 32
+// sequences of 6 tokens 12.3 / 4.0, 32 of 33 36 / 25, 1 of 40 11.6 / 3.4, 48 of 64 71 / 79).
+void attention_plan(AttnParams &p, int sm_count, int &threads) {
+    const int short_tiles = p.B * p.heads * ((p.S + kShortQueries - 1) / kShortQueries);
+    p.few_keys = p.S <= 48 || (p.S <= kShortKeys && short_tiles <= 8 * sm_count);
+    p.total_tiles = p.few_keys ? short_tiles : p.B * p.heads * ((p.S + 31) / 32);
+    threads = p.few_keys ? 32 * kShortQueries : kAttnThreads;
+}
+
 cudaError_t attention_launch(const AttnParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
+    if (p.few_keys) return launch_layer(attention_short_kernel, grid, 32 * kShortQueries, 0, s, p, blp);
     return launch_layer(attention_kernel, grid, kAttnThreads, 0, s, p, blp);
 }
 
