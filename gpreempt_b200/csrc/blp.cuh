@@ -69,12 +69,13 @@ __device__ __forceinline__ void trace_end(const BlpArgs &b, int tiles_run) {
 // Called by ONE thread of the CTA.  Returns the claimed tile index, or -1 when the CTA must
 // return (word raised, or no tiles left).  `iter` counts tiles this CTA has run so far and
 // drives the static schedule.
-__device__ __forceinline__ int blp_claim(const BlpArgs &b, int iter) {
+// (word: what a kernel has read of the preempt word already, after its predecessor ended.)
+__device__ __forceinline__ int blp_claim(const BlpArgs &b, int iter, int word) {
     if (b.preempted == nullptr) {
         long long t = (long long)blockIdx.x + (long long)iter * gridDim.x;
         return t < b.total_tiles ? (int)t : -1;
     }
-    if (load_word(b.preempted) != 0) {
+    if (word != 0) {
         if (b.trace) atomicMin(b.trace + 2, globaltimer_ns());
         // Only a kernel with unclaimed tiles left is a stop point; a kernel whose cursor has
         // already passed the end has nothing to resume.
@@ -84,6 +85,9 @@ __device__ __forceinline__ int blp_claim(const BlpArgs &b, int iter) {
     }
     int idx = atomicAdd(b.executed, 1);
     return idx < b.total_tiles ? idx : -1;
+}
+__device__ __forceinline__ int blp_claim(const BlpArgs &b, int iter) {
+    return blp_claim(b, iter, b.preempted ? load_word(b.preempted) : 0);
 }
 
 #if defined(__CUDACC__)

@@ -206,9 +206,13 @@ __device__ __forceinline__ void pagerank_pair(const GraphWlParams &p, unsigned v
 // vertex are ~16 ids apart, so the 32 reads of one instruction touch ~16 lines of L1, one a cycle, and
 // 10 M edges are 43 k cycles an SM where the 41 MB of ids are 6 us from L2.  Here the window of deltas a
 // tile can reach is copied to shared memory once (12 KB for 64 vertices of a band of 1 500) and gathered
-// there (~3.5 conflicting banks an access); ids are half as wide and a lane gets eight of them with
-// one load.  Every lane adds the same edges in the same order as in pagerank_vertex and the same tree
-// adds the lanes, so both forms give the same bits.  52 804 vertices, 10.2 M edges: 1431 -> 681 us a run.
+// there; ids are byte offsets of half the width, a lane gets eight of them with one load, and the edges of a
+// vertex are dealt to lanes and rounds so that a round's reads fall into as many banks as they can
+// (deal_edges: 1.6 reads of the fullest bank a round instead of 3.5 in list order).  What is left is a chain
+// of round trips to L2, so they overlap: window and first ids are under way together, the next ids
+// under each gather, and the sums of four vertices go through one tree of exchanges.  52 804 vertices,
+// 10.2 M edges: 1 431 us a run over the lists, 700 packed in list order with a load, a claim and a sum at a
+// time, 555 like this (the search, with its one tile a CTA, 674 -> 560).
 template <int K>
 struct IdPack;
 template <> struct IdPack<8> { typedef uint4 type; };
@@ -221,10 +225,22 @@ __device__ __forceinline__ float gather_pack(const typename IdPack<K>::type &q, 
     const unsigned short *id = reinterpret_cast<const unsigned short *>(&q);
     float d[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) d[k] = win[id[k]];
+    for (int k = 0; k < K; ++k) d[k] = *reinterpret_cast<const float *>(reinterpret_cast<const char *>(win) + id[k]);
 #pragma unroll
     for (int k = 0; k < K; ++k) s += d[k];
     return s;
+}
+
+// The sums of s[0..3] over the warp by the tree of warp_sum, four at once: lanes 16 apart exchange two of the
+// four, lanes 8 apart one of the two left.  Vertex t's sum ends in lanes 16 (t & 1) + 8 (t >> 1) .. + 7.
+__device__ __forceinline__ float warp_sum4(const float (&s)[4], int lane) {
+    const bool hi16 = lane & 16, hi8 = lane & 8;
+    float a = (hi16 ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, hi16 ? s[0] : s[1], 16);
+    const float b = (hi16 ? s[3] : s[2]) + __shfl_xor_sync(0xffffffffu, hi16 ? s[2] : s[3], 16);
+    a = (hi8 ? b : a) + __shfl_xor_sync(0xffffffffu, hi8 ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
 }
 
 template <int K>
@@ -238,39 +254,53 @@ __device__ __forceinline__ void pagerank_packed_tile(const GraphWlParams &p, int
     const int per_warp = p.tile_verts / (kGwThreads / 32);
     const unsigned v = (unsigned)tile * p.tile_verts + wid * per_warp + lane;  // the vertex this lane updates
     const bool mine = lane < per_warp && v < p.n;
+    const uint2 w = p.win[tile];  // first id, a multiple of 32, and floats to copy, a multiple of four
     unsigned b = 0, e = 0;
     if (mine) {
         b = p.blk[v];
         e = p.blk[v + 1];
     }
-    const uint2 w = p.win[tile];
-    for (unsigned i = threadIdx.x; i < w.y; i += kGwThreads) win[i] = dold[w.x + i];
+    const uint32_t win_at = (uint32_t)__cvta_generic_to_shared(win);
+    for (unsigned i = threadIdx.x * 4; i < w.y; i += kGwThreads * 4)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(win_at + i * 4), "l"(dold + w.x + i) : "memory");
     if (threadIdx.x == 0) win[w.y] = 0.f;
+    // the first blocks of vertices j and j + 1 of this warp (a missing list has no blocks)
+    auto first_blocks = [&](int j, Pack &q0, Pack &q1, unsigned &b0, unsigned &e0, unsigned &b1, unsigned &e1) {
+        b0 = __shfl_sync(0xffffffffu, b, j & 31), e0 = __shfl_sync(0xffffffffu, e, j & 31);
+        b1 = __shfl_sync(0xffffffffu, b, (j + 1) & 31), e1 = __shfl_sync(0xffffffffu, e, (j + 1) & 31);
+        if (b0 < e0) q0 = packed[(size_t)b0 * 32];
+        if (b1 < e1) q1 = packed[(size_t)b1 * 32];
+    };
+    Pack q0{}, q1{};
+    unsigned b0, e0, b1, e1;
+    first_blocks(0, q0, q1, b0, e0, b1, e1);
     float left = 0.f, val = 0.f, deg = 1.f;
     if (mine) {
         left = residual[v];
         val = value[v];
         deg = (float)p.outdeg[v];
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     float sum = 0.f;
 #pragma unroll 1
-    for (int j = 0; j < per_warp; j += 2) {  // two lists at a time (a missing one has no blocks)
-        const unsigned b0 = __shfl_sync(0xffffffffu, b, j), e0 = __shfl_sync(0xffffffffu, e, j);
-        const unsigned b1 = __shfl_sync(0xffffffffu, b, j + 1), e1 = __shfl_sync(0xffffffffu, e, j + 1);
-        float s0 = 0.f, s1 = 0.f;
-        unsigned i0 = b0, i1 = b1;
-        while (i0 < e0 && i1 < e1) {
-            const Pack q0 = packed[(size_t)i0++ * 32], q1 = packed[(size_t)i1++ * 32];
-            s0 = gather_pack<K>(q0, win, s0);
-            s1 = gather_pack<K>(q1, win, s1);
+    for (int j = 0; j < per_warp; j += 4) {
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int h = 0; h < 4; h += 2) {
+            Pack n0{}, n1{};
+            unsigned nb0 = 0, ne0 = 0, nb1 = 0, ne1 = 0;
+            if (j + h + 2 < per_warp) first_blocks(j + h + 2, n0, n1, nb0, ne0, nb1, ne1);
+            if (b0 < e0) s[h] = gather_pack<K>(q0, win, s[h]);
+            if (b1 < e1) s[h + 1] = gather_pack<K>(q1, win, s[h + 1]);
+            for (unsigned i = b0 + 1; i < e0; ++i) s[h] = gather_pack<K>(packed[(size_t)i * 32], win, s[h]);
+            for (unsigned i = b1 + 1; i < e1; ++i) s[h + 1] = gather_pack<K>(packed[(size_t)i * 32], win, s[h + 1]);
+            q0 = n0, q1 = n1, b0 = nb0, e0 = ne0, b1 = nb1, e1 = ne1;
         }
-        for (; i0 < e0; ++i0) s0 = gather_pack<K>(packed[(size_t)i0 * 32], win, s0);
-        for (; i1 < e1; ++i1) s1 = gather_pack<K>(packed[(size_t)i1 * 32], win, s1);
-        s0 = warp_sum(s0);
-        s1 = warp_sum(s1);
-        if (lane == j) sum = s0;
-        if (lane == j + 1) sum = s1;
+        const float all = warp_sum4(s, lane);
+        const int t = (lane - j) & 3;
+        const float got = __shfl_sync(0xffffffffu, all, 16 * (t & 1) + 8 * (t >> 1));
+        if (lane >= j && lane < j + 4) sum = got;
     }
     if (mine) {
         const float r = left + sum;
@@ -387,12 +417,15 @@ __device__ __forceinline__ void init_tile(const GraphWlParams &p, int tile) {
 // PACK: PageRank's packed form (ids per lane and block), 0 = edge lists.  Six CTAs of the packed form on an SM hide
 // one another's barriers and copies.
 template <int ALGO, int PHASE, int PACK = 0>
-__global__ void __launch_bounds__(kGwThreads, PACK ? 6 : 1)
+__global__ void __launch_bounds__(kGwThreads, PACK || (PHASE == GW_EDGES && (ALGO == GW_BFS || ALGO == GW_CC)) ? 6 : 1)
 graphwl_kernel(const __grid_constant__ GraphWlParams p, BlpArgs blp) {
     pdl_enter();
     extern __shared__ float s_win[];
     __shared__ int s_tile;
     const bool dynamic = blp.preempted != nullptr;
+    // (asked for together with the flag: the claim below would otherwise wait for one after the other)
+    int word = 0;
+    if (PHASE != GW_INIT && dynamic && threadIdx.x == 0) word = load_word(blp.preempted);
     if (PHASE != GW_INIT && p.active[p.iter] == 0) {
         // No flag for this iteration.  With the preempt word down that is final: every kernel before
         // this one ran to its end (the word stays up from the moment a kernel stops until the stream
@@ -401,7 +434,7 @@ graphwl_kernel(const __grid_constant__ GraphWlParams p, BlpArgs blp) {
         // the kernel then goes on to the claim below, which records it as a stop point, and it is
         // judged again when the run is resumed.
         if (dynamic) {
-            if (threadIdx.x == 0) s_tile = load_word(blp.preempted);
+            if (threadIdx.x == 0) s_tile = word;
             __syncthreads();
         }
         if (!dynamic || s_tile == 0) {
@@ -425,7 +458,7 @@ graphwl_kernel(const __grid_constant__ GraphWlParams p, BlpArgs blp) {
     for (;;) {
         int tile;
         if (dynamic) {
-            if (threadIdx.x == 0) s_tile = blp_claim(blp, iter);
+            if (threadIdx.x == 0) s_tile = PHASE != GW_INIT && iter == 0 ? blp_claim(blp, iter, word) : blp_claim(blp, iter);
             __syncthreads();
             tile = s_tile;
         } else {
@@ -441,6 +474,8 @@ graphwl_kernel(const __grid_constant__ GraphWlParams p, BlpArgs blp) {
         }
         if (PHASE == GW_VERTICES) found |= vertex_tile<ALGO>(p, tile);
         ++iter;
+        // With a CTA for every tile each runs one: asking for another would be two round trips to L2 more.
+        if (blp.total_tiles <= (int)gridDim.x) break;
         if (dynamic) __syncthreads();
     }
     if (PHASE == GW_VERTICES) {
@@ -452,7 +487,7 @@ graphwl_kernel(const __grid_constant__ GraphWlParams p, BlpArgs blp) {
 typedef void (*GraphKernel)(const GraphWlParams, BlpArgs);
 
 size_t window_bytes(const GraphWlParams &p) {
-    return p.phase == GW_EDGES && p.pack ? (size_t)(p.win_max + 1) * sizeof(float) : 0;
+    return p.phase == GW_EDGES && p.pack ? (size_t)(p.win_max + 4) * sizeof(float) : 0;
 }
 
 GraphKernel pick_kernel(const GraphWlParams &p) {
@@ -559,6 +594,40 @@ int packed_tile_verts(uint64_t n, int sm_count) {
     return n >= 32ull * 2 * sm_count ? 32 : 0;
 }
 
+// Deals the `deg` ids of a vertex to `rows` rounds of 32 lanes, row by row: at[32 r + l] is the id lane l gathers in
+// round r, or kGwInfinity.  The banks of the window are ids modulo 32.  A round takes each bank's share of
+// what is left over the rounds that are left, from the fullest banks first, so that the reads of the fullest bank, added
+// up over the rounds, come near the least there can be.
+void deal_edges(const unsigned *ids, uint64_t deg, uint64_t rows, std::vector<unsigned> &sorted, std::vector<unsigned> &at) {
+    uint64_t start[33] = {0}, end[32];  // of a bank's ids not dealt yet, in `sorted`
+    for (uint64_t i = 0; i < deg; ++i) ++start[(ids[i] & 31) + 1];
+    for (int b = 0; b < 32; ++b) start[b + 1] += start[b];
+    for (int b = 0; b < 32; ++b) end[b] = start[b];
+    sorted.resize(deg);
+    for (uint64_t i = 0; i < deg; ++i) sorted[end[ids[i] & 31]++] = ids[i];
+    at.assign(rows * 32, kGwInfinity);
+    uint64_t left = deg;
+    unsigned char order[32];
+    for (int i = 0; i < 32; ++i) order[i] = (unsigned char)i;
+    for (uint64_t r = 0; r < rows && left; ++r) {
+        for (int i = 1; i < 32; ++i) {  // (nearly in order from the round before)
+            const unsigned char x = order[i];
+            int k = i;
+            for (; k > 0 && end[order[k - 1]] - start[order[k - 1]] < end[x] - start[x]; --k) order[k] = order[k - 1];
+            order[k] = x;
+        }
+        const uint64_t rows_left = rows - r, later = 32 * (rows_left - 1);  // what the rounds after this one can take
+        uint64_t take = (end[order[0]] - start[order[0]] + rows_left - 1) / rows_left, n = 0;
+        do {
+            for (int i = 0; i < 32 && n < 32; ++i) {
+                const int b = order[i];
+                for (uint64_t k = 0; k < take && start[b] < end[b] && n < 32; ++k, ++n, --left) at[r * 32 + n] = sorted[start[b]++];
+            }
+            take = 1;
+        } while (left > later);
+    }
+}
+
 // PageRank's packed in-edge lists (GraphWlParams::packed), false if the lists are the better form:
 //  - every tile of `tile_verts` vertices has to read ids that lie within one window of kGwWindowMax;
 //  - the gathers have to be worth the copies: at least three for every four deltas copied (band of 1 500, degree
@@ -582,8 +651,10 @@ bool pack_lists(const std::vector<unsigned long long> &trow, const std::vector<u
             }
         const unsigned len = lo == kGwInfinity ? 0 : hi - lo + 1;
         if (len > (unsigned)kGwWindowMax) return false;
-        win[t] = make_uint2(len ? lo : 0, len);
-        win_max = std::max(win_max, (int)len);
+        // (copied from a multiple of 32, so that an id's bank is the same in every window, in whole 16 bytes)
+        const unsigned from = len ? lo & ~31u : 0u;
+        win[t] = make_uint2(from, len ? (hi - from + 4) / 4 * 4 : 0u);
+        win_max = std::max(win_max, (int)win[t].y);
         copies += len;
     }
     if (4 * (uint64_t)tadj.size() < 3 * copies) return false;
@@ -605,19 +676,21 @@ bool pack_lists(const std::vector<unsigned long long> &trow, const std::vector<u
     if (most * n > 4 * warp_verts * std::max<uint64_t>(blocks, n)) return false;
     packed.resize(blocks * per);
     auto fill = [&](uint64_t t0, uint64_t t1) {
+        std::vector<unsigned> sorted, at;
         for (uint64_t v = t0 * tile_verts; v < std::min<uint64_t>(n, t1 * tile_verts); ++v) {
             const uint2 w = win[v / tile_verts];
-            const uint64_t deg = trow[v + 1] - trow[v];
-            for (uint64_t b = blk[v]; b < blk[v + 1]; ++b)
+            const uint64_t blocks_v = blk[v + 1] - blk[v];
+            deal_edges(tadj.data() + trow[v], trow[v + 1] - trow[v], blocks_v * pack, sorted, at);
+            for (uint64_t b = 0; b < blocks_v; ++b)
                 for (unsigned l = 0; l < 32; ++l)
                     for (int k = 0; k < pack; ++k) {
-                        const uint64_t i = (b - blk[v]) * per + (uint64_t)k * 32 + l;
-                        packed[(b * 32 + l) * pack + k] = (uint16_t)(i < deg ? tadj[trow[v] + i] - w.x : w.y);
+                        const unsigned id = at[(b * pack + k) * 32 + l];
+                        packed[((blk[v] + b) * 32 + l) * pack + k] = (uint16_t)(4 * (id == kGwInfinity ? w.y : id - w.x));
                     }
         }
     };
     std::vector<std::thread> pool;
-    const uint64_t workers = std::min<uint64_t>(8, std::max<uint64_t>(1, tiles / 64));
+    const uint64_t workers = std::min<uint64_t>(std::max(8u, std::min(32u, std::thread::hardware_concurrency())), std::max<uint64_t>(1, tiles / 64));
     pool.reserve(workers);
     for (uint64_t i = 0; i < workers; ++i) {
         const uint64_t t0 = tiles * i / workers, t1 = tiles * (i + 1) / workers;
@@ -791,8 +864,8 @@ int build_graph_workload(gpx_model &m, const std::string &name, const gpx_model_
     GPX_TRY(add_result(m, result[algo], algo == GW_PAGERANK ? "float32" : "uint32", g.n, &base.a));
     if (algo != GW_BFS) GPX_TRY(device_zeroed(m, g.n, &base.b));
     if (algo == GW_PAGERANK) {
-        GPX_TRY(device_zeroed(m, g.n, &base.d0));
-        GPX_TRY(device_zeroed(m, g.n, &base.d1));
+        GPX_TRY(device_zeroed(m, g.n + 4, &base.d0));  // (windows are copied in whole 16 bytes)
+        GPX_TRY(device_zeroed(m, g.n + 4, &base.d1));
     }
     if (algo == GW_SSSP) GPX_TRY(device_zeroed(m, g.n, &base.f0));
     GPX_TRY(device_zeroed(m, (size_t)kGwMaxIters + 1, &base.active));

@@ -40,8 +40,10 @@ constexpr int kGwThreads = 256;
 constexpr int kGwEdgeTileVertsMax = 256;  // vertices per tile of an edge pass at most (32 per warp)
 constexpr int kGwVertexTileVerts = 1024;  // vertices per tile of a per-vertex pass
 constexpr int kGwMaxIters = 16384;        // iteration flags a graph workload has: no run may need more rounds
-// floats of a tile's window: with the zero behind it and the kernel's own variables in the default 48 KiB
+// ids of a tile's window: started at a multiple of 32 and rounded up, with the zero behind it and the kernel's own
+// variables, its copy fits the default 48 KiB
 constexpr int kGwWindowMax = (48 * 1024 - 256) / 4 - 1;
+static_assert((kGwWindowMax + 31 + 3 + 4) * 4 + 64 <= 48 * 1024, "window too long");
 constexpr unsigned kGwInfinity = 0xFFFFFFFFu;  // MYINFINITY, include/workloads/graphcompute.h:14
 
 struct GraphWlParams {
@@ -60,15 +62,15 @@ struct GraphWlParams {
     unsigned *d0, *d1;    // pagerank: delta, read from d<iter & 1>, written to the other
     unsigned char *f0;    // sssp: label (the frontier)
     int *active;          // [kGwMaxIters + 1]: active[i] != 0 <=> iteration i has work
-    // pagerank, for graphs ordered for locality (pack_lists): the ids as 16-bit offsets into the window of ids
-    // the tile can reach, at most kGwWindowMax long, in blocks of 32 x pack (lane l of a
-    // block holds edges l, l + 32, ... next to one another), padded with the window's length, where the
-    // shared-memory copy of the window holds a zero.
+    // pagerank, for graphs ordered for locality (pack_lists): the ids as 16-bit byte offsets into the copy of the
+    // window of deltas the tile can reach, at most kGwWindowMax ids long, in blocks of 32 x pack (a lane's
+    // ids of a block next to one another, in the order deal_edges gives them), padded with the offset
+    // behind the window, where the shared-memory copy holds a zero.
     int pack;                       // ids a lane holds per block: 1, 2, 4 or 8; 0 = lists in adj
     const uint16_t *packed;
     const unsigned *blk;            // [n + 1] first block of every vertex
-    const uint2 *win;               // [tiles] first id and length of the window
-    int win_max;                    // longest window
+    const uint2 *win;               // [tiles] first id (a multiple of 32) and deltas to copy (of four)
+    int win_max;                    // longest copy
     float alpha, tol;     // pagerank (0.85, 0.001: include/workloads/graphcompute.h:85-86)
 };
 
