@@ -62,7 +62,9 @@ __device__ __forceinline__ Grid grid_of(const StencilParams &p) {
 // fall to nothing within cells) may miss by one or two in the last place.  A horizontal tile that reads an
 // infinity, a NaN, a value of 1e15 or a density beyond half the hydrostatic one divides; along z
 // div_by_any keeps infinities, and a density of zero, of which either way makes NaN, needs no care.
-// 3200 x 1600, a time step: 1 727 us with divisions and pow, 958 like this.
+// 3200 x 1600, a time step: 1 727 us with divisions and pow, 958 like this; 777 with four cells a lane along x (451 ->
+// 310 instructions a cell, loads a tile ahead: 84 -> 64 us a kernel) and steps unrolled along z with all of an
+// SM's memory as cache (73 -> 64).
 template <bool DIVIDE>
 __device__ __forceinline__ float quotient(float a, float b, float y) { return DIVIDE ? __fdiv_rn(a, b) : div_by(a, b, y); }
 template <bool DIVIDE>
@@ -79,108 +81,179 @@ __device__ __forceinline__ float third_derivative(float s0, float s1, float s2, 
 __device__ __forceinline__ float advance(float init, float dt, float tend) { return __fmaf_rn(dt, tend, init); }
 
 constexpr float kWild = 1.0e15f;  // (products of two, over a third of the density, stay finite)
-constexpr int kMwCellIters = kMwTileXMax / kMwThreads;
 
-// Fluxes and update of a horizontal tile whose row segment is staged.
+struct Flux4 {
+    float v[kMwVars];
+};
+
+// Flux through an interface along x from the interpolated values and third derivatives (compute_tendencies_x, :222-258).
 template <bool DIVIDE>
-__device__ __forceinline__ void update_x(const StencilParams &p, const Grid &g, const float *sin, float *sflux, int i0, int n, unsigned row,
-                                         float hd, float hdt, const float (&init_v)[kMwCellIters][kMwVars]) {
-    constexpr int ldi = kMwTileXMax + 2 * kMwHalo;  // staged values per variable
-    constexpr int ldf = kMwTileXMax + 1;            // fluxes per variable
-    const float hv_coef = __fdiv_rn(__fmul_rn(-kHvBeta, p.dx), __fmul_rn(16.f, p.dt));
-    for (int f = threadIdx.x; f <= n; f += kMwThreads) {  // interface between cells i0+f-1 and i0+f
-        float vals[kMwVars], d3_vals[kMwVars];
+__device__ __forceinline__ Flux4 flux_x(const float (&vals)[kMwVars], const float (&d3)[kMwVars], float hd, float hdt) {
+    const double r = (double)__fadd_rn(vals[ID_DENS], hd);
+    const double inv_r = DIVIDE ? 0.0 : reciprocal(r);
+    const double u = quotient<DIVIDE>((double)vals[ID_UMOM], r, inv_r);
+    const double w = quotient<DIVIDE>((double)vals[ID_WMOM], r, inv_r);
+    const double t = quotient<DIVIDE>((double)__fadd_rn(vals[ID_RHOT], hdt), r, inv_r);
+    const double pr = __dmul_rn((double)kC0, power(__dmul_rn(r, t), (double)kGamm));
+    const double ru = __dmul_rn(r, u);
+    // r*u feeds four fluxes; the mass flux subtracts from the rounded product, the others fuse
+    Flux4 f;
+    f.v[ID_DENS] = (float)__dsub_rn(ru, (double)d3[ID_DENS]);
+    f.v[ID_UMOM] = (float)__dsub_rn(__fma_rn(ru, u, pr), (double)d3[ID_UMOM]);
+    f.v[ID_WMOM] = (float)__fma_rn(ru, w, -(double)d3[ID_WMOM]);
+    f.v[ID_RHOT] = (float)__fma_rn(ru, t, -(double)d3[ID_RHOT]);
+    return f;
+}
+
+// The fluxes through a lane's four interfaces, two at a time; interface q reads staged cells q .. q + 3 of the lane's own
+// four (at `own`) and the next lane's (at `next`).
+template <bool DIVIDE>
+__device__ __forceinline__ void lane_fluxes(const float *own, const float *next, float hv_coef, float hd, float hdt, Flux4 (&f)[kMwCells + 1]) {
+#pragma unroll
+    for (int h = 0; h < kMwCells; h += 2) {
+        float vals[2][kMwVars], d3[2][kMwVars];
 #pragma unroll
         for (int ll = 0; ll < kMwVars; ++ll) {
-            const float s0 = sin[ll * ldi + f], s1 = sin[ll * ldi + f + 1];
-            const float s2 = sin[ll * ldi + f + 2], s3 = sin[ll * ldi + f + 3];
-            vals[ll] = quotient<DIVIDE>(interp4_by_12(s0, s1, s2, s3), 12.f, 1.f / 12.f);
-            d3_vals[ll] = third_derivative(s0, s1, s2, s3, hv_coef);
-        }
-        const double r = (double)__fadd_rn(vals[ID_DENS], hd);
-        const double inv_r = DIVIDE ? 0.0 : reciprocal(r);
-        const double u = quotient<DIVIDE>((double)vals[ID_UMOM], r, inv_r);
-        const double w = quotient<DIVIDE>((double)vals[ID_WMOM], r, inv_r);
-        const double t = quotient<DIVIDE>((double)__fadd_rn(vals[ID_RHOT], hdt), r, inv_r);
-        const double pr = __dmul_rn((double)kC0, power(__dmul_rn(r, t), (double)kGamm));
-        const double ru = __dmul_rn(r, u);
-        // r*u feeds four fluxes; the mass flux subtracts from the rounded product, the others fuse
-        sflux[ID_DENS * ldf + f] = (float)__dsub_rn(ru, (double)d3_vals[ID_DENS]);
-        sflux[ID_UMOM * ldf + f] = (float)__dsub_rn(__fma_rn(ru, u, pr), (double)d3_vals[ID_UMOM]);
-        sflux[ID_WMOM * ldf + f] = (float)__fma_rn(ru, w, -(double)d3_vals[ID_WMOM]);
-        sflux[ID_RHOT * ldf + f] = (float)__fma_rn(ru, t, -(double)d3_vals[ID_RHOT]);
-    }
-    __syncthreads();
-    const float inv_dx = __frcp_rn(p.dx);
+            const float4 a = *reinterpret_cast<const float4 *>(own + ll * kMwRowFloats);
+            const float4 b = *reinterpret_cast<const float4 *>(next + ll * kMwRowFloats);
+            const float s[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-    for (int it = 0; it < kMwCellIters; ++it) {
-        const int f = threadIdx.x + it * kMwThreads;
-        if (f < n) {
-            const unsigned at = row + (unsigned)(i0 + f + kMwHalo);
-#pragma unroll
-            for (int ll = 0; ll < kMwVars; ++ll) {
-                const float tend = -quotient<DIVIDE>(__fsub_rn(sflux[ll * ldf + f + 1], sflux[ll * ldf + f]), p.dx, inv_dx);
-                p.out[ll * g.plane + at] = advance(init_v[it][ll], p.dt, tend);
+            for (int q = 0; q < 2; ++q) {
+                const int o = h + q;
+                vals[q][ll] = quotient<DIVIDE>(interp4_by_12(s[o], s[o + 1], s[o + 2], s[o + 3]), 12.f, 1.f / 12.f);
+                d3[q][ll] = third_derivative(s[o], s[o + 1], s[o + 2], s[o + 3], hv_coef);
             }
         }
+        f[h] = flux_x<DIVIDE>(vals[0], d3[0], hd, hdt);
+        f[h + 1] = flux_x<DIVIDE>(vals[1], d3[1], hd, hdt);
     }
 }
 
-// Horizontal tile: cells [i0, i1) of row k.  compute_tendencies_x (:222-258) then
-// compute_tendencies_x_r (:260-272).  The row segment with two cells on either side is staged in
-// shared memory; the cells beyond the ends of the row wrap around as set_halo_values_x (:331-341)
-// would have written them, and the tiles at the ends of the row store those halo cells.
-__device__ __forceinline__ void tile_x(const StencilParams &p, const Grid &g, int tile, float *smem) {
-    constexpr int ldi = kMwTileXMax + 2 * kMwHalo;  // staged values per variable
-    float *sin = smem, *sflux = smem + kMwVars * ldi;
-    const int k = tile / p.tiles_per_row;
-    const int i0 = (tile - k * p.tiles_per_row) * p.tile_x;
-    const int i1 = min(i0 + p.tile_x, g.nx);
-    const int n = i1 - i0;
-    const unsigned row = (unsigned)(k + kMwHalo) * (unsigned)g.W;
-    const float *__restrict__ forcing = p.forcing;
-    // Every global load of the tile is issued up front: the row segment to stage (up to three
-    // values per variable and thread) and the cells' starting values, which are not needed until
-    // the update and so overlap the flux arithmetic.
-    constexpr int kStageIters = (kMwTileXMax + 2 * kMwHalo + kMwThreads - 1) / kMwThreads;
-    float staged[kStageIters][kMwVars], init_v[kMwCellIters][kMwVars];
+template <int BYTES>
+__device__ __forceinline__ void copy_async(uint32_t dst, const float *src) {
+    if (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+}
+
+// Horizontal tiles: four segments of at most 124 cells of a row, one to a warp.  compute_tendencies_x (:222-258) then
+// compute_tendencies_x_r (:260-272).  The segment from two cells before its first to two behind its last is
+// copied to shared memory, four cells a lane: a lane has four interfaces, and with its neighbour's first flux the
+// four cells between them (the last lane has only that flux to give).  The cells beyond the ends of the row wrap around
+// as set_halo_values_x (:331-341) would have written them, and the segments at the ends of the row store those
+// halo cells.  While a warp works on a segment its next one and the starting values of its cells are on
+// their way, and the claim after that runs beside them.  (A claim for every warp is 41 600 of them in 70 us on
+// one word and one cursor of a 3 200 x 1 600 grid, which is what bounded the kernel then.)
+struct RowTile {
+    int k, i0, n;       // row, first cell, cells
+    unsigned at;        // array index of the first staged cell: column i0, which is cell i0 - 2
+    float hd, hdt;      // the row's background
+};
+__device__ __forceinline__ RowTile row_tile(const StencilParams &p, const Grid &g, int tile, int warp) {
+    RowTile r;
+    const int seg = tile * (kMwThreads / 32) + warp;
+    r.k = seg / p.segs_per_row;
+    r.i0 = (seg - r.k * p.segs_per_row) * p.tile_x;
+    r.n = r.k < g.nz ? min(p.tile_x, g.nx - r.i0) : 0;
+    if (r.n == 0) r.k = 0, r.i0 = 0;  // (the last tile may have fewer than four)
+    r.at = (unsigned)(r.k + kMwHalo) * (unsigned)g.W + (unsigned)r.i0;
+    r.hd = p.hy_dens_cell[r.k + kMwHalo], r.hdt = p.hy_dens_theta_cell[r.k + kMwHalo];
+    return r;
+}
+
+// VEC: floats a copy moves (rows of a multiple of VEC array columns are aligned to it).
+template <int VEC>
+__device__ __forceinline__ void fetch_row(const StencilParams &p, const Grid &g, const RowTile &r, float *stage, int lane) {
+    const int left = g.W - r.i0 - kMwCells * lane;  // array columns from this lane's first on
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(stage) + (uint32_t)lane * kMwCells * 4;
+    if (r.n && kMwCells * lane < r.n + 2 * kMwHalo)
 #pragma unroll
-    for (int it = 0; it < kStageIters; ++it) {
-        const int c = threadIdx.x + it * kMwThreads;
-        const int ca = i0 + c;  // array column
-        const int src = ca < kMwHalo ? ca + g.nx : (ca >= g.nx + kMwHalo ? ca - g.nx : ca);
+        for (int ll = 0; ll < kMwVars; ++ll) {
+            const float *f = p.forcing + ll * g.plane + r.at + kMwCells * lane, *i = p.init + ll * g.plane + r.at + kMwCells * lane;
 #pragma unroll
-        for (int ll = 0; ll < kMwVars; ++ll)
-            staged[it][ll] = c < n + 2 * kMwHalo ? forcing[ll * g.plane + row + src] : 0.f;
-    }
-#pragma unroll
-    for (int it = 0; it < kMwCellIters; ++it) {
-        const int f = threadIdx.x + it * kMwThreads;
-#pragma unroll
-        for (int ll = 0; ll < kMwVars; ++ll)
-            init_v[it][ll] = f < n ? p.init[ll * g.plane + row + (unsigned)(i0 + f + kMwHalo)] : 0.f;
-    }
-    const float hd = p.hy_dens_cell[k + kMwHalo], hdt = p.hy_dens_theta_cell[k + kMwHalo];
-    bool wild = !(fabsf(hdt) < kWild && hd > 1.0e-6f && hd < kWild);
-#pragma unroll
-    for (int it = 0; it < kStageIters; ++it) {
-        const int c = threadIdx.x + it * kMwThreads;
-        const int ca = i0 + c;
-        if (c < n + 2 * kMwHalo) {
-            // (four thirds of the largest density around is the most the interpolation makes of it)
-            wild |= !(2.f * fabsf(staged[it][ID_DENS]) < hd && largest(staged[it][ID_UMOM], staged[it][ID_WMOM], staged[it][ID_RHOT]) < kWild);
-            const bool halo = ca < kMwHalo || ca >= g.nx + kMwHalo;
-#pragma unroll
-            for (int ll = 0; ll < kMwVars; ++ll) {
-                sin[ll * ldi + c] = staged[it][ll];
-                if (halo) p.forcing[ll * g.plane + row + ca] = staged[it][ll];
+            for (int c = 0; c < kMwCells; c += VEC)
+                if (c < left) {
+                    copy_async<4 * VEC>(dst + (ll * kMwRowFloats + c) * 4, f + c);
+                    copy_async<4 * VEC>(dst + ((kMwVars + ll) * kMwRowFloats + c) * 4, i + c);
+                }
+        }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int VEC>
+__device__ __forceinline__ void work_row(const StencilParams &p, const Grid &g, const RowTile &r, float *stage, int lane, float hv_coef,
+                                         float inv_dx) {
+    if (r.n == 0) return;
+    if (r.i0 == 0 || r.i0 + r.n == g.nx) {
+        // an end of the row (or both): the cells beyond it
+        if (lane < 4 * kMwVars) {
+            const int ll = lane >> 2, side = lane & 3;
+            const int ca = side < 2 ? side : g.nx + side;  // array column
+            if (side < 2 ? r.i0 == 0 : r.i0 + r.n == g.nx) {
+                const unsigned row = ll * g.plane + r.at - (unsigned)r.i0;
+                const float v = p.forcing[row + (side < 2 ? ca + g.nx : ca - g.nx)];
+                stage[ll * kMwRowFloats + ca - r.i0] = v;
+                p.forcing[row + ca] = v;
             }
         }
+        __syncwarp();
     }
-    if (__syncthreads_or(wild))
-        update_x<true>(p, g, sin, sflux, i0, n, row, hd, hdt, init_v);
+    const float hd = r.hd, hdt = r.hdt;
+    const float *own = stage + kMwCells * lane;
+    // (the last lane has one interface, of its own cells; what it makes of the others is not used)
+    const float *next = stage + kMwCells * min(lane + 1, 31);
+    bool wild = !(fabsf(hdt) < kWild && hd > 1.0e-6f && hd < kWild);
+    {
+        float4 x[kMwVars];
+#pragma unroll
+        for (int ll = 0; ll < kMwVars; ++ll) {
+            x[ll] = *reinterpret_cast<const float4 *>(own + ll * kMwRowFloats);
+            const int staged = r.n + 2 * kMwHalo - kMwCells * lane;  // of this lane's four
+            if (staged < 4) x[ll].w = 0.f;
+            if (staged < 3) x[ll].z = 0.f;
+            if (staged < 2) x[ll].y = 0.f;
+            if (staged < 1) x[ll].x = 0.f;
+        }
+        const float dens = largest(largest(x[ID_DENS].x, x[ID_DENS].y, x[ID_DENS].z), x[ID_DENS].w, 0.f);
+        float rest = 0.f;
+#pragma unroll
+        for (int ll = 1; ll < kMwVars; ++ll) rest = largest(largest(rest, x[ll].x, x[ll].y), x[ll].z, x[ll].w);
+        // (four thirds of the largest density around is the most the interpolation makes of it)
+        wild |= !(2.f * dens < hd && rest < kWild);
+    }
+    const bool divide = __any_sync(0xffffffffu, wild);
+    Flux4 f[kMwCells + 1];
+    if (divide)
+        lane_fluxes<true>(own, next, hv_coef, hd, hdt, f);
     else
-        update_x<false>(p, g, sin, sflux, i0, n, row, hd, hdt, init_v);
+        lane_fluxes<false>(own, next, hv_coef, hd, hdt, f);
+#pragma unroll
+    for (int ll = 0; ll < kMwVars; ++ll) f[kMwCells].v[ll] = __shfl_down_sync(0xffffffffu, f[0].v[ll], 1);
+    const int cells = r.n - kMwCells * lane;
+    if (cells <= 0) return;
+#pragma unroll
+    for (int ll = 0; ll < kMwVars; ++ll) {
+        const float *ini = stage + (kMwVars + ll) * kMwRowFloats + kMwCells * lane + kMwHalo;
+        const float2 a = *reinterpret_cast<const float2 *>(ini), b = *reinterpret_cast<const float2 *>(ini + 2);
+        const float init_v[kMwCells] = {a.x, a.y, b.x, b.y};
+        float o[kMwCells];
+#pragma unroll
+        for (int c = 0; c < kMwCells; ++c) {
+            const float d = __fsub_rn(f[c + 1].v[ll], f[c].v[ll]);
+            const float tend = -(divide ? __fdiv_rn(d, p.dx) : div_by(d, p.dx, inv_dx));
+            o[c] = advance(init_v[c], p.dt, tend);
+        }
+        float *out = p.out + ll * g.plane + r.at + kMwHalo + kMwCells * lane;
+        if (VEC > 1 && cells >= kMwCells) {
+            *reinterpret_cast<float2 *>(out) = make_float2(o[0], o[1]);
+            *reinterpret_cast<float2 *>(out + 2) = make_float2(o[2], o[3]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < kMwCells; ++c)
+                if (c < cells) out[c] = o[c];
+        }
+    }
 }
 
 // Value of variable ll in array row ka (a row outside the interior) of column ca as the
@@ -200,12 +273,13 @@ __device__ __forceinline__ float halo_row_value(const StencilParams &p, const Gr
     return v;
 }
 
-// Vertical tile: kMwThreads columns x up to kMwTileZRows rows; one thread walks down one column
+// Vertical tile: kMwThreadsZ columns x up to kMwTileZRows rows; one thread walks down one column
 // with the four stencil rows of every variable in registers.  compute_tendencies_z (:278-318)
-// then compute_tendencies_z_r (:320-336).
+// then compute_tendencies_z_r (:320-336).  Four steps are unrolled, so that the rows change their roles by name and
+// no register is moved.
 __device__ __forceinline__ void tile_z(const StencilParams &p, const Grid &g, int tile) {
     const int tr = tile / p.tiles_cols;
-    const int i = (tile - tr * p.tiles_cols) * kMwThreads + (int)threadIdx.x;  // cell column
+    const int i = (tile - tr * p.tiles_cols) * kMwThreadsZ + (int)threadIdx.x;  // cell column
     if (i >= g.nx) return;
     const int k0 = tr * p.tile_rows;
     const int nr = min(p.tile_rows, g.nz - k0);
@@ -213,103 +287,156 @@ __device__ __forceinline__ void tile_z(const StencilParams &p, const Grid &g, in
     const float hv_coef = __fdiv_rn(__fmul_rn(-kHvBeta, p.dz), __fmul_rn(16.f, p.dt));
     const float inv_dz = __frcp_rn(p.dz);
     const float *__restrict__ forcing = p.forcing;
-    float win[kMwVars][4];  // array rows k .. k+3 of interface k
+    auto row_value = [&](int ll, int ka) {  // of array row ka
+        return ka >= kMwHalo && ka < g.nz + kMwHalo ? forcing[ll * g.plane + (unsigned)ka * (unsigned)g.W + (unsigned)ca]
+                                                    : halo_row_value(p, g, ll, ka, ca);
+    };
+    float win[4][kMwVars];  // array row r of a step's stencil is win[(j + r) & 3]
 #pragma unroll
     for (int ll = 0; ll < kMwVars; ++ll)
 #pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const int ka = k0 + s;
-            win[ll][s + 1] = ka >= kMwHalo ? forcing[ll * g.plane + (unsigned)ka * (unsigned)g.W + (unsigned)ca]
-                                           : halo_row_value(p, g, ll, ka, ca);
-        }
-    // Values of the next step are loaded one step ahead, before this step's stores (out may be
-    // the array init points to, so a load could not move above a store by itself).
-    float next_row[kMwVars], next_init[kMwVars];
-#pragma unroll
-    for (int ll = 0; ll < kMwVars; ++ll) {
-        const int ka = k0 + 3;
-        next_row[ll] = ka < g.nz + kMwHalo ? forcing[ll * g.plane + (unsigned)ka * (unsigned)g.W + (unsigned)ca]
-                                           : halo_row_value(p, g, ll, ka, ca);
-        next_init[ll] = 0.f;
-    }
+        for (int r = 0; r < 4; ++r) win[r][ll] = row_value(ll, k0 + r);
+    float next_init[kMwVars] = {0.f, 0.f, 0.f, 0.f};
     float below[kMwVars] = {0.f, 0.f, 0.f, 0.f};  // flux through the interface under the cell about to be updated
-    for (int j = 0; j <= nr; ++j) {
-        const int k = k0 + j;  // interface below cell row k
-        float init_v[kMwVars];
-        const unsigned cell = (unsigned)(k - 1 + kMwHalo) * (unsigned)g.W + (unsigned)ca;  // cell above interface k-1
+    for (int j0 = 0; j0 <= nr; j0 += 4) {
 #pragma unroll
-        for (int ll = 0; ll < kMwVars; ++ll) {
-            win[ll][0] = win[ll][1];
-            win[ll][1] = win[ll][2];
-            win[ll][2] = win[ll][3];
-            win[ll][3] = next_row[ll];
-            init_v[ll] = next_init[ll];
-        }
-        if (j < nr) {
-            const int ka = k + 4;  // last row of the next interface's stencil
+        for (int ph = 0; ph < 4; ++ph) {
+            const int j = j0 + ph;
+            if (j > nr) break;
+            const int k = k0 + j;  // interface below cell row k
+            const unsigned cell = (unsigned)(k - 1 + kMwHalo) * (unsigned)g.W + (unsigned)ca;  // cell above interface k-1
+            // Values of the next step are loaded one step ahead, before this step's stores (out may be
+            // the array init points to, so a load could not move above a store by itself).
+            float next_row[kMwVars], init_v[kMwVars];
 #pragma unroll
             for (int ll = 0; ll < kMwVars; ++ll) {
-                next_row[ll] = ka < g.nz + kMwHalo ? forcing[ll * g.plane + (unsigned)ka * (unsigned)g.W + (unsigned)ca]
-                                                   : halo_row_value(p, g, ll, ka, ca);
-                next_init[ll] = p.init[ll * g.plane + cell + (unsigned)g.W];  // cell row k, updated next step
+                init_v[ll] = next_init[ll];
+                if (j < nr) {
+                    next_row[ll] = row_value(ll, k + 4);  // last row of the next interface's stencil
+                    next_init[ll] = p.init[ll * g.plane + cell + (unsigned)g.W];  // cell row k, updated next step
+                }
             }
-        }
-        const float hd = p.hy_dens_int[k], hdt = p.hy_dens_theta_int[k];
-        float vals[kMwVars], d3_vals[kMwVars];
-#pragma unroll
-        for (int ll = 0; ll < kMwVars; ++ll) {
-            vals[ll] = div_by_any(interp4_by_12(win[ll][0], win[ll][1], win[ll][2], win[ll][3]), 12.f, 1.f / 12.f);
-            d3_vals[ll] = third_derivative(win[ll][0], win[ll][1], win[ll][2], win[ll][3], hv_coef);
-        }
-        const float r = __fadd_rn(vals[ID_DENS], hd);
-        const float inv_r = reciprocal(r);
-        const float u = div_by_any(vals[ID_UMOM], r, inv_r);
-        float w = div_by_any(vals[ID_WMOM], r, inv_r);
-        const float t = div_by_any(__fadd_rn(vals[ID_RHOT], hdt), r, inv_r);
-        const float pr = __fmaf_rn(kC0, powf(__fmul_rn(r, t), kGamm), -p.hy_pressure_int[k]);
-        if (k == 0 || k == g.nz) {
-            w = 0;
-            d3_vals[ID_DENS] = 0;
-        }
-        const float rw = __fmul_rn(r, w);
-        float flux[kMwVars];
-        flux[ID_DENS] = __fsub_rn(rw, d3_vals[ID_DENS]);  // from the rounded product, as along x
-        flux[ID_UMOM] = __fmaf_rn(rw, u, -d3_vals[ID_UMOM]);
-        flux[ID_WMOM] = __fsub_rn(__fmaf_rn(rw, w, pr), d3_vals[ID_WMOM]);
-        flux[ID_RHOT] = __fmaf_rn(rw, t, -d3_vals[ID_RHOT]);
-        if (j > 0) {
-            // Cell row k-1, whose forcing values are win[.][1] (array row k+1).  When the reference
-            // runs this stage with forcing and out in one array (the second Runge-Kutta stage) its
-            // gravity term reads the density the same launch has already updated: its threads are
-            // numbered variable-major (:322-324) and the density blocks run far ahead of the
-            // momentum blocks.  `gravity_from_out` selects that value here, where out is a
-            // separate array.
-            float dens_new = 0.f;
+            const float hd = p.hy_dens_int[k], hdt = p.hy_dens_theta_int[k];
+            float vals[kMwVars], d3_vals[kMwVars];
 #pragma unroll
             for (int ll = 0; ll < kMwVars; ++ll) {
-                float tend = -div_by_any(__fsub_rn(flux[ll], below[ll]), p.dz, inv_dz);
-                if (ll == ID_WMOM) tend = __fmaf_rn(-(p.gravity_from_out ? dens_new : win[ID_DENS][1]), kGrav, tend);
-                const float v = advance(init_v[ll], p.dt, tend);
-                if (ll == ID_DENS) dens_new = v;
-                p.out[ll * g.plane + cell] = v;
+                const float s0 = win[ph][ll], s1 = win[(ph + 1) & 3][ll], s2 = win[(ph + 2) & 3][ll], s3 = win[(ph + 3) & 3][ll];
+                vals[ll] = div_by_any(interp4_by_12(s0, s1, s2, s3), 12.f, 1.f / 12.f);
+                d3_vals[ll] = third_derivative(s0, s1, s2, s3, hv_coef);
+            }
+            const float r = __fadd_rn(vals[ID_DENS], hd);
+            const float inv_r = reciprocal(r);
+            const float u = div_by_any(vals[ID_UMOM], r, inv_r);
+            float w = div_by_any(vals[ID_WMOM], r, inv_r);
+            const float t = div_by_any(__fadd_rn(vals[ID_RHOT], hdt), r, inv_r);
+            const float pr = __fmaf_rn(kC0, powf(__fmul_rn(r, t), kGamm), -p.hy_pressure_int[k]);
+            if (k == 0 || k == g.nz) {
+                w = 0;
+                d3_vals[ID_DENS] = 0;
+            }
+            const float rw = __fmul_rn(r, w);
+            float flux[kMwVars];
+            flux[ID_DENS] = __fsub_rn(rw, d3_vals[ID_DENS]);  // from the rounded product, as along x
+            flux[ID_UMOM] = __fmaf_rn(rw, u, -d3_vals[ID_UMOM]);
+            flux[ID_WMOM] = __fsub_rn(__fmaf_rn(rw, w, pr), d3_vals[ID_WMOM]);
+            flux[ID_RHOT] = __fmaf_rn(rw, t, -d3_vals[ID_RHOT]);
+            if (j > 0) {
+                // Cell row k-1, whose forcing values are array row k+1, the stencil's second.  When the reference
+                // runs this stage with forcing and out in one array (the second Runge-Kutta stage) its
+                // gravity term reads the density the same launch has already updated: its threads are
+                // numbered variable-major (:322-324) and the density blocks run far ahead of the
+                // momentum blocks.  `gravity_from_out` selects that value here, where out is a
+                // separate array.
+                float dens_new = 0.f;
+#pragma unroll
+                for (int ll = 0; ll < kMwVars; ++ll) {
+                    float tend = -div_by_any(__fsub_rn(flux[ll], below[ll]), p.dz, inv_dz);
+                    if (ll == ID_WMOM) tend = __fmaf_rn(-(p.gravity_from_out ? dens_new : win[(ph + 1) & 3][ID_DENS]), kGrav, tend);
+                    const float v = advance(init_v[ll], p.dt, tend);
+                    if (ll == ID_DENS) dens_new = v;
+                    p.out[ll * g.plane + cell] = v;
+                }
+            }
+#pragma unroll
+            for (int ll = 0; ll < kMwVars; ++ll) {
+                below[ll] = flux[ll];
+                if (j < nr) win[ph][ll] = next_row[ll];
             }
         }
-#pragma unroll
-        for (int ll = 0; ll < kMwVars; ++ll) below[ll] = flux[ll];
     }
 }
-
-constexpr int kStageFloats = kMwVars * (kMwTileXMax + 2 * kMwHalo) + kMwVars * (kMwTileXMax + 1);
 
 }  // namespace
 
 // One kernel per direction, so each gets its own register budget (the x direction holds doubles
-// and a staged row, the z direction a 4 x 4 stencil window and two prefetched rows).
-template <int DIR>
-__global__ void __launch_bounds__(kMwThreads, 4)
-miniweather_step_kernel(const __grid_constant__ StencilParams p, BlpArgs blp) {
+// and a lane's fluxes, the z direction a 4 x 4 stencil window and two prefetched rows).
+template <int VEC>
+__global__ void __launch_bounds__(kMwThreads, 6)
+miniweather_x_kernel(const __grid_constant__ StencilParams p, BlpArgs blp) {
     pdl_enter();
-    __shared__ float smem[DIR == 1 ? kStageFloats : 1];
+    __shared__ __align__(16) float s_stage[kMwThreads / 32][2][2 * kMwVars * kMwRowFloats];
+    if (threadIdx.x == 0) trace_begin(blp);
+    const bool dynamic = blp.preempted != nullptr;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const Grid g = grid_of(p);
+    const float hv_coef = __fdiv_rn(__fmul_rn(-kHvBeta, p.dx), __fmul_rn(16.f, p.dt));
+    const float inv_dx = __frcp_rn(p.dx);
+    __shared__ int s_tile[2];
+    int tile, next = -1, iter = 0;
+    // With a CTA for every tile each has one: a second claim would be two round trips to L2 for nothing.
+    const bool more = blp.total_tiles > (int)gridDim.x;
+    if (dynamic) {
+        if (threadIdx.x == 0) s_tile[0] = blp_claim(blp, 0);
+        __syncthreads();
+        tile = s_tile[0];
+    } else {
+        tile = blp_claim(blp, 0);
+    }
+    RowTile now{}, ahead{};
+    if (tile >= 0) {
+        now = row_tile(p, g, tile, warp);
+        fetch_row<VEC>(p, g, now, s_stage[warp][0], lane);
+        if (more) {
+            if (dynamic) {
+                if (threadIdx.x == 0) s_tile[1] = blp_claim(blp, 1);
+                __syncthreads();
+                next = s_tile[1];
+            } else {
+                next = blp_claim(blp, 1);
+            }
+        }
+    }
+    while (tile >= 0) {
+        int word = 0, after = -1;
+        if (next >= 0) {
+            if (dynamic && threadIdx.x == 0) word = load_word(blp.preempted);
+            ahead = row_tile(p, g, next, warp);
+            fetch_row<VEC>(p, g, ahead, s_stage[warp][(iter + 1) & 1], lane);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncwarp();
+        // (the cursor's answer is looked at when the tile is through)
+        const bool asks = next >= 0 && (!dynamic || threadIdx.x == 0), up = word != 0;
+        if (asks) after = dynamic && !up ? atomicAdd(blp.executed, 1) : blp_claim(blp, iter + 2, word);
+        work_row<VEC>(p, g, now, s_stage[warp][iter & 1], lane, hv_coef, inv_dx);
+        ++iter;
+        if (dynamic && next >= 0) {  // (next is the same for the whole CTA)
+            if (threadIdx.x == 0) s_tile[iter & 1] = after < blp.total_tiles ? after : -1;
+            __syncthreads();
+            after = s_tile[iter & 1];
+        } else {
+            __syncwarp();  // the stage is the tile's after next
+        }
+        tile = next, now = ahead, next = after;
+    }
+    if (threadIdx.x == 0) trace_end(blp, iter);
+}
+
+__global__ void __launch_bounds__(kMwThreadsZ, 8)
+miniweather_z_kernel(const __grid_constant__ StencilParams p, BlpArgs blp) {
+    pdl_enter();
     __shared__ int s_tile;
     const bool dynamic = blp.preempted != nullptr;
     if (threadIdx.x == 0) trace_begin(blp);
@@ -326,13 +453,9 @@ miniweather_step_kernel(const __grid_constant__ StencilParams p, BlpArgs blp) {
             tile = blp_claim(blp, iter);
         }
         if (tile < 0) break;
-        if (DIR == 1) {
-            tile_x(p, g, tile, smem);
-            __syncthreads();  // the staging area is reused by the next tile
-        } else {
-            tile_z(p, g, tile);
-        }
+        tile_z(p, g, tile);
         ++iter;
+        if (blp.total_tiles <= (int)gridDim.x) break;  // a tile for every CTA: there is no second one to ask for
     }
     if (threadIdx.x == 0) trace_end(blp, iter);
 }
@@ -459,22 +582,29 @@ int add_field(gpx_model &m, const char *name, Storage::Kind kind, int rank, int6
 
 }  // namespace
 
-int stencil_grid(int dir, int total_tiles, int sm_count) {
+typedef void (*StencilKernel)(const StencilParams, BlpArgs);
+static StencilKernel stencil_kernel(int dir, int nx) {
+    if (dir != 1) return miniweather_z_kernel;
+    return nx % 4 == 0 ? miniweather_x_kernel<4> : (nx % 2 == 0 ? miniweather_x_kernel<2> : miniweather_x_kernel<1>);
+}
+// The kernels want the split of an SM's memory either way: stages of twenty-four warps, or all of it as cache (left as
+// the horizontal kernel needs it, the vertical one takes 82 us instead of 72).
+static cudaError_t stencil_prepare(int nx) {
+    cudaError_t e = cudaFuncSetAttribute(stencil_kernel(1, nx), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(stencil_kernel(2, nx), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+}
+static int stencil_threads(int dir) { return dir == 1 ? kMwThreads : kMwThreadsZ; }
+
+int stencil_grid(int dir, int nx, int total_tiles, int sm_count) {
     int blocks = 0;
-    if (dir == 1)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, miniweather_step_kernel<1>, kMwThreads, 0);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, miniweather_step_kernel<2>, kMwThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, stencil_kernel(dir, nx), stencil_threads(dir), 0);
     if (blocks < 1) blocks = 1;
-    long long grid = (long long)blocks * sm_count;
-    if (grid > total_tiles) grid = total_tiles;
-    return grid < 1 ? 1 : (int)grid;
+    return (int)std::max<long long>(1, std::min<long long>((long long)blocks * sm_count, total_tiles));
 }
 
 cudaError_t stencil_launch(const StencilParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    if (p.dir == 1)
-        return launch_layer(miniweather_step_kernel<1>, grid, kMwThreads, 0, s, p, blp);
-    return launch_layer(miniweather_step_kernel<2>, grid, kMwThreads, 0, s, p, blp);
+    return launch_layer(stencil_kernel(p.dir, p.nx), grid, stencil_threads(p.dir), 0, s, p, blp);
 }
 
 // "miniweather" is the reference's grid (3200 x 1600, miniweather.cu:21-22); "miniweather_tiny"
@@ -555,22 +685,26 @@ int build_miniweather(gpx_model &m, const std::string &name, const gpx_model_opt
     base.dz = dz;
     base.nx = nx;
     base.nz = nz;
-    const int row_tiles = (nx + kMwTileXMax - 1) / kMwTileXMax;
-    base.tile_x = ((nx + row_tiles - 1) / row_tiles + 31) / 32 * 32;
-    base.tiles_per_row = (nx + base.tile_x - 1) / base.tile_x;
-    base.tiles_cols = (nx + kMwThreads - 1) / kMwThreads;
-    // Rows per vertical tile: every tile recomputes one flux row and re-reads three stencil rows,
-    // so taller is cheaper, but the static schedule of a non-preemptible executor gives each CTA
-    // ceil(tiles / grid) tiles; pick the height that wastes least of both.
+    GPX_CUDA(stencil_prepare(nx));
+    // Segments of a row of equal width, in whole lanes.
+    base.segs_per_row = (nx + kMwTileX - 1) / kMwTileX;
+    base.tile_x = ((nx + base.segs_per_row - 1) / base.segs_per_row + kMwCells - 1) / kMwCells * kMwCells;
+    base.segs_per_row = (nx + base.tile_x - 1) / base.tile_x;
+    base.tiles_cols = (nx + kMwThreadsZ - 1) / kMwThreadsZ;
+    // Rows per vertical tile: every tile recomputes one flux row and re-reads three stencil rows, so taller is
+    // cheaper, but a step down a column takes 0.66 us however few CTAs an SM has, and 0.25 us for each of them where
+    // that is more: the height with the least of rows x steps (3 200 x 1 600: 40 rows; 1 026 x 300: 7, where a
+    // kernel takes 11 us instead of 30 with 40).
     {
-        const int grid_full = stencil_grid(2, 1 << 30, m.sm_count);
-        double best = -1.0;
-        for (int rows = 8; rows <= kMwTileZRowsMax; ++rows) {
+        const int resident = stencil_grid(2, nx, 1 << 30, m.sm_count) / m.sm_count;
+        double best = 0.0;
+        for (int rows = 4; rows <= kMwTileZRowsMax; ++rows) {
             const long long tiles = (long long)base.tiles_cols * ((nz + rows - 1) / rows);
-            const long long waves = (tiles + grid_full - 1) / grid_full;
-            const double eff = (double)tiles / (double)(waves * std::min<long long>(grid_full, tiles)) * rows / (rows + 1.5);
-            if (eff > best) {
-                best = eff;
+            long long left = (tiles + m.sm_count - 1) / m.sm_count;  // of the fullest SM
+            double us = 0.0;
+            for (; left > 0; left -= resident) us += (rows + 1.5) * std::max(0.66, 0.25 * (double)std::min<long long>(left, resident));
+            if (best == 0.0 || us < best) {
+                best = us;
                 base.tile_rows = rows;
             }
         }
@@ -598,10 +732,10 @@ int build_miniweather(gpx_model &m, const std::string &name, const gpx_model_opt
             p.dt = stage == 0 ? dt / 3 : (stage == 1 ? dt / 2 : dt / 1);
             p.gravity_from_out = stage == 1 ? 1 : 0;
             k.stencil = p;
-            k.threads = kMwThreads;
-            k.total_tiles = p.dir == 1 ? nz * p.tiles_per_row
+            k.threads = stencil_threads(p.dir);
+            k.total_tiles = p.dir == 1 ? (nz * p.segs_per_row + kMwThreads / 32 - 1) / (kMwThreads / 32)
                                        : p.tiles_cols * ((nz + p.tile_rows - 1) / p.tile_rows);
-            k.grid = stencil_grid(p.dir, k.total_tiles, m.sm_count);
+            k.grid = stencil_grid(p.dir, nx, k.total_tiles, m.sm_count);
             const double cells = (double)nx * nz;
             k.bytes = cells * kMwVars * 4.0 * 3.0;  // forcing and init read, out written
             k.flops = cells * (p.dir == 1 ? 120.0 : 100.0);

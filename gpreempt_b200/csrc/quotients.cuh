@@ -76,8 +76,11 @@ __device__ __forceinline__ double power(double x, double g) {
     p = __fma_rn(p, z, 1.0 / 5);
     p = __fma_rn(p, z, 1.0 / 3);
     const double frac = __dmul_rn(__fma_rn(__dmul_rn(p, z), s, s), 2.8853900817779268);  // 2 / ln 2
-    const double gk = __dmul_rn(g, (double)k), gk_err = __fma_rn(g, (double)k, -gk);
-    const double n = rint(__fma_rn(g, frac, gk));
+    // (integers to and from the low word of a double, by addition: the conversions are a sixteenth as fast)
+    const double kd = __dsub_rn(__hiloint2double(0x43300000, k ^ (int)0x80000000), 4503601774854144.0);  // 2^52 + 2^31
+    const double gk = __dmul_rn(g, kd), gk_err = __fma_rn(g, kd, -gk);
+    const double shifted = __dadd_rn(__fma_rn(g, frac, gk), 6755399441055744.0);  // 1.5 * 2^52: rounds to an integer
+    const double n = __dsub_rn(shifted, 6755399441055744.0);
     const double f = __dmul_rn(__dadd_rn(__dsub_rn(gk, n), __fma_rn(g, frac, gk_err)), 0.69314718055994531);
     double e = 1.0 / 6227020800.0;
     e = __fma_rn(e, f, 1.0 / 479001600.0);
@@ -92,7 +95,7 @@ __device__ __forceinline__ double power(double x, double g) {
     e = __fma_rn(e, f, 1.0 / 6.0);
     e = __fma_rn(e, f, 0.5);
     e = __dadd_rn(1.0, __fma_rn(__dmul_rn(f, f), e, f));
-    return __hiloint2double(__double2hiint(e) + ((int)n << 20), __double2loint(e));
+    return __hiloint2double(__double2hiint(e) + (__double2loint(shifted) << 20), __double2loint(e));
 }
 
 }  // namespace gpx

@@ -17,14 +17,17 @@ namespace gpx {
 
 constexpr int kMwHalo = 2;       // hs
 constexpr int kMwVars = 4;       // rho', rho*u, rho*w, (rho*theta)'
-constexpr int kMwThreads = 256;
-constexpr int kMwTileXMax = 512; // cells of one row per x-direction tile (at most)
+constexpr int kMwCells = 4;      // cells of a row a thread takes in an x-direction tile
+constexpr int kMwThreads = 128;  // x direction: four warps, each with a segment of a row
+constexpr int kMwTileX = 124;    // x direction: cells of a segment at most (31 lanes; with two on either side 128 are staged)
+constexpr int kMwRowFloats = kMwTileX + 2 * kMwHalo;  // staged values per variable
+constexpr int kMwThreadsZ = 128; // columns of a z-direction tile
 constexpr int kMwTileZRowsMax = 40;  // rows of a z-direction tile (chosen per grid); its columns are one per thread
 
 // One semi-discrete step out = init + dt * rhs(forcing) in one direction (semi_discrete_step,
 // src/workloads/miniweather.cu:204-216).  The reference runs it as three kernels (halo, flux,
 // update) with the flux array in global memory; here one kernel computes the fluxes of a tile (in
-// shared memory along x, in registers while walking down a column along z) and updates the tile,
+// registers: of four neighbouring cells a lane along x, while walking down a column along z) and updates the tile,
 // and the tiles on the domain edge produce (and store) the halo cells they read.  `out` never aliases `forcing`: the second Runge-Kutta stage writes a
 // third state buffer instead of updating its forcing array in place.
 struct StencilParams {
@@ -41,9 +44,9 @@ struct StencilParams {
     float dx, dz;
     int nx, nz;
     int dir;              // 1 = x, 2 = z
-    int tile_x;           // x direction: cells per tile; tiles_per_row = ceil(nx / tile_x)
-    int tiles_per_row;
-    int tiles_cols;       // z direction: ceil(nx / kMwThreads)
+    int tile_x;           // x direction: cells per segment (a tile is four); segs_per_row = ceil(nx / tile_x)
+    int segs_per_row;
+    int tiles_cols;       // z direction: ceil(nx / kMwThreadsZ)
     int tile_rows;        // z direction: rows per tile
     // The reference launches its vertical halo kernel with (nx + 2*hs*NUM_VARS + 255) / 256 blocks
     // (miniweather.cu:213), so only flat indices below that many threads get halo values: all of
@@ -55,7 +58,7 @@ struct StencilParams {
 };
 
 cudaError_t stencil_launch(const StencilParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
-int stencil_grid(int dir, int total_tiles, int sm_count);
+int stencil_grid(int dir, int nx, int total_tiles, int sm_count);
 
 bool is_miniweather(const std::string &name);
 int build_miniweather(gpx_model &m, const std::string &name, const gpx_model_opts &opts);
