@@ -75,6 +75,9 @@ __device__ __forceinline__ int blp_claim(const BlpArgs &b, int iter, int word) {
         long long t = (long long)blockIdx.x + (long long)iter * gridDim.x;
         return t < b.total_tiles ? (int)t : -1;
     }
+    // With a CTA for every tile each runs one (also behind a stop: there are as many CTAs as tiles left), and asking for
+    // another would be two round trips to L2 at the end of a kernel that may have lasted four.
+    if (iter > 0 && b.total_tiles <= (int)gridDim.x) return -1;
     if (word != 0) {
         if (b.trace) atomicMin(b.trace + 2, globaltimer_ns());
         // Only a kernel with unclaimed tiles left is a stop point; a kernel whose cursor has
@@ -87,7 +90,8 @@ __device__ __forceinline__ int blp_claim(const BlpArgs &b, int iter, int word) {
     return idx < b.total_tiles ? idx : -1;
 }
 __device__ __forceinline__ int blp_claim(const BlpArgs &b, int iter) {
-    return blp_claim(b, iter, b.preempted ? load_word(b.preempted) : 0);
+    const bool asks = b.preempted != nullptr && !(iter > 0 && b.total_tiles <= (int)gridDim.x);
+    return blp_claim(b, iter, asks ? load_word(b.preempted) : 0);
 }
 
 #if defined(__CUDACC__)

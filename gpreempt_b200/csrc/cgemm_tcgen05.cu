@@ -43,8 +43,6 @@ constexpr int kCAffGroups = 2;       // groups of those warps that take K blocks
 constexpr int kCAffMaxC = kCgemmMaxAffineC;
 constexpr unsigned long long kCWaitLimitNs = 2000000000ull;
 
-// fp32 spill area of one CTA: one accumulator buffer (at most 256 columns) of 128 rows.
-__host__ __device__ constexpr size_t cgemm_spill_floats() { return (size_t)kCBM * 256; }
 
 struct CgemmControlSize {
     unsigned char bytes[2560];  // room for CgemmControl (checked below)
@@ -114,25 +112,9 @@ struct CgemmControl {
 
 static_assert(sizeof(CgemmControl) <= sizeof(CgemmControlSize), "control block outgrew its shared-memory budget");
 
-// x / d for 0 <= x < 2^24 and d > 0 with `inv` = 1.0f / d: the float quotient is off by at most
-// one, which the remainder corrects.  An integer division by a run-time divisor is a chain of
-// ~30 dependent instructions; the epilogue decodes its tile and its row with six of them, about a
-// microsecond per tile for a lone warp, which is what bounded the layers with one or two K blocks.
-__device__ __forceinline__ int fast_div(int x, int d, float inv) {
-    int q = (int)((float)x * inv);
-    int r = x - q * d;
-    if (r < 0) --q;
-    if (r >= d) ++q;
-    return q;
-}
-
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<uint32_t *>(&p);
-}
-// Pulls a TMA descriptor (kernel parameter) into the descriptor cache ahead of its first use.
-__device__ __forceinline__ void prefetch_tensormap(const void *tmap) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
 // 256-bit global load (32-byte aligned): one whole sector per lane.
 __device__ __forceinline__ void ld_global_v8(const void *ptr, uint32_t *r) {
@@ -200,7 +182,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     constexpr int nst = Cfg::kRing;
 
     CgemmSlot *slot = p.slots + blockIdx.x;
-    float *spill = p.spill + (size_t)blockIdx.x * cgemm_spill_floats();
+    float *spill = p.spill + (size_t)blockIdx.x * kCgemmSpillFloats;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -1363,6 +1345,7 @@ int cgemm_max_cluster(int fmt, bool aff, int cluster) {
 }
 
 cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &blp, cudaStream_t s) {
+    if (p.narrow) return conv3x3_narrow_launch(p, grid, blp, s);
     return cgemm_instance(bn, p.fmt == PF_SPLIT, p.aff_scale != nullptr, p.cluster_reduce != 0, [&](auto k) {
         void *args[] = {const_cast<CgemmParams *>(&p), const_cast<BlpArgs *>(&blp)};
         return launch_direct(reinterpret_cast<const void *>(k.kernel()), (unsigned)grid, (unsigned)decltype(k)::Cfg::kThreads,
@@ -1373,7 +1356,5 @@ cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &
 int cgemm_threads(int bn, int fmt, bool aff) {
     return cgemm_instance(bn, fmt == PF_SPLIT, aff, false, [](auto k) { return decltype(k)::Cfg::kThreads; });
 }
-
-size_t cgemm_spill_floats_per_cta() { return cgemm_spill_floats(); }
 
 }  // namespace gpx

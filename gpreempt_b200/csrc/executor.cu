@@ -46,7 +46,7 @@ int exec_launch(gpx_exec *e, size_t idx, cudaStream_t s) {
         // and the finishing kernel.
         if (e->kind != GPX_EXEC_BASE) p.cluster_reduce = 0;
         // The same instance serves latency-critical launches of one 64-column tile a CTA (a cluster of one).
-        if (e->kind == GPX_EXEC_BASE && k.tile == 64 && p.k_splits == 1 && k.grid == k.total_tiles) p.cluster_reduce = 1;
+        if (e->kind == GPX_EXEC_BASE && k.tile == 64 && p.k_splits == 1 && !p.narrow && k.grid == k.total_tiles) p.cluster_reduce = 1;
         err = cgemm_launch(p, k.tile, k.grid, b, s);
     } else if (k.type == KernelType::SplitK) {
         // The convolution kernel before it has already finished the tiles (cluster reduction).
@@ -124,7 +124,7 @@ int gpx_exec_create(gpx_model *m, int kind, gpx_exec **out) {
     // Tensor-core convolutions: per-kernel progress slots, one spill area (only one kernel of an
     // executor can hold partial tiles at a time) and an error word.
     e->d_slots = reinterpret_cast<CgemmSlot *>(e->d_executed + cursors_padded(nk));
-    size_t spill_bytes = sizeof(float) * cgemm_spill_floats_per_cta() * (size_t)(m->max_cgemm_grid + 1);
+    size_t spill_bytes = sizeof(float) * kCgemmSpillFloats * (size_t)(m->max_cgemm_grid + 1);
     GPX_CUDA(cudaMalloc((void **)&e->d_spill, spill_bytes));
     GPX_CUDA(cudaMalloc((void **)&e->d_partial, sizeof(float) * (m->max_partial_floats + 64)));
     GPX_CUDA(cudaMalloc((void **)&e->d_error, 1024));

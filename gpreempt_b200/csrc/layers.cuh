@@ -96,6 +96,7 @@ struct CgemmParams {
     // its partial rows into their owners' shared memory - the additions of splitk_finish_kernel
     // without the workspace round trip and the second launch.
     int cluster_reduce;
+    int narrow;              // 1: launched as the 3x3 kernel for few output channels
     int alternate;           // 1: two groups of epilogue warps take the tiles in turn (short K loops, many tiles)
     SplitKParams fin;        // what the finishing pass needs (bias, residual, activation, output)
     CgemmSlot *slots;        // one per CTA of this kernel
@@ -107,7 +108,16 @@ constexpr int kCgemmMaxAffineC = 2048;  // input channels of a layer with aff_sc
 cudaError_t cgemm_prepare(int device);
 cudaError_t cgemm_launch(const CgemmParams &p, int bn, int grid, const BlpArgs &blp, cudaStream_t s);
 int cgemm_max_cluster(int fmt, bool aff, int cluster);  // CTAs of reducing clusters of this size that can be resident at once
-size_t cgemm_spill_floats_per_cta();
+// fp32 spill area of one CTA: one accumulator buffer (at most 256 columns) of 128 rows.
+constexpr size_t kCgemmSpillFloats = (size_t)128 * 256;
+// The 3x3 stride-1 layers of few output channels (conv3x3_tcgen05.cu), with the same parameters, except for tiles_m
+// and the boxes: of conv3x3_narrow_box rows in a_hi, of cout rows in w_hi.
+cudaError_t conv3x3_narrow_prepare();
+int conv3x3_narrow_threads();
+int conv3x3_narrow_tiles(int m_rows, int cout);
+int conv3x3_narrow_box(int cout);
+bool conv3x3_narrow_fits(int cout, int cin);
+cudaError_t conv3x3_narrow_launch(const CgemmParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
 int cgemm_threads(int bn, int fmt, bool aff);
 
 // ---- CUDA-core convolution / dense (conv_simt.cu) --------------------------------------------

@@ -1265,7 +1265,12 @@ int finalize_model(gpx_model &m) {
         const char *e_min = getenv("GPX_SPLITK_MIN_KB"), *e_all = getenv("GPX_SPLITK_ALLKB");
         const int min_kb = e_min ? std::max(1, atoi(e_min)) : 3;
         const int split_from = e_all ? atoi(e_all) : 8;
-        if (out_tiles * 2 <= m.sm_count && all_kb >= split_from) {
+        // The 3x3 kernel for few output channels, from 1 024 rows on (below, K split over a cluster is
+        // what a latency-critical request wants; DenseNet-201 b64 bf16 with its 64 growth layers of 14x14 and 28x28 images so: 4 072 -> 3 584 us).
+        const char *e_narrow = getenv("GPX_CONV_NARROW");
+        const bool narrow = m.fmt != PF_SPLIT && eff_k == 3 && n.stride == 1 && il.order == ACT_PADDED && !head && !aff && n.residual < 0 &&
+                            p.m_rows > 1024 && conv3x3_narrow_fits(cout_st, eff_cin) && !(e_narrow && e_narrow[0] == '0');
+        if (!narrow && out_tiles * 2 <= m.sm_count && all_kb >= split_from) {
             int s_want = std::min(all_kb / min_kb, m.sm_count / out_tiles);
             // Powers of two up to eight: the splits of an output block can then form a thread-block
             // cluster and reduce through distributed shared memory (non-preemptible launches), if that
@@ -1315,6 +1320,16 @@ int finalize_model(gpx_model &m) {
         p.alternate = p.k_splits == 1 && out_tiles > m.sm_count && (!aff || all_kb <= 8) ? 1 : 0;
         kn.total_tiles = out_tiles * p.k_splits;
         kn.grid = std::min(kn.total_tiles, m.sm_count);
+        if (narrow) {
+            p.narrow = 1;
+            p.tiles_m = conv3x3_narrow_tiles(p.m_rows, cout_st);
+            kn.total_tiles = p.tiles_m;
+            kn.grid = std::min(kn.total_tiles, m.sm_count);
+            kn.threads = conv3x3_narrow_threads();
+            GPX_CUDA(conv3x3_narrow_prepare());
+            GPX_TRY(make_tmap_2d_bf16(&p.w_hi, w.hi, (uint64_t)w.cout_pad, (uint64_t)w.split_k, cout_st, 64));
+            GPX_TRY(make_tmap_2d_bf16(&p.a_hi, in->hi, (uint64_t)il.rows, a_cols, conv3x3_narrow_box(cout_st), 64, a_ld));
+        }
         m.max_cgemm_grid = std::max(m.max_cgemm_grid, kn.grid);
         kn.flops = flops;
         kn.bytes = bytes;

@@ -80,6 +80,18 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// x / d for 0 <= x < 2^24 and d > 0 with `inv` = 1.0f / d: the float quotient is off by at most
+// one, which the remainder corrects.  An integer division by a run-time divisor is a chain of
+// ~30 dependent instructions; the epilogue decodes its tile and its row with six of them, about a
+// microsecond per tile for a lone warp, which is what bounded the layers with one or two K blocks.
+__device__ __forceinline__ int fast_div(int x, int d, float inv) {
+    int q = (int)((float)x * inv);
+    int r = x - q * d;
+    if (r < 0) --q;
+    if (r >= d) ++q;
+    return q;
+}
+
 // ---- TMA ----------------------------------------------------------------------------------
 
 // 2-D tiled load global -> shared, completion counted in bytes on an mbarrier.  x is the
@@ -91,6 +103,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const void *tmap,
         "[%0], [%1, {%3, %4}], [%2];" ::"r"(smem_dst),
         "l"(tmap), "r"(bar), "r"(x), "r"(y)
         : "memory");
+}
+
+// Pulls a TMA descriptor (kernel parameter) into the descriptor cache ahead of its first use.
+__device__ __forceinline__ void prefetch_tensormap(const void *tmap) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
 
 // ---- thread-block clusters: barrier and distributed shared memory -------------------------------
