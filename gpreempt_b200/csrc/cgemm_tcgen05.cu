@@ -279,7 +279,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         }
         __syncwarp();
     }
-    if (resumable || warp == 0) {
+    if (!CL || warp == 0) {
         pdl_wait();  // from here on the predecessor's results (and this executor's slots) are visible
         pdl_launch_dependents();
     }
@@ -977,13 +977,10 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             }
             tmem_st_wait();
         }
-        if (resumable) {
-            tc_fence_before_sync();
-            asm volatile("bar.sync 3, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
-        }
+        tc_fence_before_sync();
+        asm volatile("bar.sync 3, %0;" ::"n"(Cfg::kEpiThreads) : "memory");
         if (threadIdx.x == 64)
             for (int b = 0; b < 2; ++b) mbar_arrive(smem_u32(&ctl->tmem_empty[b]));
-        if (!resumable) pdl_wait();  // the residual is the predecessor's business, everything above is not
         int it = first_iter + group;
         int seg_k0 = group == 0 ? first_k : 0;
         int tiles_done = 0;
