@@ -28,10 +28,11 @@
 // and cycle, 22 us a layer of BERT-base s512 b32), everything else is latency between the two products;
 // two CTAs of two independent warpgroups per SM overlap each other's, to ~30 % of that unit's rate.
 // BERT-base s512 b32, a layer: one warpgroup of 128 keys a block with the output folded into registers
-// and a transposing kernel in front took 89 + 16 us; scores and context issued in line, 82; this, 78.
-// (Tried, at the same time or slower: a warp of its own for copies and products, two buffers of
-// values, the next tile claimed under the merge of this one.)
-// The first warp of a warpgroup issues TMA and MMA; every wait is bounded, and a wait that gives up raises
+// and a transposing kernel in front took 89 + 16 us; scores and context issued in line, 82; by one warp of each
+// group, 73.5; by two, with the next tile claimed under the last block of this one and its queries and first
+// keys fetched under the merge, 70.  (Tried, at the same time or slower: a warp of its own for copies and
+// products, two buffers of values, the next tile claimed under the merge without fetching anything of it.)
+// The first two warps of a warpgroup issue TMA and MMA; every wait is bounded, and a wait that gives up raises
 // a flag that ends all others, so the threads of a CTA pass the same barriers and leave together.
 //
 // A tile takes ~14 us at 512 keys with two CTAs per SM, so the word is read in every block of keys as
@@ -65,6 +66,7 @@ struct FaControl {
     unsigned long long bar_k[2][2];
     uint32_t tmem_base;
     int tile;
+    int next;         // the tile after this one, if it was claimed under this one
     int abort_flag;
     int stop;         // the word was seen raised inside the tile
     int leave[2][2];  // [warpgroup][step parity] what its first thread made of that: the same for all of them
@@ -99,8 +101,10 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
     const int tid = threadIdx.x;
     const int wg = __shfl_sync(0xffffffffu, tid >> 7, 0);  // warpgroup
     const int row = tid & 127;
-    const bool warp0 = __shfl_sync(0xffffffffu, row >> 5, 0) == 0;  // this warpgroup's TMA and MMA warp
-    const bool issuer = elect_one() && warp0;                       // its thread that issues them
+    // The first warp of a warpgroup fetches keys and issues scores, the second fetches values and issues contexts: each
+    // is ~500 cycles a block on top of the softmax, which all four warps wait for.
+    const int wq = __shfl_sync(0xffffffffu, row >> 5, 0);
+    const bool elected = elect_one(), warp0 = wq == 0, issuer = elected && warp0, issuer_v = elected && wq == 1;
     unsigned char *mine = smem + kFaQBytes + wg * kFaGroupBytes;
     const uint32_t sQ = smem_u32(smem), sK = smem_u32(mine), sV = sK + 2 * kFaKBytes, sP = sK + 3 * kFaKBytes;
     unsigned char *pV = mine + 2 * kFaKBytes, *pP = mine + 3 * kFaKBytes;
@@ -153,11 +157,45 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
         if (blp.trace) atomicMin(blp.trace + 2, globaltimer_ns());
         atomicCAS(blp.stop_index, -1, blp.kernel_id);
     };
-    int iter = 0;
+    struct At {
+        int qb, head, b, col0, key_row0;
+    };
+    auto at_tile = [&](int tile) {
+        At a;
+        a.qb = tile % qblocks;
+        a.head = (tile / qblocks) % p.heads;
+        a.b = tile / (qblocks * p.heads);
+        a.col0 = a.head * kFaD, a.key_row0 = a.b * p.S;
+        return a;
+    };
+    auto fetch = [&](const At &a, uint32_t dst, const void *map, unsigned long long *bar, int step) {
+        mbar_arrive_expect_tx(smem_u32(bar), kFaKBytes);
+        tma_load_2d(dst, map, smem_u32(bar), a.col0, a.key_row0 + (2 * step + wg) * kFaKeys);
+    };
+    // queries, and this warpgroup's first keys, of a tile
+    auto fetch_first = [&](const At &a) {
+        if (tid == 0) {
+            mbar_arrive_expect_tx(smem_u32(&ctl->bar_q), kFaQBytes);
+            tma_load_2d(sQ, &p.tq, smem_u32(&ctl->bar_q), a.col0, a.key_row0 + a.qb * kFaQ);
+        }
+        if (issuer && steps > 0) {
+            fetch(a, sK, &p.tk, &ctl->bar_k[wg][0], 0);
+            if (steps > 1) fetch(a, sK + kFaKBytes, &p.tk, &ctl->bar_k[wg][1], 1);
+        }
+    };
+    // The next tile is claimed under the last block of this one (its word and its cursor are on their way under the
+    // exponentials and behind them), when this one can no longer be given up, and its queries and first keys are
+    // fetched under the merge.
+    const bool claims = tid == 96;
+    const bool more = blp.total_tiles > (int)gridDim.x;  // (with a CTA for every tile each runs one)
+    int next = -1, iter = 0;
     for (;; ++iter) {
+        const bool fetched = next >= 0;
         if (tid == 0) {
             int t = -1;
-            if (*abort_flag) {
+            if (*abort_flag || next == -2) {  // (-2: the last tile has been claimed)
+            } else if (fetched) {
+                t = next;
             } else if (pending < 0) {
                 t = blp_claim(blp, iter);
             } else if (load_word(blp.preempted) != 0) {
@@ -168,24 +206,17 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
                 *given_up = 0;
             }
             ctl->tile = t;
+            ctl->next = -1;
             ctl->stop = ctl->gave_up = 0;
         }
         __syncthreads();
         const int tile = ctl->tile;
         if (tile < 0) break;
-        const int qb = tile % qblocks;
-        const int head = (tile / qblocks) % p.heads;
-        const int b = tile / (qblocks * p.heads);
-        const int q0 = qb * kFaQ, key_row0 = b * p.S;
-        const int col0 = head * kFaD;
-        if (tid == 0) {
-            mbar_arrive_expect_tx(smem_u32(&ctl->bar_q), kFaQBytes);
-            tma_load_2d(sQ, &p.tq, smem_u32(&ctl->bar_q), col0, key_row0 + q0);
-        }
-        auto fetch = [&](uint32_t dst, const void *map, unsigned long long *bar, int step) {
-            mbar_arrive_expect_tx(smem_u32(bar), kFaKBytes);
-            tma_load_2d(dst, map, smem_u32(bar), col0, key_row0 + (2 * step + wg) * kFaKeys);
-        };
+        next = -1;
+        const At at = at_tile(tile);
+        const int head = at.head, b = at.b, q0 = at.qb * kFaQ, col0 = at.col0;
+        if (!fetched) fetch_first(at);
+        if (issuer_v && steps > 0) fetch(at, sV, &p.tv, &ctl->bar_v[wg], 0);
         // S = Q K^T of block j (warp 0; the lane that issues it)
         auto scores = [&](int j) {
             const int kb = j & 1;
@@ -201,13 +232,8 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             __syncwarp();
         };
         float m = -INFINITY, l = 0.f;
+        __syncwarp();
         if (steps > 0 && warp0) {
-            if (issuer) {
-                fetch(sK, &p.tk, &ctl->bar_k[wg][0], 0);
-                fetch(sV, &p.tv, &ctl->bar_v[wg], 0);
-                if (steps > 1) fetch(sK + kFaKBytes, &p.tk, &ctl->bar_k[wg][1], 1);
-            }
-            __syncwarp();
             wait(&ctl->bar_q, ph_q, 401);
             scores(0);
         }
@@ -218,9 +244,10 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             ph_s ^= 1;
             tc_fence_after_sync();
             const bool may_leave = given_up && j + 1 < steps;
+            const bool ask = claims && more && j + 1 == steps;
             int word = 0;  // looked at when the softmax, which hides the read, is through
-            if (may_leave && tid == 0) word = load_word(blp.preempted);
-            if (issuer && j + 2 < steps && !*abort_flag) fetch(sK + (j & 1) * kFaKBytes, &p.tk, &ctl->bar_k[wg][j & 1], j + 2);  // S is done with the keys
+            if ((may_leave && tid == 0) || (ask && blp.preempted)) word = load_word(blp.preempted);
+            if (issuer && j + 2 < steps && !*abort_flag) fetch(at, sK + (j & 1) * kFaKBytes, &p.tk, &ctl->bar_k[wg][j & 1], j + 2);  // S is done with the keys
             uint32_t v[64];
             {
                 uint32_t a[32], c[32];
@@ -258,7 +285,7 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             if (j > 0) {
                 wait(&ctl->bar_o[wg], ph_o, 404);
                 ph_o ^= 1;
-                if (issuer && !*abort_flag) fetch(sV, &p.tv, &ctl->bar_v[wg], j);
+                if (issuer_v && !*abort_flag) fetch(at, sV, &p.tv, &ctl->bar_v[wg], j);
             } else {
                 m = m_new;
             }
@@ -296,6 +323,13 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
                 *reinterpret_cast<uint4 *>(prow + (((c >> 3) ^ r8) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
             }
             l += (lsum[0] + lsum[1]) + (lsum[2] + lsum[3]);
+            if (ask) {
+                // (with the word up nothing is claimed here; the claim at the top of the loop records the stop point)
+                if (!blp.preempted)
+                    next = (int)blockIdx.x + (iter + 1) * (int)gridDim.x;
+                else if (word == 0)
+                    next = atomicAdd(blp.executed, 1);
+            }
             if (keys < kFaKeys) {
                 // Rows past the sequence belong to the next batch item: their probabilities are zero, and
                 // so must they be (zero times an infinity is not).
@@ -319,10 +353,10 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
                 left = true;
                 break;
             }
-            if (warp0) {
+            if (wq == 1) {
                 wait(&ctl->bar_v[wg], ph_v, 405);
                 tc_fence_after_sync();
-                if (issuer && !*abort_flag) {
+                if (issuer_v && !*abort_flag) {
                     const uint64_t dp = make_smem_desc_sw128(sP);
                     // Value tile: 64 keys x 128 bytes, 128-byte swizzle.  As an MN-major operand eight keys
                     // are 1024 bytes apart from the next eight, and the 64 output columns are one swizzle
@@ -368,9 +402,12 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
             }
             ctl->ml[wg][row][0] = m;
             ctl->ml[wg][row][1] = l;
+            if (claims && next != -1) ctl->next = next < blp.total_tiles ? next : -2;
         }
         tc_fence_before_sync();
         __syncthreads();
+        next = ctl->next;
+        if (next >= 0 && !*abort_flag) fetch_first(at_tile(next));
         if (ctl->gave_up) {
             if (tid == 0) {
                 *given_up = tile + 1;
