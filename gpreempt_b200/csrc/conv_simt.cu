@@ -314,14 +314,114 @@ struct TileClaims {
     __device__ __forceinline__ int done() const { return iter; }
 };
 
-// Max / average pooling, or a strided copy, over split-plane activations; eight channels (one
+// The larger of two pairs of 16-bit values, NaN giving way as in fmaxf.
+__device__ __forceinline__ unsigned max_packed(unsigned a, unsigned b, int fmt) {
+    unsigned d;
+    if (fmt == PF_F16)
+        asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    else
+        asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+// 3x3 max pooling (K = 3) and 2x2 pooling of either kind (K = 2), without an affine map.  Bound by how many loads
+// are under way: a thread requests all taps of its vector (of two planes, a row of them and the next one) before it
+// looks at any, the largest of 16-bit values is taken as they are, and division by reciprocals keeps the
+// registers of 24 to 40 warps an SM.  112x112x64, 64 images bf16, 3x3: 70 us at two CTAs an SM with fp32 maxima, 38
+// like this (128 MB: 20 us); 299x299 Inception-v3 b16 fp16, first 3x3: 31 us, 14.
+template <int K, bool TWO>
+__global__ void __launch_bounds__(kPoolThreads, K == 3 ? (TWO ? 3 : 4) : (TWO ? 4 : 5))
+pool_window_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
+    pdl_enter();
+    __shared__ int s_tile;
+    if (threadIdx.x == 0) trace_begin(blp);
+    const int C8 = p.channels / 8, H = p.in.l.H, W = p.in.l.W;
+    const unsigned total = (unsigned)p.out.N * p.out.H * p.out.W * C8;  // < 2^31, checked when the model is built
+    const bool plain = p.in.l.order == ACT_PLAIN, is_max = K == 3 || p.mode == 0;
+    const int fmt = TWO ? (int)PF_SPLIT : p.in.l.fmt;
+    TileClaims claims(blp, blp.preempted != nullptr, s_tile);
+    for (int tile = claims.first(); tile >= 0; tile = claims.next()) {
+        const unsigned begin = (unsigned)tile * p.tile_elems;
+        const unsigned end = begin + p.tile_elems < total ? begin + p.tile_elems : total;
+        for (unsigned e = begin + threadIdx.x; e < end; e += kPoolThreads) {
+            const unsigned px = p.by_c8.div(e), py = p.by_w.div(px), n = p.by_h.div(py);
+            const int c0 = (int)(e - px * C8) * 8, wo = (int)(px - py * p.out.W), ho = (int)(py - n * p.out.H);
+            const int h0 = ho * p.stride - p.pad, w0 = wo * p.stride - p.pad;
+            const size_t out = (size_t)layout_row(p.out, n, ho, wo) * p.out.C + c0;
+            if (c0 >= p.in_valid) {
+                float zero[8] = {};
+                planes_store8(p.out_hi, p.out_lo, out, TWO ? (int)PF_SPLIT : p.out.fmt, zero);
+                continue;
+            }
+            const long long at = ((long long)((int)n * p.in.l.Hs + h0) * p.in.l.Ws + w0) * p.in.l.C + c0;
+            const long long row_step = (long long)p.in.l.Ws * p.in.l.C;
+            auto inside = [&](int t) { return (unsigned)(h0 + t / K) < (unsigned)H && (unsigned)(w0 + t % K) < (unsigned)W; };
+            auto fetch = [&](int t, uint4 &a, uint4 &b) {
+                if (!inside(t)) return;
+                const long long off = plain ? at + t / K * row_step + t % K * p.in.l.C
+                                            : (long long)layout_row(p.in.l, n, h0 + t / K, w0 + t % K) * p.in.l.C + c0;
+                planes_fetch8(p.in.hi, p.in.lo, (size_t)off, fmt, a, b);
+            };
+            float acc[8];
+            int cnt = 0;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[j] = is_max ? -INFINITY : 0.f;
+            auto take = [&](const uint4 &a, const uint4 &b) {
+                float x[8];
+                planes_decode8(a, b, fmt, x);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[j] = is_max ? fmaxf(acc[j], x[j]) : acc[j] + x[j];
+                ++cnt;
+            };
+            if (TWO) {
+                uint4 ra[2][K], rb[2][K];
+#pragma unroll
+                for (int t = 0; t < K; ++t) fetch(t, ra[0][t], rb[0][t]);
+#pragma unroll
+                for (int r = 0; r < K; ++r) {
+                    if (r + 1 < K)
+#pragma unroll
+                        for (int t = 0; t < K; ++t) fetch((r + 1) * K + t, ra[(r + 1) & 1][t], rb[(r + 1) & 1][t]);
+                    if (r == 0) claims.ahead();
+#pragma unroll
+                    for (int t = 0; t < K; ++t)
+                        if (inside(r * K + t)) take(ra[r & 1][t], rb[r & 1][t]);
+                }
+            } else {
+                uint4 ra[K * K], none;
+#pragma unroll
+                for (int t = 0; t < K * K; ++t) fetch(t, ra[t], none);
+                claims.ahead();
+                if (is_max) {
+                    const unsigned low = fmt == PF_F16 ? 0xfc00fc00u : 0xff80ff80u;  // -infinity
+                    uint4 m = make_uint4(low, low, low, low);
+#pragma unroll
+                    for (int t = 0; t < K * K; ++t)
+                        if (inside(t)) {
+                            m.x = max_packed(m.x, ra[t].x, fmt), m.y = max_packed(m.y, ra[t].y, fmt);
+                            m.z = max_packed(m.z, ra[t].z, fmt), m.w = max_packed(m.w, ra[t].w, fmt);
+                        }
+                    *reinterpret_cast<uint4 *>(p.out_hi + out) = m;
+                    continue;
+                }
+#pragma unroll
+                for (int t = 0; t < K * K; ++t)
+                    if (inside(t)) take(ra[t], none);
+            }
+            if (!is_max) {
+                const float inv = 1.0f / (float)(p.mode == 1 ? cnt : K * K);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[j] *= inv;
+            }
+            planes_store8(p.out_hi, p.out_lo, out, TWO ? (int)PF_SPLIT : p.out.fmt, acc);
+        }
+    }
+    if (threadIdx.x == 0) trace_end(blp, claims.done());
+}
+
+// Other pooling windows, pooling behind an affine map, or a strided copy, over split-plane activations; eight channels (one
 // 16-byte vector per plane) per thread-iteration.  A tile is tile_elems consecutive output
 // vectors in (n, ho, wo, c/8) order.
-// K = 3: 3x3 max pooling, K = 2: 2x2 pooling of either kind, both without an affine map: the K*K taps are
-// fetched before any is converted, so a thread waits for memory once instead of K*K times (VGG's first
-// 2x2 pooling, 16 images fp16: 61 us one tap at a time).  K = 0: every other mode, at a higher occupancy
-// than the taps in registers allow.
-template <int K>
 __global__ void __launch_bounds__(kPoolThreads)
 pool_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
     pdl_enter();
@@ -337,7 +437,7 @@ pool_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
     for (int tile = claims.first(); tile >= 0; tile = claims.next()) {
         const unsigned begin = (unsigned)tile * p.tile_elems;
         const unsigned end = begin + p.tile_elems < total ? begin + p.tile_elems : total;
-        if (K == 0 && p.mode == 1 && p.k * p.k >= 16) {
+        if (p.mode == 1 && p.k * p.k >= 16) {
             // Large averaging window (global average pool): one warp per output vector, lanes
             // take taps lane, lane+32, ...; a fixed shuffle tree adds the lane sums, so the
             // result is the same on every run.
@@ -390,42 +490,6 @@ pool_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
             int n = (int)(t / Ho);
             float acc[8];
             const bool readable = c8 * 8 < p.in_valid;
-            if (K != 0 && readable) {
-                constexpr int T = K ? K * K : 1, KW = K ? K : 1;
-                uint4 ra[T], rb[T];
-                bool ok[T];
-                const int fmt = p.in.l.fmt;
-                const bool is_max = K == 3 || p.mode == 0;
-#pragma unroll
-                for (int t9 = 0; t9 < T; ++t9) {
-                    const int hi = ho * p.stride - p.pad + t9 / KW, wi = wo * p.stride - p.pad + t9 % KW;
-                    ok[t9] = hi >= 0 && hi < H && wi >= 0 && wi < W;
-                    ra[t9] = rb[t9] = make_uint4(0, 0, 0, 0);
-                    if (ok[t9])
-                        planes_fetch8(p.in.hi, p.in.lo, (size_t)layout_row(p.in.l, n, hi, wi) * Cin + c8 * 8, fmt,
-                                      ra[t9], rb[t9]);
-                }
-                claims.ahead();
-                int cnt = 0;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[j] = is_max ? -INFINITY : 0.f;
-#pragma unroll
-                for (int t9 = 0; t9 < T; ++t9) {
-                    if (!ok[t9]) continue;
-                    ++cnt;
-                    float x[8];
-                    planes_decode8(ra[t9], rb[t9], fmt, x);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[j] = is_max ? fmaxf(acc[j], x[j]) : acc[j] + x[j];
-                }
-                if (!is_max) {
-                    const float inv = 1.0f / (float)(p.mode == 1 ? cnt : T);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[j] *= inv;
-                }
-                pool_store8(p, (size_t)layout_row(p.out, n, ho, wo) * Cout + c8 * 8, acc);
-                continue;
-            }
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[j] = (p.mode == 0 && readable) ? -INFINITY : 0.f;
             int cnt = 0;
@@ -1262,27 +1326,50 @@ cudaError_t dwconv_launch(const DwConvParams &p, int grid, const BlpArgs &blp, c
     return launch_layer(dwconv_instance(p), grid, kPoolThreads, dwconv_smem(p), s, p, blp);
 }
 
+// Taps along a side of the windows that have an instance of their own, else 0.
 static int pool_taps(const PoolParams &p) {
     if (p.scale) return 0;
     if (p.mode == 0 && p.k == 3) return 3;
     return p.mode != 2 && p.k == 2 ? 2 : 0;
 }
-
-int pool_grid(const PoolParams &p, int sm_count) {
-    int per_sm = 8;
-    if (const int t = pool_taps(p)) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, t == 3 ? pool_kernel<3> : pool_kernel<2>, kPoolThreads, 0);
-        if (per_sm < 1) per_sm = 1;
+typedef void (*PoolKernel)(const PoolParams, BlpArgs);
+static PoolKernel pool_instance(const PoolParams &p) {
+    const bool two = p.out.fmt == PF_SPLIT;
+    switch (pool_taps(p)) {
+        case 3: return two ? pool_window_kernel<3, true> : pool_window_kernel<3, false>;
+        case 2: return two ? pool_window_kernel<2, true> : pool_window_kernel<2, false>;
+        default: return pool_kernel;
     }
-    long long grid = (long long)sm_count * per_sm;
-    if (grid > p.total_tiles) grid = p.total_tiles;
-    if (grid < 1) grid = 1;
-    return (int)grid;
+}
+
+// Tiles and grid of a launch whose shapes are set.
+int pool_plan(PoolParams &p, int sm_count) {
+    const long long total = (long long)p.out.N * p.out.H * p.out.W * (p.channels / 8);
+    const int t = pool_taps(p);
+    int per_sm = 8;
+    if (t) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pool_instance(p), kPoolThreads, 0);
+        if (per_sm < 1) per_sm = 1;
+        // A small tensor is cut so that each CTA that fits runs one tile (ResNet's 3x3 at batch 1: 392 tiles of 64
+        // vectors on 296 CTAs were two rounds), a large one into tiles of whole CTAs.
+        const long long slots = (long long)per_sm * sm_count, even = (total + slots - 1) / slots;
+        p.tile_elems = even <= 256 ? (int)std::max<long long>(32, (even + 7) / 8 * 8) : (t == 2 && even >= 1024 ? 512 : 256);
+        p.by_c8 = FastDiv::of((unsigned)(p.channels / 8)), p.by_w = FastDiv::of((unsigned)p.out.W), p.by_h = FastDiv::of((unsigned)p.out.H);
+    } else {
+        // the cap is per unit of work: a copy or an affine map reads one tap per vector
+        const int taps_per_vec = p.mode == 2 ? 1 : p.k * p.k;
+        const long long cap = std::min<long long>(2048, std::max<long long>(256, 9 * 256 / taps_per_vec));
+        if (p.mode == 1 && p.k * p.k >= 16)  // (a warp to a vector: one tile a CTA while that is a few vectors a warp)
+            p.tile_elems = (int)std::max<long long>(8, std::min<long long>(64, (total + 8LL * sm_count - 1) / (8LL * sm_count) / 8 * 8 + 8));
+        else
+            p.tile_elems = (int)std::max<long long>(64, std::min<long long>(cap, total / (4LL * sm_count) / 8 * 8));
+    }
+    p.total_tiles = (int)((total + p.tile_elems - 1) / p.tile_elems);
+    return (int)std::max<long long>(1, std::min<long long>((long long)sm_count * per_sm, p.total_tiles));
 }
 
 cudaError_t pool_launch(const PoolParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    const int t = pool_taps(p);
-    return launch_layer(t == 3 ? pool_kernel<3> : (t == 2 ? pool_kernel<2> : pool_kernel<0>), grid, kPoolThreads, 0, s, p, blp);
+    return launch_layer(pool_instance(p), grid, kPoolThreads, 0, s, p, blp);
 }
 
 }  // namespace gpx

@@ -141,6 +141,19 @@ struct ConvParams {
     int tiles_m, tiles_n;
 };
 
+// n / d by a multiplication, for n below 2^31 (Granlund and Montgomery, PLDI 1994).
+struct FastDiv {
+    unsigned mul, shift;
+    static FastDiv of(unsigned d) {
+        unsigned l = 0;
+        while ((1ull << l) < d) ++l;
+        return {(unsigned)(((1ull << 32) * ((1ull << l) - d)) / d + 1), l};
+    }
+#if defined(__CUDACC__)
+    __device__ __forceinline__ unsigned div(unsigned n) const { return (__umulhi(n, mul) + n) >> shift; }
+#endif
+};
+
 struct PoolParams {
     ActView in;
     bf16_bits *out_hi, *out_lo;
@@ -159,6 +172,7 @@ struct PoolParams {
     // (a batch norm that precedes its consumer, as in DenseNet): x -> act(x * scale + shift).
     const float *scale, *shift;
     int act;
+    FastDiv by_c8, by_w, by_h;  // the windows with an instance of their own
 };
 
 // Second half of a split-K tensor-core convolution: adds the per-split fp32 partial sums in
@@ -312,6 +326,6 @@ void conv_set_tiles(ConvParams &p, int tile);
 int conv_grid(const ConvParams &p, int tile, int sm_count);
 cudaError_t conv_launch(const ConvParams &p, int tile, int grid, const BlpArgs &blp, cudaStream_t s);
 cudaError_t pool_launch(const PoolParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
-int pool_grid(const PoolParams &p, int sm_count);
+int pool_plan(PoolParams &p, int sm_count);  // fills the tiles and returns the grid
 
 }  // namespace gpx

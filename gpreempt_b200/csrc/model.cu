@@ -828,22 +828,8 @@ int finalize_model(gpx_model &m) {
                 p.act = act;
             }
             long long total = (long long)dst.layout.N * dst.layout.H * dst.layout.W * (p.channels / 8);
-            // Enough tiles to fill the GPU even when the tensor is small (global average pool).
-            long long want_tiles = 4LL * m.sm_count;
-            // 3x3 max pooling keeps two CTAs on an SM: a small tensor is cut so that each runs one tile
-            // (ResNet's at batch 1: 392 tiles of 64 vectors on 296 CTAs were two rounds).
-            const bool max3 = mode == 0 && k == 3 && scale < 0;
-            const long long max3_tile = (total + 2LL * m.sm_count - 1) / (2LL * m.sm_count);
-            // the cap is per unit of work: a copy or an affine map reads one tap per vector, a 3x3
-            // pooling nine
-            const int taps_per_vec = mode == 2 ? 1 : k * k;
-            const long long tile_cap = std::min<long long>(2048, std::max<long long>(kMaxTileVectors, 9 * kMaxTileVectors / taps_per_vec));
-            p.tile_elems = (int)std::max<long long>(mode == 1 && k * k >= 16 ? 8 : 64,
-                                                    std::min<long long>(tile_cap, total / want_tiles / 8 * 8));
-            if (max3 && max3_tile <= 256) p.tile_elems = (int)std::max<long long>(32, (max3_tile + 7) / 8 * 8);
-            p.total_tiles = (int)((total + p.tile_elems - 1) / p.tile_elems);
+            kn.grid = pool_plan(p, m.sm_count);
             kn.total_tiles = p.total_tiles;
-            kn.grid = pool_grid(p, m.sm_count);
             int taps = mode == 2 ? 1 : k * k;
             kn.flops = (double)total * 8 * taps;
             kn.bytes = 4.0 * ((double)total * 8 * (mode == 2 ? 1 : stride * stride) + (double)total * 8);
