@@ -81,7 +81,11 @@ struct CgemmCfg {
     // otherwise; two tiles' worth of them in tensor memory, so that the epilogue of one tile overlaps
     // the K loop of the next.
     static constexpr int kBufCols = (int)kPlanes * BN;
-    static constexpr int kTmemCols = 2 * kBufCols;
+    // The mapped A operand of a stage goes to tensor memory (32 columns) where the accumulators leave room: two planes
+    // do not, and a latency-critical launch of three or four K blocks a CTA gains nothing (DenseNet-201 b1 bf16 1 061 us, 1 067).
+    static constexpr int kACols = 2 * kBufCols;
+    static constexpr bool kTmemA = AFF && !TWO && !CL && kACols + 32 * kStages <= 512;
+    static constexpr int kTmemCols = kTmemA ? 512 : 2 * kBufCols;
     static_assert(kTmemCols <= 512 && kStages <= 8, "tile does not fit");
     static_assert(kRing >= 3 && (!CL || BN == 64), "no ring left beside the landing area");
 };
@@ -578,6 +582,11 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                                     mma_f16_ss(acc0, a_hi + 2 * k, w_hi + 2 * k, idesc_wide, k > 0 ? 1u : acc);
                                     mma_f16_ss(acc0 + BN, a_lo + 2 * k, w_hi + 2 * k, idesc, 1u);
                                 }
+                            } else if constexpr (Cfg::kTmemA) {
+                                const uint32_t a_cols = tmem_base + Cfg::kACols + 32 * stage;
+#pragma unroll
+                                for (int k = 0; k < kCBK / kCUmmaK; ++k)
+                                    mma_f16_ts(acc0, a_cols + 8 * k, w_hi + 2 * k, idesc, k > 0 ? 1u : acc);
                             } else {
 #pragma unroll
                                 for (int k = 0; k < kCBK / kCUmmaK; ++k)
@@ -652,6 +661,10 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         // copy of the input that a kernel of its own wrote and this one read back (DenseNet-201 b64
         // bf16: 40 % of the forward) is gone.  (One thread per row, re-reading the scales for every
         // piece, took ~1500 cycles a K block on four warps.)
+        // One-plane operands go to tensor memory instead of back to shared memory, from where the products then
+        // need not read them (32 KB less through its port a K block, of 96) and no fence between proxies is needed.
+        // DenseNet-201 b64 bf16, conv1 layers of block 1 206 -> 195 us, block 2 182 -> 173, block 3 604 -> 592,
+        // transitions 148 -> 141; a K block of block 3 still takes ~830 cycles.
         // Two groups of four warps take the K blocks in turn: a block is a chain of latencies (shared-memory
         // reads, conversions, the fence to the tensor core's proxy) that the other group's overlaps.
         constexpr int kGroupThreads = kCAffThreads / kCAffGroups;
@@ -693,6 +706,49 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 if (TWO) *reinterpret_cast<uint4 *>(a + Cfg::kABytes + r * 2048) = make_uint4(l[0], l[1], l[2], l[3]);
             }
         };
+        // Into tensor memory: a thread takes, of rows r8 + 8 i of its warp's 32, four channels of each sixteen.  Odd rows take
+        // the four sixteens in another order, so that sixteen lanes meet in no bank.
+        const int r8 = lane >> 2, quad = lane & 3, turned = (r8 & 1) << 1;
+        auto map_to_tmem = [&](const unsigned char *a, uint32_t cols, int ch, auto half) {
+            constexpr int FMT = decltype(half)::value ? PF_F16 : PF_BF16;
+            float2 ss[4][2], bb[4][2];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int c = ch + 16 * (b ^ turned) + 4 * quad;
+                const float4 s4 = *reinterpret_cast<const float4 *>(aff_s + c), o4 = *reinterpret_cast<const float4 *>(aff_s + kCAffMaxC + c);
+                ss[b][0] = make_float2(s4.x, s4.y), ss[b][1] = make_float2(s4.z, s4.w);
+                bb[b][0] = make_float2(o4.x, o4.y), bb[b][1] = make_float2(o4.z, o4.w);
+            }
+            const unsigned char *mine = a + ((warp & 3) * 32 + r8) * 128 + (quad & 1) * 8;
+            uint2 v[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    v[i][b] = *reinterpret_cast<const uint2 *>(mine + i * 1024 + (((2 * (b ^ turned) + (quad >> 1)) ^ r8) << 4));
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                uint32_t m[4][2][2], o[16];
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) {
+                            const uint32_t two = k ? v[2 * hh + i][b].y : v[2 * hh + i][b].x;
+                            float2 x = half ? pf_unpack2(two, PF_F16) : make_float2(bf16_lo_to_f32(two), bf16_hi_to_f32(two));
+                            x = fma2(x, ss[b][k], bb[b][k]);
+                            m[b][i][k] = pf_pack2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f), FMT);
+                        }
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+#pragma unroll
+                    for (int i = 0; i < 2; ++i)
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) o[4 * b + 2 * i + k] = turned ? m[b ^ 2][i][k] : m[b][i][k];
+                tmem_st_16x256x4(cols + ((uint32_t)(16 * hh) << 16), o);
+            }
+        };
         static_assert(Cfg::kKps == 1 || !AFF, "one K block per stage");
         int stage = 0, kb = first_k, turn = 0;
         uint32_t phase = 0;
@@ -710,13 +766,24 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                         go = false;
                         break;
                     }
-                    unsigned char *a = smem + stage * Cfg::kStageBytes + off;
-                    const int ch = (t.kb_base + kb) * kCBK + piece * 8;
-                    if (half_fmt)
-                        map_block(a, ch, std::true_type());
-                    else
-                        map_block(a, ch, std::false_type());
-                    fence_proxy_async();  // ordinary stores, read by the tensor core
+                    unsigned char *a = smem + stage * Cfg::kStageBytes;
+                    const int ch = (t.kb_base + kb) * kCBK;
+                    if constexpr (Cfg::kTmemA) {
+                        tc_fence_after_sync();  // the products that read this stage's columns are behind its barriers
+                        const uint32_t cols = tmem_base + Cfg::kACols + 32 * stage + ((uint32_t)((warp & 3) * 32) << 16);
+                        if (half_fmt)
+                            map_to_tmem(a, cols, ch, std::true_type());
+                        else
+                            map_to_tmem(a, cols, ch, std::false_type());
+                        tmem_st_wait();
+                        tc_fence_before_sync();
+                    } else {
+                        if (half_fmt)
+                            map_block(a + off, ch + piece * 8, std::true_type());
+                        else
+                            map_block(a + off, ch + piece * 8, std::false_type());
+                        fence_proxy_async();  // ordinary stores, read by the tensor core
+                    }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&ctl->ready[stage]));
                 }

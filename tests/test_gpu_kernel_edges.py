@@ -31,8 +31,8 @@ def _param(name, std=0.1, kind="param"):
 class _Graph:
     """A graph as an exported model directory holds it."""
 
-    def __init__(self, batch, dtype):
-        self.batch, self.dtype = batch, dtype
+    def __init__(self, batch, dtype, pad_channels=False):
+        self.batch, self.dtype, self.pad_channels = batch, dtype, pad_channels
         self.nodes, self.shapes, self.types = [], [], []
 
     def add(self, node, shape, dltype="float32"):
@@ -70,7 +70,7 @@ class _Graph:
 
         path.mkdir(exist_ok=True)
         graph = {"nodes": self.nodes, "heads": [[len(self.nodes) - 1, 0, 0]],
-                 "gpx": {"model": "edges", "batch": self.batch, "dtype": self.dtype, "pad_channels": False},
+                 "gpx": {"model": "edges", "batch": self.batch, "dtype": self.dtype, "pad_channels": self.pad_channels},
                  "attrs": {"dltype": ["list_str", self.types], "shape": ["list_shape", self.shapes]}}
         (path / "mod.json").write_text(json.dumps(graph))
         (path / "host.json").write_text(json.dumps(
@@ -83,7 +83,7 @@ class _Graph:
         return ex
 
 
-def _conv64(ex, name, src, dtype, pad=0, stride=1, groups=1, act=0, residual=None):
+def _conv64(ex, name, src, dtype, pad=0, stride=1, groups=1, act=0, residual=None, padded=False):
     import torch
 
     def image(key):
@@ -91,7 +91,7 @@ def _conv64(ex, name, src, dtype, pad=0, stride=1, groups=1, act=0, residual=Non
         return x.reshape(*x.shape[:2], 1, 1) if x.dim() == 2 else x
 
     w = torch.from_numpy(ex.model.get(name + ".weight"))
-    if dtype != "float32" and groups == 1 and w.shape[1] % 64 == 0:  # (read back as the exact 32-bit copy; tensor cores multiply 16 bits)
+    if dtype != "float32" and groups == 1 and (padded or w.shape[1] % 64 == 0):  # (read back as the exact 32-bit copy; tensor cores multiply 16 bits)
         w = w.to(getattr(torch, dtype))
     out = torch.nn.functional.conv2d(image(src), w.double(), torch.from_numpy(ex.model.get(name + ".bias")).double(),
                                      padding=pad, stride=stride, groups=groups)
@@ -204,6 +204,35 @@ def test_latency_critical_layers_of_few_rows(gpx, tmp_path, hw, cin, cout, dtype
     _close(ex.model.get("b"), _conv64(ex, "b", "a", dtype, act=1, residual="r"), dtype, "b")
     _close(ex.model.get("c"), _conv64(ex, "c", "b", dtype), dtype, "c")
     ex.clear()
+
+
+# The batch norm in the operand, mapped in shared memory (two planes, latency-critical launches) or into tensor memory: one
+# block of channels, a last one in part, more than the ring holds; a last tile of one row and a CTA's second tile.
+@pytest.mark.parametrize("cin,cout,n,hw", [(64, 128, 1, 1), (64, 64, 3, 13), (96, 128, 1, 23), (160, 128, 129, 1), (448, 128, 2, 9), (704, 64, 5, 7),
+                                           (128, 128, 64, 20)])
+@pytest.mark.parametrize("preemptible", [False, True])
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+def test_batch_norm_in_the_operand_of_one_layer(gpx, tmp_path, cin, cout, n, hw, preemptible, dtype):
+    g = _Graph(n, dtype, pad_channels=True)
+    x = g.conv("a", g.input(n, 3, hw, hw), cin)
+    x = g.op("norm", "gpx_affine", [x, g.add(_param("norm.weight"), [cin]), g.add(_param("norm.bias"), [cin])], g.shapes[x],
+             kernel=1, stride=1, padding=0, activation=1, in_channels=cin)
+    g.heads(g.conv("b", x, cout, act=1))
+    ex = g.load(gpx, tmp_path / "norm", gpx.BLPExecutor if preemptible else gpx.BaseExecutor)
+    rng, s = np.random.default_rng(cin), gpx.Stream(1)
+    ex.model.set("norm.weight", rng.normal(1, 0.3, cin).astype(np.float32))
+    ex.model.set("norm.bias", rng.normal(0, 0.3, cin).astype(np.float32))
+    if preemptible:
+        word = gpx.PreemptWord(1)
+        ex.set_word(word)
+    ex.set_input("data", gpx.synth_normal(n * 3 * hw * hw, 2, 0).reshape(n, 3, hw, hw))
+    ex.execute(s)
+    s.sync()
+    assert ex.error() == (0, 0)
+    _close(ex.model.get("b"), _conv64(ex, "b", "norm", dtype, act=1, padded=True), dtype, "b")
+    ex.clear(), s.destroy()
+    if preemptible:
+        word.destroy()
 
 
 # One to four vectors a lane, partial ones, and rows on both sides of 32 an SM (the last row of a tile alone).
