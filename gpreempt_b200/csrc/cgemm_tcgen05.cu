@@ -38,8 +38,7 @@ constexpr int kCBM = 128, kCBK = 64, kCUmmaK = 16;
 // word: kEpiParts epilogue warps per TMEM lane quarter, each taking an equal share of the columns,
 // so that enough independent TMEM loads, conversions and stores are in flight while a tile is drained
 // (the epilogue, not the tensor pipe, bounds the small-K layers).
-constexpr int kCAffThreads = 256;  // eight more warps where the A operand goes through an affine map first
-constexpr int kCAffGroups = 2;       // groups of those warps that take K blocks in turn
+constexpr int kCAffGroup = 128;  // threads of a group that maps an A operand; groups take K blocks in turn
 constexpr int kCAffMaxC = kCgemmMaxAffineC;
 constexpr unsigned long long kCWaitLimitNs = 2000000000ull;
 
@@ -58,7 +57,8 @@ struct CgemmCfg {
     static constexpr int kEpiParts = BN == 256 || (CL && !AFF) ? 4 : 2;  // epilogue warps per TMEM lane quarter
     static constexpr int kEpiThreads = 128 * kEpiParts;
     static constexpr int kPollWarp = 2 + kEpiThreads / 32;
-    static constexpr int kThreads = 64 + kEpiThreads + 32 + (AFF ? kCAffThreads : 0);
+    static constexpr int kAffGroups = !AFF ? 0 : (!TWO && !CL ? 3 : 2);
+    static constexpr int kThreads = 64 + kEpiThreads + 32 + kAffGroups * kCAffGroup;
     static constexpr uint32_t kPlanes = TWO ? 2 : 1;
     static constexpr uint32_t kABytes = kCBM * kCBK * 2;        // one plane of A: 16 KiB
     static constexpr uint32_t kWBytes = BN * kCBK * 2;          // one plane of W
@@ -192,7 +192,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(smem_u32(&ctl->full[s]), 1);
             mbar_init(smem_u32(&ctl->empty[s]), 1);
-            if (AFF) mbar_init(smem_u32(&ctl->ready[s]), kCAffThreads / 32 / kCAffGroups);
+            if (AFF) mbar_init(smem_u32(&ctl->ready[s]), kCAffGroup / 32);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&ctl->tmem_full[b]), 2);
@@ -413,7 +413,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     }
                     if (AFF) {
                         // each group of the affine map looks at its own stages only: one message for each
-                        for (int g = 1; g < kCAffGroups; ++g) {
+                        for (int g = 1; g < Cfg::kAffGroups; ++g) {
                             if (++stage == nst) {
                                 stage = 0;
                                 phase ^= 1;
@@ -664,10 +664,12 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         // One-plane operands go to tensor memory instead of back to shared memory, from where the products then
         // need not read them (32 KB less through its port a K block, of 96) and no fence between proxies is needed.
         // DenseNet-201 b64 bf16, conv1 layers of block 1 206 -> 195 us, block 2 182 -> 173, block 3 604 -> 592,
-        // transitions 148 -> 141; a K block of block 3 still takes ~830 cycles.
-        // Two groups of four warps take the K blocks in turn: a block is a chain of latencies (shared-memory
-        // reads, conversions, the fence to the tensor core's proxy) that the other group's overlaps.
-        constexpr int kGroupThreads = kCAffThreads / kCAffGroups;
+        // transitions 148 -> 141 (with three groups 192, 169, 567 and 138); a K block of block 3 still takes ~830 cycles.
+        // Groups of four warps take the K blocks in turn: a block is a chain of latencies (shared-memory
+        // reads, conversions, the fence to the tensor core's proxy or the stores to tensor memory) that the other groups'
+        // overlap.  Three groups where one plane leaves the registers for them: DenseNet-201 b64 bf16 2 767 -> 2 750 us,
+        // with the maxima taken packed; latency-critical launches have too few blocks, two planes too few stages.
+        constexpr int kGroupThreads = kCAffGroup;
         const int group = (warp - Cfg::kPollWarp - 1) / (kGroupThreads / 32);
         const int at = ((int)threadIdx.x - (Cfg::kPollWarp + 1) * 32) % kGroupThreads;
         const int piece = at & 7, row = at >> 3;
@@ -738,7 +740,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                             const uint32_t two = k ? v[2 * hh + i][b].y : v[2 * hh + i][b].x;
                             float2 x = half ? pf_unpack2(two, PF_F16) : make_float2(bf16_lo_to_f32(two), bf16_hi_to_f32(two));
                             x = fma2(x, ss[b][k], bb[b][k]);
-                            m[b][i][k] = pf_pack2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f), FMT);
+                            m[b][i][k] = max_packed(pf_pack2(x.x, x.y, FMT), 0u, FMT);
                         }
 #pragma unroll
                 for (int b = 0; b < 4; ++b)
@@ -787,7 +789,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&ctl->ready[stage]));
                 }
-                turn = turn + 1 == kCAffGroups ? 0 : turn + 1;
+                turn = turn + 1 == Cfg::kAffGroups ? 0 : turn + 1;
                 if (++stage == nst) {
                     stage = 0;
                     phase ^= 1;

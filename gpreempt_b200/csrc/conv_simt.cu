@@ -314,16 +314,6 @@ struct TileClaims {
     __device__ __forceinline__ int done() const { return iter; }
 };
 
-// The larger of two pairs of 16-bit values, NaN giving way as in fmaxf.
-__device__ __forceinline__ unsigned max_packed(unsigned a, unsigned b, int fmt) {
-    unsigned d;
-    if (fmt == PF_F16)
-        asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    else
-        asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-    return d;
-}
-
 // 3x3 max pooling (K = 3) and 2x2 pooling of either kind (K = 2), without an affine map.  Bound by how many loads
 // are under way: a thread requests all taps of its vector (of two planes, a row of them and the next one) before it
 // looks at any, the largest of 16-bit values is taken as they are, and division by reciprocals keeps the

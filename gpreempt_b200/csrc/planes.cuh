@@ -44,6 +44,16 @@ __device__ __forceinline__ unsigned pf_pack2(float a, float b, int fmt) {
     return *reinterpret_cast<unsigned *>(&v);
 }
 
+// The larger of two pairs of 16-bit values, NaN giving way as in fmaxf.
+__device__ __forceinline__ unsigned max_packed(unsigned a, unsigned b, int fmt) {
+    unsigned d;
+    if (fmt == PF_F16)
+        asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    else
+        asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
 __device__ __forceinline__ void planes_load8(const plane_bits *hi, const plane_bits *lo, size_t off, int fmt,
                                              float (&x)[8]) {
     const uint4 a = *reinterpret_cast<const uint4 *>(hi + off);
