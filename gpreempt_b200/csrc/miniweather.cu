@@ -141,8 +141,8 @@ __device__ __forceinline__ void copy_async(uint32_t dst, const float *src) {
 // compute_tendencies_x_r (:260-272).  The segment from two cells before its first to two behind its last is
 // copied to shared memory, four cells a lane: a lane has four interfaces, and with its neighbour's first flux the
 // four cells between them (the last lane has only that flux to give).  The cells beyond the ends of the row wrap around
-// as set_halo_values_x (:331-341) would have written them, and the segments at the ends of the row store those
-// halo cells.  While a warp works on a segment its next one and the starting values of its cells are on
+// as set_halo_values_x (:331-341) would have written them, whichever segment reads them, and the segments at the ends of
+// the row store those halo cells.  While a warp works on a segment its next one and the starting values of its cells are on
 // their way, and the claim after that runs beside them.  (A claim for every warp is 41 600 of them in 70 us on
 // one word and one cursor of a 3 200 x 1 600 grid, which is what bounded the kernel then.)
 struct RowTile {
@@ -185,16 +185,18 @@ template <int VEC>
 __device__ __forceinline__ void work_row(const StencilParams &p, const Grid &g, const RowTile &r, float *stage, int lane, float hv_coef,
                                          float inv_dx) {
     if (r.n == 0) return;
-    if (r.i0 == 0 || r.i0 + r.n == g.nx) {
-        // an end of the row (or both): the cells beyond it
+    const int staged_end = r.i0 + r.n + 2 * kMwHalo;  // array columns r.i0 .. staged_end - 1 are staged
+    if (r.i0 == 0 || staged_end > g.nx + kMwHalo) {
+        // an end of the row (or both) among them: the cells beyond it.  (The segment before a last one of a single cell
+        // reads one of them as well, but only the last one stores them.)
         if (lane < 4 * kMwVars) {
             const int ll = lane >> 2, side = lane & 3;
             const int ca = side < 2 ? side : g.nx + side;  // array column
-            if (side < 2 ? r.i0 == 0 : r.i0 + r.n == g.nx) {
+            if (side < 2 ? r.i0 == 0 : ca < staged_end) {
                 const unsigned row = ll * g.plane + r.at - (unsigned)r.i0;
                 const float v = p.forcing[row + (side < 2 ? ca + g.nx : ca - g.nx)];
                 stage[ll * kMwRowFloats + ca - r.i0] = v;
-                p.forcing[row + ca] = v;
+                if (side < 2 || r.i0 + r.n == g.nx) p.forcing[row + ca] = v;
             }
         }
         __syncwarp();

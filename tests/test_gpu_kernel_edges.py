@@ -354,8 +354,8 @@ def test_pool_windows(gpx, tmp_path, fn, kernel, stride, pad, n, channels, hw, d
     ex.clear()
 
 
-# Rows of four, two and one cells a lane, a last segment of one cell and a last tile of one segment; along z heights that do
-# not divide.
+# Rows of four, two and one cells a lane, last segments of 61 to 124 cells and a last tile of one segment; along z heights
+# that do not divide.
 @pytest.mark.parametrize("nx,nz", [(500, 20), (124, 10), (126, 33), (125, 17), (249, 20), (373, 9), (1026, 30)])
 def test_miniweather_remainders(gpx, nx, nz):
     from oracle import miniweather as mw
@@ -372,3 +372,66 @@ def test_miniweather_remainders(gpx, nx, nz):
         for v, bound in enumerate((2e-6, 6e-4, 6e-4, 2e-4)):
             assert np.max(np.abs(mw.interior(got)[v].astype(np.float64) - mw.interior(want)[v])) <= bound * step, (step, v)
     ex.clear()
+
+
+# Widths of 124 k + 1 cells from 3 721 on: the last segment of a row has a single cell, so the one before it reads a cell beyond
+# the row too.  A warm bubble and a wind lie on the end of the rows, and the halo columns hold nothing that would pass.
+@pytest.mark.parametrize("nx,nz", [(3721, 8), (3721, 12), (3845, 9)])
+def test_miniweather_last_segment_of_one_cell(gpx, nx, nz):
+    from oracle import miniweather as mw
+
+    segments = -(-nx // 124)
+    width = -(-(-(-nx // segments)) // 4) * 4  # in whole lanes of four cells
+    segments = -(-nx // width)
+    assert nx - (segments - 1) * width == 1
+    mw.build()
+    orc = mw.Oracle(nx, nz)
+    ex, be = gpx.BaseExecutor(), gpx.BLPExecutor()
+    for e in (ex, be):
+        e.init(f"miniweather_{nx}x{nz}")
+    # (a tile of the horizontal kernel is four segments: this is the plan the widths above are of)
+    assert be.model.get_kernel_info(0)["total_tiles"] == -(-nz * segments // 4)
+    off = (np.arange(nx) + 0.5) / nx
+    off = np.minimum(off, 1 - off)  # distance from the end of the row, around it
+    bump = np.exp(-(off * nx / 6) ** 2).astype(np.float32)
+    start = orc.state.copy()
+    start[0, 2:-2, 2:-2] += np.float32(1e-3) * bump
+    start[1, 2:-2, 2:-2] += np.float32(5.0) * bump
+    start[3, 2:-2, 2:-2] += np.float32(3.0) * bump
+    start[:, :, :2] = start[:, :, -2:] = -1.0
+    orc.state[:] = start
+    ex.model.set("state", start)
+    for step in (1, 2):
+        ex.execute()
+        orc.timestep()
+        got, want = ex.model.get("state"), orc.state
+        for v, bound in enumerate((2e-6, 6e-4, 6e-4, 2e-4)):  # (as above)
+            assert np.max(np.abs(mw.interior(got)[v].astype(np.float64) - mw.interior(want)[v])) <= bound * step, (step, v)
+    # the same bits behind stops anywhere in the two steps
+    word, s = gpx.PreemptWord(1), gpx.Stream(1)
+    be.set_word(word)
+    rng, stops = np.random.default_rng(nx + nz), 0
+    for trial in range(6):
+        be.model.set("state", start)
+        for _ in range(2):
+            if trial % 2:
+                word.raise_()  # (launched while it is up: the first kernel is the stop)
+            be.execute(s)
+            for turn in range(40):
+                if turn < 4:
+                    until = time.perf_counter() + float(rng.uniform(0, 60e-6))
+                    while time.perf_counter() < until:
+                        pass
+                    word.raise_()
+                s.sync()
+                word.clear()
+                time.sleep(0.0005)
+                if be.resume(s) == -1:
+                    break
+                stops += 1
+            else:
+                raise AssertionError("does not end")
+            s.sync()
+        assert np.array_equal(mw.interior(be.model.get("state")), mw.interior(got))
+    assert stops > 0
+    ex.clear(), be.clear(), word.destroy(), s.destroy()
