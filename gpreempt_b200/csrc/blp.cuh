@@ -94,6 +94,13 @@ __device__ __forceinline__ int blp_claim(const BlpArgs &b, int iter) {
     return blp_claim(b, iter, asks ? load_word(b.preempted) : 0);
 }
 
+// Shared-memory slots of a kernel that claims two tiles ahead of the one it works on: claim i is stored by one thread in
+// slot claim_slot(i), behind it all threads pass a barrier and read it.  The claim that comes to the same slot next
+// is stored two barriers later at least, so that the slowest warp has read this one: with two slots the third
+// claim of a kernel that reads its first two behind one barrier is stored where a warp may still have to read the second.
+constexpr int kClaimSlots = 3;
+constexpr __host__ __device__ int claim_slot(int claim) { return claim % kClaimSlots; }
+
 #if defined(__CUDACC__)
 // Layer kernels are launched with the programmatic-serialization attribute (GPX_PDL=0 turns it off).
 inline bool pdl_enabled() {

@@ -108,7 +108,7 @@ template <int NV, bool TWO, bool EMB>
 __global__ void __launch_bounds__(kTfThreads, NV <= 3 && !EMB ? 3 : 2)
 layernorm_kernel(const __grid_constant__ LayerNormParams p, BlpArgs blp) {
     __shared__ __align__(16) float s_gamma[256 * NV], s_beta[256 * NV];
-    __shared__ int s_tile[2];
+    __shared__ int s_tile[kClaimSlots];
     // (parameters: no kernel writes them, so they are fetched while the predecessor drains)
     for (int i = threadIdx.x; i < p.H / 4; i += kTfThreads) {
         reinterpret_cast<float4 *>(s_gamma)[i] = __ldg(reinterpret_cast<const float4 *>(p.gamma) + i);
@@ -123,11 +123,11 @@ layernorm_kernel(const __grid_constant__ LayerNormParams p, BlpArgs blp) {
     if (dynamic) {
         if (threadIdx.x == 0) {
             const int first = blp_claim(blp, 0);
-            s_tile[0] = first;
-            s_tile[1] = first >= 0 ? blp_claim(blp, 1) : -1;
+            s_tile[claim_slot(0)] = first;
+            s_tile[claim_slot(1)] = first >= 0 ? blp_claim(blp, 1) : -1;
         }
         __syncthreads();
-        tile = s_tile[0], next = s_tile[1];
+        tile = s_tile[claim_slot(0)], next = s_tile[claim_slot(1)];
     } else {
         __syncthreads();
         tile = blp_claim(blp, 0), next = blp_claim(blp, 1);
@@ -167,9 +167,9 @@ layernorm_kernel(const __grid_constant__ LayerNormParams p, BlpArgs blp) {
         }
         ++iter;
         if (dynamic && next >= 0) {  // (next is the same for the whole CTA)
-            if (threadIdx.x == 0) s_tile[iter & 1] = after;
+            if (threadIdx.x == 0) s_tile[claim_slot(iter + 1)] = after;
             __syncthreads();
-            after = s_tile[iter & 1];
+            after = s_tile[claim_slot(iter + 1)];
         }
         tile = next, next = after;
 #pragma unroll

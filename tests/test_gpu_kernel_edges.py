@@ -435,3 +435,72 @@ def test_miniweather_last_segment_of_one_cell(gpx, nx, nz):
         assert np.array_equal(mw.interior(be.model.get("state")), mw.interior(got))
     assert stops > 0
     ex.clear(), be.clear(), word.destroy(), s.destroy()
+
+
+def _same_bits_behind_stops(gpx, ex, data, names, transport, trials=8):
+    """Runs of a preemptible executor that are stopped up to four times each, anywhere, end with the bits of an
+    uninterrupted one."""
+    word, s = gpx.PreemptWord(transport), gpx.Stream(1)
+    ex.set_word(word)
+    ex.set_input("data", data)
+    ex.execute(s)
+    s.sync()
+    want = {k: ex.model.get(k) for k in names}
+    t0 = time.perf_counter()
+    ex.execute(s)
+    s.sync()
+    run = time.perf_counter() - t0
+    rng, stops = np.random.default_rng(11), 0
+    for _ in range(trials):
+        ex.set_input("data", data * 0)
+        ex.execute(s)
+        s.sync()  # nothing stale can pass
+        ex.set_input("data", data)
+        word.clear()
+        time.sleep(0.001)
+        ex.execute(s)
+        for turn in range(40):
+            if turn < 4:
+                until = time.perf_counter() + float(rng.uniform(0, run / 4))
+                while time.perf_counter() < until:
+                    pass
+                word.raise_()
+            s.sync()
+            word.clear()
+            time.sleep(0.0005)
+            if ex.resume(s) == -1:
+                break
+            stops += 1
+        else:
+            raise AssertionError("does not end")
+        s.sync()
+        assert ex.error() == (0, 0)
+        for k in names:
+            assert np.array_equal(ex.model.get(k), want[k]), k
+    assert stops > 0
+    ex.clear(), word.destroy(), s.destroy()
+
+
+# More rows than 32 an SM and several tiles a CTA: two tiles are claimed ahead of the one that is worked on.
+@pytest.mark.parametrize("width,dtype", [(768, "float16"), (768, "float32"), (1024, "bfloat16"), (136, "float32")])
+@pytest.mark.parametrize("transport", [0, 1])
+def test_layernorm_of_many_rows_ends_with_the_same_bits_after_a_stop(gpx, tmp_path, width, dtype, transport):
+    batch, seq = 6001, 8
+    g = _Graph(batch, dtype)
+    ids = g.input(batch, seq, ids=True)
+    tables = [g.add(_param(k, 1.0, "table"), s) for k, s in (("word", [50, width]), ("pos", [64, width]))]
+    names = ["emb"] + [f"ln{i}" for i in range(10)]
+    x = None
+    for name in names:
+        w, b = (g.add(_param(f"{name}.{k}"), [width]) for k in ("weight", "bias"))
+        x = g.op(name, "gpx_layer_norm", ([ids, *tables] if x is None else [x]) + [w, b], [batch, seq, width])
+    w, b = (g.add(_param("heads." + k), [width]) for k in ("weight", "bias"))
+    g.op("heads", "gpx_layer_norm", [x, w, b], [batch, seq, width])
+    ex = g.load(gpx, tmp_path / "ln", gpx.BLPExecutor)
+    info = ex.model.get_kernel_info(0)
+    assert info["total_tiles"] > 3 * info["launch_params"][0]
+    rng = np.random.default_rng(width)
+    for name in names + ["heads"]:
+        ex.model.set(name + ".weight", rng.normal(1, 0.1, width).astype(np.float32))
+        ex.model.set(name + ".bias", rng.normal(0, 0.1, width).astype(np.float32))
+    _same_bits_behind_stops(gpx, ex, rng.integers(0, 50, (batch, seq)).astype(np.int64), ["emb", "ln4", "ln9"], transport, trials=6)
