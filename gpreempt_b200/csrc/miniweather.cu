@@ -383,14 +383,14 @@ miniweather_x_kernel(const __grid_constant__ StencilParams p, BlpArgs blp) {
     const Grid g = grid_of(p);
     const float hv_coef = __fdiv_rn(__fmul_rn(-kHvBeta, p.dx), __fmul_rn(16.f, p.dt));
     const float inv_dx = __frcp_rn(p.dx);
-    __shared__ int s_tile[2];
+    __shared__ int s_tile[kClaimSlots];
     int tile, next = -1, iter = 0;
     // With a CTA for every tile each has one: a second claim would be two round trips to L2 for nothing.
     const bool more = blp.total_tiles > (int)gridDim.x;
     if (dynamic) {
-        if (threadIdx.x == 0) s_tile[0] = blp_claim(blp, 0);
+        if (threadIdx.x == 0) s_tile[claim_slot(0)] = blp_claim(blp, 0);
         __syncthreads();
-        tile = s_tile[0];
+        tile = s_tile[claim_slot(0)];
     } else {
         tile = blp_claim(blp, 0);
     }
@@ -400,9 +400,9 @@ miniweather_x_kernel(const __grid_constant__ StencilParams p, BlpArgs blp) {
         fetch_row<VEC>(p, g, now, s_stage[warp][0], lane);
         if (more) {
             if (dynamic) {
-                if (threadIdx.x == 0) s_tile[1] = blp_claim(blp, 1);
+                if (threadIdx.x == 0) s_tile[claim_slot(1)] = blp_claim(blp, 1);
                 __syncthreads();
-                next = s_tile[1];
+                next = s_tile[claim_slot(1)];
             } else {
                 next = blp_claim(blp, 1);
             }
@@ -425,9 +425,9 @@ miniweather_x_kernel(const __grid_constant__ StencilParams p, BlpArgs blp) {
         work_row<VEC>(p, g, now, s_stage[warp][iter & 1], lane, hv_coef, inv_dx);
         ++iter;
         if (dynamic && next >= 0) {  // (next is the same for the whole CTA)
-            if (threadIdx.x == 0) s_tile[iter & 1] = after < blp.total_tiles ? after : -1;
+            if (threadIdx.x == 0) s_tile[claim_slot(iter + 1)] = after < blp.total_tiles ? after : -1;
             __syncthreads();
-            after = s_tile[iter & 1];
+            after = s_tile[claim_slot(iter + 1)];
         } else {
             __syncwarp();  // the stage is the tile's after next
         }

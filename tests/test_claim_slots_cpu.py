@@ -10,7 +10,7 @@ from gpreempt_b200 import build as gpx_build
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "gpreempt_b200", "csrc")
-KERNELS = {"layernorm": ("transformer.cu", "layernorm_kernel")}
+KERNELS = {"layernorm": ("transformer.cu", "layernorm_kernel"), "miniweather_x": ("miniweather.cu", "miniweather_x_kernel")}
 
 
 @pytest.fixture(scope="module")
