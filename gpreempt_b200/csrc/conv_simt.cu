@@ -1055,16 +1055,19 @@ __device__ __forceinline__ PixelAt pixel_at(unsigned e, int C8, int Wo, int Ho) 
 // (MobileNetV2 b1, us a layer: 4.4 a tap at a time, 3.3 to 4.9 with nine in flight and addresses behind the wait,
 // 2.5 to 3.7 like this).
 //
-// BATCH: taps of a 3x3 filter in flight at once, where the tensor is a tile or two per CTA and the filter has
-// nine; 0: a tap at a time (other filter sizes, strides and row orders).
+// BATCH: taps of a 3x3 filter in flight at once.  Nine where all vectors are at work at once at two CTAs an SM; three (a
+// filter row) in larger tensors that the strips below do not take (fewer than four vectors a thread, rows stored with a
+// border, strides from three on), which want the occupancy that the registers of nine take; 0: a tap at a time (other
+// filter sizes), at that occupancy too.  Six such layers between a 1x1 layer and a classifier, us, all with the registers
+// of nine / like this: 3x3 over padded rows, 32 images of 56x56x64 bf16 343 / 258, stride 3 over the same image 87 / 74,
+// stride 2, 14x14x512 76 / 67; 7x7, 32 images of 14x14x512 float32 584 / 432.
 struct DwElem {
     long long in;    // element offset of tap (0, 0) in a plain input (it may lie outside)
     size_t out;      // element offset of the output
     int c0;
     unsigned taps;   // of a 3x3 filter: inside the image
 };
-__device__ __forceinline__ DwElem dw_elem(const DwConvParams &p, unsigned e, int C8) {
-    const PixelAt at = pixel_at(e, C8, p.out.W, p.out.H);
+__device__ __forceinline__ DwElem dw_elem(const DwConvParams &p, const PixelAt &at) {
     DwElem a;
     a.c0 = at.c8 * 8;
     const int h0 = at.ho * p.stride - p.pad, w0 = at.wo * p.stride - p.pad;
@@ -1081,7 +1084,7 @@ __device__ __forceinline__ DwElem dw_elem(const DwConvParams &p, unsigned e, int
 }
 
 template <int BATCH, bool TWO>
-__global__ void __launch_bounds__(kPoolThreads, 2)
+__global__ void __launch_bounds__(kPoolThreads, BATCH == 9 ? 2 : 4)
 dwconv_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
     extern __shared__ float s_w[];  // [k * k][C], or nothing where it does not fit
     __shared__ int s_tile;
@@ -1089,8 +1092,6 @@ dwconv_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
     const int C = p.out.C;
     const int C8 = p.channels / 8;
     const int H = p.in.l.H, W = p.in.l.W;
-    const bool plain = p.in.l.order == ACT_PLAIN;
-    const long long row_step = (long long)p.in.l.Ws * p.in.l.C;
     const unsigned total = (unsigned)p.out.N * p.out.H * p.out.W * C8;  // < 2^31, checked when the model is built
     const float *wts = p.w;
     if (p.w_in_smem) {
@@ -1101,80 +1102,113 @@ dwconv_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
     }
     unsigned known = (unsigned)blockIdx.x * p.tile_elems + threadIdx.x;  // found ahead for a static schedule
     if (dynamic || known >= total) known = ~0u;
-    const DwElem ahead = dw_elem(p, known == ~0u ? 0 : known, C8);
+    const PixelAt first = pixel_at(known == ~0u ? 0 : known, C8, p.out.W, p.out.H);
+    DwElem ahead;
     float4 bias_a = make_float4(0.f, 0.f, 0.f, 0.f), bias_b = bias_a;
     auto fetch_bias = [&](int c0) {
         if (!p.bias) return;
         bias_a = __ldg(reinterpret_cast<const float4 *>(p.bias + c0));
         bias_b = __ldg(reinterpret_cast<const float4 *>(p.bias + c0) + 1);
     };
-    if (BATCH == 9) fetch_bias(ahead.c0);
+    if constexpr (BATCH == 9) {
+        ahead = dw_elem(p, first);
+        fetch_bias(ahead.c0);
+    }
     __syncthreads();
     pdl_enter();
     if (threadIdx.x == 0) trace_begin(blp);
     TileClaims claims(blp, dynamic, s_tile);
+    const int fmt = TWO ? (int)PF_SPLIT : p.in.l.fmt;
     for (int tile = claims.first(); tile >= 0; tile = claims.next()) {
         const unsigned begin = (unsigned)tile * p.tile_elems;
         const unsigned end = begin + p.tile_elems < total ? begin + p.tile_elems : total;
         for (unsigned e = begin + threadIdx.x; e < end; e += kPoolThreads) {
-            const DwElem at = e == known ? ahead : dw_elem(p, e, C8);
             float2 acc[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[j] = make_float2(0.f, 0.f);
-            auto tap = [&](const float (&x)[8], int t) {
-                const float4 *wv = reinterpret_cast<const float4 *>(wts + (size_t)t * C + at.c0);
+            auto tap = [&](const float (&x)[8], int t, int c0) {
+                const float4 *wv = reinterpret_cast<const float4 *>(wts + (size_t)t * C + c0);
                 const float4 a = wv[0], b = wv[1];
-                acc[0] = fma2(make_float2(x[0], x[1]), make_float2(a.x, a.y), acc[0]);
-                acc[1] = fma2(make_float2(x[2], x[3]), make_float2(a.z, a.w), acc[1]);
-                acc[2] = fma2(make_float2(x[4], x[5]), make_float2(b.x, b.y), acc[2]);
-                acc[3] = fma2(make_float2(x[6], x[7]), make_float2(b.z, b.w), acc[3]);
+                if (BATCH == 9) {
+                    acc[0] = fma2(make_float2(x[0], x[1]), make_float2(a.x, a.y), acc[0]);
+                    acc[1] = fma2(make_float2(x[2], x[3]), make_float2(a.z, a.w), acc[1]);
+                    acc[2] = fma2(make_float2(x[4], x[5]), make_float2(b.x, b.y), acc[2]);
+                    acc[3] = fma2(make_float2(x[6], x[7]), make_float2(b.z, b.w), acc[3]);
+                } else {
+                    acc[0].x = fmaf(x[0], a.x, acc[0].x), acc[0].y = fmaf(x[1], a.y, acc[0].y);
+                    acc[1].x = fmaf(x[2], a.z, acc[1].x), acc[1].y = fmaf(x[3], a.w, acc[1].y);
+                    acc[2].x = fmaf(x[4], b.x, acc[2].x), acc[2].y = fmaf(x[5], b.y, acc[2].y);
+                    acc[3].x = fmaf(x[6], b.z, acc[3].x), acc[3].y = fmaf(x[7], b.w, acc[3].y);
+                }
             };
-            if (BATCH != 0) {
-                constexpr int B = BATCH ? BATCH : 1;
-                const int fmt = TWO ? (int)PF_SPLIT : p.in.l.fmt;
+            size_t out;
+            if constexpr (BATCH == 9) {
+                const PixelAt px = e == known ? first : pixel_at(e, C8, p.out.W, p.out.H);
+                const DwElem at = e == known ? ahead : dw_elem(p, px);
+                out = at.out;
+                uint4 ra[9], rb[TWO ? 9 : 1];
+                if (p.in.l.order == ACT_PLAIN) {
+                    const long long row_step = (long long)p.in.l.Ws * p.in.l.C;
 #pragma unroll
-                for (int t0 = 0; t0 < 9; t0 += B) {
-                    uint4 ra[B], rb[TWO ? B : 1];
-                    if (plain) {
+                    for (int t = 0; t < 9; ++t)
+                        if (at.taps >> t & 1)
+                            planes_fetch8(p.in.hi, p.in.lo, (size_t)(at.in + t / 3 * row_step + t % 3 * p.in.l.C), fmt, ra[t], rb[TWO ? t : 0]);
+                } else {
 #pragma unroll
-                        for (int t = 0; t < B; ++t)
-                            if (at.taps >> (t0 + t) & 1)
-                                planes_fetch8(p.in.hi, p.in.lo, (size_t)(at.in + (t0 + t) / 3 * row_step + (t0 + t) % 3 * p.in.l.C), fmt, ra[t],
-                                              rb[TWO ? t : 0]);
-                    } else {
-                        const PixelAt px = pixel_at(e, C8, p.out.W, p.out.H);
+                    for (int t = 0; t < 9; ++t)
+                        if (at.taps >> t & 1)
+                            planes_fetch8(p.in.hi, p.in.lo,
+                                          (size_t)layout_row(p.in.l, px.n, px.ho * p.stride - p.pad + t / 3, px.wo * p.stride - p.pad + t % 3) *
+                                                  p.in.l.C + at.c0,
+                                          fmt, ra[t], rb[TWO ? t : 0]);
+                }
+                claims.ahead();
+                if (e != known) fetch_bias(at.c0);
 #pragma unroll
-                        for (int t = 0; t < B; ++t)
-                            if (at.taps >> (t0 + t) & 1)
-                                planes_fetch8(p.in.hi, p.in.lo,
-                                              (size_t)layout_row(p.in.l, px.n, px.ho * p.stride - p.pad + (t0 + t) / 3,
-                                                                 px.wo * p.stride - p.pad + (t0 + t) % 3) * p.in.l.C + at.c0,
-                                              fmt, ra[t], rb[TWO ? t : 0]);
-                    }
-                    if (t0 == 0) claims.ahead();
-                    if (t0 == 0 && !(BATCH == 9 && e == known)) fetch_bias(at.c0);
-#pragma unroll
-                    for (int t = 0; t < B; ++t) {
-                        if (!(at.taps >> (t0 + t) & 1)) continue;
-                        float x[8];
-                        planes_decode8(ra[t], rb[TWO ? t : 0], fmt, x);
-                        tap(x, t0 + t);
-                    }
+                for (int t = 0; t < 9; ++t) {
+                    if (!(at.taps >> t & 1)) continue;
+                    float x[8];
+                    planes_decode8(ra[t], rb[TWO ? t : 0], fmt, x);
+                    tap(x, t, at.c0);
                 }
             } else {
-                fetch_bias(at.c0);
-                const PixelAt px = pixel_at(e, C8, p.out.W, p.out.H);
-                for (int fh = 0; fh < p.k; ++fh) {
-                    const int hi = px.ho * p.stride - p.pad + fh;
-                    if (hi < 0 || hi >= H) continue;
-                    for (int fw = 0; fw < p.k; ++fw) {
-                        const int wi = px.wo * p.stride - p.pad + fw;
-                        if (wi < 0 || wi >= W) continue;
-                        float x[8];
-                        planes_load8(p.in.hi, p.in.lo, (size_t)layout_row(p.in.l, px.n, hi, wi) * p.in.l.C + at.c0, p.in.l.fmt, x);
-                        tap(x, fh * p.k + fw);
+                const PixelAt px = BATCH == 0 && e == known ? first : pixel_at(e, C8, p.out.W, p.out.H);
+                const int c0 = px.c8 * 8, h0 = px.ho * p.stride - p.pad, w0 = px.wo * p.stride - p.pad;
+                const int k = BATCH ? 3 : p.k;
+#pragma unroll 1
+                for (int fh = 0; fh < k; ++fh) {
+                    const int hi = h0 + fh;
+                    if constexpr (BATCH == 3) {
+                        uint4 ra[3], rb[TWO ? 3 : 1];
+                        bool ok[3];
+#pragma unroll
+                        for (int t = 0; t < 3; ++t) {
+                            const int wi = w0 + t;
+                            ok[t] = hi >= 0 && hi < H && wi >= 0 && wi < W;
+                            if (ok[t])
+                                planes_fetch8(p.in.hi, p.in.lo, (size_t)layout_row(p.in.l, px.n, hi, wi) * p.in.l.C + c0, fmt, ra[t], rb[TWO ? t : 0]);
+                        }
+                        if (fh == 0) claims.ahead();
+#pragma unroll
+                        for (int t = 0; t < 3; ++t) {
+                            if (!ok[t]) continue;
+                            float x[8];
+                            planes_decode8(ra[t], rb[TWO ? t : 0], fmt, x);
+                            tap(x, fh * 3 + t, c0);
+                        }
+                    } else {
+                        if (hi < 0 || hi >= H) continue;
+                        for (int fw = 0; fw < k; ++fw) {
+                            const int wi = w0 + fw;
+                            if (wi < 0 || wi >= W) continue;
+                            float x[8];
+                            planes_load8(p.in.hi, p.in.lo, (size_t)layout_row(p.in.l, px.n, hi, wi) * p.in.l.C + c0, p.in.l.fmt, x);
+                            tap(x, fh * k + fw, c0);
+                        }
                     }
                 }
+                fetch_bias(c0);
+                out = (size_t)layout_row(p.out, px.n, px.ho, px.wo) * C + c0;
             }
             float f[8];
 #pragma unroll
@@ -1184,7 +1218,7 @@ dwconv_kernel(const __grid_constant__ DwConvParams p, BlpArgs blp) {
                 f[4] += bias_b.x, f[5] += bias_b.y, f[6] += bias_b.z, f[7] += bias_b.w;
             }
             apply_act_n(f, p.act);
-            planes_store8(p.out_hi, p.out_lo, at.out, TWO ? (int)PF_SPLIT : p.out.fmt, f);
+            planes_store8(p.out_hi, p.out_lo, out, TWO ? (int)PF_SPLIT : p.out.fmt, f);
         }
     }
     if (threadIdx.x == 0) trace_end(blp, claims.done());
@@ -1294,14 +1328,18 @@ static auto dwconv_instance(const DwConvParams &p) {
         return two ? dwconv_strip_kernel<2, true> : dwconv_strip_kernel<2, false>;
     }
     if (p.k != 3) return two ? dwconv_kernel<0, true> : dwconv_kernel<0, false>;
-    return two ? dwconv_kernel<9, true> : dwconv_kernel<9, false>;
+    if (p.small) return two ? dwconv_kernel<9, true> : dwconv_kernel<9, false>;
+    return two ? dwconv_kernel<3, true> : dwconv_kernel<3, false>;
 }
 static size_t dwconv_smem(const DwConvParams &p) { return p.w_in_smem ? (size_t)p.k * p.k * p.out.C * sizeof(float) : 0; }
 
 // Tiles, form and grid of a layer whose shapes, filter and stride are set.  Strips of four pixels where the tensor
-// has more than four tiles of 256 vectors an SM; below that a thread per pixel has more threads at work.
+// has more than four tiles of 256 vectors an SM; below that a thread per pixel has more threads at work.  Nine taps in flight
+// up to two tiles an SM, which is what their registers leave resident (MobileNetV2, us a latency-critical request with
+// the line at two / at four tiles: 2 images bf16 204 / 210, 8 images 277 / 283, float32 the same).
 int dwconv_plan(DwConvParams &p, int sm_count) {
     const long long pixels = (long long)p.out.N * p.out.H * p.out.W, c8 = p.channels / 8;
+    p.small = pixels * c8 <= 2LL * 256 * sm_count;
     p.strip = p.k == 3 && p.in.l.order == ACT_PLAIN && (p.stride == 1 || p.stride == 2) && pixels * c8 > 4LL * 256 * sm_count;
     const int len = dw_strip(p.stride, p.out.fmt == PF_SPLIT);
     const long long total = p.strip ? (long long)p.out.N * p.out.H * ((p.out.W + len - 1) / len) * c8 : pixels * c8;

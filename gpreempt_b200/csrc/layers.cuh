@@ -310,6 +310,7 @@ struct DwConvParams {
     bf16_bits *out_hi, *out_lo;
     ActLayout out;
     int k, stride, pad, act;
+    int small;           // 1: at most two tiles an SM: latency, not occupancy
     int strip;           // 1: a thread produces four pixels of a row
     int w_in_smem;       // 1: the filter is copied to shared memory once per CTA
     int total_tiles;

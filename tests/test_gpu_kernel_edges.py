@@ -504,3 +504,35 @@ def test_layernorm_of_many_rows_ends_with_the_same_bits_after_a_stop(gpx, tmp_pa
         ex.model.set(name + ".weight", rng.normal(1, 0.1, width).astype(np.float32))
         ex.model.set(name + ".bias", rng.normal(0, 0.1, width).astype(np.float32))
     _same_bits_behind_stops(gpx, ex, rng.integers(0, 50, (batch, seq)).astype(np.int64), ["emb", "ln4", "ln9"], transport, trials=6)
+
+
+# The forms beside the strips: nine taps in flight up to two tiles of 256 vectors an SM, three beyond (over rows stored
+# with a border, as a 3x3 layer beside it wants them, strides from three on, up to four tiles an SM), a tap at a time.
+@pytest.mark.parametrize("channels,n,hw", [(40, 1, 13), (64, 24, 56), (72, 21, 33)])
+@pytest.mark.parametrize("kernel,stride,border", [(3, 1, True), (3, 2, True), (3, 3, False), (3, 2, False), (5, 1, False), (5, 2, True), (7, 1, False)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_depthwise_forms(gpx, tmp_path, channels, n, hw, kernel, stride, border, dtype):
+    g = _Graph(n, dtype)
+    x = g.conv("a", g.input(n, 3, hw, hw), 64 if border else channels)
+    channels = g.shapes[x][1]
+    if border:
+        g.conv("beside", x, 64, 3, 1)
+    pad = kernel // 2
+    out = (hw + 2 * pad - kernel) // stride + 1
+    x = g.op("b", "gpx_depthwise_conv2d", [x, g.add(_param("b.weight", 0.2), [channels, 1, kernel, kernel]), g.add(_param("b.bias"), [channels])],
+             [n, channels, out, out], kernel=kernel, stride=stride, padding=pad, activation=1)
+    g.heads(x)
+    results = []
+    for cls in (gpx.BaseExecutor, gpx.BLPExecutor):
+        ex = g.load(gpx, tmp_path / cls.__name__, cls)
+        s, word = gpx.Stream(1), gpx.PreemptWord(1)
+        if cls is gpx.BLPExecutor:
+            ex.set_word(word)
+        ex.set_input("data", gpx.synth_normal(n * 3 * hw * hw, 2, 0).reshape(n, 3, hw, hw))
+        ex.execute(s)
+        s.sync()
+        assert ex.error() == (0, 0)
+        _close(ex.model.get("b"), _conv64(ex, "b", "a", dtype, pad=pad, stride=stride, groups=channels, act=1), dtype, "b")
+        results.append(ex.model.get("b"))
+        ex.clear(), s.destroy(), word.destroy()
+    assert np.array_equal(*results)
