@@ -1019,6 +1019,13 @@ dense_short_kernel(const __grid_constant__ DenseRowsParams p, BlpArgs blp) {
     if (threadIdx.x == 0) trace_end(blp, iter);
 }
 
+// The whole CTA reads every input row again for each of a tile's columns, from L1: it gets all of an SM's memory as cache.
+// Behind a kernel that uses it as shared memory it was left 28 KB of it, or not, by what ran between: 25088 -> 4096 of three
+// images 192 or 228 us float32, 105 or 140 bf16; 194 and 105 like this, and never the other.
+cudaError_t dense_rows_prepare() {
+    return cudaFuncSetAttribute(dense_rows_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+}
+
 cudaError_t dense_rows_launch(const DenseRowsParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
     // (input rows of the short form, beside its own variables, in the default 48 KB of shared memory)
     const size_t rows = (size_t)p.M * p.K * sizeof(float);

@@ -223,6 +223,7 @@ struct DenseRowsParams {
     int total_tiles;               // eight output columns per tile
 };
 constexpr int kDenseShortK = 2048;  // rows up to this length: one warp per column
+cudaError_t dense_rows_prepare();
 cudaError_t dense_rows_launch(const DenseRowsParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
 
 // Patch matrix of a convolution whose input has too few channels for the tensor-core kernel

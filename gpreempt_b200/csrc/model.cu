@@ -1039,6 +1039,7 @@ int finalize_model(gpx_model &m) {
                 kd.name = n.name;
                 kd.node = (int)ni;
                 kd.type = KernelType::DenseRows;
+                GPX_CUDA(dense_rows_prepare());
                 DenseRowsParams &q = kd.dense;
                 q.a_hi = in0.hi;
                 q.a_lo = in0.lo;
