@@ -416,8 +416,13 @@ __device__ __forceinline__ void init_tile(const GraphWlParams &p, int tile) {
 
 // PACK: PageRank's packed form (ids per lane and block), 0 = edge lists.  Six CTAs of the packed form on an SM hide
 // one another's barriers and copies.
-template <int ALGO, int PHASE, int PACK = 0>
-__global__ void __launch_bounds__(kGwThreads, PACK || (PHASE == GW_EDGES && (ALGO == GW_BFS || ALGO == GW_CC)) ? 6 : 1)
+// MANY: the search with six CTAs an SM instead of four, at the price of registers (40 and some spilled, not 55): where a
+// preemptible launch has more tiles than four CTAs an SM take at once, so that no CTA has to claim a second one.
+// Breadth-first search, us a run with four / six: 826 tiles of 10.6 M edges 488 / 401, of 2.1 M 487 / 438; 602 tiles 475 /
+// 454; 469 tiles 312 / 338; 47 tiles 73 / 81.  Launches that claim nothing keep their registers (469 tiles 375 / 339,
+// 391 tiles 215 / 257, 47 tiles 69 / 77, 826 tiles 619 / 654).
+template <int ALGO, int PHASE, int PACK = 0, bool MANY = false>
+__global__ void __launch_bounds__(kGwThreads, PACK || MANY || (PHASE == GW_EDGES && ALGO == GW_CC) ? 6 : 1)
 graphwl_kernel(const __grid_constant__ GraphWlParams p, BlpArgs blp) {
     pdl_enter();
     extern __shared__ float s_win[];
@@ -490,11 +495,12 @@ size_t window_bytes(const GraphWlParams &p) {
     return p.phase == GW_EDGES && p.pack ? (size_t)(p.win_max + 4) * sizeof(float) : 0;
 }
 
-GraphKernel pick_kernel(const GraphWlParams &p) {
+// many: of a preemptible launch with more tiles than the search's other form has CTAs resident
+GraphKernel pick_kernel(const GraphWlParams &p, bool many) {
     if (p.phase == GW_INIT) return graphwl_kernel<GW_BFS, GW_INIT>;
     if (p.phase == GW_VERTICES) return p.algo == GW_SSSP ? graphwl_kernel<GW_SSSP, GW_VERTICES> : graphwl_kernel<GW_CC, GW_VERTICES>;
     switch (p.algo) {
-        case GW_BFS: return graphwl_kernel<GW_BFS, GW_EDGES>;
+        case GW_BFS: return many ? graphwl_kernel<GW_BFS, GW_EDGES, 0, true> : graphwl_kernel<GW_BFS, GW_EDGES>;
         case GW_SSSP: return graphwl_kernel<GW_SSSP, GW_EDGES>;
         case GW_CC: return graphwl_kernel<GW_CC, GW_EDGES>;
         default: break;
@@ -756,17 +762,21 @@ bool split_name(const std::string &name, int &algo, std::string &path) {
 
 }  // namespace
 
-int graphwl_grid(const GraphWlParams &p, int total_tiles, int sm_count) {
+static int resident_ctas(const GraphWlParams &p, bool many, int sm_count) {
     int blocks = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, pick_kernel(p), kGwThreads, window_bytes(p));
-    if (blocks < 1) blocks = 1;
-    long long grid = (long long)blocks * sm_count;
-    if (grid > total_tiles) grid = total_tiles;
-    return grid < 1 ? 1 : (int)grid;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, pick_kernel(p, many), kGwThreads, window_bytes(p));
+    return std::max(blocks, 1) * sm_count;
+}
+
+int graphwl_plan(GraphWlParams &p, int total_tiles, int sm_count) {
+    const int resident = resident_ctas(p, false, sm_count);
+    p.many = p.algo == GW_BFS && p.phase == GW_EDGES && total_tiles > resident ? resident : 0;
+    return std::max(1, std::min(p.many ? resident_ctas(p, true, sm_count) : resident, total_tiles));
 }
 
 cudaError_t graphwl_launch(const GraphWlParams &p, int grid, const BlpArgs &blp, cudaStream_t s) {
-    return launch_layer(pick_kernel(p), grid, kGwThreads, window_bytes(p), s, p, blp);
+    const bool many = p.many && blp.preempted;
+    return launch_layer(pick_kernel(p, many), p.many && !many ? std::min(grid, p.many) : grid, kGwThreads, window_bytes(p), s, p, blp);
 }
 
 bool is_graph_workload(const std::string &name) {
@@ -879,10 +889,10 @@ int build_graph_workload(gpx_model &m, const std::string &name, const gpx_model_
         GraphWlParams p = base;
         p.phase = phase;
         p.iter = iter;
-        k.graphwl = p;
         k.threads = kGwThreads;
         k.total_tiles = phase == GW_EDGES ? edge_tiles : vertex_tiles;
-        k.grid = graphwl_grid(p, k.total_tiles, m.sm_count);
+        k.grid = graphwl_plan(p, k.total_tiles, m.sm_count);
+        k.graphwl = p;
         const char *what = phase == GW_INIT ? "init" : (phase == GW_EDGES ? "edges" : "vertices");
         k.name = std::string("graphwl_kernel.") + kAlgoNames[algo] + "." + what +
                  (phase == GW_INIT ? std::string() : "." + std::to_string(iter));

@@ -66,6 +66,7 @@ struct GraphWlParams {
     // window of deltas the tile can reach, at most kGwWindowMax ids long, in blocks of 32 x pack (a lane's
     // ids of a block next to one another, in the order deal_edges gives them), padded with the offset
     // behind the window, where the shared-memory copy holds a zero.
+    int many;                       // bfs: with more tiles than CTAs of the form of more registers are resident: their number
     int pack;                       // ids a lane holds per block: 1, 2, 4 or 8; 0 = lists in adj
     const uint16_t *packed;
     const unsigned *blk;            // [n + 1] first block of every vertex
@@ -75,7 +76,7 @@ struct GraphWlParams {
 };
 
 cudaError_t graphwl_launch(const GraphWlParams &p, int grid, const BlpArgs &blp, cudaStream_t s);
-int graphwl_grid(const GraphWlParams &p, int total_tiles, int sm_count);
+int graphwl_plan(GraphWlParams &p, int total_tiles, int sm_count);  // fills many and returns the grid
 
 // "bfs:<prefix>", "sssp:<prefix>", "cc:<prefix>", "pagerank:<prefix>".
 bool is_graph_workload(const std::string &name);

@@ -536,3 +536,26 @@ def test_depthwise_forms(gpx, tmp_path, channels, n, hw, kernel, stride, border,
         results.append(ex.model.get("b"))
         ex.clear(), s.destroy(), word.destroy()
     assert np.array_equal(*results)
+
+
+# Breadth-first search with as many tiles of 64 vertices as four CTAs an SM take, one more, and a last one of one vertex.
+@pytest.mark.parametrize("tiles,over", [(592, 0), (592, 1), (593, 0), (700, 1)])
+def test_search_tiles_around_the_resident_ctas(gpx, tmp_path, tiles, over):
+    from gpreempt_b200 import graph_files
+    from oracle import graphs
+
+    graphs.build()
+    prefix = str(tmp_path / "g.bel")
+    graph_files.write_synthetic(prefix, tiles * 64 + over, 12, 900, 3)
+    offsets, neighbours, _ = graph_files.read_bel(prefix)
+    want = graphs.bfs(offsets, neighbours)[0]
+    for cls in (gpx.BaseExecutor, gpx.BLPExecutor):
+        ex, word, s = cls(), gpx.PreemptWord(1), gpx.Stream(1)
+        ex.set_graph_path(prefix)
+        ex.init("bfs")
+        if cls is gpx.BLPExecutor:
+            ex.set_word(word)
+        ex.execute(s)
+        s.sync()
+        assert np.array_equal(ex.model.get("label").astype(np.uint64), np.asarray(want).astype(np.uint64))
+        ex.clear(), word.destroy(), s.destroy()
