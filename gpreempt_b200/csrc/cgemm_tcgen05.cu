@@ -974,7 +974,8 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&ctl->landed));
             volatile int never = 0;  // (a CTA that failed waits here as well, so that no store finds its memory gone)
-            if (!mbar_wait(smem_u32(&ctl->landed), 0, &never, kCWaitLimitNs + kCWaitLimitNs / 2)) fail(601);
+            // (at cluster scope: the stores that complete it are other CTAs')
+            if (!mbar_wait_cluster(smem_u32(&ctl->landed), 0, &never, kCWaitLimitNs + kCWaitLimitNs / 2)) fail(601);
 #pragma unroll
             for (int i = 0; i < kItems; ++i) {
                 if (!live[i]) continue;
