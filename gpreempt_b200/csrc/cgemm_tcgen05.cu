@@ -819,6 +819,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
         const uint32_t t_acc = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
         auto sums = [&](int c, float *f) {  // sixteen columns of this thread's row
             uint32_t u[16], w[16];
+            __syncwarp();  // (lanes with rows and lanes without part behind the columns before)
             tmem_ld_32x16(t_acc + c, u);
             if (TWO) tmem_ld_32x16(t_acc + BN + c, w);
             tmem_ld_wait();
@@ -940,6 +941,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     }
                 }
             }
+            __syncwarp();
             cluster_wait();  // every CTA of the cluster runs
             pdl_wait();      // the residual is the predecessor's business, everything above is not
             if (fin.res_hi)
@@ -1172,6 +1174,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                         for (int q = 0; q < CH / 16; ++q) ld_global_v8(res_hi + res_off + c + 16 * q, rh + 8 * q);
                         if (TWO) ld_global_v8(res_lo + res_off + c, rl);
                     }
+                    __syncwarp();  // (lanes with rows and lanes without part behind the piece before)
                     if constexpr (TWO) {
                         uint32_t t16[16], u16[16];
                         tmem_ld_32x16(t_acc + c, t16);
@@ -1317,6 +1320,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
     }
 
     tc_fence_before_sync();
+    __syncwarp();
     if (CL && (warp < 2 || warp >= Cfg::kPollWarp)) cluster_wait();
     __syncthreads();
     if (warp == 0 && lane == 0 && *abort_flag) {

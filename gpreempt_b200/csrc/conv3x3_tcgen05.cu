@@ -380,6 +380,7 @@ conv3x3_narrow_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 float f[32];
                 if constexpr (kFold) {
                     uint32_t l[32], m[32], r[32];
+                    __syncwarp();
                     tmem_ld_32x32(t_acc, l);
                     tmem_ld_32x32(t_acc + CO, m);
                     tmem_ld_32x32(t_acc + 2 * CO, r);
@@ -412,6 +413,7 @@ conv3x3_narrow_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                     }
                 } else {
                     uint32_t m[32];
+                    __syncwarp();  // (lanes with rows and lanes without part behind the half before)
                     tmem_ld_32x32(t_acc + 32 * half, m);
                     tmem_ld_wait();
 #pragma unroll
