@@ -1013,6 +1013,7 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
                 }
             }
         }
+        if (threadIdx.x == 64 && blp.trace && !*abort_flag) atomicAdd(blp.trace + 3, 1ull);
     } else {
         // ------------------------------------------------------------------ epilogue
         const int quarter = warp & 3;

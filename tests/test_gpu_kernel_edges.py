@@ -559,3 +559,21 @@ def test_search_tiles_around_the_resident_ctas(gpx, tmp_path, tiles, over):
         s.sync()
         assert np.array_equal(ex.model.get("label").astype(np.uint64), np.asarray(want).astype(np.uint64))
         ex.clear(), word.destroy(), s.destroy()
+
+
+# A traced latency-critical run counts the tiles of every kernel that is launched (a finishing kernel whose layer is reduced
+# inside its clusters is not).
+@pytest.mark.parametrize("model,dtype", [("resnet_tiny", "float32"), ("resnet50", "bfloat16"), ("mobilenet_v2", "bfloat16"), ("bert_tiny", "float16"),
+                                         ("densenet_tiny", "bfloat16")])
+def test_traced_latency_critical_runs_count_their_tiles(gpx, model, dtype):
+    ex = gpx.BaseExecutor()
+    ex.init(model, batch=1, seed=1, dtype=dtype, seq_len=16 if "bert" in model else 0)
+    ex.enable_trace(True)
+    ex.execute()
+    gpx.device_sync()
+    trace = ex.read_trace()
+    for i in range(ex.get_kernel_num()):
+        info = ex.model.get_kernel_info(i)
+        if not (info["name"].endswith(".finish") and trace[i, 3] == 0):
+            assert trace[i, 3] == info["total_tiles"], info["name"]
+    ex.clear()
