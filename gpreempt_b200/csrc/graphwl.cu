@@ -6,7 +6,7 @@
 
 #include <algorithm>
 #include <cstdlib>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <vector>
 
@@ -603,15 +603,14 @@ int packed_tile_verts(uint64_t n, int sm_count) {
 // Deals the `deg` ids of a vertex to `rows` rounds of 32 lanes, row by row: at[32 r + l] is the id lane l gathers in
 // round r, or kGwInfinity.  The banks of the window are ids modulo 32.  A round takes each bank's share of
 // what is left over the rounds that are left, from the fullest banks first, so that the reads of the fullest bank, added
-// up over the rounds, come near the least there can be.
-void deal_edges(const unsigned *ids, uint64_t deg, uint64_t rows, std::vector<unsigned> &sorted, std::vector<unsigned> &at) {
+// up over the rounds, come near the least there can be.  `sorted` has room for `deg` ids.
+void deal_edges(const unsigned *ids, uint64_t deg, uint64_t rows, unsigned *sorted, unsigned *at) {
     uint64_t start[33] = {0}, end[32];  // of a bank's ids not dealt yet, in `sorted`
     for (uint64_t i = 0; i < deg; ++i) ++start[(ids[i] & 31) + 1];
     for (int b = 0; b < 32; ++b) start[b + 1] += start[b];
     for (int b = 0; b < 32; ++b) end[b] = start[b];
-    sorted.resize(deg);
     for (uint64_t i = 0; i < deg; ++i) sorted[end[ids[i] & 31]++] = ids[i];
-    at.assign(rows * 32, kGwInfinity);
+    std::fill(at, at + rows * 32, kGwInfinity);
     uint64_t left = deg;
     unsigned char order[32];
     for (int i = 0; i < 32; ++i) order[i] = (unsigned char)i;
@@ -670,9 +669,10 @@ bool pack_lists(const std::vector<unsigned long long> &trow, const std::vector<u
     const unsigned per = 32u * (unsigned)pack;
     const uint64_t warp_verts = (uint64_t)tile_verts / (kGwThreads / 32);
     blk.resize(n + 1);
-    uint64_t blocks = 0, most = 0;
+    uint64_t blocks = 0, most = 0, longest = 0;  // (of a vertex: blocks of its list)
     for (uint64_t v = 0; v < n; ++v) {
         blk[v] = (unsigned)blocks;
+        longest = std::max<uint64_t>(longest, (trow[v + 1] - trow[v] + per - 1) / per);
         blocks += (trow[v + 1] - trow[v] + per - 1) / per;
         const uint64_t first = v / warp_verts * warp_verts;
         most = std::max(most, blocks - blk[first]);
@@ -681,8 +681,12 @@ bool pack_lists(const std::vector<unsigned long long> &trow, const std::vector<u
     blk[n] = (unsigned)blocks;
     if (most * n > 4 * warp_verts * std::max<uint64_t>(blocks, n)) return false;
     packed.resize(blocks * per);
-    auto fill = [&](uint64_t t0, uint64_t t1) {
-        std::vector<unsigned> sorted, at;
+    const uint64_t workers = std::min<uint64_t>(std::max(8u, std::min(32u, std::thread::hardware_concurrency())), std::max<uint64_t>(1, tiles / 64));
+    // (all memory here: an allocation that fails on a worker thread would end the process instead of the call)
+    const uint64_t room = longest * per;
+    std::vector<unsigned> scratch(workers * 2 * room);
+    auto fill = [&](uint64_t worker, uint64_t t0, uint64_t t1) noexcept {
+        unsigned *const sorted = scratch.data() + worker * 2 * room, *const at = sorted + room;
         for (uint64_t v = t0 * tile_verts; v < std::min<uint64_t>(n, t1 * tile_verts); ++v) {
             const uint2 w = win[v / tile_verts];
             const uint64_t blocks_v = blk[v + 1] - blk[v];
@@ -696,14 +700,13 @@ bool pack_lists(const std::vector<unsigned long long> &trow, const std::vector<u
         }
     };
     std::vector<std::thread> pool;
-    const uint64_t workers = std::min<uint64_t>(std::max(8u, std::min(32u, std::thread::hardware_concurrency())), std::max<uint64_t>(1, tiles / 64));
     pool.reserve(workers);
     for (uint64_t i = 0; i < workers; ++i) {
         const uint64_t t0 = tiles * i / workers, t1 = tiles * (i + 1) / workers;
         try {
-            pool.emplace_back(fill, t0, t1);
-        } catch (const std::system_error &) {
-            fill(t0, t1);  // no thread to be had
+            pool.emplace_back(fill, i, t0, t1);
+        } catch (const std::exception &) {
+            fill(i, t0, t1);  // no thread to be had
         }
     }
     for (auto &th : pool) th.join();
