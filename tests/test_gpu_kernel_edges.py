@@ -577,3 +577,40 @@ def test_traced_latency_critical_runs_count_their_tiles(gpx, model, dtype):
         if not (info["name"].endswith(".finish") and trace[i, 3] == 0):
             assert trace[i, 3] == info["total_tiles"], info["name"]
     ex.clear()
+
+
+# Stops inside the layers behind a batch norm whose mapped operand goes to tensor memory: few K blocks, whose tiles two groups
+# of epilogue warps drain in turn, and many; and float32, mapped in shared memory.
+@pytest.mark.parametrize("cin", [192, 704])
+@pytest.mark.parametrize("dtype,transport", [("bfloat16", 0), ("float16", 1), ("float32", 1)])
+def test_batch_norm_in_the_operand_ends_with_the_same_bits_after_a_stop(gpx, tmp_path, cin, dtype, transport):
+    n, hw, layers = 96, 28, 6
+    g = _Graph(n, dtype, pad_channels=True)
+    x = g.conv("in", g.input(n, 3, hw, hw), cin)
+    for i in range(layers):
+        x = g.op(f"norm{i}", "gpx_affine", [x, g.add(_param(f"norm{i}.weight"), [cin]), g.add(_param(f"norm{i}.bias"), [cin])], g.shapes[x],
+                 kernel=1, stride=1, padding=0, activation=1, in_channels=cin)
+        x = g.conv(f"b{i}", x, 128, act=1, std=0.06)
+        if i + 1 < layers:
+            x = g.conv(f"w{i}", x, cin)
+    g.heads(x)
+    ex = g.load(gpx, tmp_path / "norm", gpx.BLPExecutor)
+    rng = np.random.default_rng(cin)
+    for i in range(layers):
+        ex.model.set(f"norm{i}.weight", rng.normal(1, 0.3, cin).astype(np.float32))
+        ex.model.set(f"norm{i}.bias", rng.normal(0, 0.3, cin).astype(np.float32))
+    _same_bits_behind_stops(gpx, ex, gpx.synth_normal(n * 3 * hw * hw, 2, 0).reshape(n, 3, hw, hw), [f"b{i}" for i in range(layers)], transport)
+
+
+@pytest.mark.parametrize("cout,cin", [(32, 128), (64, 64)])
+def test_narrow_3x3_layers_in_bf16_end_with_the_same_bits_after_a_stop(gpx, tmp_path, cout, cin):
+    n, hw = 24, 56
+    g = _Graph(n, "bfloat16")
+    x = g.conv("in", g.input(n, 3, hw, hw), cin)
+    for i in range(8):
+        x = g.conv(f"n{i}", x, cout, 3, 1, act=1, std=0.05)
+        if cout != cin:
+            x = g.conv(f"w{i}", x, cin)
+    g.heads(x)
+    ex = g.load(gpx, tmp_path / "be", gpx.BLPExecutor)
+    _same_bits_behind_stops(gpx, ex, gpx.synth_normal(n * 3 * hw * hw, 2, 0).reshape(n, 3, hw, hw), [f"n{i}" for i in range(8)], 1)
