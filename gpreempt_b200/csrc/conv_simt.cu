@@ -317,10 +317,10 @@ struct TileClaims {
 // 3x3 max pooling (K = 3) and 2x2 pooling of either kind (K = 2), without an affine map.  Bound by how many loads
 // are under way: a thread requests all taps of its vector (of two planes, a row of them and the next one) before it
 // looks at any, the largest of 16-bit values is taken as they are, and division by reciprocals keeps the
-// registers of 24 to 40 warps an SM.  112x112x64, 64 images bf16, 3x3: 70 us at two CTAs an SM with fp32 maxima, 38
+// registers of 24 to 32 warps an SM.  112x112x64, 64 images bf16, 3x3: 70 us at two CTAs an SM with fp32 maxima, 38
 // like this (128 MB: 20 us); 299x299 Inception-v3 b16 fp16, first 3x3: 31 us, 14.
 template <int K, bool TWO>
-__global__ void __launch_bounds__(kPoolThreads, K == 3 ? (TWO ? 3 : 4) : (TWO ? 4 : 5))
+__global__ void __launch_bounds__(kPoolThreads, K == 3 ? (TWO ? 3 : 4) : 4)
 pool_window_kernel(const __grid_constant__ PoolParams p, BlpArgs blp) {
     pdl_enter();
     __shared__ int s_tile;
@@ -1386,9 +1386,11 @@ int pool_plan(PoolParams &p, int sm_count) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pool_instance(p), kPoolThreads, 0);
         if (per_sm < 1) per_sm = 1;
         // A small tensor is cut so that each CTA that fits runs one tile (ResNet's 3x3 at batch 1: 392 tiles of 64
-        // vectors on 296 CTAs were two rounds), a large one into tiles of whole CTAs.
+        // vectors on 296 CTAs were two rounds), a large one into tiles of whole CTAs.  2x2 windows take two warps a tile
+        // at least, and four CTAs an SM without spills (bf16, us six latency-critical layers: five CTAs and from 32
+        // vectors on / like this: 56x56x256 47 / 43, 28x28x512 of two images 38 / 35, 112x112x64 81 / 77).
         const long long slots = (long long)per_sm * sm_count, even = (total + slots - 1) / slots;
-        p.tile_elems = even <= 256 ? (int)std::max<long long>(32, (even + 7) / 8 * 8) : (t == 2 && even >= 1024 ? 512 : 256);
+        p.tile_elems = even <= 256 ? (int)std::max<long long>(t == 3 ? 32 : 64, (even + 7) / 8 * 8) : (t == 2 && even >= 1024 ? 512 : 256);
         p.by_c8 = FastDiv::of((unsigned)(p.channels / 8)), p.by_w = FastDiv::of((unsigned)p.out.W), p.by_h = FastDiv::of((unsigned)p.out.H);
     } else {
         // the cap is per unit of work: a copy or an affine map reads one tap per vector
