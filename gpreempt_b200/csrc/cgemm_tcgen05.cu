@@ -761,6 +761,13 @@ cgemm_tcgen05_kernel(const __grid_constant__ CgemmParams p, BlpArgs blp) {
             const TileAt t = tile_at(tile);
             for (; kb < t.main_kb; ++kb) {
                 if (turn == group) {
+                    // (a ring of three stages and two groups, or of eight and three: the round before may be another group's)
+                    if (ring_rounds_skipped(nst, Cfg::kAffGroups) &&
+                        !__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->ready[stage]), phase ^ 1, abort_flag, kCWaitLimitNs))) {
+                        if (lane == 0) fail(502);
+                        go = false;
+                        break;
+                    }
                     if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&ctl->full[stage]), phase, abort_flag, kCWaitLimitNs))) {
                         if (lane == 0) fail(501);
                         go = false;

@@ -80,6 +80,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
 }
 
+// Groups of warps that take the blocks of a ring in turn and wait for their own blocks alone: whether a group comes to a
+// stage in some of its rounds only.  A wait by parity tells a round from its neighbours and no further: while the block of
+// another group is still on its way to a stage, it finds the round before that complete and takes it for the one after.
+// (Copies do not land in the order they are asked for.)  Such a group first waits until the round before has been worked on.
+constexpr __host__ __device__ bool ring_rounds_skipped(int stages, int groups) { return stages % groups != 0; }
+
 // x / d for 0 <= x < 2^24 and d > 0 with `inv` = 1.0f / d: the float quotient is off by at most
 // one, which the remainder corrects.  An integer division by a run-time divisor is a chain of
 // ~30 dependent instructions; the epilogue decodes its tile and its row with six of them, about a
