@@ -517,10 +517,12 @@ attention_short_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
 
 // Tiles, form and threads of a launch.  The short form wherever it applies, except for many sequences of more
 // than 48 tokens, whose keys it stages four times as often (12 heads, us a layer, walking the keys / short: 32
-// sequences of 6 tokens 12.3 / 4.0, 32 of 33 36 / 25, 1 of 40 11.6 / 3.4, 48 of 64 71 / 79).
+// sequences of 6 tokens 12.3 / 4.0, 32 of 33 36 / 25, 1 of 40 11.6 / 3.4, 48 of 64 71 / 79).  The line at six tiles an SM:
+// DistilBERT float32, us a latency-critical request of 8, 10 and 12 sequences, 64 tokens 451 / 428, 482 / 484 and 495 / 533, 58 tokens
+// 437 / 417, 468 / 469 and 487 / 536, 52 tokens (a tile fewer of eight) 426 / 413, 453 / 444 and 469 / 474.
 void attention_plan(AttnParams &p, int sm_count, int &threads) {
     const int short_tiles = p.B * p.heads * ((p.S + kShortQueries - 1) / kShortQueries);
-    p.few_keys = p.S <= 48 || (p.S <= kShortKeys && short_tiles <= 8 * sm_count);
+    p.few_keys = p.S <= 48 || (p.S <= kShortKeys && short_tiles <= 6 * sm_count);
     p.total_tiles = p.few_keys ? short_tiles : p.B * p.heads * ((p.S + 31) / 32);
     threads = p.few_keys ? 32 * kShortQueries : kAttnThreads;
 }

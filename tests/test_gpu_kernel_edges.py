@@ -614,3 +614,9 @@ def test_narrow_3x3_layers_in_bf16_end_with_the_same_bits_after_a_stop(gpx, tmp_
     g.heads(x)
     ex = g.load(gpx, tmp_path / "be", gpx.BLPExecutor)
     _same_bits_behind_stops(gpx, ex, gpx.synth_normal(n * 3 * hw * hw, 2, 0).reshape(n, 3, hw, hw), [f"n{i}" for i in range(8)], 1)
+
+
+# Two heads of eight tiles each: the last batch whose queries get a warp each on 148 SMs, and the next.
+@pytest.mark.parametrize("batch", [55, 56])
+def test_attention_over_few_keys_at_the_line(gpx, batch):
+    test_attention_over_few_keys(gpx, batch, 64)
