@@ -214,7 +214,7 @@ attention_tc_kernel(const __grid_constant__ AttnParams p, BlpArgs blp) {
         if (tile < 0) break;
         next = -1;
         const At at = at_tile(tile);
-        const int head = at.head, b = at.b, q0 = at.qb * kFaQ, col0 = at.col0;
+        const int b = at.b, q0 = at.qb * kFaQ, col0 = at.col0;
         if (!fetched) fetch_first(at);
         if (issuer_v && steps > 0) fetch(at, sV, &p.tv, &ctl->bar_v[wg], 0);
         // S = Q K^T of block j (warp 0; the lane that issues it)

@@ -1254,6 +1254,10 @@ int finalize_model(gpx_model &m) {
         const int split_from = e_all ? atoi(e_all) : 8;
         // The 3x3 kernel for few output channels, from 1 024 rows on (below, K split over a cluster is
         // what a latency-critical request wants; DenseNet-201 b64 bf16 with its 64 growth layers of 14x14 and 28x28 images so: 4 072 -> 3 584 us).
+        // One list serves both kinds of executor.  Between the line and large batches, bf16, us a request, this kernel / the general one:
+        // latency-critical DenseNet-201 of 1, 2 and 4 images 1 076 / 1 076, 1 160 / 1 154 and 1 243 / 1 245, ResNet-50 250 / 250, 303 / 302 and
+        // 382 / 372, VGG-16 of two 341 / 350; best-effort DenseNet-201 2 054 / 2 081, 2 146 / 2 220 and 2 225 / 2 286, ResNet-50 511 / 522,
+        // 560 / 573 and 644 / 643.
         const char *e_narrow = getenv("GPX_CONV_NARROW");
         const bool narrow = m.fmt != PF_SPLIT && eff_k == 3 && n.stride == 1 && il.order == ACT_PADDED && !head && !aff && n.residual < 0 &&
                             p.m_rows > 1024 && conv3x3_narrow_fits(cout_st, eff_cin) && !(e_narrow && e_narrow[0] == '0');

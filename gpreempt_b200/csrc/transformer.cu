@@ -103,7 +103,8 @@ __device__ __forceinline__ Vec8 raw_decode(const LayerNormParams &p, int row, in
 // (a row is read and written once); what it waits for in practice is latency, so the next tile's rows are on
 // their way while this tile's are worked on, the claim after that is in flight beside them, gamma and
 // beta lie in shared memory, and the arithmetic is packed.  16 384 rows of 768 bf16: 18.9 us with a claim and a
-// load per tile and scalar arithmetic, 14.7 like this.
+// load per tile and scalar arithmetic, 15.2 like this (14.5 to 16.1 over the layers of BERT).  When the word goes up a CTA has up to three tiles to run (this one,
+// the next and the one just claimed): 6.0 us in the middle and 6.8 at most from the word being seen to the end.
 template <int NV, bool TWO, bool EMB>
 __global__ void __launch_bounds__(kTfThreads, NV <= 3 && !EMB ? 3 : 2)
 layernorm_kernel(const __grid_constant__ LayerNormParams p, BlpArgs blp) {
@@ -257,7 +258,7 @@ static auto layernorm_instance(const LayerNormParams &p, F &&f) {
 
 // A row over several warps up to 32 rows an SM: with fewer the chain is what counts, with more the loads under
 // way are.  One warp a row against several, 768 channels: 2 048 rows bf16 4.3 / 4.0 us, 4 096 rows 6.5 / 5.7 and
-// float32 8.4 / 6.6, 16 384 rows 14.7 / 16.7.
+// float32 8.4 / 6.6, 16 384 rows 15.2 / 16.6.
 void layernorm_plan(LayerNormParams &p, int sm_count, int &grid, int &threads) {
     p.few_rows = p.rows <= 32 * sm_count;
     const int nv = layernorm_vectors(p.H);
