@@ -45,8 +45,11 @@ int exec_launch(gpx_exec *e, size_t idx, cudaStream_t s) {
         // The cluster reduction has no stop / resume form: preemptible executors keep the workspace
         // and the finishing kernel.
         if (e->kind != GPX_EXEC_BASE) p.cluster_reduce = 0;
-        // The same instance serves latency-critical launches of one 64-column tile a CTA (a cluster of one).
-        if (e->kind == GPX_EXEC_BASE && k.tile == 64 && p.k_splits == 1 && !p.narrow && k.grid == k.total_tiles) p.cluster_reduce = 1;
+        // The same instance serves latency-critical launches of one 64-column tile a CTA (a cluster of one), except for two
+        // planes behind an affine map (us with the instance / without: ResNet-50 float32 of one image 313 / 324, bf16 250 / 255;
+        // DenseNet-201 bf16 1 087 / 1 099, but float32 of one to four 1 470 / 1 458, 1 543 / 1 531, 1 598 / 1 588 and 1 640 / 1 635).
+        const bool mapped_planes = p.fmt == PF_SPLIT && p.aff_scale;
+        if (e->kind == GPX_EXEC_BASE && k.tile == 64 && p.k_splits == 1 && !p.narrow && k.grid == k.total_tiles && !mapped_planes) p.cluster_reduce = 1;
         err = cgemm_launch(p, k.tile, k.grid, b, s);
     } else if (k.type == KernelType::SplitK) {
         // The convolution kernel before it has already finished the tiles (cluster reduction).
